@@ -1,10 +1,12 @@
-"""Build libb200cp.so in-tree with nvcc for sm_100a.
+"""Build libb200cp.so in-tree with nvcc for sm_100a, and the torch binding over it.
 
     python -m paralleltnnlayers_b200.build [--force] [--verbose]
 
 Each .cu under csrc/ is compiled to an object (rebuilt only when it or a header
 is newer) and linked into ``paralleltnnlayers_b200/libb200cp.so``.  The library
-has no dependency on torch; it links the CUDA runtime and NCCL only.
+has no dependency on torch; it links the CUDA runtime and NCCL only.  The one
+.cpp file there is the CPython / torch binding, ``paralleltnnlayers_b200/_C.so``,
+which links the library (found next to it) and is imported after torch.
 """
 from __future__ import annotations
 
@@ -19,6 +21,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "csrc", "_obj")
 LIB = os.path.join(PKG, "libb200cp.so")
+BINDING = os.path.join(PKG, "_C.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -63,7 +66,30 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_binding(force)
     return LIB
+
+
+def _build_binding(force):
+    src = os.path.join(CSRC, "torch_binding.cpp")
+    hdr = os.path.join(ROOT, "include", "b200cp.h")
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) > max(os.path.getmtime(src), os.path.getmtime(hdr)):
+        return
+    import sysconfig
+
+    import torch
+    tdir = os.path.dirname(torch.__file__)
+    inc = [os.path.join(ROOT, "include"), os.path.join(tdir, "include"),
+           os.path.join(tdir, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+           "/usr/local/cuda/include"]
+    cmd = ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", "-Wno-deprecated-declarations",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", src, "-o", BINDING]
+    cmd += [f for i in inc for f in ("-isystem" if i != inc[0] else "-I", i)]
+    cmd += ["-L" + os.path.join(tdir, "lib"), "-L" + PKG, "-l:libb200cp.so", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+            "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"the torch binding did not build:\n{r.stdout}\n{r.stderr}")
 
 
 if __name__ == "__main__":

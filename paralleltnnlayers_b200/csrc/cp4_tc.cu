@@ -31,6 +31,20 @@ PFN_encodeTiled get_encode_tiled() {
         q == cudaDriverEntryPointSuccess)
       fn = reinterpret_cast<PFN_encodeTiled>(p);
   });
+  // The driver call needs a current context, which a host thread that has made no runtime call yet (an autograd
+  // engine's worker) does not have; setting the device it is on binds the primary context.
+  static thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    CUcontext ctx = nullptr;
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool has = cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                     q == cudaDriverEntryPointSuccess &&
+                     reinterpret_cast<CUresult (*)(CUcontext*)>(p)(&ctx) == CUDA_SUCCESS && ctx != nullptr;
+    if (!has && cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
+    bound = true;
+  }
   return fn;
 }
 

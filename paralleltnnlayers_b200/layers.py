@@ -13,6 +13,18 @@ import math
 import torch
 from torch import nn
 
+_ops_module = None
+
+
+def _ops():
+    """The operators, loaded with the library at the first forward (the rank rules need neither)."""
+    global _ops_module
+    if _ops_module is None:
+        from . import ops
+        _ops_module = ops
+    return _ops_module
+
+
 DEFAULT_COMPRESSION_RATE = 0.1        # test/layers.py:16
 DEFAULT_FACTORIZATION_BASE = 16       # test/layers.py:17
 
@@ -99,8 +111,7 @@ class CP4Conv2d(nn.Module):
         self.bias = nn.Parameter(torch.zeros(out_channels)) if bias else None
 
     def forward(self, x):
-        from .ops import CP4Conv2dFunction
-        y = CP4Conv2dFunction.apply(x.contiguous(), self.FT, self.FC, self.FY, self.FX, self.pad, self.flags)
+        y = _ops().CP4Conv2dFunction.apply(x.contiguous(), self.FT, self.FC, self.FY, self.FX, self.pad, self.flags)
         return y if self.bias is None else y + self.bias.view(1, -1, 1, 1)
 
 
@@ -121,8 +132,7 @@ class CPConv2d(nn.Module):
         self.bias = nn.Parameter(torch.zeros(out_channels)) if bias else None
 
     def forward(self, x):
-        from .ops import CP3Conv2dFunction
-        y = CP3Conv2dFunction.apply(x.contiguous(), self.KT, self.KCin, self.KC, self.pad)
+        y = _ops().CP3Conv2dFunction.apply(x.contiguous(), self.KT, self.KCin, self.KC, self.pad)
         return y if self.bias is None else y + self.bias.view(1, -1, 1, 1)
 
 
@@ -149,8 +159,7 @@ class RCPConv2d(nn.Module):
         self.bias = nn.Parameter(torch.zeros(out_channels)) if bias else None
 
     def forward(self, x):
-        from .ops import RCPConv2dFunction
-        y = RCPConv2dFunction.apply(x.contiguous(), self.core, *self.factors)
+        y = _ops().RCPConv2dFunction.apply(x.contiguous(), self.core, *self.factors)
         return y if self.bias is None else y + self.bias.view(1, -1, 1, 1)
 
 
@@ -177,8 +186,8 @@ class CPDense(nn.Module):
         self.bias = nn.Parameter(torch.zeros(out_features)) if bias else None
 
     def forward(self, x):
-        from .ops import CPDenseFunction
-        lead = x.shape[:-1]
-        y = CPDenseFunction.apply(x.reshape(-1, x.shape[-1]).contiguous(), *self.factors)
-        y = y.reshape(*lead, -1)
+        if x.dim() == 2:
+            y = _ops().CPDenseFunction.apply(x.contiguous(), *self.factors)
+        else:
+            y = _ops().CPDenseFunction.apply(x.reshape(-1, x.shape[-1]).contiguous(), *self.factors).reshape(*x.shape[:-1], -1)
         return y if self.bias is None else y + self.bias

@@ -14,8 +14,14 @@ import ctypes as C
 
 import torch
 
-from . import _lib
-from ._lib import TensorShape, check, int_array, lib, ptr_array
+from ._lib import B200CPError, TensorShape, check, int_array, lib, ptr_array
+
+try:
+    from . import _C            # after torch and the library: the hot operators and the autograd nodes
+except ImportError as e:
+    raise ImportError("the torch binding (_C.so) is missing or does not match: build it with "
+                      f"`python -m paralleltnnlayers_b200.build` ({e})") from e
+_C.set_error_class(B200CPError)
 
 
 def _stream():
@@ -52,66 +58,26 @@ def _shape_from(inp, FT, FC, FY, FX, pad, in_is_upstream=False):
 # ---- CP4, C++ order ---------------------------------------------------------
 def cp4_conv2d_forward(Input, FT, FC, FY, FX, pad=1, flags=0):
     """``CP::Conv2dForward`` (Cuda_kernels/cp4Conv2d.cu:14-43): returns Out [N,T,H,W]."""
-    Input, FT, FC, FY, FX = (_dev(t, n) for t, n in ((Input, "Input"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(Input, FT, FC, FY, FX, pad)
-    out = torch.empty((s.N, s.T, s.H, s.W), device=Input.device, dtype=torch.float32)
-    with torch.cuda.device(Input.device):
-        check(lib.b200cp_cp4_fwd(C.byref(s), _p(Input), _p(FT), _p(FC), _p(FY), _p(FX), _p(out), _stream(), flags))
-    return out
+    return _C.cp4_forward(Input, FT, FC, FY, FX, pad, flags)
 
 
 def cp4_conv2d_backward_data(Upstream, FT, FC, FY, FX, pad=1, flags=0):
     """``CP::Conv2dBackwardData`` (Cuda_kernels/cp4Conv2d.cu:48-77): returns dX [N,C,H,W]."""
-    Upstream, FT, FC, FY, FX = (_dev(t, n) for t, n in
-                                ((Upstream, "Upstream"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(Upstream, FT, FC, FY, FX, pad, in_is_upstream=True)
-    out = torch.empty((s.N, s.C, s.H, s.W), device=Upstream.device, dtype=torch.float32)
-    with torch.cuda.device(Upstream.device):
-        check(lib.b200cp_cp4_bwd_data(C.byref(s), _p(Upstream), _p(FT), _p(FC), _p(FY), _p(FX), _p(out), _stream(),
-                                      flags))
-    return out
+    return _C.cp4_backward_data(Upstream, FT, FC, FY, FX, pad, flags)
 
 
 def cp4_conv2d_forward_backward_data(Input, Upstream, FT, FC, FY, FX, pad=1, flags=0, save=False):
     """Forward of ``Input`` and backward-data of ``Upstream`` in one call (one launch where the shape allows it): the
     two convolutions of a training step with frozen factors.  Returns ``(Out, dInput)``, with ``save`` also the rank
     planes ``(P, Q)`` for ``cp4_conv2d_backward_filter_saved``."""
-    Input, Upstream = _dev(Input, "Input"), _dev(Upstream, "Upstream")
-    FT, FC, FY, FX = (_dev(t, n) for t, n in ((FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(Input, FT, FC, FY, FX, pad)
-    if tuple(Upstream.shape) != (s.N, s.T, s.H, s.W):
-        raise ValueError("Upstream must be [N, T, H, W]")
-    U = torch.empty((s.N, s.T, s.H, s.W), device=Input.device, dtype=torch.float32)
-    dX = torch.empty_like(Input)
-    Pl = torch.empty((s.N, s.Rank, s.H, s.W), device=Input.device, dtype=torch.float32) if save else None
-    Ql = torch.empty_like(Pl) if save else None
-    with torch.cuda.device(Input.device):
-        check(lib.b200cp_cp4_fwd_bwd_data(C.byref(s), _p(Input), _p(Upstream), _p(FT), _p(FC), _p(FY), _p(FX), _p(U),
-                                          _p(dX), _p(Pl) if save else None, _p(Ql) if save else None, _stream(), flags))
-    return (U, dX, Pl, Ql) if save else (U, dX)
+    return _C.cp4_forward_backward_data(Input, Upstream, FT, FC, FY, FX, pad, flags, save)
 
 
 def cp4_conv2d_backward_filter(dLdO, In, FT, FC, FY, FX, pad=1, flags=0, packed=False):
     """The four factor gradients of ``CP::Conv2dBackwardFilter``
     (Cuda_kernels/cp4Conv2d.cu:83-153): returns (dFT, dFC, dFY, dFX), or the
     packed buffer [dFT|dFC|dFY|dFX] with ``packed=True`` (the allreduce unit)."""
-    dLdO, In, FT, FC, FY, FX = (_dev(t, n) for t, n in
-                                ((dLdO, "dLdO"), (In, "In"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(In, FT, FC, FY, FX, pad)
-    if tuple(dLdO.shape) != (s.N, s.T, s.H, s.W):
-        raise ValueError("dLdO must be [N,T,H,W]")
-    R = s.Rank
-    nT, nC, nY, nX = s.T * R, s.C * R, s.Y * R, s.X * R
-    dK = torch.empty(nT + nC + nY + nX, device=In.device, dtype=torch.float32)
-    with torch.cuda.device(In.device):
-        wsb = lib.b200cp_cp4_bwd_filter_workspace_bytes(C.byref(s), flags)
-        ws = torch.empty(max(wsb, 4) // 4, device=In.device, dtype=torch.float32)
-        check(lib.b200cp_cp4_bwd_filter(C.byref(s), _p(In), _p(dLdO), _p(FT), _p(FC), _p(FY), _p(FX), _p(dK), _p(ws),
-                                        ws.numel() * 4, _stream(), flags))
-    if packed:
-        return dK
-    return (dK[:nT].view(s.T, R), dK[nT:nT + nC].view(s.C, R), dK[nT + nC:nT + nC + nY].view(s.Y, R),
-            dK[nT + nC + nY:].view(s.X, R))
+    return _C.cp4_backward_filter(dLdO, In, FT, FC, FY, FX, pad, flags, packed)
 
 
 def cp4_conv2d_backward_filter_full(dLdO, In, Y, X, pad=1):
@@ -149,67 +115,22 @@ def allclose(A, B, tolerance=1e-3):
 def cp4_conv2d_step(X, dU, FT, FC, FY, FX, pad=1, flags=0):
     """One training step on device tensors (``b200cp_cp4_step``): returns (U, dX, dK_packed); the work forward,
     backward-data and backward-filter share is done once."""
-    X, dU, FT, FC, FY, FX = (_dev(t, n) for t, n in
-                             ((X, "X"), (dU, "dU"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(X, FT, FC, FY, FX, pad)
-    if tuple(dU.shape) != (s.N, s.T, s.H, s.W):
-        raise ValueError("dU must be [N,T,H,W]")
-    U = torch.empty((s.N, s.T, s.H, s.W), device=X.device, dtype=torch.float32)
-    dX = torch.empty_like(X)
-    dK = torch.empty((s.T + s.C + s.Y + s.X) * s.Rank, device=X.device, dtype=torch.float32)
-    with torch.cuda.device(X.device):
-        wsb = lib.b200cp_cp4_step_workspace_bytes(C.byref(s), flags)
-        ws = torch.empty(max(wsb, 4) // 4, device=X.device, dtype=torch.float32)
-        check(lib.b200cp_cp4_step(C.byref(s), _p(X), _p(dU), _p(FT), _p(FC), _p(FY), _p(FX), _p(U), _p(dX), _p(dK),
-                                  _p(ws), ws.numel() * 4, _stream(), flags))
-    return U, dX, dK
-
-
-def _shares_planes(s, flags):
-    """The library's own rule (``b200cp_cp4_shares_planes``): shape, path flags and its environment switches."""
-    return bool(lib.b200cp_cp4_shares_planes(C.byref(s), flags))
+    return _C.cp4_step(X, dU, FT, FC, FY, FX, pad, flags)
 
 
 def cp4_conv2d_forward_save(Input, FT, FC, FY, FX, pad=1, flags=0):
     """Forward that also returns its rank plane ``P = FC^T Input`` [N,R,H,W] (``b200cp_cp4_fwd_save``)."""
-    Input, FT, FC, FY, FX = (_dev(t, n) for t, n in ((Input, "Input"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(Input, FT, FC, FY, FX, pad)
-    out = torch.empty((s.N, s.T, s.H, s.W), device=Input.device, dtype=torch.float32)
-    P = torch.empty((s.N, s.Rank, s.H, s.W), device=Input.device, dtype=torch.float32)
-    with torch.cuda.device(Input.device):
-        check(lib.b200cp_cp4_fwd_save(C.byref(s), _p(Input), _p(FT), _p(FC), _p(FY), _p(FX), _p(out), _p(P), _stream(),
-                                      flags))
-    return out, P
+    return _C.cp4_forward_save(Input, FT, FC, FY, FX, pad, flags)
 
 
 def cp4_conv2d_backward_data_save(Upstream, FT, FC, FY, FX, pad=1, flags=0):
     """Backward-data that also returns its rank plane ``Q = FT^T Upstream`` (``b200cp_cp4_bwd_data_save``)."""
-    Upstream, FT, FC, FY, FX = (_dev(t, n) for t, n in
-                                ((Upstream, "Upstream"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(Upstream, FT, FC, FY, FX, pad, in_is_upstream=True)
-    out = torch.empty((s.N, s.C, s.H, s.W), device=Upstream.device, dtype=torch.float32)
-    Q = torch.empty((s.N, s.Rank, s.H, s.W), device=Upstream.device, dtype=torch.float32)
-    with torch.cuda.device(Upstream.device):
-        check(lib.b200cp_cp4_bwd_data_save(C.byref(s), _p(Upstream), _p(FT), _p(FC), _p(FY), _p(FX), _p(out), _p(Q),
-                                           _stream(), flags))
-    return out, Q
+    return _C.cp4_backward_data_save(Upstream, FT, FC, FY, FX, pad, flags)
 
 
 def cp4_conv2d_backward_filter_saved(dLdO, In, P, Q, FT, FC, FY, FX, pad=1, flags=0):
     """The four factor gradients from the saved rank planes (``b200cp_cp4_bwd_filter_saved``)."""
-    dLdO, In, P, Q, FY, FX = (_dev(t, n) for t, n in
-                              ((dLdO, "dLdO"), (In, "In"), (P, "P"), (Q, "Q"), (FY, "FY"), (FX, "FX")))
-    s = _shape_from(In, FT, FC, FY, FX, pad)
-    R = s.Rank
-    nT, nC, nY, nX = s.T * R, s.C * R, s.Y * R, s.X * R
-    dK = torch.empty(nT + nC + nY + nX, device=In.device, dtype=torch.float32)
-    with torch.cuda.device(In.device):
-        wsb = lib.b200cp_cp4_bwd_filter_saved_workspace_bytes(C.byref(s), flags)
-        ws = torch.empty(max(wsb, 4) // 4, device=In.device, dtype=torch.float32)
-        check(lib.b200cp_cp4_bwd_filter_saved(C.byref(s), _p(In), _p(dLdO), _p(P), _p(Q), _p(FY), _p(FX), _p(dK), _p(ws),
-                                              ws.numel() * 4, _stream(), flags))
-    return (dK[:nT].view(s.T, R), dK[nT:nT + nC].view(s.C, R), dK[nT + nC:nT + nC + nY].view(s.Y, R),
-            dK[nT + nC + nY:].view(s.X, R))
+    return _C.cp4_backward_filter_saved(dLdO, In, P, Q, FT, FC, FY, FX, pad, flags)
 
 
 def cp4_conv2d_step_host(X, dU, FT, FC, FY, FX, pad=1, flags=0, out=None):
@@ -292,77 +213,24 @@ def debug_cp4_tc(Input, FT, FC, FY, FX, pad=1, terms=3, p_floats=0):
 
 
 # ---- three-factor CP conv -----------------------------------------------------
-def _shape3(inp, KT, KCin, KC, pad, in_is_upstream=False):
-    if inp.dim() != 4 or KT.dim() != 2 or KCin.dim() != 2 or KC.dim() != 3:
-        raise ValueError("expected input [N,ch,H,W], KT [T,R], KCin [C,R], KC [Y,X,R]")
-    R = KT.shape[1]
-    if KCin.shape[1] != R or KC.shape[2] != R:
-        raise ValueError("all factors must have the same rank")
-    if inp.shape[1] != (KT.shape[0] if in_is_upstream else KCin.shape[0]):
-        raise ValueError("channel count of the input does not match the factor")
-    return tensor_shape(inp.shape[0], KCin.shape[0], inp.shape[2], inp.shape[3], KT.shape[0], KC.shape[0], KC.shape[1],
-                        R, pad)
-
-
 def cp3_conv2d_forward(Input, KT, KCin, KC, pad=1, flags=0):
     """Three-factor CP conv (``b200cp_cp3_fwd``): ``KT [T,R]``, ``KCin [C,R]``, free core ``KC [Y,X,R]``."""
-    Input, KT, KCin, KC = (_dev(t, n) for t, n in ((Input, "Input"), (KT, "KT"), (KCin, "KCin"), (KC, "KC")))
-    s = _shape3(Input, KT, KCin, KC, pad)
-    out = torch.empty((s.N, s.T, s.H, s.W), device=Input.device, dtype=torch.float32)
-    with torch.cuda.device(Input.device):
-        check(lib.b200cp_cp3_fwd(C.byref(s), _p(Input), _p(KT), _p(KCin), _p(KC), _p(out), _stream(), flags))
-    return out
+    return _C.cp3_forward(Input, KT, KCin, KC, pad, flags)
 
 
 def cp3_conv2d_backward_data(Upstream, KT, KCin, KC, pad=1, flags=0):
-    Upstream, KT, KCin, KC = (_dev(t, n) for t, n in ((Upstream, "Upstream"), (KT, "KT"), (KCin, "KCin"), (KC, "KC")))
-    s = _shape3(Upstream, KT, KCin, KC, pad, in_is_upstream=True)
-    out = torch.empty((s.N, s.C, s.H, s.W), device=Upstream.device, dtype=torch.float32)
-    with torch.cuda.device(Upstream.device):
-        check(lib.b200cp_cp3_bwd_data(C.byref(s), _p(Upstream), _p(KT), _p(KCin), _p(KC), _p(out), _stream(), flags))
-    return out
+    return _C.cp3_backward_data(Upstream, KT, KCin, KC, pad, flags)
 
 
 def cp3_conv2d_backward_filter(dLdO, In, KT, KCin, KC, pad=1, flags=0):
     """Factor gradients (dKT, dKCin, dKC) of the three-factor CP conv; 3x3 cores with pad 1."""
-    dLdO, In, KT, KCin, KC = (_dev(t, n) for t, n in
-                              ((dLdO, "dLdO"), (In, "In"), (KT, "KT"), (KCin, "KCin"), (KC, "KC")))
-    s = _shape3(In, KT, KCin, KC, pad)
-    R = s.Rank
-    nT, nC, nS = s.T * R, s.C * R, s.Y * s.X * R
-    dK = torch.empty(nT + nC + nS, device=In.device, dtype=torch.float32)
-    with torch.cuda.device(In.device):
-        wsb = lib.b200cp_cp3_bwd_filter_workspace_bytes(C.byref(s), flags)
-        ws = torch.empty(max(wsb, 4) // 4, device=In.device, dtype=torch.float32)
-        check(lib.b200cp_cp3_bwd_filter(C.byref(s), _p(In), _p(dLdO), _p(KT), _p(KCin), _p(KC), _p(dK), _p(ws),
-                                        ws.numel() * 4, _stream(), flags))
-    return dK[:nT].view(s.T, R), dK[nT:nT + nC].view(s.C, R), dK[nT + nC:].view(s.Y, s.X, R)
+    return _C.cp3_backward_filter(dLdO, In, KT, KCin, KC, pad, flags)
 
 
 def conv2d_cp_fused_nchw(U, K0, K1, K2, flags=0):
     """``Conv2dCpFusedNchw`` (Kernels/cp_fused_nchw.cc): K0 [C,R], K1 [FH,FW,R], K2 [R,T], SAME padding
     (test/test_conv2d_cp.py:33-38)."""
     return cp3_conv2d_forward(U, K2.t().contiguous(), K0, K1, pad=(K1.shape[0] - 1) // 2, flags=flags)
-
-
-class CP3Conv2dFunction(torch.autograd.Function):
-    """y = three-factor CP conv2d(x; KT, KCin, KC) with the fused backward kernels."""
-
-    @staticmethod
-    def forward(ctx, x, KT, KCin, KC, pad=1):
-        ctx.save_for_backward(x, KT, KCin, KC)
-        ctx.pad = pad
-        return cp3_conv2d_forward(x, KT, KCin, KC, pad)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, KT, KCin, KC = ctx.saved_tensors
-        dy = dy.contiguous()
-        dx = cp3_conv2d_backward_data(dy, KT, KCin, KC, ctx.pad) if ctx.needs_input_grad[0] else None
-        g = (None,) * 3
-        if any(ctx.needs_input_grad[1:4]):
-            g = cp3_conv2d_backward_filter(dy, x, KT, KCin, KC, ctx.pad)
-        return (dx, *g, None)
 
 
 # ---- TF custom-op order -----------------------------------------------------
@@ -386,94 +254,23 @@ def _modes(factors, what):
 def conv2d_rcp_fused_nchw(U, *kernels, flags=0):
     """``Conv2dRcpFusedNchw`` (Kernels/rcp_fused_nchw.cc:6-12): ``(U[N,S0..,H,W], K0[S0,T0,R], ..., KC[FH,FW,R])``
     -> ``V[N,T0..,H,W]``.  ``U`` may also be given as [N,C,H,W]."""
-    *A, KC = kernels
-    U = _dev(U, "input")
-    A = [_dev(a, f"kernel{k}") for k, a in enumerate(A)]
-    KC = _dev(KC, "kernelc")
-    cd, td, R = _modes(A, "conv2d_rcp_fused_nchw")
-    if KC.dim() != 3 or KC.shape[2] != R:
-        raise ValueError("kernelc must be [FH, FW, rank]")
-    Cc = 1
-    for c in cd:
-        Cc *= c
-    folded = U.dim() == 4
-    if not folded and tuple(U.shape[1:-2]) != tuple(cd):
-        raise ValueError("input modes do not match the kernels")
-    N, H, W = U.shape[0], U.shape[-2], U.shape[-1]
-    if U.numel() != N * Cc * H * W:
-        raise ValueError("input channel count does not match the kernels")
-    Tc = 1
-    for t in td:
-        Tc *= t
-    V = torch.empty((N, Tc, H, W), device=U.device, dtype=torch.float32)
-    with torch.cuda.device(U.device):
-        check(lib.b200cp_rcp_fwd(N, H, W, len(A), int_array(cd), int_array(td), R, KC.shape[0], KC.shape[1], _p(U),
-                                 ptr_array([a.data_ptr() for a in A]), _p(KC), _p(V), _stream(), flags))
-    return V if folded else V.view(N, *td, H, W)
+    return _C.rcp_forward(flags, U, kernels[-1], *kernels[:-1])
 
 
 def rcp_conv2d_backward(U, dV, *kernels, flags=0, need_dx=True, need_dw=True):
     """Gradients of ``conv2d_rcp_fused_nchw``: (dU, [dK_k], dKC)."""
-    *A, KC = kernels
-    U, dV = _dev(U, "input"), _dev(dV, "dV")
-    A = [_dev(a, f"kernel{k}") for k, a in enumerate(A)]
-    KC = _dev(KC, "kernelc")
-    cd, td, R = _modes(A, "rcp_conv2d_backward")
-    N, H, W = U.shape[0], U.shape[-2], U.shape[-1]
-    dU = torch.empty_like(U) if need_dx else None
-    dA = [torch.empty_like(a) for a in A] if need_dw else None
-    dS = torch.empty_like(KC) if need_dw else None
-    with torch.cuda.device(U.device):
-        wsb = lib.b200cp_rcp_bwd_workspace_bytes(N, H, W, len(A), int_array(cd), int_array(td), R, KC.shape[0],
-                                                 KC.shape[1], flags)
-        ws = torch.empty(max(wsb, 4) // 4, device=U.device, dtype=torch.float32)
-        check(lib.b200cp_rcp_bwd(N, H, W, len(A), int_array(cd), int_array(td), R, KC.shape[0], KC.shape[1], _p(U),
-                                 _p(dV), ptr_array([a.data_ptr() for a in A]), _p(KC),
-                                 _p(dU) if need_dx else None,
-                                 ptr_array([a.data_ptr() for a in dA]) if need_dw else None,
-                                 _p(dS) if need_dw else None, _p(ws), ws.numel() * 4, _stream(), flags))
-    return dU, dA, dS
+    return _C.rcp_backward(flags, need_dx, need_dw, U, dV, kernels[-1], *kernels[:-1])
 
 
 def dense_cp(U, *kernels, flags=0):
     """``DenseCp`` (Kernels/dense_cp.cc:6-12): ``(U[N,S0,S1,..], K0[S0,T0,R], ...)`` -> ``V[N,T0,T1,..]``
     (output dims are ``kernel_k.dim(1)``, Kernels/dense_cp.cc:86-91).  ``U`` may also be [N, I]."""
-    U = _dev(U, "input")
-    Fk = [_dev(f, f"kernel{k}") for k, f in enumerate(kernels)]
-    idims, odims, R = _modes(Fk, "dense_cp")
-    I = 1
-    for d in idims:
-        I *= d
-    O = 1
-    for d in odims:
-        O *= d
-    B = U.shape[0]
-    if U.numel() != B * I:
-        raise ValueError("input size does not match the kernels")
-    flat = U.dim() == 2
-    Y = torch.empty((B, O), device=U.device, dtype=torch.float32)
-    with torch.cuda.device(U.device):
-        check(lib.b200cp_dense_fwd(B, len(Fk), int_array(idims), int_array(odims), R, _p(U),
-                                   ptr_array([f.data_ptr() for f in Fk]), _p(Y), _stream(), flags))
-    return Y if flat else Y.view(B, *odims)
+    return _C.dense_forward(flags, U, *kernels)
 
 
 def dense_cp_backward(U, dV, *kernels, flags=0, need_dx=True, need_dw=True):
     """Gradients of ``dense_cp``: (dU, [dK_k])."""
-    U, dV = _dev(U, "input"), _dev(dV, "dV")
-    Fk = [_dev(f, f"kernel{k}") for k, f in enumerate(kernels)]
-    idims, odims, R = _modes(Fk, "dense_cp_backward")
-    B = U.shape[0]
-    dU = torch.empty_like(U) if need_dx else None
-    dF = [torch.empty_like(f) for f in Fk] if need_dw else None
-    with torch.cuda.device(U.device):
-        wsb = lib.b200cp_dense_bwd_workspace_bytes(B, len(Fk), int_array(idims), int_array(odims), R, flags)
-        ws = torch.empty(max(wsb, 4) // 4, device=U.device, dtype=torch.float32)
-        check(lib.b200cp_dense_bwd(B, len(Fk), int_array(idims), int_array(odims), R, _p(U), _p(dV),
-                                   ptr_array([f.data_ptr() for f in Fk]), _p(dU) if need_dx else None,
-                                   ptr_array([f.data_ptr() for f in dF]) if need_dw else None, _p(ws),
-                                   ws.numel() * 4, _stream(), flags))
-    return dU, dF
+    return _C.dense_backward(flags, need_dx, need_dw, U, dV, *kernels)
 
 
 # ---- the reference's "rebuild" variants: the undecomposed layer with the recomposed weight --------------------
@@ -574,59 +371,22 @@ def dense_cp_rebuild(U, *kernels):
 
 
 # ---- autograd wrappers ----------------------------------------------------------
-class CP4Conv2dFunction(torch.autograd.Function):
-    """y = CP4 conv2d(x; FT, FC, FY, FX) with the fused backward kernels."""
-
-    @staticmethod
-    def forward(ctx, x, FT, FC, FY, FX, pad=1, flags=0):
-        ctx.pad, ctx.flags = pad, flags
-        # with 3x3 filters the forward keeps its rank plane for the factor gradients (a quarter of x at C = 4R)
-        ctx.shared = (any(t.requires_grad for t in (FT, FC, FY, FX)) and x.dim() == 4 and
-                      _shares_planes(_shape_from(x, FT, FC, FY, FX, pad), flags))
-        if ctx.shared:
-            y, P = cp4_conv2d_forward_save(x, FT, FC, FY, FX, pad, flags)
-            ctx.save_for_backward(x, FT, FC, FY, FX, P)
-            return y
-        ctx.save_for_backward(x, FT, FC, FY, FX)
-        return cp4_conv2d_forward(x, FT, FC, FY, FX, pad, flags)
-
-    @staticmethod
-    def backward(ctx, dy):
-        dy = dy.contiguous()
-        if ctx.shared:
-            x, FT, FC, FY, FX, P = ctx.saved_tensors
-            dx, Q = cp4_conv2d_backward_data_save(dy, FT, FC, FY, FX, ctx.pad, ctx.flags)
-            g = cp4_conv2d_backward_filter_saved(dy, x, P, Q, FT, FC, FY, FX, ctx.pad, ctx.flags)
-            return (dx if ctx.needs_input_grad[0] else None, *g, None, None)
-        x, FT, FC, FY, FX = ctx.saved_tensors
-        dx = cp4_conv2d_backward_data(dy, FT, FC, FY, FX, ctx.pad, ctx.flags) if ctx.needs_input_grad[0] else None
-        g = (None,) * 4
-        if any(ctx.needs_input_grad[1:5]):
-            g = cp4_conv2d_backward_filter(dy, x, FT, FC, FY, FX, ctx.pad, ctx.flags)
-        return (dx, *g, None, None)
+# The nodes are native (csrc/torch_binding.cpp); each class keeps the ``apply`` its layer calls.
+class CP4Conv2dFunction:
+    """y = CP4 conv2d(x; FT, FC, FY, FX) with the fused backward kernels: ``apply(x, FT, FC, FY, FX, pad=1, flags=0)``."""
+    apply = staticmethod(_C.cp4_apply)
 
 
-class RCPConv2dFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, KC, *A):
-        ctx.save_for_backward(x, KC, *A)
-        return conv2d_rcp_fused_nchw(x, *A, KC)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, KC, *A = ctx.saved_tensors
-        dx, dA, dS = rcp_conv2d_backward(x, dy.contiguous().view(x.shape[0], -1, x.shape[-2], x.shape[-1]), *A, KC)
-        return (dx, dS, *dA)
+class CP3Conv2dFunction:
+    """y = three-factor CP conv2d(x; KT, KCin, KC) with the fused backward kernels: ``apply(x, KT, KCin, KC, pad=1)``."""
+    apply = staticmethod(_C.cp3_apply)
 
 
-class CPDenseFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, *Fk):
-        ctx.save_for_backward(x, *Fk)
-        return dense_cp(x, *Fk)
+class RCPConv2dFunction:
+    """y = reshaped-CP conv2d(x; A..., KC): ``apply(x, KC, K0, K1, ...)``."""
+    apply = staticmethod(_C.rcp_apply)
 
-    @staticmethod
-    def backward(ctx, dy):
-        x, *Fk = ctx.saved_tensors
-        dx, dF = dense_cp_backward(x.reshape(x.shape[0], -1), dy.contiguous().reshape(x.shape[0], -1), *Fk)
-        return (dx.view_as(x), *dF)
+
+class CPDenseFunction:
+    """y = CP dense(x; F...): ``apply(x, K0, K1, ...)``."""
+    apply = staticmethod(_C.dense_apply)
