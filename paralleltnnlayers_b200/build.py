@@ -2,7 +2,7 @@
 
     python -m paralleltnnlayers_b200.build [--force] [--verbose]
 
-Each .cu under csrc/ is compiled to an object (rebuilt only when it or a header
+Each .cu under csrc/ is compiled to an object (rebuilt only when it or a header it includes
 is newer) and linked into ``paralleltnnlayers_b200/libb200cp.so``.  The library
 has no dependency on torch; it links the CUDA runtime and NCCL only.  The one
 .cpp file there is the CPython / torch binding, ``paralleltnnlayers_b200/_C.so``,
@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import glob
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -34,16 +35,26 @@ NVCC_FLAGS = [
 NVCC_FLAGS += os.environ.get("B200CP_NVCC_FLAGS", "").split()
 
 
-def _newest_header():
-    hs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + \
-        glob.glob(os.path.join(ROOT, "include", "*.h"))
-    return max(os.path.getmtime(h) for h in hs)
+def _newest_source(path, seen=None):
+    """Modification time of the newest of a source and the project headers it includes, directly or through others."""
+    seen = set() if seen is None else seen
+    seen.add(path)
+    t = os.path.getmtime(path)
+    with open(path) as f:
+        names = re.findall(r'^\s*#\s*include\s+"([^"]+)"', f.read(), re.M)
+    for n in names:
+        for d in (os.path.dirname(path), CSRC, os.path.join(ROOT, "include")):
+            h = os.path.join(d, n)
+            if os.path.exists(h):
+                if h not in seen:
+                    t = max(t, _newest_source(h, seen))
+                break
+    return t
 
 
 def _compile(src, force, verbose):
     obj = os.path.join(OBJ, os.path.basename(src)[:-3] + ".o")
-    if (not force and os.path.exists(obj) and os.path.getmtime(obj) > os.path.getmtime(src)
-            and os.path.getmtime(obj) > _newest_header()):
+    if not force and os.path.exists(obj) and os.path.getmtime(obj) > _newest_source(src):
         return obj, False
     cmd = ["nvcc", "-c", src, "-o", obj] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
     r = subprocess.run(cmd, capture_output=True, text=True)

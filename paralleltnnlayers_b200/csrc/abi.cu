@@ -832,16 +832,34 @@ int b200cp_rcp_fwd(int N, int H, int W, int order, const int* cdims, const int* 
                           static_cast<cudaStream_t>(stream));
 }
 
+size_t b200cp_rcp_fwd_workspace_bytes(int N, int H, int W, int order, const int* cdims, const int* tdims, int R,
+                                      int FH, int FW, int flags) {
+  (void)flags;
+  if (order < 1 || order > 4 || !cdims || !tdims) return 0;
+  return rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, false);
+}
+
+int b200cp_rcp_fwd_ws(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
+                      const float* X, const float* const* A, const float* S, float* V, void* workspace,
+                      size_t workspace_bytes, void* stream, int flags) {
+  (void)flags;
+  if (int rc = check_modes("b200cp_rcp_fwd_ws", order, cdims, tdims, A)) return rc;
+  if (int rc = check_ptrs("b200cp_rcp_fwd_ws", {X, S, V})) return rc;
+  return rcp_product_launch(N, H, W, order, cdims, tdims, R, FH, FW, X, A, S, V, false, workspace, workspace_bytes,
+                            static_cast<cudaStream_t>(stream));
+}
+
 size_t b200cp_rcp_bwd_workspace_bytes(int N, int H, int W, int order, const int* cdims, const int* tdims, int R,
                                       int FH, int FW, int flags) {
-  (void)R; (void)flags;
+  (void)flags;
   if (order < 1 || order > 4 || !cdims || !tdims || FH < 1 || FW < 1) return 0;
   size_t C = 1, T = 1;
   for (int k = 0; k < order; ++k) { C *= (size_t)cdims[k]; T *= (size_t)tdims[k]; }
   // G itself, then the split-K partial tiles of the GEMM that produces it
   const size_t gemm = dense_grad_scratch_floats(N, (int)T, (int)C, H, W, FH, FW);
   const size_t contr = contract_scratch_floats(order, cdims, tdims, R, FH * FW, true);
-  return (T * C * FH * FW + std::max(gemm, contr)) * sizeof(float);
+  return std::max((T * C * FH * FW + std::max(gemm, contr)) * sizeof(float),
+                  rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, true));
 }
 
 int b200cp_rcp_bwd(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -851,7 +869,8 @@ int b200cp_rcp_bwd(int N, int H, int W, int order, const int* cdims, const int* 
   if (int rc = check_ptrs("b200cp_rcp_bwd", {dV, S})) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dX) {
-    if (int rc = rcp_chain_launch(N, H, W, order, cdims, tdims, R, FH, FW, dV, A, S, dX, true, st)) return rc;
+    if (int rc = rcp_product_launch(N, H, W, order, cdims, tdims, R, FH, FW, dV, A, S, dX, true, workspace, workspace_bytes, st))
+      return rc;
   }
   if (dA || dS) {
     if (!dA || !dS || !X) return fail(B200CP_ERR_INVALID_ARG, "b200cp_rcp_bwd: dA, dS and X go together");
@@ -967,14 +986,29 @@ int b200cp_dense_fwd(int B, int order, const int* idims, const int* odims, int R
   return dense_chain_launch(B, order, idims, odims, R, X, F, Y, false, static_cast<cudaStream_t>(stream));
 }
 
+size_t b200cp_dense_fwd_workspace_bytes(int B, int order, const int* idims, const int* odims, int R, int flags) {
+  (void)flags;
+  if (order < 1 || order > 4 || !idims || !odims) return 0;
+  return dense_product_workspace(B, order, idims, odims, R, false);
+}
+
+int b200cp_dense_fwd_ws(int B, int order, const int* idims, const int* odims, int R, const float* X,
+                        const float* const* F, float* Y, void* workspace, size_t workspace_bytes, void* stream, int flags) {
+  (void)flags;
+  if (int rc = check_modes("b200cp_dense_fwd_ws", order, idims, odims, F)) return rc;
+  if (int rc = check_ptrs("b200cp_dense_fwd_ws", {X, Y})) return rc;
+  return dense_product_launch(B, order, idims, odims, R, X, F, Y, false, workspace, workspace_bytes,
+                              static_cast<cudaStream_t>(stream));
+}
+
 size_t b200cp_dense_bwd_workspace_bytes(int B, int order, const int* idims, const int* odims, int R, int flags) {
-  (void)R; (void)flags;
+  (void)flags;
   if (order < 1 || order > 4 || !idims || !odims) return 0;
   size_t I = 1, O = 1;
   for (int k = 0; k < order; ++k) { I *= (size_t)idims[k]; O *= (size_t)odims[k]; }
   const size_t gemm = dense_grad_scratch_floats(B, (int)O, (int)I, 1, 1, 1, 1);
   const size_t contr = contract_scratch_floats(order, idims, odims, R, 1, false);
-  return (I * O + std::max(gemm, contr)) * sizeof(float);
+  return std::max((I * O + std::max(gemm, contr)) * sizeof(float), dense_product_workspace(B, order, idims, odims, R, true));
 }
 
 int b200cp_dense_bwd(int B, int order, const int* idims, const int* odims, int R, const float* X, const float* dY,
@@ -984,7 +1018,7 @@ int b200cp_dense_bwd(int B, int order, const int* idims, const int* odims, int R
   if (int rc = check_ptrs("b200cp_dense_bwd", {dY})) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dX) {
-    if (int rc = dense_chain_launch(B, order, idims, odims, R, dY, F, dX, true, st)) return rc;
+    if (int rc = dense_product_launch(B, order, idims, odims, R, dY, F, dX, true, workspace, workspace_bytes, st)) return rc;
   }
   if (dF) {
     if (!X) return fail(B200CP_ERR_INVALID_ARG, "b200cp_dense_bwd: X is needed for dF");

@@ -311,6 +311,11 @@ int max_items(const ChainGeom& g) {
 
 }  // namespace
 
+int check_kron_modes(int order, const int* idims, const int* odims, int R, const char* who) {
+  ChainGeom g{};
+  return fill_modes(g, order, idims, odims, R, false, who);
+}
+
 int rcp_chain_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                      const float* X, const float* const* A, const float* S, float* V, bool transposed,
                      cudaStream_t st) {

@@ -215,6 +215,25 @@ int dense_fast_launch(int B, int order, const int* din, const int* dout, const i
                       const float* X, const float* const* F, float* Y, cudaStream_t st, bool* done);
 int dense_chain_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
                        const float* const* F, float* Y, bool transposed, cudaStream_t st);
+// The two layers by their multiplied-out weight (kron_small.cu).  Weight: W[slow][ld] or, with S, W[slow][tap][ld];
+// slow = inputs and fast = outputs, or the other way round (taps reversed) with `transposed`.
+int kron_weight_ld(int fast);
+int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
+                       int taps, bool transposed, float* W, cudaStream_t st);
+int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float* Y, cudaStream_t st);
+int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, float* V, cudaStream_t st);
+// Y = X M (dense) and V = K * X (reshaped-CP conv), or their data gradients (`transposed`), by the form that is
+// fastest for the sizes (product.cu); the workspace may be null (or too small): then the factored kernels run.
+size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed);
+int dense_product_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
+                         const float* const* F, float* Y, bool transposed, void* ws, size_t ws_bytes, cudaStream_t st);
+size_t rcp_product_workspace(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
+                             bool transposed);
+int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
+                       const float* X, const float* const* A, const float* S, float* V, bool transposed, void* ws,
+                       size_t ws_bytes, cudaStream_t st);
+// argument checks the factored kernels make (order, mode sizes, rank, filter)
+int check_kron_modes(int order, const int* idims, const int* odims, int R, const char* who);
 // G[tap][t][c] = sum_{n,h,w} dV[n,t,h,w] * Xpad[n,c,h+y,w+x]; scratch holds dense_grad_scratch_floats() floats
 size_t dense_grad_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);
 int dense_grad_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,

@@ -1,0 +1,634 @@
+// Reshaped-CP conv and CP dense layer by their multiplied-out weight, for problems whose weight and product are small.
+//
+// The factored form does R times the mode products one rank after the other; on the chain kernel that is a serial loop
+// of R x (modes + 1) block-wide steps over few CTAs, and it is latency, not arithmetic, that it spends its time on
+// (0.4 TMAC/s: 430 us for a batch of 64 through 16x16x16 -> 4x4x4 at R = 137, 223 us for eight 32x32 images of 16
+// channels at R = 11).  Multiplying the weight out first costs R multiply-adds per weight entry, spread over the whole
+// GPU, and leaves one plain product:
+//   kron_weight_kernel : W[s][f] = sum_r prod_k F_k[s_k, f_k, r]   (conv: W[c][tap][t], with S as one more mode)
+//   small_gemm_kernel  : Y[m][n] = sum_k X[m][k] W[k][n]
+//   small_conv_kernel  : V[n,t,h,w] = sum_{c,y,x} W[c][y,x][t] X[n,c,h+y-1,w+x-1]
+// All exact fp32 (FFMA).  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
+// and past their set-up when the weight is done.  Formulas: Kernels/rcp_fused_nchw.cu:4-77, Kernels/dense_cp.cu:4-46.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "mma_util.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace b200cp {
+namespace {
+
+// ---- the weight ----------------------------------------------------------------------------------------------------------
+// The modes are cut into two halves, A (first modes, slow) and B (last modes): with the half products
+// A[a][r] = prod_{k in A} F_k and B[b][r] the weight is the matrix product A B^T over r.  A CTA forms a TA x 64 tile of
+// it; the half products of a chunk of 32 ranks are formed in shared memory on the way (each factor entry is read by
+// 64 lanes of a CTA at most, from L1).  b runs over the fast sizes of B's modes first, so that a row of the tile is
+// stored in runs of their product.
+constexpr int kKT = 256, kTB = 64, kRC = 32;
+
+struct KronMode {
+  const float* F;
+  int ns, nf;       // slow-side and fast-side sizes
+  int fs, ff;       // entry (s, f) at F[(s*fs + f*ff)*R + r]
+  int os, of;       // output offset per s and per f
+};
+struct KronGeom {
+  int nA, nB;              // modes of the halves
+  KronMode A[3], B[2];     // (tap +) at most two modes in A, two in B
+  int SA, FA, SB, FB;      // products of the sizes
+  int R, rper;             // ranks; ranks per CTA of a cluster
+  int flip;                // A[0] is the tap mode, stored back to front
+};
+
+// ---- sum of a cluster's partial tiles ----------------------------------------------------------------------------------
+// Every CTA of the cluster has left its partial tile in shared memory; CTA q adds slice q of all of them in CTA order
+// (the result does not depend on scheduling) and hands each sum to `put`.
+template <typename Put>
+__device__ __forceinline__ void cluster_sum(float* tile, int n, int splits, int tid, int nthreads, Put put) {
+  if (splits == 1) {
+    __syncthreads();
+    for (int i = tid; i < n; i += nthreads) put(i, tile[i]);
+    return;
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const int q = (int)cl.block_rank(), per = (n + splits - 1) / splits;
+  const int e = min(n, (q + 1) * per);
+  for (int i = q * per + tid; i < e; i += nthreads) {
+    float v = 0.f;
+    for (int p = 0; p < splits; ++p) v += cl.map_shared_rank(tile, p)[i];
+    put(i, v);
+  }
+  cl.sync();   // nobody reads this CTA's tile any more
+}
+
+// entry offset (in ranks) and output offset of half-index (s, f)
+__device__ __forceinline__ void half_decode(const KronMode* m, int n, int s, int f, int flip, int* entry, int* out) {
+  int o = 0;
+  for (int k = n - 1; k >= 0; --k) {
+    const int sk = s % m[k].ns, fk = f % m[k].nf;
+    s /= m[k].ns;
+    f /= m[k].nf;
+    entry[k] = sk * m[k].fs + fk * m[k].ff;
+    o += ((flip && k == 0) ? m[k].ns - 1 - sk : sk) * m[k].os + fk * m[k].of;
+  }
+  *out = o;
+}
+
+template <int TA, bool TAP>
+__global__ void __launch_bounds__(kKT) kron_weight_kernel(const __grid_constant__ KronGeom g, float* __restrict__ W) {
+  constexpr int NA = TA / 16;                  // rows per thread
+  __shared__ __align__(16) float tiles[kRC * (TA + 4 + kTB + 4)];
+  float (*As)[TA + 4] = reinterpret_cast<float (*)[TA + 4]>(tiles);
+  float (*Bs)[kTB + 4] = reinterpret_cast<float (*)[kTB + 4]>(tiles + kRC * (TA + 4));
+  __shared__ int ea[TA][3], eb[kTB][2], oa[TA], ob[kTB];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int a0 = blockIdx.y * TA, b0 = blockIdx.x * kTB, PA = g.SA * g.FA, PB = g.SB * g.FB;
+  const int rb0 = blockIdx.z * g.rper, re = min(g.R, rb0 + g.rper);
+  if (tid < TA) {
+    const int a = a0 + tid;
+    int e[3] = {0, 0, 0}, o = 0;
+    if (a < PA) half_decode(g.A, g.nA, a / g.FA, a % g.FA, g.flip, e, &o);
+    ea[tid][0] = e[0]; ea[tid][1] = e[1]; ea[tid][2] = e[2];
+    oa[tid] = o;
+  } else if (tid >= 128 && tid < 128 + kTB) {
+    const int i = tid - 128, b = b0 + i;
+    int e[2] = {0, 0}, o = 0;
+    if (b < PB) half_decode(g.B, g.nB, b / g.FB, b % g.FB, 0, e, &o);
+    eb[i][0] = e[0]; eb[i][1] = e[1];
+    ob[i] = o;
+  }
+  float acc[NA][4];
+#pragma unroll
+  for (int i = 0; i < NA; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  // A warp fills 8 ranks x 4 rows per turn: full sectors from global memory, all banks of the transposed tile.  The
+  // entries of the next chunk are fetched, all loads of a thread together, while the current one is multiplied; a mode
+  // that a half does not have reads nothing and counts as 1.
+  constexpr int NROW = (TA + kTB + 31) / 32, NE = NROW * (kRC / 8), NM = TAP ? 3 : 2;
+  const int rl = tid & 7, row0 = (tid >> 5) * 4 + ((tid >> 3) & 3);
+  __syncthreads();   // the entry offsets
+  const float* src[NROW][NM];
+  bool in[NROW];
+#pragma unroll
+  for (int i = 0; i < NROW; ++i) {
+    const int row = i * 32 + row0;
+    const bool inA = row < TA;
+    in[i] = inA ? a0 + row < PA : row < TA + kTB && b0 + row - TA < PB;
+#pragma unroll
+    for (int k = 0; k < NM; ++k)
+      src[i][k] = !in[i] || k >= (inA ? g.nA : g.nB) ? nullptr
+                  : inA ? g.A[k].F + (size_t)ea[row][k] * g.R + rl : g.B[k % 2].F + (size_t)eb[row - TA][k % 2] * g.R + rl;
+  }
+  float next[NM][NE];
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int i = 0; i < NROW; ++i)
+#pragma unroll
+      for (int k = 0; k < NM; ++k)
+#pragma unroll
+        for (int rb = 0; rb < kRC / 8; ++rb)
+          next[k][i * (kRC / 8) + rb] = !in[i] || r0 + rb * 8 + rl >= re ? 0.f : src[i][k] ? __ldg(src[i][k] + r0 + rb * 8) : 1.f;
+  };
+  if (rb0 < re) fetch(rb0);
+  for (int r0 = rb0; r0 < re; r0 += kRC) {
+    if (r0 > rb0) __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NROW; ++i) {
+      const int row = i * 32 + row0;
+#pragma unroll
+      for (int rb = 0; rb < kRC / 8; ++rb) {
+        const int e = i * (kRC / 8) + rb;
+        const float v = next[0][e] * next[1][e] * (TAP ? next[NM - 1][e] : 1.f);
+        if (row < TA) As[rb * 8 + rl][row] = v;
+        else if (row < TA + kTB) Bs[rb * 8 + rl][row - TA] = v;
+      }
+    }
+    __syncthreads();
+    if (r0 + kRC < re) fetch(r0 + kRC);
+    const int rn = min(kRC, re - r0);
+#pragma unroll 4
+    for (int r = 0; r < rn; ++r) {
+      const float4 b = *reinterpret_cast<const float4*>(&Bs[r][tx * 4]);
+      float a[NA];
+      if (NA == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(&As[r][ty * 4]);
+        a[0] = t.x; a[1] = t.y; a[2 % NA] = t.z; a[3 % NA] = t.w;
+      } else {
+        a[0] = As[r][ty * NA];
+        if (NA > 1) a[1 % NA] = As[r][ty * NA + 1];
+      }
+#pragma unroll
+      for (int i = 0; i < NA; ++i) {
+        acc[i][0] = fmaf(a[i], b.x, acc[i][0]);
+        acc[i][1] = fmaf(a[i], b.y, acc[i][1]);
+        acc[i][2] = fmaf(a[i], b.z, acc[i][2]);
+        acc[i][3] = fmaf(a[i], b.w, acc[i][3]);
+      }
+    }
+  }
+  // Not earlier: CTAs of the product that start while this grid still fills up are stacked on few SMs (138 CTAs of
+  // small_conv_kernel took 170 us instead of 60).
+  grid_launch_dependents();
+  if (gridDim.z > 1) {   // a small weight: the CTAs of a cluster took a share of the ranks each
+    __syncthreads();
+    float* t = tiles;    // [TA][64] fits: TA * 64 <= 32 * (TA + 72)
+#pragma unroll
+    for (int i = 0; i < NA; ++i)
+      *reinterpret_cast<float4*>(t + (ty * NA + i) * kTB + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    cluster_sum(t, TA * kTB, gridDim.z, tid, kKT, [&](int i, float v) {
+      const int a = i / kTB, b = i % kTB;
+      if (a0 + a < PA && b0 + b < PB) W[oa[a] + ob[b]] = v;
+    });
+    return;
+  }
+  const int b = b0 + tx * 4;
+  const bool run4 = b + 3 < PB && ob[tx * 4 + 3] - ob[tx * 4] == 3 && !(ob[tx * 4] & 3);
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    if (a0 + ty * NA + i >= PA) continue;
+    float* d = W + oa[ty * NA + i];
+    const int o0 = oa[ty * NA + i];
+    if (run4 && !(o0 & 3)) {
+      *reinterpret_cast<float4*>(d + ob[tx * 4]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (b + j < PB) d[ob[tx * 4 + j]] = acc[i][j];
+    }
+  }
+}
+
+// ---- Y[M][N] = X[M][K] W[K][N] -------------------------------------------------------------------------------------------
+// CTA tile BM x BN, 4 x 4 results per thread; KG groups of threads share the K rows of a stage (a small tile has few
+// results, so the threads are spread over K instead).  The CTAs of a cluster split K further.
+constexpr int kGStages = 3;
+template <int BM, int BN>
+struct GemmTile {
+  static constexpr int NT = BM == 64 ? 512 : 256;     // 16 warps hide the FFMA and shared-memory latency that 8 do not
+  static constexpr int KG = NT * 16 / (BM * BN);      // 64x64 -> 2, 32x64 -> 2, 16x64 -> 4, 16x32 -> 8
+  static constexpr int BK = KG > 2 ? 64 : 32;         // K rows of a stage
+  static constexpr int PA = BK + 4;
+  static constexpr int stage = BM * PA + BK * (BN + 4);
+  static constexpr size_t smem = sizeof(float) * (size_t)(kGStages * stage > KG * BM * BN ? kGStages * stage : KG * BM * BN);
+};
+
+template <int BM, int BN, bool VECA>
+__global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const float* __restrict__ X, const float* __restrict__ W,
+                                                         float* __restrict__ Y, int M, int N, int K, int ldw, int kper,
+                                                         int splits) {
+  using T = GemmTile<BM, BN>;
+  constexpr int kBN = BN, kGT = T::NT, TXN = BN / 4;
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x;
+  const int kg = tid / (kGT / T::KG), gt = tid - kg * (kGT / T::KG), tx = gt % TXN, ty = gt / TXN;
+  const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * BM;
+  const int kb = blockIdx.z * kper, ke = min(K, kb + kper);
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  auto load_a = [&](int st, int k0) {
+    const unsigned d = sbase + (unsigned)(st * T::stage) * 4u;
+    if (VECA) {
+      for (int i = tid; i < BM * (T::BK / 4); i += kGT) {
+        const int m = i / (T::BK / 4), k = (i - m * (T::BK / 4)) * 4;
+        const bool in = m0 + m < M && k0 + k < ke;
+        mma::cp_async16_s(d + (unsigned)(m * T::PA + k) * 4u, in ? X + (size_t)(m0 + m) * K + k0 + k : X, in ? 16 : 0);
+      }
+    } else {
+      for (int i = tid; i < BM * T::BK; i += kGT) {
+        const int m = i / T::BK, k = i - m * T::BK;
+        const bool in = m0 + m < M && k0 + k < ke;
+        mma::cp_async4_s(d + (unsigned)(m * T::PA + k) * 4u, in ? X + (size_t)(m0 + m) * K + k0 + k : X, in ? 4 : 0);
+      }
+    }
+  };
+  auto load_b = [&](int st, int k0) {
+    const unsigned d = sbase + (unsigned)(st * T::stage + BM * T::PA) * 4u;
+    for (int i = tid; i < T::BK * (kBN / 4); i += kGT) {
+      const int k = i / (kBN / 4), n = (i - k * (kBN / 4)) * 4;
+      const bool in = k0 + k < ke && n0 + n < N;
+      mma::cp_async16_s(d + (unsigned)(k * (kBN + 4) + n) * 4u, in ? W + (size_t)(k0 + k) * ldw + n0 + n : W, in ? 16 : 0);
+    }
+  };
+  const int steps = ke > kb ? (ke - kb + T::BK - 1) / T::BK : 0;
+  for (int s = 0; s < kGStages - 1; ++s)
+    if (s < steps) load_a(s, kb + s * T::BK);
+  grid_dependency_wait();   // the weight kernel's stores
+  for (int s = 0; s < kGStages - 1; ++s) {
+    if (s < steps) load_b(s, kb + s * T::BK);
+    mma::cp_async_commit();
+  }
+  for (int s = 0; s < steps; ++s) {
+    mma::cp_async_wait<kGStages - 2>();
+    __syncthreads();
+    const int nx = s + kGStages - 1;
+    if (nx < steps) {
+      load_a(nx % kGStages, kb + nx * T::BK);
+      load_b(nx % kGStages, kb + nx * T::BK);
+    }
+    mma::cp_async_commit();
+    const float* As = smem + (s % kGStages) * T::stage + (ty * 4) * T::PA;
+    const float* Bs = smem + (s % kGStages) * T::stage + BM * T::PA + tx * 4;
+#pragma unroll
+    for (int kk = 0; kk < T::BK / T::KG; kk += 4) {
+      const int k = kg * (T::BK / T::KG) + kk;
+      float4 a[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(As + i * T::PA + k);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 b = *reinterpret_cast<const float4*>(Bs + (k + u) * (kBN + 4));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float av = u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w;
+          acc[i][0] = fmaf(av, b.x, acc[i][0]);
+          acc[i][1] = fmaf(av, b.y, acc[i][1]);
+          acc[i][2] = fmaf(av, b.z, acc[i][2]);
+          acc[i][3] = fmaf(av, b.w, acc[i][3]);
+        }
+      }
+    }
+  }
+  mma::cp_async_wait<0>();
+  // the groups' partial results, then the sum over groups, then over the cluster
+  __syncthreads();
+  float* red = smem;   // [KG][BM][64]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4*>(red + (kg * BM + ty * 4 + i) * kBN + tx * 4) =
+        make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  __syncthreads();
+  for (int i = tid; i < BM * kBN; i += kGT) {
+    float v = red[i];
+#pragma unroll
+    for (int q = 1; q < T::KG; ++q) v += red[q * BM * kBN + i];
+    red[i] = v;
+  }
+  cluster_sum(red, BM * kBN, splits, tid, kGT, [&](int i, float v) {
+    const int m = m0 + i / kBN, n = n0 + i % kBN;
+    if (m < M && n < N) Y[(size_t)m * N + n] = v;
+  });
+}
+
+// ---- 3 x 3 convolution with W[c][tap][t] -----------------------------------------------------------------------------------
+// CTA tile: TT output channels x a TR x TC block of pixels of one image; 4 channels x 4 pixels of a row per thread.  Eight
+// input channels per stage; a thread's at most kHaloPer halo positions are the same for every channel, so their offsets
+// are worked out once.  The CTAs of a cluster split the input channels.
+constexpr int kCC = 8, kHaloPer = 2, kCT = 512;   // channels per stage, halo positions per thread, threads
+
+struct SmallConvGeom {
+  int C, T, H, W, ldw, cper, splits;
+  int TR, TC, tilesW, tiles, PXQ;   // tile rows / columns (a multiple of 4), pixel quads in use
+  int P, CS;                        // halo row pitch, halo floats per channel
+};
+
+template <int TT, int CG>
+__global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, const float* __restrict__ X,
+                                                         const float* __restrict__ Wt, float* __restrict__ V) {
+  constexpr int TG = TT / 4;
+  constexpr int WS = kCC * 9 * TT;
+  extern __shared__ __align__(16) float smem[];
+  const int xs = kCC * g.CS, stage = xs + WS;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int grp = tid / (kCT / CG), warp = (tid >> 5) % (kCT / CG / 32);   // CG groups of warps share a stage's channels
+  // lanes: 8 pixel quads x 4 channel quads; warps: the remaining channel quads first
+  const int tq = (lane >> 3) + 4 * (warp % (TG / 4)), pq = (lane & 7) + 8 * (warp / (TG / 4));
+  const int n = blockIdx.x / g.tiles, tile = blockIdx.x - n * g.tiles;
+  const int h0 = (tile / g.tilesW) * g.TR, w0 = (tile % g.tilesW) * g.TC, t0 = blockIdx.y * TT;
+  const int cb = blockIdx.z * g.cper, ce = min(g.C, cb + g.cper);
+  const int HW = g.H * g.W;
+  const float* Xn = X + (size_t)n * g.C * HW;
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
+  // halo position p -> row p / (TC + 2), column p % (TC + 2); column -1 is stored at index 3 so that pixel 0 is aligned
+  int hg[kHaloPer], hs[kHaloPer];
+#pragma unroll
+  for (int j = 0; j < kHaloPer; ++j) {
+    const int p = tid + j * kCT, hr = p / (g.TC + 2), hc = p - hr * (g.TC + 2);
+    const int h = h0 + hr - 1, w = w0 + hc - 1;
+    hs[j] = hr < g.TR + 2 ? hr * g.P + hc + 3 : -1;
+    hg[j] = (hr < g.TR + 2 && h >= 0 && h < g.H && w >= 0 && w < g.W) ? h * g.W + w : -1;
+  }
+  auto load_x = [&](int st, int c0) {
+    const unsigned d = sbase + (unsigned)(st * stage) * 4u;
+#pragma unroll
+    for (int j = 0; j < kHaloPer; ++j)
+      if (hs[j] >= 0) {
+#pragma unroll
+        for (int c = 0; c < kCC; ++c) {
+          const bool in = hg[j] >= 0 && c0 + c < ce;
+          mma::cp_async4_s(d + (unsigned)(c * g.CS + hs[j]) * 4u, in ? Xn + (size_t)(c0 + c) * HW + hg[j] : Xn, in ? 4 : 0);
+        }
+      }
+  };
+  auto load_w = [&](int st, int c0) {
+    const unsigned d = sbase + (unsigned)(st * stage + xs) * 4u;
+    for (int i = tid; i < kCC * 9 * (TT / 4); i += kCT) {
+      const int row = i / (TT / 4), t = (i - row * (TT / 4)) * 4;
+      const bool in = c0 + row / 9 < ce && t0 + t < g.T;
+      mma::cp_async16_s(d + (unsigned)(row * TT + t) * 4u, in ? Wt + ((size_t)c0 * 9 + row) * g.ldw + t0 + t : Wt, in ? 16 : 0);
+    }
+  };
+  float acc[4][4];   // [t][px]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  const bool active = pq < g.PXQ;
+  const int pr = active ? pq / (g.TC / 4) : 0, pc = active ? (pq - pr * (g.TC / 4)) * 4 : 0;
+  const int steps = ce > cb ? (ce - cb + kCC - 1) / kCC : 0;
+  if (steps > 0) load_x(0, cb);
+  grid_dependency_wait();
+  if (steps > 0) load_w(0, cb);
+  mma::cp_async_commit();
+  for (int s = 0; s < steps; ++s) {
+    if (s + 1 < steps) {
+      load_x((s + 1) & 1, cb + (s + 1) * kCC);
+      load_w((s + 1) & 1, cb + (s + 1) * kCC);
+    }
+    mma::cp_async_commit();
+    mma::cp_async_wait<1>();
+    __syncthreads();
+    if (active) {
+      const float* xb = smem + (s & 1) * stage + pr * g.P + pc + 4;
+      const float* wb = smem + (s & 1) * stage + xs + tq * 4;
+#pragma unroll 2
+      for (int cc = 0; cc < kCC / CG; ++cc) {
+        const int c = grp * (kCC / CG) + cc;
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+          const float* xr = xb + c * g.CS + y * g.P;
+          const float4 m = *reinterpret_cast<const float4*>(xr);
+          const float x[6] = {xr[-1], m.x, m.y, m.z, m.w, xr[4]};
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const float4 wv = *reinterpret_cast<const float4*>(wb + (c * 9 + y * 3 + k) * TT);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              acc[0][j] = fmaf(wv.x, x[j + k], acc[0][j]);
+              acc[1][j] = fmaf(wv.y, x[j + k], acc[1][j]);
+              acc[2][j] = fmaf(wv.z, x[j + k], acc[2][j]);
+              acc[3][j] = fmaf(wv.w, x[j + k], acc[3][j]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  float* Vn = V + (size_t)n * g.T * HW;
+  const int npx = g.TR * g.TC;
+  // the channel groups, then the cluster, are added in shared memory over the stage buffers: [group][t][px] (every
+  // thread is past its last read)
+  if (active)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float4*>(smem + (grp * TT + tq * 4 + i) * npx + pr * g.TC + pc) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  __syncthreads();
+  for (int i = tid; i < TT * npx; i += kCT) {
+    float v = smem[i];
+#pragma unroll
+    for (int q = 1; q < CG; ++q) v += smem[q * TT * npx + i];
+    smem[i] = v;
+  }
+  cluster_sum(smem, TT * npx, g.splits, tid, kCT, [&](int i, float v) {
+    const int t = t0 + i / npx, px = i % npx, h = h0 + px / g.TC, w = w0 + px % g.TC;
+    if (t < g.T && h < g.H && w < g.W) Vn[(size_t)t * HW + h * g.W + w] = v;
+  });
+}
+
+// Dynamic shared memory that lets no more CTAs share an SM than the grid needs: CTAs of a programmatic dependent start
+// while the kernel before drains and would otherwise be stacked on the SMs that are free first.
+size_t spread_smem(size_t need, long ctas, const DeviceInfo& di) {
+  const long per = (ctas + di.sm_count - 1) / di.sm_count;
+  return per > 4 ? need : std::max(need, (size_t)di.smem_optin / per - (per > 1 ? 1024 : 0));
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster_z,
+                           bool programmatic, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  static const bool off = [] {
+    const char* e = getenv("B200CP_PDL");
+    return e && e[0] == '0';
+  }();
+  at[0].val.programmaticStreamSerializationAllowed = programmatic && !off ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = (unsigned)cluster_z;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster_z > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// K units per CTA of a cluster: as many CTAs (at most 8 per cluster) as fill the GPU once, at least `least` units each
+int pick_cluster(long tiles, int units, int least, int sm_count) {
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= sm_count && units / (s * 2) >= least) s *= 2;
+  return s;
+}
+
+}  // namespace
+
+// Row pitch of the weight: 16-byte rows.
+int kron_weight_ld(int fast) { return (fast + 3) / 4 * 4; }
+
+// W[s][ld] (dense) or W[s][tap][ld] (S given): slow side = inputs, or outputs with `transposed` (taps then run backwards)
+int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
+                       int taps, bool transposed, float* W, cudaStream_t st) {
+  KronMode m[4];
+  long slow = 1, fast = 1;
+  for (int k = 0; k < order; ++k) {
+    m[k].F = F[k];
+    m[k].ns = transposed ? odims[k] : idims[k];
+    m[k].nf = transposed ? idims[k] : odims[k];
+    m[k].fs = transposed ? 1 : odims[k];
+    m[k].ff = transposed ? odims[k] : 1;
+    slow *= m[k].ns;
+    fast *= m[k].nf;
+  }
+  const int ld = kron_weight_ld((int)fast), row = S ? taps * ld : ld;
+  if (slow * row > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight too large");
+  long os = row, of = 1;
+  for (int k = order - 1; k >= 0; --k) {
+    m[k].os = (int)os;
+    m[k].of = (int)of;
+    os *= m[k].ns;
+    of *= m[k].nf;
+  }
+  KronGeom g{};
+  g.R = R;
+  g.SA = g.FA = g.SB = g.FB = 1;
+  const int ha = order / 2;
+  if (S) {
+    g.A[g.nA++] = KronMode{S, taps, 1, 1, 0, ld, 0};
+    g.SA *= taps;
+    g.flip = transposed ? 1 : 0;
+  }
+  for (int k = 0; k < ha; ++k) { g.A[g.nA++] = m[k]; g.SA *= m[k].ns; g.FA *= m[k].nf; }
+  for (int k = ha; k < order; ++k) { g.B[g.nB++] = m[k]; g.SB *= m[k].ns; g.FB *= m[k].nf; }
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const int PA = g.SA * g.FA, PB = g.SB * g.FB, nb = ceil_div(PB, kTB);
+  // The tallest tile that leaves a CTA for most SMs (tall tiles form fewer half products per entry); a weight too small
+  // even for 16-row tiles is shared out over the ranks as well.
+  int ta = 64;
+  while (ta > 16 && (long)nb * ceil_div(PA, ta) * 5 < 4L * di.sm_count) ta /= 2;
+  const int splits = pick_cluster((long)nb * ceil_div(PA, ta), R, 16, di.sm_count);
+  g.rper = ceil_div(R, splits);
+  const dim3 grid(nb, ceil_div(PA, ta), splits);
+#define KRON(TAV)                                                                                                       \
+  do {                                                                                                                 \
+    if (S) B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, true>, grid, dim3(kKT), 0, st, splits, false, g, W));  \
+    else B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, false>, grid, dim3(kKT), 0, st, splits, false, g, W));   \
+  } while (0)
+  if (ta == 64) KRON(64);
+  else if (ta == 32) KRON(32);
+  else KRON(16);
+#undef KRON
+  B200CP_LAUNCH_OK("kron_weight_kernel");
+  return B200CP_OK;
+}
+
+int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float* Y, cudaStream_t st) {
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const int ldw = kron_weight_ld(N);
+  const bool vec = !(K & 3) && !(reinterpret_cast<uintptr_t>(X) & 15);
+  // the tallest tile that leaves enough CTAs for one wave once a cluster splits K eight ways
+  const auto enough = [&](int bm) { return M > bm / 2 && (long)ceil_div(M, bm) * ceil_div(N, 64) * 8 >= di.sm_count; };
+  const int bm = enough(64) ? 64 : enough(32) ? 32 : 16;
+  const int bn = bm == 16 && (long)ceil_div(M, 16) * ceil_div(N, 64) * 8 < di.sm_count ? 32 : 64;
+  const long tiles = (long)ceil_div(M, bm) * ceil_div(N, bn);
+  const int splits = pick_cluster(tiles, K, 64, di.sm_count);
+  const int kper = (int)align_up((size_t)ceil_div(K, splits), 4);
+  dim3 grid(ceil_div(N, bn), ceil_div(M, bm), splits);
+  if (grid.y > 65535) return fail(B200CP_ERR_UNSUPPORTED, "dense: batch too large for the small product kernel");
+#define SMALL_GEMM(BMV, BNV, V)                                                                                       \
+  do {                                                                                                                \
+    static std::atomic<int> set[64];                                                                                  \
+    const size_t smem = spread_smem(GemmTile<BMV, BNV>::smem, tiles * splits, di);                                    \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(small_gemm_kernel<BMV, BNV, V>), set, di.smem_optin)); \
+    B200CP_CUDA_OK(launch_cluster(small_gemm_kernel<BMV, BNV, V>, grid, dim3(GemmTile<BMV, BNV>::NT), smem, st, splits, true, \
+                                  X, W, Y, M, N, K, ldw, kper, splits));                                              \
+  } while (0)
+  if (bn == 32) { if (vec) SMALL_GEMM(16, 32, true); else SMALL_GEMM(16, 32, false); }
+  else if (bm == 16) { if (vec) SMALL_GEMM(16, 64, true); else SMALL_GEMM(16, 64, false); }
+  else if (bm == 32) { if (vec) SMALL_GEMM(32, 64, true); else SMALL_GEMM(32, 64, false); }
+  else { if (vec) SMALL_GEMM(64, 64, true); else SMALL_GEMM(64, 64, false); }
+#undef SMALL_GEMM
+  B200CP_LAUNCH_OK("small_gemm_kernel");
+  return B200CP_OK;
+}
+
+int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, float* V, cudaStream_t st) {
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const int tt = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  // two channel groups share the 16 warps; eight (four with 64 output channels: a warp holds 16 of them), with a quarter
+  // or half of the pixels per CTA, where there are few pixels
+  const bool few = (long)N * ceil_div(H * W, kCT * 2 / (tt / 4)) * ceil_div(T, tt) * 2 <= di.sm_count;
+  const int cgroups = few ? (tt == 64 ? 4 : 8) : 2;
+  const int quads = kCT / cgroups / (tt / 4);      // pixel quads per CTA
+  SmallConvGeom g{};
+  g.C = C; g.T = T; g.H = H; g.W = W; g.ldw = kron_weight_ld(T);
+  // columns of the tile: the width that covers the image with the least waste and halo
+  int best = 4;
+  double best_cost = 1e300;
+  for (int tc = 4; tc <= std::min(32, (W + 3) / 4 * 4); tc += 4) {
+    const int tr = std::min(quads / (tc / 4), H);
+    if (tr < 1 || (tr + 2) * (tc + 2) > kHaloPer * kCT) continue;
+    const double cost = (double)ceil_div(W, tc) * ceil_div(H, tr) * (1.0 + 0.1 * (tr + 2.0) * (tc + 2.0) / (tr * tc));
+    if (cost < best_cost) { best_cost = cost; best = tc; }
+  }
+  g.TC = best;
+  g.TR = std::min(quads / (g.TC / 4), H);
+  g.tilesW = ceil_div(W, g.TC);
+  g.tiles = g.tilesW * ceil_div(H, g.TR);
+  g.PXQ = g.TR * (g.TC / 4);
+  g.P = g.TC + 8;
+  g.CS = (int)align_up((size_t)(g.TR + 2) * g.P, 4);
+  const long tiles = (long)N * g.tiles * ceil_div(T, tt);
+  g.splits = pick_cluster(tiles, C, 2 * kCC, di.sm_count);
+  g.cper = (int)align_up((size_t)ceil_div(C, g.splits), kCC);
+  const size_t smem = sizeof(float) * std::max<size_t>(2 * ((size_t)kCC * g.CS + kCC * 9 * tt), (size_t)cgroups * tt * g.TR * g.TC);
+  dim3 grid((unsigned)(N * g.tiles), ceil_div(T, tt), g.splits);
+  if ((long)N * g.tiles > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");
+#define SMALL_CONV(TTV, CGV)                                                                                              \
+  do {                                                                                                                \
+    static std::atomic<int> set[64];                                                                                  \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(small_conv_kernel<TTV, CGV>), set, di.smem_optin));   \
+    B200CP_CUDA_OK(launch_cluster(small_conv_kernel<TTV, CGV>, grid, dim3(kCT), spread_smem(smem, tiles * g.splits, di), st, \
+                                  g.splits, true, g, X, Wt, V));                                                      \
+  } while (0)
+  if (cgroups == 2) {
+    if (tt == 16) SMALL_CONV(16, 2);
+    else if (tt == 32) SMALL_CONV(32, 2);
+    else SMALL_CONV(64, 2);
+  } else {
+    if (tt == 16) SMALL_CONV(16, 8);
+    else if (tt == 32) SMALL_CONV(32, 8);
+    else SMALL_CONV(64, 4);
+  }
+#undef SMALL_CONV
+  B200CP_LAUNCH_OK("small_conv_kernel");
+  return B200CP_OK;
+}
+
+}  // namespace b200cp

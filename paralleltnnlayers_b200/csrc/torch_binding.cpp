@@ -249,8 +249,11 @@ Tensor rcp_forward(const Tensor& U_, at::TensorList A, const Tensor& KC_, int fl
   TORCH_CHECK_VALUE(U.numel() == N * m.na * H * W, "input channel count does not match the kernels");
   const c10::cuda::OptionalCUDAGuard guard(U.device());
   Tensor V = empty({N, m.nb, H, W}, U);
-  ok(b200cp_rcp_fwd((int)N, (int)H, (int)W, m.order, m.a.data(), m.b.data(), m.R, (int)KC.size(0), (int)KC.size(1), cp(U),
-                    m.ptr.data(), cp(KC), mp(V), stream(U), flags));
+  const int FH = (int)KC.size(0), FW = (int)KC.size(1);
+  Tensor ws = workspace(b200cp_rcp_fwd_workspace_bytes((int)N, (int)H, (int)W, m.order, m.a.data(), m.b.data(), m.R, FH, FW,
+                                                       flags), U);
+  ok(b200cp_rcp_fwd_ws((int)N, (int)H, (int)W, m.order, m.a.data(), m.b.data(), m.R, FH, FW, cp(U), m.ptr.data(), cp(KC),
+                       mp(V), mp(ws), ws_bytes(ws), stream(U), flags));
   if (folded) return V;
   std::vector<int64_t> shape{N};
   for (int t : m.b) shape.push_back(t);
@@ -297,7 +300,9 @@ Tensor dense_forward(const Tensor& U_, at::TensorList F, int flags) {
   TORCH_CHECK_VALUE(U.numel() == B * m.na, "input size does not match the kernels");
   const c10::cuda::OptionalCUDAGuard guard(U.device());
   Tensor Y = empty({B, m.nb}, U);
-  ok(b200cp_dense_fwd((int)B, m.order, m.a.data(), m.b.data(), m.R, cp(U), m.ptr.data(), mp(Y), stream(U), flags));
+  Tensor ws = workspace(b200cp_dense_fwd_workspace_bytes((int)B, m.order, m.a.data(), m.b.data(), m.R, flags), U);
+  ok(b200cp_dense_fwd_ws((int)B, m.order, m.a.data(), m.b.data(), m.R, cp(U), m.ptr.data(), mp(Y), mp(ws), ws_bytes(ws),
+                         stream(U), flags));
   if (U.dim() == 2) return Y;
   std::vector<int64_t> shape{B};
   for (int o : m.b) shape.push_back(o);

@@ -1,0 +1,46 @@
+"""The multiplied-out forms of the dense and reshaped-CP layers on CUDA cores, at the edges of their tiles."""
+import numpy as np
+import pytest
+
+from oracle import cp_oracle as O
+from tests.gpu_util import check, dev
+
+pytestmark = pytest.mark.gpu
+
+DENSE = [  # B, idims, odims, R: product tiles of 16 / 32 / 64 x 64, K split over 1-8 CTAs, weight tiles of 16 / 32 / 64 x 64
+    (1, (5,), (3,), 1), (16, (16, 16), (4, 4), 31), (17, (5, 5, 5), (3, 5, 7), 33), (64, (16, 16, 16), (4, 4, 4), 137),
+    (65, (3, 2, 5, 4), (2, 7, 3, 2), 5), (300, (8, 8), (13, 11), 32), (33, (4, 4), (16, 16, 16)[:2], 65),
+    (700, (4, 6, 4), (4, 6, 4), 40), (130, (9, 7), (16, 16), 8), (2, (16, 16, 16), (16, 16, 8), 3),
+]
+
+
+@pytest.mark.parametrize("case", DENSE, ids=str)
+def test_dense_forward_and_data_gradient(case):
+    import paralleltnnlayers_b200 as P
+    B, idims, odims, R = case
+    X, F, dY = O.make_dense_inputs(11, B, idims, odims, R)
+    x, dy = dev(X, dY)
+    f = dev(*F)
+    ref = O.dense_cp_forward(X, F)
+    check(P.dense_cp(x, *f), ref, "dense forward", atol=1e-5 * max(1.0, float(np.abs(ref).max())))
+    rX = O.dense_cp_backward(X, dY, F)[0]
+    check(P.dense_cp_backward(x, dy, *f, need_dw=False)[0], rX, "dense dX", atol=1e-5 * max(1.0, float(np.abs(rX).max())))
+
+
+RCP = [  # N, cdims, tdims, H, W, R: channel tiles of 16 / 32 / 64, pixel tiles of 256 / 128 / 64, channels split over a cluster
+    (1, (3,), (5,), 1, 1, 2), (2, (4, 4), (4, 4), 32, 32, 11), (1, (2, 9), (3, 11), 7, 33, 5), (3, (5, 5), (6, 6), 9, 5, 33),
+    (1, (16, 16), (5, 13), 7, 7, 4), (1, (16, 16), (16, 16), 8, 30, 16), (2, (2, 3, 4), (3, 3, 8), 13, 40, 7),
+]
+
+
+@pytest.mark.parametrize("case", RCP, ids=str)
+def test_rcp_forward_and_data_gradient(case):
+    import paralleltnnlayers_b200 as P
+    N, cd, td, H, W, R = case
+    X, A, S, dV = O.make_rcp_inputs(12, N, cd, td, H, W, 3, 3, R)
+    x, s, dv = dev(X, S, dV)
+    a = dev(*A)
+    ref = O.rcp_forward(X, A, S)
+    check(P.conv2d_rcp_fused_nchw(x, *a, s), ref, "rcp forward", atol=1e-5 * max(1.0, float(np.abs(ref).max())))
+    rX = O.rcp_backward(X, dV, A, S)[0]
+    check(P.rcp_conv2d_backward(x, dv, *a, s, need_dw=False)[0], rX, "rcp dX", atol=1e-5 * max(1.0, float(np.abs(rX).max())))
