@@ -67,6 +67,24 @@ int b200cp_cp4_fwd(const b200cp_tensor_shape* s, const float* X, const float* K0
 int b200cp_cp4_bwd_data(const b200cp_tensor_shape* s, const float* dU, const float* K0, const float* K1,
                         const float* KH, const float* KW, float* dX, void* stream, int flags);
 
+/* The two convolutions with a workspace (16-byte aligned, of the size the _workspace_bytes call gives, which may be 0):
+ * shapes for which that is not 0 run as products over whole rank planes, up to several times faster than without.  With P
+ * (or Q) not NULL (saves_plane = 1) the rank plane is written there as by the _save calls below.  Workspace too small
+ * or NULL: as the calls without one. */
+size_t b200cp_cp4_fwd_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags);
+int b200cp_cp4_fwd_ws(const b200cp_tensor_shape* s, const float* X, const float* K0, const float* K1, const float* KH,
+                      const float* KW, float* U, float* P, void* workspace, size_t workspace_bytes, void* stream, int flags);
+size_t b200cp_cp4_bwd_data_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags);
+int b200cp_cp4_bwd_data_ws(const b200cp_tensor_shape* s, const float* dU, const float* K0, const float* K1,
+                           const float* KH, const float* KW, float* dX, float* Q, void* workspace, size_t workspace_bytes,
+                           void* stream, int flags);
+
+/* The whole backward of a layer whose forward kept its rank plane P: dX and the packed factor gradients. */
+size_t b200cp_cp4_bwd_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags);
+int b200cp_cp4_bwd_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P, const float* K0,
+                         const float* K1, const float* KH, const float* KW, float* dX, float* dK_packed, void* workspace,
+                         size_t workspace_bytes, void* stream, int flags);
+
 /* Bytes of device scratch b200cp_cp4_bwd_filter needs for this shape (0 on error). */
 size_t b200cp_cp4_bwd_filter_workspace_bytes(const b200cp_tensor_shape* s, int flags);
 
@@ -167,6 +185,19 @@ size_t b200cp_cp3_bwd_filter_workspace_bytes(const b200cp_tensor_shape* s, int f
 int b200cp_cp3_bwd_filter(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* KT,
                           const float* KCin, const float* KC, float* dK_packed, void* workspace,
                           size_t workspace_bytes, void* stream, int flags);
+/* With a workspace, as for CP4.  The rank plane P can be kept by the forward, and the backward run from it, for the
+ * shapes for which b200cp_cp3_shares_planes says so. */
+int b200cp_cp3_shares_planes(const b200cp_tensor_shape* s, int flags);
+size_t b200cp_cp3_fwd_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags);
+int b200cp_cp3_fwd_ws(const b200cp_tensor_shape* s, const float* X, const float* KT, const float* KCin, const float* KC,
+                      float* U, float* P, void* workspace, size_t workspace_bytes, void* stream, int flags);
+size_t b200cp_cp3_bwd_data_workspace_bytes(const b200cp_tensor_shape* s, int flags);
+int b200cp_cp3_bwd_data_ws(const b200cp_tensor_shape* s, const float* dU, const float* KT, const float* KCin,
+                           const float* KC, float* dX, void* workspace, size_t workspace_bytes, void* stream, int flags);
+size_t b200cp_cp3_bwd_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags);
+int b200cp_cp3_bwd_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P, const float* KT,
+                         const float* KCin, const float* KC, float* dX, float* dK_packed, void* workspace,
+                         size_t workspace_bytes, void* stream, int flags);
 
 /* Host-memory variants: copy in, run, copy out, synchronise.  They allocate
  * (and cache per device) their own device buffers.  `dK_packed` may be NULL in

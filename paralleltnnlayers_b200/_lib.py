@@ -57,6 +57,19 @@ def _load():
         "b200cp_cp4_bwd_data_save": (i, [sp, fp, fp, fp, fp, fp, fp, fp, vp, i]),
         "b200cp_cp4_bwd_filter_saved_workspace_bytes": (sz, [sp, i]),
         "b200cp_cp4_bwd_filter_saved": (i, [sp, fp, fp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
+        "b200cp_cp4_fwd_workspace_bytes": (sz, [sp, i, i]),
+        "b200cp_cp4_fwd_ws": (i, [sp, fp, fp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
+        "b200cp_cp4_bwd_data_workspace_bytes": (sz, [sp, i, i]),
+        "b200cp_cp4_bwd_data_ws": (i, [sp, fp, fp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
+        "b200cp_cp4_bwd_saved_workspace_bytes": (sz, [sp, i]),
+        "b200cp_cp4_bwd_saved": (i, [sp, fp, fp, fp, fp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
+        "b200cp_cp3_shares_planes": (i, [sp, i]),
+        "b200cp_cp3_fwd_workspace_bytes": (sz, [sp, i, i]),
+        "b200cp_cp3_fwd_ws": (i, [sp, fp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
+        "b200cp_cp3_bwd_data_workspace_bytes": (sz, [sp, i]),
+        "b200cp_cp3_bwd_data_ws": (i, [sp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
+        "b200cp_cp3_bwd_saved_workspace_bytes": (sz, [sp, i]),
+        "b200cp_cp3_bwd_saved": (i, [sp, fp, fp, fp, fp, fp, fp, fp, fp, vp, sz, vp, i]),
         "b200cp_cp3_fwd": (i, [sp, fp, fp, fp, fp, fp, vp, i]),
         "b200cp_cp3_bwd_data": (i, [sp, fp, fp, fp, fp, fp, vp, i]),
         "b200cp_cp3_bwd_filter_workspace_bytes": (sz, [sp, i]),

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "cp_planes.cuh"
 #include "b200cp_test.h"
 
 namespace b200cp {
@@ -93,6 +94,41 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
   a.Rs = s->Rank;
   a.R = s->Rank;
   return a;
+}
+
+// Which 3x3 / pad 1 convolutions and backward passes run as products over whole rank planes (cp_planes.cu); B200CP_PLANES=0
+// switches them off.  The tile and row kernels they compete with keep a plane in shared memory, so they win while one
+// chunk of ranks and enough tiles of one image keep every SM busy; the products have a fixed cost of three to five
+// dependent launches (about 14 us for a convolution at R > 32) and take any split of channels and pixels.  Measured, tile
+// or row kernels / products, us, shapes N x C x T x H x W:
+//   convolution, R = 128: 32x64x64x56x56 254 / 136, 8x256x256x14x14 131 / 23, 64x32x32x63x61 328 / 280
+//   R = 64: 8x256x256x14x14 59 / 23, 64x512x512x7x7 52 / 31, 32x64x64x56x56 90 / 76, 8x48x256x55x55 62 / 53,
+//     32x128x128x28x28 41 / 41, but 16x64x128x28x28 23 / 27, 16x256x384x27x27 52 / 54, 64x32x32x63x61 133 / 149
+//   R = 32: 8x256x256x14x14 27 / 15, 64x512x512x7x7 29 / 25, 1x512x512x7x7 17 / 17, but 16x256x384x27x27 33 / 37,
+//     32x64x64x56x56 41 / 48
+//   training step, R = 50: every shape measured, 1.15 to 3 times faster; R = 32: 64x256x256x14x14 101 / 75,
+//     64x512x512x7x7 91 / 59, 16x256x384x27x27 111 / 110, but 32x64x64x56x56 142 / 152, 2x33x70x45x31 31 / 41
+//   R = 8: 64x512x512x7x7 53 / 46, 8x256x256x14x14 28 / 25, but 64x256x256x14x14 52 / 54, 16x256x384x27x27 66 / 84
+//   backward of the three-factor convolution, whose other kernels contract the channels twice: R = 32 32x64x64x56x56
+//     233 / 179 with the forward, but 64x32x32x63x61 334 / 399; R = 16: 64x512x512x7x7 121 / 94, 32x64x64x56x56 109 / 124
+const bool g_planes = [] {
+  const char* e = getenv("B200CP_PLANES");
+  return !(e && e[0] == '0');
+}();
+enum class Planes { kConv, kBackward, kBackward3 };   // one convolution; a step or the factor gradients; those of CP3
+bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
+  if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !g_planes || !planes_supported(*s)) return false;
+  const size_t px = (size_t)s->N * s->H * s->W, ch = (size_t)s->C + s->T;
+  const unsigned R = s->Rank;
+  const bool few = px <= 4096 && ch >= 512;   // small images, many channels: few tiles, each a long chain
+  switch (use) {
+    case Planes::kConv:
+      return R > 64 || (R > 32 && ((px <= 4096 && ch >= 256) || (px >= 16384 && ch >= 128))) || (R > 16 && few);
+    case Planes::kBackward:
+      return R > 32 || (R > 16 && px <= 16384 && ch >= 384) || (few && (s->W & 3));   // (the row kernels take W % 4 == 0)
+    default:
+      return R > 32 || (R > 16 && ch >= 128) || ch >= 512;
+  }
 }
 
 bool takes_mma(int path, const float* KC, const float* save) {
@@ -186,6 +222,81 @@ int b200cp_cp4_bwd_data(const b200cp_tensor_shape* s, const float* dU, const flo
   return run_conv(s, dU, K0, K1, KH, KW, dX, static_cast<cudaStream_t>(stream), flags, true);
 }
 
+// ---- the convolutions with a workspace, and the whole backward from the forward's rank plane ----------------------
+static size_t conv_ws_bytes(const b200cp_tensor_shape* s, int part, int saves_plane, int flags) {
+  if (!takes_planes(s, flags, Planes::kConv)) return 0;
+  return planes_workspace(*s, part | (saves_plane ? kPlanesNoP | kPlanesNoQ : 0));
+}
+static bool has_ws(const void* ws, size_t have, size_t need) {
+  return need && ws && have >= need && !(reinterpret_cast<uintptr_t>(ws) & 15);
+}
+
+size_t b200cp_cp4_fwd_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags) {
+  if (check_shape(s, "b200cp_cp4_fwd_workspace_bytes")) return 0;
+  return conv_ws_bytes(s, kPlanesFwd, saves_plane, flags);
+}
+
+int b200cp_cp4_fwd_ws(const b200cp_tensor_shape* s, const float* X, const float* K0, const float* K1, const float* KH,
+                      const float* KW, float* U, float* P, void* workspace, size_t workspace_bytes, void* stream, int flags) {
+  if (int rc = check_shape(s, "b200cp_cp4_fwd_ws")) return rc;
+  if (int rc = check_ptrs("b200cp_cp4_fwd_ws", {X, K0, K1, KH, KW, U})) return rc;
+  if (!has_ws(workspace, workspace_bytes, conv_ws_bytes(s, kPlanesFwd, P != nullptr, flags)))
+    return P ? b200cp_cp4_fwd_save(s, X, K0, K1, KH, KW, U, P, stream, flags)
+             : b200cp_cp4_fwd(s, X, K0, K1, KH, KW, U, stream, flags);
+  if (P)
+    if (int rc = check_ptrs("b200cp_cp4_fwd_ws", {P})) return rc;
+  PlanesJob j;
+  j.s = s; j.X = X; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.U = U; j.Psave = P;
+  return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+size_t b200cp_cp4_bwd_data_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags) {
+  if (check_shape(s, "b200cp_cp4_bwd_data_workspace_bytes")) return 0;
+  return conv_ws_bytes(s, kPlanesBwd, saves_plane, flags);
+}
+
+int b200cp_cp4_bwd_data_ws(const b200cp_tensor_shape* s, const float* dU, const float* K0, const float* K1,
+                           const float* KH, const float* KW, float* dX, float* Q, void* workspace, size_t workspace_bytes,
+                           void* stream, int flags) {
+  if (int rc = check_shape(s, "b200cp_cp4_bwd_data_ws")) return rc;
+  if (int rc = check_ptrs("b200cp_cp4_bwd_data_ws", {dU, K0, K1, KH, KW, dX})) return rc;
+  if (!has_ws(workspace, workspace_bytes, conv_ws_bytes(s, kPlanesBwd, Q != nullptr, flags)))
+    return Q ? b200cp_cp4_bwd_data_save(s, dU, K0, K1, KH, KW, dX, Q, stream, flags)
+             : b200cp_cp4_bwd_data(s, dU, K0, K1, KH, KW, dX, stream, flags);
+  if (Q)
+    if (int rc = check_ptrs("b200cp_cp4_bwd_data_ws", {Q})) return rc;
+  PlanesJob j;
+  j.s = s; j.dU = dU; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.dX = dX; j.Qsave = Q;
+  return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+size_t b200cp_cp4_bwd_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
+  if (check_shape(s, "b200cp_cp4_bwd_saved_workspace_bytes")) return 0;
+  if (takes_planes(s, flags, Planes::kBackward)) return planes_workspace(*s, kPlanesBwd | kPlanesGrads | kPlanesNoP);
+  return align_up((size_t)s->N * s->Rank * s->H * s->W * sizeof(float), 256) + b200cp_cp4_bwd_filter_saved_workspace_bytes(s, flags);
+}
+
+int b200cp_cp4_bwd_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P, const float* K0,
+                         const float* K1, const float* KH, const float* KW, float* dX, float* dK_packed, void* workspace,
+                         size_t workspace_bytes, void* stream, int flags) {
+  if (int rc = check_shape(s, "b200cp_cp4_bwd_saved")) return rc;
+  if (int rc = check_ptrs("b200cp_cp4_bwd_saved", {X, dU, P, K0, K1, KH, KW, dX, dK_packed})) return rc;
+  const size_t need = b200cp_cp4_bwd_saved_workspace_bytes(s, flags);
+  if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15))
+    return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_saved: a 16-byte aligned workspace of %zu bytes needed, %zu given", need,
+                workspace_bytes);
+  if (takes_planes(s, flags, Planes::kBackward)) {
+    PlanesJob j;
+    j.s = s; j.X = X; j.dU = dU; j.P = P; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.dX = dX; j.dK = dK_packed;
+    return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+  }
+  const size_t plane = align_up((size_t)s->N * s->Rank * s->H * s->W * sizeof(float), 256);
+  float* Q = static_cast<float*>(workspace);
+  if (int rc = b200cp_cp4_bwd_data_save(s, dU, K0, K1, KH, KW, dX, Q, stream, flags)) return rc;
+  return b200cp_cp4_bwd_filter_saved(s, X, dU, P, Q, KH, KW, dK_packed, static_cast<char*>(workspace) + plane,
+                                     workspace_bytes - plane, stream, flags);
+}
+
 // 3x3 / pad 1 / at most 16 ranks: the stand-alone backward-filter can write the two rank planes with plane-only
 // convolutions and form the gradients from them with the step's band kernel; that needs room for the planes
 static size_t bwd_filter_plane_bytes(const b200cp_tensor_shape* s) {
@@ -201,6 +312,7 @@ size_t b200cp_cp4_bwd_filter_workspace_bytes(const b200cp_tensor_shape* s, int f
   if (check_shape(s, "b200cp_cp4_bwd_filter_workspace_bytes")) return 0;
   if (path_of(flags) == B200CP_PATH_SIMT) return cp4_bwd_filter_simt_workspace(*s);
   size_t need = std::max(cp4_bwd_filter_simt_workspace(*s), cp4_bwd_filter_mma_workspace(*s));
+  if (takes_planes(s, flags, Planes::kBackward)) need = std::max(need, planes_workspace(*s, kPlanesGrads));
   if (bwd_filter_by_planes(s, flags)) need = std::max(need, 2 * bwd_filter_plane_bytes(s) + cp4_grad_band_workspace(*s));
   return need;
 }
@@ -217,6 +329,11 @@ int b200cp_cp4_bwd_filter(const b200cp_tensor_shape* s, const float* X, const fl
   if (path == B200CP_PATH_TC3X || path == B200CP_PATH_TC1X)
     return fail(B200CP_ERR_UNSUPPORTED, "cp4 bwd-filter: the tcgen05 path is not available for this operation");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_filter: workspace is null");
+  if (takes_planes(s, flags, Planes::kBackward) && has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads))) {
+    PlanesJob j;
+    j.s = s; j.X = X; j.dU = dU; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.dK = dK_packed;
+    return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+  }
   Cp4BwdFilterArgs a{};
   a.N = s->N; a.C = s->C; a.T = s->T; a.H = s->H; a.W = s->W; a.F = s->Y; a.pad = s->pad;
   a.Rs = s->Rank;
@@ -276,10 +393,68 @@ int b200cp_cp3_bwd_data(const b200cp_tensor_shape* s, const float* dU, const flo
   return run_conv(s, dU, KT, KCin, nullptr, nullptr, dX, static_cast<cudaStream_t>(stream), flags, true, KC);
 }
 
+int b200cp_cp3_shares_planes(const b200cp_tensor_shape* s, int flags) {
+  if (check_shape(s, "b200cp_cp3_shares_planes")) return 0;
+  return takes_planes(s, flags, Planes::kBackward3) ? 1 : 0;
+}
+
+size_t b200cp_cp3_fwd_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags) {
+  if (check_shape(s, "b200cp_cp3_fwd_workspace_bytes")) return 0;
+  return conv_ws_bytes(s, kPlanesFwd, saves_plane, flags);
+}
+
+int b200cp_cp3_fwd_ws(const b200cp_tensor_shape* s, const float* X, const float* KT, const float* KCin, const float* KC,
+                      float* U, float* P, void* workspace, size_t workspace_bytes, void* stream, int flags) {
+  if (int rc = check_shape(s, "b200cp_cp3_fwd_ws")) return rc;
+  if (int rc = check_ptrs("b200cp_cp3_fwd_ws", {X, KT, KCin, KC, U})) return rc;
+  if (P) {
+    if (int rc = check_ptrs("b200cp_cp3_fwd_ws", {P})) return rc;
+    if (!b200cp_cp3_shares_planes(s, flags))
+      return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp3_fwd_ws: the rank plane is for shapes of b200cp_cp3_shares_planes only");
+  }
+  if (!has_ws(workspace, workspace_bytes, conv_ws_bytes(s, kPlanesFwd, P != nullptr, flags)))
+    return run_conv(s, X, KT, KCin, nullptr, nullptr, U, static_cast<cudaStream_t>(stream), flags, false, KC, P);
+  PlanesJob j;
+  j.s = s; j.X = X; j.K0 = KT; j.K1 = KCin; j.KC = KC; j.U = U; j.Psave = P;
+  return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+size_t b200cp_cp3_bwd_data_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
+  if (check_shape(s, "b200cp_cp3_bwd_data_workspace_bytes")) return 0;
+  return conv_ws_bytes(s, kPlanesBwd, 0, flags);
+}
+
+int b200cp_cp3_bwd_data_ws(const b200cp_tensor_shape* s, const float* dU, const float* KT, const float* KCin,
+                           const float* KC, float* dX, void* workspace, size_t workspace_bytes, void* stream, int flags) {
+  if (int rc = check_shape(s, "b200cp_cp3_bwd_data_ws")) return rc;
+  if (int rc = check_ptrs("b200cp_cp3_bwd_data_ws", {dU, KT, KCin, KC, dX})) return rc;
+  if (!has_ws(workspace, workspace_bytes, conv_ws_bytes(s, kPlanesBwd, 0, flags)))
+    return b200cp_cp3_bwd_data(s, dU, KT, KCin, KC, dX, stream, flags);
+  PlanesJob j;
+  j.s = s; j.dU = dU; j.K0 = KT; j.K1 = KCin; j.KC = KC; j.dX = dX;
+  return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+size_t b200cp_cp3_bwd_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
+  if (check_shape(s, "b200cp_cp3_bwd_saved_workspace_bytes") || !takes_planes(s, flags, Planes::kBackward3)) return 0;
+  return planes_workspace(*s, kPlanesBwd | kPlanesGrads | kPlanesNoP);
+}
+
+int b200cp_cp3_bwd_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P, const float* KT,
+                         const float* KCin, const float* KC, float* dX, float* dK_packed, void* workspace,
+                         size_t workspace_bytes, void* stream, int flags) {
+  if (int rc = check_shape(s, "b200cp_cp3_bwd_saved")) return rc;
+  if (int rc = check_ptrs("b200cp_cp3_bwd_saved", {X, dU, P, KT, KCin, KC, dX, dK_packed})) return rc;
+  if (!takes_planes(s, flags, Planes::kBackward3))
+    return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp3_bwd_saved: for shapes of b200cp_cp3_shares_planes only");
+  PlanesJob j;
+  j.s = s; j.X = X; j.dU = dU; j.P = P; j.K0 = KT; j.K1 = KCin; j.KC = KC; j.dX = dX; j.dK = dK_packed;
+  return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
 size_t b200cp_cp3_bwd_filter_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
-  (void)flags;
   if (check_shape(s, "b200cp_cp3_bwd_filter_workspace_bytes")) return 0;
-  return cp4_bwd_filter_mma_workspace(*s);
+  return std::max(cp4_bwd_filter_mma_workspace(*s), takes_planes(s, flags, Planes::kBackward3) ? planes_workspace(*s, kPlanesGrads) : 0);
 }
 
 int b200cp_cp3_bwd_filter(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* KT,
@@ -294,6 +469,11 @@ int b200cp_cp3_bwd_filter(const b200cp_tensor_shape* s, const float* X, const fl
   if (path != B200CP_PATH_AUTO && path != B200CP_PATH_MMA)
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp3_bwd_filter: runs on the mma path only (flags AUTO or MMA)");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp3_bwd_filter: workspace is null");
+  if (takes_planes(s, flags, Planes::kBackward3) && has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads))) {
+    PlanesJob j;
+    j.s = s; j.X = X; j.dU = dU; j.K0 = KT; j.K1 = KCin; j.KC = KC; j.dK = dK_packed;
+    return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+  }
   Cp4BwdFilterArgs a{};
   a.N = s->N; a.C = s->C; a.T = s->T; a.H = s->H; a.W = s->W; a.F = 3; a.pad = 1;
   a.Rs = s->Rank;
@@ -408,8 +588,9 @@ size_t b200cp_cp4_step_workspace_bytes(const b200cp_tensor_shape* s, int flags) 
   if (check_shape(s, "b200cp_cp4_step_workspace_bytes")) return 0;
   const size_t plain = b200cp_cp4_bwd_filter_workspace_bytes(s, flags);
   if (!step_shares_planes(s, flags)) return plain;
+  const size_t products = takes_planes(s, flags, Planes::kBackward) ? planes_workspace(*s, kPlanesFwd | kPlanesBwd | kPlanesGrads) : 0;
   const size_t plane = align_up((size_t)s->N * s->Rank * s->H * s->W * sizeof(float), 256);
-  return 2 * plane + std::max(std::max(plain, cp4_bwd_filter_saved_workspace(*s)), cp4_grad_band_workspace(*s));
+  return std::max(products, 2 * plane + std::max(std::max(plain, cp4_bwd_filter_saved_workspace(*s)), cp4_grad_band_workspace(*s)));
 }
 
 // The step.  `exchange` (may be null): the peer-memory exchange to run as the tail of the gradient reduction;
@@ -431,6 +612,12 @@ static int cp4_step_impl(const b200cp_tensor_shape* s, const float* X, const flo
     if (int rc = b200cp_cp4_fwd(s, X, K0, K1, KH, KW, U, stream, flags)) return rc;
     if (int rc = b200cp_cp4_bwd_data(s, dU, K0, K1, KH, KW, dX, stream, flags)) return rc;
     return b200cp_cp4_bwd_filter(s, X, dU, K0, K1, KH, KW, dK_packed, workspace, workspace_bytes, stream, fflags);
+  }
+  if (takes_planes(s, flags, Planes::kBackward) &&
+      has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesFwd | kPlanesBwd | kPlanesGrads))) {
+    PlanesJob j;
+    j.s = s; j.X = X; j.dU = dU; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.U = U; j.dX = dX; j.dK = dK_packed;
+    return planes_launch(j, workspace, workspace_bytes, st);
   }
   const size_t plane = align_up((size_t)s->N * s->Rank * s->H * s->W * sizeof(float), 256);
   float* P = static_cast<float*>(workspace);
@@ -645,9 +832,9 @@ int b200cp_cp4_fwd_bwd_data(const b200cp_tensor_shape* s, const float* X, const 
 }
 
 size_t b200cp_cp4_bwd_filter_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
-  (void)flags;
   if (check_shape(s, "b200cp_cp4_bwd_filter_saved_workspace_bytes")) return 0;
-  return std::max(cp4_bwd_filter_saved_workspace(*s), cp4_grad_band_workspace(*s));
+  const size_t need = std::max(cp4_bwd_filter_saved_workspace(*s), cp4_grad_band_workspace(*s));
+  return takes_planes(s, flags, Planes::kBackward) ? std::max(need, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ)) : need;
 }
 
 int b200cp_cp4_bwd_filter_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P,
@@ -658,6 +845,12 @@ int b200cp_cp4_bwd_filter_saved(const b200cp_tensor_shape* s, const float* X, co
   if (!step_shares_planes(s, flags))
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp4_bwd_filter_saved: 3x3 filters with pad 1 on the default (mma) path only");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_filter_saved: workspace is null");
+  if (takes_planes(s, flags, Planes::kBackward) &&
+      has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ))) {
+    PlanesJob j;
+    j.s = s; j.X = X; j.dU = dU; j.P = P; j.Q = Q; j.KH = KH; j.KW = KW; j.dK = dK_packed;
+    return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+  }
   Cp4BwdFilterArgs a{};
   a.N = s->N; a.C = s->C; a.T = s->T; a.H = s->H; a.W = s->W; a.F = 3; a.pad = 1;
   a.Rs = s->Rank;

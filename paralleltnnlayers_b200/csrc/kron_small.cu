@@ -10,14 +10,11 @@
 //   small_conv_kernel  : V[n,t,h,w] = sum_{c,y,x} W[c][y,x][t] X[n,c,h+y-1,w+x-1]
 // All exact fp32 (FFMA).  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
 // and past their set-up when the weight is done.  Formulas: Kernels/rcp_fused_nchw.cu:4-77, Kernels/dense_cp.cu:4-46.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 
+#include "cluster_util.cuh"
 #include "common.cuh"
 #include "mma_util.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace b200cp {
 namespace {
@@ -43,28 +40,6 @@ struct KronGeom {
   int R, rper;             // ranks; ranks per CTA of a cluster
   int flip;                // A[0] is the tap mode, stored back to front
 };
-
-// ---- sum of a cluster's partial tiles ----------------------------------------------------------------------------------
-// Every CTA of the cluster has left its partial tile in shared memory; CTA q adds slice q of all of them in CTA order
-// (the result does not depend on scheduling) and hands each sum to `put`.
-template <typename Put>
-__device__ __forceinline__ void cluster_sum(float* tile, int n, int splits, int tid, int nthreads, Put put) {
-  if (splits == 1) {
-    __syncthreads();
-    for (int i = tid; i < n; i += nthreads) put(i, tile[i]);
-    return;
-  }
-  cg::cluster_group cl = cg::this_cluster();
-  cl.sync();
-  const int q = (int)cl.block_rank(), per = (n + splits - 1) / splits;
-  const int e = min(n, (q + 1) * per);
-  for (int i = q * per + tid; i < e; i += nthreads) {
-    float v = 0.f;
-    for (int p = 0; p < splits; ++p) v += cl.map_shared_rank(tile, p)[i];
-    put(i, v);
-  }
-  cl.sync();   // nobody reads this CTA's tile any more
-}
 
 // entry offset (in ranks) and output offset of half-index (s, f)
 __device__ __forceinline__ void half_decode(const KronMode* m, int n, int s, int f, int flip, int* entry, int* out) {
@@ -451,37 +426,6 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
 size_t spread_smem(size_t need, long ctas, const DeviceInfo& di) {
   const long per = (ctas + di.sm_count - 1) / di.sm_count;
   return per > 4 ? need : std::max(need, (size_t)di.smem_optin / per - (per > 1 ? 1024 : 0));
-}
-
-template <typename... KArgs, typename... Args>
-cudaError_t launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster_z,
-                           bool programmatic, Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  static const bool off = [] {
-    const char* e = getenv("B200CP_PDL");
-    return e && e[0] == '0';
-  }();
-  at[0].val.programmaticStreamSerializationAllowed = programmatic && !off ? 1 : 0;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = 1;
-  at[1].val.clusterDim.y = 1;
-  at[1].val.clusterDim.z = (unsigned)cluster_z;
-  cfg.attrs = at;
-  cfg.numAttrs = cluster_z > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-}
-
-// K units per CTA of a cluster: as many CTAs (at most 8 per cluster) as fill the GPU once, at least `least` units each
-int pick_cluster(long tiles, int units, int least, int sm_count) {
-  int s = 1;
-  while (s < 8 && tiles * s * 2 <= sm_count && units / (s * 2) >= least) s *= 2;
-  return s;
 }
 
 }  // namespace

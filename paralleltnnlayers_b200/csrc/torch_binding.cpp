@@ -62,6 +62,16 @@ inline Tensor workspace(size_t bytes, const Tensor& like) {
   return empty({(int64_t)(std::max<size_t>(bytes, 4) / 4)}, like);
 }
 inline size_t ws_bytes(const Tensor& ws) { return (size_t)ws.numel() * 4; }
+struct Scratch {   // a workspace that may be of no bytes (then nothing is allocated)
+  Tensor t;
+  void* ptr = nullptr;
+  size_t bytes;
+  Scratch(size_t n, const Tensor& like) : bytes(n) {
+    if (n == 0) return;
+    t = workspace(n, like);
+    ptr = t.mutable_data_ptr();
+  }
+};
 
 // ---- CP4 / three-factor CP ------------------------------------------------------------------------------------------
 struct Conv {  // operands of a CP4 convolution, checked and contiguous
@@ -105,12 +115,10 @@ Tensor cp4_forward(const Tensor& X, const Tensor& FT, const Tensor& FC, const Te
   const Conv c(X, "Input", FT, FC, FY, FX, pad, false);
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   Tensor U = c.out_like(c.s.T);
-  if (plane) {
-    *plane = c.out_like(c.s.Rank);
-    ok(b200cp_cp4_fwd_save(&c.s, cp(c.in), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(U), mp(*plane), stream(c.in), flags));
-  } else {
-    ok(b200cp_cp4_fwd(&c.s, cp(c.in), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(U), stream(c.in), flags));
-  }
+  if (plane) *plane = c.out_like(c.s.Rank);
+  const Scratch ws(b200cp_cp4_fwd_workspace_bytes(&c.s, plane != nullptr, flags), c.in);
+  ok(b200cp_cp4_fwd_ws(&c.s, cp(c.in), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(U), plane ? mp(*plane) : nullptr, ws.ptr,
+                       ws.bytes, stream(c.in), flags));
   return U;
 }
 
@@ -119,13 +127,26 @@ Tensor cp4_backward_data(const Tensor& dU, const Tensor& FT, const Tensor& FC, c
   const Conv c(dU, "Upstream", FT, FC, FY, FX, pad, true);
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   Tensor dX = c.out_like(c.s.C);
-  if (plane) {
-    *plane = c.out_like(c.s.Rank);
-    ok(b200cp_cp4_bwd_data_save(&c.s, cp(c.in), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(dX), mp(*plane), stream(c.in),
-                                flags));
-  } else {
-    ok(b200cp_cp4_bwd_data(&c.s, cp(c.in), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(dX), stream(c.in), flags));
-  }
+  if (plane) *plane = c.out_like(c.s.Rank);
+  const Scratch ws(b200cp_cp4_bwd_data_workspace_bytes(&c.s, plane != nullptr, flags), c.in);
+  ok(b200cp_cp4_bwd_data_ws(&c.s, cp(c.in), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(dX), plane ? mp(*plane) : nullptr,
+                            ws.ptr, ws.bytes, stream(c.in), flags));
+  return dX;
+}
+
+// dX and the packed factor gradients from the forward's rank plane
+Tensor cp4_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, const Tensor& FT, const Tensor& FC,
+                          const Tensor& FY, const Tensor& FX, int64_t pad, int flags, Tensor* dK, b200cp_tensor_shape* shape) {
+  const Tensor P = dev(P_, "P"), X = dev(In, "In");
+  const Conv c(dU, "Upstream", FT, FC, FY, FX, pad, true);
+  const c10::cuda::OptionalCUDAGuard guard(c.in.device());
+  const b200cp_tensor_shape& s = c.s;
+  Tensor dX = c.out_like(s.C);
+  *dK = empty({(int64_t)(s.T + s.C + s.Y + s.X) * s.Rank}, c.in);
+  const Scratch ws(b200cp_cp4_bwd_saved_workspace_bytes(&s, flags), c.in);
+  ok(b200cp_cp4_bwd_saved(&s, cp(X), cp(c.in), cp(P), cp(c.FT), cp(c.FC), cp(c.FY), cp(c.FX), mp(dX), mp(*dK), ws.ptr, ws.bytes,
+                          stream(c.in), flags));
+  *shape = s;
   return dX;
 }
 
@@ -177,11 +198,15 @@ struct Conv3 {
   }
 };
 
-Tensor cp3_forward(const Tensor& X, const Tensor& KT, const Tensor& KCin, const Tensor& KC, int64_t pad, int flags) {
+Tensor cp3_forward(const Tensor& X, const Tensor& KT, const Tensor& KCin, const Tensor& KC, int64_t pad, int flags,
+                   Tensor* plane = nullptr) {
   const Conv3 c(X, "Input", KT, KCin, KC, pad, false);
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   Tensor U = empty({c.s.N, c.s.T, c.s.H, c.s.W}, c.in);
-  ok(b200cp_cp3_fwd(&c.s, cp(c.in), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(U), stream(c.in), flags));
+  if (plane) *plane = empty({c.s.N, c.s.Rank, c.s.H, c.s.W}, c.in);
+  const Scratch ws(b200cp_cp3_fwd_workspace_bytes(&c.s, plane != nullptr, flags), c.in);
+  ok(b200cp_cp3_fwd_ws(&c.s, cp(c.in), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(U), plane ? mp(*plane) : nullptr, ws.ptr, ws.bytes,
+                       stream(c.in), flags));
   return U;
 }
 
@@ -189,7 +214,30 @@ Tensor cp3_backward_data(const Tensor& dU, const Tensor& KT, const Tensor& KCin,
   const Conv3 c(dU, "Upstream", KT, KCin, KC, pad, true);
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   Tensor dX = empty({c.s.N, c.s.C, c.s.H, c.s.W}, c.in);
-  ok(b200cp_cp3_bwd_data(&c.s, cp(c.in), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(dX), stream(c.in), flags));
+  const Scratch ws(b200cp_cp3_bwd_data_workspace_bytes(&c.s, flags), c.in);
+  ok(b200cp_cp3_bwd_data_ws(&c.s, cp(c.in), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(dX), ws.ptr, ws.bytes, stream(c.in), flags));
+  return dX;
+}
+
+std::array<Tensor, 3> split3(const Tensor& dK, const b200cp_tensor_shape& s) {
+  const int64_t R = s.Rank, nT = s.T * R, nC = s.C * R, nS = (int64_t)s.Y * s.X * R;
+  return {dK.narrow(0, 0, nT).view({s.T, R}), dK.narrow(0, nT, nC).view({s.C, R}),
+          dK.narrow(0, nT + nC, nS).view({s.Y, s.X, R})};
+}
+
+// dX and the factor gradients from the forward's rank plane
+Tensor cp3_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, const Tensor& KT, const Tensor& KCin,
+                          const Tensor& KC, int64_t pad, int flags, std::array<Tensor, 3>* grads) {
+  const Tensor P = dev(P_, "P"), X = dev(In, "In");
+  const Conv3 c(dU, "Upstream", KT, KCin, KC, pad, true);
+  const c10::cuda::OptionalCUDAGuard guard(c.in.device());
+  const b200cp_tensor_shape& s = c.s;
+  Tensor dX = empty({s.N, s.C, s.H, s.W}, c.in);
+  Tensor dK = empty({(int64_t)(s.T + s.C + s.Y * s.X) * s.Rank}, c.in);
+  const Scratch ws(b200cp_cp3_bwd_saved_workspace_bytes(&s, flags), c.in);
+  ok(b200cp_cp3_bwd_saved(&s, cp(X), cp(c.in), cp(P), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(dX), mp(dK), ws.ptr, ws.bytes,
+                          stream(c.in), flags));
+  *grads = split3(dK, s);
   return dX;
 }
 
@@ -199,13 +247,11 @@ std::array<Tensor, 3> cp3_backward_filter(const Tensor& dU_, const Tensor& In, c
   const Conv3 c(In, "In", KT, KCin, KC, pad, false);
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   const b200cp_tensor_shape& s = c.s;
-  const int64_t R = s.Rank, nT = s.T * R, nC = s.C * R, nS = (int64_t)s.Y * s.X * R;
-  Tensor dK = empty({nT + nC + nS}, c.in);
+  Tensor dK = empty({(int64_t)(s.T + s.C + s.Y * s.X) * s.Rank}, c.in);
   Tensor ws = workspace(b200cp_cp3_bwd_filter_workspace_bytes(&s, flags), c.in);
   ok(b200cp_cp3_bwd_filter(&s, cp(c.in), cp(dU), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(dK), mp(ws), ws_bytes(ws),
                            stream(c.in), flags));
-  return {dK.narrow(0, 0, nT).view({s.T, R}), dK.narrow(0, nT, nC).view({s.C, R}),
-          dK.narrow(0, nT + nC, nS).view({s.Y, s.X, R})};
+  return split3(dK, s);
 }
 
 // ---- reshaped-CP conv and CP dense ------------------------------------------------------------------------------------
@@ -358,9 +404,9 @@ struct CP4Node : torch::autograd::Function<CP4Node> {
     b200cp_tensor_shape s;
     variable_list out(7);
     if (v.size() == 6) {
-      Tensor Q;
-      Tensor dx = cp4_backward_data(dy, FT, FC, FY, FX, pad, flags, &Q);
-      const Grads4 g = split4(cp4_backward_filter_saved(dy, x, v[5], Q, FT, FC, FY, FX, pad, flags, &s), s);
+      Tensor dK;
+      Tensor dx = cp4_backward_saved(dy, x, v[5], FT, FC, FY, FX, pad, flags, &dK, &s);
+      const Grads4 g = split4(dK, s);
       if (ctx->needs_input_grad(0)) out[0] = dx;
       for (int i = 0; i < 4; ++i) out[1 + i] = g[i];
       return out;
@@ -378,6 +424,18 @@ struct CP3Node : torch::autograd::Function<CP3Node> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& KT, const Tensor& KCin, const Tensor& KC,
                         int64_t pad) {
     ctx->saved_data["pad"] = pad;
+    // where the gradients are formed from whole rank planes the forward keeps its own
+    bool shared = false;
+    if ((KT.requires_grad() || KCin.requires_grad() || KC.requires_grad()) && x.dim() == 4) {
+      const Conv3 c(x, "Input", KT, KCin, KC, pad, false);
+      shared = b200cp_cp3_shares_planes(&c.s, 0) != 0;
+    }
+    if (shared) {
+      Tensor P;
+      Tensor y = cp3_forward(x, KT, KCin, KC, pad, 0, &P);
+      ctx->save_for_backward({x, KT, KCin, KC, P});
+      return y;
+    }
     ctx->save_for_backward({x, KT, KCin, KC});
     return cp3_forward(x, KT, KCin, KC, pad, 0);
   }
@@ -386,6 +444,13 @@ struct CP3Node : torch::autograd::Function<CP3Node> {
     const int64_t pad = ctx->saved_data["pad"].toInt();
     const Tensor dy = grads[0].contiguous();
     variable_list out(5);
+    if (v.size() == 5) {
+      std::array<Tensor, 3> g;
+      Tensor dx = cp3_backward_saved(dy, v[0], v[4], v[1], v[2], v[3], pad, 0, &g);
+      if (ctx->needs_input_grad(0)) out[0] = dx;
+      for (int i = 0; i < 3; ++i) out[1 + i] = g[i];
+      return out;
+    }
     if (ctx->needs_input_grad(0)) out[0] = cp3_backward_data(dy, v[1], v[2], v[3], pad, 0);
     if (ctx->needs_input_grad(1) || ctx->needs_input_grad(2) || ctx->needs_input_grad(3)) {
       const std::array<Tensor, 3> g = cp3_backward_filter(dy, v[0], v[1], v[2], v[3], pad, 0);

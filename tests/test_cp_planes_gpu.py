@@ -1,0 +1,119 @@
+"""CP4 and three-factor CP convolutions over whole rank planes, against the float64 oracle.
+
+Sizes at the edges of the products' tiles (16 / 32 / 64 rows, 64 / 128 pixels, 16 channels or ranks and 32 pixels per
+stage): rows, ranks and channels one above and below them, pixel counts that are no multiple of 4 (unaligned rows) and
+that straddle images, images of one row or column, one image, splits over a cluster and none, ranks above one tile.
+Bound: the one of the other parity tests, 1e-4 relative + 1e-5 of the largest value."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from gpu_util import check
+from oracle import cp_oracle as O
+
+# N, C, T, H, W, R
+SHAPES = [
+    (1, 3, 5, 1, 1, 65), (2, 17, 15, 5, 7, 66), (3, 16, 33, 1, 9, 67), (1, 64, 64, 12, 1, 129), (5, 70, 65, 7, 7, 64),
+    (2, 255, 257, 8, 8, 33), (64, 256, 256, 7, 7, 17), (3, 300, 212, 6, 6, 32), (1, 512, 64, 9, 9, 16),
+    (4, 500, 12, 5, 13, 3), (2, 12, 500, 11, 6, 5), (33, 64, 64, 23, 23, 40), (1, 4, 4, 64, 64, 128),
+    (12, 64, 70, 28, 28, 40),   # only the backward over planes, from the plane another kernel wrote
+]
+
+
+def assert_parity(got, ref):
+    check(got, ref, "cp planes", rtol=1e-4, atol=1e-5 * float(np.abs(ref).max()))
+
+
+def make(shape, cp3):
+    N, C, T, H, W, R = shape
+    rng = np.random.default_rng(sum(shape))
+    X = rng.uniform(-1, 1, (N, C, H, W)).astype(np.float32)
+    dU = rng.standard_normal((N, T, H, W)).astype(np.float32)
+    dims = [(T, R), (C, R)] + ([(3, 3, R)] if cp3 else [(3, R), (3, R)])
+    K = [(rng.standard_normal(d) * (9 * C) ** -0.5).astype(np.float32) for d in dims]
+    return X, dU, K
+
+
+def expect(X, dU, K):
+    """Forward, data gradient and factor gradients by float64 autograd of the recomposed convolution."""
+    x = torch.tensor(X, dtype=torch.float64, requires_grad=True)
+    k = [torch.tensor(f, dtype=torch.float64, requires_grad=True) for f in K]
+    w = torch.einsum("tr,cr,yxr->tcyx", *k) if len(k) == 3 else torch.einsum("tr,cr,yr,xr->tcyx", *k)
+    u = torch.nn.functional.conv2d(x, w, padding=1)
+    g = torch.autograd.grad(u, [x] + k, torch.tensor(dU, dtype=torch.float64))
+    return [t.detach().numpy() for t in (u, *g)]
+
+
+def offset(a):
+    """The array on the GPU, contiguous but not 16-byte aligned."""
+    buf = torch.empty(a.size + 1, device="cuda")
+    t = buf[1:].view(a.shape)
+    t.copy_(torch.from_numpy(a))
+    return t
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_cp4(shape, aligned):
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make(shape, False)
+    want = expect(X, dU, K)
+    assert np.allclose(want[0], O.cp4_forward(X, *K, 1), rtol=1e-9, atol=1e-9)
+    put = (lambda a: torch.from_numpy(a).cuda()) if aligned else offset
+    x, du, k = put(X), put(dU), [put(f) for f in K]
+    assert_parity(P.cp4_conv2d_forward(x, *k), want[0])
+    assert_parity(P.cp4_conv2d_backward_data(du, *k), want[1])
+    for got, ref in zip(P.cp4_conv2d_backward_filter(du, x, *k), want[2:]):
+        assert_parity(got, ref)
+    U, dX, dK = P.cp4_conv2d_step(x, du, *k)
+    assert_parity(U, want[0])
+    assert_parity(dX, want[1])
+    o = 0
+    for ref in want[2:]:
+        assert_parity(dK[o:o + ref.size].view(ref.shape), ref)
+        o += ref.size
+    # the layer's node: forward with its plane kept, and the backward from it
+    leaves = [t.clone().requires_grad_() for t in (x, *k)]
+    y = P.CP4Conv2dFunction.apply(*leaves)
+    for got, ref in zip((y, *torch.autograd.grad(y, leaves, du)), want):
+        assert_parity(got, ref)
+
+
+@pytest.mark.parametrize("shape", [s for s in SHAPES if s[5] <= 66])
+def test_cp3(shape):
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make(shape, True)
+    want = expect(X, dU, K)
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+    assert_parity(P.cp3_conv2d_forward(x, *k), want[0])
+    assert_parity(P.cp3_conv2d_backward_data(du, *k), want[1])
+    for got, ref in zip(P.cp3_conv2d_backward_filter(du, x, *k), want[2:]):
+        assert_parity(got, ref)
+    leaves = [t.clone().requires_grad_() for t in (x, *k)]
+    y = P.CP3Conv2dFunction.apply(*leaves)
+    for got, ref in zip((y, *torch.autograd.grad(y, leaves, du)), want):
+        assert_parity(got, ref)
+
+
+def test_streams_and_capture():
+    """Two streams at once, and a captured step: the workspace belongs to the call, nothing is shared."""
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make((4, 96, 40, 9, 9, 70), False)
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+    ref = [t.clone() for t in P.cp4_conv2d_step(x, du, *k)]
+    streams, outs = [torch.cuda.Stream(), torch.cuda.Stream()], []
+    torch.cuda.synchronize()
+    for i in range(6):
+        with torch.cuda.stream(streams[i % 2]):
+            outs.append(P.cp4_conv2d_step(x, du, *k))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs.append(P.cp4_conv2d_step(x, du, *k))
+    graph.replay()
+    torch.cuda.synchronize()
+    for o in outs:
+        for a, b in zip(o, ref):
+            assert torch.equal(a, b)   # fixed summation order
