@@ -245,7 +245,9 @@ cp4_band_kernel(const BandGeom g, const __grid_constant__ CUtensorMap map0, cons
       }
       if (!g.tensor) {
         // what the bulk copies of this band never write must read as zero: halo rows outside the image (the
-        // padding) in every slot, and the channels past Cin in the last stage's slot
+        // padding) in every slot, and the channels past Cin in the last stage's slot.  With more stages than slots that
+        // slot holds an earlier stage first, which may have landed already; its values are what stands there in the
+        // last round, and the factor is zero for them.
         const int zr = ra + (g.TH + 2 - rb);   // rows outside: [0, ra) and [rb, TH + 2)
         if (zr > 0) {
           const int per = zr * W;
@@ -257,7 +259,7 @@ cp4_band_kernel(const BandGeom g, const __grid_constant__ CUtensorMap map0, cons
           }
         }
         const int tail = nst * g.CB - p.Cin;   // channels of the last stage that do not exist
-        if (tail > 0) {
+        if (tail > 0 && nst <= S) {
           float* z0 = ring + (size_t)((nst - 1) % S) * g.stage_floats + (size_t)(g.CB - tail) * XP;
           for (int i = tid; i < tail * XP; i += NTC) z0[i] = 0.f;
         }

@@ -108,3 +108,19 @@ def test_band_step(case):
     U2, gX2, dK2 = P.cp4_conv2d_step(t[0], t[5], *t[1:5], 1)
     assert torch.equal(U, U2) and torch.equal(gX, gX2) and torch.equal(dK, dK2)
     P.device_status()
+
+
+@pytest.mark.parametrize("shape", [(1, 464, 16, 8, 8, 11), (3, 131, 131, 28, 28, 15), (2, 203, 40, 12, 16, 16)])
+def test_more_stages_than_slots_with_a_partial_last_one(shape):
+    """Input channels that do not fill the last stage of a ring that has gone round: the slot of that stage holds
+    another stage first, whose channels must not be cleared.  Bound: 1e-4 relative + 1e-5 of the largest value."""
+    import paralleltnnlayers_b200 as P
+    N, C, T, H, W, R = shape
+    rng = np.random.default_rng(C)
+    X = rng.uniform(-1, 1, (N, C, H, W)).astype(np.float32)
+    K = [(rng.standard_normal((d, R)) * (9 * C) ** -0.5).astype(np.float32) for d in (T, C, 3, 3)]
+    want = O.cp4_forward(X, *K, 1)
+    x, *k = (torch.from_numpy(a).cuda() for a in (X, *K))
+    for _ in range(3):
+        got = P.cp4_conv2d_forward(x, *k).cpu().numpy()
+        assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max() + 1e-4 * np.abs(want).max()
