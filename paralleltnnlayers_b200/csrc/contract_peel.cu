@@ -24,6 +24,7 @@ namespace {
 constexpr int kPT = 256;      // threads per CTA: lane = rank within a block of 32, warp = row / entry group
 constexpr int kRB = 32;       // ranks per CTA
 constexpr int kRows0 = 64;    // rows of G per batch in the first peel
+constexpr int kGPad = 4;      // padding of a staged row of G, floats
 constexpr int kMaxNb = 256;   // entries of one mode (c_dim * t_dim)
 constexpr int kGridCap = 592; // CTAs per level (fixed: the order of the partial sums must not depend on the device)
 
@@ -49,9 +50,13 @@ struct PeelGeom {
 template <int NPW>  // entries of the peeled mode per warp: nbp = 8 * NPW
 __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
   extern __shared__ __align__(16) float smem_f[];
-  const int nbp = 8 * NPW;
-  float* Gs = smem_f;                       // [kRows0][nbp]
-  float* Vs = Gs + kRows0 * nbp;            // [nbp][kRB]
+  // Rows of G four banks apart: the lanes that store a t slab hold eight c (nt floats apart) of four rows, which without
+  // the padding share four banks (8-way conflicts, a quarter of the kernel's shared-memory wavefronts at 8 x 8 entries).  With
+  // the batched loads below: 148 -> 122 us for G of 4096 x 4096 at R = 32; what bounds it now is the shared-memory pipe
+  // (three wavefronts per eight FFMA).
+  const int nbp = 8 * NPW, GP = nbp + kGPad;
+  float* Gs = smem_f;                       // [kRows0][GP]
+  float* Vs = Gs + kRows0 * GP;             // [nbp][kRB]
   float* Ls = Vs + nbp * kRB;               // [kRows0][kRB]
   int* goff = reinterpret_cast<int*>(Ls + kRows0 * kRB);  // [kRows0] G offset of the row, -1 past the end
   int* orow = goff + kRows0;                // [kRows0] row index in the layout of `next`
@@ -79,7 +84,7 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
   if (g.nb < nbp)
     for (int i = tid; i < kRows0 * (nbp - g.nb); i += kPT) {
       const int row = i / (nbp - g.nb), e = g.nb + i - row * (nbp - g.nb);
-      Gs[row * nbp + e] = 0.f;
+      Gs[row * GP + e] = 0.f;
     }
   const int rows = (int)g.rows;  // the host checks that rows and the G offsets fit 31 bits
   const int batches = (rows + kRows0 - 1) / kRows0;
@@ -134,12 +139,21 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
     {
       const int nc = g.b.nc, nt = g.b.nt, per_t = kRows0 * nc;
       const int gc = (int)g.b.gc, gt = (int)g.b.gt;
-      for (int t = 0; t < nt; ++t)
-        for (int i = tid; i < per_t; i += kPT) {
-          const int rc = slab[i], row = rc >> 16, c = rc & 0xffff;
-          const int go = goff[row];
-          Gs[row * nbp + c * nt + t] = go >= 0 ? __ldg(g.src + go + t * gt + c * gc) : 0.f;
+      // eight loads of a thread in flight at a time
+      for (int i = tid; i < per_t; i += kPT) {
+        const int rc = slab[i], row = rc >> 16, c = rc & 0xffff;
+        const int go = goff[row];
+        const float* src = g.src + (go >= 0 ? go : 0) + c * gc;
+        float* dst = Gs + row * GP + c * nt;
+        for (int t0 = 0; t0 < nt; t0 += 8) {
+          float v[8];
+#pragma unroll
+          for (int t = 0; t < 8; ++t) v[t] = go >= 0 && t0 + t < nt ? __ldg(src + (t0 + t) * gt) : 0.f;
+#pragma unroll
+          for (int t = 0; t < 8; ++t)
+            if (t0 + t < nt) dst[t0 + t] = v[t];
         }
+      }
     }
     __syncthreads();
     // next[row][r] = sum_p G[row][p] * vec_b[p][r]: each warp takes kRows0 / 8 rows
@@ -152,7 +166,7 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
         const float v2 = Vs[(p4 + 2) * kRB + lane], v3 = Vs[(p4 + 3) * kRB + lane];
 #pragma unroll
         for (int i = 0; i < kRows0 / 8; ++i) {
-          const float4 gq = *reinterpret_cast<const float4*>(Gs + (wg * (kRows0 / 8) + i) * nbp + p4);
+          const float4 gq = *reinterpret_cast<const float4*>(Gs + (wg * (kRows0 / 8) + i) * GP + p4);
           acc1[i] = fmaf(gq.x, v0, acc1[i]);
           acc1[i] = fmaf(gq.y, v1, acc1[i]);
           acc1[i] = fmaf(gq.z, v2, acc1[i]);
@@ -173,7 +187,7 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
       const float l = Ls[row * kRB + lane];
 #pragma unroll
       for (int i4 = 0; i4 < NPW / 4; ++i4) {
-        const float4 gq = *reinterpret_cast<const float4*>(Gs + row * nbp + wg * NPW + i4 * 4);
+        const float4 gq = *reinterpret_cast<const float4*>(Gs + row * GP + wg * NPW + i4 * 4);
         acc2[i4 * 4 + 0] = fmaf(gq.x, l, acc2[i4 * 4 + 0]);
         acc2[i4 * 4 + 1] = fmaf(gq.y, l, acc2[i4 * 4 + 1]);
         acc2[i4 * 4 + 2] = fmaf(gq.z, l, acc2[i4 * 4 + 2]);
@@ -358,7 +372,7 @@ int contract_factors_launch(int order, const int* cdims, const int* tdims, int R
     dim3 grid(pl.grid[k], ceil_div(R, kRB));
     // partial blocks are per (CTA, rank block): the rank blocks write disjoint columns of the same [nb][R] block
     if (first) {
-      const size_t smem = sizeof(float) * ((size_t)kRows0 * g.nbp + (size_t)g.nbp * kRB + kRows0 * kRB) +
+      const size_t smem = sizeof(float) * ((size_t)kRows0 * (g.nbp + kGPad) + (size_t)g.nbp * kRB + kRows0 * kRB) +
                           sizeof(int) * (6 * kRows0 + kRows0 * g.b.nc);
       if (g.rows > 0x7fffffffL / 2 || (long)taps * T * C > 0x7fffffffL)
         return fail(B200CP_ERR_UNSUPPORTED, "factor contraction: the dense gradient has too many entries");
