@@ -12,6 +12,7 @@
 // programmatic dependents of one another.  Everything is exact fp32 (FFMA).
 // Formulas: Cuda_kernels/cp4Conv2dForward.cu:42-134, cp4Conv2dBackwardData.cu:29-109, cp4Conv2dBackwardFilter.cu:64-257.
 #include <algorithm>
+#include <type_traits>
 
 #include "cluster_util.cuh"
 #include "common.cuh"
@@ -330,28 +331,37 @@ __global__ void __launch_bounds__(kThreads) plane_grad_kernel(const __grid_const
   const float* Z = half ? g.Z[1] : g.Z[0];
   const bool vecD = half ? g.vecD[1] : g.vecD[0], vecZ = g.vecZ;
   const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
-  // rows base .. base + nb - 1 of src [n][total][HW], 32 pixels from q0 on
-  auto load = [&](unsigned dst, const float* src, int base, int total, int nb, int q0, bool vec) {
+  // rows base .. base + NB - 1 of src [n][total][HW], 32 pixels from q0 on; a full tile needs no predicates, which with
+  // the 4-byte copies (H * W not a multiple of 4) are most of the instructions around the FFMA (16 x 256 -> 384 27x27 R = 50: 58 -> 35 us)
+  auto load = [&](auto nb, unsigned dst, const float* src, int base, int total, int q0, bool vec) {
+    constexpr int NB = decltype(nb)::value;
+    const int step = vec ? kThreads / 8 : kThreads / 32, i0 = vec ? tid >> 3 : tid >> 5;
+    const int col = vec ? (tid & 7) * 4 : tid & 31, q = q0 + col, n = q / g.HW;
+    const float* s = src + ((size_t)n * total + base + i0) * g.HW + (q - n * g.HW);
+    const size_t inc = (size_t)step * g.HW;
+    unsigned d = dst + (unsigned)(i0 * kDP + col) * 4u;
+    const bool qin = q < qe;
     if (vec) {
-      const int col = (tid & 7) * 4, q = q0 + col, n = q / g.HW;
-      const float* s = src + ((size_t)n * total + base) * g.HW + (q - n * g.HW);
-      for (int i = tid >> 3; i < nb; i += kThreads / 8) {
-        const bool v = q < qe && base + i < total;
-        mma::cp_async16_s(dst + (unsigned)(i * kDP + col) * 4u, v ? s + (size_t)i * g.HW : src, v ? 16 : 0);
+#pragma unroll
+      for (int i = 0; i < NB / (kThreads / 8); ++i, s += inc, d += (kThreads / 8) * kDP * 4u) {
+        const bool v = qin && base + i0 + i * (kThreads / 8) < total;
+        mma::cp_async16_s(d, v ? s : src, v ? 16 : 0);
       }
+    } else if (base + NB <= total && q0 + kDK <= qe) {
+#pragma unroll
+      for (int i = 0; i < NB / (kThreads / 32); ++i, s += inc, d += (kThreads / 32) * kDP * 4u) mma::cp_async4_s(d, s, 4);
     } else {
-      const int col = tid & 31, q = q0 + col, n = q / g.HW;
-      const float* s = src + ((size_t)n * total + base) * g.HW + (q - n * g.HW);
-      for (int i = tid >> 5; i < nb; i += kThreads / 32) {
-        const bool v = q < qe && base + i < total;
-        mma::cp_async4_s(dst + (unsigned)(i * kDP + col) * 4u, v ? s + (size_t)i * g.HW : src, v ? 4 : 0);
+#pragma unroll
+      for (int i = 0; i < NB / (kThreads / 32); ++i, s += inc, d += (kThreads / 32) * kDP * 4u) {
+        const bool v = qin && base + i0 + i * (kThreads / 32) < total;
+        mma::cp_async4_s(d, v ? s : src, v ? 4 : 0);
       }
     }
   };
   auto load_stage = [&](int st, int q) {
     const unsigned d = sbase + (unsigned)(st * kStage) * 4u;
-    load(d, D, m0, rows, BM, q, vecD);
-    load(d + BM * kDP * 4u, Z, r0, g.R, BN, q, vecZ);
+    load(std::integral_constant<int, BM>{}, d, D, m0, rows, q, vecD);
+    load(std::integral_constant<int, BN>{}, d + BM * kDP * 4u, Z, r0, g.R, q, vecZ);
   };
   float acc[8][TN], total[8][TN];
 #pragma unroll
