@@ -72,54 +72,56 @@ __global__ void __launch_bounds__(kThreads) plane_gemm_kernel(const __grid_const
   const int n = colin ? (q0 + col) / g.HW : 0, p = colin ? q0 + col - n * g.HW : 0;
   const float* in = a.in + (size_t)n * a.K * g.HW + p;
 
-  auto load_f = [&](int st, int k0) {
-    const unsigned d = sbase + (unsigned)(st * kStage) * 4u;
-    if (AK) {
-      if (a.vecF) {
-        for (int i = tid; i < BM * (kGK / 4); i += kThreads) {
-          const int m = i / (kGK / 4), k = (i % (kGK / 4)) * 4;
-          const bool v = m0 + m < a.M && k0 + k < ke;
-          mma::cp_async16_s(d + (unsigned)(m * PA + k) * 4u, v ? a.F + (size_t)(m0 + m) * a.K + k0 + k : a.F, v ? 16 : 0);
-        }
-      } else {
-        for (int i = tid; i < BM * kGK; i += kThreads) {
-          const int m = i / kGK, k = i % kGK;
-          const bool v = m0 + m < a.M && k0 + k < ke;
-          mma::cp_async4_s(d + (unsigned)(m * PA + k) * 4u, v ? a.F + (size_t)(m0 + m) * a.K + k0 + k : a.F, v ? 4 : 0);
-        }
+  // Every thread copies the same column of each stage, so its address runs and what is outside M or the pixels is a copy
+  // of no bytes (zero fill); only the last stage of a K that is no multiple of the stage looks at k.
+  const float* inp = in + (size_t)(kb + row0) * g.HW;
+  auto load_in = [&](int st, int k0) {
+    const unsigned d = sbase + (unsigned)(st * kStage + kAF + row0 * BN + col) * 4u;
+    const float* src = inp;
+    inp += (size_t)kGK * g.HW;
+    const bool full = k0 + kGK <= ke;
+    if (a.vecIn) {
+      const size_t inc = (size_t)R4 * g.HW;
+#pragma unroll
+      for (int i = 0; i < kGK / R4; ++i, src += inc) {
+        const bool v = colin && (full || k0 + row0 + i * R4 < ke);
+        mma::cp_async16_s(d + (unsigned)(i * R4 * BN) * 4u, v ? src : a.in, v ? 16 : 0);
       }
+    } else if (full && q0 + BN <= g.Q) {
+      const size_t inc = (size_t)R1 * g.HW;
+#pragma unroll
+      for (int i = 0; i < kGK / R1; ++i, src += inc) mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, src, 4);
     } else {
-      if (a.vecF) {
-        for (int i = tid; i < kGK * (BM / 4); i += kThreads) {
-          const int k = i / (BM / 4), m = (i % (BM / 4)) * 4;
-          const bool v = m0 + m < a.M && k0 + k < ke;
-          mma::cp_async16_s(d + (unsigned)(k * PA + m) * 4u, v ? a.F + (size_t)(k0 + k) * a.M + m0 + m : a.F, v ? 16 : 0);
-        }
-      } else {
-        for (int i = tid; i < kGK * BM; i += kThreads) {
-          const int k = i / BM, m = i % BM;
-          const bool v = m0 + m < a.M && k0 + k < ke;
-          mma::cp_async4_s(d + (unsigned)(k * PA + m) * 4u, v ? a.F + (size_t)(k0 + k) * a.M + m0 + m : a.F, v ? 4 : 0);
-        }
+      const size_t inc = (size_t)R1 * g.HW;
+#pragma unroll
+      for (int i = 0; i < kGK / R1; ++i, src += inc) {
+        const bool v = colin && k0 + row0 + i * R1 < ke;
+        mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, v ? src : a.in, v ? 4 : 0);
       }
     }
   };
-  auto load_in = [&](int st, int k0) {
-    const unsigned d = sbase + (unsigned)(st * kStage + kAF + row0 * BN + col) * 4u;
-    const float* src = in + (size_t)(k0 + row0) * g.HW;
-    if (a.vecIn) {
+  auto load_f = [&](int st, int k0) {
+    const unsigned d0 = sbase + (unsigned)(st * kStage) * 4u;
+    // groups of 4 floats or single floats along the contiguous index; ROWS threads apart along the other
+    const auto copy = [&](auto width) {
+      constexpr int V = decltype(width)::value, COLS = (AK ? kGK : BM) / V, ROWS = AK ? BM : kGK, RT = kThreads / COLS;
+      const int c = (tid % COLS) * V, r0 = tid / COLS, ld = AK ? a.K : a.M;
+      const int kc = AK ? k0 + c : m0 + c, kr = AK ? m0 + r0 : k0 + r0;
+      const bool cin = kc < (AK ? ke : a.M);
+      const int rend = AK ? a.M : ke;
+      const float* src = a.F + (size_t)kr * ld + kc;
+      const size_t inc = (size_t)RT * ld;
+      unsigned d = d0 + (unsigned)(r0 * PA + c) * 4u;
 #pragma unroll
-      for (int i = 0; i < kGK / R4; ++i) {
-        const bool v = colin && k0 + row0 + i * R4 < ke;
-        mma::cp_async16_s(d + (unsigned)(i * R4 * BN) * 4u, v ? src + (size_t)(i * R4) * g.HW : a.in, v ? 16 : 0);
+      for (int i = 0; i < (ROWS + RT - 1) / RT; ++i, src += inc, d += (unsigned)(RT * PA) * 4u) {
+        if (ROWS % RT && r0 + i * RT >= ROWS) break;
+        const bool v = cin && kr + i * RT < rend;
+        if (V == 4) mma::cp_async16_s(d, v ? src : a.F, v ? 16 : 0);
+        else mma::cp_async4_s(d, v ? src : a.F, v ? 4 : 0);
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < kGK / R1; ++i) {
-        const bool v = colin && k0 + row0 + i * R1 < ke;
-        mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, v ? src + (size_t)(i * R1) * g.HW : a.in, v ? 4 : 0);
-      }
-    }
+    };
+    if (a.vecF) copy(std::integral_constant<int, 4>{});
+    else copy(std::integral_constant<int, 1>{});
   };
 
   float acc[TM][4];
