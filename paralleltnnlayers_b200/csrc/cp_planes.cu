@@ -7,7 +7,7 @@
 // The tile kernels do the three phases of a convolution one after the other in each CTA, on tiles of one image: with
 // many ranks or channels, small images, or widths the row kernels do not take, a CTA is one long serial chain with idle
 // lanes (64 images of 512 x 7x7 at R = 64: 52 us per convolution, 77 us for the factor gradients, for 0.1 GMAC per
-// product; here 31 us and 45 us).  Here a phase is a launch of its own, over the pixels of all images as one flat range, so that a tile is
+// product; here 31 us and 37 us).  Here a phase is a launch of its own, over the pixels of all images as one flat range, so that a tile is
 // always full and the sum can be split over a cluster; the planes (R of C channels) pass through L2.  The launches are
 // programmatic dependents of one another.  Everything is exact fp32 (FFMA).
 // Formulas: Cuda_kernels/cp4Conv2dForward.cu:42-134, cp4Conv2dBackwardData.cu:29-109, cp4Conv2dBackwardFilter.cu:64-257.
