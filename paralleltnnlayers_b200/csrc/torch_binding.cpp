@@ -52,6 +52,17 @@ Tensor dev(const Tensor& t, const char* name) {
   TORCH_CHECK_TYPE(t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat, name, " must be a float32 CUDA tensor");
   return t.is_contiguous() ? t : t.contiguous();
 }
+// The same, on the device of the call: the kernels read every operand by address.
+Tensor dev(const Tensor& t, const char* name, const Tensor& input) {
+  Tensor c = dev(t, name);
+  TORCH_CHECK_VALUE(c.device() == input.device(), name, " is on ", c.device(), ", the input on ", input.device());
+  return c;
+}
+// A tensor the kernels index by another operand's sizes
+void check_size(const Tensor& t, const char* name, at::IntArrayRef size) {
+  TORCH_CHECK_VALUE(t.numel() == c10::multiply_integers(size), name, " has ", t.numel(), " values where the shapes of the call give ",
+                    size);
+}
 inline const float* cp(const Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); }
 inline float* mp(const Tensor& t) { return static_cast<float*>(t.mutable_data_ptr()); }
 inline Tensor empty(at::IntArrayRef size, const Tensor& like) {
@@ -79,7 +90,7 @@ struct Conv {  // operands of a CP4 convolution, checked and contiguous
   b200cp_tensor_shape s;
   Conv(const Tensor& in_, const char* in_name, const Tensor& ft, const Tensor& fc, const Tensor& fy, const Tensor& fx,
        int64_t pad, bool in_is_upstream)
-      : in(dev(in_, in_name)), FT(dev(ft, "FT")), FC(dev(fc, "FC")), FY(dev(fy, "FY")), FX(dev(fx, "FX")) {
+      : in(dev(in_, in_name)), FT(dev(ft, "FT", in)), FC(dev(fc, "FC", in)), FY(dev(fy, "FY", in)), FX(dev(fx, "FX", in)) {
     TORCH_CHECK_VALUE(in.dim() == 4, "input must be a rank-4 NCHW tensor");
     const Tensor* f[4] = {&FT, &FC, &FY, &FX};
     const char* nm[4] = {"FT", "FC", "FY", "FX"};
@@ -92,6 +103,10 @@ struct Conv {  // operands of a CP4 convolution, checked and contiguous
          (unsigned)FC.size(0), (unsigned)FY.size(0), (unsigned)FX.size(0), (unsigned)FT.size(1)};
   }
   Tensor out_like(unsigned channels) const { return empty({s.N, channels, s.H, s.W}, in); }
+  // the rank planes, the upstream gradient and the input of a convolution of this shape
+  void check_plane(const Tensor& P, const char* name) const { check_size(P, name, {s.N, s.Rank, s.H, s.W}); }
+  void check_out(const Tensor& dU, const char* name) const { check_size(dU, name, {s.N, s.T, s.H, s.W}); }
+  void check_in(const Tensor& X, const char* name) const { check_size(X, name, {s.N, s.C, s.H, s.W}); }
   void check_upstream(const Tensor& dU, const char* what) const {
     TORCH_CHECK_VALUE(dU.dim() == 4 && dU.size(0) == s.N && dU.size(1) == s.T && dU.size(2) == s.H && dU.size(3) == s.W,
                       what);
@@ -137,8 +152,10 @@ Tensor cp4_backward_data(const Tensor& dU, const Tensor& FT, const Tensor& FC, c
 // dX and the packed factor gradients from the forward's rank plane
 Tensor cp4_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, const Tensor& FT, const Tensor& FC,
                           const Tensor& FY, const Tensor& FX, int64_t pad, int flags, Tensor* dK, b200cp_tensor_shape* shape) {
-  const Tensor P = dev(P_, "P"), X = dev(In, "In");
   const Conv c(dU, "Upstream", FT, FC, FY, FX, pad, true);
+  const Tensor P = dev(P_, "P", c.in), X = dev(In, "In", c.in);
+  c.check_plane(P, "P");
+  c.check_in(X, "In");
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   const b200cp_tensor_shape& s = c.s;
   Tensor dX = c.out_like(s.C);
@@ -153,8 +170,8 @@ Tensor cp4_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, 
 // the packed gradient buffer [dFT|dFC|dFY|dFX]
 Tensor cp4_backward_filter(const Tensor& dU_, const Tensor& In, const Tensor& FT, const Tensor& FC, const Tensor& FY,
                            const Tensor& FX, int64_t pad, int flags, b200cp_tensor_shape* shape) {
-  const Tensor dU = dev(dU_, "dLdO");
   const Conv c(In, "In", FT, FC, FY, FX, pad, false);
+  const Tensor dU = dev(dU_, "dLdO", c.in);
   c.check_upstream(dU, "dLdO must be [N,T,H,W]");
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   const b200cp_tensor_shape& s = c.s;
@@ -169,8 +186,11 @@ Tensor cp4_backward_filter(const Tensor& dU_, const Tensor& In, const Tensor& FT
 Tensor cp4_backward_filter_saved(const Tensor& dU_, const Tensor& In, const Tensor& P_, const Tensor& Q_, const Tensor& FT,
                                  const Tensor& FC, const Tensor& FY, const Tensor& FX, int64_t pad, int flags,
                                  b200cp_tensor_shape* shape) {
-  const Tensor dU = dev(dU_, "dLdO"), P = dev(P_, "P"), Q = dev(Q_, "Q");
   const Conv c(In, "In", FT, FC, FY, FX, pad, false);
+  const Tensor dU = dev(dU_, "dLdO", c.in), P = dev(P_, "P", c.in), Q = dev(Q_, "Q", c.in);
+  c.check_out(dU, "dLdO");
+  c.check_plane(P, "P");
+  c.check_plane(Q, "Q");
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   const b200cp_tensor_shape& s = c.s;
   Tensor dK = empty({(int64_t)(s.T + s.C + s.Y + s.X) * s.Rank}, c.in);
@@ -186,7 +206,7 @@ struct Conv3 {
   b200cp_tensor_shape s;
   Conv3(const Tensor& in_, const char* in_name, const Tensor& kt, const Tensor& kcin, const Tensor& kc, int64_t pad,
         bool in_is_upstream)
-      : in(dev(in_, in_name)), KT(dev(kt, "KT")), KC_in(dev(kcin, "KCin")), KC(dev(kc, "KC")) {
+      : in(dev(in_, in_name)), KT(dev(kt, "KT", in)), KC_in(dev(kcin, "KCin", in)), KC(dev(kc, "KC", in)) {
     TORCH_CHECK_VALUE(in.dim() == 4 && KT.dim() == 2 && KC_in.dim() == 2 && KC.dim() == 3,
                       "expected input [N,ch,H,W], KT [T,R], KCin [C,R], KC [Y,X,R]");
     const int64_t R = KT.size(1);
@@ -228,10 +248,12 @@ std::array<Tensor, 3> split3(const Tensor& dK, const b200cp_tensor_shape& s) {
 // dX and the factor gradients from the forward's rank plane
 Tensor cp3_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, const Tensor& KT, const Tensor& KCin,
                           const Tensor& KC, int64_t pad, int flags, std::array<Tensor, 3>* grads) {
-  const Tensor P = dev(P_, "P"), X = dev(In, "In");
   const Conv3 c(dU, "Upstream", KT, KCin, KC, pad, true);
-  const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   const b200cp_tensor_shape& s = c.s;
+  const Tensor P = dev(P_, "P", c.in), X = dev(In, "In", c.in);
+  check_size(P, "P", {s.N, s.Rank, s.H, s.W});
+  check_size(X, "In", {s.N, s.C, s.H, s.W});
+  const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   Tensor dX = empty({s.N, s.C, s.H, s.W}, c.in);
   Tensor dK = empty({(int64_t)(s.T + s.C + s.Y * s.X) * s.Rank}, c.in);
   const Scratch ws(b200cp_cp3_bwd_saved_workspace_bytes(&s, flags), c.in);
@@ -243,10 +265,11 @@ Tensor cp3_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, 
 
 std::array<Tensor, 3> cp3_backward_filter(const Tensor& dU_, const Tensor& In, const Tensor& KT, const Tensor& KCin,
                                           const Tensor& KC, int64_t pad, int flags) {
-  const Tensor dU = dev(dU_, "dLdO");
   const Conv3 c(In, "In", KT, KCin, KC, pad, false);
-  const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   const b200cp_tensor_shape& s = c.s;
+  const Tensor dU = dev(dU_, "dLdO", c.in);
+  check_size(dU, "dLdO", {s.N, s.T, s.H, s.W});
+  const c10::cuda::OptionalCUDAGuard guard(c.in.device());
   Tensor dK = empty({(int64_t)(s.T + s.C + s.Y * s.X) * s.Rank}, c.in);
   Tensor ws = workspace(b200cp_cp3_bwd_filter_workspace_bytes(&s, flags), c.in);
   ok(b200cp_cp3_bwd_filter(&s, cp(c.in), cp(dU), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(dK), mp(ws), ws_bytes(ws),
@@ -261,11 +284,11 @@ struct Modes {
   std::vector<int> a, b;
   std::vector<const float*> ptr;
   int64_t na = 1, nb = 1;
-  Modes(at::TensorList f, const char* what) {
+  Modes(at::TensorList f, const char* what, const Tensor& input) {
     order = (int)f.size();
     TORCH_CHECK_VALUE(order >= 1, what, ": no kernels given");
     for (int k = 0; k < order; ++k) {
-      F.push_back(dev(f[k], ("kernel" + std::to_string(k)).c_str()));
+      F.push_back(dev(f[k], ("kernel" + std::to_string(k)).c_str(), input));
       const Tensor& t = F.back();
       TORCH_CHECK_VALUE(t.dim() == 3 && t.size(2) == F[0].size(2), what, ": kernel ", k,
                         " must be [in, out, rank] with a common rank");
@@ -277,13 +300,17 @@ struct Modes {
     }
     R = (int)F[0].size(2);
   }
+  Tensor core(const Tensor& KC_, const Tensor& input) const {   // the spatial core of a convolution with these modes
+    const Tensor KC = dev(KC_, "kernelc", input);
+    TORCH_CHECK_VALUE(KC.dim() == 3 && KC.size(2) == R, "kernelc must be [FH, FW, rank]");
+    return KC;
+  }
 };
 
 Tensor rcp_forward(const Tensor& U_, at::TensorList A, const Tensor& KC_, int flags) {
   const Tensor U = dev(U_, "input");
-  const Modes m(A, "conv2d_rcp_fused_nchw");
-  const Tensor KC = dev(KC_, "kernelc");
-  TORCH_CHECK_VALUE(KC.dim() == 3 && KC.size(2) == m.R, "kernelc must be [FH, FW, rank]");
+  const Modes m(A, "conv2d_rcp_fused_nchw", U);
+  const Tensor KC = m.core(KC_, U);
   const int64_t nd = U.dim();
   const bool folded = nd == 4;
   if (!folded) {
@@ -315,10 +342,14 @@ struct FactorGrads {
 
 FactorGrads rcp_backward(const Tensor& U_, const Tensor& dV_, at::TensorList A, const Tensor& KC_, int flags, bool need_dx,
                          bool need_dw) {
-  const Tensor U = dev(U_, "input"), dV = dev(dV_, "dV");
-  const Modes m(A, "rcp_conv2d_backward");
-  const Tensor KC = dev(KC_, "kernelc");
-  const int64_t nd = U.dim(), N = U.size(0), H = U.size(nd - 2), W = U.size(nd - 1);
+  const Tensor U = dev(U_, "input"), dV = dev(dV_, "dV", U);
+  const Modes m(A, "rcp_conv2d_backward", U);
+  const Tensor KC = m.core(KC_, U);
+  const int64_t nd = U.dim();
+  TORCH_CHECK_VALUE(nd >= 2, "input must be [N, S0, .., H, W]");
+  const int64_t N = U.size(0), H = U.size(nd - 2), W = U.size(nd - 1);
+  check_size(U, "input", {N, m.na, H, W});
+  check_size(dV, "dV", {N, m.nb, H, W});
   const c10::cuda::OptionalCUDAGuard guard(U.device());
   FactorGrads g;
   std::vector<float*> dp;
@@ -341,7 +372,7 @@ FactorGrads rcp_backward(const Tensor& U_, const Tensor& dV_, at::TensorList A, 
 
 Tensor dense_forward(const Tensor& U_, at::TensorList F, int flags) {
   const Tensor U = dev(U_, "input");
-  const Modes m(F, "dense_cp");
+  const Modes m(F, "dense_cp", U);
   const int64_t B = U.size(0);
   TORCH_CHECK_VALUE(U.numel() == B * m.na, "input size does not match the kernels");
   const c10::cuda::OptionalCUDAGuard guard(U.device());
@@ -356,9 +387,11 @@ Tensor dense_forward(const Tensor& U_, at::TensorList F, int flags) {
 }
 
 FactorGrads dense_backward(const Tensor& U_, const Tensor& dV_, at::TensorList F, int flags, bool need_dx, bool need_dw) {
-  const Tensor U = dev(U_, "input"), dV = dev(dV_, "dV");
-  const Modes m(F, "dense_cp_backward");
+  const Tensor U = dev(U_, "input"), dV = dev(dV_, "dV", U);
+  const Modes m(F, "dense_cp_backward", U);
   const int B = (int)U.size(0);
+  check_size(U, "input", {B, m.na});
+  check_size(dV, "dV", {B, m.nb});
   const c10::cuda::OptionalCUDAGuard guard(U.device());
   FactorGrads g;
   std::vector<float*> dp;
@@ -590,8 +623,8 @@ PYFN(py_cp4_forward_backward_data) {
   if (save < 0) throw python_error();
   std::array<Tensor, 4> r;
   unlocked([&] {
-    const Tensor dU = dev(du, "Upstream");
     const Conv c(x, "Input", ft, fc, fy, fx, pad, false);
+    const Tensor dU = dev(du, "Upstream", c.in);
     c.check_upstream(dU, "Upstream must be [N, T, H, W]");
     const c10::cuda::OptionalCUDAGuard guard(c.in.device());
     r[0] = c.out_like(c.s.T);
@@ -639,8 +672,8 @@ PYFN(py_cp4_step) {
   const int64_t pad = int_arg(a[6]), flags = int_arg(a[7]);
   std::array<Tensor, 3> r;
   unlocked([&] {
-    const Tensor dU = dev(du, "dU");
     const Conv c(x, "X", ft, fc, fy, fx, pad, false);
+    const Tensor dU = dev(du, "dU", c.in);
     c.check_upstream(dU, "dU must be [N,T,H,W]");
     const c10::cuda::OptionalCUDAGuard guard(c.in.device());
     const b200cp_tensor_shape& s = c.s;

@@ -21,6 +21,50 @@ def test_wrong_tensors_are_type_errors(lib_built, call):
         call(P)
 
 
+# N, C, T, H, W, R = 2, 4, 6, 5, 5, 3; modes 2x2 -> 3x2.  Each call has one operand whose size or device does not go
+# with the others; `c` makes fake CUDA tensors, so that nothing can be launched.
+def _k4(c):
+    return c(6, 3), c(4, 3), c(3, 3), c(3, 3)
+
+
+def _k3(c):
+    return c(6, 3), c(4, 3), c(3, 3, 3)
+
+
+def _modes(c):
+    return c(2, 3, 3), c(2, 2, 3)
+
+
+MISFITS = {
+    "saved dLdO": lambda P, c: P.cp4_conv2d_backward_filter_saved(c(2, 6, 5, 4), c(2, 4, 5, 5), c(2, 3, 5, 5), c(2, 3, 5, 5), *_k4(c)),
+    "saved P": lambda P, c: P.cp4_conv2d_backward_filter_saved(c(2, 6, 5, 5), c(2, 4, 5, 5), c(1, 3, 5, 5), c(2, 3, 5, 5), *_k4(c)),
+    "saved Q": lambda P, c: P.cp4_conv2d_backward_filter_saved(c(2, 6, 5, 5), c(2, 4, 5, 5), c(2, 3, 5, 5), c(2, 2, 5, 5), *_k4(c)),
+    "cp3 dLdO": lambda P, c: P.cp3_conv2d_backward_filter(c(2, 6, 4, 5), c(2, 4, 5, 5), *_k3(c)),
+    "rcp input": lambda P, c: P.rcp_conv2d_backward(c(2, 3, 5, 5), c(2, 6, 5, 5), *_modes(c), c(3, 3, 3)),
+    "rcp dV": lambda P, c: P.rcp_conv2d_backward(c(2, 4, 5, 5), c(2, 5, 5, 5), *_modes(c), c(3, 3, 3)),
+    "rcp core": lambda P, c: P.rcp_conv2d_backward(c(2, 4, 5, 5), c(2, 6, 5, 5), *_modes(c), c(3, 3, 2)),
+    "rcp vector": lambda P, c: P.rcp_conv2d_backward(c(1), c(6), c(1, 6, 3), c(1, 1, 3)),
+    "dense input": lambda P, c: P.dense_cp_backward(c(2, 3), c(2, 6), *_modes(c)),
+    "dense dV": lambda P, c: P.dense_cp_backward(c(2, 4), c(1, 6), *_modes(c)),
+    "cp4 device": lambda P, c: P.cp4_conv2d_forward(c(2, 4, 5, 5), *_k4(c)[:3], c(3, 3, dev=1)),
+    "cp4 dLdO device": lambda P, c: P.cp4_conv2d_backward_filter(c(2, 6, 5, 5, dev=1), c(2, 4, 5, 5), *_k4(c)),
+    "cp4 pair device": lambda P, c: P.cp4_conv2d_forward_backward_data(c(2, 4, 5, 5), c(2, 6, 5, 5, dev=1), *_k4(c)),
+    "step device": lambda P, c: P.cp4_conv2d_step(c(2, 4, 5, 5), c(2, 6, 5, 5, dev=1), *_k4(c)),
+    "cp3 device": lambda P, c: P.cp3_conv2d_forward(c(2, 4, 5, 5), *_k3(c)[:2], c(3, 3, 3, dev=1)),
+    "rcp device": lambda P, c: P.conv2d_rcp_fused_nchw(c(2, 4, 5, 5), *_modes(c), c(3, 3, 3, dev=1)),
+    "dense device": lambda P, c: P.dense_cp(c(2, 4), c(2, 3, 3, dev=1), c(2, 2, 3)),
+    "dense dV device": lambda P, c: P.dense_cp_backward(c(2, 4), c(2, 6, dev=1), *_modes(c)),
+}
+
+
+@pytest.mark.parametrize("what", MISFITS)
+def test_operands_that_do_not_fit_are_value_errors(lib_built, what):
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    import paralleltnnlayers_b200 as P
+    with FakeTensorMode(), pytest.raises(ValueError):
+        MISFITS[what](P, lambda *size, dev=0: torch.empty(*size, device=f"cuda:{dev}"))
+
+
 @pytest.mark.gpu
 def test_shape_errors_and_status_errors():
     import paralleltnnlayers_b200 as P
