@@ -28,10 +28,38 @@ def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _dev(t, name):
+def _dev(t, name, like=None):
+    """``t`` contiguous; with ``like`` it has to be on that tensor's device (the kernels read by address)."""
     if not isinstance(t, torch.Tensor) or not t.is_cuda or t.dtype != torch.float32:
         raise TypeError(f"{name} must be a float32 CUDA tensor")
+    if like is not None and t.device != like.device:
+        raise ValueError(f"{name} is on {t.device}, the first operand on {like.device}")
     return t.contiguous()
+
+
+def _factors4(ts, like=None):
+    """FT, FC, FY, FX ``[dim, rank]`` with one rank, on one device."""
+    like = ts[0] if like is None else like
+    ts = [_dev(t, n, like) for t, n in zip(ts, ("FT", "FC", "FY", "FX"))]
+    if any(f.dim() != 2 or f.shape[1] != ts[0].shape[1] for f in ts):
+        raise ValueError("FT, FC, FY and FX must be [dim, rank] with one rank")
+    return ts
+
+
+def _host_shape(X, dU, FT, FC, FY, FX, pad, out):
+    """Checked operands of the host-buffer step: contiguous float32 CPU tensors of the sizes the copies take."""
+    for t in [X, dU, FT, FC, FY, FX] + list(out or ()):
+        if t.is_cuda or t.dtype != torch.float32 or not t.is_contiguous():
+            raise TypeError("host entry point takes contiguous float32 CPU tensors")
+    s = _shape_from(X, FT, FC, FY, FX, pad)
+    n_out = s.N * s.T * s.H * s.W
+    if dU.numel() != n_out:
+        raise ValueError("dU must be [N,T,H,W]")
+    if out is not None:
+        U, dX, dK = out
+        if U.numel() != n_out or dX.numel() != X.numel() or dK.numel() != (s.T + s.C + s.Y + s.X) * s.Rank:
+            raise ValueError("out must be (U [N,T,H,W], dX [N,C,H,W], dK_packed [(T+C+Y+X)*R])")
+    return s
 
 
 def _p(t):
@@ -82,7 +110,10 @@ def cp4_conv2d_backward_filter(dLdO, In, FT, FC, FY, FX, pad=1, flags=0, packed=
 
 def cp4_conv2d_backward_filter_full(dLdO, In, Y, X, pad=1):
     """``cp4_conv2d_backward_filter_full_gpu`` (Cuda_kernels/cp4Conv2dBackwardFilter.cu:23-59): dK [T,C,Y,X]."""
-    dLdO, In = _dev(dLdO, "dLdO"), _dev(In, "In")
+    In = _dev(In, "In")
+    dLdO = _dev(dLdO, "dLdO", In)
+    if In.dim() != 4 or dLdO.dim() < 2 or dLdO.numel() != In.shape[0] * dLdO.shape[1] * In.shape[2] * In.shape[3]:
+        raise ValueError("dLdO must be [N,T,H,W] for In [N,C,H,W]")
     s = tensor_shape(In.shape[0], In.shape[1], In.shape[2], In.shape[3], dLdO.shape[1], Y, X, 1, pad)
     dK = torch.empty((s.T, s.C, Y, X), device=In.device, dtype=torch.float32)
     with torch.cuda.device(In.device):
@@ -92,7 +123,7 @@ def cp4_conv2d_backward_filter_full(dLdO, In, Y, X, pad=1):
 
 def cp4recom(FT, FC, FY, FX):
     """``cp4recom`` (Cuda_kernels/Utils.cu:67-98): dense K [T,C,Y,X]."""
-    FT, FC, FY, FX = (_dev(t, n) for t, n in ((FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
+    FT, FC, FY, FX = _factors4((FT, FC, FY, FX))
     s = tensor_shape(1, FC.shape[0], 1, 1, FT.shape[0], FY.shape[0], FX.shape[0], FT.shape[1], 0)
     K = torch.empty((s.T, s.C, s.Y, s.X), device=FT.device, dtype=torch.float32)
     with torch.cuda.device(FT.device):
@@ -103,7 +134,8 @@ def cp4recom(FT, FC, FY, FX):
 def allclose(A, B, tolerance=1e-3):
     """``AllClose`` (Cuda_kernels/Utils.cu:159-180): True when no element's relative difference
     max(|a-b|/|a|, |a-b|/|b|) exceeds ``tolerance``; the count runs on the device."""
-    A, B = _dev(A, "A"), _dev(B, "B")
+    A = _dev(A, "A")
+    B = _dev(B, "B", A)
     if A.numel() != B.numel():
         return False
     n = C.c_ulonglong(0)
@@ -137,12 +169,7 @@ def cp4_conv2d_step_host(X, dU, FT, FC, FY, FX, pad=1, flags=0, out=None):
     """Forward + both backward passes through the host-buffer entry point
     (``b200cp_cp4_step_host``): CPU tensors in, CPU tensors out, transfers included.
     ``out`` may hold preallocated (pinned) ``(U, dX, dK_packed)``."""
-    ts = [X, dU, FT, FC, FY, FX]
-    for t in ts:
-        if t.is_cuda or t.dtype != torch.float32 or not t.is_contiguous():
-            raise TypeError("host entry point takes contiguous float32 CPU tensors")
-    s = tensor_shape(X.shape[0], FC.shape[0], X.shape[2], X.shape[3], FT.shape[0], FY.shape[0], FX.shape[0],
-                     FT.shape[1], pad)
+    s = _host_shape(X, dU, FT, FC, FY, FX, pad, out)
     R = s.Rank
     if out is None:
         out = (torch.empty((s.N, s.T, s.H, s.W)), torch.empty((s.N, s.C, s.H, s.W)),
@@ -157,15 +184,8 @@ def cp4_conv2d_step_host_submit(X, dU, FT, FC, FY, FX, out, pad=1, flags=0, slot
     """Queue one step on ``slot`` (0 .. 3) through ``b200cp_cp4_step_host_submit``; ``out`` holds the pinned
     ``(U, dX, dK_packed)`` that ``cp4_conv2d_step_host_wait(slot)`` fills.  Inputs and outputs must stay
     alive and untouched until that wait returns."""
-    ts = [X, dU, FT, FC, FY, FX] + list(out)
-    for t in ts:
-        if t.is_cuda or t.dtype != torch.float32 or not t.is_contiguous():
-            raise TypeError("host entry point takes contiguous float32 CPU tensors")
-    s = tensor_shape(X.shape[0], FC.shape[0], X.shape[2], X.shape[3], FT.shape[0], FY.shape[0], FX.shape[0],
-                     FT.shape[1], pad)
+    s = _host_shape(X, dU, FT, FC, FY, FX, pad, out)
     U, dX, dK = out
-    if U.numel() != s.N * s.T * s.H * s.W or dX.numel() != X.numel() or dK.numel() != (s.T + s.C + s.Y + s.X) * s.Rank:
-        raise ValueError("out must be (U [N,T,H,W], dX [N,C,H,W], dK_packed [(T+C+Y+X)*R])")
     check(lib.b200cp_cp4_step_host_submit(C.byref(s), _p(X), _p(dU), _p(FT), _p(FC), _p(FY), _p(FX), _p(U), _p(dX),
                                           _p(dK), flags, slot))
 
@@ -202,7 +222,8 @@ def set_stream(on):
 
 def debug_cp4_tc(Input, FT, FC, FY, FX, pad=1, terms=3, p_floats=0):
     """Diagnostic forward on the tensor path; also returns the first CTA's rank-R intermediate."""
-    Input, FT, FC, FY, FX = (_dev(t, n) for t, n in ((Input, "Input"), (FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
+    Input = _dev(Input, "Input")
+    FT, FC, FY, FX = _factors4((FT, FC, FY, FX), Input)
     s = _shape_from(Input, FT, FC, FY, FX, pad)
     out = torch.empty((s.N, s.T, s.H, s.W), device=Input.device, dtype=torch.float32)
     P = torch.zeros(max(p_floats, 1), device=Input.device, dtype=torch.float32)
@@ -278,8 +299,9 @@ def dense_cp_backward(U, dV, *kernels, flags=0, need_dx=True, need_dw=True):
 def conv2d_dense_forward(Input, K, pad=1):
     """Ordinary conv2d with a dense filter ``K [T,C,Y,X]``, H x W output: the ``tf.nn.conv2d(U, K, ..., 'SAME')`` of
     test/benchmark_conv2d_cp4.py:41."""
-    Input, K = _dev(Input, "Input"), _dev(K, "K")
-    if K.dim() != 4 or K.shape[1] != Input.shape[1]:
+    Input = _dev(Input, "Input")
+    K = _dev(K, "K", Input)
+    if Input.dim() != 4 or K.dim() != 4 or K.shape[1] != Input.shape[1]:
         raise ValueError("K must be [T, C, Y, X] with C the input's channel count")
     s = tensor_shape(Input.shape[0], Input.shape[1], Input.shape[2], Input.shape[3], K.shape[0], K.shape[2],
                      K.shape[3], 1, pad)
@@ -294,7 +316,7 @@ def conv2d_dense_forward(Input, K, pad=1):
 def cp4_conv2d_rebuild_forward(Input, FT, FC, FY, FX, pad=1):
     """The CP4 layer's "rebuild" line (test/benchmark_conv2d_cp4.py:35-42): ``cp4recom`` then an ordinary conv2d."""
     Input = _dev(Input, "Input")
-    FT, FC, FY, FX = (_dev(t, n) for t, n in ((FT, "FT"), (FC, "FC"), (FY, "FY"), (FX, "FX")))
+    FT, FC, FY, FX = _factors4((FT, FC, FY, FX), Input)
     s = _shape_from(Input, FT, FC, FY, FX, pad)
     U = torch.empty((s.N, s.T, s.H, s.W), device=Input.device, dtype=torch.float32)
     with torch.cuda.device(Input.device):
@@ -308,8 +330,8 @@ def cp4_conv2d_rebuild_forward(Input, FT, FC, FY, FX, pad=1):
 def rcp_recompose(*kernels):
     """Dense filter ``[T, C, FH, FW]`` of the reshaped-CP conv from ``(K0[S0,T0,R], ..., KC[FH,FW,R])``."""
     *A, KC = kernels
-    A = [_dev(a, f"kernel{k}") for k, a in enumerate(A)]
     KC = _dev(KC, "kernelc")
+    A = [_dev(a, f"kernel{k}", KC) for k, a in enumerate(A)]
     cd, td, R = _modes(A, "rcp_recompose")
     if KC.dim() != 3 or KC.shape[2] != R:
         raise ValueError("kernelc must be [FH, FW, rank]")
@@ -334,7 +356,7 @@ def conv2d_rcp_rebuild_nchw(U, *kernels):
 
 def dense_cp_recompose(*kernels):
     """``M [I, O]`` of the CP dense layer (the einsum + reshape of test/benchmark_dense_cp.py:43-44)."""
-    Fk = [_dev(f, f"kernel{k}") for k, f in enumerate(kernels)]
+    Fk = [_dev(f, f"kernel{k}", kernels[0]) for k, f in enumerate(kernels)]
     idims, odims, R = _modes(Fk, "dense_cp_recompose")
     I, O = 1, 1
     for a, b in zip(idims, odims):
@@ -352,7 +374,8 @@ def dense_cp_recompose(*kernels):
 
 def dense_matmul(U, M):
     """``U [B, I] @ M [I, O]`` with fp32-grade results (test/benchmark_dense_cp.py:45-48)."""
-    U, M = _dev(U, "input"), _dev(M, "M")
+    U = _dev(U, "input")
+    M = _dev(M, "M", U)
     B = U.shape[0]
     I, O = M.shape
     if U.numel() != B * I:

@@ -53,6 +53,16 @@ MISFITS = {
     "cp3 device": lambda P, c: P.cp3_conv2d_forward(c(2, 4, 5, 5), *_k3(c)[:2], c(3, 3, 3, dev=1)),
     "rcp device": lambda P, c: P.conv2d_rcp_fused_nchw(c(2, 4, 5, 5), *_modes(c), c(3, 3, 3, dev=1)),
     "dense device": lambda P, c: P.dense_cp(c(2, 4), c(2, 3, 3, dev=1), c(2, 2, 3)),
+    "full dLdO": lambda P, c: P.cp4_conv2d_backward_filter_full(c(2, 6, 4, 5), c(2, 4, 5, 5), 3, 3),
+    "full device": lambda P, c: P.cp4_conv2d_backward_filter_full(c(2, 6, 5, 5, dev=1), c(2, 4, 5, 5), 3, 3),
+    "recompose rank": lambda P, c: P.cp4recom(c(6, 3), c(4, 2), c(3, 3), c(3, 3)),
+    "recompose device": lambda P, c: P.cp4recom(c(6, 3), c(4, 3, dev=1), c(3, 3), c(3, 3)),
+    "rcp recompose device": lambda P, c: P.rcp_recompose(*_modes(c), c(3, 3, 3, dev=1)),
+    "dense recompose device": lambda P, c: P.dense_cp_recompose(c(2, 3, 3), c(2, 2, 3, dev=1)),
+    "rebuild device": lambda P, c: P.cp4_conv2d_rebuild_forward(c(2, 4, 5, 5, dev=1), *_k4(c)),
+    "conv device": lambda P, c: P.conv2d_dense_forward(c(2, 4, 5, 5), c(6, 4, 3, 3, dev=1)),
+    "matmul device": lambda P, c: P.dense_matmul(c(2, 4), c(4, 6, dev=1)),
+    "allclose device": lambda P, c: P.allclose(c(2, 4), c(2, 4, dev=1)),
     "dense dV device": lambda P, c: P.dense_cp_backward(c(2, 4), c(2, 6, dev=1), *_modes(c)),
 }
 
@@ -63,6 +73,19 @@ def test_operands_that_do_not_fit_are_value_errors(lib_built, what):
     import paralleltnnlayers_b200 as P
     with FakeTensorMode(), pytest.raises(ValueError):
         MISFITS[what](P, lambda *size, dev=0: torch.empty(*size, device=f"cuda:{dev}"))
+
+
+@pytest.mark.parametrize("dU, fc, out", [((2, 6, 5, 4), (4, 3), None), ((2, 6, 5, 5), (5, 3), None),
+                                         ((2, 6, 5, 5), (4, 2), None), ((2, 6, 5, 5), (4, 3), [(2, 6, 5, 4), (2, 4, 5, 5), (48,)]),
+                                         ((2, 6, 5, 5), (4, 3), [(2, 6, 5, 5), (2, 4, 5, 5), (47,)])])
+def test_host_buffers_that_do_not_fit_are_value_errors(lib_built, dU, fc, out):
+    import paralleltnnlayers_b200 as P
+    args = (Z(2, 4, 5, 5), Z(*dU), Z(6, 3), Z(*fc), Z(3, 3), Z(3, 3))
+    out = out and [Z(*size) for size in out]
+    with pytest.raises(ValueError):
+        P.cp4_conv2d_step_host(*args, out=out)
+    with pytest.raises(ValueError):
+        P.cp4_conv2d_step_host_submit(*args, out=out or [Z(2, 6, 5, 5), Z(2, 4, 5, 5), Z(48)])
 
 
 @pytest.mark.gpu
