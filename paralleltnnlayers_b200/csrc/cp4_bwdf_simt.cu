@@ -381,7 +381,7 @@ __device__ __forceinline__ float exchange_gather(const ExchangeArgs& ex, bool li
 // In pipelined mode (ex.mode == 1) the kernel only posts its sums and completes the *previous* step's exchange, whose
 // flags have long arrived: the exchange latency then costs the step nothing.
 template <bool EXCHANGE>
-__global__ void __launch_bounds__(1024) cp4_reduce_partials_kernel(const float* __restrict__ partial, int nparts_high,
+__global__ void __launch_bounds__(1024) cp4_reduce_partials_kernel(const float* partial, int nparts_high,
                                                                    int nparam, int R, int Rs, int r0,
                                                                    float* __restrict__ dK, const ExchangeArgs ex,
                                                                    int split, int nparts_low) {
@@ -393,11 +393,12 @@ __global__ void __launch_bounds__(1024) cp4_reduce_partials_kernel(const float* 
   const int i0 = sl * per, i1 = min(nparts, i0 + per);
   float s0 = 0.f;
   if (j < nparam) {
-    // eight loads in flight, then added in index order
+    // eight loads in flight, then added in index order (ordinary loads, and no __restrict__: the kernel before still
+    // writes the partials when this grid starts, which the read-only path does not allow)
     for (int i = i0; i < i1; i += 8) {
       float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = i + u < i1 ? __ldg(partial + (size_t)(i + u) * nparam + j) : 0.f;
+      for (int u = 0; u < 8; ++u) v[u] = i + u < i1 ? partial[(size_t)(i + u) * nparam + j] : 0.f;
 #pragma unroll
       for (int u = 0; u < 8; ++u) s0 += v[u];
     }

@@ -230,14 +230,16 @@ struct PlaneStencil {
   int R, H, W, HB, units, per;   // HB = row groups of four per image, units = N * HB * W
 };
 
+// Ordinary loads: this grid starts while the one that writes the planes still runs, and the read-only path (__ldg) is for
+// memory that nothing writes during the kernel's life.
 __device__ __forceinline__ void load_window(const float* s, int h, int w, int H, int W, float (&v)[6][3]) {
 #pragma unroll
   for (int y = 0; y < 6; ++y) {
     const bool row = (unsigned)(h + y - 1) < (unsigned)H;
     const float* t = s + (y - 1) * W;
-    v[y][0] = row && w > 0 ? __ldg(t - 1) : 0.f;
-    v[y][1] = row ? __ldg(t) : 0.f;
-    v[y][2] = row && w + 1 < W ? __ldg(t + 1) : 0.f;
+    v[y][0] = row && w > 0 ? t[-1] : 0.f;
+    v[y][1] = row ? t[0] : 0.f;
+    v[y][2] = row && w + 1 < W ? t[1] : 0.f;
   }
 }
 __device__ __forceinline__ void stencil_store(const float (&v)[6][3], const float (&w)[9], float* d, int h, int H, int W) {
