@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const 
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x;
   const int kg = tid / (kGT / T::KG), gt = tid - kg * (kGT / T::KG), tx = gt % TXN, ty = gt / TXN;
-  const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * BM;
+  const int ntiles = (N + kBN - 1) / kBN, mt = blockIdx.x / ntiles;   // column tiles first: they share the rows of X
+  const int n0 = (blockIdx.x - mt * ntiles) * kBN, m0 = mt * BM;
   const int kb = blockIdx.z * kper, ke = min(K, kb + kper);
   const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
   float acc[4][4];
@@ -502,8 +503,8 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
   const long tiles = (long)ceil_div(M, bm) * ceil_div(N, bn);
   const int splits = pick_cluster(tiles, K, 64, di.sm_count);
   const int kper = (int)align_up((size_t)ceil_div(K, splits), 4);
-  dim3 grid(ceil_div(N, bn), ceil_div(M, bm), splits);
-  if (grid.y > 65535) return fail(B200CP_ERR_UNSUPPORTED, "dense: batch too large for the small product kernel");
+  if (tiles > 0x7fffffffL || M > 0x7fffffff - 64) return fail(B200CP_ERR_UNSUPPORTED, "dense: batch of %d rows too large", M);
+  const dim3 grid((unsigned)tiles, 1, splits);   // (grid y would end at 65535 row tiles)
 #define SMALL_GEMM(BMV, BNV, V)                                                                                       \
   do {                                                                                                                \
     static std::atomic<int> set[64];                                                                                  \

@@ -27,6 +27,19 @@ def test_dense_forward_and_data_gradient(case):
     check(P.dense_cp_backward(x, dy, *f, need_dw=False)[0], rX, "dense dX", atol=1e-5 * max(1.0, float(np.abs(rX).max())))
 
 
+def test_more_row_tiles_than_a_grid_dimension():
+    """65536 row tiles of 64: the batch of a wide but shallow input."""
+    import torch
+    import paralleltnnlayers_b200 as P
+    B, R = 65535 * 64 + 1, 64
+    x = torch.empty(B, 4, device="cuda").uniform_(-1, 1)
+    F = [torch.randn(2, 2, R, device="cuda") * 0.35 for _ in range(2)]
+    M = torch.einsum("aoR,bpR->abop", *[f.double() for f in F]).reshape(4, 4)
+    for got, ref in ((P.dense_cp(x, *F), x.double() @ M), (P.dense_cp_backward(x, x, *F, need_dw=False)[0], x.double() @ M.T)):
+        # sums of 64 then 4 products: (64 + 4) ulp of the terms' size, far below this
+        assert float((got.double() - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
+
+
 RCP = [  # N, cdims, tdims, H, W, R: channel tiles of 16 / 32 / 64, pixel tiles of 256 / 128 / 64, channels split over a cluster
     (1, (3,), (5,), 1, 1, 2), (2, (4, 4), (4, 4), 32, 32, 11), (1, (2, 9), (3, 11), 7, 33, 5), (3, (5, 5), (6, 6), 9, 5, 33),
     (1, (16, 16), (5, 13), 7, 7, 4), (1, (16, 16), (16, 16), 8, 30, 16), (2, (2, 3, 4), (3, 3, 8), 13, 40, 7),
