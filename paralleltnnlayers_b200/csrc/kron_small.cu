@@ -19,6 +19,32 @@
 namespace b200cp {
 namespace {
 
+// The products add up to thousands of terms per result.  One accumulator over all of them rounds like sqrt(terms): relative
+// to float64 8e-7 for 4096 inputs, where the factored form, whose longest chain is ranks x one mode, has 2e-7 (R = 8).  So
+// an accumulator holds about kChain terms and is then added to a total: 1.8e-7 for the same sums.  The totals are in shared
+// memory, [4][threads] float4, and cost 5 % (4096 samples of 4096 -> 4096: 3.68 to 3.88 ms; 16 more registers instead would leave one CTA of 512
+// threads per SM instead of two: 4.73 ms).  A chain of at most kChain terms has none.
+constexpr int kChain = 64;
+template <int NT>
+__device__ __forceinline__ void flush_sums(float (&acc)[4][4], float* total, int tid, bool first) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float4* t = reinterpret_cast<float4*>(total) + i * NT + tid;
+    float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
+    v.x += acc[i][0]; v.y += acc[i][1]; v.z += acc[i][2]; v.w += acc[i][3];
+    *t = v;
+    acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  }
+}
+template <int NT>
+__device__ __forceinline__ void add_totals(float (&acc)[4][4], const float* total, int tid) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(total)[i * NT + tid];
+    acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
+  }
+}
+
 // ---- the weight ----------------------------------------------------------------------------------------------------------
 // The modes are cut into two halves, A (first modes, slow) and B (last modes): with the half products
 // A[a][r] = prod_{k in A} F_k and B[b][r] the weight is the matrix product A B^T over r.  A CTA forms a TA x 64 tile of
@@ -190,7 +216,9 @@ struct GemmTile {
   static constexpr int BK = KG > 2 ? 64 : 32;         // K rows of a stage
   static constexpr int PA = BK + 4;
   static constexpr int stage = BM * PA + BK * (BN + 4);
-  static constexpr size_t smem = sizeof(float) * (size_t)(kGStages * stage > KG * BM * BN ? kGStages * stage : KG * BM * BN);
+  static constexpr int flush = kChain / (BK / KG);    // stages of an accumulator
+  static constexpr int buf = kGStages * stage > KG * BM * BN ? kGStages * stage : KG * BM * BN;
+  static size_t smem(int kper) { return sizeof(float) * ((size_t)buf + ((kper + BK - 1) / BK > flush ? 16 * NT : 0)); }
 };
 
 template <int BM, int BN, bool VECA>
@@ -273,7 +301,9 @@ __global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const 
         }
       }
     }
+    if (s % T::flush == T::flush - 1 && s + 1 < steps) flush_sums<kGT>(acc, smem + T::buf, tid, s + 1 == T::flush);
   }
+  if (steps > T::flush) add_totals<kGT>(acc, smem + T::buf, tid);
   mma::cp_async_wait<0>();
   // the groups' partial results, then the sum over groups, then over the cluster
   __syncthreads();
@@ -301,10 +331,13 @@ __global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const 
 // are worked out once.  The CTAs of a cluster split the input channels.
 constexpr int kCC = 8, kHaloPer = 2, kCT = 512;   // channels per stage, halo positions per thread, threads
 
+constexpr int conv_flush(int groups) { return (kChain + 9 * kCC / groups / 2) / (9 * kCC / groups); }   // stages of an accumulator
+
 struct SmallConvGeom {
   int C, T, H, W, ldw, cper, splits;
   int TR, TC, tilesW, tiles, PXQ;   // tile rows / columns (a multiple of 4), pixel quads in use
   int P, CS;                        // halo row pitch, halo floats per channel
+  int buf;                          // floats of the stages (and the sum over the groups); the totals follow
 };
 
 template <int TT, int CG>
@@ -358,6 +391,8 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  constexpr int kFlush = conv_flush(CG);
+  float* total = smem + g.buf;
   const bool active = pq < g.PXQ;
   const int pr = active ? pq / (g.TC / 4) : 0, pc = active ? (pq - pr * (g.TC / 4)) * 4 : 0;
   const int steps = ce > cb ? (ce - cb + kCC - 1) / kCC : 0;
@@ -398,8 +433,10 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
         }
       }
     }
+    if (s % kFlush == kFlush - 1 && s + 1 < steps) flush_sums<kCT>(acc, total, tid, s + 1 == kFlush);
     __syncthreads();
   }
+  if (steps > kFlush) add_totals<kCT>(acc, total, tid);
   float* Vn = V + (size_t)n * g.T * HW;
   const int npx = g.TR * g.TC;
   // the channel groups, then the cluster, are added in shared memory over the stage buffers: [group][t][px] (every
@@ -508,7 +545,7 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
 #define SMALL_GEMM(BMV, BNV, V)                                                                                       \
   do {                                                                                                                \
     static std::atomic<int> set[64];                                                                                  \
-    const size_t smem = spread_smem(GemmTile<BMV, BNV>::smem, tiles * splits, di);                                    \
+    const size_t smem = spread_smem(GemmTile<BMV, BNV>::smem(kper), tiles * splits, di);                                    \
     B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(small_gemm_kernel<BMV, BNV, V>), set, di.smem_optin)); \
     B200CP_CUDA_OK(launch_cluster(small_gemm_kernel<BMV, BNV, V>, grid, dim3(GemmTile<BMV, BNV>::NT), smem, st, splits, true, \
                                   X, W, Y, M, N, K, ldw, kper, splits));                                              \
@@ -552,7 +589,8 @@ int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const f
   const long tiles = (long)N * g.tiles * ceil_div(T, tt);
   g.splits = pick_cluster(tiles, C, 2 * kCC, di.sm_count);
   g.cper = (int)align_up((size_t)ceil_div(C, g.splits), kCC);
-  const size_t smem = sizeof(float) * std::max<size_t>(2 * ((size_t)kCC * g.CS + kCC * 9 * tt), (size_t)cgroups * tt * g.TR * g.TC);
+  g.buf = std::max(2 * (kCC * g.CS + kCC * 9 * tt), cgroups * tt * g.TR * g.TC);
+  const size_t smem = sizeof(float) * ((size_t)g.buf + (ceil_div(g.cper, kCC) > conv_flush(cgroups) ? 16 * kCT : 0));
   dim3 grid((unsigned)(N * g.tiles), ceil_div(T, tt), g.splits);
   if ((long)N * g.tiles > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");
 #define SMALL_CONV(TTV, CGV)                                                                                              \

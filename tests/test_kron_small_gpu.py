@@ -57,3 +57,21 @@ def test_rcp_forward_and_data_gradient(case):
     check(P.conv2d_rcp_fused_nchw(x, *a, s), ref, "rcp forward", atol=1e-5 * max(1.0, float(np.abs(ref).max())))
     rX = O.rcp_backward(X, dV, A, S)[0]
     check(P.rcp_conv2d_backward(x, dv, *a, s, need_dw=False)[0], rX, "rcp dX", atol=1e-5 * max(1.0, float(np.abs(rX).max())))
+
+
+def test_rounding_of_long_sums():
+    """4096 inputs and 256 channels x 9 taps, not split over CTAs.  A chain of n fp32 additions of random signs is off by about
+    2**-24 * sqrt(n / 6) of its result: 1.9e-7 for the 64 to 72 terms of an accumulator, 1.4e-7 for the at most 32 totals,
+    1e-7 to 2e-7 for the weight's sum over the ranks; one chain over all terms would be at 8e-7 and 6e-7."""
+    import torch
+    import paralleltnnlayers_b200 as P
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    normal = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    rel = lambda got, ref: float((got.double() - ref).norm() / ref.norm())
+    x, F = normal(256, 4096), [normal(16, 16, 64) * 0.35 for _ in range(3)]
+    M = torch.einsum("aor,bpr,cqr->abcopq", *[f.double() for f in F]).reshape(4096, 4096)
+    assert rel(P.dense_cp(x, *F), x.double() @ M) < 4e-7
+    x, A, S = normal(32, 256, 28, 28), [normal(16, 16, 16) * 0.3 for _ in range(2)], normal(3, 3, 16) * 0.3
+    K = torch.einsum("aor,bpr,yxr->opabyx", *[f.double() for f in (*A, S)]).reshape(256, 256, 3, 3)
+    ref = torch.nn.functional.conv2d(x[:2].double(), K, padding=1)
+    assert rel(P.conv2d_rcp_fused_nchw(x, *A, S)[:2], ref) < 4e-7
