@@ -186,7 +186,7 @@ int b200cp_cp3_bwd_filter(const b200cp_tensor_shape* s, const float* X, const fl
                           const float* KCin, const float* KC, float* dK_packed, void* workspace,
                           size_t workspace_bytes, void* stream, int flags);
 /* With a workspace, as for CP4.  The rank plane P can be kept by the forward, and the backward run from it, for the
- * shapes for which b200cp_cp3_shares_planes says so. */
+ * shapes for which b200cp_cp3_shares_planes says so; with dX NULL that backward forms the factor gradients only. */
 int b200cp_cp3_shares_planes(const b200cp_tensor_shape* s, int flags);
 size_t b200cp_cp3_fwd_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags);
 int b200cp_cp3_fwd_ws(const b200cp_tensor_shape* s, const float* X, const float* KT, const float* KCin, const float* KC,

@@ -444,7 +444,7 @@ int b200cp_cp3_bwd_saved(const b200cp_tensor_shape* s, const float* X, const flo
                          const float* KCin, const float* KC, float* dX, float* dK_packed, void* workspace,
                          size_t workspace_bytes, void* stream, int flags) {
   if (int rc = check_shape(s, "b200cp_cp3_bwd_saved")) return rc;
-  if (int rc = check_ptrs("b200cp_cp3_bwd_saved", {X, dU, P, KT, KCin, KC, dX, dK_packed})) return rc;
+  if (int rc = check_ptrs("b200cp_cp3_bwd_saved", {X, dU, P, KT, KCin, KC, dK_packed})) return rc;
   if (!takes_planes(s, flags, Planes::kBackward3))
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp3_bwd_saved: for shapes of b200cp_cp3_shares_planes only");
   PlanesJob j;

@@ -245,19 +245,19 @@ std::array<Tensor, 3> split3(const Tensor& dK, const b200cp_tensor_shape& s) {
           dK.narrow(0, nT + nC, nS).view({s.Y, s.X, R})};
 }
 
-// dX and the factor gradients from the forward's rank plane
+// dX (where it is wanted) and the factor gradients from the forward's rank plane
 Tensor cp3_backward_saved(const Tensor& dU, const Tensor& In, const Tensor& P_, const Tensor& KT, const Tensor& KCin,
-                          const Tensor& KC, int64_t pad, int flags, std::array<Tensor, 3>* grads) {
+                          const Tensor& KC, int64_t pad, int flags, bool need_dx, std::array<Tensor, 3>* grads) {
   const Conv3 c(dU, "Upstream", KT, KCin, KC, pad, true);
   const b200cp_tensor_shape& s = c.s;
   const Tensor P = dev(P_, "P", c.in), X = dev(In, "In", c.in);
   check_size(P, "P", {s.N, s.Rank, s.H, s.W});
   check_size(X, "In", {s.N, s.C, s.H, s.W});
   const c10::cuda::OptionalCUDAGuard guard(c.in.device());
-  Tensor dX = empty({s.N, s.C, s.H, s.W}, c.in);
+  Tensor dX = need_dx ? empty({s.N, s.C, s.H, s.W}, c.in) : Tensor();
   Tensor dK = empty({(int64_t)(s.T + s.C + s.Y * s.X) * s.Rank}, c.in);
   const Scratch ws(b200cp_cp3_bwd_saved_workspace_bytes(&s, flags), c.in);
-  ok(b200cp_cp3_bwd_saved(&s, cp(X), cp(c.in), cp(P), cp(c.KT), cp(c.KC_in), cp(c.KC), mp(dX), mp(dK), ws.ptr, ws.bytes,
+  ok(b200cp_cp3_bwd_saved(&s, cp(X), cp(c.in), cp(P), cp(c.KT), cp(c.KC_in), cp(c.KC), need_dx ? mp(dX) : nullptr, mp(dK), ws.ptr, ws.bytes,
                           stream(c.in), flags));
   *grads = split3(dK, s);
   return dX;
@@ -477,15 +477,15 @@ struct CP3Node : torch::autograd::Function<CP3Node> {
     const int64_t pad = ctx->saved_data["pad"].toInt();
     const Tensor dy = grads[0].contiguous();
     variable_list out(5);
-    if (v.size() == 5) {
+    const bool need_dw = ctx->needs_input_grad(1) || ctx->needs_input_grad(2) || ctx->needs_input_grad(3);
+    if (v.size() == 5 && need_dw) {
       std::array<Tensor, 3> g;
-      Tensor dx = cp3_backward_saved(dy, v[0], v[4], v[1], v[2], v[3], pad, 0, &g);
-      if (ctx->needs_input_grad(0)) out[0] = dx;
+      out[0] = cp3_backward_saved(dy, v[0], v[4], v[1], v[2], v[3], pad, 0, ctx->needs_input_grad(0), &g);
       for (int i = 0; i < 3; ++i) out[1 + i] = g[i];
       return out;
     }
     if (ctx->needs_input_grad(0)) out[0] = cp3_backward_data(dy, v[1], v[2], v[3], pad, 0);
-    if (ctx->needs_input_grad(1) || ctx->needs_input_grad(2) || ctx->needs_input_grad(3)) {
+    if (need_dw) {
       const std::array<Tensor, 3> g = cp3_backward_filter(dy, v[0], v[1], v[2], v[3], pad, 0);
       for (int i = 0; i < 3; ++i) out[1 + i] = g[i];
     }

@@ -138,3 +138,33 @@ def test_back_to_back_calls_on_new_inputs(shape):
         for got, want in zip([P.cp4_conv2d_step(*s) for s in sets], alone):
             for a, b in zip(got, want):
                 assert torch.equal(a, b)
+
+
+def test_cp3_backward_forms_what_is_asked_for():
+    """A layer whose input needs no gradient forms the factor gradients only, one product (launch) less; one asked for the
+    input's gradient alone runs the data gradient's launches and no others."""
+    import paralleltnnlayers_b200 as P
+    from paralleltnnlayers_b200._lib import lib
+    X, dU, K = make((3, 70, 65, 9, 9, 40), True)
+    want = expect(X, dU, K)
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda().requires_grad_() for f in K]
+
+    def launched(run):
+        before = lib.b200cp_launch_count()
+        out = run()
+        return lib.b200cp_launch_count() - before, out
+
+    def backward(x, *leaves):
+        y = P.CP3Conv2dFunction.apply(x, *k)
+        return launched(lambda: torch.autograd.grad(y, leaves, du))
+
+    xr = x.clone().requires_grad_()
+    n_all, g_all = backward(xr, xr, *k)
+    n_factors, g_factors = backward(x, *k)
+    n_data, g_data = backward(xr, xr)
+    for grads, refs in ((g_all, want[1:]), (g_factors, want[2:]), (g_data, want[1:2])):
+        for got, ref in zip(grads, refs):
+            assert_parity(got, ref)
+    assert n_factors == n_all - 1
+    with torch.no_grad():
+        assert n_data == launched(lambda: P.cp3_conv2d_backward_data(du, *k))[0]
