@@ -408,14 +408,16 @@ FactorGrads dense_backward(const Tensor& U_, const Tensor& dV_, at::TensorList F
 }
 
 // ---- autograd nodes -------------------------------------------------------------------------------------------------------
+// `grad`: gradients are recorded where the node is applied (inside a forward the mode is always off; the factors of a
+// module require a gradient under no_grad too, where a rank plane would be written and dropped)
 struct CP4Node : torch::autograd::Function<CP4Node> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& FT, const Tensor& FC, const Tensor& FY,
-                        const Tensor& FX, int64_t pad, int64_t flags) {
+                        const Tensor& FX, int64_t pad, int64_t flags, bool grad) {
     ctx->saved_data["pad"] = pad;
     ctx->saved_data["flags"] = flags;
     // with 3x3 filters the forward keeps its rank plane for the factor gradients (a quarter of x at C = 4R)
     bool shared = false;
-    if ((FT.requires_grad() || FC.requires_grad() || FY.requires_grad() || FX.requires_grad()) && x.dim() == 4) {
+    if (grad && (FT.requires_grad() || FC.requires_grad() || FY.requires_grad() || FX.requires_grad()) && x.dim() == 4) {
       const Conv c(x, "Input", FT, FC, FY, FX, pad, false);
       shared = b200cp_cp4_shares_planes(&c.s, (int)flags) != 0;
     }
@@ -435,7 +437,7 @@ struct CP4Node : torch::autograd::Function<CP4Node> {
     const Tensor dy = grads[0].contiguous();
     const Tensor &x = v[0], &FT = v[1], &FC = v[2], &FY = v[3], &FX = v[4];
     b200cp_tensor_shape s;
-    variable_list out(7);
+    variable_list out(8);
     if (v.size() == 6) {
       Tensor dK;
       Tensor dx = cp4_backward_saved(dy, x, v[5], FT, FC, FY, FX, pad, flags, &dK, &s);
@@ -455,11 +457,11 @@ struct CP4Node : torch::autograd::Function<CP4Node> {
 
 struct CP3Node : torch::autograd::Function<CP3Node> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& KT, const Tensor& KCin, const Tensor& KC,
-                        int64_t pad) {
+                        int64_t pad, bool grad) {
     ctx->saved_data["pad"] = pad;
     // where the gradients are formed from whole rank planes the forward keeps its own
     bool shared = false;
-    if ((KT.requires_grad() || KCin.requires_grad() || KC.requires_grad()) && x.dim() == 4) {
+    if (grad && (KT.requires_grad() || KCin.requires_grad() || KC.requires_grad()) && x.dim() == 4) {
       const Conv3 c(x, "Input", KT, KCin, KC, pad, false);
       shared = b200cp_cp3_shares_planes(&c.s, 0) != 0;
     }
@@ -476,7 +478,7 @@ struct CP3Node : torch::autograd::Function<CP3Node> {
     const variable_list v = ctx->get_saved_variables();
     const int64_t pad = ctx->saved_data["pad"].toInt();
     const Tensor dy = grads[0].contiguous();
-    variable_list out(5);
+    variable_list out(6);
     const bool need_dw = ctx->needs_input_grad(1) || ctx->needs_input_grad(2) || ctx->needs_input_grad(3);
     if (v.size() == 5 && need_dw) {
       std::array<Tensor, 3> g;
@@ -786,7 +788,7 @@ PYFN(py_cp4_apply) {
   const Tensor &x = tensor_arg(a[0], "Input"), &ft = tensor_arg(a[1], "FT"), &fc = tensor_arg(a[2], "FC"),
                &fy = tensor_arg(a[3], "FY"), &fx = tensor_arg(a[4], "FX");
   const int64_t pad = n > 5 ? int_arg(a[5]) : 1, flags = n > 6 ? int_arg(a[6]) : 0;
-  return wrap(unlocked([&] { return CP4Node::apply(x, ft, fc, fy, fx, pad, flags); }));
+  return wrap(unlocked([&] { return CP4Node::apply(x, ft, fc, fy, fx, pad, flags, at::GradMode::is_enabled()); }));
   END_HANDLE_TH_ERRORS
 }
 PYFN(py_cp3_apply) {
@@ -795,7 +797,7 @@ PYFN(py_cp3_apply) {
   const Tensor &x = tensor_arg(a[0], "Input"), &kt = tensor_arg(a[1], "KT"), &kcin = tensor_arg(a[2], "KCin"),
                &kc = tensor_arg(a[3], "KC");
   const int64_t pad = n > 4 ? int_arg(a[4]) : 1;
-  return wrap(unlocked([&] { return CP3Node::apply(x, kt, kcin, kc, pad); }));
+  return wrap(unlocked([&] { return CP3Node::apply(x, kt, kcin, kc, pad, at::GradMode::is_enabled()); }));
   END_HANDLE_TH_ERRORS
 }
 PYFN(py_rcp_apply) {

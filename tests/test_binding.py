@@ -125,3 +125,30 @@ print("ok")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", ["CP4Conv2d", "CPConv2d"])
+def test_inference_of_a_module_keeps_no_plane(make):
+    """Under no_grad the factors of a module still require a gradient: its forward is the plain operator's, with the
+    output as the only allocation, and the same bits."""
+    import paralleltnnlayers_b200 as P
+    from paralleltnnlayers_b200 import layers
+    layer = getattr(layers, make)(512, 512, rank=8).cuda()
+    x = torch.randn(2, 512, 50, 50, device="cuda")
+    op = P.cp4_conv2d_forward if make == "CP4Conv2d" else P.cp3_conv2d_forward
+
+    def allocations(run):
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        return run(), torch.cuda.memory_stats()["allocation.all.allocated"] - before
+
+    with torch.no_grad():
+        allocations(lambda: layer(x))
+        y, n = allocations(lambda: layer(x))
+        want, n_op = allocations(lambda: op(x, *layer.parameters()))
+    assert n == n_op == 1 and torch.equal(y, want)
+    y, n = allocations(lambda: layer(x))
+    assert n == 2 and y.requires_grad     # with gradients the plane is kept
+    with torch.inference_mode():
+        assert allocations(lambda: layer(x))[1] == 1
