@@ -14,6 +14,7 @@
 // the stencil flipped).  Formulas: Kernels/rcp_fused_nchw.cu:4-77 and
 // Kernels/dense_cp.cu:4-46 (fixed shapes there), test/layers.py:445-465,716-773.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -309,11 +310,111 @@ int max_items(const ChainGeom& g) {
   return (ok <= 4 ? 8 : ok <= 8 ? 4 : 2) * kNT;
 }
 
+long chain_ctas(const ChainGeom& g) {
+  return g.conv ? (long)g.N * g.tilesH * g.tilesW : (g.B + (long)g.PIX - 1) / g.PIX;
+}
+
+// Columns per CTA of the dense layer (g.B given); false: the layer does not fit on chip.
+bool dense_tile(ChainGeom& g, const DeviceInfo& di) {
+  const int Alast = g.Cout / g.dout[g.m - 1];
+  for (int cand = 16; cand >= 4; cand -= 4) {
+    g.PIX = cand;
+    if ((long)Alast * (cand / 4) > max_items(g)) continue;
+    if ((int)chain_smem(g) > di.smem_optin) continue;
+    // keep at least ~2 waves of tiles when the batch allows it
+    if (cand > 4 && (long)ceil_div(g.B, cand) < 2L * di.sm_count) continue;
+    return true;
+  }
+  return false;
+}
+
+// Tile of the convolution (g.N .. g.FW given): the best (halo efficiency x padding efficiency x wave efficiency).
+bool rcp_tile(ChainGeom& g, const DeviceInfo& di) {
+  const int H = g.H, W = g.W;
+  g.conv = 1;
+  g.mH = (g.FH - 1) / 2; g.mW = (g.FW - 1) / 2;  // "same" padding per axis (test/test_conv2d_rcp.py:11)
+  g.pad = g.mH;
+  g.bufElems = std::max(g.bufElems, g.Cin);  // the stencil output [Cin][PIX] also lives in a buffer
+  const int Alast = g.Cout / g.dout[g.m - 1];
+  const auto set = [](ChainGeom& t, int TH, int TW) {
+    t.TH = TH; t.TW = TW; t.PIX = (int)align_up((size_t)TH * TW, 4); t.TWh = TW + 2 * t.mW;
+    t.HPX = (TH + 2 * t.mH) * t.TWh; t.HPXs = (int)align_up(t.HPX, 4);
+  };
+  double best = 0;
+  int bestTH = 0, bestTW = 0;
+  const int tws[4] = {W, 64, 32, 16};
+  for (int ti = 0; ti < 4; ++ti) {
+    const int TW = tws[ti];
+    if (TW > W || (ti == 0 && W > 64) || (ti > 0 && TW >= W)) continue;
+    for (int TH = 1; TH <= std::min(H, 32); ++TH) {
+      ChainGeom t = g;
+      set(t, TH, TW);
+      if ((long)Alast * (t.PIX / 4) > max_items(g)) break;
+      const size_t sm = chain_smem(t);
+      if ((int)sm > di.smem_optin) break;
+      const long ctas = (long)g.N * ceil_div(H, TH) * ceil_div(W, TW);
+      const long slots = (long)di.sm_count * std::max<long>(1, (228 * 1024) / (long)(sm + 1024));
+      const double wave_eff = (double)ctas / (double)(ceil_div((int)ctas, (int)slots) * slots);
+      const double cover = (double)H * W / ((double)ceil_div(H, TH) * TH * ceil_div(W, TW) * TW);
+      const double score = cover * ((double)TH * TW / t.HPX + 1.0) * ((double)TH * TW / t.PIX) * (0.5 + 0.5 * wave_eff);
+      if (score > best) { best = score; bestTH = TH; bestTW = TW; }
+    }
+  }
+  if (!bestTH) return false;
+  set(g, bestTH, bestTW);
+  g.tilesH = ceil_div(H, g.TH); g.tilesW = ceil_div(W, g.TW);
+  return true;
+}
+
+// Estimated microseconds.  The kernel's registers allow one CTA per SM, so it runs in waves of one CTA per SM, each R times
+// (barriers, factors, mode steps); a mode step costs the larger part of its latency per pass over the items and of the work,
+// both per contracted index.  Least-squares fit (of the relative error) to 1202 layers of 1-4 modes of 1-16, up to 8192
+// channels, batches to 8192 and images to 64 x 64, at ranks 1-300: 0.91-1.06 of the measured time for eight of ten.
+constexpr double kChainRank = 0.134, kChainMode = 0.4745;
+double chain_us(const ChainGeom& g, const DeviceInfo& di) {
+  double rank = kChainRank + kChainMode * g.m, A = 1, Bn = (double)g.Cin * g.PIX;
+  for (int k = 0; k < g.m; ++k) {
+    Bn /= g.din[k];
+    const double items = A * Bn / 4;
+    const int w = g.dout[k] <= 4 ? 0 : g.dout[k] <= 8 ? 1 : 2;
+    constexpr double kPass[3] = {0.0127, 0.0249, 0.0656}, kWork[3] = {0.0473, 0.0529, 0.0604};
+    rank += g.din[k] * (kPass[w] * std::ceil(items / kNT) + kWork[w] * items / kNT);
+    A *= g.dout[k];
+  }
+  if (g.conv) rank += 0.565 * std::ceil((double)g.Cin * g.PIX / kNT);
+  const double waves = std::ceil((double)chain_ctas(g) / di.sm_count);
+  const double io = ((double)g.Cin * (g.conv ? g.HPXs : g.PIX) + (double)g.Cout * g.PIX) / kNT;
+  return 1.0 + waves * (2.44 + 0.0884 * io + g.R * rank);
+}
+// what no rank of any size stays below
+double chain_least_us(const ChainGeom& g) { return 3.4 + g.R * (kChainRank + kChainMode * g.m); }
+
 }  // namespace
 
 int check_kron_modes(int order, const int* idims, const int* odims, int R, const char* who) {
   ChainGeom g{};
   return fill_modes(g, order, idims, odims, R, false, who);
+}
+
+double rcp_factored_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
+                       bool transposed, double enough) {
+  DeviceInfo di;
+  ChainGeom g{};
+  if (device_info(&di) || fill_modes(g, order, cdims, tdims, R, transposed, "rcp")) return -1;
+  if (rcp_fast_takes(order, g.din, g.dout, R, FH, FW, N, H, W, di)) return rcp_fast_us(N, H, W, R, di);
+  if (chain_least_us(g) > enough) return chain_least_us(g);
+  g.N = N; g.H = H; g.W = W; g.FH = FH; g.FW = FW;
+  return rcp_tile(g, di) ? chain_us(g, di) : -1;
+}
+
+double dense_factored_us(int B, int order, const int* idims, const int* odims, int R, bool transposed, double enough) {
+  DeviceInfo di;
+  ChainGeom g{};
+  if (device_info(&di) || fill_modes(g, order, idims, odims, R, transposed, "dense_cp")) return -1;
+  if (dense_fast_takes(order, g.din, g.dout, R, di)) return dense_fast_us(B, R, di);
+  if (chain_least_us(g) > enough) return chain_least_us(g);
+  g.B = B;
+  return dense_tile(g, di) ? chain_us(g, di) : -1;
 }
 
 int rcp_chain_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -326,47 +427,14 @@ int rcp_chain_launch(int N, int H, int W, int order, const int* cdims, const int
   if (FH < 1 || FW < 1 || FH > 31 || FW > 31 || !(FH & 1) || !(FW & 1))
     return fail(B200CP_ERR_UNSUPPORTED, "rcp: filter %dx%d must be odd and at most 31", FH, FW);
   if (N < 1 || H < 1 || W < 1) return fail(B200CP_ERR_INVALID_ARG, "rcp: non-positive N/H/W");
-  {
-    bool done = false;
-    if (int rc = rcp_fast_launch(N, H, W, order, g.din, g.dout, g.fsi, g.fso, R, FH, FW, X, A, S, V, transposed, st, &done))
-      return rc;
-    if (done) return B200CP_OK;
-  }
-  g.conv = 1; g.N = N; g.H = H; g.W = W; g.FH = FH; g.FW = FW; g.flip = transposed ? 1 : 0;
-  g.mH = (FH - 1) / 2; g.mW = (FW - 1) / 2;  // "same" padding per axis (test/test_conv2d_rcp.py:11)
-  g.pad = g.mH;
-  g.bufElems = std::max(g.bufElems, g.Cin);  // the stencil output [Cin][PIX] also lives in a buffer
-  const int Alast = g.Cout / g.dout[g.m - 1];
-  // pick the tile with the best (halo efficiency x padding efficiency x wave efficiency)
-  double best = 0;
-  int bestTH = 0, bestTW = 0;
-  const int tws[4] = {W, 64, 32, 16};
-  for (int ti = 0; ti < 4; ++ti) {
-    const int TW = tws[ti];
-    if (TW > W || (ti == 0 && W > 64) || (ti > 0 && TW >= W)) continue;
-    for (int TH = 1; TH <= std::min(H, 32); ++TH) {
-      ChainGeom t = g;
-      t.TH = TH; t.TW = TW; t.PIX = (int)align_up((size_t)TH * TW, 4); t.TWh = TW + 2 * g.mW;
-      t.HPX = (TH + 2 * g.mH) * t.TWh; t.HPXs = (int)align_up(t.HPX, 4);
-      if ((long)Alast * (t.PIX / 4) > max_items(g)) break;
-      const size_t sm = chain_smem(t);
-      if ((int)sm > di.smem_optin) break;
-      const long ctas = (long)N * ceil_div(H, TH) * ceil_div(W, TW);
-      const long slots = (long)di.sm_count * std::max<long>(1, (228 * 1024) / (long)(sm + 1024));
-      const double wave_eff = (double)ctas / (double)(ceil_div((int)ctas, (int)slots) * slots);
-      const double cover = (double)H * W / ((double)ceil_div(H, TH) * TH * ceil_div(W, TW) * TW);
-      const double score = cover * ((double)TH * TW / t.HPX + 1.0) * ((double)TH * TW / t.PIX) * (0.5 + 0.5 * wave_eff);
-      if (score > best) { best = score; bestTH = TH; bestTW = TW; }
-    }
-  }
-  if (!bestTH) return fail(B200CP_ERR_UNSUPPORTED, "rcp: no tile fits (channels %d -> %d)", g.Cin, g.Cout);
-  g.TH = bestTH; g.TW = bestTW; g.PIX = (int)align_up((size_t)bestTH * bestTW, 4);
-  g.TWh = g.TW + 2 * g.mW; g.HPX = (g.TH + 2 * g.mH) * g.TWh; g.HPXs = (int)align_up(g.HPX, 4);
-  g.tilesH = ceil_div(H, g.TH); g.tilesW = ceil_div(W, g.TW);
+  if (rcp_fast_takes(order, g.din, g.dout, R, FH, FW, N, H, W, di))
+    return rcp_fast_launch(N, H, W, g.fsi, g.fso, R, X, A, S, V, transposed, di, st);
+  g.N = N; g.H = H; g.W = W; g.FH = FH; g.FW = FW; g.flip = transposed ? 1 : 0;
+  if (!rcp_tile(g, di)) return fail(B200CP_ERR_UNSUPPORTED, "rcp: no tile fits (channels %d -> %d)", g.Cin, g.Cout);
   ChainPtrs p{};
   p.X = X; p.S = S; p.Y = V;
   for (int k = 0; k < order; ++k) p.F[k] = A[k];
-  const long ctas = (long)N * g.tilesH * g.tilesW;
+  const long ctas = chain_ctas(g);
   if (ctas > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");
   return dispatch_chain(g, p, ctas, st);
 }
@@ -378,30 +446,13 @@ int dense_chain_launch(int B, int order, const int* idims, const int* odims, int
   ChainGeom g{};
   if (int rc = fill_modes(g, order, idims, odims, R, transposed, "dense_cp")) return rc;
   if (B < 1) return fail(B200CP_ERR_INVALID_ARG, "dense_cp: batch must be positive");
-  {
-    bool done = false;
-    if (int rc = dense_fast_launch(B, order, g.din, g.dout, g.fsi, g.fso, R, X, F, Y, st, &done)) return rc;
-    if (done) return B200CP_OK;
-  }
+  if (dense_fast_takes(order, g.din, g.dout, R, di)) return dense_fast_launch(B, g.fsi, g.fso, R, X, F, Y, st);
   g.conv = 0; g.B = B;
-  const int Alast = g.Cout / g.dout[g.m - 1];
-  int pix = 0;
-  for (int cand = 16; cand >= 4; cand -= 4) {
-    ChainGeom t = g;
-    t.PIX = cand;
-    if ((long)Alast * (cand / 4) > max_items(g)) continue;
-    if ((int)chain_smem(t) > di.smem_optin) continue;
-    // keep at least ~2 waves of tiles when the batch allows it
-    if (cand > 4 && (long)ceil_div(B, cand) < 2L * di.sm_count) continue;
-    pix = cand;
-    break;
-  }
-  if (!pix) return fail(B200CP_ERR_UNSUPPORTED, "dense_cp: layer %d -> %d does not fit on chip", g.Cin, g.Cout);
-  g.PIX = pix;
+  if (!dense_tile(g, di)) return fail(B200CP_ERR_UNSUPPORTED, "dense_cp: layer %d -> %d does not fit on chip", g.Cin, g.Cout);
   ChainPtrs p{};
   p.X = X; p.Y = Y;
   for (int k = 0; k < order; ++k) p.F[k] = F[k];
-  return dispatch_chain(g, p, ceil_div(B, pix), st);
+  return dispatch_chain(g, p, chain_ctas(g), st);
 }
 
 }  // namespace b200cp

@@ -207,12 +207,16 @@ int tc_selftest_launch(int mode, const float* A, const float* B, float* D, int* 
 int rcp_chain_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                      const float* X, const float* const* A, const float* S, float* V, bool transposed,
                      cudaStream_t st);
-// register-tiled kernel for the shapes it is compiled for; *done = false means "not this shape, use the chain kernel"
-int rcp_fast_launch(int N, int H, int W, int order, const int* din, const int* dout, const int* fsi, const int* fso,
-                    int R, int FH, int FW, const float* X, const float* const* A, const float* S, float* V, bool flip,
-                    cudaStream_t st, bool* done);
-int dense_fast_launch(int B, int order, const int* din, const int* dout, const int* fsi, const int* fso, int R,
-                      const float* X, const float* const* F, float* Y, cudaStream_t st, bool* done);
+// register-tiled kernels: which layers they take, their estimated microseconds, and the launch (the chain launchers call it)
+bool rcp_fast_takes(int order, const int* din, const int* dout, int R, int FH, int FW, int N, int H, int W,
+                    const DeviceInfo& di);
+double rcp_fast_us(int N, int H, int W, int R, const DeviceInfo& di);
+int rcp_fast_launch(int N, int H, int W, const int* fsi, const int* fso, int R, const float* X, const float* const* A,
+                    const float* S, float* V, bool flip, const DeviceInfo& di, cudaStream_t st);
+bool dense_fast_takes(int order, const int* din, const int* dout, int R, const DeviceInfo& di);
+double dense_fast_us(int B, int R, const DeviceInfo& di);
+int dense_fast_launch(int B, const int* fsi, const int* fso, int R, const float* X, const float* const* F, float* Y,
+                      cudaStream_t st);
 int dense_chain_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
                        const float* const* F, float* Y, bool transposed, cudaStream_t st);
 // The two layers by their multiplied-out weight (kron_small.cu).  Weight: W[slow][ld] or, with S, W[slow][tap][ld];
@@ -220,6 +224,13 @@ int dense_chain_launch(int B, int order, const int* idims, const int* odims, int
 int kron_weight_ld(int fast);
 int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
                        int taps, bool transposed, float* W, cudaStream_t st);
+// Estimated microseconds of the factored form (negative: it does not take the sizes; above `enough` any value above that
+// will do) and of the multiplied-out one.
+double rcp_factored_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
+                       bool transposed, double enough);
+double dense_factored_us(int B, int order, const int* idims, const int* odims, int R, bool transposed, double enough);
+double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, bool transposed);
+double dense_kron_us(int B, int order, const int* idims, const int* odims, int R, bool transposed);
 int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float* Y, cudaStream_t st);
 int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, float* V, cudaStream_t st);
 // Y = X M (dense) and V = K * X (reshaped-CP conv), or their data gradients (`transposed`), by the form that is

@@ -1,16 +1,18 @@
-// Reshaped-CP conv and CP dense layer by their multiplied-out weight, for problems whose weight and product are small.
+// Reshaped-CP conv and CP dense layer by their multiplied-out weight, where that is faster than the factored kernels.
 //
 // The factored form does R times the mode products one rank after the other; on the chain kernel that is a serial loop
-// of R x (modes + 1) block-wide steps over few CTAs, and it is latency, not arithmetic, that it spends its time on
-// (0.4 TMAC/s: 430 us for a batch of 64 through 16x16x16 -> 4x4x4 at R = 137, 223 us for eight 32x32 images of 16
-// channels at R = 11).  Multiplying the weight out first costs R multiply-adds per weight entry, spread over the whole
-// GPU, and leaves one plain product:
+// of R x (modes + 1) block-wide steps, one CTA per SM, and with few CTAs it is latency, not arithmetic, that it spends its
+// time on (430 us for a batch of 64 through 16x16x16 -> 4x4x4 at R = 137, 16 CTAs on 148 SMs; 223 us for eight 32x32 images
+// of 16 channels at R = 11).  Multiplying the weight out first costs R multiply-adds per weight entry, spread over the whole
+// GPU, and leaves one plain product, whatever R is; at low ranks and large batches the factored form does several times
+// less and is faster (product.cu has the rule).
 //   kron_weight_kernel : W[s][f] = sum_r prod_k F_k[s_k, f_k, r]   (conv: W[c][tap][t], with S as one more mode)
 //   small_gemm_kernel  : Y[m][n] = sum_k X[m][k] W[k][n]
 //   small_conv_kernel  : V[n,t,h,w] = sum_{c,y,x} W[c][y,x][t] X[n,c,h+y-1,w+x-1]
 // All exact fp32 (FFMA).  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
 // and past their set-up when the weight is done.  Formulas: Kernels/rcp_fused_nchw.cu:4-77, Kernels/dense_cp.cu:4-46.
 #include <algorithm>
+#include <cmath>
 
 #include "cluster_util.cuh"
 #include "common.cuh"
@@ -22,8 +24,8 @@ namespace {
 // The products add up to thousands of terms per result.  One accumulator over all of them rounds like sqrt(terms): relative
 // to float64 8e-7 for 4096 inputs, where the factored form, whose longest chain is ranks x one mode, has 2e-7 (R = 8).  So
 // an accumulator holds about kChain terms and is then added to a total: 1.8e-7 for the same sums.  The totals are in shared
-// memory, [4][threads] float4, and cost 5 % (4096 samples of 4096 -> 4096: 3.68 to 3.88 ms; 16 more registers instead would leave one CTA of 512
-// threads per SM instead of two: 4.73 ms).  A chain of at most kChain terms has none.
+// memory, [4][threads] float4, and cost 5 % (4096 samples of 4096 -> 4096: 3.68 to 3.88 ms; 16 more registers instead would
+// leave one CTA of 512 threads per SM instead of two: 4.73 ms).  A chain of at most kChain terms has none.
 constexpr int kChain = 64;
 template <int NT>
 __device__ __forceinline__ void flush_sums(float (&acc)[4][4], float* total, int tid, bool first) {
@@ -466,7 +468,128 @@ size_t spread_smem(size_t need, long ctas, const DeviceInfo& di) {
   return per > 4 ? need : std::max(need, (size_t)di.smem_optin / per - (per > 1 ? 1024 : 0));
 }
 
+// The tallest tile that leaves a CTA for most SMs (tall tiles form fewer half products per entry); a weight too small
+// even for 16-row tiles is shared out over the ranks as well.
+struct KronPlan {
+  int PA, nb, ta, splits, rper;
+  long ctas;
+};
+KronPlan kron_plan(int order, const int* slow, const int* fast, int R, int taps, const DeviceInfo& di) {
+  KronPlan p{};
+  int PB = 1;
+  p.PA = taps;
+  for (int k = 0; k < order; ++k) (k < order / 2 ? p.PA : PB) *= slow[k] * fast[k];
+  p.nb = ceil_div(PB, kTB);
+  p.ta = 64;
+  while (p.ta > 16 && (long)p.nb * ceil_div(p.PA, p.ta) * 5 < 4L * di.sm_count) p.ta /= 2;
+  const long tiles = (long)p.nb * ceil_div(p.PA, p.ta);
+  p.splits = pick_cluster(tiles, R, 16, di.sm_count);
+  p.rper = ceil_div(R, p.splits);
+  p.ctas = tiles * p.splits;
+  return p;
+}
+
+struct GemmPlan {
+  int bm, bn, splits, kper;
+  long tiles;
+};
+GemmPlan gemm_plan(int M, int N, int K, const DeviceInfo& di) {
+  GemmPlan p{};
+  // the tallest tile that leaves enough CTAs for one wave once a cluster splits K eight ways
+  const auto enough = [&](int bm) { return M > bm / 2 && (long)ceil_div(M, bm) * ceil_div(N, 64) * 8 >= di.sm_count; };
+  p.bm = enough(64) ? 64 : enough(32) ? 32 : 16;
+  p.bn = p.bm == 16 && (long)ceil_div(M, 16) * ceil_div(N, 64) * 8 < di.sm_count ? 32 : 64;
+  p.tiles = (long)ceil_div(M, p.bm) * ceil_div(N, p.bn);
+  p.splits = pick_cluster(p.tiles, K, 64, di.sm_count);
+  p.kper = (int)align_up((size_t)ceil_div(K, p.splits), 4);
+  return p;
+}
+
+struct ConvPlan {
+  int tt, cgroups;
+  long tiles;
+  SmallConvGeom g;
+};
+ConvPlan conv_plan(int N, int C, int T, int H, int W, const DeviceInfo& di) {
+  ConvPlan p{};
+  SmallConvGeom& g = p.g;
+  const int tt = p.tt = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  // two channel groups share the 16 warps; eight (four with 64 output channels: a warp holds 16 of them), with a quarter
+  // or half of the pixels per CTA, where there are few pixels
+  const bool few = (long)N * ceil_div(H * W, kCT * 2 / (tt / 4)) * ceil_div(T, tt) * 2 <= di.sm_count;
+  p.cgroups = few ? (tt == 64 ? 4 : 8) : 2;
+  const int quads = kCT / p.cgroups / (tt / 4);      // pixel quads per CTA
+  g.C = C; g.T = T; g.H = H; g.W = W; g.ldw = (T + 3) / 4 * 4;
+  // columns of the tile: the width that covers the image with the least waste and halo
+  int best = 4;
+  double best_cost = 1e300;
+  for (int tc = 4; tc <= std::min(32, (W + 3) / 4 * 4); tc += 4) {
+    const int tr = std::min(quads / (tc / 4), H);
+    if (tr < 1 || (tr + 2) * (tc + 2) > kHaloPer * kCT) continue;
+    const double cost = (double)ceil_div(W, tc) * ceil_div(H, tr) * (1.0 + 0.1 * (tr + 2.0) * (tc + 2.0) / (tr * tc));
+    if (cost < best_cost) { best_cost = cost; best = tc; }
+  }
+  g.TC = best;
+  g.TR = std::min(quads / (g.TC / 4), H);
+  g.tilesW = ceil_div(W, g.TC);
+  g.tiles = g.tilesW * ceil_div(H, g.TR);
+  g.PXQ = g.TR * (g.TC / 4);
+  g.P = g.TC + 8;
+  g.CS = (int)align_up((size_t)(g.TR + 2) * g.P, 4);
+  p.tiles = (long)N * g.tiles * ceil_div(T, tt);
+  g.splits = pick_cluster(p.tiles, C, 2 * kCC, di.sm_count);
+  g.cper = (int)align_up((size_t)ceil_div(C, g.splits), kCC);
+  g.buf = std::max(2 * (kCC * g.CS + kCC * 9 * tt), p.cgroups * tt * g.TR * g.TC);
+  return p;
+}
+
+double waves(long ctas, const DeviceInfo& di) { return (double)((ctas + di.sm_count - 1) / di.sm_count); }
+
 }  // namespace
+
+// Estimated microseconds of the two forms: waves of CTAs times the work of one, and the weight's entries written.  Least-
+// squares fit to the layers that the factored kernels' estimate is fitted to (chain_simt.cu).  Choosing by the two, 5 of
+// 1202 layers run more than 10 % and 2 us behind the other form, and all together 0.3 % behind the best choice.
+static double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed,
+                             const DeviceInfo& di) {
+  const KronPlan p = kron_plan(order, transposed ? odims : idims, transposed ? idims : odims, R, taps, di);
+  double slow = taps, fast = 1;
+  for (int k = 0; k < order; ++k) {
+    slow *= transposed ? odims[k] : idims[k];
+    fast *= transposed ? idims[k] : odims[k];
+  }
+  return 3.05e-6 * slow * std::ceil(fast / 4) * 4 + 4.07e-4 * waves(p.ctas, di) * p.rper * (p.ta + 64);
+}
+
+double dense_kron_us(int B, int order, const int* idims, const int* odims, int R, bool transposed) {
+  DeviceInfo di;
+  if (device_info(&di)) return -1;
+  int K = 1, N = 1;
+  for (int k = 0; k < order; ++k) {
+    K *= transposed ? odims[k] : idims[k];
+    N *= transposed ? idims[k] : odims[k];
+  }
+  const GemmPlan p = gemm_plan(B, N, K, di);
+  const double work = waves(p.tiles * p.splits, di) * p.kper * p.bm * p.bn;
+  return 5.1 + kron_weight_us(order, idims, odims, R, 1, transposed, di) +
+         (p.bm == 64 ? 7.93e-6 : p.bm == 32 ? 9.39e-6 : 7.69e-6) * work + 1.54e-6 * ((double)B * K + (double)B * N);
+}
+
+double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, bool transposed) {
+  DeviceInfo di;
+  if (device_info(&di)) return -1;
+  int C = 1, T = 1;
+  for (int k = 0; k < order; ++k) {
+    C *= transposed ? tdims[k] : cdims[k];
+    T *= transposed ? cdims[k] : tdims[k];
+  }
+  const ConvPlan p = conv_plan(N, C, T, H, W, di);
+  const SmallConvGeom& g = p.g;
+  const int px = kCT / p.cgroups / (p.tt / 4) * 4;
+  const double w = waves(p.tiles * g.splits, di) * g.cper;
+  return 5.1 + kron_weight_us(order, cdims, tdims, R, 9, transposed, di) +
+         (p.tt == 64 ? 6.71e-6 : 5.19e-6) * w * 9 * p.tt * px + 8.04e-4 * w * (g.TR + 2) * (g.TC + 2);
+}
 
 // Row pitch of the weight: 16-byte rows.
 int kron_weight_ld(int fast) { return (fast + 3) / 4 * 4; }
@@ -507,14 +630,10 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   for (int k = ha; k < order; ++k) { g.B[g.nB++] = m[k]; g.SB *= m[k].ns; g.FB *= m[k].nf; }
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
-  const int PA = g.SA * g.FA, PB = g.SB * g.FB, nb = ceil_div(PB, kTB);
-  // The tallest tile that leaves a CTA for most SMs (tall tiles form fewer half products per entry); a weight too small
-  // even for 16-row tiles is shared out over the ranks as well.
-  int ta = 64;
-  while (ta > 16 && (long)nb * ceil_div(PA, ta) * 5 < 4L * di.sm_count) ta /= 2;
-  const int splits = pick_cluster((long)nb * ceil_div(PA, ta), R, 16, di.sm_count);
-  g.rper = ceil_div(R, splits);
-  const dim3 grid(nb, ceil_div(PA, ta), splits);
+  const KronPlan p = kron_plan(order, transposed ? odims : idims, transposed ? idims : odims, R, S ? taps : 1, di);
+  const int ta = p.ta, splits = p.splits;
+  g.rper = p.rper;
+  const dim3 grid(p.nb, ceil_div(p.PA, ta), splits);
 #define KRON(TAV)                                                                                                       \
   do {                                                                                                                 \
     if (S) B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, true>, grid, dim3(kKT), 0, st, splits, false, g, W));  \
@@ -533,13 +652,9 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
   if (int rc = device_info(&di)) return rc;
   const int ldw = kron_weight_ld(N);
   const bool vec = !(K & 3) && !(reinterpret_cast<uintptr_t>(X) & 15);
-  // the tallest tile that leaves enough CTAs for one wave once a cluster splits K eight ways
-  const auto enough = [&](int bm) { return M > bm / 2 && (long)ceil_div(M, bm) * ceil_div(N, 64) * 8 >= di.sm_count; };
-  const int bm = enough(64) ? 64 : enough(32) ? 32 : 16;
-  const int bn = bm == 16 && (long)ceil_div(M, 16) * ceil_div(N, 64) * 8 < di.sm_count ? 32 : 64;
-  const long tiles = (long)ceil_div(M, bm) * ceil_div(N, bn);
-  const int splits = pick_cluster(tiles, K, 64, di.sm_count);
-  const int kper = (int)align_up((size_t)ceil_div(K, splits), 4);
+  const GemmPlan p = gemm_plan(M, N, K, di);
+  const int bm = p.bm, bn = p.bn, splits = p.splits, kper = p.kper;
+  const long tiles = p.tiles;
   if (tiles > 0x7fffffffL || M > 0x7fffffff - 64) return fail(B200CP_ERR_UNSUPPORTED, "dense: batch of %d rows too large", M);
   const dim3 grid((unsigned)tiles, 1, splits);   // (grid y would end at 65535 row tiles)
 #define SMALL_GEMM(BMV, BNV, V)                                                                                       \
@@ -562,34 +677,10 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
 int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, float* V, cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
-  const int tt = T <= 16 ? 16 : T <= 32 ? 32 : 64;
-  // two channel groups share the 16 warps; eight (four with 64 output channels: a warp holds 16 of them), with a quarter
-  // or half of the pixels per CTA, where there are few pixels
-  const bool few = (long)N * ceil_div(H * W, kCT * 2 / (tt / 4)) * ceil_div(T, tt) * 2 <= di.sm_count;
-  const int cgroups = few ? (tt == 64 ? 4 : 8) : 2;
-  const int quads = kCT / cgroups / (tt / 4);      // pixel quads per CTA
-  SmallConvGeom g{};
-  g.C = C; g.T = T; g.H = H; g.W = W; g.ldw = kron_weight_ld(T);
-  // columns of the tile: the width that covers the image with the least waste and halo
-  int best = 4;
-  double best_cost = 1e300;
-  for (int tc = 4; tc <= std::min(32, (W + 3) / 4 * 4); tc += 4) {
-    const int tr = std::min(quads / (tc / 4), H);
-    if (tr < 1 || (tr + 2) * (tc + 2) > kHaloPer * kCT) continue;
-    const double cost = (double)ceil_div(W, tc) * ceil_div(H, tr) * (1.0 + 0.1 * (tr + 2.0) * (tc + 2.0) / (tr * tc));
-    if (cost < best_cost) { best_cost = cost; best = tc; }
-  }
-  g.TC = best;
-  g.TR = std::min(quads / (g.TC / 4), H);
-  g.tilesW = ceil_div(W, g.TC);
-  g.tiles = g.tilesW * ceil_div(H, g.TR);
-  g.PXQ = g.TR * (g.TC / 4);
-  g.P = g.TC + 8;
-  g.CS = (int)align_up((size_t)(g.TR + 2) * g.P, 4);
-  const long tiles = (long)N * g.tiles * ceil_div(T, tt);
-  g.splits = pick_cluster(tiles, C, 2 * kCC, di.sm_count);
-  g.cper = (int)align_up((size_t)ceil_div(C, g.splits), kCC);
-  g.buf = std::max(2 * (kCC * g.CS + kCC * 9 * tt), cgroups * tt * g.TR * g.TC);
+  const ConvPlan p = conv_plan(N, C, T, H, W, di);
+  const SmallConvGeom& g = p.g;
+  const int tt = p.tt, cgroups = p.cgroups;
+  const long tiles = p.tiles;
   const size_t smem = sizeof(float) * ((size_t)g.buf + (ceil_div(g.cper, kCC) > conv_flush(cgroups) ? 16 * kCT : 0));
   dim3 grid((unsigned)(N * g.tiles), ceil_div(T, tt), g.splits);
   if ((long)N * g.tiles > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");

@@ -13,56 +13,40 @@ long prod(const int* d, int n) {
   return p;
 }
 
-// Estimated times in seconds.  Rates are what the kernels measured on a B200: multiply-adds per second of the small FFMA
-// products and of the register-tiled factored kernels at their own shapes; the multiplied-out form has one launch more.
-constexpr double kSmallGemmRate = 15e12, kSmallConvRate = 14e12, kDenseFastRate = 21e12, kRcpFastRate = 11e12;
-constexpr double kLaunch = 3e-6;
-
-bool is_fast_dense(int order, const int* a, const int* b) {
-  if (order != 4) return false;
-  for (int k = 0; k < 4; ++k)
-    if (a[k] != 8 || b[k] != 8) return false;
-  return true;
-}
-bool is_fast_rcp(int order, const int* a, const int* b, int FH, int FW) {
-  return order == 3 && FH == 3 && FW == 3 && a[0] == 4 && b[0] == 4 && a[1] == 8 && b[1] == 8 && a[2] == 8 && b[2] == 8;
-}
-
 // the weight as kron_weight_launch writes it
 size_t weight_floats(int order, const int* idims, const int* odims, int taps, bool transposed) {
   const long slow = prod(transposed ? odims : idims, order), fast = prod(transposed ? idims : odims, order);
   return (size_t)slow * taps * kron_weight_ld((int)fast);
 }
 
-enum class Form { kFactored, kSmall };
+// The form with the smaller estimated time runs (what the estimates are made of, and how good they are, stands beside
+// them: chain_kernel, the register-tiled kernels, kron_small.cu).  Either side of the line, us, factored / multiplied out:
+//   4096 samples of 16x16x16 -> 16x16x16   R = 4 386 / 3823    R = 16 1102 / 3830    R = 64 4006 / 3880    R = 256 15551 / 4095
+//   64 samples of the same                 R = 4 49 / 125      R = 16 152 / 134
+//   4096 samples of 10x10x10 -> 10x10x10   R = 4 127 / 257     R = 16 401 / 259
+//   one sample of 8x8x8x8 -> 8x8x8x4       R = 4 39 / 40       R = 16 131 / 45
+//   32 images of 28x28, 16x16 -> 16x16     R = 4 616 / 968     R = 8 1130 / 968;   4x8x8 -> 4x8x8 R = 64 894 / 973
+//   8 images of 32x32, 6x6x6 -> 6x6x6      R = 4 161 / 275     R = 8 300 / 275
+// A weight of more than kMostWeight bytes of scratch is multiplied out only for what the factored form does not take (it does
+// not fit on chip), up to kMostEntries.
+constexpr size_t kMostWeight = size_t{256} << 20;
+constexpr double kMostEntries = 1e9;
 
-Form dense_form(int B, int order, const int* idims, const int* odims, int R) {
-  const double I = (double)prod(idims, order), O = (double)prod(odims, order);
-  if (I * O > 1e9) return Form::kFactored;
-  if (is_fast_dense(order, idims, odims)) {
-    const double fact = (double)B * R * 4 * 4096 * 8;
-    if (fact / kDenseFastRate < (double)B * I * O / kSmallGemmRate + kLaunch) return Form::kFactored;
-  }
-  return Form::kSmall;
-}
-
-Form rcp_form(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW) {
-  if (FH != 3 || FW != 3) return Form::kFactored;
-  const double C = (double)prod(cdims, order), T = (double)prod(tdims, order), px = (double)N * H * W;
-  if (C * T * 9 > 1e9) return Form::kFactored;
-  if (is_fast_rcp(order, cdims, tdims, FH, FW)) {
-    const double fact = px * R * (256.0 * 9 + 256.0 * 20);
-    if (fact / kRcpFastRate < px * C * T * 9 / kSmallConvRate + kLaunch) return Form::kFactored;
-  }
-  return Form::kSmall;
+bool multiplies_out(size_t floats, double entries, double kron_us, double factored_us) {
+  if (factored_us < 0) return entries <= kMostEntries;
+  return factored_us > kron_us && floats * sizeof(float) <= kMostWeight;
 }
 
 }  // namespace
 
 size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed) {
   if (check_kron_modes(order, idims, odims, R, "dense_cp") || B < 1) return 0;
-  if (dense_form(B, order, idims, odims, R) == Form::kFactored) return 0;
-  return align_up(weight_floats(order, idims, odims, 1, transposed) * sizeof(float), 256);
+  if (B > 0x7fffffff - 64) return 0;
+  const size_t floats = weight_floats(order, idims, odims, 1, transposed);
+  const double kron = dense_kron_us(B, order, idims, odims, R, transposed);
+  const double entries = (double)prod(idims, order) * prod(odims, order);
+  if (!multiplies_out(floats, entries, kron, dense_factored_us(B, order, idims, odims, R, transposed, kron))) return 0;
+  return align_up(floats * sizeof(float), 256);
 }
 
 int dense_product_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
@@ -81,8 +65,12 @@ int dense_product_launch(int B, int order, const int* idims, const int* odims, i
 size_t rcp_product_workspace(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                              bool transposed) {
   if (check_kron_modes(order, cdims, tdims, R, "rcp") || N < 1 || H < 1 || W < 1) return 0;
-  if (rcp_form(N, H, W, order, cdims, tdims, R, FH, FW) == Form::kFactored) return 0;
-  return align_up(weight_floats(order, cdims, tdims, FH * FW, transposed) * sizeof(float), 256);
+  if (FH != 3 || FW != 3) return 0;
+  const size_t floats = weight_floats(order, cdims, tdims, 9, transposed);
+  const double kron = rcp_kron_us(N, H, W, order, cdims, tdims, R, transposed);
+  const double entries = 9.0 * prod(cdims, order) * prod(tdims, order);
+  if (!multiplies_out(floats, entries, kron, rcp_factored_us(N, H, W, order, cdims, tdims, R, FH, FW, transposed, kron))) return 0;
+  return align_up(floats * sizeof(float), 256);
 }
 
 int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,

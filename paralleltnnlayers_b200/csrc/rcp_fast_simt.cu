@@ -208,56 +208,59 @@ __global__ void __launch_bounds__(NT, 1) rcp3_fast_kernel(const RcpFastArgs a) {
   }
 }
 
-template <int I1, int O1, int I2, int O2, int I3, int O3, int TH, int TW, int SW, int NT>
-int launch_fast(RcpFastArgs a, const DeviceInfo& di, cudaStream_t st, bool* fits) {
-  using K = RcpFastCfg<I1, O1, I2, O2, I3, O3, TH, TW, SW, NT>;
-  const size_t smem = K::smem_bytes(a.R);
-  *fits = smem <= (size_t)di.smem_optin;
-  if (!*fits) return B200CP_OK;
+template <int TH, int TW, int NT>
+using RcpFast = RcpFastCfg<4, 4, 8, 8, 8, 8, TH, TW, TW, NT>;
+
+template <int TH, int TW, int NT>
+int launch_fast(RcpFastArgs a, cudaStream_t st) {
+  const size_t smem = RcpFast<TH, TW, NT>::smem_bytes(a.R);
   a.tilesH = ceil_div(a.H, TH);
   a.tilesW = ceil_div(a.W, TW);
-  const long ctas = (long)a.N * a.tilesH * a.tilesW;
-  if (ctas > 0x7fffffffL) { *fits = false; return B200CP_OK; }
-  auto kern = rcp3_fast_kernel<I1, O1, I2, O2, I3, O3, TH, TW, SW, NT>;
+  auto kern = rcp3_fast_kernel<4, 4, 8, 8, 8, 8, TH, TW, TW, NT>;
   B200CP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<(unsigned)ctas, NT, smem, st>>>(a);
+  kern<<<(unsigned)((long)a.N * a.tilesH * a.tilesW), NT, smem, st>>>(a);
   B200CP_LAUNCH_OK("rcp3_fast_kernel");
   return B200CP_OK;
 }
 
+long tiles(int N, int H, int W, int t) { return (long)N * ceil_div(H, t) * ceil_div(W, t); }
+
+// 7x7 tiles waste no pixels when 7 divides the image; 8x8 tiles otherwise
+bool seven(int N, int H, int W, const DeviceInfo& di) {
+  const char* force = getenv("B200CP_RCP_TILE");  // "7" or "8": experiments and tests
+  if (force) return force[0] == '7';
+  const auto cost = [&](int t) { return (tiles(N, H, W, t) + di.sm_count - 1) / di.sm_count * t * t; };
+  return cost(7) <= cost(8);
+}
+
 }  // namespace
 
-// Launches the register-tiled kernel when the layer has the shape it is compiled for (order 3, modes
-// (4,8,8) -> (4,8,8), 3x3 core); *done tells the caller whether it did.  din/dout and the strides describe the
-// factors as the chain kernel's host code does (contracted index first).
-int rcp_fast_launch(int N, int H, int W, int order, const int* din, const int* dout, const int* fsi, const int* fso,
-                    int R, int FH, int FW, const float* X, const float* const* A, const float* S, float* V, bool flip,
-                    cudaStream_t st, bool* done) {
-  *done = false;
-  if (order != 3 || FH != 3 || FW != 3) return B200CP_OK;
-  if (!(din[0] == 4 && dout[0] == 4 && din[1] == 8 && dout[1] == 8 && din[2] == 8 && dout[2] == 8)) return B200CP_OK;
-  if (getenv("B200CP_NO_FAST")) return B200CP_OK;
-  DeviceInfo di;
-  if (int rc = device_info(&di)) return rc;
+// The shape the register-tiled kernel is compiled for (order 3, modes (4,8,8) -> (4,8,8), 3x3 core), at a rank whose
+// factors fit beside the tile in shared memory.
+bool rcp_fast_takes(int order, const int* din, const int* dout, int R, int FH, int FW, int N, int H, int W,
+                    const DeviceInfo& di) {
+  if (order != 3 || FH != 3 || FW != 3) return false;
+  if (!(din[0] == 4 && dout[0] == 4 && din[1] == 8 && dout[1] == 8 && din[2] == 8 && dout[2] == 8)) return false;
+  const bool s = seven(N, H, W, di);
+  const size_t smem = s ? RcpFast<7, 7, 448>::smem_bytes(R) : RcpFast<8, 8, 512>::smem_bytes(R);
+  return smem <= (size_t)di.smem_optin && tiles(N, H, W, s ? 7 : 8) <= 0x7fffffffL && !getenv("B200CP_NO_FAST");
+}
+
+// Estimated microseconds: waves of one CTA per SM.  Measured, R = 4 / 16 / 64: 32 x 28x28 (four waves of 7x7 tiles)
+// 92 / 250 / 894, 32 x 32x32 (four of 8x8) 97 / 266 / 949, one wave 25 / 64 / 225.
+double rcp_fast_us(int N, int H, int W, int R, const DeviceInfo& di) {
+  const bool s = seven(N, H, W, di);
+  return 1.0 + (double)((tiles(N, H, W, s ? 7 : 8) + di.sm_count - 1) / di.sm_count) * (9.9 + (s ? 3.36 : 3.56) * R);
+}
+
+// for layers rcp_fast_takes; the strides describe the factors as the chain kernel's host code does (contracted index first)
+int rcp_fast_launch(int N, int H, int W, const int* fsi, const int* fso, int R, const float* X, const float* const* A,
+                    const float* S, float* V, bool flip, const DeviceInfo& di, cudaStream_t st) {
   RcpFastArgs a{};
   a.X = X; a.S = S; a.V = V;
   a.N = N; a.H = H; a.W = W; a.R = R; a.flip = flip ? 1 : 0;
   for (int k = 0; k < 3; ++k) { a.A[k] = A[k]; a.fsi[k] = fsi[k]; a.fso[k] = fso[k]; }
-  // 7x7 tiles waste no pixels when 7 divides the image; 8x8 tiles otherwise
-  const auto cost = [&](int th, int tw) {
-    const long ctas = (long)N * ceil_div(H, th) * ceil_div(W, tw);
-    return (double)((ctas + di.sm_count - 1) / di.sm_count) * th * tw;
-  };
-  bool fits = false;
-  const char* force = getenv("B200CP_RCP_TILE");  // "7" or "8": experiments and tests
-  const bool seven = force ? force[0] == '7' : cost(7, 7) <= cost(8, 8);
-  if (seven) {
-    if (int rc = launch_fast<4, 4, 8, 8, 8, 8, 7, 7, 7, 448>(a, di, st, &fits)) return rc;
-  } else {
-    if (int rc = launch_fast<4, 4, 8, 8, 8, 8, 8, 8, 8, 512>(a, di, st, &fits)) return rc;
-  }
-  *done = fits;
-  return B200CP_OK;
+  return seven(N, H, W, di) ? launch_fast<7, 7, 448>(a, st) : launch_fast<8, 8, 512>(a, st);
 }
 
 }  // namespace b200cp
