@@ -99,35 +99,61 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // Which 3x3 / pad 1 convolutions and backward passes run as products over whole rank planes (cp_planes.cu); B200CP_PLANES=0
 // switches them off.  The tile and row kernels they compete with keep a plane in shared memory, so they win while one
 // chunk of ranks and enough tiles of one image keep every SM busy; the products have a fixed cost of three to five
-// dependent launches (about 14 us for a convolution at R > 32) and take any split of channels and pixels.  Measured, tile
-// or row kernels / products, us, shapes N x C x T x H x W:
-//   convolution, R = 128: 32x64x64x56x56 254 / 136, 8x256x256x14x14 131 / 23, 64x32x32x63x61 328 / 280
-//   R = 64: 8x256x256x14x14 59 / 23, 64x512x512x7x7 52 / 31, 32x64x64x56x56 90 / 76, 8x48x256x55x55 62 / 53,
-//     32x128x128x28x28 41 / 41, but 16x64x128x28x28 23 / 27, 16x256x384x27x27 52 / 54, 64x32x32x63x61 133 / 149
-//   R = 32: 8x256x256x14x14 27 / 15, 64x512x512x7x7 29 / 25, 1x512x512x7x7 17 / 17, but 16x256x384x27x27 33 / 37,
-//     32x64x64x56x56 41 / 48
-//   training step, R = 50: every shape measured, 1.15 to 3 times faster; R = 32: 64x256x256x14x14 101 / 75,
-//     64x512x512x7x7 91 / 59, 16x256x384x27x27 111 / 110, but 32x64x64x56x56 142 / 152, 2x33x70x45x31 31 / 41
+// dependent launches (about 14 us for a convolution at R > 32) and take any split of channels and pixels, but pad ranks and
+// channels to tiles of 64.  Measured, tile or row kernels / products, us, shapes N x C x T x H x W:
+//   convolution  R = 128: 32x64x64x56x56 254 / 136, 8x256x256x14x14 131 / 23, but 32x8x8x63x61 74 / 113
+//     R = 65: 16x16x16x27x27 18 / 20, 16x8x8x27x27 15 / 21;  R = 100: 16x8x8x27x27 19 / 23
+//     R = 64: 8x256x256x14x14 59 / 23, 64x512x512x7x7 52 / 31, 32x64x64x56x56 90 / 76, 16x64x128x28x28 23 / 27
+//     R = 32: 8x256x256x14x14 27 / 15, 64x512x512x7x7 29 / 25, 1x512x512x7x7 17 / 17, but 32x64x64x56x56 41 / 48
+//   training step  R = 50: 1.15 to 3 times faster with 32 channels and more, 8x8x14x14 64 images 37 / 39;  R = 32:
+//     64x256x256x14x14 101 / 75, 64x512x512x7x7 91 / 59, but 32x64x64x56x56 142 / 152
 //   R = 8: 64x512x512x7x7 53 / 46, 8x256x256x14x14 28 / 25, but 64x256x256x14x14 52 / 54, 16x256x384x27x27 66 / 84
-//   backward of the three-factor convolution, whose other kernels contract the channels twice: R = 32 32x64x64x56x56
-//     233 / 179 with the forward, but 64x32x32x63x61 334 / 399; R = 16: 64x512x512x7x7 121 / 94, 32x64x64x56x56 109 / 124
+//   factor gradients alone  R = 64: 64x16x16x7x7 15 / 21, 32x16x16x28x28 37 / 41, but 32x24x24x28x28 50 / 39; with the tile
+//     kernel's 9x9 tiles in one full round 16x16x16x27x27 17 / 35, 16x64x64x27x27 36 / 38;  R = 65 (padded to 128)
+//     32x16x16x56x56 123 / 169, 64x16x16x7x7 27 / 23;  R = 128 32x16x16x28x28 65 / 57
+//   backward from the saved plane  R = 64, with the forward: 64x16x16x14x14 37 / 51, 4x16x16x56x56 46 / 42
+//   three-factor convolution, whose other kernels contract the channels twice: with the forward R = 32 32x64x64x56x56
+//     233 / 179, 16x64x64x27x27 45 / 54, 32x64x64x28x28 76 / 78; R = 64 16x16x16x27x27 35 / 53, 64x16x16x32x32 124 / 112;
+//     R = 16 64x512x512x7x7 121 / 94.  Its factor gradients alone: R = 32 32x64x64x28x28 31 / 40, 4x80x80x56x56 about 30 / 23
 const bool g_planes = [] {
   const char* e = getenv("B200CP_PLANES");
   return !(e && e[0] == '0');
 }();
-enum class Planes { kConv, kBackward, kBackward3 };   // one convolution; a step or the factor gradients; those of CP3
+// one convolution; the step; the backward from the forward's plane; the factor gradients; the last two of CP3
+enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3 };
 bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !g_planes || !planes_supported(*s)) return false;
+  DeviceInfo di;
+  if (device_info(&di)) return false;
   const size_t px = (size_t)s->N * s->H * s->W, ch = (size_t)s->C + s->T;
   const unsigned R = s->Rank;
   const bool few = px <= 4096 && ch >= 512;   // small images, many channels: few tiles, each a long chain
+  // the tile kernels' tiles (9x9 pixels for 33 to 64 ranks, 14x14 for 17 to 32) fill the SMs once: no idle SM, no last round
+  const auto one_round = [&](unsigned side) {
+    return px > 8192 && (size_t)s->N * ceil_div((int)s->H, (int)side) * ceil_div((int)s->W, (int)side) <= (size_t)di.sm_count;
+  };
+  const bool full14 = one_round(14) && (10 * px > 7 * 14 * 14 * (size_t)di.sm_count || (s->H * s->W & 1));
+  const bool step = R > 32 || (R > 16 && px <= 16384 && ch >= 384) || (few && (s->W & 3));   // (the row kernels take W % 4 == 0)
+  const bool mid = R > 32 && R <= 64;
   switch (use) {
     case Planes::kConv:
-      return R > 64 || (R > 32 && ((px <= 4096 && ch >= 256) || (px >= 16384 && ch >= 128))) || (R > 16 && few);
-    case Planes::kBackward:
-      return R > 32 || (R > 16 && px <= 16384 && ch >= 384) || (few && (s->W & 3));   // (the row kernels take W % 4 == 0)
+      return (R > 64 && ch >= 32) || (mid && ((px <= 4096 && ch >= 256) || (px >= 16384 && ch >= 128))) || (R > 16 && few);
+    case Planes::kStep:
+      return step;
+    case Planes::kSaved:
+      return step && !(mid && ((ch < 64 && (s->W & 3)) || (ch < 128 && one_round(9))));
+    case Planes::kFilter:
+    case Planes::kFilter3:
+      if (mid) return ch >= 48 && !(ch < 160 && one_round(9));
+      if (R > 64) {
+        const bool padded = 3 * R <= 2 * ((R + 63) / 64 * 64);   // a third and more of the rank tiles is padding
+        return ch >= 48 ? !(ch < 96 && one_round(9)) : px <= 4096 || (!padded && px < 65536 && !one_round(9));
+      }
+      if (use == Planes::kFilter) return step;
+      return ch >= 512 || (R > 16 && ch >= 128 && !(ch < 224 && full14));
     default:
-      return R > 32 || (R > 16 && ch >= 128) || ch >= 512;
+      if (mid) return px >= 32768 || (ch >= 48 && !(ch < 128 && one_round(9)));
+      return R > 64 || ch >= 512 || (R > 16 && ch >= 128 && !(ch < 160 && full14));
   }
 }
 
@@ -272,7 +298,7 @@ int b200cp_cp4_bwd_data_ws(const b200cp_tensor_shape* s, const float* dU, const 
 
 size_t b200cp_cp4_bwd_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
   if (check_shape(s, "b200cp_cp4_bwd_saved_workspace_bytes")) return 0;
-  if (takes_planes(s, flags, Planes::kBackward)) return planes_workspace(*s, kPlanesBwd | kPlanesGrads | kPlanesNoP);
+  if (takes_planes(s, flags, Planes::kSaved)) return planes_workspace(*s, kPlanesBwd | kPlanesGrads | kPlanesNoP);
   return align_up((size_t)s->N * s->Rank * s->H * s->W * sizeof(float), 256) + b200cp_cp4_bwd_filter_saved_workspace_bytes(s, flags);
 }
 
@@ -285,7 +311,7 @@ int b200cp_cp4_bwd_saved(const b200cp_tensor_shape* s, const float* X, const flo
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15))
     return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_saved: a 16-byte aligned workspace of %zu bytes needed, %zu given", need,
                 workspace_bytes);
-  if (takes_planes(s, flags, Planes::kBackward)) {
+  if (takes_planes(s, flags, Planes::kSaved)) {
     PlanesJob j;
     j.s = s; j.X = X; j.dU = dU; j.P = P; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.dX = dX; j.dK = dK_packed;
     return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
@@ -312,7 +338,7 @@ size_t b200cp_cp4_bwd_filter_workspace_bytes(const b200cp_tensor_shape* s, int f
   if (check_shape(s, "b200cp_cp4_bwd_filter_workspace_bytes")) return 0;
   if (path_of(flags) == B200CP_PATH_SIMT) return cp4_bwd_filter_simt_workspace(*s);
   size_t need = std::max(cp4_bwd_filter_simt_workspace(*s), cp4_bwd_filter_mma_workspace(*s));
-  if (takes_planes(s, flags, Planes::kBackward)) need = std::max(need, planes_workspace(*s, kPlanesGrads));
+  if (takes_planes(s, flags, Planes::kFilter)) need = std::max(need, planes_workspace(*s, kPlanesGrads));
   if (bwd_filter_by_planes(s, flags)) need = std::max(need, 2 * bwd_filter_plane_bytes(s) + cp4_grad_band_workspace(*s));
   return need;
 }
@@ -329,7 +355,7 @@ int b200cp_cp4_bwd_filter(const b200cp_tensor_shape* s, const float* X, const fl
   if (path == B200CP_PATH_TC3X || path == B200CP_PATH_TC1X)
     return fail(B200CP_ERR_UNSUPPORTED, "cp4 bwd-filter: the tcgen05 path is not available for this operation");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_filter: workspace is null");
-  if (takes_planes(s, flags, Planes::kBackward) && has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads))) {
+  if (takes_planes(s, flags, Planes::kFilter) && has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads))) {
     PlanesJob j;
     j.s = s; j.X = X; j.dU = dU; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.dK = dK_packed;
     return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
@@ -395,7 +421,7 @@ int b200cp_cp3_bwd_data(const b200cp_tensor_shape* s, const float* dU, const flo
 
 int b200cp_cp3_shares_planes(const b200cp_tensor_shape* s, int flags) {
   if (check_shape(s, "b200cp_cp3_shares_planes")) return 0;
-  return takes_planes(s, flags, Planes::kBackward3) ? 1 : 0;
+  return takes_planes(s, flags, Planes::kSaved3) ? 1 : 0;
 }
 
 size_t b200cp_cp3_fwd_workspace_bytes(const b200cp_tensor_shape* s, int saves_plane, int flags) {
@@ -436,7 +462,7 @@ int b200cp_cp3_bwd_data_ws(const b200cp_tensor_shape* s, const float* dU, const 
 }
 
 size_t b200cp_cp3_bwd_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
-  if (check_shape(s, "b200cp_cp3_bwd_saved_workspace_bytes") || !takes_planes(s, flags, Planes::kBackward3)) return 0;
+  if (check_shape(s, "b200cp_cp3_bwd_saved_workspace_bytes") || !takes_planes(s, flags, Planes::kSaved3)) return 0;
   return planes_workspace(*s, kPlanesBwd | kPlanesGrads | kPlanesNoP);
 }
 
@@ -445,7 +471,7 @@ int b200cp_cp3_bwd_saved(const b200cp_tensor_shape* s, const float* X, const flo
                          size_t workspace_bytes, void* stream, int flags) {
   if (int rc = check_shape(s, "b200cp_cp3_bwd_saved")) return rc;
   if (int rc = check_ptrs("b200cp_cp3_bwd_saved", {X, dU, P, KT, KCin, KC, dK_packed})) return rc;
-  if (!takes_planes(s, flags, Planes::kBackward3))
+  if (!takes_planes(s, flags, Planes::kSaved3))
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp3_bwd_saved: for shapes of b200cp_cp3_shares_planes only");
   PlanesJob j;
   j.s = s; j.X = X; j.dU = dU; j.P = P; j.K0 = KT; j.K1 = KCin; j.KC = KC; j.dX = dX; j.dK = dK_packed;
@@ -454,7 +480,7 @@ int b200cp_cp3_bwd_saved(const b200cp_tensor_shape* s, const float* X, const flo
 
 size_t b200cp_cp3_bwd_filter_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
   if (check_shape(s, "b200cp_cp3_bwd_filter_workspace_bytes")) return 0;
-  return std::max(cp4_bwd_filter_mma_workspace(*s), takes_planes(s, flags, Planes::kBackward3) ? planes_workspace(*s, kPlanesGrads) : 0);
+  return std::max(cp4_bwd_filter_mma_workspace(*s), takes_planes(s, flags, Planes::kFilter3) ? planes_workspace(*s, kPlanesGrads) : 0);
 }
 
 int b200cp_cp3_bwd_filter(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* KT,
@@ -469,7 +495,7 @@ int b200cp_cp3_bwd_filter(const b200cp_tensor_shape* s, const float* X, const fl
   if (path != B200CP_PATH_AUTO && path != B200CP_PATH_MMA)
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp3_bwd_filter: runs on the mma path only (flags AUTO or MMA)");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp3_bwd_filter: workspace is null");
-  if (takes_planes(s, flags, Planes::kBackward3) && has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads))) {
+  if (takes_planes(s, flags, Planes::kFilter3) && has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads))) {
     PlanesJob j;
     j.s = s; j.X = X; j.dU = dU; j.K0 = KT; j.K1 = KCin; j.KC = KC; j.dK = dK_packed;
     return planes_launch(j, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
@@ -588,7 +614,7 @@ size_t b200cp_cp4_step_workspace_bytes(const b200cp_tensor_shape* s, int flags) 
   if (check_shape(s, "b200cp_cp4_step_workspace_bytes")) return 0;
   const size_t plain = b200cp_cp4_bwd_filter_workspace_bytes(s, flags);
   if (!step_shares_planes(s, flags)) return plain;
-  const size_t products = takes_planes(s, flags, Planes::kBackward) ? planes_workspace(*s, kPlanesFwd | kPlanesBwd | kPlanesGrads) : 0;
+  const size_t products = takes_planes(s, flags, Planes::kStep) ? planes_workspace(*s, kPlanesFwd | kPlanesBwd | kPlanesGrads) : 0;
   const size_t plane = align_up((size_t)s->N * s->Rank * s->H * s->W * sizeof(float), 256);
   return std::max(products, 2 * plane + std::max(std::max(plain, cp4_bwd_filter_saved_workspace(*s)), cp4_grad_band_workspace(*s)));
 }
@@ -613,7 +639,7 @@ static int cp4_step_impl(const b200cp_tensor_shape* s, const float* X, const flo
     if (int rc = b200cp_cp4_bwd_data(s, dU, K0, K1, KH, KW, dX, stream, flags)) return rc;
     return b200cp_cp4_bwd_filter(s, X, dU, K0, K1, KH, KW, dK_packed, workspace, workspace_bytes, stream, fflags);
   }
-  if (takes_planes(s, flags, Planes::kBackward) &&
+  if (takes_planes(s, flags, Planes::kStep) &&
       has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesFwd | kPlanesBwd | kPlanesGrads))) {
     PlanesJob j;
     j.s = s; j.X = X; j.dU = dU; j.K0 = K0; j.K1 = K1; j.KH = KH; j.KW = KW; j.U = U; j.dX = dX; j.dK = dK_packed;
@@ -834,7 +860,7 @@ int b200cp_cp4_fwd_bwd_data(const b200cp_tensor_shape* s, const float* X, const 
 size_t b200cp_cp4_bwd_filter_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
   if (check_shape(s, "b200cp_cp4_bwd_filter_saved_workspace_bytes")) return 0;
   const size_t need = std::max(cp4_bwd_filter_saved_workspace(*s), cp4_grad_band_workspace(*s));
-  return takes_planes(s, flags, Planes::kBackward) ? std::max(need, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ)) : need;
+  return takes_planes(s, flags, Planes::kFilter) ? std::max(need, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ)) : need;
 }
 
 int b200cp_cp4_bwd_filter_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P,
@@ -845,7 +871,7 @@ int b200cp_cp4_bwd_filter_saved(const b200cp_tensor_shape* s, const float* X, co
   if (!step_shares_planes(s, flags))
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp4_bwd_filter_saved: 3x3 filters with pad 1 on the default (mma) path only");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_filter_saved: workspace is null");
-  if (takes_planes(s, flags, Planes::kBackward) &&
+  if (takes_planes(s, flags, Planes::kFilter) &&
       has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ))) {
     PlanesJob j;
     j.s = s; j.X = X; j.dU = dU; j.P = P; j.Q = Q; j.KH = KH; j.KW = KW; j.dK = dK_packed;

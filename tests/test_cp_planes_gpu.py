@@ -168,3 +168,33 @@ def test_cp3_backward_forms_what_is_asked_for():
     assert n_factors == n_all - 1
     with torch.no_grad():
         assert n_data == launched(lambda: P.cp3_conv2d_backward_data(du, *k))[0]
+
+
+# Which kernels form the factor gradients alone: the tile kernels (two launches per 64 ranks) where their tiles fill the SMs
+# once or the channels are few, the plane products (four launches) elsewhere; the times stand beside the rule.
+@pytest.mark.parametrize("shape, cp3, launches", [
+    ((16, 16, 16, 27, 27, 64), False, 2), ((16, 16, 16, 27, 27, 64), True, 2), ((32, 16, 16, 28, 28, 50), False, 2),
+    ((64, 8, 8, 7, 7, 64), True, 2), ((32, 64, 64, 28, 28, 32), True, 2), ((16, 64, 64, 27, 27, 24), True, 2),
+    ((32, 24, 24, 28, 28, 64), False, 4), ((8, 256, 256, 14, 14, 33), False, 4), ((4, 96, 96, 28, 28, 32), True, 4),
+])
+def test_filter_rule(shape, cp3, launches):
+    import paralleltnnlayers_b200 as P
+    from paralleltnnlayers_b200._lib import lib
+    X, dU, K = make(shape, cp3)
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+    before = lib.b200cp_launch_count()
+    grads = (P.cp3_conv2d_backward_filter if cp3 else P.cp4_conv2d_backward_filter)(du, x, *k)
+    assert lib.b200cp_launch_count() - before == launches
+    for got, ref in zip(grads, expect(X, dU, K)[2:]):
+        assert_parity(got, ref)
+
+
+@pytest.mark.parametrize("shape, shared", [((16, 64, 64, 27, 27, 32), False), ((16, 16, 16, 27, 27, 64), False), ((64, 8, 8, 7, 7, 50), False),
+                                           ((32, 64, 64, 56, 56, 32), True), ((64, 16, 16, 32, 32, 50), True),
+                                           ((64, 512, 512, 7, 7, 16), True)])
+def test_cp3_shared_plane_rule(shape, shared):
+    from paralleltnnlayers_b200._lib import TensorShape, lib
+    import ctypes as C
+    N, Cc, T, H, W, R = shape
+    s = TensorShape(N=N, H=H, W=W, pad=1, T=T, C=Cc, Y=3, X=3, Rank=R)
+    assert bool(lib.b200cp_cp3_shares_planes(C.byref(s), 0)) is shared
