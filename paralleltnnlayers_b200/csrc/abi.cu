@@ -123,16 +123,16 @@ const bool g_planes = [] {
 enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3 };
 bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !g_planes || !planes_supported(*s)) return false;
-  DeviceInfo di;
-  if (device_info(&di)) return false;
   const size_t px = (size_t)s->N * s->H * s->W, ch = (size_t)s->C + s->T;
   const unsigned R = s->Rank;
   const bool few = px <= 4096 && ch >= 512;   // small images, many channels: few tiles, each a long chain
   // the tile kernels' tiles (9x9 pixels for 33 to 64 ranks, 14x14 for 17 to 32) fill the SMs once: no idle SM, no last round
   const auto one_round = [&](unsigned side) {
-    return px > 8192 && (size_t)s->N * ceil_div((int)s->H, (int)side) * ceil_div((int)s->W, (int)side) <= (size_t)di.sm_count;
+    DeviceInfo di;
+    return px > 8192 && device_info(&di) == B200CP_OK &&
+           (size_t)s->N * ceil_div((int)s->H, (int)side) * ceil_div((int)s->W, (int)side) <= (size_t)di.sm_count;
   };
-  const bool full14 = one_round(14) && (10 * px > 7 * 14 * 14 * (size_t)di.sm_count || (s->H * s->W & 1));
+  const auto full14 = [&] { return one_round(14) && (px > 20000 || (s->H * s->W & 1)); };   // (odd images: 4-byte copies)
   const bool step = R > 32 || (R > 16 && px <= 16384 && ch >= 384) || (few && (s->W & 3));   // (the row kernels take W % 4 == 0)
   const bool mid = R > 32 && R <= 64;
   switch (use) {
@@ -150,10 +150,10 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
         return ch >= 48 ? !(ch < 96 && one_round(9)) : px <= 4096 || (!padded && px < 65536 && !one_round(9));
       }
       if (use == Planes::kFilter) return step;
-      return ch >= 512 || (R > 16 && ch >= 128 && !(ch < 224 && full14));
+      return ch >= 512 || (R > 16 && ch >= 128 && !(ch < 224 && full14()));
     default:
       if (mid) return px >= 32768 || (ch >= 48 && !(ch < 128 && one_round(9)));
-      return R > 64 || ch >= 512 || (R > 16 && ch >= 128 && !(ch < 160 && full14));
+      return R > 64 || ch >= 512 || (R > 16 && ch >= 128 && !(ch < 160 && full14()));
   }
 }
 
