@@ -230,8 +230,9 @@ int b200cp_cp4_step_host_wait(int slot);
 int b200cp_rcp_fwd(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                    const float* X, const float* const* A, const float* S, float* V, void* stream, int flags);
 
-/* The same with a workspace (16-byte aligned; b200cp_rcp_fwd_workspace_bytes bytes, which may be 0), in which the layer's
- * weight can be multiplied out: several times faster wherever the size is not 0.  Too small or NULL: as b200cp_rcp_fwd. */
+/* The same with a workspace (16-byte aligned; b200cp_rcp_fwd_workspace_bytes bytes), in which the layer's weight is multiplied
+ * out.  The size is 0 where the factored kernels are estimated to be faster (low ranks, many pixels), at most 256 MB where
+ * they take the layer, and up to 4 GB for layers that only this call takes.  Too small or NULL: as b200cp_rcp_fwd. */
 size_t b200cp_rcp_fwd_workspace_bytes(int N, int H, int W, int order, const int* cdims, const int* tdims, int R,
                                       int FH, int FW, int flags);
 int b200cp_rcp_fwd_ws(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -292,8 +293,9 @@ int b200cp_dense_matmul(int B, int I, int O, const float* X, const float* M, flo
 int b200cp_dense_fwd(int B, int order, const int* idims, const int* odims, int R, const float* X,
                      const float* const* F, float* Y, void* stream, int flags);
 
-/* The same with a workspace (16-byte aligned; b200cp_dense_fwd_workspace_bytes bytes, which may be 0), in which the
- * layer's weight can be multiplied out: several times faster wherever the size is not 0.  Too small or NULL: as
+/* The same with a workspace (16-byte aligned; b200cp_dense_fwd_workspace_bytes bytes), in which the layer's weight is
+ * multiplied out.  The size is 0 where the factored kernels are estimated to be faster (low ranks, large batches), at most
+ * 256 MB where they take the layer, and up to 4 GB for layers that only this call takes.  Too small or NULL: as
  * b200cp_dense_fwd. */
 size_t b200cp_dense_fwd_workspace_bytes(int B, int order, const int* idims, const int* odims, int R, int flags);
 int b200cp_dense_fwd_ws(int B, int order, const int* idims, const int* odims, int R, const float* X,

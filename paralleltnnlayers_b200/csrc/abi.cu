@@ -100,21 +100,23 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // switches them off.  The tile and row kernels they compete with keep a plane in shared memory, so they win while one
 // chunk of ranks and enough tiles of one image keep every SM busy; the products have a fixed cost of three to five
 // dependent launches (about 14 us for a convolution at R > 32) and take any split of channels and pixels, but pad ranks and
-// channels to tiles of 64.  Measured, tile or row kernels / products, us, shapes N x C x T x H x W:
-//   convolution  R = 128: 32x64x64x56x56 254 / 136, 8x256x256x14x14 131 / 23, but 32x8x8x63x61 74 / 113
-//     R = 65: 16x16x16x27x27 18 / 20, 16x8x8x27x27 15 / 21;  R = 100: 16x8x8x27x27 19 / 23
-//     R = 64: 8x256x256x14x14 59 / 23, 64x512x512x7x7 52 / 31, 32x64x64x56x56 90 / 76, 16x64x128x28x28 23 / 27
-//     R = 32: 8x256x256x14x14 27 / 15, 64x512x512x7x7 29 / 25, 1x512x512x7x7 17 / 17, but 32x64x64x56x56 41 / 48
-//   training step  R = 50: 1.15 to 3 times faster with 32 channels and more, 8x8x14x14 64 images 37 / 39;  R = 32:
-//     64x256x256x14x14 101 / 75, 64x512x512x7x7 91 / 59, but 32x64x64x56x56 142 / 152
-//   R = 8: 64x512x512x7x7 53 / 46, 8x256x256x14x14 28 / 25, but 64x256x256x14x14 52 / 54, 16x256x384x27x27 66 / 84
-//   factor gradients alone  R = 64: 64x16x16x7x7 15 / 21, 32x16x16x28x28 37 / 41, but 32x24x24x28x28 50 / 39; with the tile
-//     kernel's 9x9 tiles in one full round 16x16x16x27x27 17 / 35, 16x64x64x27x27 36 / 38;  R = 65 (padded to 128)
-//     32x16x16x56x56 123 / 169, 64x16x16x7x7 27 / 23;  R = 128 32x16x16x28x28 65 / 57
-//   backward from the saved plane  R = 64, with the forward: 64x16x16x14x14 37 / 51, 4x16x16x56x56 46 / 42
-//   three-factor convolution, whose other kernels contract the channels twice: with the forward R = 32 32x64x64x56x56
-//     233 / 179, 16x64x64x27x27 45 / 54, 32x64x64x28x28 76 / 78; R = 64 16x16x16x27x27 35 / 53, 64x16x16x32x32 124 / 112;
-//     R = 16 64x512x512x7x7 121 / 94.  Its factor gradients alone: R = 32 32x64x64x28x28 31 / 40, 4x80x80x56x56 about 30 / 23
+// channels to tiles of 64.  Measured on the device, tile or row kernels / products, us, shapes N x C x T x H x W:
+//   convolution  R = 128: 32x64x64x56x56 246 / 131, 8x256x256x14x14 128 / 23, 64x32x32x63x61 323 / 262, but 32x8x8x63x61 74 / 114
+//     R = 100: 16x8x8x27x27 19 / 23;  R = 65: 16x8x8x27x27 16 / 21, 16x16x16x27x27 19 / 21
+//     R = 64: 8x256x256x14x14 60 / 23, 64x512x512x7x7 51 / 29, 32x64x64x56x56 86 / 74, 32x128x128x28x28 42 / 38, but
+//       32x128x32x28x28 27 / 35
+//     R = 32: 8x256x256x14x14 27 / 15, 64x512x512x7x7 29 / 23, 1x512x512x7x7 17 / 15
+//   training step  R = 128: 32x8x8x63x61 399 / 357;  R = 64: 32x16x16x28x28 69 / 49, but 64x8x8x14x14 37 / 41
+//     R = 32: 64x256x256x14x14 102 / 69, 64x512x512x7x7 93 / 53, 16x256x384x27x27 109 / 91
+//     R = 8: 64x512x512x7x7 58 / 42
+//   factor gradients alone  R = 64: 64x16x16x7x7 15 / 21, 32x16x16x28x28 37 / 42, but 32x24x24x28x28 56 / 44; with the tile
+//     kernel's 9x9 tiles in one full round 16x16x16x27x27 18 / 35, 16x64x64x27x27 37 / 39;  R = 65 (padded to 128)
+//     32x16x16x56x56 123 / 169, 64x16x16x7x7 27 / 23;  R = 128: 32x16x16x28x28 73 / 64
+//   layer, forward and backward from the saved plane  R = 64: 64x16x16x14x14 37 / 52, 16x64x64x27x27 62 / 71, but
+//     4x16x16x56x56 56 / 51;  R = 50: 16x256x384x27x27 207 / 148
+//   three-factor layer, whose other kernels contract the channels twice  R = 64: 16x16x16x27x27 35 / 56, 64x16x16x32x32 125 / 113;
+//     R = 32: 32x64x64x56x56 222 / 158, 16x64x64x27x27 45 / 53;  R = 16: 64x512x512x7x7 117 / 52, 32x256x256x63x61 724 / 446;
+//     R = 4: 32x256x256x63x61 507 / 384.  Its factor gradients alone  R = 32: 32x64x64x28x28 31 / 41, 4x96x96x56x56 47 / 37
 const bool g_planes = [] {
   const char* e = getenv("B200CP_PLANES");
   return !(e && e[0] == '0');
