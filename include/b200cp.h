@@ -49,7 +49,11 @@ enum {
   B200CP_PATH_TC3X = 2,   /* tcgen05 kind::tf32, 3-term split (fp32-grade accuracy) */
   B200CP_PATH_TC1X = 3,   /* tcgen05 kind::tf32, single pass (about 1e-3 relative)  */
   B200CP_PATH_MMA = 4,    /* warp-level mma.sync tf32, 3-term split (fp32-grade)    */
-  B200CP_PATH_MASK = 7
+  B200CP_PATH_MASK = 7,
+  /* Reshaped-CP and dense layers, forward and data gradient: the product with the multiplied-out weight may also run on the
+   * tensor cores (scaled fp16 hi / lo operands: 22 bits, sums as accurate as fp32 ones).  Set in the workspace query and in
+   * the call.  Without it these products are FFMA only. */
+  B200CP_TENSOR_PRODUCTS = 8
 };
 
 /* ---- CP4 conv2d ------------------------------------------------------- */

@@ -1055,9 +1055,8 @@ int b200cp_rcp_fwd(int N, int H, int W, int order, const int* cdims, const int* 
 
 size_t b200cp_rcp_fwd_workspace_bytes(int N, int H, int W, int order, const int* cdims, const int* tdims, int R,
                                       int FH, int FW, int flags) {
-  (void)flags;
   if (order < 1 || order > 4 || !cdims || !tdims) return 0;
-  return rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, false);
+  return rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, false, flags);
 }
 
 int b200cp_rcp_fwd_ws(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -1067,12 +1066,11 @@ int b200cp_rcp_fwd_ws(int N, int H, int W, int order, const int* cdims, const in
   if (int rc = check_modes("b200cp_rcp_fwd_ws", order, cdims, tdims, A)) return rc;
   if (int rc = check_ptrs("b200cp_rcp_fwd_ws", {X, S, V})) return rc;
   return rcp_product_launch(N, H, W, order, cdims, tdims, R, FH, FW, X, A, S, V, false, workspace, workspace_bytes,
-                            static_cast<cudaStream_t>(stream));
+                            static_cast<cudaStream_t>(stream), flags);
 }
 
 size_t b200cp_rcp_bwd_workspace_bytes(int N, int H, int W, int order, const int* cdims, const int* tdims, int R,
                                       int FH, int FW, int flags) {
-  (void)flags;
   if (order < 1 || order > 4 || !cdims || !tdims || FH < 1 || FW < 1) return 0;
   size_t C = 1, T = 1;
   for (int k = 0; k < order; ++k) { C *= (size_t)cdims[k]; T *= (size_t)tdims[k]; }
@@ -1080,7 +1078,7 @@ size_t b200cp_rcp_bwd_workspace_bytes(int N, int H, int W, int order, const int*
   const size_t gemm = dense_grad_scratch_floats(N, (int)T, (int)C, H, W, FH, FW);
   const size_t contr = contract_scratch_floats(order, cdims, tdims, R, FH * FW, true);
   return std::max((T * C * FH * FW + std::max(gemm, contr)) * sizeof(float),
-                  rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, true));
+                  rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, true, flags));
 }
 
 int b200cp_rcp_bwd(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -1090,7 +1088,7 @@ int b200cp_rcp_bwd(int N, int H, int W, int order, const int* cdims, const int* 
   if (int rc = check_ptrs("b200cp_rcp_bwd", {dV, S})) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dX) {
-    if (int rc = rcp_product_launch(N, H, W, order, cdims, tdims, R, FH, FW, dV, A, S, dX, true, workspace, workspace_bytes, st))
+    if (int rc = rcp_product_launch(N, H, W, order, cdims, tdims, R, FH, FW, dV, A, S, dX, true, workspace, workspace_bytes, st, flags))
       return rc;
   }
   if (dA || dS) {
@@ -1208,9 +1206,8 @@ int b200cp_dense_fwd(int B, int order, const int* idims, const int* odims, int R
 }
 
 size_t b200cp_dense_fwd_workspace_bytes(int B, int order, const int* idims, const int* odims, int R, int flags) {
-  (void)flags;
   if (order < 1 || order > 4 || !idims || !odims) return 0;
-  return dense_product_workspace(B, order, idims, odims, R, false);
+  return dense_product_workspace(B, order, idims, odims, R, false, flags);
 }
 
 int b200cp_dense_fwd_ws(int B, int order, const int* idims, const int* odims, int R, const float* X,
@@ -1219,17 +1216,16 @@ int b200cp_dense_fwd_ws(int B, int order, const int* idims, const int* odims, in
   if (int rc = check_modes("b200cp_dense_fwd_ws", order, idims, odims, F)) return rc;
   if (int rc = check_ptrs("b200cp_dense_fwd_ws", {X, Y})) return rc;
   return dense_product_launch(B, order, idims, odims, R, X, F, Y, false, workspace, workspace_bytes,
-                              static_cast<cudaStream_t>(stream));
+                              static_cast<cudaStream_t>(stream), flags);
 }
 
 size_t b200cp_dense_bwd_workspace_bytes(int B, int order, const int* idims, const int* odims, int R, int flags) {
-  (void)flags;
   if (order < 1 || order > 4 || !idims || !odims) return 0;
   size_t I = 1, O = 1;
   for (int k = 0; k < order; ++k) { I *= (size_t)idims[k]; O *= (size_t)odims[k]; }
   const size_t gemm = dense_grad_scratch_floats(B, (int)O, (int)I, 1, 1, 1, 1);
   const size_t contr = contract_scratch_floats(order, idims, odims, R, 1, false);
-  return std::max((I * O + std::max(gemm, contr)) * sizeof(float), dense_product_workspace(B, order, idims, odims, R, true));
+  return std::max((I * O + std::max(gemm, contr)) * sizeof(float), dense_product_workspace(B, order, idims, odims, R, true, flags));
 }
 
 int b200cp_dense_bwd(int B, int order, const int* idims, const int* odims, int R, const float* X, const float* dY,
@@ -1239,7 +1235,7 @@ int b200cp_dense_bwd(int B, int order, const int* idims, const int* odims, int R
   if (int rc = check_ptrs("b200cp_dense_bwd", {dY})) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dX) {
-    if (int rc = dense_product_launch(B, order, idims, odims, R, dY, F, dX, true, workspace, workspace_bytes, st)) return rc;
+    if (int rc = dense_product_launch(B, order, idims, odims, R, dY, F, dX, true, workspace, workspace_bytes, st, flags)) return rc;
   }
   if (dF) {
     if (!X) return fail(B200CP_ERR_INVALID_ARG, "b200cp_dense_bwd: X is needed for dF");

@@ -220,10 +220,11 @@ int dense_fast_launch(int B, const int* fsi, const int* fso, int R, const float*
 int dense_chain_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
                        const float* const* F, float* Y, bool transposed, cudaStream_t st);
 // The two layers by their multiplied-out weight (kron_small.cu).  Weight: W[slow][ld] or, with S, W[slow][tap][ld];
-// slow = inputs and fast = outputs, or the other way round (taps reversed) with `transposed`.
+// slow = inputs and fast = outputs, or the other way round with `transposed`; `flip`: taps back to front.
 int kron_weight_ld(int fast);
+double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed);
 int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
-                       int taps, bool transposed, float* W, cudaStream_t st);
+                       int taps, bool transposed, bool flip, float* W, cudaStream_t st);
 // Estimated microseconds of the factored form (negative: it does not take the sizes; above `enough` any value above that
 // will do) and of the multiplied-out one.
 double rcp_factored_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -235,21 +236,23 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
 int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, float* V, cudaStream_t st);
 // Y = X M (dense) and V = K * X (reshaped-CP conv), or their data gradients (`transposed`), by the form that is
 // fastest for the sizes (product.cu); the workspace may be null (or too small): then the factored kernels run.
-size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed);
+size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed, int flags);
 int dense_product_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
-                         const float* const* F, float* Y, bool transposed, void* ws, size_t ws_bytes, cudaStream_t st);
+                         const float* const* F, float* Y, bool transposed, void* ws, size_t ws_bytes, cudaStream_t st,
+                         int flags);
 size_t rcp_product_workspace(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
-                             bool transposed);
+                             bool transposed, int flags);
 int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                        const float* X, const float* const* A, const float* S, float* V, bool transposed, void* ws,
-                       size_t ws_bytes, cudaStream_t st);
+                       size_t ws_bytes, cudaStream_t st, int flags);
 // argument checks the factored kernels make (order, mode sizes, rank, filter)
 int check_kron_modes(int order, const int* idims, const int* odims, int R, const char* who);
 // G[tap][t][c] = sum_{n,h,w} dV[n,t,h,w] * Xpad[n,c,h+y,w+x]; scratch holds dense_grad_scratch_floats() floats
 size_t dense_grad_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);
 int dense_grad_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
                       float* scratch, cudaStream_t st);
-// tcgen05 form of the flat gradient GEMM (G[M][N] = A^T B, A [K][M], B [K][N]); three-term tf32 split, fp32-grade
+// tcgen05 products (gemm_tc.cu; scaled fp16 hi / lo operands, fp32-grade).  Gradient product: G[M][N] = A^T B, A [K][M], B [K][N]
+int gemm_tc_mode();   // 0 off, 1 by the rules, 2 always
 bool gemm_tc_supported(int K, int M, int N);
 size_t gemm_tc_scratch_floats(int K, int M, int N);
 int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st);
@@ -259,6 +262,16 @@ bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW);
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
                         float* scratch, cudaStream_t st);
+// products with the multiplied-out weight: Y[B][N] = X[B][K] W^T (W [N][ldw]), and the 3x3 convolution with W [T][9][ldw]
+bool dense_tc_takes();
+double dense_tc_us(int B, int K, int N);
+size_t dense_tc_scratch_floats(int B, int K, int N);
+int dense_tc_launch(int B, int K, int N, const float* X, const float* W, int ldw, float* Y, float* scratch, cudaStream_t st);
+bool conv_tc_takes(int N, int C, int T, int H, int W);
+double conv_tc_us(int N, int C, int T, int H, int W);
+size_t conv_tc_scratch_floats(int N, int C, int T, int H, int W);
+int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, int ldw, float* V, float* scratch,
+                   cudaStream_t st);
 // the reference's "rebuild" variants: dense conv2d forward with an undecomposed filter K [T][C][FH][FW]; recomposed
 // weights of the dense ([I][O]) and reshaped-CP ([T][C][FH][FW], S != nullptr) layers; Y = X M for the dense layer
 bool conv_dense_supported(const b200cp_tensor_shape& s);

@@ -1,18 +1,28 @@
-// G[m][n] = sum_k A[k][m] * B[k][n] on the tcgen05 tensor cores with fp32-grade accuracy: the gradient GEMM of the CP
-// dense layer (G = dY^T X: A = dY [batch][out], B = X [batch][in], K = batch), which is the one GEMM-shaped step
-// of the hot path large enough to keep a 128 x 256 tile busy.
+// D[m][n] = sum_k A[m][k] B[n][k] on the tcgen05 tensor cores with the accuracy of fp32 sums: the gradient product of the
+// CP dense layer and of the reshaped-CP convolution, and the product of either layer with its multiplied-out weight.
 //
-// Both operands are "MN-major" (contiguous along m / n, K = rows), which tcgen05 takes directly for tf32:
-//   * a first pass splits each operand once into hi = tf32(x) and lo = x - hi (two planes per operand),
-//   * TMA streams 16-row slabs of the four planes into shared memory (32-float boxes, 128-byte span with
-//     32-byte swizzle atoms -- the only MN-major tf32 layout), four stages deep,
-//   * one thread issues, per 8 rows of K and per 128-row half of the 256 x 256 tile, the three products
-//     hi*hi + lo*hi + hi*lo as 128 x 256 x 8 tcgen05.mma into two fp32 accumulators in TMEM (2 x 256 columns),
-//   * four warps read the finished accumulators out of TMEM and store the tile.
-// The kernel is bound by the L2 -> shared-memory stream of the operand planes (8 bytes per element and K row),
-// which is why the tile is as large as TMEM allows: 256 x 256 moves a third less per product than 128 x 256.
-// Roles (TMA warp, MMA warp, four read-out warps) meet only through mbarriers; every wait is bounded and a
-// wait that runs out sets a status word and lets the CTA leave through its normal exit (TMEM released).
+// Accuracy.  A value x is scaled by a power of two (exact) so that the largest of its row is in [2^14, 2^15), and split into
+// hi = fp16(x), lo = fp16(x - hi): 22 bits, down to 2^-18 of the row's largest value; smaller values have an absolute
+// error of 2^-40 of it.  The product is hi*hi + hi*lo + lo*hi (three tcgen05.mma.kind::f16; a tf32 split has the same 22
+// bits at half the rate).  The tensor core cuts its fp32 sums off instead of rounding them, which over thousands of terms
+// is a bias of 1e-5 (4096 terms in one accumulator: 2.9e-5 against float64 in the factor gradients).  So an accumulator
+// holds 64 or 32 terms, the small products first, and is then added to a total in registers, in fp32 with rounding.
+//
+// Layout.  A pair of CTAs (cta_group::2) forms a 256 x BN tile: each loads its 128 rows of A and half of the columns of B,
+// 64 KB a step for 3 x 128 x 256 x 64 multiply-adds.  With one CTA per 128 x 256 tile it would be 96 KB, and the
+// stream from L2 is what bounds such a kernel.  TMA fills a ring of three or four stages, one thread of the pair issues the
+// products into two accumulators in turn, and the other warps of each CTA move the other accumulator to the totals meanwhile
+// (the totals are half of the register file: that is what ends the tile at 128 x 256 per CTA).  The pairs are persistent: the
+// totals of a tile are stored while the products of the next have begun.
+// Operands: K-major ([row][k], 64 k = one 128-byte swizzled row) or MN-major ([k][row], boxes of 64 rows), both taken by
+// tcgen05 directly, so that neither the batch-major activations of a gradient nor the weight are transposed in memory.
+// Measured, 4096 x 4096 x 4096: 305 to 335 us = 1.35 to 1.23 PFLOP/s of fp16 products, where cuBLAS sustains 1.40 under the power
+// cap (tf32 planes and one accumulator over all of K: 671 us, and 100 times the error).  Without the cut of the last round of
+// tiles 348 us; with eight read-out warps of 128 columns instead of sixteen 317 against 307.
+// Roles (TMA warp, MMA warp, read-out warps) meet only through mbarriers; every wait is bounded, and a wait that
+// runs out sets a status word and lets the CTA leave through its normal exit (TMEM released).
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -28,28 +38,111 @@ namespace {
 
 using namespace tc;
 
-constexpr int kBM = 256, kBN = 256, kKS = 16;          // tile and the K rows of one stage
-constexpr int kMH = kBM / 128;                         // accumulators (tcgen05.mma has M = 128 per CTA)
-constexpr int kStages = 3;
-constexpr int kGroupBytes = kKS * 128;                 // one TMA box: 32 floats x kKS rows
-constexpr int kAPlane = (kBM / 32) * kGroupBytes;      // 16 KB
-constexpr int kBPlane = (kBN / 32) * kGroupBytes;      // 16 KB
-constexpr int kStageBytes = 2 * (kAPlane + kBPlane);   // A hi, A lo, B hi, B lo = 64 KB
-constexpr int kTmemCols = kMH * kBN;                   // 512: all of TMEM (one CTA per SM by its shared memory)
-constexpr int kThreads = 192;                          // warp 0 TMA, warp 1 MMA, warps 2..5 read-out
-constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024 + 256;
+constexpr int kBM = 256;              // rows of a pair's tile: 128 per CTA
+constexpr int kKS = 64;               // K of one step: 128 bytes of fp16
+constexpr int kRowShift = 24;         // see SplitGemm::ea
+constexpr int kAPlane = 128 * 128;    // bytes of one plane (hi or lo) of A in a stage
 
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+template <int BN>
+struct Tile {
+  static constexpr int bplane = BN / 2 * 128;
+  static constexpr int stage = 2 * (kAPlane + bplane);                  // 64, 48, 40 KB
+  static constexpr int stages = BN == 256 ? 3 : BN == 128 ? 4 : 5;
+  static constexpr int depth = BN == 256 ? 2 : 4;                       // accumulators
+  static constexpr int tmem_cols = depth * BN;                          // 512, 512, 256
+  static constexpr int cols = BN == 64 ? 32 : 64;                       // of a read-out warp
+  static constexpr int readers = 4 * BN / cols;                         // read-out warps: 16, 8, 8
+  static constexpr int threads = 64 + 32 * readers;                     // warp 0 TMA, warp 1 MMA, the others read-out
+  static constexpr size_t smem = (size_t)stages * stage + 1024 + 256;
+};
+
+struct SplitGemm {
+  int M, N;
+  int tiles_m, tiles_n;          // tiles of one result (a weight gradient has one result per tap)
+  // Work units in the order in which the pairs take them: `whole` tiles with all K steps, as many as fill the pairs an
+  // integer number of times, then the tiles left over, each cut into `splits` ranges of `steps` K steps.
+  int whole, units, splits, steps, total;
+  int group;                     // K of an accumulator, in instructions of 16 (see kShortSum)
+  int kc, Kc;                    // K-major: steps and channels per tap (dense: one tap); MN-major: Kc = rows of K
+  int FW, padH, padW, Wp;        // a filter tap (y, x) shifts the rows of A by (y - padH) * Wp + (x - padW)
+  // A value of A stands for 2^ea of itself, one of B for 2^eb.  Rows of A with one exponent over all of K: added at the end.
+  // In a convolution the row that a step reads moves with the tap, so the totals take 2^(ea - 24) of each step and
+  // 2^(eb + 24) at the end: 24 binades for sums of values near the largest float.
+  const int *ea, *eb;
+  float* out;                    // entry (m, n) of result p at out + p * result + off(m) + n * ldn
+  size_t result;
+  float* partial;                // [unit - whole][BN][256] sums of the cut tiles, without the exponents
+  long ldm, ldn;                 // off(m) = m * ldm, or, for the pixels of a convolution:
+  int vec;                       // ldn == 1 and 16-byte rows
+  int H, W, PP;                  // rows are n * PP + h * Wp + w; off = (n * N * H + h) * W + w, ring pixels have none
+};
+
+// ---- PTX of a CTA pair --------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// the same shared variable in the leader CTA of the pair
+__device__ __forceinline__ uint32_t leader_addr(uint32_t p) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(p), "r"(0));
+  return r;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// into this CTA's shared memory, counted on a barrier of either CTA of the pair (no multicast)
+__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
+      "[%2];" ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(0)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void mma_f16_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+      : "memory");
+}
+// one arrival on the barrier of both CTAs when the products issued so far have completed
+__device__ __forceinline__ void commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"((uint16_t)3)
+      : "memory");
+}
+// registers -> TMEM: 16 columns of the warp's lane quarter
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"f"(v[0]),
+      "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]),
+      "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "r"(taddr)
       : "memory");
 }
 
-// Bounded wait shared by the roles: gives up after about a second, or as soon as another role has given up.
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  const uint32_t a = smem_u32(bar);
-  const long long t0 = clock64();
+// Instruction descriptor for kind::f16 with fp16 operands and fp32 accumulation, M = 256 (a pair).
+__host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n, uint32_t mn) {
+  return (1u << 4) | (mn << 15) | (mn << 16) | ((n >> 3) << 17) | ((256u >> 4) << 24);
+}
+
+// Bounded wait shared by the roles: gives up after about a second, or as soon as another role of the CTA has given up.
+// (Shared-memory addresses in 32 bits: the read-out warps have no register to spare.)
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
+  long long t0 = 0;
   for (int it = 0;; ++it) {
     uint32_t done;
     asm volatile(
@@ -59,335 +152,962 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
         "selp.u32 %0, 1, 0, p;\n"
         "}\n"
         : "=r"(done)
-        : "r"(a), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     if (done) return true;
     if ((it & 31) == 31) {
-      if (*abort_flag) return false;
+      uint32_t given_up;
+      asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(given_up) : "r"(abort_flag) : "memory");
+      if (given_up) return false;
+      if (t0 == 0) t0 = clock64();
       if (clock64() - t0 > 1500000000ll) {
-        *abort_flag = 1;
+        asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_flag), "r"(1) : "memory");
         return false;
       }
     }
   }
 }
 
-// hi = tf32(x) (round to nearest), lo = x - hi (exact); n4 = number of float4
-__global__ void __launch_bounds__(256) split_tf32_kernel(const float4* __restrict__ src, float4* __restrict__ hi,
-                                                         float4* __restrict__ lo, size_t n4) {
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
-    const float4 v = __ldg(src + i);
-    float4 h, d;
-    h.x = tf32_hi(v.x); h.y = tf32_hi(v.y); h.z = tf32_hi(v.z); h.w = tf32_hi(v.w);
-    d.x = v.x - h.x; d.y = v.y - h.y; d.z = v.z - h.z; d.w = v.w - h.w;
-    hi[i] = h;
-    lo[i] = d;
-  }
+// 2^e for e in [-126, 127]
+__device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
+// v * 2^e for e in [-252, 254], in two steps of the same sign
+__device__ __forceinline__ float scale_by(float v, int e) {
+  const int h = e >> 1;
+  return v * exp2_int(h) * exp2_int(e - h);
 }
 
-struct GemmTcGeom {
-  int M, N, K;
-  int NS;            // stages of kKS rows per CTA (per K split)
-  int splits;        // blockIdx.z = tap * splits + split; the tile goes to G + (split * taps + tap) * M * N
-  int taps, FW, padH, padW, Wp;  // conv form: the B rows of tap (y, x) are shifted by (y - padH) * Wp + (x - padW)
+__device__ __forceinline__ int tap_shift(const SplitGemm& g, int tap);
+struct UnitAt {
+  int m0, n0, tap, shift, first, nsteps;   // tap of the result; shift: of the rows of A (MN-major), by that tap
 };
-
-// NCHW -> [n][padded pixel][channel] hi / lo planes with a zero ring of (padH, padW) pixels: the layout in which a
-// filter tap is a shift of the row index, which TMA takes at any value (only the contiguous coordinate has an
-// alignment rule).  grid = (pixel tiles, channel tiles, N), block = (32, 8).
-__global__ void __launch_bounds__(256) pad_transpose_split_kernel(const float* __restrict__ src, float* __restrict__ hi,
-                                                                  float* __restrict__ lo, int CH, int H, int W,
-                                                                  int padH, int padW) {
-  __shared__ float tile[32][33];
-  const int Hp = H + 2 * padH, Wp = W + 2 * padW, PP = Hp * Wp;
-  const int n = blockIdx.z, p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  {
-    const int p = p0 + tx, ph = p / Wp, pw = p - ph * Wp;
-    const int h = ph - padH, w = pw - padW;
-    const bool in = p < PP && h >= 0 && h < H && w >= 0 && w < W;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = c0 + ty + 8 * j;
-      tile[ty + 8 * j][tx] = (in && c < CH) ? __ldg(src + (((size_t)n * CH + c) * H + h) * W + w) : 0.f;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int p = p0 + ty + 8 * j, c = c0 + tx;
-    if (p < PP && c < CH) {
-      const float v = tile[tx][ty + 8 * j];
-      const float h = tf32_hi(v);
-      const size_t o = ((size_t)n * PP + p) * CH + c;
-      hi[o] = h;
-      lo[o] = v - h;
-    }
+template <int BN, bool MN>
+__device__ __forceinline__ UnitAt unit_at(const SplitGemm& g, int unit) {
+  UnitAt t;
+  const int v = unit - g.whole, tile = v < 0 ? unit : g.whole + v / g.splits;
+  const int per = g.tiles_m * g.tiles_n, r = tile % per;
+  t.tap = tile / per;
+  t.n0 = (r / g.tiles_m) * BN;
+  t.m0 = (r % g.tiles_m) * kBM;
+  t.shift = MN ? tap_shift(g, t.tap) : 0;
+  t.first = v < 0 ? 0 : (v % g.splits) * g.steps;
+  t.nsteps = v < 0 ? g.total : min(g.steps, g.total - t.first);
+  return t;
+}
+// Where a step of a unit is in K: its tap (of the sum over taps of a convolution) and its place in the tap.
+struct StepAt {
+  int tap, c;
+};
+template <bool CONV>
+__device__ __forceinline__ StepAt step_at(const SplitGemm& g, int k) {
+  const int tap = CONV ? k / g.kc : 0;
+  return StepAt{tap, k - tap * g.kc * (CONV ? 1 : 0)};
+}
+template <bool CONV>
+__device__ __forceinline__ void next_step(const SplitGemm& g, StepAt& k) {
+  if (++k.c == g.kc && CONV) {
+    k.c = 0;
+    ++k.tap;
   }
 }
+// instructions of 16 k of a step
+__device__ __forceinline__ int k16_of(const SplitGemm& g, int c) {
+  const int left = g.Kc - c * kKS;
+  return left >= kKS ? kKS / 16 : (left + 15) / 16;
+}
+__device__ __forceinline__ int tap_shift(const SplitGemm& g, int tap) {
+  const int y = tap / g.FW;
+  return (y - g.padH) * g.Wp + (tap - y * g.FW - g.padW);
+}
+// where row m of a result begins, and whether it has one (a convolution's ring pixels have none)
+template <bool CONV>
+__device__ __forceinline__ bool row_at(const SplitGemm& g, int m, long* off) {
+  bool in = m < g.M;
+  *off = (long)m * g.ldm;
+  if (CONV) {
+    const int n = m / g.PP, p = m - n * g.PP, h = p / g.Wp, w = p - h * g.Wp;
+    in = in && h < g.H && w < g.W;
+    *off = ((long)n * g.N * g.H + h) * g.W + w;
+  }
+  return in;
+}
 
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_kernel(const GemmTcGeom g, const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUtensorMap mAlo,
-               const __grid_constant__ CUtensorMap mBhi, const __grid_constant__ CUtensorMap mBlo,
-               float* __restrict__ G) {
+template <int BN, bool MN, bool CONV>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Tile<BN>::threads, 1)
+split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ CUtensorMap mapA,
+                  const __grid_constant__ CUtensorMap mapB) {
+  using T = Tile<BN>;
+  constexpr int kStages = T::stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kStages * kStageBytes);
-  uint64_t* full = bars;               // [kStages] TMA landed                     (tx bytes)
-  uint64_t* empty = full + kStages;    // [kStages] MMAs that read the stage done  (commit)
-  uint64_t* accfull = empty + kStages; // accumulator complete                     (commit)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfull + 1);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kStages * T::stage);
+  uint64_t* full = bars;                 // [kStages] the leader's: the stage of both CTAs has landed  (tx bytes)
+  uint64_t* empty = full + kStages;      // [kStages] the products that read the stage are done         (commit, both CTAs)
+  uint64_t* accfull = empty + kStages;   // [depth] the accumulator is complete                         (commit, both CTAs)
+  uint64_t* accfree = accfull + 4;       // [depth] the leader's: read out by the warps of both CTAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * kBM;
-  const int tap = blockIdx.z / g.splits, split = blockIdx.z - tap * g.splits;
-  const int k0 = split * g.NS * kKS;
-  const int bshift = (tap / g.FW - g.padH) * g.Wp + (tap % g.FW - g.padW);
-  G += ((size_t)split * g.taps + tap) * g.M * g.N;
+  const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
-    mbar_init(accfull, 1);
+    for (int i = 0; i < T::depth; ++i) {
+      mbar_init(&accfull[i], 1);
+      mbar_init(&accfree[i], 2 * T::readers);
+    }
     *abort_flag = 0;
     fence_barrier_init();
-    tma_prefetch_desc(&mAhi);
-    tma_prefetch_desc(&mAlo);
-    tma_prefetch_desc(&mBhi);
-    tma_prefetch_desc(&mBlo);
+    tma_prefetch_desc(&mapA);
+    tma_prefetch_desc(&mapB);
   }
-  if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, T::tmem_cols);
   tc_fence_before_sync();
   __syncthreads();
+  cluster_sync();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  const uint32_t fullb = smem_u32(full), emptyb = smem_u32(empty), accfullb = smem_u32(accfull), accfreeb = smem_u32(accfree),
+                 abortb = smem_u32(const_cast<int*>(abort_flag));
+  grid_dependency_wait();   // the operand planes
 
   if (warp == 0) {
-    // ================= TMA producer =====================================================================
+    // ================= TMA producer: this CTA's rows of A and its half of the columns of B ==================================
     if (lane == 0) {
-      for (int s = 0; s < g.NS; ++s) {
-        const int slot = s % kStages;
-        if (s >= kStages && !wait_or_abort(&empty[slot], ((s / kStages) - 1) & 1, abort_flag)) break;
-        uint8_t* dst = sm + slot * kStageBytes;
-        mbar_expect_tx(&full[slot], kStageBytes);
-        const int k = k0 + s * kKS;  // rows past K (and shifted rows outside the tensor) read as zero
+      int it = 0;
+      bool ok = true;
+      for (int unit = pair; unit < g.units && ok; unit += npairs) {
+        const UnitAt t = unit_at<BN, MN>(g, unit);
+        StepAt k = step_at<CONV>(g, t.first);
+        for (int s = 0; s < t.nsteps; ++s, ++it, next_step<CONV>(g, k)) {
+          const int slot = it % kStages;
+          if (it >= kStages && !(ok = wait_or_abort(emptyb + slot * 8, ((it / kStages) - 1) & 1, abortb))) break;
+          if (rank == 0) mbar_expect_tx(&full[slot], 2 * T::stage);
+          const uint32_t bar = leader_addr(fullb + slot * 8);
+          const uint32_t a = smem_u32(sm) + slot * T::stage, b = a + 2 * kAPlane;
+          if (MN) {   // boxes of 64 rows x 64 k, both planes; rows of K outside the tensor read as zero
 #pragma unroll
-        for (int grp = 0; grp < kBM / 32; ++grp) {
-          tma_load_2d(dst + grp * kGroupBytes, &mAhi, &full[slot], m0 + grp * 32, k);
-          tma_load_2d(dst + kAPlane + grp * kGroupBytes, &mAlo, &full[slot], m0 + grp * 32, k);
-        }
+            for (int q = 0; q < 2; ++q)
+              tma_load_pair(a + q * kAPlane, &mapA, bar, t.m0 + rank * 128 + q * 64, k.c * kKS + t.shift, 0);
 #pragma unroll
-        for (int grp = 0; grp < kBN / 32; ++grp) {
-          tma_load_2d(dst + 2 * kAPlane + grp * kGroupBytes, &mBhi, &full[slot], n0 + grp * 32, k + bshift);
-          tma_load_2d(dst + 2 * kAPlane + kBPlane + grp * kGroupBytes, &mBlo, &full[slot], n0 + grp * 32, k + bshift);
+            for (int q = 0; q < BN / 128; ++q)
+              tma_load_pair(b + q * kAPlane, &mapB, bar, t.n0 + rank * (BN / 2) + q * 64, k.c * kKS, 0);
+          } else {    // boxes of 64 k x the rows, both planes; channels past Kc read as zero
+            const int shift = CONV ? tap_shift(g, k.tap) : 0;
+            tma_load_pair(a, &mapA, bar, k.c * kKS, 0, t.m0 + rank * 128 + shift);
+            tma_load_pair(b, &mapB, bar, k.c * kKS, k.tap, t.n0 + rank * (BN / 2));
+          }
         }
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer ========================================================================
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_tf32(kBN, 1, 1);
-      // MN-major tf32 operand: rows of 32 floats (128 B), one row per k, 32-byte chunks swizzled within groups
-      // of 4 rows.  LBO: next group of 32 columns, SBO: next 4 rows; 8 rows of K per instruction = 1024 bytes.
-      const uint64_t d0 = make_smem_desc(0, kGroupBytes, 512, kSwizzle128B_32B);
+    // ================= MMA issuer: one thread of the pair ====================================================================
+    if (rank == 0 && lane == 0) {
+      const uint32_t idesc = make_idesc_f16(BN, MN ? 1 : 0);
+      // K-major: rows of 128 bytes, 8 rows per swizzle atom (SBO 1024); 16 k = 32 bytes on.
+      // MN-major: 64 rows of the operand (128 bytes) per k, 8 k per atom (SBO 1024), the next 64 rows LBO on; 16 k = 2048 bytes on.
+      const uint64_t d0 = make_smem_desc(0, MN ? kAPlane : 16, 1024, kSwizzle128B);
+      constexpr uint32_t kstep = MN ? 2048 : 32;
+      constexpr uint32_t alo = MN ? kAPlane / 2 : kAPlane, blo = MN ? kAPlane / 2 : T::bplane;
       const uint32_t base = smem_u32(sm);
+      int it = 0, gi = 0;   // steps, accumulators
       bool ok = true;
-      for (int s = 0; s < g.NS && ok; ++s) {
-        const int slot = s % kStages;
-        ok = wait_or_abort(&full[slot], (s / kStages) & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint32_t st = base + slot * kStageBytes;
-#pragma unroll
-        for (int kk = 0; kk < kKS / 8; ++kk) {
-          const uint64_t ah = d0 + (uint64_t)((st + kk * 1024) >> 4);
-          const uint64_t al = d0 + (uint64_t)((st + kAPlane + kk * 1024) >> 4);
-          const uint64_t bh = d0 + (uint64_t)((st + 2 * kAPlane + kk * 1024) >> 4);
-          const uint64_t bl = d0 + (uint64_t)((st + 2 * kAPlane + kBPlane + kk * 1024) >> 4);
-#pragma unroll
-          for (int h = 0; h < kMH; ++h) {  // the 128-row halves: 4 groups of 32 columns further on in the A planes
-            const uint64_t ho = (uint64_t)((h * 4 * kGroupBytes) >> 4);
-            mma_tf32_ss(tmem_base + h * kBN, al + ho, bh, idesc, !(s == 0 && kk == 0));
-            mma_tf32_ss(tmem_base + h * kBN, ah + ho, bl, idesc, true);
-            mma_tf32_ss(tmem_base + h * kBN, ah + ho, bh, idesc, true);
+      for (int unit = pair; unit < g.units && ok; unit += npairs) {
+        const UnitAt t = unit_at<BN, MN>(g, unit);
+        StepAt k = step_at<CONV>(g, t.first);
+        for (int s = 0; s < t.nsteps && ok; ++s, ++it, next_step<CONV>(g, k)) {
+          const int slot = it % kStages, kk = k16_of(g, k.c);
+          if (!(ok = wait_or_abort(fullb + slot * 8, (it / kStages) & 1, abortb))) break;
+          tc_fence_after_sync();
+          const uint32_t a = base + slot * T::stage, b = a + 2 * kAPlane;
+          const uint64_t ah = d0 + (a >> 4), al = d0 + ((a + alo) >> 4), bh = d0 + (b >> 4), bl = d0 + ((b + blo) >> 4);
+          for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
+            const int buf = gi % T::depth, i1 = min(kk, i0 + g.group);
+            if (gi >= T::depth && !(ok = wait_or_abort(accfreeb + buf * 8, (gi / T::depth - 1) & 1, abortb))) break;
+            tc_fence_after_sync();
+            const uint32_t d = tmem_base + buf * BN;
+            for (int i = i0; i < i1; ++i) {
+              const uint64_t o = (uint64_t)((i * kstep) >> 4);
+              mma_f16_pair(d, al + o, bh + o, idesc, i > i0);
+              mma_f16_pair(d, ah + o, bl + o, idesc, true);
+            }
+            for (int i = i0; i < i1; ++i) {
+              const uint64_t o = (uint64_t)((i * kstep) >> 4);
+              mma_f16_pair(d, ah + o, bh + o, idesc, true);
+            }
+            commit_pair(accfullb + buf * 8);
           }
+          if (!ok) break;
+          commit_pair(emptyb + slot * 8);
         }
-        mma_commit(&empty[slot]);
       }
-      if (ok) mma_commit(accfull);
     }
   } else {
-    // ================= read-out: TMEM -> global ===========================================================
-    const int qd = warp & 3;  // the TMEM lane quarter this warp may read
-    if (wait_or_abort(accfull, 0, abort_flag)) {
-      tc_fence_after_sync();
-#pragma unroll 1
-      for (int hc = 0; hc < kMH * (kBN / 16); ++hc) {
-        const int h = hc / (kBN / 16), c = hc % (kBN / 16);
-        const int m = m0 + h * 128 + qd * 32 + lane;
-        float* dst = G + (size_t)m * g.N + n0;
-        float v[16];
-        tmem_ld16(tmem_base + ((uint32_t)(qd * 32) << 16) + h * kBN + c * 16, v);
-        if (m < g.M) {
-          if (n0 + c * 16 + 16 <= g.N) {
+    // ================= read-out: accumulators -> totals -> global =============================================================
+    constexpr int NC = T::cols;
+    const int qd = warp & 3, c0 = ((warp - 2) >> 2) * NC;   // the TMEM lane quarter this warp may read, and its columns
+    const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + c0;
+    int gi = 0;
+    bool ok = true;
+    for (int unit = pair; unit < g.units && ok; unit += npairs) {
+      float tot[NC];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              *reinterpret_cast<float4*>(dst + c * 16 + i * 4) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          } else {
+      for (int j = 0; j < NC; ++j) tot[j] = 0.f;
+      int buf = 0;
+      {
+        const UnitAt t = unit_at<BN, MN>(g, unit);
+        StepAt k = step_at<CONV>(g, t.first);
+        for (int left = t.nsteps; left > 0 && ok; --left, next_step<CONV>(g, k)) {
+          float f = 0.f;
+          if (CONV) {
+            const int px = t.m0 + rank * 128 + qd * 32 + lane + tap_shift(g, k.tap);
+            if (px >= 0 && px < g.M) f = exp2_int(__ldg(g.ea + px) - kRowShift);
+          }
+          const int kk = k16_of(g, k.c);
+          for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
+            buf = gi % T::depth;
+            if (!(ok = __all_sync(0xffffffffu, wait_or_abort(accfullb + buf * 8, (gi / T::depth) & 1, abortb)))) break;
+            tc_fence_after_sync();
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (n0 + c * 16 + i < g.N) dst[c * 16 + i] = v[i];
+            for (int j0 = 0; j0 < NC; j0 += 16) {
+              float v[16];
+              tmem_ld16(taddr + buf * BN + j0, v);
+              if (j0 + 16 == NC && (left > 1 || i0 + g.group < kk)) {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) arrive_cluster(leader_addr(accfreeb + buf * 8));
+              }
+#pragma unroll
+              for (int j = 0; j < 16; ++j) tot[j0 + j] = CONV ? fmaf(v[j], f, tot[j0 + j]) : tot[j0 + j] + v[j];
+            }
           }
         }
       }
+      if (!ok) break;
+      // The totals go through the accumulator just read, so that a short loop stores them: unrolled over registers the
+      // stores are 30 KB of code that every tile fetches anew: 8 us a tile (4096 x 4096 x 1024: 121 us, now 99).
+#pragma unroll
+      for (int j0 = 0; j0 < NC; j0 += 16) tmem_st16(taddr + buf * BN + j0, tot + j0);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      const UnitAt t = unit_at<BN, MN>(g, unit);   // again: cheaper than registers held through the loop
+      const int row = rank * 128 + qd * 32 + lane, m = t.m0 + row;
+      const bool cut = unit >= g.whole && g.splits > 1;
+      long off = row;
+      bool in = true;
+      if (!cut) in = row_at<CONV>(g, m, &off);
+      const long ldn = cut ? kBM : g.ldn;
+      const int e = cut ? 0 : CONV ? kRowShift : in ? __ldg(g.ea + m) : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
+      float* dst = cut ? g.partial + ((size_t)(unit - g.whole) * BN + c0) * kBM + off
+                       : g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn;
+      const int* eb = g.eb + n0 + (lane & 15);
+      int next = !cut && n0 + (lane & 15) < N ? __ldg(eb) : 0;
+#pragma unroll 1
+      for (int j0 = 0; j0 < NC; j0 += 16) {
+        float v[16];
+        tmem_ld16(taddr + buf * BN + j0, v);
+        const int ebv = next, left = N - n0 - j0;
+        next = !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? __ldg(eb + j0 + 16) : 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
+        if (!CONV && g.vec && !cut) {   // 16-byte stores along a row
+#pragma unroll
+          for (int j = 0; j < 16; j += 4)
+            if (in && j < left) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          dst += 16;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j, dst += ldn)
+            if (in && j < left) *dst = v[j];
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) arrive_cluster(leader_addr(accfreeb + buf * 8));
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 0 && *abort_flag)
-    atomicCAS(&g_gemm_tc_status, 0,
-              (1 << 16) | (((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) & 0xffff));
+  if (tid == 0 && *abort_flag) {
+    atomicCAS(&g_gemm_tc_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
+    const long long t0 = clock64();   // copies in flight land before the shared memory is given back
+    while (clock64() - t0 < 40000000ll) {
+    }
+  }
+  cluster_sync();   // the peer's products read this CTA's shared memory, and its commits arrive on its barriers
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc_pair(tmem_base, T::tmem_cols);
   }
 }
 
-bool enabled() {  // B200CP_GEMM_TC=0 keeps the CUDA-core GEMM (read per call: tests switch it)
-  const char* e = getenv("B200CP_GEMM_TC");
-  return !(e && e[0] == '0');
+// The sums of a cut tile, in the order of K, and the exponents.  grid (cut tiles, BN / 8), one row per
+// thread: enough CTAs to keep the L2 busy (34 tiles cut in two: 24 us with 32 columns per CTA, 6 with 8).
+constexpr int kJoinCols = 8;
+template <int BN, bool MN, bool CONV>
+__global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__ SplitGemm g) {
+  grid_dependency_wait();
+  const UnitAt t = unit_at<BN, MN>(g, g.whole + blockIdx.x * g.splits);
+  const int m = t.m0 + threadIdx.x;
+  long off;
+  if (!row_at<CONV>(g, m, &off)) return;
+  const int e = CONV ? kRowShift : __ldg(g.ea + m);
+  const int n0 = t.n0 + blockIdx.y * kJoinCols;
+  const float* src = g.partial + ((size_t)blockIdx.x * g.splits * BN + blockIdx.y * kJoinCols) * kBM + threadIdx.x;
+  float* dst = g.out + (size_t)t.tap * g.result + off;
+  float v[kJoinCols];
+#pragma unroll
+  for (int j = 0; j < kJoinCols; ++j) v[j] = __ldcs(src + j * kBM);
+  for (int q = 1; q < g.splits; ++q)
+#pragma unroll
+    for (int j = 0; j < kJoinCols; ++j) v[j] += __ldcs(src + ((size_t)q * BN + j) * kBM);
+#pragma unroll
+  for (int j = 0; j < kJoinCols; ++j)
+    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = scale_by(v[j], e + __ldg(g.eb + n0 + j));
 }
 
-int encode_plane(PFN_encodeTiled enc, CUtensorMap* map, const float* base, int cols, int rows) {
-  const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t gstr[1] = {(cuuint64_t)cols * 4};
-  const cuuint32_t box[2] = {32, (cuuint32_t)kKS};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), gdim, gstr, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+// ---- operand planes -----------------------------------------------------------------------------------------------------
+// Exponent e of a row whose largest magnitude has these bits: x * 2^-e is below 2^15.  (Infinities and NaN leave the
+// finite values of their row in range and themselves non-finite.)
+__device__ __forceinline__ int row_exponent(unsigned bits, int least) {
+  return bits == 0 ? 0 : max((int)(bits >> 23) - 141, least);
+}
+constexpr int kLeast = -126, kLeastConv = -100;   // 2^-e and (convolutions) 2^(e - 24) stay normal numbers
+
+struct alignas(8) Half4 {
+  __half2 a, b;
+};
+__device__ __forceinline__ void split4(float4 v, float sc, Half4& hi, Half4& lo) {
+  v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
+  hi.a = __floats2half2_rn(v.x, v.y);
+  hi.b = __floats2half2_rn(v.z, v.w);
+  const float2 p = __half22float2(hi.a), q = __half22float2(hi.b);
+  lo.a = __floats2half2_rn(v.x - p.x, v.y - p.y);
+  lo.b = __floats2half2_rn(v.z - q.x, v.w - q.y);
+}
+__device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned max4(unsigned m, float4 v) {
+  return max(max(max(m, abs_bits(v.x)), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
+}
+// four values from c on of a row of `len`, zero past its end (`vec`: the row is 16-byte aligned)
+__device__ __forceinline__ float4 load4(const float* row, int c, int len, bool vec) {
+  if (vec && c + 4 <= len) return __ldg(reinterpret_cast<const float4*>(row + c));
+  return make_float4(c < len ? __ldg(row + c) : 0.f, c + 1 < len ? __ldg(row + c + 1) : 0.f,
+                     c + 2 < len ? __ldg(row + c + 2) : 0.f, c + 3 < len ? __ldg(row + c + 3) : 0.f);
+}
+
+// Both operands of a product are split in one launch: the CTAs below `first` take the first.
+struct SplitJob {
+  const float* src;
+  int rows, segs, len, ld;   // rows of `segs` segments of `len` values, `ld` apart (columns and pixels: see the kernels)
+  int ldo;                   // of a segment of the planes: a multiple of 8
+  bool vec;
+  __half* hi;
+  size_t plane;
+  int* ex;
+  unsigned* part;            // column / channel maxima, [parts][len]
+  int per, parts;
+};
+struct SplitJobs {
+  SplitJob job[2];
+  int first;
+};
+
+// One exponent per row.  A warp takes a row of up to 512 values, a CTA a longer one; a row of up to 4096 values is read once.
+__global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__ SplitJobs jobs) {
+  constexpr int Q = 4;
+  __shared__ unsigned red[8];
+  grid_dependency_wait();
+  const bool second = (int)blockIdx.x >= jobs.first;
+  const SplitJob& p = jobs.job[second];
+  const int block = blockIdx.x - (second ? jobs.first : 0), segs = p.segs, len = p.len;
+  const bool wide = segs * (long)len > 512;
+  const int tpr = wide ? 256 : 32, sub = wide ? threadIdx.x : threadIdx.x & 31;
+  const int row = wide ? block : block * 8 + (threadIdx.x >> 5);
+  const bool in = row < p.rows;
+  const int quads = (len + 3) / 4, n = in ? segs * quads : 0;
+  const float* s = p.src + (size_t)row * segs * p.ld;
+  float4 v[Q];
+  unsigned mx = 0;
+  auto at = [&](int i) {
+    const int seg = segs == 1 ? 0 : i / quads;
+    return load4(s + (size_t)seg * p.ld, (i - seg * quads) * 4, len, p.vec);
+  };
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    v[q] = q * tpr + sub < n ? at(q * tpr + sub) : make_float4(0.f, 0.f, 0.f, 0.f);
+    mx = max4(mx, v[q]);
+  }
+  for (int i = Q * tpr + sub; i < n; i += tpr) mx = max4(mx, at(i));
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (wide) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = max(mx, red[i]);
+  }
+  const int e = row_exponent(mx, kLeast);
+  const float sc = exp2_int(-e);
+  if (in && sub == 0) p.ex[row] = e;
+  __half* d = p.hi + (size_t)row * segs * p.ldo;
+  auto put = [&](int i, float4 x) {
+    const int seg = segs == 1 ? 0 : i / quads;
+    const size_t o = (size_t)seg * p.ldo + (i - seg * quads) * 4;
+    Half4 h, l;
+    split4(x, sc, h, l);
+    *reinterpret_cast<Half4*>(d + o) = h;
+    *reinterpret_cast<Half4*>(d + p.plane + o) = l;
+  };
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (q * tpr + sub < n) put(q * tpr + sub, v[q]);
+  for (int i = Q * tpr + sub; i < n; i += tpr) put(i, at(i));
+}
+
+// [rows][len] with one exponent per column, in two launches: the largest magnitude per column and range of rows, then the
+// planes.  Block (64, 4): 256 columns, every fourth row.
+__global__ void __launch_bounds__(256) column_max_kernel(const __grid_constant__ SplitJobs jobs) {
+  __shared__ uint4 red[4][64];
+  grid_dependency_wait();
+  const bool second = (int)blockIdx.x >= jobs.first;
+  const SplitJob& p = jobs.job[second];
+  const int cols = p.len, c = (blockIdx.x - (second ? jobs.first : 0)) * 256 + threadIdx.x * 4;
+  const int r0 = blockIdx.y * p.per, r1 = min(p.rows, r0 + p.per);
+  uint4 m = make_uint4(0, 0, 0, 0);
+  if (c < cols)
+#pragma unroll 8
+    for (int r = r0 + threadIdx.y; r < r1; r += 4) {
+      const float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
+      m.x = max(m.x, abs_bits(v.x)); m.y = max(m.y, abs_bits(v.y));
+      m.z = max(m.z, abs_bits(v.z)); m.w = max(m.w, abs_bits(v.w));
+    }
+  red[threadIdx.y][threadIdx.x] = m;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < cols && r0 < r1) {
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      const uint4 o = red[i][threadIdx.x];
+      m.x = max(m.x, o.x); m.y = max(m.y, o.y); m.z = max(m.z, o.z); m.w = max(m.w, o.w);
+    }
+    unsigned* d = p.part + (size_t)blockIdx.y * cols + c;
+    d[0] = m.x;
+    if (c + 1 < cols) d[1] = m.y;
+    if (c + 2 < cols) d[2] = m.z;
+    if (c + 3 < cols) d[3] = m.w;
+  }
+}
+__global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constant__ SplitJobs jobs) {
+  __shared__ float scale[256];
+  grid_dependency_wait();
+  const bool second = (int)blockIdx.x >= jobs.first;
+  const SplitJob& p = jobs.job[second];
+  const int cols = p.len, c0 = (blockIdx.x - (second ? jobs.first : 0)) * 256;
+  const int r0 = blockIdx.y * p.per, r1 = min(p.rows, r0 + p.per);
+  {
+    const int i = threadIdx.y * 64 + threadIdx.x, c = c0 + i;
+    unsigned m = 0;
+    if (c < cols)
+#pragma unroll 8
+      for (int q = 0; q < p.parts; ++q) m = max(m, __ldcg(p.part + (size_t)q * cols + c));
+    const int e = row_exponent(m, kLeast);
+    scale[i] = exp2_int(-e);
+    if (blockIdx.y == 0 && c < cols) p.ex[c] = e;
+  }
+  __syncthreads();
+  const int c = c0 + threadIdx.x * 4;
+  if (c >= cols) return;
+  const float4 sc = *reinterpret_cast<const float4*>(scale + threadIdx.x * 4);
+#pragma unroll 4
+  for (int r = r0 + threadIdx.y; r < r1; r += 4) {
+    float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
+    v.x *= sc.x; v.y *= sc.y; v.z *= sc.z; v.w *= sc.w;
+    Half4 h, l;
+    split4(v, 1.f, h, l);
+    __half* d = p.hi + (size_t)r * p.ldo + c;
+    *reinterpret_cast<Half4*>(d) = h;
+    *reinterpret_cast<Half4*>(d + p.plane) = l;
+  }
+}
+
+// NCHW -> [n][pixel][channel] planes with padW zero pixels after each row and padH zero rows after each image: what a filter
+// tap reads beside an image is then the end of the row or image before, and a tap is a shift of the row index, which TMA
+// takes at any value (only the contiguous coordinate has an alignment rule).  Exponents per channel, from the maxima of
+// ranges of images, or per pixel.  In a job: len = channels, rows = N (H + padH) (W + padW).
+struct Images {
+  int N, H, W, padH, padW;
+};
+__global__ void __launch_bounds__(256) channel_max_kernel(const __grid_constant__ SplitJobs jobs, const Images im) {
+  __shared__ unsigned red[8];
+  grid_dependency_wait();
+  const bool second = (int)blockIdx.x >= jobs.first;
+  const SplitJob& p = jobs.job[second];
+  const int c = blockIdx.x - (second ? jobs.first : 0), tid = threadIdx.x, HW = im.H * im.W;
+  const int n0 = blockIdx.y * p.per, n1 = min(im.N, n0 + p.per);
+  if (n0 >= n1) return;
+  const float* src = p.src + ((size_t)n0 * p.len + c) * HW;
+  const size_t image = (size_t)p.len * HW;
+  unsigned m = 0;
+  // (image, pixel) pairs in one loop, so that a thread's loads do not end with an image
+  if (p.vec) {
+    const int q = HW / 4;
+#pragma unroll 4
+    for (int i = tid; i < (n1 - n0) * q; i += 256) {
+      const int n = i / q;
+      m = max4(m, __ldg(reinterpret_cast<const float4*>(src + n * image) + i - n * q));
+    }
+  } else {
+#pragma unroll 8
+    for (int i = tid; i < (n1 - n0) * HW; i += 256) {
+      const int n = i / HW;
+      m = max(m, abs_bits(__ldg(src + n * image + i - n * HW)));
+    }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((tid & 31) == 0) red[tid >> 5] = m;
+  __syncthreads();
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) m = max(m, red[i]);
+    p.part[(size_t)blockIdx.y * p.len + c] = m;
+  }
+}
+constexpr int kPxTile = 32, kPxPitch = kPxTile + 1;
+__global__ void __launch_bounds__(256) split_pixels_kernel(const __grid_constant__ SplitJobs jobs, const Images im) {
+  extern __shared__ float px_smem[];
+  __shared__ unsigned red[8][kPxTile];
+  const bool second = (int)blockIdx.x >= jobs.first;
+  const SplitJob& job = jobs.job[second];
+  const int CH = job.len, HW = im.H * im.W;
+  float* tile = px_smem;                                  // [CH][kPxPitch]
+  float* scale = tile + CH * kPxPitch;                    // [CH] or [kPxTile]
+  const int Wp = im.W + im.padW, PP = (im.H + im.padH) * Wp, rows = job.rows;
+  const int p0 = (blockIdx.x - (second ? jobs.first : 0)) * kPxTile, tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+  grid_dependency_wait();
+  {
+    const int p = p0 + tx, n = p / PP, q = p - n * PP, h = q / Wp, w = q - h * Wp;
+    const bool in = p < rows && h < im.H && w < im.W;
+    const float* s = job.src + (((size_t)n * CH) * im.H + h) * im.W + w;
+    unsigned m = 0;
+#pragma unroll 16
+    for (int c = ty; c < CH; c += 8) {
+      const float v = in ? __ldg(s + (size_t)c * HW) : 0.f;
+      tile[c * kPxPitch + tx] = v;
+      m = max(m, abs_bits(v));
+    }
+    red[ty][tx] = m;
+  }
+  if (job.part) {
+    for (int c = tid; c < CH; c += 256) {
+      unsigned m = 0;
+      for (int i = 0; i < job.parts; ++i) m = max(m, __ldcg(job.part + (size_t)i * CH + c));
+      const int e = row_exponent(m, kLeast);
+      scale[c] = exp2_int(-e);
+      if (p0 == 0) job.ex[c] = e;
+    }
+  }
+  __syncthreads();
+  if (!job.part) {
+    if (tid < kPxTile) {
+      unsigned m = red[0][tid];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) m = max(m, red[i][tid]);
+      const int e = row_exponent(m, kLeastConv);
+      scale[tid] = exp2_int(-e);
+      if (p0 + tid < rows) job.ex[p0 + tid] = e;
+    }
+    __syncthreads();
+  }
+  // a warp writes the channels of a pixel, two per lane
+  for (int i = ty; i < kPxTile && p0 + i < rows; i += 8) {
+    __half* d = job.hi + (size_t)(p0 + i) * job.ldo;
+#pragma unroll 4
+    for (int c = tx * 2; c < CH; c += 64) {
+      const bool two = c + 1 < CH;
+      float a = tile[c * kPxPitch + i], b = two ? tile[(c + 1) * kPxPitch + i] : 0.f;
+      a *= job.part ? scale[c] : scale[i];
+      if (two) b *= job.part ? scale[c + 1] : scale[i];
+      const __half2 h = __floats2half2_rn(a, b);
+      const float2 f = __half22float2(h);
+      *reinterpret_cast<__half2*>(d + c) = h;
+      *reinterpret_cast<__half2*>(d + job.plane + c) = __floats2half2_rn(a - f.x, b - f.y);
+    }
+  }
+}
+
+// ---- host ----------------------------------------------------------------------------------------------------------------
+}  // namespace
+// B200CP_GEMM_TC=0 keeps the CUDA-core products, 2 takes the tensor ones at every size (read per call: tests switch it)
+int gemm_tc_mode() {
+  const char* e = getenv("B200CP_GEMM_TC");
+  return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
+}
+namespace {
+
+// fp16 tensor of two planes: dimensions from the contiguous one outwards, strides in elements
+int encode_planes(CUtensorMap* map, const __half* base, const size_t (&dim)[3], const size_t (&stride)[2], size_t plane,
+                  const unsigned (&box)[3]) {
+  PFN_encodeTiled enc = get_encode_tiled();
+  if (!enc) return fail(B200CP_ERR_NO_DEVICE, "cuTensorMapEncodeTiled entry point not available");
+  const cuuint64_t gdim[4] = {dim[0], dim[1], dim[2], 2};
+  const cuuint64_t gstr[3] = {stride[0] * 2, stride[1] * 2, plane * 2};
+  const cuuint32_t bx[4] = {box[0], box[1], box[2], 2}, estr[4] = {1, 1, 1, 1};
+  const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half*>(base), gdim, gstr, bx, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (cr != CUDA_SUCCESS) return fail(B200CP_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
   return B200CP_OK;
 }
 
-}  // namespace
-
-// The tensor path takes a flat GEMM with 16-byte rows that is large enough to fill a good part of a 256 x 256 tile.
-bool gemm_tc_supported(int K, int M, int N) {
-  return enabled() && M % 4 == 0 && N % 4 == 0 && M >= 128 && N >= kBN && K >= 256 && get_encode_tiled() != nullptr;
+// hi / lo planes of one operand and its exponents in the scratch
+struct Planes {
+  __half* hi;
+  int* ex;
+  unsigned* part;       // column / channel maxima
+  size_t rows, plane;   // plane: values of one plane
+  int ld;
+};
+constexpr int kMaxParts = 64;
+size_t planes_floats(size_t rows, size_t ld, size_t exps, bool columns) {
+  return align_up(rows * ld, 64) + align_up(exps, 64) + (columns ? align_up(exps * kMaxParts, 64) : 0);
 }
+Planes take_planes(float*& at, size_t rows, size_t ld, size_t exps, bool columns) {
+  Planes p{};
+  p.hi = reinterpret_cast<__half*>(at);
+  p.rows = rows;
+  p.ld = (int)ld;
+  p.plane = rows * ld;
+  at += align_up(rows * ld, 64);     // two planes of 2-byte values: rows * ld floats
+  p.ex = reinterpret_cast<int*>(at);
+  at += align_up(exps, 64);
+  if (columns) {
+    p.part = reinterpret_cast<unsigned*>(at);
+    at += align_up(exps * kMaxParts, 64);
+  }
+  return p;
+}
+int ld8(int n) { return (n + 7) / 8 * 8; }
 
-// floats of scratch: the hi / lo planes of both operands
-size_t gemm_tc_scratch_floats(int K, int M, int N) { return 2 * (size_t)K * ((size_t)M + (size_t)N); }
-
-// G[M][N] = A^T B with A [K][M], B [K][N]; scratch holds gemm_tc_scratch_floats() floats, 16-byte aligned
-int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st) {
-  PFN_encodeTiled enc = get_encode_tiled();
-  if (!enc) return fail(B200CP_ERR_NO_DEVICE, "cuTensorMapEncodeTiled entry point not available");
-  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(G) |
-       reinterpret_cast<uintptr_t>(scratch)) & 15)
-    return fail(B200CP_ERR_INVALID_ARG, "tensor-core gradient GEMM: operands must be 16-byte aligned");
-  const size_t na = (size_t)K * M, nb = (size_t)K * N;
-  float *Ahi = scratch, *Alo = Ahi + na, *Bhi = Alo + na, *Blo = Bhi + nb;
-  DeviceInfo di;
-  if (int rc = device_info(&di)) return rc;
-  split_tf32_kernel<<<(unsigned)std::min<size_t>((na / 4 + 255) / 256, (size_t)di.sm_count * 16), 256, 0, st>>>(
-      reinterpret_cast<const float4*>(A), reinterpret_cast<float4*>(Ahi), reinterpret_cast<float4*>(Alo), na / 4);
-  B200CP_LAUNCH_OK("split_tf32_kernel");
-  split_tf32_kernel<<<(unsigned)std::min<size_t>((nb / 4 + 255) / 256, (size_t)di.sm_count * 16), 256, 0, st>>>(
-      reinterpret_cast<const float4*>(B), reinterpret_cast<float4*>(Bhi), reinterpret_cast<float4*>(Blo), nb / 4);
-  B200CP_LAUNCH_OK("split_tf32_kernel");
-  CUtensorMap mAhi, mAlo, mBhi, mBlo;
-  if (int rc = encode_plane(enc, &mAhi, Ahi, M, K)) return rc;
-  if (int rc = encode_plane(enc, &mAlo, Alo, M, K)) return rc;
-  if (int rc = encode_plane(enc, &mBhi, Bhi, N, K)) return rc;
-  if (int rc = encode_plane(enc, &mBlo, Blo, N, K)) return rc;
-  GemmTcGeom g{M, N, K, ceil_div(K, kKS), 1, 1, 1, 0, 0, 0};
-  dim3 grid(ceil_div(N, kBN), ceil_div(M, kBM));
-  if (grid.y > 65535) return fail(B200CP_ERR_UNSUPPORTED, "tensor-core gradient GEMM: too many tiles");
-  B200CP_CUDA_OK(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-  gemm_tc_kernel<<<grid, kThreads, kSmem, st>>>(g, mAhi, mAlo, mBhi, mBlo, G);
-  B200CP_LAUNCH_OK("gemm_tc_kernel");
+// (The kernels are programmatic dependents of one another; what comes before the first of a call is not this file's.)
+SplitJob job_of(const float* src, int rows, int segs, int len, int ld, const Planes& p) {
+  SplitJob j{};
+  j.src = src; j.rows = rows; j.segs = segs; j.len = len; j.ld = ld;
+  j.ldo = p.ld; j.hi = p.hi; j.plane = p.plane; j.ex = p.ex; j.part = p.part;
+  j.vec = ld % 4 == 0 && !(reinterpret_cast<uintptr_t>(src) & 15);
+  return j;
+}
+int split_rows(const SplitJob& a, const SplitJob& b, cudaStream_t st) {
+  const auto ctas = [](const SplitJob& j) { return (long)j.segs * j.len > 512 ? j.rows : ceil_div(j.rows, 8); };
+  SplitJobs jobs{{a, b}, ctas(a)};
+  B200CP_CUDA_OK(launch_kernel(split_rows_kernel, dim3(ctas(a) + ctas(b)), dim3(256), 0, st, true, jobs));
+  B200CP_LAUNCH_OK("split_rows_kernel");
+  return B200CP_OK;
+}
+int split_columns(SplitJob a, SplitJob b, cudaStream_t st) {   // of the same number of rows
+  a.per = b.per = std::max(16, ceil_div(a.rows, kMaxParts));
+  a.parts = b.parts = ceil_div(a.rows, a.per);
+  SplitJobs jobs{{a, b}, ceil_div(a.len, 256)};
+  const dim3 grid(jobs.first + ceil_div(b.len, 256), a.parts), block(64, 4);
+  B200CP_CUDA_OK(launch_kernel(column_max_kernel, grid, block, 0, st, true, jobs));
+  B200CP_LAUNCH_OK("column_max_kernel");
+  B200CP_CUDA_OK(launch_kernel(split_columns_kernel, grid, block, 0, st, true, jobs));
+  B200CP_LAUNCH_OK("split_columns_kernel");
+  return B200CP_OK;
+}
+constexpr int kMostChannels = 1024;   // of split_pixels_kernel's tile: 139 KB
+// the pixel planes of one tensor, or (with `part`) the planes with exponents per channel of two
+int split_pixels(SplitJob a, SplitJob b, int count, const Images& im, const DeviceInfo& di, cudaStream_t st) {
+  SplitJobs jobs{{a, b}, a.len};
+  if (a.part) {
+    const int channels = a.len + (count == 2 ? b.len : 0);
+    const int per = std::max(1, ceil_div(im.N, std::min(kMaxParts, std::max(1, 16 * di.sm_count / channels))));
+    for (SplitJob& j : jobs.job) {
+      j.per = per;
+      j.parts = ceil_div(im.N, per);
+      j.vec = im.H * im.W % 4 == 0 && !(reinterpret_cast<uintptr_t>(j.src) & 15);
+    }
+    B200CP_CUDA_OK(launch_kernel(channel_max_kernel, dim3(channels, jobs.job[0].parts), dim3(256), 0, st, true, jobs, im));
+    B200CP_LAUNCH_OK("channel_max_kernel");
+  }
+  jobs.first = ceil_div(a.rows, kPxTile);
+  const int most = count == 2 ? std::max(a.len, b.len) : a.len;
+  const size_t smem = sizeof(float) * ((size_t)most * kPxPitch + std::max(most, kPxTile));
+  static std::atomic<int> set[64];
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_pixels_kernel), set, (int)smem));
+  B200CP_CUDA_OK(launch_kernel(split_pixels_kernel, dim3(jobs.first + (count == 2 ? ceil_div(b.rows, kPxTile) : 0)), dim3(32, 8),
+                               smem, st, true, jobs, im));
+  B200CP_LAUNCH_OK("split_pixels_kernel");
   return B200CP_OK;
 }
 
-// ---- conv form: G[tap][t][c] = sum_{n,h,w} dV[n,t,h,w] * Xpad[n,c,h+y,w+x] ------------------------------------------------
-// Both operands are rewritten once as [n][padded pixel][channel] hi / lo planes (K = padded pixel index, rows);
-// the nine taps are then nine GEMMs over the same planes with the X rows shifted, each split over K so that the
-// (tile, tap, split) grid fills the GPU; a last kernel adds the splits in order.
-namespace {
-struct ConvGemmPlan {
-  int Hp, Wp, taps, splits, NS;
-  long K;
-  size_t plane_a, plane_b, partial;
+// Accumulators of 64 terms, and of 32 where the sum has at most kShortSum steps.  Against float64 an accumulator of 32, 64, 128,
+// 256 terms is cut off by about 0.5, 1.1, 4, 8e-7, and the roundings of n totals add 2.5e-8 sqrt(n / 2): 64 terms are best for
+// long sums (2.2e-7 for 4096 terms; 32 terms: 2.5e-7, and the read-out falls behind the products), 32 for short ones.
+constexpr int kShortSum = 16;
+// Tiles of a product, and the cut of the tiles that do not fill the pairs (see SplitGemm).
+struct TcTiles {
+  int bn, tiles_m, tiles_n, whole, splits, steps, cut;   // cut: tiles that are cut
+  double us;
 };
-bool conv_plan(ConvGemmPlan& p, int N, int T, int C, int H, int W, int FH, int FW) {
-  if (!(enabled() && T % 4 == 0 && C % 4 == 0 && T >= 128 && C >= 128 && FH % 2 == 1 && FW % 2 == 1)) return false;
-  p.Hp = H + FH - 1; p.Wp = W + FW - 1; p.taps = FH * FW;
-  p.K = (long)N * p.Hp * p.Wp;
-  if (p.K < 1024 || p.K > 0x7fffff00L) return false;
-  const long tiles = (long)ceil_div(C, kBN) * ceil_div(T, kBM) * p.taps;
-  const int stages = (int)((p.K + kKS - 1) / kKS);
-  // one wave of CTAs (one CTA per SM by its shared memory); at least 32 stages per split
-  int splits = (int)std::max<long>(1, std::min<long>(148 / std::max<long>(1, tiles), stages / 32));
-  p.NS = ceil_div(stages, splits);
-  p.splits = ceil_div(stages, p.NS);
-  p.plane_a = (size_t)p.K * T;
-  p.plane_b = (size_t)p.K * C;
-  p.partial = p.splits > 1 ? (size_t)p.splits * p.taps * T * C : 0;
+// Measured us of a step (64 k) and of a unit beside its steps.  128 and 64 columns are not in proportion: the rows of A are read
+// from shared memory once per instruction, whatever its width.
+double step_us(int bn) { return bn == 256 ? 1.35 : bn == 128 ? 0.95 : 0.7; }
+constexpr double kUnitUs = 2.0;
+TcTiles tc_tiles(long M, long N, int total, int results, bool mn, const DeviceInfo& di) {
+  TcTiles best{};
+  best.us = 1e300;
+  const int pairs = di.sm_count / 2;
+  for (int bn = 256; bn >= (mn ? 128 : 64); bn /= 2) {
+    const long tm = (M + kBM - 1) / kBM, tn = (N + bn - 1) / bn, tiles = tm * tn * results;
+    if (tiles > 0x3fffffff) continue;
+    TcTiles t{bn, (int)tm, (int)tn, (int)(tiles / pairs * pairs), 1, total, (int)(tiles % pairs), 0.0};
+    t.us = tiles / pairs * (total * step_us(bn) + kUnitUs);
+    if (t.cut) {
+      double tail = 1e300;
+      for (int q = 1; q * t.cut <= pairs && (q == 1 || total / q >= 4); ++q) {
+        const int steps = ceil_div(total, q);
+        if ((q - 1) * steps >= total) continue;
+        // a cut costs the launch that joins the sums, and their way through L2
+        const double us = steps * step_us(bn) + kUnitUs + (q > 1 ? 3.0 + (double)t.cut * (q + 1) * kBM * bn * 4e-6 / 4.0 : 0.0);
+        if (us < tail) { tail = us; t.splits = q; t.steps = steps; }
+      }
+      t.us += tail;
+    }
+    if (t.us < best.us) best = t;
+  }
+  return best;
+}
+size_t partial_floats(const TcTiles& t) { return t.splits > 1 ? (size_t)t.cut * t.splits * t.bn * kBM : 0; }
+
+template <int BN, bool MN, bool CONV>
+int launch_tile(const SplitGemm& g, int cut, const CUtensorMap& a, const CUtensorMap& b, const DeviceInfo& di, cudaStream_t st) {
+  static std::atomic<int> set[64];
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_gemm_kernel<BN, MN, CONV>), set, (int)Tile<BN>::smem));
+  const int pairs = std::min(g.units, di.sm_count / 2);
+  B200CP_CUDA_OK(launch_kernel(split_gemm_kernel<BN, MN, CONV>, dim3(2 * pairs), dim3(Tile<BN>::threads), Tile<BN>::smem, st, true,
+                               g, a, b));
+  B200CP_LAUNCH_OK("split_gemm_kernel");
+  if (g.splits > 1) {
+    B200CP_CUDA_OK(launch_kernel(join_tiles_kernel<BN, MN, CONV>, dim3(cut, BN / kJoinCols), dim3(kBM), 0, st, true, g));
+    B200CP_LAUNCH_OK("join_tiles_kernel");
+  }
+  return B200CP_OK;
+}
+// g has the sizes, exponents and strides of the result; `partial` holds partial_floats(t)
+int run_split_gemm(SplitGemm g, const TcTiles& t, size_t result, bool mn, bool conv, const CUtensorMap& a, const CUtensorMap& b,
+                   float* out, float* partial, const DeviceInfo& di, cudaStream_t st) {
+  g.tiles_m = t.tiles_m; g.tiles_n = t.tiles_n; g.whole = t.whole; g.splits = t.splits; g.steps = t.steps;
+  g.units = t.whole + t.cut * t.splits;
+  g.group = g.total <= kShortSum ? 2 : 4;
+  g.result = result;
+  g.out = out;
+  g.partial = partial;
+#define TILE(BN, MN, CONV) launch_tile<BN, MN, CONV>(g, t.cut, a, b, di, st)
+  if (mn) return t.bn == 256 ? TILE(256, true, false) : TILE(128, true, false);
+  if (conv) return t.bn == 256 ? TILE(256, false, true) : t.bn == 128 ? TILE(128, false, true) : TILE(64, false, true);
+  return t.bn == 256 ? TILE(256, false, false) : t.bn == 128 ? TILE(128, false, false) : TILE(64, false, false);
+#undef TILE
+}
+
+}  // namespace
+
+// ---- gradient products: both operands have the batch (or pixels) as rows -------------------------------------------------
+// G[M][N] = A^T B with A [K][M], B [K][N]: rows of the kernel's result are the N columns of G, which are contiguous.
+namespace {
+TcTiles grad_tiles(int K, int M, int N, const DeviceInfo& di) { return tc_tiles(N, M, ceil_div(K, kKS), 1, true, di); }
+}  // namespace
+
+bool gemm_tc_supported(int K, int M, int N) {
+  const int mode = gemm_tc_mode();
+  return mode && (mode == 2 || (M >= 128 && N >= 128 && K >= 256)) && get_encode_tiled() != nullptr;
+}
+
+size_t gemm_tc_scratch_floats(int K, int M, int N) {
+  DeviceInfo di;
+  if (device_info(&di)) di.sm_count = 148;
+  return planes_floats(K, ld8(M), M, true) + planes_floats(K, ld8(N), N, true) +
+         partial_floats(grad_tiles(K, M, N, di));
+}
+
+int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st) {
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  float* at = scratch;
+  const Planes pn = take_planes(at, K, ld8(N), N, true), pm = take_planes(at, K, ld8(M), M, true);
+  if (int rc = split_columns(job_of(B, K, 1, N, N, pn), job_of(A, K, 1, M, M, pm), st)) return rc;
+  CUtensorMap mn, mm;
+  if (int rc = encode_planes(&mn, pn.hi, {(size_t)N, (size_t)K, 1}, {(size_t)pn.ld, pn.plane}, pn.plane, {64, 64, 1})) return rc;
+  if (int rc = encode_planes(&mm, pm.hi, {(size_t)M, (size_t)K, 1}, {(size_t)pm.ld, pm.plane}, pm.plane, {64, 64, 1})) return rc;
+  const TcTiles t = grad_tiles(K, M, N, di);
+  SplitGemm g{};
+  g.M = N; g.N = M; g.total = ceil_div(K, kKS); g.kc = g.total; g.Kc = K;
+  g.FW = 1;
+  g.ea = pn.ex; g.eb = pm.ex;
+  g.ldm = 1; g.ldn = N;
+  return run_split_gemm(g, t, (size_t)M * N, true, false, mn, mm, G, at, di, st);
+}
+
+// G[tap][t][c] = sum_{n,h,w} dV[n,t,h,w] * Xpad[n,c,h+y,w+x]: K = the pixels of the padded planes; the taps are as many
+// products over the same planes, with the rows of X shifted.
+namespace {
+struct GradConv {
+  int PP, taps;
+  long K;
+  TcTiles t;
+};
+bool grad_conv(GradConv& p, int N, int T, int C, int H, int W, int FH, int FW) {
+  const int mode = gemm_tc_mode();
+  if (!(mode && T <= kMostChannels && C <= kMostChannels && FH % 2 == 1 && FW % 2 == 1)) return false;
+  p.PP = (H + (FH - 1) / 2) * (W + (FW - 1) / 2);
+  p.taps = FH * FW;
+  p.K = (long)N * p.PP;
+  if (p.K > 0x3fffff00L || (mode == 1 && (p.K < 1024 || T < 128 || C < 128))) return false;
+  DeviceInfo di;
+  if (device_info(&di)) di.sm_count = 148;
+  p.t = tc_tiles(C, T, (int)((p.K + kKS - 1) / kKS), p.taps, true, di);
   return get_encode_tiled() != nullptr;
 }
 }  // namespace
 
 bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW) {
-  ConvGemmPlan p;
-  return conv_plan(p, N, T, C, H, W, FH, FW);
+  GradConv p;
+  return grad_conv(p, N, T, C, H, W, FH, FW);
 }
 
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW) {
-  ConvGemmPlan p;
-  if (!conv_plan(p, N, T, C, H, W, FH, FW)) return 0;
-  return 2 * (p.plane_a + p.plane_b) + p.partial;
+  GradConv p;
+  if (!grad_conv(p, N, T, C, H, W, FH, FW)) return 0;
+  return planes_floats(p.K, ld8(C), C, true) + planes_floats(p.K, ld8(T), T, true) + partial_floats(p.t);
 }
 
-// G is written as [tap][T][C]; dV [N][T][H][W], X [N][C][H][W]
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
                         float* scratch, cudaStream_t st) {
-  ConvGemmPlan p;
-  if (!conv_plan(p, N, T, C, H, W, FH, FW)) return fail(B200CP_ERR_UNSUPPORTED, "tensor-core conv gradient: shape not taken");
-  PFN_encodeTiled enc = get_encode_tiled();
-  if ((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(scratch)) & 15)
-    return fail(B200CP_ERR_INVALID_ARG, "tensor-core conv gradient: buffers must be 16-byte aligned");
-  float *Ahi = scratch, *Alo = Ahi + p.plane_a, *Bhi = Alo + p.plane_a, *Blo = Bhi + p.plane_b;
-  float* part = Blo + p.plane_b;
-  const int padH = (FH - 1) / 2, padW = (FW - 1) / 2, PP = p.Hp * p.Wp;
-  if (N > 65535) return fail(B200CP_ERR_UNSUPPORTED, "tensor-core conv gradient: batch too large");
-  pad_transpose_split_kernel<<<dim3(ceil_div(PP, 32), ceil_div(T, 32), N), dim3(32, 8), 0, st>>>(dV, Ahi, Alo, T, H, W,
-                                                                                                 padH, padW);
-  B200CP_LAUNCH_OK("pad_transpose_split_kernel");
-  pad_transpose_split_kernel<<<dim3(ceil_div(PP, 32), ceil_div(C, 32), N), dim3(32, 8), 0, st>>>(X, Bhi, Blo, C, H, W,
-                                                                                                 padH, padW);
-  B200CP_LAUNCH_OK("pad_transpose_split_kernel");
-  CUtensorMap mAhi, mAlo, mBhi, mBlo;
-  if (int rc = encode_plane(enc, &mAhi, Ahi, T, (int)p.K)) return rc;
-  if (int rc = encode_plane(enc, &mAlo, Alo, T, (int)p.K)) return rc;
-  if (int rc = encode_plane(enc, &mBhi, Bhi, C, (int)p.K)) return rc;
-  if (int rc = encode_plane(enc, &mBlo, Blo, C, (int)p.K)) return rc;
-  GemmTcGeom g{T, C, (int)p.K, p.NS, p.splits, p.taps, FW, padH, padW, p.Wp};
-  dim3 grid(ceil_div(C, kBN), ceil_div(T, kBM), p.taps * p.splits);
-  if (grid.y > 65535 || grid.z > 65535) return fail(B200CP_ERR_UNSUPPORTED, "tensor-core conv gradient: too many tiles");
-  B200CP_CUDA_OK(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-  gemm_tc_kernel<<<grid, kThreads, kSmem, st>>>(g, mAhi, mAlo, mBhi, mBlo, p.splits > 1 ? part : G);
-  B200CP_LAUNCH_OK("gemm_tc_kernel");
-  if (p.splits > 1) {
-    const size_t n = (size_t)p.taps * T * C;
-    sum_splits_launch(part, G, n, p.splits, st);
-    B200CP_LAUNCH_OK("sum_splits_kernel");
-  }
-  return B200CP_OK;
+  GradConv p;
+  if (!grad_conv(p, N, T, C, H, W, FH, FW)) return fail(B200CP_ERR_UNSUPPORTED, "tensor-core conv gradient: shape not taken");
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const int padH = (FH - 1) / 2, padW = (FW - 1) / 2;
+  float* at = scratch;
+  const Planes px = take_planes(at, p.K, ld8(C), C, true), pv = take_planes(at, p.K, ld8(T), T, true);
+  if (int rc = split_pixels(job_of(X, (int)p.K, 1, C, 0, px), job_of(dV, (int)p.K, 1, T, 0, pv), 2, Images{N, H, W, padH, padW}, di, st))
+    return rc;
+  CUtensorMap mx, mv;
+  if (int rc = encode_planes(&mx, px.hi, {(size_t)C, (size_t)p.K, 1}, {(size_t)px.ld, px.plane}, px.plane, {64, 64, 1})) return rc;
+  if (int rc = encode_planes(&mv, pv.hi, {(size_t)T, (size_t)p.K, 1}, {(size_t)pv.ld, pv.plane}, pv.plane, {64, 64, 1})) return rc;
+  SplitGemm g{};
+  g.M = C; g.N = T; g.total = ceil_div((int)p.K, kKS); g.kc = g.total; g.Kc = (int)p.K;
+  g.FW = FW; g.padH = padH; g.padW = padW; g.Wp = W + padW;
+  g.ea = px.ex; g.eb = pv.ex;
+  g.ldm = 1; g.ldn = C;
+  return run_split_gemm(g, p.t, (size_t)T * C, true, false, mx, mv, G, at, di, st);
+}
+
+// ---- products with the multiplied-out weight --------------------------------------------------------------------------------
+// Y[B][N] = X[B][K] W^T with the weight W[N][ldw] as kron_weight_launch writes it.  The rows of the kernel's result are the
+// outputs (a warp then stores 32 neighbours of Y), or the batch where that leaves less of the tiles empty.
+namespace {
+struct DenseTc {
+  TcTiles t;
+  bool rows_are_batch;
+};
+DenseTc dense_tc(int B, int K, int N, const DeviceInfo& di) {
+  const int total = ceil_div(K, kKS);
+  const DenseTc a{tc_tiles(N, B, total, 1, false, di), false}, b{tc_tiles(B, N, total, 1, false, di), true};
+  return b.t.us < 0.9 * a.t.us ? b : a;
+}
+// operand planes: a launch each, one pass that reads 4 bytes and writes 4
+double split_us(double values) { return 2.5 + values * 8 / 4.5e6; }
+}  // namespace
+
+bool dense_tc_takes() { return gemm_tc_mode() && get_encode_tiled() != nullptr; }
+
+// without the time of the weight
+double dense_tc_us(int B, int K, int N) {
+  DeviceInfo di;
+  if (device_info(&di)) return 1e300;
+  return 8.0 + split_us((double)N * K) + split_us((double)B * K) + dense_tc(B, K, N, di).t.us;
+}
+
+size_t dense_tc_scratch_floats(int B, int K, int N) {
+  DeviceInfo di;
+  if (device_info(&di)) return 0;
+  return planes_floats(N, ld8(K), N, false) + planes_floats(B, ld8(K), B, false) + partial_floats(dense_tc(B, K, N, di).t);
+}
+
+int dense_tc_launch(int B, int K, int N, const float* X, const float* W, int ldw, float* Y, float* scratch, cudaStream_t st) {
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const DenseTc d = dense_tc(B, K, N, di);
+  float* at = scratch;
+  const Planes pw = take_planes(at, N, ld8(K), N, false), px = take_planes(at, B, ld8(K), B, false);
+  if (int rc = split_rows(job_of(W, N, 1, K, ldw, pw), job_of(X, B, 1, K, K, px), st)) return rc;
+  const Planes &pa = d.rows_are_batch ? px : pw, &pb = d.rows_are_batch ? pw : px;
+  CUtensorMap ma, mb;
+  if (int rc = encode_planes(&ma, pa.hi, {(size_t)K, 1, pa.rows}, {(size_t)pa.ld, (size_t)pa.ld}, pa.plane, {64, 1, 128})) return rc;
+  if (int rc = encode_planes(&mb, pb.hi, {(size_t)K, 1, pb.rows}, {(size_t)pb.ld, (size_t)pb.ld}, pb.plane,
+                             {64, 1, (unsigned)d.t.bn / 2})) return rc;
+  SplitGemm g{};
+  g.M = (int)pa.rows; g.N = (int)pb.rows; g.total = ceil_div(K, kKS); g.kc = g.total; g.Kc = K;
+  g.FW = 1;
+  g.ea = pa.ex; g.eb = pb.ex;
+  g.ldm = d.rows_are_batch ? N : 1;
+  g.ldn = d.rows_are_batch ? 1 : N;
+  g.vec = d.rows_are_batch && N % 4 == 0 && !(reinterpret_cast<uintptr_t>(Y) & 15);
+  return run_split_gemm(g, d.t, 0, false, false, ma, mb, Y, at, di, st);
+}
+
+// V[n,t,h,w] = sum_{c,y,x} W[t][y,x][c] X[n,c,h+y-1,w+x-1] (3 x 3), the weight [T][9][ldw]: rows are the padded pixels, and a
+// step is 64 channels of one tap.
+namespace {
+constexpr int kPad = 1, kTaps = 9;
+TcTiles conv_tc(int N, int C, int T, int H, int W, const DeviceInfo& di) {
+  return tc_tiles((long)N * (H + kPad) * (W + kPad), T, kTaps * ceil_div(C, kKS), 1, false, di);
+}
+}  // namespace
+
+bool conv_tc_takes(int N, int C, int T, int H, int W) {
+  return gemm_tc_mode() && C <= kMostChannels && (long)N * (H + kPad) * (W + kPad) < 0x3fffff00L && get_encode_tiled() != nullptr;
+}
+
+double conv_tc_us(int N, int C, int T, int H, int W) {
+  DeviceInfo di;
+  if (device_info(&di)) return 1e300;
+  return 8.0 + split_us((double)T * C * kTaps) + split_us((double)N * (H + kPad) * (W + kPad) * C) + conv_tc(N, C, T, H, W, di).us;
+}
+
+size_t conv_tc_scratch_floats(int N, int C, int T, int H, int W) {
+  DeviceInfo di;
+  if (device_info(&di)) return 0;
+  const size_t px = (size_t)N * (H + kPad) * (W + kPad);
+  return planes_floats(T, (size_t)kTaps * ld8(C), T, false) + planes_floats(px, ld8(C), px, false) +
+         partial_floats(conv_tc(N, C, T, H, W, di));
+}
+
+int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, int ldw, float* V, float* scratch,
+                   cudaStream_t st) {
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const TcTiles t = conv_tc(N, C, T, H, W, di);
+  const int Wp = W + kPad, PP = (H + kPad) * Wp;
+  const size_t px = (size_t)N * PP, ldk = ld8(C);
+  float* at = scratch;
+  Planes pw = take_planes(at, T, kTaps * ldk, T, false), pa = take_planes(at, px, ldk, px, false);
+  pw.ld = (int)ldk;
+  const SplitJob none{};
+  if (int rc = split_rows(job_of(Wt, T, kTaps, C, ldw, pw), none, st)) return rc;
+  if (int rc = split_pixels(job_of(X, (int)px, 1, C, 0, pa), none, 1, Images{N, H, W, kPad, kPad}, di, st)) return rc;
+  CUtensorMap ma, mb;
+  if (int rc = encode_planes(&ma, pa.hi, {(size_t)C, 1, px}, {ldk, ldk}, pa.plane, {64, 1, 128})) return rc;
+  if (int rc = encode_planes(&mb, pw.hi, {(size_t)C, kTaps, (size_t)T}, {ldk, kTaps * ldk}, pw.plane, {64, 1, (unsigned)t.bn / 2}))
+    return rc;
+  SplitGemm g{};
+  g.M = (int)px; g.N = T; g.kc = ceil_div(C, kKS); g.total = kTaps * g.kc; g.Kc = C;
+  g.FW = 3; g.padH = g.padW = kPad; g.Wp = Wp;
+  g.ea = pa.ex; g.eb = pw.ex;
+  g.ldn = (long)H * W;
+  g.H = H; g.W = W; g.PP = PP;
+  return run_split_gemm(g, t, 0, false, true, ma, mb, V, at, di, st);
 }
 
 // Reads (and clears) the status word of the GEMM kernel; the caller has synchronised the device.

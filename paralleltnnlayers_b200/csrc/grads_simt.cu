@@ -233,6 +233,8 @@ void sum_splits_launch(const float* P, float* G, size_t n, int splits, cudaStrea
 
 namespace {
 
+constexpr size_t kPlaneAlign = 256;   // of the tensor path's scratch, which follows G
+
 int pick_splits(long tiles, int kunits, int sm_count) {
   // aim at two waves of CTAs; never more splits than K units, at most 16
   int s = (int)std::min<long>(16, std::max<long>(1, (2L * sm_count + tiles - 1) / tiles));
@@ -249,9 +251,9 @@ size_t dense_grad_scratch_floats(int N, int T, int C, int H, int W, int FH, int 
   const long tiles = (long)ceil_div(C, BN) * ceil_div(T, BM) * FH * FW;
   const int splits = pick_splits(tiles, N, di.sm_count);
   const size_t simt = splits > 1 ? (size_t)splits * T * C * FH * FW : 0;
-  if (H * W == 1 && FH * FW == 1 && gemm_tc_supported(N, T, C)) return std::max(simt, gemm_tc_scratch_floats(N, T, C));
+  if (H * W == 1 && FH * FW == 1 && gemm_tc_supported(N, T, C)) return std::max(simt, gemm_tc_scratch_floats(N, T, C) + kPlaneAlign / 4);
   if (H * W > 1 && conv_gemm_tc_supported(N, T, C, H, W, FH, FW))
-    return std::max(simt, conv_gemm_tc_scratch_floats(N, T, C, H, W, FH, FW));
+    return std::max(simt, conv_gemm_tc_scratch_floats(N, T, C, H, W, FH, FW) + kPlaneAlign / 4);
   return simt;
 }
 
@@ -261,14 +263,13 @@ int dense_grad_launch(int N, int T, int C, int H, int W, int FH, int FW, const f
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   const int taps = FH * FW;
-  // large flat GEMMs go to the tensor cores (16-byte aligned operands; the scratch then holds the hi / lo planes)
-  if (H * W == 1 && taps == 1 && gemm_tc_supported(N, T, C) && scratch &&
-      ((reinterpret_cast<uintptr_t>(dV) | reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(G) |
-        reinterpret_cast<uintptr_t>(scratch)) & 15) == 0)
-    return gemm_tc_launch(N, T, C, dV, X, G, scratch, st);
-  if (H * W > 1 && scratch && conv_gemm_tc_supported(N, T, C, H, W, FH, FW) &&
-      ((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0)
-    return conv_gemm_tc_launch(N, T, C, H, W, FH, FW, dV, X, G, scratch, st);
+  // large products go to the tensor cores (the scratch then holds the operands' hi / lo planes)
+  if (scratch) {
+    float* planes = reinterpret_cast<float*>(align_up(reinterpret_cast<uintptr_t>(scratch), kPlaneAlign));
+    if (H * W == 1 && taps == 1 && gemm_tc_supported(N, T, C)) return gemm_tc_launch(N, T, C, dV, X, G, planes, st);
+    if (H * W > 1 && conv_gemm_tc_supported(N, T, C, H, W, FH, FW))
+      return conv_gemm_tc_launch(N, T, C, H, W, FH, FW, dV, X, G, planes, st);
+  }
   const long tiles = (long)ceil_div(C, BN) * ceil_div(T, BM) * taps;
   const int splits = pick_splits(tiles, N, di.sm_count);
   GemmArgs g{};

@@ -552,8 +552,9 @@ double waves(long ctas, const DeviceInfo& di) { return (double)((ctas + di.sm_co
 // Estimated microseconds of the two forms: waves of CTAs times the work of one, and the weight's entries written.  Least-
 // squares fit to the layers that the factored kernels' estimate is fitted to (chain_simt.cu).  Choosing by the two, 5 of
 // 1202 layers run more than 10 % and 2 us behind the other form, and all together 0.3 % behind the best choice.
-static double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed,
-                             const DeviceInfo& di) {
+double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed) {
+  DeviceInfo di;
+  if (device_info(&di)) return 1e300;
   const KronPlan p = kron_plan(order, transposed ? odims : idims, transposed ? idims : odims, R, taps, di);
   double slow = taps, fast = 1;
   for (int k = 0; k < order; ++k) {
@@ -573,7 +574,7 @@ double dense_kron_us(int B, int order, const int* idims, const int* odims, int R
   }
   const GemmPlan p = gemm_plan(B, N, K, di);
   const double work = waves(p.tiles * p.splits, di) * p.kper * p.bm * p.bn;
-  return 5.1 + kron_weight_us(order, idims, odims, R, 1, transposed, di) +
+  return 5.1 + kron_weight_us(order, idims, odims, R, 1, transposed) +
          (p.bm == 64 ? 7.93e-6 : p.bm == 32 ? 9.39e-6 : 7.69e-6) * work + 1.54e-6 * ((double)B * K + (double)B * N);
 }
 
@@ -589,16 +590,17 @@ double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* 
   const SmallConvGeom& g = p.g;
   const int px = kCT / p.cgroups / (p.tt / 4) * 4;
   const double w = waves(p.tiles * g.splits, di) * g.cper;
-  return 5.1 + kron_weight_us(order, cdims, tdims, R, 9, transposed, di) +
+  return 5.1 + kron_weight_us(order, cdims, tdims, R, 9, transposed) +
          (p.tt == 64 ? 6.71e-6 : 5.19e-6) * w * 9 * p.tt * px + 8.04e-4 * w * (g.TR + 2) * (g.TC + 2);
 }
 
 // Row pitch of the weight: 16-byte rows.
 int kron_weight_ld(int fast) { return (fast + 3) / 4 * 4; }
 
-// W[s][ld] (dense) or W[s][tap][ld] (S given): slow side = inputs, or outputs with `transposed` (taps then run backwards)
+// W[s][ld] (dense) or W[s][tap][ld] (S given): slow side = inputs, or outputs with `transposed`; with `flip` the taps run
+// backwards (a data gradient)
 int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
-                       int taps, bool transposed, float* W, cudaStream_t st) {
+                       int taps, bool transposed, bool flip, float* W, cudaStream_t st) {
   KronMode m[4];
   long slow = 1, fast = 1;
   for (int k = 0; k < order; ++k) {
@@ -626,7 +628,7 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   if (S) {
     g.A[g.nA++] = KronMode{S, taps, 1, 1, 0, ld, 0};
     g.SA *= taps;
-    g.flip = transposed ? 1 : 0;
+    g.flip = flip ? 1 : 0;
   }
   for (int k = 0; k < ha; ++k) { g.A[g.nA++] = m[k]; g.SA *= m[k].ns; g.FA *= m[k].nf; }
   for (int k = ha; k < order; ++k) { g.B[g.nB++] = m[k]; g.SB *= m[k].ns; g.FB *= m[k].nf; }

@@ -32,58 +32,116 @@ size_t weight_floats(int order, const int* idims, const int* odims, int taps, bo
 constexpr size_t kMostWeight = size_t{256} << 20;
 constexpr double kMostEntries = 1e9;
 
-bool multiplies_out(size_t floats, double entries, double kron_us, double factored_us) {
-  if (factored_us < 0) return entries <= kMostEntries;
-  return factored_us > kron_us && floats * sizeof(float) <= kMostWeight;
+// With fewer ranks the factored kernels' sums are short enough to round less than the tensor product does (R = 4, 4096 samples of
+// 10x10x10 -> 10x10x10: 1.4e-7 of the result against 1.55e-7), and they are not far behind or ahead.
+constexpr int kLeastRanks = 8;
+
+enum class Form { factored, ffma, tensor };
+
+// `floats`: of the weight; a form's time is negative where it does not take the sizes
+Form pick(size_t floats, double entries, double ffma_us, double tensor_us, double factored_us) {
+  if (tensor_us >= 0 && gemm_tc_mode() == 2) return Form::tensor;
+  const bool tensor = tensor_us >= 0 && tensor_us < ffma_us && floats * sizeof(float) <= kMostWeight;
+  const Form out = tensor ? Form::tensor : Form::ffma;
+  if (factored_us < 0) return entries <= kMostEntries ? out : Form::factored;
+  return factored_us > (tensor ? tensor_us : ffma_us) && floats * sizeof(float) <= kMostWeight ? out : Form::factored;
+}
+
+struct DensePlan {
+  Form form;
+  int K, N;               // inputs and outputs of the product
+  size_t weight, bytes;   // floats of the weight, bytes of the workspace
+};
+// the tensor form reads the weight with the other side contiguous
+DensePlan dense_plan(int B, int order, const int* idims, const int* odims, int R, bool transposed, int flags) {
+  DensePlan p{};
+  p.K = (int)prod(transposed ? odims : idims, order);
+  p.N = (int)prod(transposed ? idims : odims, order);
+  const double ffma = dense_kron_us(B, order, idims, odims, R, transposed);
+  const double tensor = (flags & B200CP_TENSOR_PRODUCTS) && dense_tc_takes() && (R >= kLeastRanks || gemm_tc_mode() == 2)
+                            ? kron_weight_us(order, idims, odims, R, 1, !transposed) + dense_tc_us(B, p.K, p.N) : -1;
+  const double least = tensor >= 0 ? std::min(ffma, tensor) : ffma;
+  p.weight = weight_floats(order, idims, odims, 1, transposed);
+  p.form = pick(p.weight, (double)p.K * p.N, ffma, tensor, dense_factored_us(B, order, idims, odims, R, transposed, least));
+  if (p.form == Form::tensor) {
+    p.weight = weight_floats(order, idims, odims, 1, !transposed);
+    p.bytes = align_up(p.weight * sizeof(float), 256) + align_up(dense_tc_scratch_floats(B, p.K, p.N) * sizeof(float), 256);
+  } else if (p.form == Form::ffma) {
+    p.bytes = align_up(p.weight * sizeof(float), 256);
+  }
+  return p;
+}
+
+DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW, bool transposed,
+                   int flags) {
+  DensePlan p{};
+  if (FH != 3 || FW != 3) return p;
+  p.K = (int)prod(transposed ? tdims : cdims, order);
+  p.N = (int)prod(transposed ? cdims : tdims, order);
+  const double ffma = rcp_kron_us(N, H, W, order, cdims, tdims, R, transposed);
+  const double tensor = (flags & B200CP_TENSOR_PRODUCTS) && conv_tc_takes(N, p.K, p.N, H, W) && (R >= kLeastRanks || gemm_tc_mode() == 2)
+                            ? kron_weight_us(order, cdims, tdims, R, 9, !transposed) + conv_tc_us(N, p.K, p.N, H, W) : -1;
+  const double least = tensor >= 0 ? std::min(ffma, tensor) : ffma;
+  p.weight = weight_floats(order, cdims, tdims, 9, transposed);
+  p.form = pick(p.weight, 9.0 * p.K * p.N, ffma, tensor,
+                rcp_factored_us(N, H, W, order, cdims, tdims, R, FH, FW, transposed, least));
+  if (p.form == Form::tensor) {
+    p.weight = weight_floats(order, cdims, tdims, 9, !transposed);
+    p.bytes = align_up(p.weight * sizeof(float), 256) + align_up(conv_tc_scratch_floats(N, p.K, p.N, H, W) * sizeof(float), 256);
+  } else if (p.form == Form::ffma) {
+    p.bytes = align_up(p.weight * sizeof(float), 256);
+  }
+  return p;
+}
+
+bool fits(const DensePlan& p, const void* ws, size_t ws_bytes) {
+  return p.bytes && ws && ws_bytes >= p.bytes && !(reinterpret_cast<uintptr_t>(ws) & 15);
+}
+float* after_weight(const DensePlan& p, void* ws) {
+  return reinterpret_cast<float*>(static_cast<char*>(ws) + align_up(p.weight * sizeof(float), 256));
 }
 
 }  // namespace
 
-size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed) {
+size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed, int flags) {
   if (check_kron_modes(order, idims, odims, R, "dense_cp") || B < 1) return 0;
   if (B > 0x7fffffff - 64) return 0;
-  const size_t floats = weight_floats(order, idims, odims, 1, transposed);
-  const double kron = dense_kron_us(B, order, idims, odims, R, transposed);
-  const double entries = (double)prod(idims, order) * prod(odims, order);
-  if (!multiplies_out(floats, entries, kron, dense_factored_us(B, order, idims, odims, R, transposed, kron))) return 0;
-  return align_up(floats * sizeof(float), 256);
+  return dense_plan(B, order, idims, odims, R, transposed, flags).bytes;
 }
 
 int dense_product_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
-                         const float* const* F, float* Y, bool transposed, void* ws, size_t ws_bytes, cudaStream_t st) {
+                         const float* const* F, float* Y, bool transposed, void* ws, size_t ws_bytes, cudaStream_t st,
+                         int flags) {
   if (int rc = check_kron_modes(order, idims, odims, R, "dense_cp")) return rc;
   if (B < 1) return fail(B200CP_ERR_INVALID_ARG, "dense_cp: batch must be positive");
-  const size_t need = dense_product_workspace(B, order, idims, odims, R, transposed);
-  if (!need || !ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15))
-    return dense_chain_launch(B, order, idims, odims, R, X, F, Y, transposed, st);
+  const DensePlan p = B > 0x7fffffff - 64 ? DensePlan{} : dense_plan(B, order, idims, odims, R, transposed, flags);
+  if (!fits(p, ws, ws_bytes)) return dense_chain_launch(B, order, idims, odims, R, X, F, Y, transposed, st);
   float* Wt = static_cast<float*>(ws);
-  if (int rc = kron_weight_launch(order, idims, odims, R, F, nullptr, 1, transposed, Wt, st)) return rc;
-  const int I = (int)prod(idims, order), O = (int)prod(odims, order);
-  return small_gemm_launch(B, transposed ? I : O, transposed ? O : I, X, Wt, Y, st);
+  const bool tensor = p.form == Form::tensor;
+  if (int rc = kron_weight_launch(order, idims, odims, R, F, nullptr, 1, transposed != tensor, false, Wt, st)) return rc;
+  return tensor ? dense_tc_launch(B, p.K, p.N, X, Wt, kron_weight_ld(p.K), Y, after_weight(p, ws), st)
+                : small_gemm_launch(B, p.N, p.K, X, Wt, Y, st);
 }
 
 size_t rcp_product_workspace(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
-                             bool transposed) {
+                             bool transposed, int flags) {
   if (check_kron_modes(order, cdims, tdims, R, "rcp") || N < 1 || H < 1 || W < 1) return 0;
-  if (FH != 3 || FW != 3) return 0;
-  const size_t floats = weight_floats(order, cdims, tdims, 9, transposed);
-  const double kron = rcp_kron_us(N, H, W, order, cdims, tdims, R, transposed);
-  const double entries = 9.0 * prod(cdims, order) * prod(tdims, order);
-  if (!multiplies_out(floats, entries, kron, rcp_factored_us(N, H, W, order, cdims, tdims, R, FH, FW, transposed, kron))) return 0;
-  return align_up(floats * sizeof(float), 256);
+  return rcp_plan(N, H, W, order, cdims, tdims, R, FH, FW, transposed, flags).bytes;
 }
 
 int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                        const float* X, const float* const* A, const float* S, float* V, bool transposed, void* ws,
-                       size_t ws_bytes, cudaStream_t st) {
+                       size_t ws_bytes, cudaStream_t st, int flags) {
   if (int rc = check_kron_modes(order, cdims, tdims, R, "rcp")) return rc;
-  const size_t need = rcp_product_workspace(N, H, W, order, cdims, tdims, R, FH, FW, transposed);
-  if (!need || !ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15))
+  const bool sizes = N >= 1 && H >= 1 && W >= 1;
+  const DensePlan p = sizes ? rcp_plan(N, H, W, order, cdims, tdims, R, FH, FW, transposed, flags) : DensePlan{};
+  if (!fits(p, ws, ws_bytes))
     return rcp_chain_launch(N, H, W, order, cdims, tdims, R, FH, FW, X, A, S, V, transposed, st);
   float* Wt = static_cast<float*>(ws);
-  if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, FH * FW, transposed, Wt, st)) return rc;
-  const int C = (int)prod(cdims, order), T = (int)prod(tdims, order);
-  return small_conv_launch(N, transposed ? T : C, transposed ? C : T, H, W, X, Wt, V, st);
+  const bool tensor = p.form == Form::tensor;
+  if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, FH * FW, transposed != tensor, transposed, Wt, st)) return rc;
+  return tensor ? conv_tc_launch(N, p.K, p.N, H, W, X, Wt, kron_weight_ld(p.K), V, after_weight(p, ws), st)
+                : small_conv_launch(N, p.K, p.N, H, W, X, Wt, V, st);
 }
 
 }  // namespace b200cp

@@ -277,6 +277,9 @@ std::array<Tensor, 3> cp3_backward_filter(const Tensor& dU_, const Tensor& In, c
   return split3(dK, s);
 }
 
+// The default path of these layers takes the fastest product; a caller who names a path keeps to FFMA.
+int product_flags(int flags) { return (flags & B200CP_PATH_MASK) == B200CP_PATH_AUTO ? flags | B200CP_TENSOR_PRODUCTS : flags; }
+
 // ---- reshaped-CP conv and CP dense ------------------------------------------------------------------------------------
 struct Modes {
   std::vector<Tensor> F;
@@ -308,6 +311,7 @@ struct Modes {
 };
 
 Tensor rcp_forward(const Tensor& U_, at::TensorList A, const Tensor& KC_, int flags) {
+  flags = product_flags(flags);
   const Tensor U = dev(U_, "input");
   const Modes m(A, "conv2d_rcp_fused_nchw", U);
   const Tensor KC = m.core(KC_, U);
@@ -342,6 +346,7 @@ struct FactorGrads {
 
 FactorGrads rcp_backward(const Tensor& U_, const Tensor& dV_, at::TensorList A, const Tensor& KC_, int flags, bool need_dx,
                          bool need_dw) {
+  flags = product_flags(flags);
   const Tensor U = dev(U_, "input"), dV = dev(dV_, "dV", U);
   const Modes m(A, "rcp_conv2d_backward", U);
   const Tensor KC = m.core(KC_, U);
@@ -371,6 +376,7 @@ FactorGrads rcp_backward(const Tensor& U_, const Tensor& dV_, at::TensorList A, 
 }
 
 Tensor dense_forward(const Tensor& U_, at::TensorList F, int flags) {
+  flags = product_flags(flags);
   const Tensor U = dev(U_, "input");
   const Modes m(F, "dense_cp", U);
   const int64_t B = U.size(0);
@@ -387,6 +393,7 @@ Tensor dense_forward(const Tensor& U_, at::TensorList F, int flags) {
 }
 
 FactorGrads dense_backward(const Tensor& U_, const Tensor& dV_, at::TensorList F, int flags, bool need_dx, bool need_dw) {
+  flags = product_flags(flags);
   const Tensor U = dev(U_, "input"), dV = dev(dV_, "dV", U);
   const Modes m(F, "dense_cp_backward", U);
   const int B = (int)U.size(0);

@@ -1,0 +1,150 @@
+"""The tensor-core products of the dense and reshaped-CP layers (scaled fp16 hi / lo operands) at the edges of their tiles:
+256 x 256 / 128 / 64 results, K steps of 64 in instructions of 16, odd row lengths, operands off the 16-byte grid, rows of very
+different magnitude.  B200CP_GEMM_TC=2 takes them at every size.
+
+Bound: a product of two 22-bit operands without the product of their low parts is off by at most 2**-21; an accumulator of
+n <= 4 instructions is cut off by at most n * 2**-23 of its partial sums, and the totals round by 2**-24 each.  In the norm over a
+result, with random signs, that is 2.5e-7 (measured: 1.0 to 2.5e-7); the weight's own fp32 sum adds 1e-7."""
+import math
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+REL = 5e-7
+
+
+@pytest.fixture(autouse=True)
+def always(monkeypatch):
+    monkeypatch.setenv("B200CP_GEMM_TC", "2")
+
+
+def _normal(seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return lambda *s: torch.randn(*s, generator=gen, device="cuda")
+
+
+def _kron(F):
+    M = torch.ones(1, 1, F[0].shape[2], device="cuda", dtype=torch.float64)
+    for f in F:
+        M = torch.einsum("abr,ijr->aibjr", M, f.double()).reshape(M.shape[0] * f.shape[0], M.shape[1] * f.shape[1], -1)
+    return M
+
+
+def _rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
+DENSE = [(1, (4, 4), (2, 4)), (63, (3, 5), (3, 3)), (65, (16, 4), (16, 4)), (130, (5, 13), (11, 12)), (257, (16, 8), (16, 16)),
+         (300, (16, 12), (16, 9)), (77, (16, 16), (16, 16, 1)[:2]), (700, (7, 9), (16, 16)), (40, (16, 16), (13, 7))]
+
+
+@pytest.mark.parametrize("case", DENSE, ids=str)
+@pytest.mark.parametrize("offset", [0, 1])   # floats off the 16-byte grid
+def test_dense(case, offset):
+    import paralleltnnlayers_b200 as P
+    B, idims, odims = case
+    normal = _normal(B + offset)
+    I, O = math.prod(idims), math.prod(odims)
+    x, dy = normal(B * I + offset)[offset:].view(B, I), normal(B * O + offset)[offset:].view(B, O)
+    F = [normal(i, o, 9) * 0.35 for i, o in zip(idims, odims)]
+    M = _kron(F).sum(-1)
+    n0 = P.launch_count()
+    assert _rel(P.dense_cp(x, *F), x.double() @ M) < REL
+    assert P.launch_count() - n0 >= 3   # weight, operand planes, product
+    dx, dF = P.dense_cp_backward(x, dy, *F)
+    assert _rel(dx, dy.double() @ M.T) < REL
+    leaves = [f.double().requires_grad_() for f in F]
+    ref = torch.autograd.grad(x.double() @ _kron(leaves).sum(-1), leaves, dy.double())
+    for got, want in zip(dF, ref):
+        assert _rel(got, want) < 1e-6   # and the contraction with the other factors, in fp32
+    P.device_status()
+
+
+RCP = [(1, 3, 5, (3, 3), (4, 3)), (2, 7, 9, (4, 4), (5, 5)), (3, 8, 8, (5, 13), (16, 4)), (1, 16, 17, (16, 8), (13, 10)),
+       (5, 9, 4, (16, 12), (16, 16))]
+
+
+@pytest.mark.parametrize("case", RCP, ids=str)
+def test_rcp(case):
+    import paralleltnnlayers_b200 as P
+    N, H, W, cd, td = case
+    normal = _normal(H * W)
+    C, T, R = math.prod(cd), math.prod(td), 9
+    x, dy = normal(N, C, H, W), normal(N, T, H, W)
+    A, S = [normal(c, t, R) * 0.3 for c, t in zip(cd, td)], normal(3, 3, R) * 0.3
+
+    def forward(x, A, S):
+        K = torch.einsum("ctr,yxr->tcyx", _kron(A), S.double())
+        return torch.nn.functional.conv2d(x.cpu(), K.cpu(), padding=1)
+
+    leaves = [t.double().requires_grad_() for t in (x, *A, S)]
+    y = forward(leaves[0], leaves[1:-1], leaves[-1])
+    ref = torch.autograd.grad(y, leaves, dy.double().cpu())
+    assert _rel(P.conv2d_rcp_fused_nchw(x, *A, S).cpu(), y.detach()) < REL
+    dx, dA, dS = P.rcp_conv2d_backward(x, dy, *A, S)
+    assert _rel(dx, ref[0]) < REL
+    for got, want in zip((*dA, dS), ref[1:]):
+        assert _rel(got, want) < 1e-6
+    P.device_status()
+
+
+def test_rows_keep_their_own_scale():
+    """Every row of the batch has its own power of two, so that a row is as accurate beside any other: magnitudes from 1e-30 to
+    the largest float.  Infinities and NaN stay in their row."""
+    import paralleltnnlayers_b200 as P
+    normal = _normal(5)
+    F = [normal(16, 16, 9) * 0.1 for _ in range(2)]
+    M = _kron(F).sum(-1)
+    scale = torch.tensor([1e-30, 1e-8, 1.0, 1e8, 1e30, 1e-18, 3e37], device="cuda")
+    x = normal(7, 256) * scale[:, None]
+    ref = x.double() @ M
+    y = P.dense_cp(x, *F)
+    for i in range(7):
+        assert _rel(y[i], ref[i]) < REL, i
+    x[2, 3], x[4, 7] = float("nan"), float("inf")
+    z = P.dense_cp(x, *F)
+    assert bool(torch.isnan(z[2]).all()) and not bool(torch.isfinite(z[4]).any())
+    for i in (0, 1, 3, 5):
+        assert torch.equal(z[i], y[i]), i
+    # the pixels of a convolution
+    A, S = [normal(8, 8, 9) * 0.2 for _ in range(2)], normal(3, 3, 9) * 0.3
+    u = normal(4, 64, 6, 7) * torch.tensor([1e-25, 1.0, 1e25, 1e-10], device="cuda")[:, None, None, None]
+    K = torch.einsum("ctr,yxr->tcyx", _kron(A), S.double()).cpu()
+    ref, v = torch.nn.functional.conv2d(u.double().cpu(), K, padding=1), P.conv2d_rcp_fused_nchw(u, *A, S)
+    for i in range(4):
+        assert _rel(v[i].cpu(), ref[i]) < REL, i
+    u[1, 5, 2, 3] = float("nan")
+    w = P.conv2d_rcp_fused_nchw(u, *A, S)
+    hit = torch.zeros(6, 7, dtype=torch.bool, device="cuda")
+    hit[1:4, 2:5] = True
+    assert bool(torch.isnan(w[1][:, hit]).all()) and torch.equal(w[1][:, ~hit], v[1][:, ~hit])
+    assert torch.equal(w[[0, 2, 3]], v[[0, 2, 3]])
+
+
+def test_whole_numbers_are_exact():
+    """Small integers have no low part and sums below 2**24 are not cut off."""
+    import paralleltnnlayers_b200 as P
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    integers = lambda *s: torch.randint(-3, 4, s, generator=gen, device="cuda").float()
+    x, F = integers(130, 144), [integers(12, 12, 2) for _ in range(2)]
+    assert torch.equal(P.dense_cp(x, *F).double(), x.double() @ _kron(F).sum(-1))
+
+
+def test_under_capture_and_on_another_stream():
+    import paralleltnnlayers_b200 as P
+    normal = _normal(8)
+    x, F = normal(128, 256), [normal(16, 16, 12) * 0.35 for _ in range(2)]
+    want = P.dense_cp(x, *F)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        assert torch.equal(P.dense_cp(x, *F), want)
+    torch.cuda.current_stream().wait_stream(s)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = P.dense_cp(x, *F)
+    x.copy_(normal(128, 256))
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, P.dense_cp(x, *F))
