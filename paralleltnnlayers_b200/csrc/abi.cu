@@ -1,5 +1,6 @@
 // extern "C" surface of libb200cp: argument validation, rank chunking, host-buffer helpers.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -97,65 +98,48 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 }
 
 // Which 3x3 / pad 1 convolutions and backward passes run as products over whole rank planes (cp_planes.cu); B200CP_PLANES=0
-// switches them off.  The tile and row kernels they compete with keep a plane in shared memory, so they win while one
-// chunk of ranks and enough tiles of one image keep every SM busy; the products have a fixed cost of three to five
-// dependent launches (about 14 us for a convolution at R > 32) and take any split of channels and pixels, but pad ranks and
-// channels to tiles of 64.  Measured on the device, tile or row kernels / products, us, shapes N x C x T x H x W:
-//   convolution  R = 128: 32x64x64x56x56 246 / 131, 8x256x256x14x14 128 / 23, 64x32x32x63x61 323 / 262, but 32x8x8x63x61 74 / 114
-//     R = 100: 16x8x8x27x27 19 / 23;  R = 65: 16x8x8x27x27 16 / 21, 16x16x16x27x27 19 / 21
-//     R = 64: 8x256x256x14x14 60 / 23, 64x512x512x7x7 51 / 29, 32x64x64x56x56 86 / 74, 32x128x128x28x28 42 / 38, but
-//       32x128x32x28x28 27 / 35
-//     R = 32: 8x256x256x14x14 27 / 15, 64x512x512x7x7 29 / 23, 1x512x512x7x7 17 / 15
-//   training step  R = 128: 32x8x8x63x61 399 / 357;  R = 64: 32x16x16x28x28 69 / 49, but 64x8x8x14x14 37 / 41
-//     R = 32: 64x256x256x14x14 102 / 69, 64x512x512x7x7 93 / 53, 16x256x384x27x27 109 / 91
-//     R = 8: 64x512x512x7x7 58 / 42
-//   factor gradients alone  R = 64: 64x16x16x7x7 15 / 21, 32x16x16x28x28 37 / 42, but 32x24x24x28x28 56 / 44; with the tile
-//     kernel's 9x9 tiles in one full round 16x16x16x27x27 18 / 35, 16x64x64x27x27 37 / 39;  R = 65 (padded to 128)
-//     32x16x16x56x56 123 / 169, 64x16x16x7x7 27 / 23;  R = 128: 32x16x16x28x28 73 / 64
-//   layer, forward and backward from the saved plane  R = 64: 64x16x16x14x14 37 / 52, 16x64x64x27x27 62 / 71, but
-//     4x16x16x56x56 56 / 51;  R = 50: 16x256x384x27x27 207 / 148
-//   three-factor layer, whose other kernels contract the channels twice  R = 64: 16x16x16x27x27 35 / 56, 64x16x16x32x32 125 / 113;
-//     R = 32: 32x64x64x56x56 222 / 158, 16x64x64x27x27 45 / 53;  R = 16: 64x512x512x7x7 117 / 52, 32x256x256x63x61 724 / 446;
-//     R = 4: 32x256x256x63x61 507 / 384.  Its factor gradients alone  R = 32: 32x64x64x28x28 31 / 41, 4x96x96x56x56 47 / 37
-const bool g_planes = [] {
+// switches them off, 2 takes them wherever they can run.  The tile and row kernels they compete with keep a plane in shared
+// memory and do the three phases in one launch (5 us for a small convolution); the products have a fixed cost of three to five
+// dependent launches (about 20 us for a convolution), and after that cost little per rank and channel.  The more ranks and
+// channels a pixel has, the sooner they win; with more pixels the fixed cost counts for less.
+// The lines are the best ones over 620 random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together, ranks
+// 6 to 128), each measured both ways; against the better form of each shape the choice costs 2 % for a convolution, 1 % for
+// a step or a layer, 0.6 % for a three-factor layer (geometric mean).  Tile or row kernels / products, us:
+//   ranks       6-16    17-32   33-64   65-128   (sums over the shapes of one sample, of 73, 57, 36, 54)
+//   convolution 1148/1619  1148/1230  1126/860  4350/1989
+//   step        3334/4656  3657/3343  3846/2267  12037/4992
+//   gradients   2897/3671  3110/2636  3259/1808  8777/3821
+//   layer       4017/5548  4164/4072  4255/2798  13463/6167
+//   layer (3)   5442/5528  5340/4058  5583/2793  17411/6153
+const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
-  return !(e && e[0] == '0');
+  return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
 }();
 // one convolution; the step; the backward from the forward's plane; the factor gradients; the last two of CP3
 enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3 };
 bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !g_planes || !planes_supported(*s)) return false;
-  const size_t px = (size_t)s->N * s->H * s->W, ch = (size_t)s->C + s->T;
-  const unsigned R = s->Rank;
-  const bool few = px <= 4096 && ch >= 512;   // small images, many channels: few tiles, each a long chain
-  // the tile kernels' tiles (9x9 pixels for 33 to 64 ranks, 14x14 for 17 to 32) fill the SMs once: no idle SM, no last round
-  const auto one_round = [&](unsigned side) {
-    DeviceInfo di;
-    return px > 8192 && device_info(&di) == B200CP_OK &&
-           (size_t)s->N * ceil_div((int)s->H, (int)side) * ceil_div((int)s->W, (int)side) <= (size_t)di.sm_count;
-  };
-  const auto full14 = [&] { return one_round(14) && (px > 20000 || (s->H * s->W & 1)); };   // (odd images: 4-byte copies)
-  const bool step = R > 32 || (R > 16 && px <= 16384 && ch >= 384) || (few && (s->W & 3));   // (the row kernels take W % 4 == 0)
-  const bool mid = R > 32 && R <= 64;
+  if (g_planes == 2) return true;
+  const double px = (double)s->N * s->H * s->W, ch = (double)s->C + s->T, weighted = ch * std::sqrt(std::sqrt(px));
+  const int ranks = s->Rank <= 16 ? 0 : s->Rank <= 32 ? 1 : s->Rank <= 64 ? 2 : 3;
   switch (use) {
-    case Planes::kConv:
-      return (R > 64 && ch >= 32) || (mid && ((px <= 4096 && ch >= 256) || (px >= 16384 && ch >= 128))) || (R > 16 && few);
-    case Planes::kStep:
-      return step;
-    case Planes::kSaved:
-      return step && !(mid && ((ch < 64 && (s->W & 3)) || (ch < 128 && one_round(9))));
+    case Planes::kConv: {
+      constexpr double line[4] = {12000, 2400, 800, 420};
+      return weighted >= line[ranks];
+    }
+    case Planes::kStep: {
+      constexpr double line[4] = {12000, 1300, 300, 0};
+      return weighted >= line[ranks];
+    }
+    case Planes::kSaved: {
+      constexpr double line[4] = {12000, 2200, 530, 0};
+      return weighted >= line[ranks];
+    }
     case Planes::kFilter:
     case Planes::kFilter3:
-      if (mid) return ch >= 48 && !(ch < 160 && one_round(9));
-      if (R > 64) {
-        const bool padded = 3 * R <= 2 * ((R + 63) / 64 * 64);   // a third and more of the rank tiles is padding
-        return ch >= 48 ? !(ch < 96 && one_round(9)) : px <= 4096 || (!padded && px < 65536 && !one_round(9));
-      }
-      if (use == Planes::kFilter) return step;
-      return ch >= 512 || (R > 16 && ch >= 128 && !(ch < 224 && full14()));
+      return ranks == 0 ? ch >= 4 * std::sqrt(px) : ranks == 1 ? ch > 128 : ranks == 2 ? weighted >= 540 : ch >= 44;
     default:
-      if (mid) return px >= 32768 || (ch >= 48 && !(ch < 128 && one_round(9)));
-      return R > 64 || ch >= 512 || (R > 16 && ch >= 128 && !(ch < 160 && full14()));
+      return ranks == 0 ? ch >= 160 : ranks == 1 ? weighted >= 1400 : ranks == 2 ? weighted >= 490 : ch >= 18;
   }
 }
 
@@ -1267,6 +1251,8 @@ int b200cp_device_status(void) {
   if (v) return fail(B200CP_ERR_TIMEOUT, "cp4 row-stream kernel: a bounded wait ran out in block %d", v & 0xffff);
   if (int rc = grad_band_device_status(&v)) return rc;
   if (v) return fail(B200CP_ERR_TIMEOUT, "cp4 gradient band kernel: a bounded wait ran out in block %d", v & 0xffff);
+  if (int rc = planes_device_status(&v)) return rc;
+  if (v) return fail(B200CP_ERR_TIMEOUT, "cp plane products: a bounded wait ran out in block %d", v & 0xffff);
   return B200CP_OK;
 }
 

@@ -18,203 +18,252 @@
 #include "common.cuh"
 #include "cp_planes.cuh"
 #include "mma_util.cuh"
+#include "tc_common.cuh"
 
 namespace b200cp {
+
+__device__ int g_planes_status = 0;  // 0 ok; otherwise (1 << 16) | (block index & 0xffff): a bounded wait ran out
+
 namespace {
 
 constexpr int kThreads = 128;
 
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void fma4(float (&d)[4], float a, const float4& b) {
-  d[0] = fmaf(a, b.x, d[0]);
-  d[1] = fmaf(a, b.y, d[1]);
-  d[2] = fmaf(a, b.z, d[2]);
-  d[3] = fmaf(a, b.w, d[3]);
-}
 
-// ---- out[n][m][p] = sum_k F(m, k) in[n][k][p] --------------------------------------------------------------------------
-// AK false: F is [K][M] (channels to ranks); true: F is [M][K] (ranks to channels).  A warp forms 4*TM rows x 32 pixels,
-// TM x 4 per lane (4 row groups x 8 pixel quads): three shared-memory wavefronts per 32 FFMA at TM = 8.  128 threads per
-// CTA, four and more CTAs per SM.
-struct PlaneProduct {
+// ---- out[n][m][p] = sum_k F(m, k) in[n][k][p] on the tensor cores ---------------------------------------------------------
+// The products of a CP convolution with whole rank planes: P = K1^T X (F is [K][M]) and U = K0 Z (AK: F is [M][K]).  Scaled fp16
+// hi / lo operands as in gemm_tc.cu: three products, accumulators of 64 terms.
+//
+// 128 pixels are the rows of the tensor-core tile, one per thread and per TMEM lane: a thread loads 64 values of its pixel (the
+// lanes of a warp read 32 neighbours of a plane, at any width or alignment), finds their exponent, and writes the swizzled
+// operand rows itself, so no pass over memory and no exchange between threads is needed.  Two groups of 128 threads take the
+// chunks of 64 in turn: one loads and splits while the other's products run.  Every chunk has its own accumulator in TMEM
+// (chunks x rows <= 512 columns); at the end they are added up, each with its pixel's power of two.  F is split once per CTA,
+// which then walks the pixel tiles; where the pixels alone leave SMs idle the sum is split over a cluster instead.
+//
+// What bounds it is latency: about 3 us until F is split, 1 to 2 us per half chunk loaded, 1 us for the products and 1 to 3 us to
+// store.  Both products of 64 x 256 14x14 at R = 32: P and Q 21.7 us on FFMA, 16.8 here; the outputs 21 and 17.
+constexpr int kTcThreads = 256, kTcPx = 128, kTcK = 64;
+constexpr int kTcPlane = kTcPx * 128;   // bytes of one operand plane (hi or lo) of a chunk
+constexpr int kTcMaxChunks = 16;
+
+struct PlaneTcProduct {
   const float* F;
   const float* in;
   float* out;
-  int M, K, mtiles, kper;
-  int vecF, vecIn, vecOut;
+  int M, K, mtiles, kper;   // kper: of a CTA of the cluster, a multiple of 64
 };
-struct PlaneGemm {
-  PlaneProduct p[2];
-  int HW, Q, maxmt, splits;     // Q = N * HW
+struct PlaneTc {
+  PlaneTcProduct p[2];
+  int HW, Q, maxmt, splits, pxtiles;
+  int nt, chunks, cols;     // rows of a tile, a multiple of 32; chunks of a CTA; TMEM columns
+  int first;                // the input is not the work of the kernel before
 };
-constexpr int kGK = 16, kGS = 3;
 
-template <int TM, int WM, int WN, bool AK>
-__global__ void __launch_bounds__(kThreads) plane_gemm_kernel(const __grid_constant__ PlaneGemm g) {
-  constexpr int BM = 4 * TM * WM, BN = 32 * WN, PA = AK ? kGK + 4 : BM;
-  constexpr int kAF = AK ? BM * PA : kGK * PA, kStage = kAF + kGK * BN;
-  static_assert(WM * WN == 4 && kGS * kStage >= BM * BN, "");
-  __shared__ __align__(16) float smem[kGS * kStage];
-  const PlaneProduct& a = g.p[blockIdx.z / g.splits];
-  const int mt = blockIdx.x % g.maxmt, q0 = (blockIdx.x / g.maxmt) * BN;
+// eight fp32 values (four at d, four at d2, one plane on) become their hi and lo halves
+__device__ __forceinline__ void split_in_place(uint8_t* d, uint8_t* d2, float sc) {
+  const float4 x = *reinterpret_cast<const float4*>(d), y = *reinterpret_cast<const float4*>(d2);
+  const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  uint4 hi, lo;
+  tc::split8(v, sc, hi, lo);
+  *reinterpret_cast<uint4*>(d) = hi;
+  *reinterpret_cast<uint4*>(d2) = lo;
+}
+
+template <bool AK>
+__global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_constant__ PlaneTc g) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t done[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ unsigned rowmax[256];
+  __shared__ __align__(16) float2 rowscale[256];
+  __shared__ float ea[kTcMaxChunks][kTcPx];
+  const int tid = threadIdx.x, warp = tid >> 5, grp = tid >> 7, t = tid & 127;
+  const PlaneTcProduct& a = g.p[blockIdx.z / g.splits];
+  const int mt = blockIdx.y;
   if (mt >= a.mtiles) {     // (the other product of the launch has more row tiles; a whole cluster leaves)
     grid_dependency_wait();
     return;
   }
-  const int m0 = mt * BM, kb = (blockIdx.z % g.splits) * a.kper, ke = min(a.K, kb + a.kper);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp / WN, wn = warp % WN;
-  const int ty = lane >> 3, tx = lane & 7;
-  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
-  // this thread's pixel column of a stage
-  constexpr int G4 = BN / 4, R4 = kThreads / G4, R1 = kThreads / BN;
-  const int col = a.vecIn ? (tid % G4) * 4 : tid % BN, row0 = a.vecIn ? tid / G4 : tid / BN;
-  const bool colin = q0 + col < g.Q;
-  const int n = colin ? (q0 + col) / g.HW : 0, p = colin ? q0 + col - n * g.HW : 0;
-  const float* in = a.in + (size_t)n * a.K * g.HW + p;
-
-  // Every thread copies the same column of each stage, so its address runs and what is outside M or the pixels is a copy
-  // of no bytes (zero fill); only the last stage of a K that is no multiple of the stage looks at k.
-  const float* inp = in + (size_t)(kb + row0) * g.HW;
-  auto load_in = [&](int st, int k0) {
-    const unsigned d = sbase + (unsigned)(st * kStage + kAF + row0 * BN + col) * 4u;
-    const float* src = inp;
-    inp += (size_t)kGK * g.HW;
-    const bool full = k0 + kGK <= ke;
-    if (a.vecIn) {
-      const size_t inc = (size_t)R4 * g.HW;
+  const int nt = g.nt, m0 = mt * nt, kb = (blockIdx.z % g.splits) * a.kper, ke = min(a.K, kb + a.kper);
+  const int nch = ke > kb ? (ke - kb + kTcK - 1) / kTcK : 0;
+  uint8_t* Bs = sm + (g.chunks > 1 ? 4 : 2) * kTcPlane;   // [chunk][hi, lo][nt] rows of 128 bytes
+  if (tid == 0) {
+    tc::mbar_init(&done[0], 1);
+    tc::mbar_init(&done[1], 1);
+    tc::fence_barrier_init();
+  }
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, g.cols);
+  rowmax[tid] = 0;
+  __syncthreads();
+  // a sum of one chunk is shared by the groups, half of it (an accumulator of 32 terms) each
+  const bool halved = nch == 1;
+  const int nacc = halved ? (ke - kb > 32 ? 2 : 1) : nch, span = halved ? 32 : kTcK, slot0 = halved ? grp * 4 : 0;
+  // Half a chunk of this thread's pixel at a time, its loads in flight while the half before is worked on.  (cp.async into the
+  // thread's own row is four lanes to a bank, 4 us a chunk; 64 values at once spill, and code that runs once costs its fetch.)
+  constexpr int kHalf = kTcK / 2;
+  const int halves = (span == kTcK ? 2 : 1) * ((nacc - grp + 1) / 2);   // of this group
+  bool qin;
+  int n, p;             // this thread's pixel
+  float v[kHalf];
+  auto pixel = [&](int tile) {
+    const int q = tile * kTcPx + t;
+    qin = q < g.Q;
+    n = qin ? q / g.HW : 0;
+    p = qin ? q - n * g.HW : 0;
+  };
+  auto load_half = [&](int u) {
+    const int k0 = span == kTcK ? ((u >> 1) * 2 + grp) * kTcK + (u & 1) * kHalf : grp * kHalf, kn = ke - kb - k0;
+    const float* src = a.in + ((size_t)n * a.K + kb + k0) * g.HW + p;
 #pragma unroll
-      for (int i = 0; i < kGK / R4; ++i, src += inc) {
-        const bool v = colin && (full || k0 + row0 + i * R4 < ke);
-        mma::cp_async16_s(d + (unsigned)(i * R4 * BN) * 4u, v ? src : a.in, v ? 16 : 0);
-      }
-    } else if (full && q0 + BN <= g.Q) {
-      const size_t inc = (size_t)R1 * g.HW;
-#pragma unroll
-      for (int i = 0; i < kGK / R1; ++i, src += inc) mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, src, 4);
-    } else {
-      const size_t inc = (size_t)R1 * g.HW;
-#pragma unroll
-      for (int i = 0; i < kGK / R1; ++i, src += inc) {
-        const bool v = colin && k0 + row0 + i * R1 < ke;
-        mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, v ? src : a.in, v ? 4 : 0);
-      }
+    for (int k = 0; k < kHalf; ++k) v[k] = qin && k < kn ? src[(size_t)k * g.HW] : 0.f;
+  };
+  pixel(blockIdx.x);
+  if (g.first && halves) load_half(0);
+  // ---- F by items of eight k (lanes along the contiguous index): largest magnitude per row, then the planes.  In between the
+  // values wait as fp32 in the 16 bytes of hi and the 16 of lo that they become.
+  const int k8s = nch * (kTcK / 8), along = max(AK ? k8s : nt, 1), dfast = kTcThreads % along, dslow = kTcThreads / along;
+  auto each_item = [&](auto&& fn) {
+    int fast = tid % along, slow = tid / along;
+    for (int i = tid; i < nt * k8s; i += kTcThreads) {
+      const int r = AK ? slow : fast, k8 = AK ? fast : slow;
+      fn(r, k8, Bs + (k8 >> 3) * 2 * nt * 128 + r * 128 + (((k8 & 7) ^ (r & 7)) << 4));
+      fast += dfast;
+      slow += dslow;
+      if (fast >= along) { fast -= along; ++slow; }
     }
   };
-  auto load_f = [&](int st, int k0) {
-    const unsigned d0 = sbase + (unsigned)(st * kStage) * 4u;
-    // groups of 4 floats or single floats along the contiguous index; ROWS threads apart along the other
-    const auto copy = [&](auto width) {
-      constexpr int V = decltype(width)::value, COLS = (AK ? kGK : BM) / V, ROWS = AK ? BM : kGK, RT = kThreads / COLS;
-      const int c = (tid % COLS) * V, r0 = tid / COLS, ld = AK ? a.K : a.M;
-      const int kc = AK ? k0 + c : m0 + c, kr = AK ? m0 + r0 : k0 + r0;
-      const bool cin = kc < (AK ? ke : a.M);
-      const int rend = AK ? a.M : ke;
-      const float* src = a.F + (size_t)kr * ld + kc;
-      const size_t inc = (size_t)RT * ld;
-      unsigned d = d0 + (unsigned)(r0 * PA + c) * 4u;
+  each_item([&](int r, int k8, uint8_t* d) {
+    const int m = m0 + r, k = kb + k8 * 8;
+    const size_t inc = AK ? 1 : a.M;
+    const float* src = AK ? a.F + (size_t)m * a.K + k : a.F + (size_t)k * a.M + m;
+    float f[8];
+    unsigned mx = 0;
 #pragma unroll
-      for (int i = 0; i < (ROWS + RT - 1) / RT; ++i, src += inc, d += (unsigned)(RT * PA) * 4u) {
-        if (ROWS % RT && r0 + i * RT >= ROWS) break;
-        const bool v = cin && kr + i * RT < rend;
-        if (V == 4) mma::cp_async16_s(d, v ? src : a.F, v ? 16 : 0);
-        else mma::cp_async4_s(d, v ? src : a.F, v ? 4 : 0);
-      }
-    };
-    if (a.vecF) copy(std::integral_constant<int, 4>{});
-    else copy(std::integral_constant<int, 1>{});
-  };
-
-  float acc[TM][4];
+    for (int j = 0; j < 8; ++j) f[j] = m < a.M && k + j < ke ? __ldg(src + j * inc) : 0.f;
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  const int steps = ke > kb ? (ke - kb + kGK - 1) / kGK : 0;
-  for (int s = 0; s < kGS - 1; ++s)
-    if (s < steps) load_f(s, kb + s * kGK);
+    for (int j = 0; j < 8; ++j) mx = max(mx, tc::abs_bits(f[j]));
+    *reinterpret_cast<float4*>(d) = make_float4(f[0], f[1], f[2], f[3]);
+    *reinterpret_cast<float4*>(d + nt * 128) = make_float4(f[4], f[5], f[6], f[7]);
+    atomicMax(&rowmax[r], mx);
+  });
+  __syncthreads();
+  each_item([&](int r, int, uint8_t* d) { split_in_place(d, d + nt * 128, tc::exp2_int(-tc::row_exponent(rowmax[r], tc::kLeast))); });
+  if (tid < nt) {   // 2^(24 + e) of a row in two factors
+    const int e = tc::kRowShift + tc::row_exponent(rowmax[tid], tc::kLeast);
+    rowscale[tid] = make_float2(tc::exp2_int(e >> 1), tc::exp2_int(e - (e >> 1)));
+  }
+  tc::fence_proxy_async();
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  uint8_t *As = sm + (nch > 1 ? grp * 2 * kTcPlane : 0), *row = As + t * 128;
+  const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
+  const uint32_t idesc = tc::make_idesc_f16(nt);
+  float* sums = reinterpret_cast<float*>(sm);     // [nt][128], for the cluster
+  const int half = grp * (nt / 2);                // the groups read out half of the rows each
+  bool fine = true;
+  int commits = 0;                                // of this group
   grid_dependency_wait();
-  for (int s = 0; s < kGS - 1; ++s) {
-    if (s < steps) load_in(s, kb + s * kGK);
-    mma::cp_async_commit();
-  }
-  for (int s = 0; s < steps; ++s) {
-    mma::cp_async_wait<kGS - 2>();
-    __syncthreads();
-    const int nx = s + kGS - 1;
-    if (nx < steps) {
-      load_f(nx % kGS, kb + nx * kGK);
-      load_in(nx % kGS, kb + nx * kGK);
+  if (!g.first && halves) load_half(0);
+  for (int tile = blockIdx.x; tile < g.pxtiles; tile += gridDim.x) {
+    unsigned mx = 0;
+    for (int u = 0; u < halves; ++u) {
+      // c: the chunk's accumulator; the group's buffer is free when the products of its last chunk are done
+      const int c = span == kTcK ? (u >> 1) * 2 + grp : grp;
+      const bool second = span == kTcK && (u & 1);
+      if (!second) {
+        if (c >= 2) fine = tc::mbar_wait(&done[grp], (commits - 1) & 1) && fine;
+        mx = 0;
+      }
+      const int slot = slot0 + (second ? 4 : 0);
+      // the values wait as fp32 in the hi and lo bytes that they become
+#pragma unroll
+      for (int j = 0; j < kHalf / 8; ++j) {
+        uint8_t* d = row + (((slot + j) ^ (t & 7)) << 4);
+        *reinterpret_cast<float4*>(d) = make_float4(v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3]);
+        *reinterpret_cast<float4*>(d + kTcPlane) = make_float4(v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) mx = max(mx, tc::abs_bits(v[8 * j + k]));
+      }
+      if (u + 1 < halves) load_half(u + 1);
+      if (span == kTcK && !second) continue;
+      const int e = tc::row_exponent(mx, tc::kLeastConv);
+      const float sc = tc::exp2_int(-e);
+      ea[c][t] = tc::exp2_int(e - tc::kRowShift);
+#pragma unroll 2
+      for (int j = 0; j < span / 8; ++j) {
+        uint8_t* d = row + (((slot0 + j) ^ (t & 7)) << 4);
+        split_in_place(d, d + kTcPlane, sc);
+      }
+      tc::fence_proxy_async();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+      if (t == 0) {
+        tc::tc_fence_after_sync();
+        const uint32_t as = tc::smem_u32(As) + slot0 * 16, d = tmem + c * nt;
+        const uint32_t bs = tc::smem_u32(Bs) + (halved ? slot0 * 16 : c * 2 * nt * 128);
+        const uint64_t ah = d0 + (as >> 4), al = d0 + ((as + kTcPlane) >> 4), bh = d0 + (bs >> 4), bl = d0 + ((bs + nt * 128) >> 4);
+        const int kk = (min(span, ke - kb - c * span) + 15) / 16;
+        for (int i = 0; i < kk; ++i) {
+          tc::mma_f16_ss(d, al + i * 2, bh + i * 2, idesc, i > 0);
+          tc::mma_f16_ss(d, ah + i * 2, bl + i * 2, idesc, true);
+        }
+        for (int i = 0; i < kk; ++i) tc::mma_f16_ss(d, ah + i * 2, bh + i * 2, idesc, true);
+        tc::mma_commit(&done[grp]);
+      }
+      ++commits;
     }
-    mma::cp_async_commit();
-    const float* As = smem + (s % kGS) * kStage;
-    const float* Bs = As + kAF + wn * 32 + tx * 4;
+    float* out = a.out + ((size_t)n * a.M + m0) * g.HW + p;
+    const int rows = g.splits > 1 ? nt : qin ? a.M - m0 : 0;   // to be written
+    if (tile + gridDim.x < g.pxtiles) {   // the next tile's first loads, while the products run
+      pixel(tile + gridDim.x);
+      if (halves) load_half(0);
+    }
+    if (halves) fine = tc::mbar_wait(&done[grp], (commits - 1) & 1) && fine;
+    tc::tc_fence_before_sync();
+    __syncthreads();
+    tc::tc_fence_after_sync();
+    if (tile + gridDim.x >= g.pxtiles) grid_launch_dependents();
+    // ---- the accumulators of the chunks, 16 rows at a time
+    float* dst = g.splits > 1 ? sums + half * kTcPx + t : out + (size_t)half * g.HW;
+    const size_t inc = g.splits > 1 ? kTcPx : g.HW;
+    for (int c0 = half; c0 < half + nt / 2; c0 += 16) {
+      float s[16];
 #pragma unroll
-    for (int k = 0; k < kGK; k += 4) {
-      if (AK) {
-        float4 f[TM];
+      for (int j = 0; j < 16; ++j) s[j] = 0.f;
+      for (int c = 0; c < nacc; ++c) {
+        float x[16];
+        tc::tmem_ld16(lanes + c * nt + c0, x);
+        const float f = ea[c][t];
 #pragma unroll
-        for (int i = 0; i < TM; ++i) f[i] = lds4(As + (wm * 4 * TM + ty + 4 * i) * PA + k);
+        for (int j = 0; j < 16; ++j) s[j] = fmaf(x[j], f, s[j]);
+      }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4 b = lds4(Bs + (k + u) * BN);
-#pragma unroll
-          for (int i = 0; i < TM; ++i) fma4(acc[i], u == 0 ? f[i].x : u == 1 ? f[i].y : u == 2 ? f[i].z : f[i].w, b);
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4 b = lds4(Bs + (k + u) * BN);
-#pragma unroll
-          for (int i = 0; i < TM; i += 4) {
-            const float4 f = lds4(As + (k + u) * PA + wm * 4 * TM + ty * TM + i);
-            fma4(acc[i], f.x, b);
-            fma4(acc[i + 1], f.y, b);
-            fma4(acc[i + 2], f.z, b);
-            fma4(acc[i + 3], f.w, b);
-          }
-        }
+      for (int j = 0; j < 16; j += 2) {
+        const float4 f = *reinterpret_cast<const float4*>(rowscale + c0 + j);
+        const float y0 = s[j] * f.x * f.y, y1 = s[j + 1] * f.z * f.w;
+        if (c0 + j < rows) *dst = y0;
+        dst += inc;
+        if (c0 + j + 1 < rows) *dst = y1;
+        dst += inc;
       }
     }
+    tc::tc_fence_before_sync();
+    __syncthreads();   // the accumulators and ea are free
+    tc::tc_fence_after_sync();
   }
-  mma::cp_async_wait<0>();
-  grid_launch_dependents();
-  if (g.splits > 1) {
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int m = wm * 4 * TM + (AK ? ty + 4 * i : ty * TM + i);
-      *reinterpret_cast<float4*>(smem + m * BN + wn * 32 + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    }
-    cluster_sum(smem, BM * BN, g.splits, tid, kThreads, [&](int i, float v) {
-      const int m = m0 + i / BN, q = q0 + i % BN;
+  if (!fine) atomicCAS(&g_planes_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
+  if (warp == 0) tc::tmem_dealloc(tmem, g.cols);
+  if (g.splits > 1)
+    cluster_sum(sums, nt * kTcPx, g.splits, tid, kTcThreads, [&](int i, float x) {
+      const int m = m0 + i / kTcPx, q = blockIdx.x * kTcPx + i % kTcPx;
       if (m < a.M && q < g.Q) {
         const int nn = q / g.HW;
-        a.out[((size_t)nn * a.M + m) * g.HW + (q - nn * g.HW)] = v;
+        a.out[((size_t)nn * a.M + m) * g.HW + (q - nn * g.HW)] = x;
       }
     });
-    return;
-  }
-  // this thread's four pixels
-  const int q = q0 + wn * 32 + tx * 4;
-  size_t o[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int nn = (q + j) / g.HW;
-    o[j] = (size_t)nn * a.M * g.HW + (q + j - nn * g.HW);
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + wm * 4 * TM + (AK ? ty + 4 * i : ty * TM + i);
-    if (m >= a.M) continue;
-    float* d = a.out + (size_t)m * g.HW;
-    if (a.vecOut) {
-      if (q < g.Q) *reinterpret_cast<float4*>(d + o[0]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (q + j < g.Q) d[o[j]] = acc[i][j];
-    }
-  }
 }
 
 // ---- the stencils --------------------------------------------------------------------------------------------------------
@@ -306,123 +355,186 @@ __global__ void __launch_bounds__(kThreads) plane_stencil_kernel(const __grid_co
 }
 
 // ---- partial factor gradients: part[split][row][r] = sum over a pixel range of D[row][q] Z[r][q] ------------------------
-// Both operands have the pixels contiguous, so a lane reads four pixels of a row at once: 8 + TN reads of 16 bytes (one
-// wavefront each: the pitch of 36 floats puts eight consecutive rows on all banks) per 32*TN FFMA.  The running sum of a
-// group of eight stages (256 pixels) is added to the total separately: a plain chain over thousands of pixels would round
-// more than the split tensor-core sums this kernel replaces.
+// On the tensor cores: 128 rows of dU or X and NT ranks per CTA, K = pixels, which both operands have contiguous.  A warp
+// takes a row at a time: 64 pixels, two per lane, their largest magnitude by one warp reduction, and 4 bytes of each plane per
+// lane.  A chunk of 64 pixels has an accumulator of its own in half of TMEM (two CTAs per SM); once these are used up
+// they are added to totals in registers, each with the powers of two of its row and its rank in that chunk.
+//
+// What bounds it is the splitting (about 25 instructions per row and chunk) and latency: 64 x 256 14x14 at R = 32 19 us on FFMA,
+// 1x here; 16 x 256 -> 384 27x27 at R = 50 (4-byte loads) 35 and 1x.
 struct PlaneGrad {
   const float* D[2];     // dU, X
   const float* Z[2];     // Z, Zt
   float* part;
   int rows[2], mtiles[2], row0[2];
-  int vecD[2], vecZ;
-  int R, rtiles, HW, Q, per;
+  int R, rtiles, HW, Q, per;   // per: pixels of a split, a multiple of 64
   size_t nrows;          // T + C
 };
-constexpr int kDK = 32, kDP = kDK + 4, kDS = 3;
+constexpr int kGradThreads = 256, kGradRows = 128;
+constexpr int kGradShift = 12;   // between the two powers of two of a sum, for values near the ends of the range
 
-template <int TN, int WM, int WN>
-__global__ void __launch_bounds__(kThreads) plane_grad_kernel(const __grid_constant__ PlaneGrad g) {
-  constexpr int BM = 32 * WM, BN = 8 * TN * WN, kStage = (BM + BN) * kDP;
-  static_assert(WM * WN == 4, "");
-  extern __shared__ __align__(16) float smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp / WN, wn = warp % WN;
-  const int ty = lane >> 3, tx = lane & 7;
+template <int NT>
+struct GradTile {
+  static constexpr int chunks = 256 / NT;                            // accumulators
+  static constexpr int bplane = NT * 128;
+  static constexpr int stage = 2 * (kTcPlane + bplane);
+  static constexpr size_t smem = 1024 + 2 * (size_t)stage;           // at least the [128][NT + 1] floats of the result
+};
+
+template <int NT>
+__global__ void __launch_bounds__(kGradThreads, 2) plane_grad_kernel(const __grid_constant__ PlaneGrad g) {
+  using T = GradTile<NT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t done[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ float fa[T::chunks][kGradRows];
+  __shared__ __align__(16) float fb[T::chunks][NT];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = warp >> 2;
   const int rt = blockIdx.x % g.rtiles, mi = blockIdx.x / g.rtiles, half = mi >= g.mtiles[0] ? 1 : 0;
-  const int m0 = (mi - (half ? g.mtiles[0] : 0)) * BM, r0 = rt * BN, rows = half ? g.rows[1] : g.rows[0];
+  const int m0 = (mi - (half ? g.mtiles[0] : 0)) * kGradRows, r0 = rt * NT, rows = half ? g.rows[1] : g.rows[0];
   const int qb = blockIdx.y * g.per, qe = min(g.Q, qb + g.per);
-  const float* D = half ? g.D[1] : g.D[0];
-  const float* Z = half ? g.Z[1] : g.Z[0];
-  const bool vecD = half ? g.vecD[1] : g.vecD[0], vecZ = g.vecZ;
-  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
-  // rows base .. base + NB - 1 of src [n][total][HW], 32 pixels from q0 on; a full tile needs no predicates, which with
-  // the 4-byte copies (H * W not a multiple of 4) are most of the instructions around the FFMA (16 x 256 -> 384 27x27 R = 50: 58 -> 35 us)
-  auto load = [&](auto nb, unsigned dst, const float* src, int base, int total, int q0, bool vec) {
-    constexpr int NB = decltype(nb)::value;
-    const int step = vec ? kThreads / 8 : kThreads / 32, i0 = vec ? tid >> 3 : tid >> 5;
-    const int col = vec ? (tid & 7) * 4 : tid & 31, q = q0 + col, n = q / g.HW;
-    const float* s = src + ((size_t)n * total + base + i0) * g.HW + (q - n * g.HW);
-    const size_t inc = (size_t)step * g.HW;
-    unsigned d = dst + (unsigned)(i0 * kDP + col) * 4u;
-    const bool qin = q < qe;
-    if (vec) {
+  const float* D = (half ? g.D[1] : g.D[0]) + (size_t)m0 * g.HW;
+  const float* Z = (half ? g.Z[1] : g.Z[0]) + (size_t)r0 * g.HW;
+  const int arows = min(kGradRows, rows - m0), brows = min(NT, g.R - r0);
+  if (tid == 0) {
+    tc::mbar_init(&done[0], 1);
+    tc::mbar_init(&done[1], 1);
+    tc::fence_barrier_init();
+  }
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, 256);
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
+  const uint32_t idesc = tc::make_idesc_f16(NT);
+  const int steps = qe > qb ? (qe - qb + kTcK - 1) / kTcK : 0;
+  float tot[NT / 2];
 #pragma unroll
-      for (int i = 0; i < NB / (kThreads / 8); ++i, s += inc, d += (kThreads / 8) * kDP * 4u) {
-        const bool v = qin && base + i0 + i * (kThreads / 8) < total;
-        mma::cp_async16_s(d, v ? s : src, v ? 16 : 0);
-      }
-    } else if (base + NB <= total && q0 + kDK <= qe) {
+  for (int j = 0; j < NT / 2; ++j) tot[j] = 0.f;
+  bool fine = true;
+  // eight rows at a time, the rows of D and then those of Z; the next eight (of the next chunk after the last) are on their way
+  // while eight are split
+  constexpr int kGroups = (kGradRows + NT) / 8, kWarps = kGradThreads / 32;
+  size_t a0 = 0, a1 = 0, b0 = 0, b1 = 0;   // this lane's two pixels of the chunk that is loaded
+  bool in0 = false, in1 = false;
+  auto pixels = [&](int s) {
+    const int q = qb + s * kTcK + lane * 2;
+    in0 = q < qe;
+    in1 = q + 1 < qe;
+    const int n0 = in0 ? q / g.HW : 0, n1 = in1 ? (q + 1) / g.HW : 0, p0 = in0 ? q - n0 * g.HW : 0, p1 = in1 ? q + 1 - n1 * g.HW : 0;
+    a0 = (size_t)n0 * rows * g.HW + p0; a1 = (size_t)n1 * rows * g.HW + p1;
+    b0 = (size_t)n0 * g.R * g.HW + p0; b1 = (size_t)n1 * g.R * g.HW + p1;
+  };
+  float x[8], y[8];
+  auto load_rows = [&](int i) {
+    const bool isb = i >= kGradRows / 8;
+    const int first = (isb ? i - kGradRows / 8 : i) * 8, have = isb ? brows : arows;
+    const float* src = (isb ? Z : D) + (size_t)first * g.HW;
+    const float *s0 = src + (isb ? b0 : a0), *s1 = src + (isb ? b1 : a1);
 #pragma unroll
-      for (int i = 0; i < NB / (kThreads / 32); ++i, s += inc, d += (kThreads / 32) * kDP * 4u) mma::cp_async4_s(d, s, 4);
-    } else {
-#pragma unroll
-      for (int i = 0; i < NB / (kThreads / 32); ++i, s += inc, d += (kThreads / 32) * kDP * 4u) {
-        const bool v = qin && base + i0 + i * (kThreads / 32) < total;
-        mma::cp_async4_s(d, v ? s : src, v ? 4 : 0);
-      }
+    for (int k = 0; k < 8; ++k) {
+      const bool row = first + k < have;
+      x[k] = row && in0 ? s0[(size_t)k * g.HW] : 0.f;
+      y[k] = row && in1 ? s1[(size_t)k * g.HW] : 0.f;
     }
   };
-  auto load_stage = [&](int st, int q) {
-    const unsigned d = sbase + (unsigned)(st * kStage) * 4u;
-    load(std::integral_constant<int, BM>{}, d, D, m0, rows, q, vecD);
-    load(std::integral_constant<int, BN>{}, d + BM * kDP * 4u, Z, r0, g.R, q, vecZ);
-  };
-  float acc[8][TN], total[8][TN];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = total[i][j] = 0.f;
-  auto flush = [&] {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        total[i][j] += acc[i][j];
-        acc[i][j] = 0.f;
-      }
-  };
-  const int steps = qe > qb ? (qe - qb + kDK - 1) / kDK : 0;
   grid_dependency_wait();
-  for (int s = 0; s < kDS - 1; ++s) {
-    if (s < steps) load_stage(s, qb + s * kDK);
-    mma::cp_async_commit();
+  if (steps) {
+    pixels(0);
+    load_rows(warp);
   }
   for (int s = 0; s < steps; ++s) {
-    mma::cp_async_wait<kDS - 2>();
-    __syncthreads();
-    const int nx = s + kDS - 1;
-    if (nx < steps) load_stage(nx % kDS, qb + nx * kDK);
-    mma::cp_async_commit();
-    const float* As = smem + (s % kDS) * kStage + (wm * 32 + ty) * kDP;
-    const float* Bs = smem + (s % kDS) * kStage + (BM + wn * 8 * TN + tx) * kDP;
+    const int st = s & 1, c = s % T::chunks;
+    uint8_t* As = sm + st * T::stage;
+    if (s >= 2) fine = tc::mbar_wait(&done[st], (s / 2 - 1) & 1) && fine;
+#pragma unroll 1
+    for (int i = warp; i < kGroups; i += kWarps) {
+      const bool isb = i >= kGradRows / 8;
+      const int first = (isb ? i - kGradRows / 8 : i) * 8;
+      float u[8], v[8];
 #pragma unroll
-    for (int k = 0; k < kDK; k += 4) {
-      float4 b[TN];
+      for (int k = 0; k < 8; ++k) { u[k] = x[k]; v[k] = y[k]; }
+      if (i + kWarps < kGroups) {
+        load_rows(i + kWarps);
+      } else if (s + 1 < steps) {
+        pixels(s + 1);
+        load_rows(warp);
+      }
+      uint8_t* d = As + (isb ? 2 * kTcPlane : 0) + first * 128;
+      const uint32_t lo = isb ? T::bplane : kTcPlane;
+      int mine = 0;
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = lds4(Bs + j * 8 * kDP + k);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 a = lds4(As + i * 4 * kDP + k);
-#pragma unroll
-        for (int j = 0; j < TN; ++j)
-          acc[i][j] = fmaf(a.w, b[j].w, fmaf(a.z, b[j].z, fmaf(a.y, b[j].y, fmaf(a.x, b[j].x, acc[i][j]))));
+      for (int k = 0; k < 8; ++k) {
+        const int e = tc::row_exponent(__reduce_max_sync(0xffffffffu, max(tc::abs_bits(u[k]), tc::abs_bits(v[k]))), tc::kLeastConv);
+        if (lane == k) mine = e;
+        const float sc = tc::exp2_int(-e), p = u[k] * sc, q = v[k] * sc;
+        const __half2 h = __floats2half2_rn(p, q);
+        const float2 f = __half22float2(h);
+        uint8_t* o = d + k * 128 + (((lane >> 2) ^ k) << 4) + (lane & 3) * 4;
+        *reinterpret_cast<__half2*>(o) = h;
+        *reinterpret_cast<__half2*>(o + lo) = __floats2half2_rn(p - f.x, q - f.y);
+      }
+      if (lane < 8) {
+        if (isb) fb[c][first + lane] = tc::exp2_int(mine + kGradShift);
+        else fa[c][first + lane] = tc::exp2_int(mine - kGradShift);
       }
     }
-    if ((s & 7) == 7) flush();
-  }
-  flush();
-  mma::cp_async_wait<0>();
-  grid_launch_dependents();
-  float* out = g.part + ((size_t)blockIdx.y * g.nrows + (half ? g.row0[1] : 0)) * g.R;
+    tc::fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      tc::tc_fence_after_sync();
+      const uint32_t as = tc::smem_u32(As), bs = as + 2 * kTcPlane, d = tmem + c * NT;
+      const uint64_t ah = d0 + (as >> 4), al = d0 + ((as + kTcPlane) >> 4), bh = d0 + (bs >> 4), bl = d0 + ((bs + T::bplane) >> 4);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int m = m0 + wm * 32 + ty + 4 * i;
-    if (m >= rows) continue;
+      for (int i = 0; i < kTcK / 16; ++i) {
+        tc::mma_f16_ss(d, al + i * 2, bh + i * 2, idesc, i > 0);
+        tc::mma_f16_ss(d, ah + i * 2, bl + i * 2, idesc, true);
+      }
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int r = r0 + wn * 8 * TN + tx + 8 * j;
-      if (r < g.R) out[(size_t)m * g.R + r] = total[i][j];
+      for (int i = 0; i < kTcK / 16; ++i) tc::mma_f16_ss(d, ah + i * 2, bh + i * 2, idesc, true);
+      tc::mma_commit(&done[st]);
     }
+    if (c + 1 < T::chunks && s + 1 < steps) continue;
+    // the accumulators, in the order of the pixels
+    fine = tc::mbar_wait(&done[st], (s / 2) & 1) && fine;
+    tc::tc_fence_after_sync();
+    for (int k = 0; k <= c; ++k) {
+      const float f = fa[k][(warp & 3) * 32 + lane];
+#pragma unroll
+      for (int j0 = 0; j0 < NT / 2; j0 += 16) {
+        float v[16];
+        tc::tmem_ld16(lanes + k * NT + grp * (NT / 2) + j0, v);
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          const float4 w = lds4(&fb[k][grp * (NT / 2) + j0 + j]);
+          tot[j0 + j] = fmaf(v[j], f * w.x, tot[j0 + j]);
+          tot[j0 + j + 1] = fmaf(v[j + 1], f * w.y, tot[j0 + j + 1]);
+          tot[j0 + j + 2] = fmaf(v[j + 2], f * w.z, tot[j0 + j + 2]);
+          tot[j0 + j + 3] = fmaf(v[j + 3], f * w.w, tot[j0 + j + 3]);
+        }
+      }
+    }
+    tc::tc_fence_before_sync();
+    __syncthreads();   // the accumulators and the powers of two are free
+  }
+  if (!fine) atomicCAS(&g_planes_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
+  grid_launch_dependents();
+  // through shared memory, for stores along the rows
+  float* tile = reinterpret_cast<float*>(sm);   // [128][NT + 1]
+#pragma unroll
+  for (int j = 0; j < NT / 2; ++j) tile[((warp & 3) * 32 + lane) * (NT + 1) + grp * (NT / 2) + j] = tot[j];
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc::tc_fence_after_sync();
+    tc::tmem_dealloc(tmem, 256);
+  }
+  float* out = g.part + ((size_t)blockIdx.y * g.nrows + (half ? g.row0[1] : 0) + m0) * g.R + r0;
+  for (int i = tid; i < arows * NT; i += kGradThreads) {
+    const int m = i / NT, r = i % NT;
+    if (r < brows) out[(size_t)m * g.R + r] = tile[m * (NT + 1) + r];
   }
 }
 
@@ -484,60 +596,72 @@ __global__ void __launch_bounds__(256) plane_reduce_kernel(const PlaneReduce g) 
 // ---- launches --------------------------------------------------------------------------------------------------------------
 bool aligned16(const void* p) { return !(reinterpret_cast<uintptr_t>(p) & 15); }
 
-int gemm_launch(PlaneGemm g, int nprod, bool ak, bool programmatic, const DeviceInfo& di, cudaStream_t st) {
+// Rows of a tile, the cluster split and the launch.
+int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo& di, cudaStream_t st) {
   int M = 0, K = 0;
   for (int i = 0; i < nprod; ++i) {
     M = std::max(M, g.p[i].M);
     K = std::max(K, g.p[i].K);
   }
-  // the smallest row tile that holds all rows, at most 64; row and pixel tiles trade off at 128 threads
-  const int bm = M <= 16 ? 16 : M <= 32 ? 32 : 64, bn = bm == 64 ? 64 : 128;
+  const int pxt = ceil_div(g.Q, kTcPx), kchunks = ceil_div(K, kTcK);
+  // outputs: half of TMEM, for two CTAs per SM; ranks: all of them in one tile, which reads the channels once
+  const int most = ak ? 256 : 512;
+  g.nt = (int)align_up(std::min(M, 256), 32);
+  auto fit = [&] {
+    g.chunks = ceil_div(kchunks, g.splits);
+    while (std::max(g.chunks, 2) * g.nt > most && g.nt > 32) g.nt = (int)align_up(g.nt / 2, 32);
+  };
+  g.splits = 1;
+  fit();
   long tiles = 0;
+  for (int i = 0; i < nprod; ++i) tiles += (long)ceil_div(g.p[i].M, g.nt) * pxt;
+  g.splits = pick_cluster(tiles, kchunks, 1, di.sm_count);
+  while (ceil_div(kchunks, g.splits) > kTcMaxChunks && g.splits < 8) g.splits *= 2;
+  g.nt = (int)align_up(std::min(M, 256), 32);
+  fit();
+  if (g.chunks > kTcMaxChunks) return fail(B200CP_ERR_UNSUPPORTED, "cp planes: %d channels", K);
   g.maxmt = 0;
   for (int i = 0; i < nprod; ++i) {
-    PlaneProduct& p = g.p[i];
-    p.mtiles = ceil_div(p.M, bm);
-    g.maxmt = std::max(g.maxmt, p.mtiles);
-    tiles += (long)p.mtiles * ceil_div(g.Q, bn);
-    p.vecF = !((ak ? p.K : p.M) & 3) && aligned16(p.F);
-    p.vecIn = !(g.HW & 3) && aligned16(p.in);
-    p.vecOut = !(g.HW & 3) && aligned16(p.out);
+    g.p[i].mtiles = ceil_div(g.p[i].M, g.nt);
+    g.p[i].kper = g.chunks * kTcK;
+    g.maxmt = std::max(g.maxmt, g.p[i].mtiles);
   }
-  // two CTAs of 128 threads and more per SM are needed to hide the FFMA and shared-memory latency
-  g.splits = pick_cluster(tiles, K, 2 * kGK, 3 * di.sm_count);
-  for (int i = 0; i < nprod; ++i) g.p[i].kper = (int)align_up((size_t)ceil_div(g.p[i].K, g.splits), kGK);
-  const dim3 grid((unsigned)((long)g.maxmt * ceil_div(g.Q, bn)), 1, nprod * g.splits);
-#define PLANE_GEMM(TM, WM, WN)                                                                                          \
-  do {                                                                                                                 \
-    if (ak) B200CP_CUDA_OK(launch_cluster(plane_gemm_kernel<TM, WM, WN, true>, grid, dim3(kThreads), 0, st, g.splits,   \
-                                          programmatic, g));                                                           \
-    else B200CP_CUDA_OK(launch_cluster(plane_gemm_kernel<TM, WM, WN, false>, grid, dim3(kThreads), 0, st, g.splits,     \
-                                       programmatic, g));                                                              \
+  for (g.cols = 32; g.cols < std::max(g.chunks, 2) * g.nt;) g.cols *= 2;
+  g.pxtiles = pxt;
+  const size_t smem = 1024 + std::max<size_t>((g.chunks > 1 ? 4 : 2) * kTcPlane + (size_t)g.chunks * 2 * g.nt * 128,
+                                              g.splits > 1 ? sizeof(float) * g.nt * kTcPx : 0);
+  // a CTA per tile, or as many as are resident at once and walk the tiles
+  const int per_sm = g.cols > 256 || smem > 100 * 1024 ? 1 : 2;
+  const int walkers = g.splits > 1 ? pxt : std::min(pxt, std::max(1, per_sm * di.sm_count / (g.maxmt * nprod)));
+  const dim3 grid((unsigned)ceil_div(pxt, ceil_div(pxt, walkers)), g.maxmt, nprod * g.splits);
+#define PLANE_TC(AK)                                                                                                     \
+  do {                                                                                                                  \
+    static std::atomic<int> set[64];                                                                                    \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(plane_tc_kernel<AK>), set, (int)smem));            \
+    B200CP_CUDA_OK(launch_cluster(plane_tc_kernel<AK>, grid, dim3(kTcThreads), smem, st, g.splits, programmatic, g));   \
   } while (0)
-  if (bm == 16) PLANE_GEMM(4, 1, 4);
-  else if (bm == 32) PLANE_GEMM(8, 1, 4);
-  else PLANE_GEMM(8, 2, 2);
-#undef PLANE_GEMM
-  B200CP_LAUNCH_OK("plane_gemm_kernel");
+  if (ak) PLANE_TC(true);
+  else PLANE_TC(false);
+#undef PLANE_TC
+  B200CP_LAUNCH_OK("plane_tc_kernel");
   return B200CP_OK;
 }
 
 struct GradPlan {
-  int bm, bn, mt0, mt1, rtiles, splits, per;   // gradient products
+  int bn, mt0, mt1, rtiles, splits, per;       // gradient products
   int units, chunks, cper;                     // stencil ranges
 };
 GradPlan grad_plan(const b200cp_tensor_shape& s, int sm_count) {
   GradPlan p{};
   const int R = (int)s.Rank, Q = (int)(s.N * s.H * s.W);
-  p.bn = R <= 16 ? 16 : R <= 32 ? 32 : 64;
-  p.bm = p.bn == 64 ? 64 : 128;
-  p.mt0 = ceil_div((int)s.T, p.bm);
-  p.mt1 = ceil_div((int)s.C, p.bm);
+  p.bn = R <= 32 ? 32 : 64;
+  p.mt0 = ceil_div((int)s.T, kGradRows);
+  p.mt1 = ceil_div((int)s.C, kGradRows);
   p.rtiles = ceil_div(R, p.bn);
   const int tiles = (p.mt0 + p.mt1) * p.rtiles;
-  // three CTAs per SM (shared memory), at least two stages each
-  const int want = std::max(1, std::min({3 * sm_count / tiles, ceil_div(Q, 2 * kDK), 65535}));
-  p.per = (int)align_up((size_t)ceil_div(Q, want), kDK);
+  // two CTAs per SM, at least two chunks each
+  const int want = std::max(1, std::min({2 * sm_count / tiles, ceil_div(Q, 2 * kTcK), 65535}));
+  p.per = (int)align_up((size_t)ceil_div(Q, want), kTcK);
   p.splits = ceil_div(Q, p.per);
   p.units = (int)s.N * ceil_div((int)s.H, 4) * (int)s.W;
   const int cw = std::max(1, std::min({ceil_div(8 * sm_count, R), ceil_div(p.units, kThreads), 65535}));
@@ -579,7 +703,8 @@ Buffers carve(Carve& c, const b200cp_tensor_shape& s, bool P, bool Q, bool Z, bo
 bool planes_supported(const b200cp_tensor_shape& s) {
   const size_t HW = (size_t)s.H * s.W, most = std::max({s.T, s.C, s.Rank});
   return s.Y == 3 && s.X == 3 && s.pad == 1 && (size_t)s.N * (s.H + 3) * s.W < (1u << 30) && s.Rank < 65536 &&
-         ((size_t)s.T + s.C) * s.Rank < (1u << 30) && (most / 16 + 1) * (s.N * HW / 64 + 1) < (1u << 30);
+         ((size_t)s.T + s.C) * s.Rank < (1u << 30) && most <= 8 * kTcMaxChunks * kTcK &&
+         (most / 16 + 1) * (s.N * HW / 64 + 1) < (1u << 30);
 }
 
 // `parts`: what the call computes (the workspace of more parts is enough for fewer)
@@ -606,18 +731,19 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   const float* Q = j.Q ? j.Q : j.Qsave ? j.Qsave : b.Q;
   const int R = (int)s.Rank, T = (int)s.T, C = (int)s.C, HW = (int)(s.H * s.W), NQ = (int)s.N * HW;
   bool chained = false;
-  PlaneGemm g{};
+  PlaneTc g{};
   g.HW = HW;
   g.Q = NQ;
   int np = 0;
   auto product = [&](const float* F, const float* in, float* out, int M, int K) {
-    PlaneProduct& p = g.p[np++];
+    PlaneTcProduct& p = g.p[np++];
     p.F = F; p.in = in; p.out = out; p.M = M; p.K = K;
   };
   if (needP && !j.P) product(j.K1, j.X, j.Psave ? j.Psave : b.P, R, C);
   if (needQ && !j.Q) product(j.K0, j.dU, j.Qsave ? j.Qsave : b.Q, R, T);
   if (np) {
-    if (int rc = gemm_launch(g, np, false, false, di, st)) return rc;
+    g.first = 1;
+    if (int rc = tc_launch(g, np, false, false, di, st)) return rc;
     chained = true;
   }
   const GradPlan gp = grad_plan(s, di.sm_count);
@@ -635,31 +761,28 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   }
   B200CP_LAUNCH_OK("plane_stencil_kernel");
   np = 0;
+  g.first = 0;
   if (fwd) product(j.K0, b.Z, j.U, T, R);
   if (bwd) product(j.K1, b.Zt, j.dX, C, R);
   if (np)
-    if (int rc = gemm_launch(g, np, true, true, di, st)) return rc;
+    if (int rc = tc_launch(g, np, true, true, di, st)) return rc;
   if (!grads) return B200CP_OK;
   PlaneGrad d{};
   d.D[0] = j.dU; d.D[1] = j.X; d.Z[0] = b.Z; d.Z[1] = b.Zt;
   d.part = b.part;
   d.rows[0] = T; d.rows[1] = C; d.row0[1] = T;
   d.mtiles[0] = gp.mt0; d.mtiles[1] = gp.mt1;
-  d.vecZ = !(HW & 3);
-  for (int i = 0; i < 2; ++i) d.vecD[i] = !(HW & 3) && aligned16(d.D[i]);
   d.R = R; d.rtiles = gp.rtiles; d.HW = HW; d.Q = NQ; d.per = gp.per;
   d.nrows = (size_t)T + C;
   const dim3 grid((gp.mt0 + gp.mt1) * gp.rtiles, gp.splits);
-  const size_t smem = sizeof(float) * kDS * (gp.bm + gp.bn) * kDP;
-#define PLANE_GRAD(TN, WM, WN)                                                                                           \
-  do {                                                                                                                  \
-    static std::atomic<int> set[64];                                                                                    \
-    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(plane_grad_kernel<TN, WM, WN>), set, (int)smem));  \
-    B200CP_CUDA_OK(launch_kernel(plane_grad_kernel<TN, WM, WN>, grid, dim3(kThreads), smem, st, true, d));              \
+#define PLANE_GRAD(NT)                                                                                                  \
+  do {                                                                                                                 \
+    static std::atomic<int> set[64];                                                                                   \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(plane_grad_kernel<NT>), set, (int)GradTile<NT>::smem)); \
+    B200CP_CUDA_OK(launch_kernel(plane_grad_kernel<NT>, grid, dim3(kGradThreads), GradTile<NT>::smem, st, true, d));   \
   } while (0)
-  if (gp.bn == 16) PLANE_GRAD(2, 4, 1);
-  else if (gp.bn == 32) PLANE_GRAD(4, 4, 1);
-  else PLANE_GRAD(4, 2, 2);
+  if (gp.bn == 32) PLANE_GRAD(32);
+  else PLANE_GRAD(64);
 #undef PLANE_GRAD
   B200CP_LAUNCH_OK("plane_grad_kernel");
   PlaneReduce r{};
@@ -668,6 +791,15 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   r.eblocks = ceil_div(r.entries, 32);
   B200CP_CUDA_OK(launch_kernel(plane_reduce_kernel, dim3(r.eblocks + ceil_div(R, 32)), dim3(32, 8), 0, st, true, r));
   B200CP_LAUNCH_OK("plane_reduce_kernel");
+  return B200CP_OK;
+}
+
+// Reads (and clears) the status word of the tensor-core products; the caller has synchronised the device.
+int planes_device_status(int* out) {
+  int v = 0, zero = 0;
+  B200CP_CUDA_OK(cudaMemcpyFromSymbol(&v, g_planes_status, sizeof(int)));
+  if (v) B200CP_CUDA_OK(cudaMemcpyToSymbol(g_planes_status, &zero, sizeof(int)));
+  *out = v;
   return B200CP_OK;
 }
 

@@ -20,5 +20,6 @@ enum { kPlanesFwd = 1, kPlanesBwd = 2, kPlanesGrads = 4, kPlanesNoP = 8, kPlanes
 bool planes_supported(const b200cp_tensor_shape& s);
 size_t planes_workspace(const b200cp_tensor_shape& s, int parts);
 int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st);
+int planes_device_status(int* out);
 
 }  // namespace b200cp

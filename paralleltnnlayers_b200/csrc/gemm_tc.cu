@@ -21,8 +21,6 @@
 // tiles 348 us; with eight read-out warps of 128 columns instead of sixteen 317 against 307.
 // Roles (TMA warp, MMA warp, read-out warps) meet only through mbarriers; every wait is bounded, and a wait that
 // runs out sets a status word and lets the CTA leave through its normal exit (TMEM released).
-#include <cuda_fp16.h>
-
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -40,7 +38,6 @@ using namespace tc;
 
 constexpr int kBM = 256;              // rows of a pair's tile: 128 per CTA
 constexpr int kKS = 64;               // K of one step: 128 bytes of fp16
-constexpr int kRowShift = 24;         // see SplitGemm::ea
 constexpr int kAPlane = 128 * 128;    // bytes of one plane (hi or lo) of A in a stage
 
 template <int BN>
@@ -166,14 +163,6 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, uin
       }
     }
   }
-}
-
-// 2^e for e in [-126, 127]
-__device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
-// v * 2^e for e in [-252, 254], in two steps of the same sign
-__device__ __forceinline__ float scale_by(float v, int e) {
-  const int h = e >> 1;
-  return v * exp2_int(h) * exp2_int(e - h);
 }
 
 __device__ __forceinline__ int tap_shift(const SplitGemm& g, int tap);
@@ -469,13 +458,6 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
 }
 
 // ---- operand planes -----------------------------------------------------------------------------------------------------
-// Exponent e of a row whose largest magnitude has these bits: x * 2^-e is below 2^15.  (Infinities and NaN leave the
-// finite values of their row in range and themselves non-finite.)
-__device__ __forceinline__ int row_exponent(unsigned bits, int least) {
-  return bits == 0 ? 0 : max((int)(bits >> 23) - 141, least);
-}
-constexpr int kLeast = -126, kLeastConv = -100;   // 2^-e and (convolutions) 2^(e - 24) stay normal numbers
-
 struct alignas(8) Half4 {
   __half2 a, b;
 };
@@ -487,7 +469,6 @@ __device__ __forceinline__ void split4(float4 v, float sc, Half4& hi, Half4& lo)
   lo.a = __floats2half2_rn(v.x - p.x, v.y - p.y);
   lo.b = __floats2half2_rn(v.z - q.x, v.w - q.y);
 }
-__device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned max4(unsigned m, float4 v) {
   return max(max(max(m, abs_bits(v.x)), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
 }

@@ -6,6 +6,7 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -150,6 +151,51 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // half an ulp added to the magnitude bits, low 13 bits cut (two integer instructions).
 __device__ __forceinline__ float tf32_hi(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+}
+
+// ---- scaled fp16 split: x = (hi + lo) * 2^e with one exponent per row (gemm_tc.cu) ---------------------------------
+// 2^e for e in [-126, 127]
+__device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
+// v * 2^e for e in [-252, 254], in two steps of the same sign
+__device__ __forceinline__ float scale_by(float v, int e) {
+  const int h = e >> 1;
+  return v * exp2_int(h) * exp2_int(e - h);
+}
+
+// Exponent e of a row whose largest magnitude has these bits: x * 2^-e is below 2^15.  (Infinities and NaN leave the
+// finite values of their row in range and themselves non-finite.)
+__device__ __forceinline__ int row_exponent(unsigned bits, int least) {
+  return bits == 0 ? 0 : max((int)(bits >> 23) - 141, least);
+}
+constexpr int kLeast = -126, kLeastConv = -100;   // 2^-e and (convolutions) 2^(e - 24) stay normal numbers
+
+__device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+constexpr int kRowShift = 24;   // of totals that take a power of two per step: see SplitGemm::ea
+// eight scaled values to 16 bytes of hi and of lo
+__device__ __forceinline__ void split8(const float* v, float sc, uint4& hi, uint4& lo) {
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = v[2 * i] * sc, b = v[2 * i + 1] * sc;
+    const __half2 t = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(t);
+    const __half2 r = __floats2half2_rn(a - f.x, b - f.y);
+    h[i] = *reinterpret_cast<const uint32_t*>(&t);
+    l[i] = *reinterpret_cast<const uint32_t*>(&r);
+  }
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+// Instruction descriptor for kind::f16 with K-major fp16 operands and fp32 accumulation, M = 128 (one CTA).
+__host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+      : "memory");
 }
 
 }  // namespace tc
