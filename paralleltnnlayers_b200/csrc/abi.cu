@@ -100,17 +100,18 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // Which 3x3 / pad 1 convolutions and backward passes run as products over whole rank planes (cp_planes.cu); B200CP_PLANES=0
 // switches them off, 2 takes them wherever they can run.  The tile and row kernels they compete with keep a plane in shared
 // memory and do the three phases in one launch (5 us for a small convolution); the products have a fixed cost of three to five
-// dependent launches (about 20 us for a convolution), and after that cost little per rank and channel.  The more ranks and
-// channels a pixel has, the sooner they win; with more pixels the fixed cost counts for less.
-// The lines are the best ones over 620 random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together, ranks
-// 6 to 128), each measured both ways; against the better form of each shape the choice costs 2 % for a convolution, 1 % for
-// a step or a layer, 0.6 % for a three-factor layer (geometric mean).  Tile or row kernels / products, us:
-//   ranks       6-16    17-32   33-64   65-128   (sums over the shapes of one sample, of 73, 57, 36, 54)
-//   convolution 1148/1619  1148/1230  1126/860  4350/1989
-//   step        3334/4656  3657/3343  3846/2267  12037/4992
-//   gradients   2897/3671  3110/2636  3259/1808  8777/3821
-//   layer       4017/5548  4164/4072  4255/2798  13463/6167
-//   layer (3)   5442/5528  5340/4058  5583/2793  17411/6153
+// dependent launches (about 20 us for a convolution), and after that cost little per rank and channel.  More ranks and
+// channels per pixel speak for them.  From 17 ranks on the fixed cost counts for less with more pixels; up to 16, where a
+// tile kernel holds every rank of its pixels in one tile, more pixels speak for the tile kernels, which then fill the GPU.
+// The lines are the best ones over 520 random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together,
+// ranks 4 to 128), each measured both ways; against the better form of each shape the choice costs 2 % for a convolution or a
+// step, 1 % for a layer or the gradients (geometric mean).  Tile or row kernels / products, us:
+//   ranks       4-16    17-32   33-64   65-128   (sums over the shapes: 210, 113, 88, 109)
+//   convolution 3619/3925  2282/2254  4060/2426  12273/3956
+//   step        10289/10705  7209/6075  14375/7043  33665/12089
+//   gradients   9198/7498  6696/4748  13028/5473  24193/9483
+//   layer       12490/12711  8184/7419  15888/7943  37391/13645
+//   layer (3)   17362/12654  11210/7385  21503/7925  48043/13615
 const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
   return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
@@ -120,26 +121,31 @@ enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3 };
 bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !g_planes || !planes_supported(*s)) return false;
   if (g_planes == 2) return true;
-  const double px = (double)s->N * s->H * s->W, ch = (double)s->C + s->T, weighted = ch * std::sqrt(std::sqrt(px));
-  const int ranks = s->Rank <= 16 ? 0 : s->Rank <= 32 ? 1 : s->Rank <= 64 ? 2 : 3;
+  const double ch = (double)s->C + s->T, root4 = std::sqrt(std::sqrt((double)s->N * s->H * s->W));
+  if (s->Rank <= 16) {
+    const double few = ch * std::sqrt((double)s->Rank) / root4;
+    switch (use) {
+      case Planes::kConv: return s->Rank > 8 && few >= 130;
+      case Planes::kStep: return few >= 110;
+      case Planes::kSaved: return few >= 100;
+      case Planes::kFilter: return few >= 42;
+      case Planes::kFilter3: return few >= 47;
+      default: return ch >= 64 && few >= 27;
+    }
+  }
+  const int ranks = s->Rank <= 32 ? 0 : s->Rank <= 64 ? 1 : 2;
+  const auto past = [&](const double (&least)[3], const double (&weighted)[3]) {
+    return ch >= least[ranks] || ch * root4 >= weighted[ranks];
+  };
   switch (use) {
-    case Planes::kConv: {
-      constexpr double line[4] = {12000, 2400, 800, 420};
-      return weighted >= line[ranks];
-    }
-    case Planes::kStep: {
-      constexpr double line[4] = {12000, 1300, 300, 0};
-      return weighted >= line[ranks];
-    }
-    case Planes::kSaved: {
-      constexpr double line[4] = {12000, 2200, 530, 0};
-      return weighted >= line[ranks];
-    }
+    case Planes::kConv: return past({256, 129, 0}, {2800, 1000, 0});
+    case Planes::kStep: return past({200, 0, 0}, {1300, 0, 0});
+    case Planes::kSaved:
+      if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // narrow: the stencil's 16-byte rows decide
+      return past({160, 0, 0}, {2200, 0, 0});
     case Planes::kFilter:
-    case Planes::kFilter3:
-      return ranks == 0 ? ch >= 4 * std::sqrt(px) : ranks == 1 ? ch > 128 : ranks == 2 ? weighted >= 540 : ch >= 44;
-    default:
-      return ranks == 0 ? ch >= 160 : ranks == 1 ? weighted >= 1400 : ranks == 2 ? weighted >= 490 : ch >= 18;
+    case Planes::kFilter3: return past({129, 48, 0}, {2200, 490, 0});
+    default: return past({129, 40, 0}, {2200, 400, 0});
   }
 }
 

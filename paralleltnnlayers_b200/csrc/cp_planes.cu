@@ -12,6 +12,7 @@
 // programmatic dependents of one another.  Everything is exact fp32 (FFMA).
 // Formulas: Cuda_kernels/cp4Conv2dForward.cu:42-134, cp4Conv2dBackwardData.cu:29-109, cp4Conv2dBackwardFilter.cu:64-257.
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "cluster_util.cuh"
@@ -29,6 +30,198 @@ namespace {
 constexpr int kThreads = 128;
 
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+__device__ __forceinline__ void fma4(float (&d)[4], float a, const float4& b) {
+  d[0] = fmaf(a, b.x, d[0]);
+  d[1] = fmaf(a, b.y, d[1]);
+  d[2] = fmaf(a, b.z, d[2]);
+  d[3] = fmaf(a, b.w, d[3]);
+}
+
+// ---- out[n][m][p] = sum_k F(m, k) in[n][k][p] --------------------------------------------------------------------------
+// AK false: F is [K][M] (channels to ranks); true: F is [M][K] (ranks to channels).  A warp forms 4*TM rows x 32 pixels,
+// TM x 4 per lane (4 row groups x 8 pixel quads): three shared-memory wavefronts per 32 FFMA at TM = 8.  128 threads per
+// CTA, four and more CTAs per SM.
+struct PlaneProduct {
+  const float* F;
+  const float* in;
+  float* out;
+  int M, K, mtiles, kper;
+  int vecF, vecIn, vecOut;
+};
+struct PlaneGemm {
+  PlaneProduct p[2];
+  int HW, Q, maxmt, splits;     // Q = N * HW
+};
+constexpr int kGK = 16, kGS = 3;
+
+template <int TM, int WM, int WN, bool AK>
+__global__ void __launch_bounds__(kThreads) plane_gemm_kernel(const __grid_constant__ PlaneGemm g) {
+  constexpr int BM = 4 * TM * WM, BN = 32 * WN, PA = AK ? kGK + 4 : BM;
+  constexpr int kAF = AK ? BM * PA : kGK * PA, kStage = kAF + kGK * BN;
+  static_assert(WM * WN == 4 && kGS * kStage >= BM * BN, "");
+  __shared__ __align__(16) float smem[kGS * kStage];
+  const PlaneProduct& a = g.p[blockIdx.z / g.splits];
+  const int mt = blockIdx.x % g.maxmt, q0 = (blockIdx.x / g.maxmt) * BN;
+  if (mt >= a.mtiles) {     // (the other product of the launch has more row tiles; a whole cluster leaves)
+    grid_dependency_wait();
+    return;
+  }
+  const int m0 = mt * BM, kb = (blockIdx.z % g.splits) * a.kper, ke = min(a.K, kb + a.kper);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp / WN, wn = warp % WN;
+  const int ty = lane >> 3, tx = lane & 7;
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
+  // this thread's pixel column of a stage
+  constexpr int G4 = BN / 4, R4 = kThreads / G4, R1 = kThreads / BN;
+  const int col = a.vecIn ? (tid % G4) * 4 : tid % BN, row0 = a.vecIn ? tid / G4 : tid / BN;
+  const bool colin = q0 + col < g.Q;
+  const int n = colin ? (q0 + col) / g.HW : 0, p = colin ? q0 + col - n * g.HW : 0;
+  const float* in = a.in + (size_t)n * a.K * g.HW + p;
+
+  // Every thread copies the same column of each stage, so its address runs and what is outside M or the pixels is a copy
+  // of no bytes (zero fill); only the last stage of a K that is no multiple of the stage looks at k.
+  const float* inp = in + (size_t)(kb + row0) * g.HW;
+  auto load_in = [&](int st, int k0) {
+    const unsigned d = sbase + (unsigned)(st * kStage + kAF + row0 * BN + col) * 4u;
+    const float* src = inp;
+    inp += (size_t)kGK * g.HW;
+    const bool full = k0 + kGK <= ke;
+    if (a.vecIn) {
+      const size_t inc = (size_t)R4 * g.HW;
+#pragma unroll
+      for (int i = 0; i < kGK / R4; ++i, src += inc) {
+        const bool v = colin && (full || k0 + row0 + i * R4 < ke);
+        mma::cp_async16_s(d + (unsigned)(i * R4 * BN) * 4u, v ? src : a.in, v ? 16 : 0);
+      }
+    } else if (full && q0 + BN <= g.Q) {
+      const size_t inc = (size_t)R1 * g.HW;
+#pragma unroll
+      for (int i = 0; i < kGK / R1; ++i, src += inc) mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, src, 4);
+    } else {
+      const size_t inc = (size_t)R1 * g.HW;
+#pragma unroll
+      for (int i = 0; i < kGK / R1; ++i, src += inc) {
+        const bool v = colin && k0 + row0 + i * R1 < ke;
+        mma::cp_async4_s(d + (unsigned)(i * R1 * BN) * 4u, v ? src : a.in, v ? 4 : 0);
+      }
+    }
+  };
+  auto load_f = [&](int st, int k0) {
+    const unsigned d0 = sbase + (unsigned)(st * kStage) * 4u;
+    // groups of 4 floats or single floats along the contiguous index; ROWS threads apart along the other
+    const auto copy = [&](auto width) {
+      constexpr int V = decltype(width)::value, COLS = (AK ? kGK : BM) / V, ROWS = AK ? BM : kGK, RT = kThreads / COLS;
+      const int c = (tid % COLS) * V, r0 = tid / COLS, ld = AK ? a.K : a.M;
+      const int kc = AK ? k0 + c : m0 + c, kr = AK ? m0 + r0 : k0 + r0;
+      const bool cin = kc < (AK ? ke : a.M);
+      const int rend = AK ? a.M : ke;
+      const float* src = a.F + (size_t)kr * ld + kc;
+      const size_t inc = (size_t)RT * ld;
+      unsigned d = d0 + (unsigned)(r0 * PA + c) * 4u;
+#pragma unroll
+      for (int i = 0; i < (ROWS + RT - 1) / RT; ++i, src += inc, d += (unsigned)(RT * PA) * 4u) {
+        if (ROWS % RT && r0 + i * RT >= ROWS) break;
+        const bool v = cin && kr + i * RT < rend;
+        if (V == 4) mma::cp_async16_s(d, v ? src : a.F, v ? 16 : 0);
+        else mma::cp_async4_s(d, v ? src : a.F, v ? 4 : 0);
+      }
+    };
+    if (a.vecF) copy(std::integral_constant<int, 4>{});
+    else copy(std::integral_constant<int, 1>{});
+  };
+
+  float acc[TM][4];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  const int steps = ke > kb ? (ke - kb + kGK - 1) / kGK : 0;
+  for (int s = 0; s < kGS - 1; ++s)
+    if (s < steps) load_f(s, kb + s * kGK);
+  grid_dependency_wait();
+  for (int s = 0; s < kGS - 1; ++s) {
+    if (s < steps) load_in(s, kb + s * kGK);
+    mma::cp_async_commit();
+  }
+  for (int s = 0; s < steps; ++s) {
+    mma::cp_async_wait<kGS - 2>();
+    __syncthreads();
+    const int nx = s + kGS - 1;
+    if (nx < steps) {
+      load_f(nx % kGS, kb + nx * kGK);
+      load_in(nx % kGS, kb + nx * kGK);
+    }
+    mma::cp_async_commit();
+    const float* As = smem + (s % kGS) * kStage;
+    const float* Bs = As + kAF + wn * 32 + tx * 4;
+#pragma unroll
+    for (int k = 0; k < kGK; k += 4) {
+      if (AK) {
+        float4 f[TM];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) f[i] = lds4(As + (wm * 4 * TM + ty + 4 * i) * PA + k);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 b = lds4(Bs + (k + u) * BN);
+#pragma unroll
+          for (int i = 0; i < TM; ++i) fma4(acc[i], u == 0 ? f[i].x : u == 1 ? f[i].y : u == 2 ? f[i].z : f[i].w, b);
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 b = lds4(Bs + (k + u) * BN);
+#pragma unroll
+          for (int i = 0; i < TM; i += 4) {
+            const float4 f = lds4(As + (k + u) * PA + wm * 4 * TM + ty * TM + i);
+            fma4(acc[i], f.x, b);
+            fma4(acc[i + 1], f.y, b);
+            fma4(acc[i + 2], f.z, b);
+            fma4(acc[i + 3], f.w, b);
+          }
+        }
+      }
+    }
+  }
+  mma::cp_async_wait<0>();
+  grid_launch_dependents();
+  if (g.splits > 1) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const int m = wm * 4 * TM + (AK ? ty + 4 * i : ty * TM + i);
+      *reinterpret_cast<float4*>(smem + m * BN + wn * 32 + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+    cluster_sum(smem, BM * BN, g.splits, tid, kThreads, [&](int i, float v) {
+      const int m = m0 + i / BN, q = q0 + i % BN;
+      if (m < a.M && q < g.Q) {
+        const int nn = q / g.HW;
+        a.out[((size_t)nn * a.M + m) * g.HW + (q - nn * g.HW)] = v;
+      }
+    });
+    return;
+  }
+  // this thread's four pixels
+  const int q = q0 + wn * 32 + tx * 4;
+  size_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int nn = (q + j) / g.HW;
+    o[j] = (size_t)nn * a.M * g.HW + (q + j - nn * g.HW);
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + wm * 4 * TM + (AK ? ty + 4 * i : ty * TM + i);
+    if (m >= a.M) continue;
+    float* d = a.out + (size_t)m * g.HW;
+    if (a.vecOut) {
+      if (q < g.Q) *reinterpret_cast<float4*>(d + o[0]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (q + j < g.Q) d[o[j]] = acc[i][j];
+    }
+  }
+}
 
 // ---- out[n][m][p] = sum_k F(m, k) in[n][k][p] on the tensor cores ---------------------------------------------------------
 // The products of a CP convolution with whole rank planes: P = K1^T X (F is [K][M]) and U = K0 Z (AK: F is [M][K]).  Scaled fp16
@@ -124,32 +317,50 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
   // ---- F by items of eight k (lanes along the contiguous index): largest magnitude per row, then the planes.  In between the
   // values wait as fp32 in the 16 bytes of hi and the 16 of lo that they become.
   const int k8s = nch * (kTcK / 8), along = max(AK ? k8s : nt, 1), dfast = kTcThreads % along, dslow = kTcThreads / along;
-  auto each_item = [&](auto&& fn) {
+  const int items = nt * k8s;
+  auto place = [&](int r, int k8) { return Bs + (k8 >> 3) * 2 * nt * 128 + r * 128 + (((k8 & 7) ^ (r & 7)) << 4); };
+  {
+    constexpr int kBatch = 4;   // items of a thread whose loads are in flight together (one after the other 0.65 us each)
     int fast = tid % along, slow = tid / along;
-    for (int i = tid; i < nt * k8s; i += kTcThreads) {
-      const int r = AK ? slow : fast, k8 = AK ? fast : slow;
-      fn(r, k8, Bs + (k8 >> 3) * 2 * nt * 128 + r * 128 + (((k8 & 7) ^ (r & 7)) << 4));
-      fast += dfast;
-      slow += dslow;
-      if (fast >= along) { fast -= along; ++slow; }
+    for (int i = tid; i < items; i += kBatch * kTcThreads) {
+      float f[kBatch][8];
+      int r[kBatch], k8[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        r[b] = AK ? slow : fast;
+        k8[b] = AK ? fast : slow;
+        const int m = m0 + r[b], k = kb + k8[b] * 8;
+        const bool in = i + b * kTcThreads < items && m < a.M;
+        const size_t inc = AK ? 1 : a.M;
+        const float* src = AK ? a.F + (size_t)m * a.K + k : a.F + (size_t)k * a.M + m;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[b][j] = in && k + j < ke ? __ldg(src + j * inc) : 0.f;
+        fast += dfast;
+        slow += dslow;
+        if (fast >= along) { fast -= along; ++slow; }
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        if (i + b * kTcThreads >= items) break;
+        unsigned mx = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mx = max(mx, tc::abs_bits(f[b][j]));
+        uint8_t* d = place(r[b], k8[b]);
+        *reinterpret_cast<float4*>(d) = make_float4(f[b][0], f[b][1], f[b][2], f[b][3]);
+        *reinterpret_cast<float4*>(d + nt * 128) = make_float4(f[b][4], f[b][5], f[b][6], f[b][7]);
+        atomicMax(&rowmax[r[b]], mx);
+      }
     }
-  };
-  each_item([&](int r, int k8, uint8_t* d) {
-    const int m = m0 + r, k = kb + k8 * 8;
-    const size_t inc = AK ? 1 : a.M;
-    const float* src = AK ? a.F + (size_t)m * a.K + k : a.F + (size_t)k * a.M + m;
-    float f[8];
-    unsigned mx = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = m < a.M && k + j < ke ? __ldg(src + j * inc) : 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) mx = max(mx, tc::abs_bits(f[j]));
-    *reinterpret_cast<float4*>(d) = make_float4(f[0], f[1], f[2], f[3]);
-    *reinterpret_cast<float4*>(d + nt * 128) = make_float4(f[4], f[5], f[6], f[7]);
-    atomicMax(&rowmax[r], mx);
-  });
+  }
   __syncthreads();
-  each_item([&](int r, int, uint8_t* d) { split_in_place(d, d + nt * 128, tc::exp2_int(-tc::row_exponent(rowmax[r], tc::kLeast))); });
+  for (int i = tid, fast = tid % along, slow = tid / along; i < items; i += kTcThreads) {
+    const int r = AK ? slow : fast;
+    uint8_t* d = place(r, AK ? fast : slow);
+    split_in_place(d, d + nt * 128, tc::exp2_int(-tc::row_exponent(rowmax[r], tc::kLeast)));
+    fast += dfast;
+    slow += dslow;
+    if (fast >= along) { fast -= along; ++slow; }
+  }
   if (tid < nt) {   // 2^(24 + e) of a row in two factors
     const int e = tc::kRowShift + tc::row_exponent(rowmax[tid], tc::kLeast);
     rowscale[tid] = make_float2(tc::exp2_int(e >> 1), tc::exp2_int(e - (e >> 1)));
@@ -256,14 +467,40 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
   }
   if (!fine) atomicCAS(&g_planes_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
   if (warp == 0) tc::tmem_dealloc(tmem, g.cols);
-  if (g.splits > 1)
-    cluster_sum(sums, nt * kTcPx, g.splits, tid, kTcThreads, [&](int i, float x) {
-      const int m = m0 + i / kTcPx, q = blockIdx.x * kTcPx + i % kTcPx;
-      if (m < a.M && q < g.Q) {
-        const int nn = q / g.HW;
-        a.out[((size_t)nn * a.M + m) * g.HW + (q - nn * g.HW)] = x;
+  if (g.splits == 1) return;
+  // The sum over the cluster, a slice of the tile per CTA, in CTA order; four pixels per load and four loads of a thread in
+  // flight (one value at a time the 128 x 128 tile took 10 us and more).
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const int quads = nt * (kTcPx / 4), share = (quads + g.splits - 1) / g.splits, e0 = (int)cl.block_rank() * share;
+  const int e1 = min(quads, e0 + share);
+  for (int i0 = e0 + tid; i0 < e1; i0 += 4 * kTcThreads) {
+    float4 x[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) x[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < g.splits; ++k) {
+      const float* from = cl.map_shared_rank(sums, k);
+      float4 y[4];
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        y[b] = i0 + b * kTcThreads < e1 ? lds4(from + (size_t)(i0 + b * kTcThreads) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) { x[b].x += y[b].x; x[b].y += y[b].y; x[b].z += y[b].z; x[b].w += y[b].w; }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int i = i0 + b * kTcThreads, m = m0 + i / (kTcPx / 4);
+      if (i >= e1 || m >= a.M) break;
+      const float w[4] = {x[b].x, x[b].y, x[b].z, x[b].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int q = blockIdx.x * kTcPx + i % (kTcPx / 4) * 4 + j, nn = q / g.HW;
+        if (q < g.Q) a.out[((size_t)nn * a.M + m) * g.HW + (q - nn * g.HW)] = w[j];
       }
-    });
+    }
+  }
+  cl.sync();   // nobody reads this CTA's sums any more
 }
 
 // ---- the stencils --------------------------------------------------------------------------------------------------------
@@ -361,13 +598,14 @@ __global__ void __launch_bounds__(kThreads) plane_stencil_kernel(const __grid_co
 // they are added to totals in registers, each with the powers of two of its row and its rank in that chunk.
 //
 // What bounds it is the splitting (about 25 instructions per row and chunk) and latency: 64 x 256 14x14 at R = 32 19 us on FFMA,
-// 1x here; 16 x 256 -> 384 27x27 at R = 50 (4-byte loads) 35 and 1x.
+// 20 here; 16 x 256 -> 384 27x27 at R = 50 (4-byte loads) 36 and 28.
 struct PlaneGrad {
   const float* D[2];     // dU, X
   const float* Z[2];     // Z, Zt
   float* part;
   int rows[2], mtiles[2], row0[2];
-  int R, rtiles, HW, Q, per;   // per: pixels of a split, a multiple of 64
+  int vecD[2], vecZ;           // (FFMA kernel)
+  int R, rtiles, HW, Q, per;   // per: pixels of a split, a multiple of 64 (FFMA: 32)
   size_t nrows;          // T + C
 };
 constexpr int kGradThreads = 256, kGradRows = 128;
@@ -382,7 +620,7 @@ struct GradTile {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(kGradThreads, 2) plane_grad_kernel(const __grid_constant__ PlaneGrad g) {
+__global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __grid_constant__ PlaneGrad g) {
   using T = GradTile<NT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -538,6 +776,118 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_kernel(const __gri
   }
 }
 
+// ---- the same on FFMA ------------------------------------------------------------------------------------------------------
+// Both operands have the pixels contiguous, so a lane reads four pixels of a row at once: 8 + TN reads of 16 bytes (one
+// wavefront each: the pitch of 36 floats puts eight consecutive rows on all banks) per 32*TN FFMA.  The running sum of a
+// group of eight stages (256 pixels) is added to the total separately: a plain chain over thousands of pixels would round
+// more than split tensor-core sums.
+constexpr int kDK = 32, kDP = kDK + 4, kDS = 3;
+
+template <int TN, int WM, int WN>
+__global__ void __launch_bounds__(kThreads) plane_grad_kernel(const __grid_constant__ PlaneGrad g) {
+  constexpr int BM = 32 * WM, BN = 8 * TN * WN, kStage = (BM + BN) * kDP;
+  static_assert(WM * WN == 4, "");
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp / WN, wn = warp % WN;
+  const int ty = lane >> 3, tx = lane & 7;
+  const int rt = blockIdx.x % g.rtiles, mi = blockIdx.x / g.rtiles, half = mi >= g.mtiles[0] ? 1 : 0;
+  const int m0 = (mi - (half ? g.mtiles[0] : 0)) * BM, r0 = rt * BN, rows = half ? g.rows[1] : g.rows[0];
+  const int qb = blockIdx.y * g.per, qe = min(g.Q, qb + g.per);
+  const float* D = half ? g.D[1] : g.D[0];
+  const float* Z = half ? g.Z[1] : g.Z[0];
+  const bool vecD = half ? g.vecD[1] : g.vecD[0], vecZ = g.vecZ;
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
+  // rows base .. base + NB - 1 of src [n][total][HW], 32 pixels from q0 on; a full tile needs no predicates, which with
+  // the 4-byte copies (H * W not a multiple of 4) are most of the instructions around the FFMA (16 x 256 -> 384 27x27 R = 50: 58 -> 35 us)
+  auto load = [&](auto nb, unsigned dst, const float* src, int base, int total, int q0, bool vec) {
+    constexpr int NB = decltype(nb)::value;
+    const int step = vec ? kThreads / 8 : kThreads / 32, i0 = vec ? tid >> 3 : tid >> 5;
+    const int col = vec ? (tid & 7) * 4 : tid & 31, q = q0 + col, n = q / g.HW;
+    const float* s = src + ((size_t)n * total + base + i0) * g.HW + (q - n * g.HW);
+    const size_t inc = (size_t)step * g.HW;
+    unsigned d = dst + (unsigned)(i0 * kDP + col) * 4u;
+    const bool qin = q < qe;
+    if (vec) {
+#pragma unroll
+      for (int i = 0; i < NB / (kThreads / 8); ++i, s += inc, d += (kThreads / 8) * kDP * 4u) {
+        const bool v = qin && base + i0 + i * (kThreads / 8) < total;
+        mma::cp_async16_s(d, v ? s : src, v ? 16 : 0);
+      }
+    } else if (base + NB <= total && q0 + kDK <= qe) {
+#pragma unroll
+      for (int i = 0; i < NB / (kThreads / 32); ++i, s += inc, d += (kThreads / 32) * kDP * 4u) mma::cp_async4_s(d, s, 4);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NB / (kThreads / 32); ++i, s += inc, d += (kThreads / 32) * kDP * 4u) {
+        const bool v = qin && base + i0 + i * (kThreads / 32) < total;
+        mma::cp_async4_s(d, v ? s : src, v ? 4 : 0);
+      }
+    }
+  };
+  auto load_stage = [&](int st, int q) {
+    const unsigned d = sbase + (unsigned)(st * kStage) * 4u;
+    load(std::integral_constant<int, BM>{}, d, D, m0, rows, q, vecD);
+    load(std::integral_constant<int, BN>{}, d + BM * kDP * 4u, Z, r0, g.R, q, vecZ);
+  };
+  float acc[8][TN], total[8][TN];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = total[i][j] = 0.f;
+  auto flush = [&] {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        total[i][j] += acc[i][j];
+        acc[i][j] = 0.f;
+      }
+  };
+  const int steps = qe > qb ? (qe - qb + kDK - 1) / kDK : 0;
+  grid_dependency_wait();
+  for (int s = 0; s < kDS - 1; ++s) {
+    if (s < steps) load_stage(s, qb + s * kDK);
+    mma::cp_async_commit();
+  }
+  for (int s = 0; s < steps; ++s) {
+    mma::cp_async_wait<kDS - 2>();
+    __syncthreads();
+    const int nx = s + kDS - 1;
+    if (nx < steps) load_stage(nx % kDS, qb + nx * kDK);
+    mma::cp_async_commit();
+    const float* As = smem + (s % kDS) * kStage + (wm * 32 + ty) * kDP;
+    const float* Bs = smem + (s % kDS) * kStage + (BM + wn * 8 * TN + tx) * kDP;
+#pragma unroll
+    for (int k = 0; k < kDK; k += 4) {
+      float4 b[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) b[j] = lds4(Bs + j * 8 * kDP + k);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 a = lds4(As + i * 4 * kDP + k);
+#pragma unroll
+        for (int j = 0; j < TN; ++j)
+          acc[i][j] = fmaf(a.w, b[j].w, fmaf(a.z, b[j].z, fmaf(a.y, b[j].y, fmaf(a.x, b[j].x, acc[i][j]))));
+      }
+    }
+    if ((s & 7) == 7) flush();
+  }
+  flush();
+  mma::cp_async_wait<0>();
+  grid_launch_dependents();
+  float* out = g.part + ((size_t)blockIdx.y * g.nrows + (half ? g.row0[1] : 0)) * g.R;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + wm * 32 + ty + 4 * i;
+    if (m >= rows) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int r = r0 + wn * 8 * TN + tx + 8 * j;
+      if (r < g.R) out[(size_t)m * g.R + r] = total[i][j];
+    }
+  }
+}
+
 // ---- the sums of the partials, in a fixed order ----------------------------------------------------------------------------
 // 32 entries x 8 groups of partials per CTA; the last CTAs turn the correlation sums into the spatial factors' gradients.
 struct PlaneReduce {
@@ -596,6 +946,45 @@ __global__ void __launch_bounds__(256) plane_reduce_kernel(const PlaneReduce g) 
 // ---- launches --------------------------------------------------------------------------------------------------------------
 bool aligned16(const void* p) { return !(reinterpret_cast<uintptr_t>(p) & 15); }
 
+// FFMA products
+int gemm_launch(PlaneGemm g, int nprod, bool ak, bool programmatic, const DeviceInfo& di, cudaStream_t st) {
+  int M = 0, K = 0;
+  for (int i = 0; i < nprod; ++i) {
+    M = std::max(M, g.p[i].M);
+    K = std::max(K, g.p[i].K);
+  }
+  // the smallest row tile that holds all rows, at most 64; row and pixel tiles trade off at 128 threads
+  const int bm = M <= 16 ? 16 : M <= 32 ? 32 : 64, bn = bm == 64 ? 64 : 128;
+  long tiles = 0;
+  g.maxmt = 0;
+  for (int i = 0; i < nprod; ++i) {
+    PlaneProduct& p = g.p[i];
+    p.mtiles = ceil_div(p.M, bm);
+    g.maxmt = std::max(g.maxmt, p.mtiles);
+    tiles += (long)p.mtiles * ceil_div(g.Q, bn);
+    p.vecF = !((ak ? p.K : p.M) & 3) && aligned16(p.F);
+    p.vecIn = !(g.HW & 3) && aligned16(p.in);
+    p.vecOut = !(g.HW & 3) && aligned16(p.out);
+  }
+  // two CTAs of 128 threads and more per SM are needed to hide the FFMA and shared-memory latency
+  g.splits = pick_cluster(tiles, K, 2 * kGK, 3 * di.sm_count);
+  for (int i = 0; i < nprod; ++i) g.p[i].kper = (int)align_up((size_t)ceil_div(g.p[i].K, g.splits), kGK);
+  const dim3 grid((unsigned)((long)g.maxmt * ceil_div(g.Q, bn)), 1, nprod * g.splits);
+#define PLANE_GEMM(TM, WM, WN)                                                                                          \
+  do {                                                                                                                 \
+    if (ak) B200CP_CUDA_OK(launch_cluster(plane_gemm_kernel<TM, WM, WN, true>, grid, dim3(kThreads), 0, st, g.splits,   \
+                                          programmatic, g));                                                           \
+    else B200CP_CUDA_OK(launch_cluster(plane_gemm_kernel<TM, WM, WN, false>, grid, dim3(kThreads), 0, st, g.splits,     \
+                                       programmatic, g));                                                              \
+  } while (0)
+  if (bm == 16) PLANE_GEMM(4, 1, 4);
+  else if (bm == 32) PLANE_GEMM(8, 1, 4);
+  else PLANE_GEMM(8, 2, 2);
+#undef PLANE_GEMM
+  B200CP_LAUNCH_OK("plane_gemm_kernel");
+  return B200CP_OK;
+}
+
 // Rows of a tile, the cluster split and the launch.
 int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo& di, cudaStream_t st) {
   int M = 0, K = 0;
@@ -615,10 +1004,17 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
   fit();
   long tiles = 0;
   for (int i = 0; i < nprod; ++i) tiles += (long)ceil_div(g.p[i].M, g.nt) * pxt;
-  g.splits = pick_cluster(tiles, kchunks, 1, di.sm_count);
-  while (ceil_div(kchunks, g.splits) > kTcMaxChunks && g.splits < 8) g.splits *= 2;
+  // a cluster where that leaves no SM idle that has two chunks to do (one per group)
+  while (g.splits < 8 && ceil_div(kchunks, g.splits) > (tiles * g.splits * 2 <= di.sm_count ? 2 : kTcMaxChunks)) g.splits *= 2;
   g.nt = (int)align_up(std::min(M, 256), 32);
   fit();
+  // few pixels: narrower tiles, whose part of F is split and whose sums are stored sooner
+  const auto ctas = [&] {
+    long n = 0;
+    for (int i = 0; i < nprod; ++i) n += (long)ceil_div(g.p[i].M, g.nt) * pxt * g.splits;
+    return n;
+  };
+  while (g.nt > 32 && ctas() * 2 <= di.sm_count) g.nt = (int)align_up(g.nt / 2, 32);
   if (g.chunks > kTcMaxChunks) return fail(B200CP_ERR_UNSUPPORTED, "cp planes: %d channels", K);
   g.maxmt = 0;
   for (int i = 0; i < nprod; ++i) {
@@ -647,21 +1043,47 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
   return B200CP_OK;
 }
 
+// Which kernels form the products and the gradients: lines in multiply-adds (pixels x ranks x channels) per rank class, over 520
+// random shapes measured both ways.  Tensor cores / FFMA, geometric mean over the shapes between 2^26 and 2^27, 2^27 and 2^28,
+// 2^28 and 2^29 multiply-adds:
+//              ranks 4-16         17-32              33-64              65-128
+//   convolution 1.23 1.09 1.03    0.97 0.99 0.82     1.06 0.79 0.80     0.92 0.93 0.78  (smaller shapes 0.85 to 0.97)
+//   gradients   1.47 1.48 1.44    1.12 1.05 1.08     1.05 0.93 0.93     1.02 0.94 0.87  (with the two products before them)
+struct PlanesOn {
+  bool products, gradients;   // on the tensor cores
+};
+PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
+  static const int mode = [] {   // B200CP_PLANES_TC: 0 FFMA, 2 tensor cores, else by the rule
+    const char* e = getenv("B200CP_PLANES_TC");
+    return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
+  }();
+  if (mode != 1) return {mode == 2, mode == 2};
+  const double macs = (double)s.N * s.H * s.W * s.Rank * ((double)s.C + s.T);
+  if (s.Rank <= 16) return {false, false};
+  if (s.Rank <= 32) return {macs >= 1e8, macs >= 1e9};
+  if (s.Rank > 64 && s.C + s.T <= 32) return {false, false};   // half of a K stage is padding: a step 1.01 to 1.28 times as long
+  return {s.Rank > 64 || macs >= 1.3e8, macs >= 1.3e8};
+}
+
 struct GradPlan {
-  int bn, mt0, mt1, rtiles, splits, per;       // gradient products
+  bool tc;
+  int bm, bn, mt0, mt1, rtiles, splits, per;   // gradient products
   int units, chunks, cper;                     // stencil ranges
 };
 GradPlan grad_plan(const b200cp_tensor_shape& s, int sm_count) {
   GradPlan p{};
   const int R = (int)s.Rank, Q = (int)(s.N * s.H * s.W);
-  p.bn = R <= 32 ? 32 : 64;
-  p.mt0 = ceil_div((int)s.T, kGradRows);
-  p.mt1 = ceil_div((int)s.C, kGradRows);
+  p.tc = planes_on_tensor_cores(s).gradients;
+  p.bn = !p.tc && R <= 16 ? 16 : R <= 32 ? 32 : 64;
+  p.bm = p.tc || p.bn < 64 ? 128 : 64;
+  p.mt0 = ceil_div((int)s.T, p.bm);
+  p.mt1 = ceil_div((int)s.C, p.bm);
   p.rtiles = ceil_div(R, p.bn);
   const int tiles = (p.mt0 + p.mt1) * p.rtiles;
-  // two CTAs per SM, at least two chunks each
-  const int want = std::max(1, std::min({2 * sm_count / tiles, ceil_div(Q, 2 * kTcK), 65535}));
-  p.per = (int)align_up((size_t)ceil_div(Q, want), kTcK);
+  // two CTAs per SM, at least a chunk each; on FFMA three (shared memory) of at least two stages
+  const int want = p.tc ? std::max(1, std::min({2 * sm_count / tiles, ceil_div(Q, kTcK), 65535}))
+                        : std::max(1, std::min({3 * sm_count / tiles, ceil_div(Q, 2 * kDK), 65535}));
+  p.per = (int)align_up((size_t)ceil_div(Q, want), p.tc ? kTcK : kDK);
   p.splits = ceil_div(Q, p.per);
   p.units = (int)s.N * ceil_div((int)s.H, 4) * (int)s.W;
   const int cw = std::max(1, std::min({ceil_div(8 * sm_count, R), ceil_div(p.units, kThreads), 65535}));
@@ -735,6 +1157,20 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   g.HW = HW;
   g.Q = NQ;
   int np = 0;
+  const bool tc = planes_on_tensor_cores(s).products;
+  auto products = [&](bool ak, bool programmatic) {
+    if (tc) {
+      g.first = !programmatic;
+      return tc_launch(g, np, ak, programmatic, di, st);
+    }
+    PlaneGemm f{};
+    f.HW = HW;
+    f.Q = NQ;
+    for (int i = 0; i < np; ++i) {
+      f.p[i].F = g.p[i].F; f.p[i].in = g.p[i].in; f.p[i].out = g.p[i].out; f.p[i].M = g.p[i].M; f.p[i].K = g.p[i].K;
+    }
+    return gemm_launch(f, np, ak, programmatic, di, st);
+  };
   auto product = [&](const float* F, const float* in, float* out, int M, int K) {
     PlaneTcProduct& p = g.p[np++];
     p.F = F; p.in = in; p.out = out; p.M = M; p.K = K;
@@ -742,8 +1178,7 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   if (needP && !j.P) product(j.K1, j.X, j.Psave ? j.Psave : b.P, R, C);
   if (needQ && !j.Q) product(j.K0, j.dU, j.Qsave ? j.Qsave : b.Q, R, T);
   if (np) {
-    g.first = 1;
-    if (int rc = tc_launch(g, np, false, false, di, st)) return rc;
+    if (int rc = products(false, false)) return rc;
     chained = true;
   }
   const GradPlan gp = grad_plan(s, di.sm_count);
@@ -761,28 +1196,34 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   }
   B200CP_LAUNCH_OK("plane_stencil_kernel");
   np = 0;
-  g.first = 0;
   if (fwd) product(j.K0, b.Z, j.U, T, R);
   if (bwd) product(j.K1, b.Zt, j.dX, C, R);
   if (np)
-    if (int rc = tc_launch(g, np, true, true, di, st)) return rc;
+    if (int rc = products(true, true)) return rc;
   if (!grads) return B200CP_OK;
   PlaneGrad d{};
   d.D[0] = j.dU; d.D[1] = j.X; d.Z[0] = b.Z; d.Z[1] = b.Zt;
   d.part = b.part;
   d.rows[0] = T; d.rows[1] = C; d.row0[1] = T;
   d.mtiles[0] = gp.mt0; d.mtiles[1] = gp.mt1;
+  d.vecZ = !(HW & 3);
+  for (int i = 0; i < 2; ++i) d.vecD[i] = !(HW & 3) && aligned16(d.D[i]);
   d.R = R; d.rtiles = gp.rtiles; d.HW = HW; d.Q = NQ; d.per = gp.per;
   d.nrows = (size_t)T + C;
   const dim3 grid((gp.mt0 + gp.mt1) * gp.rtiles, gp.splits);
-#define PLANE_GRAD(NT)                                                                                                  \
+#define PLANE_GRAD(KERNEL, THREADS, SMEM)                                                                               \
   do {                                                                                                                 \
     static std::atomic<int> set[64];                                                                                   \
-    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(plane_grad_kernel<NT>), set, (int)GradTile<NT>::smem)); \
-    B200CP_CUDA_OK(launch_kernel(plane_grad_kernel<NT>, grid, dim3(kGradThreads), GradTile<NT>::smem, st, true, d));   \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(KERNEL), set, (int)(SMEM)));                      \
+    B200CP_CUDA_OK(launch_kernel(KERNEL, grid, dim3(THREADS), SMEM, st, true, d));                                     \
   } while (0)
-  if (gp.bn == 32) PLANE_GRAD(32);
-  else PLANE_GRAD(64);
+  const size_t smem = sizeof(float) * kDS * (gp.bm + gp.bn) * kDP;   // FFMA
+  if (gp.tc) {
+    if (gp.bn == 32) PLANE_GRAD(plane_grad_tc_kernel<32>, kGradThreads, GradTile<32>::smem);
+    else PLANE_GRAD(plane_grad_tc_kernel<64>, kGradThreads, GradTile<64>::smem);
+  } else if (gp.bn == 16) PLANE_GRAD((plane_grad_kernel<2, 4, 1>), kThreads, smem);
+  else if (gp.bn == 32) PLANE_GRAD((plane_grad_kernel<4, 4, 1>), kThreads, smem);
+  else PLANE_GRAD((plane_grad_kernel<4, 2, 2>), kThreads, smem);
 #undef PLANE_GRAD
   B200CP_LAUNCH_OK("plane_grad_kernel");
   PlaneReduce r{};
