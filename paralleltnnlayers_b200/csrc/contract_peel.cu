@@ -52,8 +52,8 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
   extern __shared__ __align__(16) float smem_f[];
   // Rows of G four banks apart: the lanes that store a t slab hold eight c (nt floats apart) of four rows, which without
   // the padding share four banks (8-way conflicts, a quarter of the kernel's shared-memory wavefronts at 8 x 8 entries).  With
-  // the batched loads below: 148 -> 122 us for G of 4096 x 4096 at R = 32; what bounds it now is the shared-memory pipe
-  // (three wavefronts per eight FFMA).
+  // the batched loads below: 148 -> 122 us for G of 4096 x 4096 at R = 32, and 104 with two ranks per lane; what bounds it is the
+  // shared-memory pipe.
   const int nbp = 8 * NPW, GP = nbp + kGPad;
   float* Gs = smem_f;                       // [kRows0][GP]
   float* Vs = Gs + kRows0 * GP;             // [nbp][kRB]
@@ -76,9 +76,10 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
     const int row = i / g.b.nc;
     slab[i] = (row << 16) | (i - row * g.b.nc);
   }
-  float acc2[NPW];
+  const int half = lane >> 4, pair = (lane & 15) * 2, r2 = blockIdx.y * kRB + pair;   // the products: see below
+  float acc2[NPW][2];
 #pragma unroll
-  for (int i = 0; i < NPW; ++i) acc2[i] = 0.f;
+  for (int i = 0; i < NPW; ++i) acc2[i][0] = acc2[i][1] = 0.f;
 
   // entries past nb stay zero for the whole kernel
   if (g.nb < nbp)
@@ -156,51 +157,59 @@ __global__ void __launch_bounds__(kPT) peel_first_kernel(const PeelGeom g) {
       }
     }
     __syncthreads();
-    // next[row][r] = sum_p G[row][p] * vec_b[p][r]: each warp takes kRows0 / 8 rows
+    // Two ranks per lane and half a warp per row: a 16-byte read of G then feeds eight FFMA and not four, and four reads of V and
+    // four of G, a shared-memory wavefront each, 32 FFMA (one rank per lane: twelve).
+    // next[row][r] = sum_p G[row][p] * vec_b[p][r]: each half warp takes kRows0 / 16 rows
     if (g.next != nullptr) {
-      float acc1[kRows0 / 8];
+      constexpr int NR = kRows0 / 16;
+      const int first = (wg * 2 + half) * NR;
+      float acc1[NR][2];
 #pragma unroll
-      for (int i = 0; i < kRows0 / 8; ++i) acc1[i] = 0.f;
+      for (int i = 0; i < NR; ++i) acc1[i][0] = acc1[i][1] = 0.f;
+#pragma unroll 2
       for (int p4 = 0; p4 < nbp; p4 += 4) {
-        const float v0 = Vs[(p4 + 0) * kRB + lane], v1 = Vs[(p4 + 1) * kRB + lane];
-        const float v2 = Vs[(p4 + 2) * kRB + lane], v3 = Vs[(p4 + 3) * kRB + lane];
+        float2 v[4];
 #pragma unroll
-        for (int i = 0; i < kRows0 / 8; ++i) {
-          const float4 gq = *reinterpret_cast<const float4*>(Gs + (wg * (kRows0 / 8) + i) * GP + p4);
-          acc1[i] = fmaf(gq.x, v0, acc1[i]);
-          acc1[i] = fmaf(gq.y, v1, acc1[i]);
-          acc1[i] = fmaf(gq.z, v2, acc1[i]);
-          acc1[i] = fmaf(gq.w, v3, acc1[i]);
+        for (int k = 0; k < 4; ++k) v[k] = *reinterpret_cast<const float2*>(Vs + (p4 + k) * kRB + pair);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          const float4 gq = *reinterpret_cast<const float4*>(Gs + (first + i) * GP + p4);
+          acc1[i][0] = fmaf(gq.x, v[0].x, acc1[i][0]); acc1[i][1] = fmaf(gq.x, v[0].y, acc1[i][1]);
+          acc1[i][0] = fmaf(gq.y, v[1].x, acc1[i][0]); acc1[i][1] = fmaf(gq.y, v[1].y, acc1[i][1]);
+          acc1[i][0] = fmaf(gq.z, v[2].x, acc1[i][0]); acc1[i][1] = fmaf(gq.z, v[2].y, acc1[i][1]);
+          acc1[i][0] = fmaf(gq.w, v[3].x, acc1[i][0]); acc1[i][1] = fmaf(gq.w, v[3].y, acc1[i][1]);
         }
       }
-      if (rok) {
 #pragma unroll
-        for (int i = 0; i < kRows0 / 8; ++i) {
-          const int row = wg * (kRows0 / 8) + i;
-          if (goff[row] >= 0) g.next[(size_t)orow[row] * g.R + r] = acc1[i];
+      for (int i = 0; i < NR; ++i)
+        if (goff[first + i] >= 0) {
+          float* d = g.next + (size_t)orow[first + i] * g.R + r2;
+          if (r2 < g.R) d[0] = acc1[i][0];
+          if (r2 + 1 < g.R) d[1] = acc1[i][1];
         }
-      }
     }
-    // d vec_b[p][r] += sum_rows G[row][p] * L[row][r]: each warp takes NPW entries
-#pragma unroll 4
-    for (int row = 0; row < kRows0; ++row) {
-      const float l = Ls[row * kRB + lane];
+    // d vec_b[p][r] += sum_rows G[row][p] * L[row][r]: each warp takes NPW entries, its halves every other row
+#pragma unroll 2
+    for (int row = half; row < kRows0; row += 2) {
+      const float2 l = *reinterpret_cast<const float2*>(Ls + row * kRB + pair);
 #pragma unroll
       for (int i4 = 0; i4 < NPW / 4; ++i4) {
         const float4 gq = *reinterpret_cast<const float4*>(Gs + row * GP + wg * NPW + i4 * 4);
-        acc2[i4 * 4 + 0] = fmaf(gq.x, l, acc2[i4 * 4 + 0]);
-        acc2[i4 * 4 + 1] = fmaf(gq.y, l, acc2[i4 * 4 + 1]);
-        acc2[i4 * 4 + 2] = fmaf(gq.z, l, acc2[i4 * 4 + 2]);
-        acc2[i4 * 4 + 3] = fmaf(gq.w, l, acc2[i4 * 4 + 3]);
+        acc2[i4 * 4 + 0][0] = fmaf(gq.x, l.x, acc2[i4 * 4 + 0][0]); acc2[i4 * 4 + 0][1] = fmaf(gq.x, l.y, acc2[i4 * 4 + 0][1]);
+        acc2[i4 * 4 + 1][0] = fmaf(gq.y, l.x, acc2[i4 * 4 + 1][0]); acc2[i4 * 4 + 1][1] = fmaf(gq.y, l.y, acc2[i4 * 4 + 1][1]);
+        acc2[i4 * 4 + 2][0] = fmaf(gq.z, l.x, acc2[i4 * 4 + 2][0]); acc2[i4 * 4 + 2][1] = fmaf(gq.z, l.y, acc2[i4 * 4 + 2][1]);
+        acc2[i4 * 4 + 3][0] = fmaf(gq.w, l.x, acc2[i4 * 4 + 3][0]); acc2[i4 * 4 + 3][1] = fmaf(gq.w, l.y, acc2[i4 * 4 + 3][1]);
       }
     }
   }
-  if (rok) {
-    float* out = g.part + (size_t)blockIdx.x * g.nb * g.R;
+  float* out = g.part + (size_t)blockIdx.x * g.nb * g.R;
 #pragma unroll
-    for (int i = 0; i < NPW; ++i) {
-      const int p = wg * NPW + i;
-      if (p < g.nb) out[(size_t)p * g.R + r] = acc2[i];
+  for (int i = 0; i < NPW; ++i) {
+    const int p = wg * NPW + i;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float v = acc2[i][k] + __shfl_xor_sync(0xffffffffu, acc2[i][k], 16);
+      if (half == 0 && p < g.nb && r2 + k < g.R) out[(size_t)p * g.R + r2 + k] = v;
     }
   }
 }
@@ -378,7 +387,8 @@ int contract_factors_launch(int order, const int* cdims, const int* tdims, int R
         return fail(B200CP_ERR_UNSUPPORTED, "factor contraction: the dense gradient has too many entries");
 #define LAUNCH_FIRST(N)                                                                                       \
   do {                                                                                                        \
-    B200CP_CUDA_OK(cudaFuncSetAttribute(peel_first_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    static std::atomic<int> set[64];                                                                          \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(peel_first_kernel<N>), set, (int)smem)); \
     peel_first_kernel<N><<<grid, kPT, smem, st>>>(g);                                                         \
   } while (0)
       if (npw == 4) LAUNCH_FIRST(4);
