@@ -20,6 +20,7 @@
 // filter is a free [3,3,R] core instead of the outer product KH x KW, and its gradient has nine rows,
 // dKC[y, x, r] = sum_px Q[r, px] * P[r, px + (y-1, x-1)].
 #include <algorithm>
+#include <cstring>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -839,15 +840,46 @@ __global__ void __launch_bounds__(kNT, 2) cp4_bwdf_saved_kernel(const SGeom g_in
   }
 }
 
-template <int RP>
-bool plan_saved(const Cp4BwdFilterArgs& a, const DeviceInfo& di, SGeom* out, size_t* smem_out) {
-  SGeom best{};
-  double best_cost = 1e300;
-  size_t best_smem = 0;
+// A tile search runs once per shape and forced tile: the plans of the last few shapes are kept per host thread.  (Searched anew
+// for each workspace query and each launch of a call it was most of the host's time: a step of 9 x 16 x 54 x 54 at R = 6 took 69 to
+// 96 us for 30 us on the device.)
+template <int RP, typename Geom>
+bool cached_plan(const Cp4BwdFilterArgs& a, const DeviceInfo& di, Geom* out, size_t* smem_out,
+                 bool (*search)(const Cp4BwdFilterArgs&, const DeviceInfo&, int, int, Geom*, size_t*)) {
   int fTH = 0, fTW = 0;
   if (const char* e = getenv("B200CP_MMA_TILE")) {  // "TH,TW": experiments
     if (sscanf(e, "%d,%d", &fTH, &fTW) != 2) fTH = fTW = 0;
   }
+  struct Entry {
+    int key[9];
+    bool ok;
+    Geom g;
+    size_t smem;
+  };
+  thread_local Entry cache[8];
+  thread_local int used = 0, next = 0;
+  const int key[9] = {a.N, a.C, a.T, a.H, a.W, fTH, fTW, di.sm_count, di.smem_optin};
+  Entry* e = nullptr;
+  for (int i = 0; i < used && !e; ++i)
+    if (std::memcmp(cache[i].key, key, sizeof(key)) == 0) e = &cache[i];
+  if (!e) {
+    e = &cache[next];
+    next = (next + 1) % 8;
+    used = std::min(used + 1, 8);
+    std::memcpy(e->key, key, sizeof(key));
+    e->ok = search(a, di, fTH, fTW, &e->g, &e->smem);
+  }
+  if (!e->ok) return false;
+  *out = e->g;
+  *smem_out = e->smem;
+  return true;
+}
+
+template <int RP>
+bool plan_saved_search(const Cp4BwdFilterArgs& a, const DeviceInfo& di, int fTH, int fTW, SGeom* out, size_t* smem_out) {
+  SGeom best{};
+  double best_cost = 1e300;
+  size_t best_smem = 0;
   for (int TW = 1; TW <= std::min(a.W, 64); ++TW) {
     if (fTW ? TW != std::min(fTW, a.W) : (TW != a.W && a.W % TW != 0 && TW % 8 != 0)) continue;
     for (int TH = 1; TH <= std::min(a.H, 64); ++TH) {
@@ -884,11 +916,17 @@ bool plan_saved(const Cp4BwdFilterArgs& a, const DeviceInfo& di, SGeom* out, siz
   return true;
 }
 
+template <int RP>
+bool plan_saved(const Cp4BwdFilterArgs& a, const DeviceInfo& di, SGeom* out, size_t* smem_out) {
+  return cached_plan<RP, SGeom>(a, di, out, smem_out, plan_saved_search<RP>);
+}
+
 template <int RP, int MBW, bool CORE, int PART>
 int launch_saved_part(const SGeom& g, size_t smem, long ctas, const Cp4BwdFilterArgs& a, const float* P, const float* Q,
                       cudaStream_t st) {
   auto kern = cp4_bwdf_saved_kernel<RP, MBW, CORE, PART>;
-  B200CP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<int> smem_set[64];
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_set, (int)smem));
   kern<<<dim3((unsigned)ctas, (unsigned)g.S), kNT, smem, st>>>(g, a.X, a.dU, P, Q, a.KH, a.KW, a.KC, (float*)a.ws);
   B200CP_LAUNCH_OK("cp4_bwdf_saved_kernel");
   return B200CP_OK;
@@ -958,14 +996,10 @@ int run_saved(const Cp4BwdFilterArgs& a, const float* P, const float* Q, const D
 }
 
 template <int RP>
-bool plan_bwdf(const Cp4BwdFilterArgs& a, const DeviceInfo& di, BGeom* out, size_t* smem_out) {
+bool plan_bwdf_search(const Cp4BwdFilterArgs& a, const DeviceInfo& di, int fTH, int fTW, BGeom* out, size_t* smem_out) {
   BGeom best{};
   double best_cost = 1e300;
   size_t best_smem = 0;
-  int fTH = 0, fTW = 0;
-  if (const char* e = getenv("B200CP_MMA_TILE")) {  // "TH,TW": experiments
-    if (sscanf(e, "%d,%d", &fTH, &fTW) != 2) fTH = fTW = 0;
-  }
   for (int TW = 1; TW <= std::min(a.W, 64); ++TW) {
     if (fTW ? TW != std::min(fTW, a.W) : (TW != a.W && a.W % TW != 0 && TW % 8 != 0)) continue;
     for (int TH = 1; TH <= std::min(a.H, 64); ++TH) {
@@ -997,10 +1031,16 @@ bool plan_bwdf(const Cp4BwdFilterArgs& a, const DeviceInfo& di, BGeom* out, size
   return true;
 }
 
+template <int RP>
+bool plan_bwdf(const Cp4BwdFilterArgs& a, const DeviceInfo& di, BGeom* out, size_t* smem_out) {
+  return cached_plan<RP, BGeom>(a, di, out, smem_out, plan_bwdf_search<RP>);
+}
+
 template <int RP, int MBW, bool CORE>
 int launch_bwdf_core(const BGeom& g, size_t smem, const Cp4BwdFilterArgs& a, cudaStream_t st) {
   auto kern = cp4_bwdf_mma_kernel<RP, MBW, CORE>;
-  B200CP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<int> smem_set[64];
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_set, (int)smem));
   const long ctas = (long)a.N * g.tilesH * g.tilesW;
   if (ctas > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "cp4 bwd-filter: too many tiles");
   const size_t need = (size_t)ctas * g.nparam * sizeof(float);

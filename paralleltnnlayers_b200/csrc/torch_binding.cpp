@@ -117,9 +117,9 @@ using Grads4 = std::array<Tensor, 4>;
 Grads4 split4(const Tensor& dK, const b200cp_tensor_shape& s) {
   const int64_t R = s.Rank, d[4] = {s.T, s.C, s.Y, s.X};
   Grads4 g;
-  int64_t o = 0;
+  int64_t o = dK.storage_offset();
   for (int i = 0; i < 4; ++i) {
-    g[i] = dK.narrow(0, o, d[i] * R).view({d[i], R});
+    g[i] = dK.as_strided({d[i], R}, {R, 1}, o);   // (one operator where narrow and view are three)
     o += d[i] * R;
   }
   return g;
@@ -240,9 +240,9 @@ Tensor cp3_backward_data(const Tensor& dU, const Tensor& KT, const Tensor& KCin,
 }
 
 std::array<Tensor, 3> split3(const Tensor& dK, const b200cp_tensor_shape& s) {
-  const int64_t R = s.Rank, nT = s.T * R, nC = s.C * R, nS = (int64_t)s.Y * s.X * R;
-  return {dK.narrow(0, 0, nT).view({s.T, R}), dK.narrow(0, nT, nC).view({s.C, R}),
-          dK.narrow(0, nT + nC, nS).view({s.Y, s.X, R})};
+  const int64_t R = s.Rank, nT = s.T * R, nC = s.C * R, o = dK.storage_offset();
+  return {dK.as_strided({s.T, R}, {R, 1}, o), dK.as_strided({s.C, R}, {R, 1}, o + nT),
+          dK.as_strided({s.Y, s.X, R}, {s.X * R, R, 1}, o + nT + nC)};
 }
 
 // dX (where it is wanted) and the factor gradients from the forward's rank plane
