@@ -225,6 +225,18 @@ int kron_weight_ld(int fast);
 double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed);
 int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
                        int taps, bool transposed, bool flip, float* W, cudaStream_t st);
+// the same as operand planes of the tensor-core product: rows of ldo values, hi and `plane` on lo, an exponent per row
+bool kron_planes_takes(int order, const int* idims, const int* odims, int R, int sm_count);   // where that is faster
+int kron_planes_launch(int order, const int* idims, const int* odims, int R, const float* const* F, bool transposed, int ldo,
+                       void* hi, size_t plane, int* ex, cudaStream_t st);
+struct KronWeight {   // of a product with the multiplied-out weight: rows are the product's outputs (F, S: null in queries)
+  int order;
+  const int *idims, *odims;
+  int R;
+  const float* const* F;
+  const float* S;
+  bool transposed, flip;
+};
 // Estimated microseconds of the factored form (negative: it does not take the sizes; above `enough` any value above that
 // will do) and of the multiplied-out one.
 double rcp_factored_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -262,15 +274,15 @@ bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW);
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
                         float* scratch, cudaStream_t st);
-// products with the multiplied-out weight: Y[B][N] = X[B][K] W^T (W [N][ldw]), and the 3x3 convolution with W [T][9][ldw]
+// products with the multiplied-out weight, which is formed in the scratch: Y[B][N] = X[B][K] W^T, and the 3x3 convolution
 bool dense_tc_takes();
-double dense_tc_us(int B, int K, int N);
-size_t dense_tc_scratch_floats(int B, int K, int N);
-int dense_tc_launch(int B, int K, int N, const float* X, const float* W, int ldw, float* Y, float* scratch, cudaStream_t st);
+double dense_tc_us(int B, int K, int N, const KronWeight& w);   // with the weight
+size_t dense_tc_scratch_floats(int B, int K, int N, const KronWeight& w);
+int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, float* Y, float* scratch, cudaStream_t st);
 bool conv_tc_takes(int N, int C, int T, int H, int W);
 double conv_tc_us(int N, int C, int T, int H, int W);
-size_t conv_tc_scratch_floats(int N, int C, int T, int H, int W);
-int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, int ldw, float* V, float* scratch,
+size_t conv_tc_scratch_floats(int N, int C, int T, int H, int W);   // with the weight
+int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const KronWeight& w, float* V, float* scratch,
                    cudaStream_t st);
 // the reference's "rebuild" variants: dense conv2d forward with an undecomposed filter K [T][C][FH][FW]; recomposed
 // weights of the dense ([I][O]) and reshaped-CP ([T][C][FH][FW], S != nullptr) layers; Y = X M for the dense layer

@@ -985,7 +985,7 @@ int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const
 }
 
 // ---- products with the multiplied-out weight --------------------------------------------------------------------------------
-// Y[B][N] = X[B][K] W^T with the weight W[N][ldw] as kron_weight_launch writes it.  The rows of the kernel's result are the
+// Y[B][N] = X[B][K] W^T.  The rows of the kernel's result are the
 // outputs (a warp then stores 32 neighbours of Y), or the batch where that leaves less of the tiles empty.
 namespace {
 struct DenseTc {
@@ -1003,26 +1003,38 @@ double split_us(double values) { return 2.5 + values * 8 / 4.5e6; }
 
 bool dense_tc_takes() { return gemm_tc_mode() && get_encode_tiled() != nullptr; }
 
-// without the time of the weight
-double dense_tc_us(int B, int K, int N) {
+double dense_tc_us(int B, int K, int N, const KronWeight& w) {
   DeviceInfo di;
   if (device_info(&di)) return 1e300;
-  return 8.0 + split_us((double)N * K) + split_us((double)B * K) + dense_tc(B, K, N, di).t.us;
+  const double entries = (double)N * K;   // as planes: 62 us for 2^24 at R = 32
+  const double weight = kron_planes_takes(w.order, w.idims, w.odims, w.R, di.sm_count)
+                            ? 8.0 + entries * (1.0e-6 + 7.0e-8 * w.R)
+                            : kron_weight_us(w.order, w.idims, w.odims, w.R, 1, w.transposed) + split_us(entries);
+  return 8.0 + weight + split_us((double)B * K) + dense_tc(B, K, N, di).t.us;
 }
 
-size_t dense_tc_scratch_floats(int B, int K, int N) {
+size_t dense_tc_scratch_floats(int B, int K, int N, const KronWeight& w) {
   DeviceInfo di;
   if (device_info(&di)) return 0;
-  return planes_floats(N, ld8(K), N, false) + planes_floats(B, ld8(K), B, false) + partial_floats(dense_tc(B, K, N, di).t);
+  return (kron_planes_takes(w.order, w.idims, w.odims, w.R, di.sm_count) ? 0 : align_up((size_t)N * kron_weight_ld(K), 64)) +
+         planes_floats(N, ld8(K), N, false) + planes_floats(B, ld8(K), B, false) + partial_floats(dense_tc(B, K, N, di).t);
 }
 
-int dense_tc_launch(int B, int K, int N, const float* X, const float* W, int ldw, float* Y, float* scratch, cudaStream_t st) {
+int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, float* Y, float* scratch, cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   const DenseTc d = dense_tc(B, K, N, di);
-  float* at = scratch;
+  const bool direct = kron_planes_takes(w.order, w.idims, w.odims, w.R, di.sm_count);
+  float *at = scratch, *W = scratch;
+  if (!direct) at += align_up((size_t)N * kron_weight_ld(K), 64);
   const Planes pw = take_planes(at, N, ld8(K), N, false), px = take_planes(at, B, ld8(K), B, false);
-  if (int rc = split_rows(job_of(W, N, 1, K, ldw, pw), job_of(X, B, 1, K, K, px), st)) return rc;
+  if (direct) {
+    if (int rc = kron_planes_launch(w.order, w.idims, w.odims, w.R, w.F, w.transposed, pw.ld, pw.hi, pw.plane, pw.ex, st)) return rc;
+    if (int rc = split_rows(job_of(X, B, 1, K, K, px), SplitJob{}, st)) return rc;
+  } else {
+    if (int rc = kron_weight_launch(w.order, w.idims, w.odims, w.R, w.F, nullptr, 1, w.transposed, false, W, st)) return rc;
+    if (int rc = split_rows(job_of(W, N, 1, K, kron_weight_ld(K), pw), job_of(X, B, 1, K, K, px), st)) return rc;
+  }
   const Planes &pa = d.rows_are_batch ? px : pw, &pb = d.rows_are_batch ? pw : px;
   CUtensorMap ma, mb;
   if (int rc = encode_planes(&ma, pa.hi, {(size_t)K, 1, pa.rows}, {(size_t)pa.ld, (size_t)pa.ld}, pa.plane, {64, 1, 128})) return rc;
@@ -1038,7 +1050,7 @@ int dense_tc_launch(int B, int K, int N, const float* X, const float* W, int ldw
   return run_split_gemm(g, d.t, 0, false, false, ma, mb, Y, at, di, st);
 }
 
-// V[n,t,h,w] = sum_{c,y,x} W[t][y,x][c] X[n,c,h+y-1,w+x-1] (3 x 3), the weight [T][9][ldw]: rows are the padded pixels, and a
+// V[n,t,h,w] = sum_{c,y,x} W[t][y,x][c] X[n,c,h+y-1,w+x-1] (3 x 3): rows are the padded pixels, and a
 // step is 64 channels of one tap.
 namespace {
 constexpr int kPad = 1, kTaps = 9;
@@ -1061,18 +1073,20 @@ size_t conv_tc_scratch_floats(int N, int C, int T, int H, int W) {
   DeviceInfo di;
   if (device_info(&di)) return 0;
   const size_t px = (size_t)N * (H + kPad) * (W + kPad);
-  return planes_floats(T, (size_t)kTaps * ld8(C), T, false) + planes_floats(px, ld8(C), px, false) +
+  return align_up((size_t)T * kTaps * kron_weight_ld(C), 64) + planes_floats(T, (size_t)kTaps * ld8(C), T, false) + planes_floats(px, ld8(C), px, false) +
          partial_floats(conv_tc(N, C, T, H, W, di));
 }
 
-int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, int ldw, float* V, float* scratch,
+int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const KronWeight& w, float* V, float* scratch,
                    cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   const TcTiles t = conv_tc(N, C, T, H, W, di);
   const int Wp = W + kPad, PP = (H + kPad) * Wp;
   const size_t px = (size_t)N * PP, ldk = ld8(C);
-  float* at = scratch;
+  const int ldw = kron_weight_ld(C);
+  float *Wt = scratch, *at = scratch + align_up((size_t)T * kTaps * ldw, 64);
+  if (int rc = kron_weight_launch(w.order, w.idims, w.odims, w.R, w.F, w.S, kTaps, w.transposed, w.flip, Wt, st)) return rc;
   Planes pw = take_planes(at, T, kTaps * ldk, T, false), pa = take_planes(at, px, ldk, px, false);
   pw.ld = (int)ldk;
   const SplitJob none{};

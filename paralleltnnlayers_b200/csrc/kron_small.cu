@@ -17,6 +17,7 @@
 #include "cluster_util.cuh"
 #include "common.cuh"
 #include "mma_util.cuh"
+#include "tc_common.cuh"
 
 namespace b200cp {
 namespace {
@@ -203,6 +204,144 @@ __global__ void __launch_bounds__(kKT) kron_weight_kernel(const __grid_constant_
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (b + j < PB) d[ob[tx * 4 + j]] = acc[i][j];
+    }
+  }
+}
+
+// ---- the weight as the operand planes of the tensor-core product (gemm_tc.cu) ------------------------------------------
+// Row s of the weight gets the exponent of a bound, sum_r prod_k max_f |F_k[s_k, f, r]|, which needs no pass over the weight (it is
+// some 2^5 above the largest entry; of the 18 binades below a row's largest value that keep 22 bits this costs five).
+// One warp per row.
+__global__ void __launch_bounds__(256) kron_exponent_kernel(const __grid_constant__ KronGeom g, int rows, int* __restrict__ ex) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  float sum = 0.f;
+  for (int r = lane; r < g.R; r += 32) {
+    float prod = 1.f;
+    int s = row;
+    for (int k = g.nA + g.nB - 1; k >= 0; --k) {
+      const KronMode& m = k < g.nA ? g.A[k] : g.B[k - g.nA];
+      const int sk = s % m.ns;
+      s /= m.ns;
+      unsigned mx = 0;
+#pragma unroll 4
+      for (int f = 0; f < m.nf; ++f) mx = max(mx, tc::abs_bits(__ldg(m.F + (size_t)(sk * m.fs + f * m.ff) * g.R + r)));
+      prod *= __uint_as_float(mx);
+    }
+    sum += prod;
+  }
+#pragma unroll
+  for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+  if (lane == 0) ex[row] = tc::row_exponent(tc::abs_bits(sum * 1.001f), tc::kLeast);
+}
+
+// 128 x 128 entries per CTA and tile, 8 x 8 per thread (four 16-byte reads per 64 FFMA).  A CTA keeps its half products A and
+// walks the tiles of B; ranks in chunks of 32, A's formed once.  Each entry is stored as its hi and lo
+// halves, 8 bytes of each where four are neighbours.
+// 4096 x 4096 at R = 32: the weight in fp32 (64 x 64 tiles, one per CTA) 68 us and 18 us more to split it, here 56 and 6 for the exponents.
+constexpr int kPT = 128, kPP = kPT + 4, kKeep = 256;
+__global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_constant__ KronGeom g, int pitch, int btiles,
+                                                          const int* __restrict__ ex, __half* __restrict__ hi, size_t plane) {
+  extern __shared__ __align__(16) float smem[];
+  const int keep = (g.R + kRC - 1) / kRC * kRC;   // at most kKeep
+  float* As = smem;                       // [keep][kPP]
+  float* Bs = As + keep * kPP;            // [kRC][kPP]
+  __shared__ int ea[kPT][2], eb[kPT][2], oa[kPT], ob[kPT];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int a0 = blockIdx.y * kPT, PA = g.SA * g.FA, PB = g.SB * g.FB;
+  constexpr int NM = 2;   // modes of a half
+  if (tid < kPT) {
+    int e[3] = {0, 0, 0}, o = 0;
+    if (a0 + tid < PA) half_decode(g.A, g.nA, (a0 + tid) / g.FA, (a0 + tid) % g.FA, 0, e, &o);
+    ea[tid][0] = e[0]; ea[tid][1] = e[1];
+    oa[tid] = o;
+  }
+  // half products of ranks r0 .. r0 + 31 to dst[rank][row]; a warp forms 8 ranks x 4 rows per turn
+  const int rl = tid & 7, row0 = (tid >> 5) * 4 + ((tid >> 3) & 3);
+  auto form = [&](bool isA, int first, int count, int r0, float* dst) {
+    const KronMode* m = isA ? g.A : g.B;
+    const int n = isA ? g.nA : g.nB;
+#pragma unroll
+    for (int i = 0; i < kPT / 32; ++i) {
+      const int row = i * 32 + row0;
+      const bool in = first + row < count;
+      float v[kRC / 8];
+#pragma unroll
+      for (int rb = 0; rb < kRC / 8; ++rb) v[rb] = in && r0 + rb * 8 + rl < g.R ? 1.f : 0.f;
+#pragma unroll
+      for (int k = 0; k < NM; ++k)
+        if (in && k < n) {
+          const float* src = m[k].F + (size_t)(isA ? ea[row][k] : eb[row][k]) * g.R + r0 + rl;
+#pragma unroll
+          for (int rb = 0; rb < kRC / 8; ++rb)
+            if (r0 + rb * 8 + rl < g.R) v[rb] *= __ldg(src + rb * 8);
+        }
+#pragma unroll
+      for (int rb = 0; rb < kRC / 8; ++rb) dst[(rb * 8 + rl) * kPP + row] = v[rb];
+    }
+  };
+  __syncthreads();
+  for (int r0 = 0; r0 < keep; r0 += kRC) form(true, a0, PA, r0, As + r0 * kPP);
+  for (int bt = blockIdx.x; bt < btiles; bt += gridDim.x) {
+    const int b0 = bt * kPT;
+    __syncthreads();   // the tile before is done with the tables
+    if (tid < kPT) {
+      int e[2] = {0, 0}, o = 0;
+      if (b0 + tid < PB) half_decode(g.B, g.nB, (b0 + tid) / g.FB, (b0 + tid) % g.FB, 0, e, &o);
+      eb[tid][0] = e[0]; eb[tid][1] = e[1];
+      ob[tid] = o;
+    }
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int r0 = 0; r0 < g.R; r0 += kRC) {
+      __syncthreads();
+      form(false, b0, PB, r0, Bs);
+      __syncthreads();
+      const float* Ar = As + r0 * kPP;
+      const int rn = min(kRC, g.R - r0);
+#pragma unroll 2
+      for (int r = 0; r < rn; ++r) {
+        const float4 x0 = *reinterpret_cast<const float4*>(Ar + r * kPP + ty * 4), x1 = *reinterpret_cast<const float4*>(Ar + r * kPP + 64 + ty * 4);
+        const float4 y0 = *reinterpret_cast<const float4*>(Bs + r * kPP + tx * 4), y1 = *reinterpret_cast<const float4*>(Bs + r * kPP + 64 + tx * 4);
+        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+      }
+    }
+#pragma unroll
+    for (int j4 = 0; j4 < 2; ++j4) {
+      const int jb = j4 * 64 + tx * 4, left = PB - (b0 + jb);
+      const bool run4 = left >= 4 && ob[jb + 3] - ob[jb] == 3 && !(ob[jb] & 3);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int ia = (i >> 2) * 64 + ty * 4 + (i & 3);
+        if (a0 + ia >= PA) continue;
+        const float* v = acc[i] + j4 * 4;
+        const int o = oa[ia] + ob[jb];
+        if (run4 && !(oa[ia] & 3)) {   // four neighbours of one row
+          const float sc = tc::exp2_int(-__ldg(ex + o / pitch));
+          const __half2 h0 = __floats2half2_rn(v[0] * sc, v[1] * sc), h1 = __floats2half2_rn(v[2] * sc, v[3] * sc);
+          const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+          const __half2 l0 = __floats2half2_rn(v[0] * sc - f0.x, v[1] * sc - f0.y), l1 = __floats2half2_rn(v[2] * sc - f1.x, v[3] * sc - f1.y);
+          *reinterpret_cast<uint2*>(hi + o) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+          *reinterpret_cast<uint2*>(hi + plane + o) = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < left) {
+              const int oj = oa[ia] + ob[jb + j];
+              const float w = v[j] * tc::exp2_int(-__ldg(ex + oj / pitch));
+              const __half h = __float2half_rn(w);
+              hi[oj] = h;
+              hi[plane + oj] = __float2half_rn(w - __half2float(h));
+            }
+        }
+      }
     }
   }
 }
@@ -597,10 +736,9 @@ double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* 
 // Row pitch of the weight: 16-byte rows.
 int kron_weight_ld(int fast) { return (fast + 3) / 4 * 4; }
 
-// W[s][ld] (dense) or W[s][tap][ld] (S given): slow side = inputs, or outputs with `transposed`; with `flip` the taps run
-// backwards (a data gradient)
-int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
-                       int taps, bool transposed, bool flip, float* W, cudaStream_t st) {
+// the modes and halves of a weight with rows of `ld` entries per tap
+static int kron_geom(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S, int taps,
+                     bool transposed, bool flip, int ld, long* rows, KronGeom* out) {
   KronMode m[4];
   long slow = 1, fast = 1;
   for (int k = 0; k < order; ++k) {
@@ -612,7 +750,7 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
     slow *= m[k].ns;
     fast *= m[k].nf;
   }
-  const int ld = kron_weight_ld((int)fast), row = S ? taps * ld : ld;
+  const int row = S ? taps * ld : ld;
   if (slow * row > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight too large");
   long os = row, of = 1;
   for (int k = order - 1; k >= 0; --k) {
@@ -632,6 +770,19 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   }
   for (int k = 0; k < ha; ++k) { g.A[g.nA++] = m[k]; g.SA *= m[k].ns; g.FA *= m[k].nf; }
   for (int k = ha; k < order; ++k) { g.B[g.nB++] = m[k]; g.SB *= m[k].ns; g.FB *= m[k].nf; }
+  *rows = slow;
+  *out = g;
+  return B200CP_OK;
+}
+
+// W[s][ld] (dense) or W[s][tap][ld] (S given): slow side = inputs, or outputs with `transposed`; with `flip` the taps run
+// backwards (a data gradient)
+int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
+                       int taps, bool transposed, bool flip, float* W, cudaStream_t st) {
+  long fast = 1, rows;
+  for (int k = 0; k < order; ++k) fast *= transposed ? idims[k] : odims[k];
+  KronGeom g;
+  if (int rc = kron_geom(order, idims, odims, R, F, S, taps, transposed, flip, kron_weight_ld((int)fast), &rows, &g)) return rc;
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   const KronPlan p = kron_plan(order, transposed ? odims : idims, transposed ? idims : odims, R, S ? taps : 1, di);
@@ -648,6 +799,37 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   else KRON(16);
 #undef KRON
   B200CP_LAUNCH_OK("kron_weight_kernel");
+  return B200CP_OK;
+}
+
+// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 62 us with the exponents, against 86 for the fp32 weight and
+// its split; but 1000 x 1000 at R = 16 21 against 13, 4096 x 64 at R = 64 50 against 20.
+bool kron_planes_takes(int order, const int* idims, const int* odims, int R, int sm_count) {
+  double pa = 1, pb = 1;
+  for (int k = 0; k < order; ++k) (k < order / 2 ? pa : pb) *= (double)idims[k] * odims[k];
+  return R <= kKeep && std::ceil(pa / kPT) * std::ceil(pb / kPT) >= 2.0 * sm_count && pa >= kPT && pb >= kPT;
+}
+
+// The same weight as hi / lo planes of `plane` values with rows of ldo, a multiple of 4, and one exponent per row (kron_planes_takes).
+int kron_planes_launch(int order, const int* idims, const int* odims, int R, const float* const* F, bool transposed, int ldo,
+                       void* hi, size_t plane, int* ex, cudaStream_t st) {
+  KronGeom g;
+  long rows;
+  if (int rc = kron_geom(order, idims, odims, R, F, nullptr, 1, transposed, false, ldo, &rows, &g)) return rc;
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  kron_exponent_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(g, (int)rows, ex);
+  B200CP_LAUNCH_OK("kron_exponent_kernel");
+  const int atiles = ceil_div(g.SA * g.FA, kPT), btiles = ceil_div(g.SB * g.FB, kPT);
+  if (atiles > 65535 || R > kKeep) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight too large");
+  const size_t smem = sizeof(float) * (align_up((size_t)R, kRC) + kRC) * kPP;
+  static std::atomic<int> set[64];
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_planes_kernel), set, (int)smem));
+  // as many CTAs as are resident at once share the tiles of B
+  const int walkers = std::min(btiles, std::max(1, 2 * di.sm_count / atiles));
+  const dim3 grid(ceil_div(btiles, ceil_div(btiles, walkers)), atiles);
+  kron_planes_kernel<<<grid, 256, smem, st>>>(g, ldo, btiles, ex, static_cast<__half*>(hi), plane);
+  B200CP_LAUNCH_OK("kron_planes_kernel");
   return B200CP_OK;
 }
 

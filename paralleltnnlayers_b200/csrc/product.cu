@@ -35,6 +35,15 @@ constexpr double kMostEntries = 1e9;
 // With fewer ranks the factored kernels' sums are short enough to round less than the tensor product does (R = 4, 4096 samples of
 // 10x10x10 -> 10x10x10: 1.4e-7 of the result against 1.55e-7), and they are not far behind or ahead.
 constexpr int kLeastRanks = 8;
+// Below this many multiply-adds the FFMA product takes less than the tensor one's fixed 20 us (512 x 512 -> 512: 19 us), and the
+// search for its tiles is not worth the host's time.
+constexpr double kLeastMacs = 1e8;
+// The tensor product holds hi / lo planes of the weight and of the activations: as much again as the layer's input.
+constexpr size_t kMostPlanes = size_t{1} << 30;
+bool tensor_may(int flags, int R, double macs) {
+  if (!(flags & B200CP_TENSOR_PRODUCTS)) return false;
+  return gemm_tc_mode() == 2 || (R >= kLeastRanks && macs >= kLeastMacs);
+}
 
 enum class Form { factored, ffma, tensor };
 
@@ -58,14 +67,15 @@ DensePlan dense_plan(int B, int order, const int* idims, const int* odims, int R
   p.K = (int)prod(transposed ? odims : idims, order);
   p.N = (int)prod(transposed ? idims : odims, order);
   const double ffma = dense_kron_us(B, order, idims, odims, R, transposed);
-  const double tensor = (flags & B200CP_TENSOR_PRODUCTS) && dense_tc_takes() && (R >= kLeastRanks || gemm_tc_mode() == 2)
-                            ? kron_weight_us(order, idims, odims, R, 1, !transposed) + dense_tc_us(B, p.K, p.N) : -1;
+  const bool may = tensor_may(flags, R, (double)B * p.K * p.N) && dense_tc_takes();
+  const KronWeight w{order, idims, odims, R, nullptr, nullptr, !transposed, false};
+  const size_t planes = may ? align_up(dense_tc_scratch_floats(B, p.K, p.N, w) * sizeof(float), 256) : 0;
+  const double tensor = may && planes <= kMostPlanes ? dense_tc_us(B, p.K, p.N, w) : -1;
   const double least = tensor >= 0 ? std::min(ffma, tensor) : ffma;
   p.weight = weight_floats(order, idims, odims, 1, transposed);
   p.form = pick(p.weight, (double)p.K * p.N, ffma, tensor, dense_factored_us(B, order, idims, odims, R, transposed, least));
   if (p.form == Form::tensor) {
-    p.weight = weight_floats(order, idims, odims, 1, !transposed);
-    p.bytes = align_up(p.weight * sizeof(float), 256) + align_up(dense_tc_scratch_floats(B, p.K, p.N) * sizeof(float), 256);
+    p.bytes = planes;
   } else if (p.form == Form::ffma) {
     p.bytes = align_up(p.weight * sizeof(float), 256);
   }
@@ -79,15 +89,16 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
   p.K = (int)prod(transposed ? tdims : cdims, order);
   p.N = (int)prod(transposed ? cdims : tdims, order);
   const double ffma = rcp_kron_us(N, H, W, order, cdims, tdims, R, transposed);
-  const double tensor = (flags & B200CP_TENSOR_PRODUCTS) && conv_tc_takes(N, p.K, p.N, H, W) && (R >= kLeastRanks || gemm_tc_mode() == 2)
+  const bool may = tensor_may(flags, R, 9.0 * N * H * W * p.K * p.N) && conv_tc_takes(N, p.K, p.N, H, W);
+  const size_t planes = may ? align_up(conv_tc_scratch_floats(N, p.K, p.N, H, W) * sizeof(float), 256) : 0;
+  const double tensor = may && planes <= kMostPlanes
                             ? kron_weight_us(order, cdims, tdims, R, 9, !transposed) + conv_tc_us(N, p.K, p.N, H, W) : -1;
   const double least = tensor >= 0 ? std::min(ffma, tensor) : ffma;
   p.weight = weight_floats(order, cdims, tdims, 9, transposed);
   p.form = pick(p.weight, 9.0 * p.K * p.N, ffma, tensor,
                 rcp_factored_us(N, H, W, order, cdims, tdims, R, FH, FW, transposed, least));
   if (p.form == Form::tensor) {
-    p.weight = weight_floats(order, cdims, tdims, 9, !transposed);
-    p.bytes = align_up(p.weight * sizeof(float), 256) + align_up(conv_tc_scratch_floats(N, p.K, p.N, H, W) * sizeof(float), 256);
+    p.bytes = planes;
   } else if (p.form == Form::ffma) {
     p.bytes = align_up(p.weight * sizeof(float), 256);
   }
@@ -97,10 +108,6 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
 bool fits(const DensePlan& p, const void* ws, size_t ws_bytes) {
   return p.bytes && ws && ws_bytes >= p.bytes && !(reinterpret_cast<uintptr_t>(ws) & 15);
 }
-float* after_weight(const DensePlan& p, void* ws) {
-  return reinterpret_cast<float*>(static_cast<char*>(ws) + align_up(p.weight * sizeof(float), 256));
-}
-
 }  // namespace
 
 size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed, int flags) {
@@ -117,10 +124,10 @@ int dense_product_launch(int B, int order, const int* idims, const int* odims, i
   const DensePlan p = B > 0x7fffffff - 64 ? DensePlan{} : dense_plan(B, order, idims, odims, R, transposed, flags);
   if (!fits(p, ws, ws_bytes)) return dense_chain_launch(B, order, idims, odims, R, X, F, Y, transposed, st);
   float* Wt = static_cast<float*>(ws);
-  const bool tensor = p.form == Form::tensor;
-  if (int rc = kron_weight_launch(order, idims, odims, R, F, nullptr, 1, transposed != tensor, false, Wt, st)) return rc;
-  return tensor ? dense_tc_launch(B, p.K, p.N, X, Wt, kron_weight_ld(p.K), Y, after_weight(p, ws), st)
-                : small_gemm_launch(B, p.N, p.K, X, Wt, Y, st);
+  if (p.form == Form::tensor)
+    return dense_tc_launch(B, p.K, p.N, X, KronWeight{order, idims, odims, R, F, nullptr, !transposed, false}, Y, Wt, st);
+  if (int rc = kron_weight_launch(order, idims, odims, R, F, nullptr, 1, transposed, false, Wt, st)) return rc;
+  return small_gemm_launch(B, p.N, p.K, X, Wt, Y, st);
 }
 
 size_t rcp_product_workspace(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
@@ -138,10 +145,10 @@ int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const i
   if (!fits(p, ws, ws_bytes))
     return rcp_chain_launch(N, H, W, order, cdims, tdims, R, FH, FW, X, A, S, V, transposed, st);
   float* Wt = static_cast<float*>(ws);
-  const bool tensor = p.form == Form::tensor;
-  if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, FH * FW, transposed != tensor, transposed, Wt, st)) return rc;
-  return tensor ? conv_tc_launch(N, p.K, p.N, H, W, X, Wt, kron_weight_ld(p.K), V, after_weight(p, ws), st)
-                : small_conv_launch(N, p.K, p.N, H, W, X, Wt, V, st);
+  if (p.form == Form::tensor)
+    return conv_tc_launch(N, p.K, p.N, H, W, X, KronWeight{order, cdims, tdims, R, A, S, !transposed, transposed}, V, Wt, st);
+  if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, FH * FW, transposed, transposed, Wt, st)) return rc;
+  return small_conv_launch(N, p.K, p.N, H, W, X, Wt, V, st);
 }
 
 }  // namespace b200cp

@@ -36,7 +36,9 @@ def _rel(got, ref):
 
 
 DENSE = [(1, (4, 4), (2, 4)), (63, (3, 5), (3, 3)), (65, (16, 4), (16, 4)), (130, (5, 13), (11, 12)), (257, (16, 8), (16, 16)),
-         (300, (16, 12), (16, 9)), (77, (16, 16), (16, 16, 1)[:2]), (700, (7, 9), (16, 16)), (40, (16, 16), (13, 7))]
+         (300, (16, 12), (16, 9)), (77, (16, 16), (16, 16)), (700, (7, 9), (16, 16)), (40, (16, 16), (13, 7)),
+         (33, (13,), (9,)), (50, (4, 3, 5), (5, 4, 3)), (129, (4, 5, 3, 2), (2, 3, 4, 5)), (66, (16, 9), (12, 12)),
+         (21, (45, 49), (47, 47)), (22, (6, 7, 5, 9), (8, 7, 9, 7))]   # the last two: the weight written as operand planes
 
 
 @pytest.mark.parametrize("case", DENSE, ids=str)
@@ -47,7 +49,8 @@ def test_dense(case, offset):
     normal = _normal(B + offset)
     I, O = math.prod(idims), math.prod(odims)
     x, dy = normal(B * I + offset)[offset:].view(B, I), normal(B * O + offset)[offset:].view(B, O)
-    F = [normal(i, o, 9) * 0.35 for i, o in zip(idims, odims)]
+    R = {21: 40, 33: 33, 50: 64, 66: 300}.get(B, 9)   # the weight is formed 32 ranks at a time
+    F = [normal(i, o, R) * 0.35 for i, o in zip(idims, odims)]
     M = _kron(F).sum(-1)
     n0 = P.launch_count()
     assert _rel(P.dense_cp(x, *F), x.double() @ M) < REL
@@ -62,7 +65,7 @@ def test_dense(case, offset):
 
 
 RCP = [(1, 3, 5, (3, 3), (4, 3)), (2, 7, 9, (4, 4), (5, 5)), (3, 8, 8, (5, 13), (16, 4)), (1, 16, 17, (16, 8), (13, 10)),
-       (5, 9, 4, (16, 12), (16, 16))]
+       (5, 9, 4, (16, 12), (16, 16)), (2, 5, 6, (7,), (10,)), (2, 6, 5, (3, 4, 2), (2, 5, 3)), (1, 9, 9, (2, 3, 2, 3), (4, 2, 3, 2))]
 
 
 @pytest.mark.parametrize("case", RCP, ids=str)
