@@ -125,7 +125,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (s->Rank <= 16) {
     const double few = ch * std::sqrt((double)s->Rank) / root4;
     switch (use) {
-      case Planes::kConv: return s->Rank > 8 && few >= 130;
+      case Planes::kConv: return s->Rank > 8 && few >= 130 && s->W % 4;   // (the row stream takes the others)
       case Planes::kStep: return few >= 110;
       case Planes::kSaved: return few >= 100;
       case Planes::kFilter: return few >= 42;
