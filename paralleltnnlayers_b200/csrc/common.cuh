@@ -263,13 +263,14 @@ int check_kron_modes(int order, const int* idims, const int* odims, int R, const
 size_t dense_grad_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);
 int dense_grad_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
                       float* scratch, cudaStream_t st);
-// tcgen05 products (gemm_tc.cu; scaled fp16 hi / lo operands, fp32-grade).  Gradient product: G[M][N] = A^T B, A [K][M], B [K][N]
+// tcgen05 products (gemm_tc.cu; scaled fp16 hi / lo operands, in gradients three bf16 parts).  Gradient product: G[M][N] = A^T B, A [K][M],
+// B [K][N]
 int gemm_tc_mode();   // 0 off, 1 by the rules, 2 always
 bool gemm_tc_supported(int K, int M, int N);
 size_t gemm_tc_scratch_floats(int K, int M, int N);
 int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st);
 int gemm_tc_status(int* out);
-// conv form of the same kernel: G[tap][T][C] from NCHW operands (padded, transposed hi / lo planes in the scratch)
+// conv form of the same kernel: G[tap][T][C] from NCHW operands (padded, transposed planes in the scratch)
 bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW);
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,

@@ -1,29 +1,37 @@
 // D[m][n] = sum_k A[m][k] B[n][k] on the tcgen05 tensor cores with the accuracy of fp32 sums: the gradient product of the
 // CP dense layer and of the reshaped-CP convolution, and the product of either layer with its multiplied-out weight.
 //
-// Accuracy.  A value x is scaled by a power of two (exact) so that the largest of its row is in [2^14, 2^15), and split into
-// hi = fp16(x), lo = fp16(x - hi): 22 bits, down to 2^-18 of the row's largest value; smaller values have an absolute
-// error of 2^-40 of it.  The product is hi*hi + hi*lo + lo*hi (three tcgen05.mma.kind::f16; a tf32 split has the same 22
-// bits at half the rate).  The tensor core cuts its fp32 sums off instead of rounding them, which over thousands of terms
-// is a bias of 1e-5 (4096 terms in one accumulator: 2.9e-5 against float64 in the factor gradients).  So an accumulator
-// holds 64 or 32 terms, the small products first, and is then added to a total in registers, in fp32 with rounding.
+// Accuracy, products with the weight.  A value x is scaled by a power of two (exact) so that the largest of its row is in
+// [2^14, 2^15), and split into hi = fp16(x), lo = fp16(x - hi): 22 bits, down to 2^-18 of the row's largest value; smaller values
+// have an absolute error of 2^-40 of it.  The product is hi*hi + hi*lo + lo*hi (three tcgen05.mma.kind::f16; a tf32 split has
+// the same 22 bits at half the rate).
+// Gradient products.  The sum runs over samples (pixels) there, and one of them may be any number of binades above the others and
+// still add nothing (a masked sample: its gradient is zero).  No exponent that samples share keeps the others exact, so each
+// value keeps its own: x is the sum of three bf16 values, 24 bits, and the product six of theirs (without those below 2^-24).
+// Twice the tensor work: 4096 x 4096 x 4096 637 us, nine taps of 256 x 256 at 32 x 28 x 28 153, where fp16 pairs with
+// an exponent per column took 326 and 84 and lost all others beside one sample of 1e12.
+// The tensor core cuts its fp32 sums off instead of rounding them, which over thousands of terms is a bias of 1e-5 (4096
+// terms in one accumulator: 2.9e-5 against float64 in the factor gradients).  So an accumulator holds 64 or 32 terms, the small
+// products first, and is then added to a total in registers, in fp32 with rounding.
 //
 // Layout.  A pair of CTAs (cta_group::2) forms a 256 x BN tile: each loads its 128 rows of A and half of the columns of B,
-// 64 KB a step for 3 x 128 x 256 x 64 multiply-adds.  With one CTA per 128 x 256 tile it would be 96 KB, and the
-// stream from L2 is what bounds such a kernel.  TMA fills a ring of three or four stages, one thread of the pair issues the
-// products into two accumulators in turn, and the other warps of each CTA move the other accumulator to the totals meanwhile
-// (the totals are half of the register file: that is what ends the tile at 128 x 256 per CTA).  The pairs are persistent: the
-// totals of a tile are stored while the products of the next have begun.
+// 64 KB a step for 3 x 128 x 256 x 64 multiply-adds (gradients: 48 KB for 6 x 128 x 256 x 32).  With one CTA per 128 x 256 tile
+// it would be 96 KB, and the stream from L2 is what bounds such a kernel.  TMA fills a ring of three to five stages, one thread
+// of the pair issues the products into two (narrower tiles: four) accumulators in turn, and the other warps of each CTA move the
+// finished ones to the totals meanwhile (the totals are half of the register file: that is what ends the tile at 128 x 256 per CTA).
+// The pairs are persistent: the totals of a tile are stored while the products of the next have begun.
 // Operands: K-major ([row][k], 64 k = one 128-byte swizzled row) or MN-major ([k][row], boxes of 64 rows), both taken by
 // tcgen05 directly, so that neither the batch-major activations of a gradient nor the weight are transposed in memory.
-// Measured, 4096 x 4096 x 4096: 305 to 335 us = 1.35 to 1.23 PFLOP/s of fp16 products, where cuBLAS sustains 1.40 under the power
-// cap (tf32 planes and one accumulator over all of K: 671 us, and 100 times the error).  Without the cut of the last round of
-// tiles 348 us; with eight read-out warps of 128 columns instead of sixteen 317 against 307.
+// Measured, 4096 x 4096 x 4096 with the weight: 305 to 335 us = 1.35 to 1.23 PFLOP/s of fp16 products, and 1.29 of bf16 products in
+// the gradient, where cuBLAS sustains 1.40 under the power cap.  Without the cut of the last round of tiles 348 us; with eight
+// read-out warps of 128 columns instead of sixteen 317 against 307.
 // Roles (TMA warp, MMA warp, read-out warps) meet only through mbarriers; every wait is bounded, and a wait that
 // runs out sets a status word and lets the CTA leave through its normal exit (TMEM released).
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+
+#include <cuda_bf16.h>
 
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -37,14 +45,16 @@ namespace {
 using namespace tc;
 
 constexpr int kBM = 256;              // rows of a pair's tile: 128 per CTA
-constexpr int kKS = 64;               // K of one step: 128 bytes of fp16
-constexpr int kAPlane = 128 * 128;    // bytes of one plane (hi or lo) of A in a stage
+constexpr int kKS = 64, kGradKS = 32; // K of one step, K-major and MN-major
 
-template <int BN>
+template <int BN, bool MN>
 struct Tile {
-  static constexpr int bplane = BN / 2 * 128;
-  static constexpr int stage = 2 * (kAPlane + bplane);                  // 64, 48, 40 KB
-  static constexpr int stages = BN == 256 ? 3 : BN == 128 ? 4 : 5;
+  static constexpr int ks = MN ? kGradKS : kKS, planes = MN ? 3 : 2;
+  static constexpr int box = planes * ks * 128;                         // MN-major: 64 rows, all planes
+  static constexpr int aplane = MN ? ks * 128 : 128 * 128, bplane = MN ? ks * 128 : BN / 2 * 128;   // from one plane to the next
+  static constexpr int abytes = planes * 128 * ks * 2;
+  static constexpr int stage = abytes + planes * BN / 2 * ks * 2;       // 64, 48, 40 KB; MN-major: 48, 36 KB
+  static constexpr int stages = MN ? (BN == 256 ? 4 : 5) : BN == 256 ? 3 : BN == 128 ? 4 : 5;
   static constexpr int depth = BN == 256 ? 2 : 4;                       // accumulators
   static constexpr int tmem_cols = depth * BN;                          // 512, 512, 256
   static constexpr int cols = BN == 64 ? 32 : 64;                       // of a read-out warp
@@ -62,7 +72,7 @@ struct SplitGemm {
   int group;                     // K of an accumulator, in instructions of 16 (see kShortSum)
   int kc, Kc;                    // K-major: steps and channels per tap (dense: one tap); MN-major: Kc = rows of K
   int FW, padH, padW, Wp;        // a filter tap (y, x) shifts the rows of A by (y - padH) * Wp + (x - padW)
-  // A value of A stands for 2^ea of itself, one of B for 2^eb.  Rows of A with one exponent over all of K: added at the end.
+  // K-major: a value of A stands for 2^ea of itself, one of B for 2^eb.  Rows of A with one exponent over all of K: added at the end.
   // In a convolution the row that a step reads moves with the tap, so the totals take 2^(ea - 24) of each step and
   // 2^(eb + 24) at the end: 24 binades for sums of values near the largest float.
   const int *ea, *eb;
@@ -131,9 +141,10 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
       : "memory");
 }
 
-// Instruction descriptor for kind::f16 with fp16 operands and fp32 accumulation, M = 256 (a pair).
+// Instruction descriptor for kind::f16 with fp32 accumulation, M = 256 (a pair).
+// MN-major operands are bf16.
 __host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n, uint32_t mn) {
-  return (1u << 4) | (mn << 15) | (mn << 16) | ((n >> 3) << 17) | ((256u >> 4) << 24);
+  return (1u << 4) | (mn << 7) | (mn << 10) | (mn << 15) | (mn << 16) | ((n >> 3) << 17) | ((256u >> 4) << 24);
 }
 
 // Bounded wait shared by the roles: gives up after about a second, or as soon as another role of the CTA has given up.
@@ -199,9 +210,10 @@ __device__ __forceinline__ void next_step(const SplitGemm& g, StepAt& k) {
   }
 }
 // instructions of 16 k of a step
+template <int KS>
 __device__ __forceinline__ int k16_of(const SplitGemm& g, int c) {
-  const int left = g.Kc - c * kKS;
-  return left >= kKS ? kKS / 16 : (left + 15) / 16;
+  const int left = g.Kc - c * KS;
+  return left >= KS ? KS / 16 : (left + 15) / 16;
 }
 __device__ __forceinline__ int tap_shift(const SplitGemm& g, int tap) {
   const int y = tap / g.FW;
@@ -221,10 +233,10 @@ __device__ __forceinline__ bool row_at(const SplitGemm& g, int m, long* off) {
 }
 
 template <int BN, bool MN, bool CONV>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Tile<BN>::threads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Tile<BN, MN>::threads, 1)
 split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ CUtensorMap mapA,
                   const __grid_constant__ CUtensorMap mapB) {
-  using T = Tile<BN>;
+  using T = Tile<BN, MN>;
   constexpr int kStages = T::stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -276,14 +288,14 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
           if (it >= kStages && !(ok = wait_or_abort(emptyb + slot * 8, ((it / kStages) - 1) & 1, abortb))) break;
           if (rank == 0) mbar_expect_tx(&full[slot], 2 * T::stage);
           const uint32_t bar = leader_addr(fullb + slot * 8);
-          const uint32_t a = smem_u32(sm) + slot * T::stage, b = a + 2 * kAPlane;
-          if (MN) {   // boxes of 64 rows x 64 k, both planes; rows of K outside the tensor read as zero
+          const uint32_t a = smem_u32(sm) + slot * T::stage, b = a + T::abytes;
+          if (MN) {   // boxes of 64 rows x 32 k, all planes; rows of K outside the tensor read as zero
 #pragma unroll
             for (int q = 0; q < 2; ++q)
-              tma_load_pair(a + q * kAPlane, &mapA, bar, t.m0 + rank * 128 + q * 64, k.c * kKS + t.shift, 0);
+              tma_load_pair(a + q * T::box, &mapA, bar, t.m0 + rank * 128 + q * 64, k.c * T::ks + t.shift, 0);
 #pragma unroll
             for (int q = 0; q < BN / 128; ++q)
-              tma_load_pair(b + q * kAPlane, &mapB, bar, t.n0 + rank * (BN / 2) + q * 64, k.c * kKS, 0);
+              tma_load_pair(b + q * T::box, &mapB, bar, t.n0 + rank * (BN / 2) + q * 64, k.c * T::ks, 0);
           } else {    // boxes of 64 k x the rows, both planes; channels past Kc read as zero
             const int shift = CONV ? tap_shift(g, k.tap) : 0;
             tma_load_pair(a, &mapA, bar, k.c * kKS, 0, t.m0 + rank * 128 + shift);
@@ -298,9 +310,8 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       const uint32_t idesc = make_idesc_f16(BN, MN ? 1 : 0);
       // K-major: rows of 128 bytes, 8 rows per swizzle atom (SBO 1024); 16 k = 32 bytes on.
       // MN-major: 64 rows of the operand (128 bytes) per k, 8 k per atom (SBO 1024), the next 64 rows LBO on; 16 k = 2048 bytes on.
-      const uint64_t d0 = make_smem_desc(0, MN ? kAPlane : 16, 1024, kSwizzle128B);
+      const uint64_t d0 = make_smem_desc(0, MN ? T::box : 16, 1024, kSwizzle128B);
       constexpr uint32_t kstep = MN ? 2048 : 32;
-      constexpr uint32_t alo = MN ? kAPlane / 2 : kAPlane, blo = MN ? kAPlane / 2 : T::bplane;
       const uint32_t base = smem_u32(sm);
       int it = 0, gi = 0;   // steps, accumulators
       bool ok = true;
@@ -308,20 +319,29 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
         const UnitAt t = unit_at<BN, MN>(g, unit);
         StepAt k = step_at<CONV>(g, t.first);
         for (int s = 0; s < t.nsteps && ok; ++s, ++it, next_step<CONV>(g, k)) {
-          const int slot = it % kStages, kk = k16_of(g, k.c);
+          const int slot = it % kStages, kk = k16_of<T::ks>(g, k.c);
           if (!(ok = wait_or_abort(fullb + slot * 8, (it / kStages) & 1, abortb))) break;
           tc_fence_after_sync();
-          const uint32_t a = base + slot * T::stage, b = a + 2 * kAPlane;
-          const uint64_t ah = d0 + (a >> 4), al = d0 + ((a + alo) >> 4), bh = d0 + (b >> 4), bl = d0 + ((b + blo) >> 4);
+          const uint32_t a = base + slot * T::stage, b = a + T::abytes;
+          const uint64_t ah = d0 + (a >> 4), bh = d0 + (b >> 4);
+          constexpr uint64_t A1 = T::aplane >> 4, B1 = T::bplane >> 4, A2 = 2 * A1, B2 = 2 * B1;   // to the further planes
           for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
             const int buf = gi % T::depth, i1 = min(kk, i0 + g.group);
             if (gi >= T::depth && !(ok = wait_or_abort(accfreeb + buf * 8, (gi / T::depth - 1) & 1, abortb))) break;
             tc_fence_after_sync();
             const uint32_t d = tmem_base + buf * BN;
+            if (MN) {   // products of 2^-16 first
+              for (int i = i0; i < i1; ++i) {
+                const uint64_t o = (uint64_t)((i * kstep) >> 4);
+                mma_f16_pair(d, ah + A2 + o, bh + o, idesc, i > i0);
+                mma_f16_pair(d, ah + o, bh + B2 + o, idesc, true);
+                mma_f16_pair(d, ah + A1 + o, bh + B1 + o, idesc, true);
+              }
+            }
             for (int i = i0; i < i1; ++i) {
               const uint64_t o = (uint64_t)((i * kstep) >> 4);
-              mma_f16_pair(d, al + o, bh + o, idesc, i > i0);
-              mma_f16_pair(d, ah + o, bl + o, idesc, true);
+              mma_f16_pair(d, ah + A1 + o, bh + o, idesc, MN || i > i0);
+              mma_f16_pair(d, ah + o, bh + B1 + o, idesc, true);
             }
             for (int i = i0; i < i1; ++i) {
               const uint64_t o = (uint64_t)((i * kstep) >> 4);
@@ -355,7 +375,7 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
             const int px = t.m0 + rank * 128 + qd * 32 + lane + tap_shift(g, k.tap);
             if (px >= 0 && px < g.M) f = exp2_int(__ldg(g.ea + px) - kRowShift);
           }
-          const int kk = k16_of(g, k.c);
+          const int kk = k16_of<T::ks>(g, k.c);
           for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
             buf = gi % T::depth;
             if (!(ok = __all_sync(0xffffffffu, wait_or_abort(accfullb + buf * 8, (gi / T::depth) & 1, abortb)))) break;
@@ -388,19 +408,21 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       bool in = true;
       if (!cut) in = row_at<CONV>(g, m, &off);
       const long ldn = cut ? kBM : g.ldn;
-      const int e = cut ? 0 : CONV ? kRowShift : in ? __ldg(g.ea + m) : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
+      const int e = cut || MN ? 0 : CONV ? kRowShift : in ? __ldg(g.ea + m) : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
       float* dst = cut ? g.partial + ((size_t)(unit - g.whole) * BN + c0) * kBM + off
                        : g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn;
       const int* eb = g.eb + n0 + (lane & 15);
-      int next = !cut && n0 + (lane & 15) < N ? __ldg(eb) : 0;
+      int next = !MN && !cut && n0 + (lane & 15) < N ? __ldg(eb) : 0;
 #pragma unroll 1
       for (int j0 = 0; j0 < NC; j0 += 16) {
         float v[16];
         tmem_ld16(taddr + buf * BN + j0, v);
         const int ebv = next, left = N - n0 - j0;
-        next = !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? __ldg(eb + j0 + 16) : 0;
+        next = !MN && !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? __ldg(eb + j0 + 16) : 0;
+        if (!MN) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
+          for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
+        }
         if (!CONV && g.vec && !cut) {   // 16-byte stores along a row
 #pragma unroll
           for (int j = 0; j < 16; j += 4)
@@ -442,7 +464,7 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
   const int m = t.m0 + threadIdx.x;
   long off;
   if (!row_at<CONV>(g, m, &off)) return;
-  const int e = CONV ? kRowShift : __ldg(g.ea + m);
+  const int e = MN ? 0 : CONV ? kRowShift : __ldg(g.ea + m);
   const int n0 = t.n0 + blockIdx.y * kJoinCols;
   const float* src = g.partial + ((size_t)blockIdx.x * g.splits * BN + blockIdx.y * kJoinCols) * kBM + threadIdx.x;
   float* dst = g.out + (size_t)t.tap * g.result + off;
@@ -454,7 +476,7 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
     for (int j = 0; j < kJoinCols; ++j) v[j] += __ldcs(src + ((size_t)q * BN + j) * kBM);
 #pragma unroll
   for (int j = 0; j < kJoinCols; ++j)
-    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = scale_by(v[j], e + __ldg(g.eb + n0 + j));
+    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + __ldg(g.eb + n0 + j));
 }
 
 // ---- operand planes -----------------------------------------------------------------------------------------------------
@@ -468,6 +490,28 @@ __device__ __forceinline__ void split4(float4 v, float sc, Half4& hi, Half4& lo)
   const float2 p = __half22float2(hi.a), q = __half22float2(hi.b);
   lo.a = __floats2half2_rn(v.x - p.x, v.y - p.y);
   lo.b = __floats2half2_rn(v.z - q.x, v.w - q.y);
+}
+// Two values as three bf16 parts each, x = p[0] + p[1] + p[2] exactly (8 + 8 + 8 bits, each part with its own exponent; the last
+// may fall below the smallest float).  A value that would round up to infinity is cut instead.
+struct Bf3 {
+  uint32_t p[3];
+};
+__device__ __forceinline__ Bf3 split3(float a, float b) {
+  Bf3 out;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    float2 f = __bfloat1622float2(h);
+    if (q == 0 && (isinf(f.x) || isinf(f.y))) {
+      if (isinf(f.x)) h.x = __float2bfloat16_rz(a);
+      if (isinf(f.y)) h.y = __float2bfloat16_rz(b);
+      f = __bfloat1622float2(h);
+    }
+    a -= f.x;
+    b -= f.y;
+    out.p[q] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return out;
 }
 __device__ __forceinline__ unsigned max4(unsigned m, float4 v) {
   return max(max(max(m, abs_bits(v.x)), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
@@ -485,11 +529,10 @@ struct SplitJob {
   int rows, segs, len, ld;   // rows of `segs` segments of `len` values, `ld` apart (columns and pixels: see the kernels)
   int ldo;                   // of a segment of the planes: a multiple of 8
   bool vec;
-  __half* hi;
+  uint16_t* hi;
   size_t plane;
   int* ex;
-  unsigned* part;            // column / channel maxima, [parts][len]
-  int per, parts;
+  int per;                   // rows of a CTA
 };
 struct SplitJobs {
   SplitJob job[2];
@@ -532,7 +575,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
   const int e = row_exponent(mx, kLeast);
   const float sc = exp2_int(-e);
   if (in && sub == 0) p.ex[row] = e;
-  __half* d = p.hi + (size_t)row * segs * p.ldo;
+  uint16_t* d = p.hi + (size_t)row * segs * p.ldo;
   auto put = [&](int i, float4 x) {
     const int seg = segs == 1 ? 0 : i / quads;
     const size_t o = (size_t)seg * p.ldo + (i - seg * quads) * 4;
@@ -547,114 +590,33 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
   for (int i = Q * tpr + sub; i < n; i += tpr) put(i, at(i));
 }
 
-// [rows][len] with one exponent per column, in two launches: the largest magnitude per column and range of rows, then the
-// planes.  Block (64, 4): 256 columns, every fourth row.
-__global__ void __launch_bounds__(256) column_max_kernel(const __grid_constant__ SplitJobs jobs) {
-  __shared__ uint4 red[4][64];
+// [rows][len] as three bf16 planes.  Block (64, 4): 256 columns, every fourth row of a range.
+__global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constant__ SplitJobs jobs) {
   grid_dependency_wait();
   const bool second = (int)blockIdx.x >= jobs.first;
   const SplitJob& p = jobs.job[second];
   const int cols = p.len, c = (blockIdx.x - (second ? jobs.first : 0)) * 256 + threadIdx.x * 4;
   const int r0 = blockIdx.y * p.per, r1 = min(p.rows, r0 + p.per);
-  uint4 m = make_uint4(0, 0, 0, 0);
-  if (c < cols)
-#pragma unroll 8
-    for (int r = r0 + threadIdx.y; r < r1; r += 4) {
-      const float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
-      m.x = max(m.x, abs_bits(v.x)); m.y = max(m.y, abs_bits(v.y));
-      m.z = max(m.z, abs_bits(v.z)); m.w = max(m.w, abs_bits(v.w));
-    }
-  red[threadIdx.y][threadIdx.x] = m;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < cols && r0 < r1) {
-#pragma unroll
-    for (int i = 1; i < 4; ++i) {
-      const uint4 o = red[i][threadIdx.x];
-      m.x = max(m.x, o.x); m.y = max(m.y, o.y); m.z = max(m.z, o.z); m.w = max(m.w, o.w);
-    }
-    unsigned* d = p.part + (size_t)blockIdx.y * cols + c;
-    d[0] = m.x;
-    if (c + 1 < cols) d[1] = m.y;
-    if (c + 2 < cols) d[2] = m.z;
-    if (c + 3 < cols) d[3] = m.w;
-  }
-}
-__global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constant__ SplitJobs jobs) {
-  __shared__ float scale[256];
-  grid_dependency_wait();
-  const bool second = (int)blockIdx.x >= jobs.first;
-  const SplitJob& p = jobs.job[second];
-  const int cols = p.len, c0 = (blockIdx.x - (second ? jobs.first : 0)) * 256;
-  const int r0 = blockIdx.y * p.per, r1 = min(p.rows, r0 + p.per);
-  {
-    const int i = threadIdx.y * 64 + threadIdx.x, c = c0 + i;
-    unsigned m = 0;
-    if (c < cols)
-#pragma unroll 8
-      for (int q = 0; q < p.parts; ++q) m = max(m, __ldcg(p.part + (size_t)q * cols + c));
-    const int e = row_exponent(m, kLeast);
-    scale[i] = exp2_int(-e);
-    if (blockIdx.y == 0 && c < cols) p.ex[c] = e;
-  }
-  __syncthreads();
-  const int c = c0 + threadIdx.x * 4;
   if (c >= cols) return;
-  const float4 sc = *reinterpret_cast<const float4*>(scale + threadIdx.x * 4);
 #pragma unroll 4
   for (int r = r0 + threadIdx.y; r < r1; r += 4) {
-    float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
-    v.x *= sc.x; v.y *= sc.y; v.z *= sc.z; v.w *= sc.w;
-    Half4 h, l;
-    split4(v, 1.f, h, l);
-    __half* d = p.hi + (size_t)r * p.ldo + c;
-    *reinterpret_cast<Half4*>(d) = h;
-    *reinterpret_cast<Half4*>(d + p.plane) = l;
+    const float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
+    const Bf3 x = split3(v.x, v.y), y = split3(v.z, v.w);
+    uint16_t* d = p.hi + (size_t)r * p.ldo + c;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(d + q * p.plane) = make_uint2(x.p[q], y.p[q]);
   }
 }
 
 // NCHW -> [n][pixel][channel] planes with padW zero pixels after each row and padH zero rows after each image: what a filter
 // tap reads beside an image is then the end of the row or image before, and a tap is a shift of the row index, which TMA
-// takes at any value (only the contiguous coordinate has an alignment rule).  Exponents per channel, from the maxima of
-// ranges of images, or per pixel.  In a job: len = channels, rows = N (H + padH) (W + padW).
+// takes at any value (only the contiguous coordinate has an alignment rule).  Fp16 planes with an exponent per pixel, or
+// (THREE) bf16 planes.  In a job: len = channels, rows = N (H + padH) (W + padW).
 struct Images {
   int N, H, W, padH, padW;
 };
-__global__ void __launch_bounds__(256) channel_max_kernel(const __grid_constant__ SplitJobs jobs, const Images im) {
-  __shared__ unsigned red[8];
-  grid_dependency_wait();
-  const bool second = (int)blockIdx.x >= jobs.first;
-  const SplitJob& p = jobs.job[second];
-  const int c = blockIdx.x - (second ? jobs.first : 0), tid = threadIdx.x, HW = im.H * im.W;
-  const int n0 = blockIdx.y * p.per, n1 = min(im.N, n0 + p.per);
-  if (n0 >= n1) return;
-  const float* src = p.src + ((size_t)n0 * p.len + c) * HW;
-  const size_t image = (size_t)p.len * HW;
-  unsigned m = 0;
-  // (image, pixel) pairs in one loop, so that a thread's loads do not end with an image
-  if (p.vec) {
-    const int q = HW / 4;
-#pragma unroll 4
-    for (int i = tid; i < (n1 - n0) * q; i += 256) {
-      const int n = i / q;
-      m = max4(m, __ldg(reinterpret_cast<const float4*>(src + n * image) + i - n * q));
-    }
-  } else {
-#pragma unroll 8
-    for (int i = tid; i < (n1 - n0) * HW; i += 256) {
-      const int n = i / HW;
-      m = max(m, abs_bits(__ldg(src + n * image + i - n * HW)));
-    }
-  }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((tid & 31) == 0) red[tid >> 5] = m;
-  __syncthreads();
-  if (tid == 0) {
-#pragma unroll
-    for (int i = 1; i < 8; ++i) m = max(m, red[i]);
-    p.part[(size_t)blockIdx.y * p.len + c] = m;
-  }
-}
 constexpr int kPxTile = 32, kPxPitch = kPxTile + 1;
+template <bool THREE>
 __global__ void __launch_bounds__(256) split_pixels_kernel(const __grid_constant__ SplitJobs jobs, const Images im) {
   extern __shared__ float px_smem[];
   __shared__ unsigned red[8][kPxTile];
@@ -662,7 +624,7 @@ __global__ void __launch_bounds__(256) split_pixels_kernel(const __grid_constant
   const SplitJob& job = jobs.job[second];
   const int CH = job.len, HW = im.H * im.W;
   float* tile = px_smem;                                  // [CH][kPxPitch]
-  float* scale = tile + CH * kPxPitch;                    // [CH] or [kPxTile]
+  float* scale = tile + CH * kPxPitch;                    // [kPxTile]
   const int Wp = im.W + im.padW, PP = (im.H + im.padH) * Wp, rows = job.rows;
   const int p0 = (blockIdx.x - (second ? jobs.first : 0)) * kPxTile, tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
   grid_dependency_wait();
@@ -679,17 +641,8 @@ __global__ void __launch_bounds__(256) split_pixels_kernel(const __grid_constant
     }
     red[ty][tx] = m;
   }
-  if (job.part) {
-    for (int c = tid; c < CH; c += 256) {
-      unsigned m = 0;
-      for (int i = 0; i < job.parts; ++i) m = max(m, __ldcg(job.part + (size_t)i * CH + c));
-      const int e = row_exponent(m, kLeast);
-      scale[c] = exp2_int(-e);
-      if (p0 == 0) job.ex[c] = e;
-    }
-  }
   __syncthreads();
-  if (!job.part) {
+  if (!THREE) {
     if (tid < kPxTile) {
       unsigned m = red[0][tid];
 #pragma unroll
@@ -702,17 +655,22 @@ __global__ void __launch_bounds__(256) split_pixels_kernel(const __grid_constant
   }
   // a warp writes the channels of a pixel, two per lane
   for (int i = ty; i < kPxTile && p0 + i < rows; i += 8) {
-    __half* d = job.hi + (size_t)(p0 + i) * job.ldo;
+    uint16_t* d = job.hi + (size_t)(p0 + i) * job.ldo;
 #pragma unroll 4
     for (int c = tx * 2; c < CH; c += 64) {
-      const bool two = c + 1 < CH;
-      float a = tile[c * kPxPitch + i], b = two ? tile[(c + 1) * kPxPitch + i] : 0.f;
-      a *= job.part ? scale[c] : scale[i];
-      if (two) b *= job.part ? scale[c + 1] : scale[i];
-      const __half2 h = __floats2half2_rn(a, b);
-      const float2 f = __half22float2(h);
-      *reinterpret_cast<__half2*>(d + c) = h;
-      *reinterpret_cast<__half2*>(d + job.plane + c) = __floats2half2_rn(a - f.x, b - f.y);
+      float a = tile[c * kPxPitch + i], b = c + 1 < CH ? tile[(c + 1) * kPxPitch + i] : 0.f;
+      if (THREE) {
+        const Bf3 x = split3(a, b);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint32_t*>(d + q * job.plane + c) = x.p[q];
+      } else {
+        a *= scale[i];
+        b *= scale[i];
+        const __half2 h = __floats2half2_rn(a, b);
+        const float2 f = __half22float2(h);
+        *reinterpret_cast<__half2*>(d + c) = h;
+        *reinterpret_cast<__half2*>(d + job.plane + c) = __floats2half2_rn(a - f.x, b - f.y);
+      }
     }
   }
 }
@@ -726,46 +684,39 @@ int gemm_tc_mode() {
 }
 namespace {
 
-// fp16 tensor of two planes: dimensions from the contiguous one outwards, strides in elements
-int encode_planes(CUtensorMap* map, const __half* base, const size_t (&dim)[3], const size_t (&stride)[2], size_t plane,
+// tensor of all planes: dimensions from the contiguous one outwards, strides in elements
+int encode_planes(CUtensorMap* map, const uint16_t* base, int planes, const size_t (&dim)[3], const size_t (&stride)[2], size_t plane,
                   const unsigned (&box)[3]) {
   PFN_encodeTiled enc = get_encode_tiled();
   if (!enc) return fail(B200CP_ERR_NO_DEVICE, "cuTensorMapEncodeTiled entry point not available");
-  const cuuint64_t gdim[4] = {dim[0], dim[1], dim[2], 2};
+  const cuuint64_t gdim[4] = {dim[0], dim[1], dim[2], (cuuint64_t)planes};
   const cuuint64_t gstr[3] = {stride[0] * 2, stride[1] * 2, plane * 2};
-  const cuuint32_t bx[4] = {box[0], box[1], box[2], 2}, estr[4] = {1, 1, 1, 1};
-  const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half*>(base), gdim, gstr, bx, estr,
+  const cuuint32_t bx[4] = {box[0], box[1], box[2], (cuuint32_t)planes}, estr[4] = {1, 1, 1, 1};
+  const CUresult cr = enc(map, planes == 3 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<uint16_t*>(base), gdim, gstr, bx, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (cr != CUDA_SUCCESS) return fail(B200CP_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
   return B200CP_OK;
 }
 
-// hi / lo planes of one operand and its exponents in the scratch
+// planes of one operand in the scratch: fp16 hi / lo with exponents, or three of bf16
 struct Planes {
-  __half* hi;
+  uint16_t* hi;
   int* ex;
-  unsigned* part;       // column / channel maxima
   size_t rows, plane;   // plane: values of one plane
   int ld;
 };
-constexpr int kMaxParts = 64;
-size_t planes_floats(size_t rows, size_t ld, size_t exps, bool columns) {
-  return align_up(rows * ld, 64) + align_up(exps, 64) + (columns ? align_up(exps * kMaxParts, 64) : 0);
+size_t pair_floats(size_t rows, size_t ld, size_t exps) { return align_up(rows * ld, 64) + align_up(exps, 64); }
+size_t triple_floats(size_t rows, size_t ld) { return align_up(rows * ld / 2 * 3, 64); }   // (ld is even)
+Planes take_pair(float*& at, size_t rows, size_t ld, size_t exps) {
+  Planes p{reinterpret_cast<uint16_t*>(at), nullptr, rows, rows * ld, (int)ld};
+  p.ex = reinterpret_cast<int*>(at + align_up(rows * ld, 64));
+  at += pair_floats(rows, ld, exps);
+  return p;
 }
-Planes take_planes(float*& at, size_t rows, size_t ld, size_t exps, bool columns) {
-  Planes p{};
-  p.hi = reinterpret_cast<__half*>(at);
-  p.rows = rows;
-  p.ld = (int)ld;
-  p.plane = rows * ld;
-  at += align_up(rows * ld, 64);     // two planes of 2-byte values: rows * ld floats
-  p.ex = reinterpret_cast<int*>(at);
-  at += align_up(exps, 64);
-  if (columns) {
-    p.part = reinterpret_cast<unsigned*>(at);
-    at += align_up(exps * kMaxParts, 64);
-  }
+Planes take_triple(float*& at, size_t rows, size_t ld) {
+  const Planes p{reinterpret_cast<uint16_t*>(at), nullptr, rows, rows * ld, (int)ld};
+  at += triple_floats(rows, ld);
   return p;
 }
 int ld8(int n) { return (n + 7) / 8 * 8; }
@@ -774,7 +725,7 @@ int ld8(int n) { return (n + 7) / 8 * 8; }
 SplitJob job_of(const float* src, int rows, int segs, int len, int ld, const Planes& p) {
   SplitJob j{};
   j.src = src; j.rows = rows; j.segs = segs; j.len = len; j.ld = ld;
-  j.ldo = p.ld; j.hi = p.hi; j.plane = p.plane; j.ex = p.ex; j.part = p.part;
+  j.ldo = p.ld; j.hi = p.hi; j.plane = p.plane; j.ex = p.ex;
   j.vec = ld % 4 == 0 && !(reinterpret_cast<uintptr_t>(src) & 15);
   return j;
 }
@@ -786,38 +737,24 @@ int split_rows(const SplitJob& a, const SplitJob& b, cudaStream_t st) {
   return B200CP_OK;
 }
 int split_columns(SplitJob a, SplitJob b, cudaStream_t st) {   // of the same number of rows
-  a.per = b.per = std::max(16, ceil_div(a.rows, kMaxParts));
-  a.parts = b.parts = ceil_div(a.rows, a.per);
+  a.per = b.per = std::max(16, ceil_div(a.rows, 64));
   SplitJobs jobs{{a, b}, ceil_div(a.len, 256)};
-  const dim3 grid(jobs.first + ceil_div(b.len, 256), a.parts), block(64, 4);
-  B200CP_CUDA_OK(launch_kernel(column_max_kernel, grid, block, 0, st, true, jobs));
-  B200CP_LAUNCH_OK("column_max_kernel");
-  B200CP_CUDA_OK(launch_kernel(split_columns_kernel, grid, block, 0, st, true, jobs));
+  B200CP_CUDA_OK(launch_kernel(split_columns_kernel, dim3(jobs.first + ceil_div(b.len, 256), ceil_div(a.rows, a.per)), dim3(64, 4), 0,
+                               st, true, jobs));
   B200CP_LAUNCH_OK("split_columns_kernel");
   return B200CP_OK;
 }
 constexpr int kMostChannels = 1024;   // of split_pixels_kernel's tile: 139 KB
-// the pixel planes of one tensor, or (with `part`) the planes with exponents per channel of two
-int split_pixels(SplitJob a, SplitJob b, int count, const Images& im, const DeviceInfo& di, cudaStream_t st) {
-  SplitJobs jobs{{a, b}, a.len};
-  if (a.part) {
-    const int channels = a.len + (count == 2 ? b.len : 0);
-    const int per = std::max(1, ceil_div(im.N, std::min(kMaxParts, std::max(1, 16 * di.sm_count / channels))));
-    for (SplitJob& j : jobs.job) {
-      j.per = per;
-      j.parts = ceil_div(im.N, per);
-      j.vec = im.H * im.W % 4 == 0 && !(reinterpret_cast<uintptr_t>(j.src) & 15);
-    }
-    B200CP_CUDA_OK(launch_kernel(channel_max_kernel, dim3(channels, jobs.job[0].parts), dim3(256), 0, st, true, jobs, im));
-    B200CP_LAUNCH_OK("channel_max_kernel");
-  }
-  jobs.first = ceil_div(a.rows, kPxTile);
-  const int most = count == 2 ? std::max(a.len, b.len) : a.len;
-  const size_t smem = sizeof(float) * ((size_t)most * kPxPitch + std::max(most, kPxTile));
+// the fp16 planes of one tensor, or (THREE) the bf16 planes of two
+template <bool THREE>
+int split_pixels(const SplitJob& a, const SplitJob& b, const Images& im, cudaStream_t st) {
+  const SplitJobs jobs{{a, b}, ceil_div(a.rows, kPxTile)};
+  const int most = std::max(a.len, b.len);
+  const size_t smem = sizeof(float) * ((size_t)most * kPxPitch + kPxTile);
   static std::atomic<int> set[64];
-  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_pixels_kernel), set, (int)smem));
-  B200CP_CUDA_OK(launch_kernel(split_pixels_kernel, dim3(jobs.first + (count == 2 ? ceil_div(b.rows, kPxTile) : 0)), dim3(32, 8),
-                               smem, st, true, jobs, im));
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_pixels_kernel<THREE>), set, (int)smem));
+  B200CP_CUDA_OK(launch_kernel(split_pixels_kernel<THREE>, dim3(jobs.first + ceil_div(b.rows, kPxTile)), dim3(32, 8), smem, st, true, jobs,
+                               im));
   B200CP_LAUNCH_OK("split_pixels_kernel");
   return B200CP_OK;
 }
@@ -831,7 +768,7 @@ struct TcTiles {
   int bn, tiles_m, tiles_n, whole, splits, steps, cut;   // cut: tiles that are cut
   double us;
 };
-// Measured us of a step (64 k) and of a unit beside its steps.  128 and 64 columns are not in proportion: the rows of A are read
+// Measured us of a step (twelve instructions: 64 k, MN-major 32) and of a unit beside its steps.  128 and 64 columns are not in proportion: the rows of A are read
 // from shared memory once per instruction, whatever its width.
 double step_us(int bn) { return bn == 256 ? 1.35 : bn == 128 ? 0.95 : 0.7; }
 constexpr double kUnitUs = 2.0;
@@ -864,10 +801,10 @@ size_t partial_floats(const TcTiles& t) { return t.splits > 1 ? (size_t)t.cut * 
 template <int BN, bool MN, bool CONV>
 int launch_tile(const SplitGemm& g, int cut, const CUtensorMap& a, const CUtensorMap& b, const DeviceInfo& di, cudaStream_t st) {
   static std::atomic<int> set[64];
-  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_gemm_kernel<BN, MN, CONV>), set, (int)Tile<BN>::smem));
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_gemm_kernel<BN, MN, CONV>), set, (int)Tile<BN, MN>::smem));
   const int pairs = std::min(g.units, di.sm_count / 2);
-  B200CP_CUDA_OK(launch_kernel(split_gemm_kernel<BN, MN, CONV>, dim3(2 * pairs), dim3(Tile<BN>::threads), Tile<BN>::smem, st, true,
-                               g, a, b));
+  B200CP_CUDA_OK(launch_kernel(split_gemm_kernel<BN, MN, CONV>, dim3(2 * pairs), dim3(Tile<BN, MN>::threads),
+                               Tile<BN, MN>::smem, st, true, g, a, b));
   B200CP_LAUNCH_OK("split_gemm_kernel");
   if (g.splits > 1) {
     B200CP_CUDA_OK(launch_kernel(join_tiles_kernel<BN, MN, CONV>, dim3(cut, BN / kJoinCols), dim3(kBM), 0, st, true, g));
@@ -880,7 +817,7 @@ int run_split_gemm(SplitGemm g, const TcTiles& t, size_t result, bool mn, bool c
                    float* out, float* partial, const DeviceInfo& di, cudaStream_t st) {
   g.tiles_m = t.tiles_m; g.tiles_n = t.tiles_n; g.whole = t.whole; g.splits = t.splits; g.steps = t.steps;
   g.units = t.whole + t.cut * t.splits;
-  g.group = g.total <= kShortSum ? 2 : 4;
+  g.group = mn || g.total <= kShortSum ? 2 : 4;
   g.result = result;
   g.out = out;
   g.partial = partial;
@@ -896,7 +833,11 @@ int run_split_gemm(SplitGemm g, const TcTiles& t, size_t result, bool mn, bool c
 // ---- gradient products: both operands have the batch (or pixels) as rows -------------------------------------------------
 // G[M][N] = A^T B with A [K][M], B [K][N]: rows of the kernel's result are the N columns of G, which are contiguous.
 namespace {
-TcTiles grad_tiles(int K, int M, int N, const DeviceInfo& di) { return tc_tiles(N, M, ceil_div(K, kKS), 1, true, di); }
+TcTiles grad_tiles(int K, int M, int N, const DeviceInfo& di) { return tc_tiles(N, M, ceil_div(K, kGradKS), 1, true, di); }
+// planes of an operand with K rows of n values
+int encode_rows(CUtensorMap* map, const Planes& p, int n, size_t K) {
+  return encode_planes(map, p.hi, 3, {(size_t)n, K, 1}, {(size_t)p.ld, p.plane}, p.plane, {64, kGradKS, 1});
+}
 }  // namespace
 
 bool gemm_tc_supported(int K, int M, int N) {
@@ -907,24 +848,22 @@ bool gemm_tc_supported(int K, int M, int N) {
 size_t gemm_tc_scratch_floats(int K, int M, int N) {
   DeviceInfo di;
   if (device_info(&di)) di.sm_count = 148;
-  return planes_floats(K, ld8(M), M, true) + planes_floats(K, ld8(N), N, true) +
-         partial_floats(grad_tiles(K, M, N, di));
+  return triple_floats(K, ld8(M)) + triple_floats(K, ld8(N)) + partial_floats(grad_tiles(K, M, N, di));
 }
 
 int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   float* at = scratch;
-  const Planes pn = take_planes(at, K, ld8(N), N, true), pm = take_planes(at, K, ld8(M), M, true);
+  const Planes pn = take_triple(at, K, ld8(N)), pm = take_triple(at, K, ld8(M));
   if (int rc = split_columns(job_of(B, K, 1, N, N, pn), job_of(A, K, 1, M, M, pm), st)) return rc;
   CUtensorMap mn, mm;
-  if (int rc = encode_planes(&mn, pn.hi, {(size_t)N, (size_t)K, 1}, {(size_t)pn.ld, pn.plane}, pn.plane, {64, 64, 1})) return rc;
-  if (int rc = encode_planes(&mm, pm.hi, {(size_t)M, (size_t)K, 1}, {(size_t)pm.ld, pm.plane}, pm.plane, {64, 64, 1})) return rc;
+  if (int rc = encode_rows(&mn, pn, N, K)) return rc;
+  if (int rc = encode_rows(&mm, pm, M, K)) return rc;
   const TcTiles t = grad_tiles(K, M, N, di);
   SplitGemm g{};
-  g.M = N; g.N = M; g.total = ceil_div(K, kKS); g.kc = g.total; g.Kc = K;
+  g.M = N; g.N = M; g.total = ceil_div(K, kGradKS); g.kc = g.total; g.Kc = K;
   g.FW = 1;
-  g.ea = pn.ex; g.eb = pm.ex;
   g.ldm = 1; g.ldn = N;
   return run_split_gemm(g, t, (size_t)M * N, true, false, mn, mm, G, at, di, st);
 }
@@ -946,7 +885,7 @@ bool grad_conv(GradConv& p, int N, int T, int C, int H, int W, int FH, int FW) {
   if (p.K > 0x3fffff00L || (mode == 1 && (p.K < 1024 || T < 128 || C < 128))) return false;
   DeviceInfo di;
   if (device_info(&di)) di.sm_count = 148;
-  p.t = tc_tiles(C, T, (int)((p.K + kKS - 1) / kKS), p.taps, true, di);
+  p.t = tc_tiles(C, T, (int)((p.K + kGradKS - 1) / kGradKS), p.taps, true, di);
   return get_encode_tiled() != nullptr;
 }
 }  // namespace
@@ -959,7 +898,7 @@ bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW) {
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW) {
   GradConv p;
   if (!grad_conv(p, N, T, C, H, W, FH, FW)) return 0;
-  return planes_floats(p.K, ld8(C), C, true) + planes_floats(p.K, ld8(T), T, true) + partial_floats(p.t);
+  return triple_floats(p.K, ld8(C)) + triple_floats(p.K, ld8(T)) + partial_floats(p.t);
 }
 
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
@@ -970,16 +909,15 @@ int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const
   if (int rc = device_info(&di)) return rc;
   const int padH = (FH - 1) / 2, padW = (FW - 1) / 2;
   float* at = scratch;
-  const Planes px = take_planes(at, p.K, ld8(C), C, true), pv = take_planes(at, p.K, ld8(T), T, true);
-  if (int rc = split_pixels(job_of(X, (int)p.K, 1, C, 0, px), job_of(dV, (int)p.K, 1, T, 0, pv), 2, Images{N, H, W, padH, padW}, di, st))
+  const Planes px = take_triple(at, p.K, ld8(C)), pv = take_triple(at, p.K, ld8(T));
+  if (int rc = split_pixels<true>(job_of(X, (int)p.K, 1, C, 0, px), job_of(dV, (int)p.K, 1, T, 0, pv), Images{N, H, W, padH, padW}, st))
     return rc;
   CUtensorMap mx, mv;
-  if (int rc = encode_planes(&mx, px.hi, {(size_t)C, (size_t)p.K, 1}, {(size_t)px.ld, px.plane}, px.plane, {64, 64, 1})) return rc;
-  if (int rc = encode_planes(&mv, pv.hi, {(size_t)T, (size_t)p.K, 1}, {(size_t)pv.ld, pv.plane}, pv.plane, {64, 64, 1})) return rc;
+  if (int rc = encode_rows(&mx, px, C, p.K)) return rc;
+  if (int rc = encode_rows(&mv, pv, T, p.K)) return rc;
   SplitGemm g{};
-  g.M = C; g.N = T; g.total = ceil_div((int)p.K, kKS); g.kc = g.total; g.Kc = (int)p.K;
+  g.M = C; g.N = T; g.total = ceil_div((int)p.K, kGradKS); g.kc = g.total; g.Kc = (int)p.K;
   g.FW = FW; g.padH = padH; g.padW = padW; g.Wp = W + padW;
-  g.ea = px.ex; g.eb = pv.ex;
   g.ldm = 1; g.ldn = C;
   return run_split_gemm(g, p.t, (size_t)T * C, true, false, mx, mv, G, at, di, st);
 }
@@ -1017,7 +955,7 @@ size_t dense_tc_scratch_floats(int B, int K, int N, const KronWeight& w) {
   DeviceInfo di;
   if (device_info(&di)) return 0;
   return (kron_planes_takes(w.order, w.idims, w.odims, w.R, di.sm_count) ? 0 : align_up((size_t)N * kron_weight_ld(K), 64)) +
-         planes_floats(N, ld8(K), N, false) + planes_floats(B, ld8(K), B, false) + partial_floats(dense_tc(B, K, N, di).t);
+         pair_floats(N, ld8(K), N) + pair_floats(B, ld8(K), B) + partial_floats(dense_tc(B, K, N, di).t);
 }
 
 int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, float* Y, float* scratch, cudaStream_t st) {
@@ -1027,7 +965,7 @@ int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, fl
   const bool direct = kron_planes_takes(w.order, w.idims, w.odims, w.R, di.sm_count);
   float *at = scratch, *W = scratch;
   if (!direct) at += align_up((size_t)N * kron_weight_ld(K), 64);
-  const Planes pw = take_planes(at, N, ld8(K), N, false), px = take_planes(at, B, ld8(K), B, false);
+  const Planes pw = take_pair(at, N, ld8(K), N), px = take_pair(at, B, ld8(K), B);
   if (direct) {
     if (int rc = kron_planes_launch(w.order, w.idims, w.odims, w.R, w.F, w.transposed, pw.ld, pw.hi, pw.plane, pw.ex, st)) return rc;
     if (int rc = split_rows(job_of(X, B, 1, K, K, px), SplitJob{}, st)) return rc;
@@ -1037,8 +975,8 @@ int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, fl
   }
   const Planes &pa = d.rows_are_batch ? px : pw, &pb = d.rows_are_batch ? pw : px;
   CUtensorMap ma, mb;
-  if (int rc = encode_planes(&ma, pa.hi, {(size_t)K, 1, pa.rows}, {(size_t)pa.ld, (size_t)pa.ld}, pa.plane, {64, 1, 128})) return rc;
-  if (int rc = encode_planes(&mb, pb.hi, {(size_t)K, 1, pb.rows}, {(size_t)pb.ld, (size_t)pb.ld}, pb.plane,
+  if (int rc = encode_planes(&ma, pa.hi, 2, {(size_t)K, 1, pa.rows}, {(size_t)pa.ld, (size_t)pa.ld}, pa.plane, {64, 1, 128})) return rc;
+  if (int rc = encode_planes(&mb, pb.hi, 2, {(size_t)K, 1, pb.rows}, {(size_t)pb.ld, (size_t)pb.ld}, pb.plane,
                              {64, 1, (unsigned)d.t.bn / 2})) return rc;
   SplitGemm g{};
   g.M = (int)pa.rows; g.N = (int)pb.rows; g.total = ceil_div(K, kKS); g.kc = g.total; g.Kc = K;
@@ -1073,7 +1011,7 @@ size_t conv_tc_scratch_floats(int N, int C, int T, int H, int W) {
   DeviceInfo di;
   if (device_info(&di)) return 0;
   const size_t px = (size_t)N * (H + kPad) * (W + kPad);
-  return align_up((size_t)T * kTaps * kron_weight_ld(C), 64) + planes_floats(T, (size_t)kTaps * ld8(C), T, false) + planes_floats(px, ld8(C), px, false) +
+  return align_up((size_t)T * kTaps * kron_weight_ld(C), 64) + pair_floats(T, (size_t)kTaps * ld8(C), T) + pair_floats(px, ld8(C), px) +
          partial_floats(conv_tc(N, C, T, H, W, di));
 }
 
@@ -1087,14 +1025,14 @@ int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const Kron
   const int ldw = kron_weight_ld(C);
   float *Wt = scratch, *at = scratch + align_up((size_t)T * kTaps * ldw, 64);
   if (int rc = kron_weight_launch(w.order, w.idims, w.odims, w.R, w.F, w.S, kTaps, w.transposed, w.flip, Wt, st)) return rc;
-  Planes pw = take_planes(at, T, kTaps * ldk, T, false), pa = take_planes(at, px, ldk, px, false);
+  Planes pw = take_pair(at, T, kTaps * ldk, T), pa = take_pair(at, px, ldk, px);
   pw.ld = (int)ldk;
   const SplitJob none{};
   if (int rc = split_rows(job_of(Wt, T, kTaps, C, ldw, pw), none, st)) return rc;
-  if (int rc = split_pixels(job_of(X, (int)px, 1, C, 0, pa), none, 1, Images{N, H, W, kPad, kPad}, di, st)) return rc;
+  if (int rc = split_pixels<false>(job_of(X, (int)px, 1, C, 0, pa), none, Images{N, H, W, kPad, kPad}, st)) return rc;
   CUtensorMap ma, mb;
-  if (int rc = encode_planes(&ma, pa.hi, {(size_t)C, 1, px}, {ldk, ldk}, pa.plane, {64, 1, 128})) return rc;
-  if (int rc = encode_planes(&mb, pw.hi, {(size_t)C, kTaps, (size_t)T}, {ldk, kTaps * ldk}, pw.plane, {64, 1, (unsigned)t.bn / 2}))
+  if (int rc = encode_planes(&ma, pa.hi, 2, {(size_t)C, 1, px}, {ldk, ldk}, pa.plane, {64, 1, 128})) return rc;
+  if (int rc = encode_planes(&mb, pw.hi, 2, {(size_t)C, kTaps, (size_t)T}, {ldk, kTaps * ldk}, pw.plane, {64, 1, (unsigned)t.bn / 2}))
     return rc;
   SplitGemm g{};
   g.M = (int)px; g.N = T; g.kc = ceil_div(C, kKS); g.total = kTaps * g.kc; g.Kc = C;

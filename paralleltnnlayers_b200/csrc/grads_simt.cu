@@ -263,7 +263,7 @@ int dense_grad_launch(int N, int T, int C, int H, int W, int FH, int FW, const f
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   const int taps = FH * FW;
-  // large products go to the tensor cores (the scratch then holds the operands' hi / lo planes)
+  // large products go to the tensor cores (the scratch then holds the operands' planes)
   if (scratch) {
     float* planes = reinterpret_cast<float*>(align_up(reinterpret_cast<uintptr_t>(scratch), kPlaneAlign));
     if (H * W == 1 && taps == 1 && gemm_tc_supported(N, T, C)) return gemm_tc_launch(N, T, C, dV, X, G, planes, st);

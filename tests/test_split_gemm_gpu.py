@@ -1,10 +1,11 @@
-"""The tensor-core products of the dense and reshaped-CP layers (scaled fp16 hi / lo operands) at the edges of their tiles:
-256 x 256 / 128 / 64 results, K steps of 64 in instructions of 16, odd row lengths, operands off the 16-byte grid, rows of very
+"""The tensor-core products of the dense and reshaped-CP layers (scaled fp16 hi / lo operands, in the gradients three bf16 parts) at the
+edges of their tiles: 256 x 256 / 128 / 64 results, K steps of 64 (gradients: 32) in instructions of 16, odd row lengths, operands off the 16-byte grid, rows of very
 different magnitude.  B200CP_GEMM_TC=2 takes them at every size.
 
 Bound: a product of two 22-bit operands without the product of their low parts is off by at most 2**-21; an accumulator of
 n <= 4 instructions is cut off by at most n * 2**-23 of its partial sums, and the totals round by 2**-24 each.  In the norm over a
-result, with random signs, that is 2.5e-7 (measured: 1.0 to 2.5e-7); the weight's own fp32 sum adds 1e-7."""
+result, with random signs, that is 2.5e-7 (measured: 1.0 to 2.5e-7); the weight's own fp32 sum adds 1e-7.  The six products of
+three bf16 parts leave out 3 * 2**-24 of a term."""
 import math
 
 import pytest
@@ -151,3 +152,46 @@ def test_under_capture_and_on_another_stream():
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, P.dense_cp(x, *F))
+
+
+@pytest.mark.parametrize("size", [1e6, 1e9, 1e20])
+@pytest.mark.parametrize("where", ["input", "gradient"])
+def test_dense_gradients_beside_a_large_sample(size, where):
+    """A sample whose gradient (or input) is zero adds nothing to the factor gradients, however large its input (gradient): every
+    value of both operands keeps its own exponent."""
+    import paralleltnnlayers_b200 as P
+    normal = _normal(7)
+    x, dy = normal(500, 144), normal(500, 160)
+    big, none = (x, dy) if where == "input" else (dy, x)
+    big[7] *= size
+    none[7] = 0
+    big[300, 3], none[300] = size, 0   # one value of a sample
+    F = [normal(i, o, 9) * 0.35 for i, o in ((12, 16), (12, 10))]
+    leaves = [f.double().requires_grad_() for f in F]
+    ref = torch.autograd.grad(x.double() @ _kron(leaves).sum(-1), leaves, dy.double())
+    for got, want in zip(P.dense_cp_backward(x, dy, *F)[1], ref):
+        assert _rel(got, want) < 1e-6
+    P.device_status()
+
+
+@pytest.mark.parametrize("size", [1e6, 1e9, 1e20])
+@pytest.mark.parametrize("where", ["input", "gradient"])
+def test_rcp_gradients_beside_a_large_sample(size, where):
+    """The same for a convolution: an image, and a pixel with zeros wherever a tap reaches."""
+    import paralleltnnlayers_b200 as P
+    normal = _normal(8)
+    x, dy = normal(3, 144, 10, 12), normal(3, 160, 10, 12)
+    big, none = (x, dy) if where == "input" else (dy, x)
+    big[1] *= size
+    none[1] = 0
+    big[0, :, 4, 5] *= size
+    none[0, :, 3:6, 4:7] = 0
+    A, S = [normal(i, o, 9) * 0.3 for i, o in ((12, 16), (12, 10))], normal(3, 3, 9) * 0.3
+    leaves = [t.double().requires_grad_() for t in (*A, S)]
+    K = torch.einsum("ctr,yxr->tcyx", _kron(leaves[:2]), leaves[2])
+    y = torch.nn.functional.conv2d(x.double().cpu(), K.cpu(), padding=1)
+    ref = torch.autograd.grad(y, leaves, dy.double().cpu())
+    _, dA, dS = P.rcp_conv2d_backward(x, dy, *A, S)
+    for got, want in zip((*dA, dS), ref):
+        assert _rel(got, want) < 1e-6
+    P.device_status()
