@@ -373,7 +373,7 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
           float f = 0.f;
           if (CONV) {
             const int px = t.m0 + rank * 128 + qd * 32 + lane + tap_shift(g, k.tap);
-            if (px >= 0 && px < g.M) f = exp2_int(__ldg(g.ea + px) - kRowShift);
+            if (px >= 0 && px < g.M) f = exp2_int(g.ea[px] - kRowShift);
           }
           const int kk = k16_of<T::ks>(g, k.c);
           for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
@@ -408,17 +408,17 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       bool in = true;
       if (!cut) in = row_at<CONV>(g, m, &off);
       const long ldn = cut ? kBM : g.ldn;
-      const int e = cut || MN ? 0 : CONV ? kRowShift : in ? __ldg(g.ea + m) : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
+      const int e = cut || MN ? 0 : CONV ? kRowShift : in ? g.ea[m] : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
       float* dst = cut ? g.partial + ((size_t)(unit - g.whole) * BN + c0) * kBM + off
                        : g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn;
       const int* eb = g.eb + n0 + (lane & 15);
-      int next = !MN && !cut && n0 + (lane & 15) < N ? __ldg(eb) : 0;
+      int next = !MN && !cut && n0 + (lane & 15) < N ? *eb : 0;
 #pragma unroll 1
       for (int j0 = 0; j0 < NC; j0 += 16) {
         float v[16];
         tmem_ld16(taddr + buf * BN + j0, v);
         const int ebv = next, left = N - n0 - j0;
-        next = !MN && !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? __ldg(eb + j0 + 16) : 0;
+        next = !MN && !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? eb[j0 + 16] : 0;
         if (!MN) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
   const int m = t.m0 + threadIdx.x;
   long off;
   if (!row_at<CONV>(g, m, &off)) return;
-  const int e = MN ? 0 : CONV ? kRowShift : __ldg(g.ea + m);
+  const int e = MN ? 0 : CONV ? kRowShift : g.ea[m];
   const int n0 = t.n0 + blockIdx.y * kJoinCols;
   const float* src = g.partial + ((size_t)blockIdx.x * g.splits * BN + blockIdx.y * kJoinCols) * kBM + threadIdx.x;
   float* dst = g.out + (size_t)t.tap * g.result + off;
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
     for (int j = 0; j < kJoinCols; ++j) v[j] += __ldcs(src + ((size_t)q * BN + j) * kBM);
 #pragma unroll
   for (int j = 0; j < kJoinCols; ++j)
-    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + __ldg(g.eb + n0 + j));
+    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
 }
 
 // ---- operand planes -----------------------------------------------------------------------------------------------------
@@ -516,11 +516,13 @@ __device__ __forceinline__ Bf3 split3(float a, float b) {
 __device__ __forceinline__ unsigned max4(unsigned m, float4 v) {
   return max(max(max(m, abs_bits(v.x)), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
 }
-// four values from c on of a row of `len`, zero past its end (`vec`: the row is 16-byte aligned)
+// four values from c on of a row of `len`, zero past its end (`vec`: the row is 16-byte aligned).  Ordinary loads: the kernels here
+// start while the one that writes the row may still run (the multiplied-out weight, or the result of another call), and the
+// read-only path (__ldg) is for memory that nothing writes during the kernel's life.
 __device__ __forceinline__ float4 load4(const float* row, int c, int len, bool vec) {
-  if (vec && c + 4 <= len) return __ldg(reinterpret_cast<const float4*>(row + c));
-  return make_float4(c < len ? __ldg(row + c) : 0.f, c + 1 < len ? __ldg(row + c + 1) : 0.f,
-                     c + 2 < len ? __ldg(row + c + 2) : 0.f, c + 3 < len ? __ldg(row + c + 3) : 0.f);
+  if (vec && c + 4 <= len) return *reinterpret_cast<const float4*>(row + c);
+  return make_float4(c < len ? row[c] : 0.f, c + 1 < len ? row[c + 1] : 0.f, c + 2 < len ? row[c + 2] : 0.f,
+                     c + 3 < len ? row[c + 3] : 0.f);
 }
 
 // Both operands of a product are split in one launch: the CTAs below `first` take the first.
@@ -635,7 +637,7 @@ __global__ void __launch_bounds__(256) split_pixels_kernel(const __grid_constant
     unsigned m = 0;
 #pragma unroll 16
     for (int c = ty; c < CH; c += 8) {
-      const float v = in ? __ldg(s + (size_t)c * HW) : 0.f;
+      const float v = in ? s[(size_t)c * HW] : 0.f;
       tile[c * kPxPitch + tx] = v;
       m = max(m, abs_bits(v));
     }
