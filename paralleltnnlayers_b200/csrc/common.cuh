@@ -9,6 +9,7 @@
 #include <cstdio>
 
 #include "b200cp.h"
+#include "raise_limit.hpp"
 
 namespace b200cp {
 
@@ -49,11 +50,8 @@ inline cudaError_t ensure_dynamic_smem(const void* kernel, std::atomic<int>* slo
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (slot[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) slot[dev].store(bytes, std::memory_order_relaxed);
-  return e;
+  const auto set = [kernel](int n) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n); };
+  return dev < 0 || dev >= 64 ? set(bytes) : raise_limit(slot[dev], bytes, set);
 }
 
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
