@@ -46,6 +46,9 @@ void b200cp_test_set_stream(int on);
  * checks that the count moved. */
 long long b200cp_test_stream_launches(void);
 
+/* Which plane products run on the tensor cores for a shape (3x3, pad 1): bit 0 the channel products, bit 1 the factor gradients. */
+int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s);
+
 /* Diagnostics: the row-band kernel writes 64 cycle stamps (long long) per CTA for its first 512 CTAs into this
  * device buffer (512 * 64 * 8 bytes); NULL switches it off.  Process-wide. */
 void b200cp_test_set_band_trace(void* device_buffer);

@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "b200cp_test.h"
 #include "cluster_util.cuh"
 #include "common.cuh"
 #include "cp_planes.cuh"
@@ -1049,6 +1050,11 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
 //              ranks 4-16         17-32              33-64              65-128
 //   convolution 1.23 1.09 1.03    0.97 0.99 0.82     1.06 0.79 0.80     0.92 0.93 0.78  (smaller shapes 0.85 to 0.97)
 //   gradients   1.47 1.48 1.44    1.12 1.05 1.08     1.05 0.93 0.93     1.02 0.94 0.87  (with the two products before them)
+// 17 to 32 ranks: products from 2^28 on (0.85, 0.78, 0.78 up to 2^31, over 40 more shapes).  Below, images of H W a multiple of 4
+// gain nothing (step of 64x256x256x14x14 R = 32 73.5 / 73.5, FFMA last; the error of the outputs against float64 is 1.03 times that of
+// FFMA, above 32 ranks 0.9 times); for the others FFMA loads single floats: steps of 64x512x512x13x13 R = 18 107 / 120,
+// 32x256x256x11x27 R = 31 59 / 69.  Gradients the same: 16x512x512x47x47 R = 20 213 / 243, 64x432x432x18x37 R = 23 249 / 280, but
+// 64x336x96x40x40 R = 23 358 / 337, 16x448x448x52x52 R = 18 247 / 231.
 struct PlanesOn {
   bool products, gradients;   // on the tensor cores
 };
@@ -1060,7 +1066,10 @@ PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
   if (mode != 1) return {mode == 2, mode == 2};
   const double macs = (double)s.N * s.H * s.W * s.Rank * ((double)s.C + s.T);
   if (s.Rank <= 16) return {false, false};
-  if (s.Rank <= 32) return {macs >= 1e8, macs >= 1e9};
+  if (s.Rank <= 32) {
+    const bool single = (size_t)s.H * s.W % 4 != 0;
+    return {macs >= (single ? 1e8 : 268435456.0), macs >= 1e9 && single};
+  }
   if (s.Rank > 64 && s.C + s.T <= 32) return {false, false};   // half of a K stage is padding: a step 1.01 to 1.28 times as long
   return {s.Rank > 64 || macs >= 1.3e8, macs >= 1.3e8};
 }
@@ -1245,3 +1254,8 @@ int planes_device_status(int* out) {
 }
 
 }  // namespace b200cp
+
+extern "C" int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s) {
+  const b200cp::PlanesOn on = b200cp::planes_on_tensor_cores(*s);
+  return (on.products ? 1 : 0) | (on.gradients ? 2 : 0);
+}

@@ -55,3 +55,21 @@ def test_argument_errors_without_gpu(lib_built):
     assert _lib.lib.b200cp_cp4_bwd_filter_workspace_bytes(ctypes.byref(s), 0) > 0
     assert _lib.lib.b200cp_status_string(-3) == b"workspace missing or too small"
     assert _lib.lib.b200cp_version() >= 100
+
+
+def test_planes_of_17_to_32_ranks_stay_on_ffma_where_tensor_cores_gain_nothing(lib_built):
+    from paralleltnnlayers_b200 import _lib
+
+    def on(N, C, T, H, W, R):
+        s = _lib.TensorShape(N=N, H=H, W=W, pad=1, T=T, C=C, Y=3, X=3, Rank=R)
+        return _lib.lib.b200cp_test_planes_on_tensor_cores(ctypes.byref(s))
+
+    assert on(64, 256, 256, 14, 14, 32) == 0            # 2.1e8 multiply-adds
+    assert on(64, 512, 512, 13, 13, 18) == 1            # 2.0e8, rows off sixteen bytes
+    assert on(32, 32, 32, 39, 39, 24) == 0
+    assert on(64, 320, 320, 14, 14, 32) == 0            # 2.6e8
+    assert on(64, 384, 384, 14, 14, 32) == 1            # 3.1e8
+    assert on(64, 256, 256, 50, 50, 32) == 1            # 2.6e9, rows of sixteen bytes
+    assert on(64, 256, 256, 51, 51, 32) == 3
+    assert on(64, 256, 256, 14, 14, 33) == 3
+    assert on(64, 256, 256, 14, 14, 16) == 0
