@@ -1063,15 +1063,17 @@ PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
     const char* e = getenv("B200CP_PLANES_TC");
     return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
   }();
-  if (mode != 1) return {mode == 2, mode == 2};
+  // a sum in a cluster of eight; FFMA has no such limit
+  const bool sums = std::max({s.T, s.C, s.Rank}) <= 8u * kTcMaxChunks * kTcK;
+  if (mode != 1) return {mode == 2 && sums, mode == 2};
   const double macs = (double)s.N * s.H * s.W * s.Rank * ((double)s.C + s.T);
   if (s.Rank <= 16) return {false, false};
   if (s.Rank <= 32) {
     const bool single = (size_t)s.H * s.W % 4 != 0;
-    return {macs >= (single ? 1e8 : 268435456.0), macs >= 1e9 && single};
+    return {sums && macs >= (single ? 1e8 : 268435456.0), macs >= 1e9 && single};
   }
   if (s.Rank > 64 && s.C + s.T <= 32) return {false, false};   // half of a K stage is padding: a step 1.01 to 1.28 times as long
-  return {s.Rank > 64 || macs >= 1.3e8, macs >= 1.3e8};
+  return {sums && (s.Rank > 64 || macs >= 1.3e8), macs >= 1.3e8};
 }
 
 struct GradPlan {
@@ -1134,8 +1136,7 @@ Buffers carve(Carve& c, const b200cp_tensor_shape& s, bool P, bool Q, bool Z, bo
 bool planes_supported(const b200cp_tensor_shape& s) {
   const size_t HW = (size_t)s.H * s.W, most = std::max({s.T, s.C, s.Rank});
   return s.Y == 3 && s.X == 3 && s.pad == 1 && (size_t)s.N * (s.H + 3) * s.W < (1u << 30) && s.Rank < 65536 &&
-         ((size_t)s.T + s.C) * s.Rank < (1u << 30) && most <= 8 * kTcMaxChunks * kTcK &&
-         (most / 16 + 1) * (s.N * HW / 64 + 1) < (1u << 30);
+         ((size_t)s.T + s.C) * s.Rank < (1u << 30) && (most / 16 + 1) * (s.N * HW / 64 + 1) < (1u << 30);
 }
 
 // `parts`: what the call computes (the workspace of more parts is enough for fewer)

@@ -57,7 +57,7 @@ def test_argument_errors_without_gpu(lib_built):
     assert _lib.lib.b200cp_version() >= 100
 
 
-def test_planes_of_17_to_32_ranks_stay_on_ffma_where_tensor_cores_gain_nothing(lib_built):
+def test_rule_of_the_plane_products(lib_built):
     from paralleltnnlayers_b200 import _lib
 
     def on(N, C, T, H, W, R):
@@ -73,3 +73,4 @@ def test_planes_of_17_to_32_ranks_stay_on_ffma_where_tensor_cores_gain_nothing(l
     assert on(64, 256, 256, 51, 51, 32) == 3
     assert on(64, 256, 256, 14, 14, 33) == 3
     assert on(64, 256, 256, 14, 14, 16) == 0
+    assert on(1, 8192, 24, 20, 20, 65) == 3 and on(1, 8193, 24, 20, 20, 65) == 2   # a cluster's sum has 8192 terms

@@ -97,6 +97,26 @@ def test_cp3(shape):
         assert_parity(got, ref)
 
 
+def test_more_than_8192_channels():
+    """The sum over the channels on the tensor cores ends at 8192 channels (ranks); the products take more, on FFMA, in the same
+    launches."""
+    import paralleltnnlayers_b200 as P
+    from paralleltnnlayers_b200._lib import lib
+    launches = []
+    for C in (8192, 8200):
+        X, dU, K = make((1, C, 24, 7, 7, 65), False)
+        x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+        before = lib.b200cp_launch_count()
+        U, dX, dK = P.cp4_conv2d_step(x, du, *k)
+        launches.append(lib.b200cp_launch_count() - before)
+        want = expect(X, dU, K)
+        assert_parity(U, want[0])
+        assert_parity(dX, want[1])
+        for got, ref in zip(torch.split(dK.flatten(), [w.size for w in want[2:]]), want[2:]):
+            assert_parity(got.view(ref.shape), ref)
+    assert launches[0] == launches[1]
+
+
 def test_streams_and_capture():
     """Two streams at once, and a captured step: the workspace belongs to the call, nothing is shared."""
     import paralleltnnlayers_b200 as P
