@@ -46,6 +46,11 @@ void b200cp_test_set_stream(int on);
  * checks that the count moved. */
 long long b200cp_test_stream_launches(void);
 
+/* Plane products (3x3, pad 1): `planes` 0 = never, 1 = by the rule, 2 = wherever they can run; `tensor_cores` likewise for the form of
+ * the channel products and factor gradients (0 = FFMA); -1 = what the environment variables B200CP_PLANES / B200CP_PLANES_TC say
+ * (by the rule unless set).  A workspace query and its call want the same setting.  Process-wide. */
+void b200cp_test_set_planes(int planes, int tensor_cores);
+
 /* Which plane products run on the tensor cores for a shape (3x3, pad 1): bit 0 the channel products, bit 1 the factor gradients. */
 int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s);
 

@@ -119,6 +119,7 @@ def _load():
         "b200cp_test_set_band_max_rank": (None, [i]),
         "b200cp_test_set_stream": (None, [i]),
         "b200cp_test_stream_launches": (C.c_longlong, []),
+        "b200cp_test_set_planes": (None, [i, i]),
         "b200cp_test_planes_on_tensor_cores": (i, [sp]),
         "b200cp_test_set_p2p_wait_cycles": (None, [C.c_longlong]),
         "b200cp_test_p2p_connect_local": (i, [vp, pp]),

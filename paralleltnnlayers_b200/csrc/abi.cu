@@ -119,8 +119,9 @@ const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
 // one convolution; the step; the backward from the forward's plane; the factor gradients; the last two of CP3
 enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3 };
 bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
-  if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !g_planes || !planes_supported(*s)) return false;
-  if (g_planes == 2) return true;
+  const int forced = g_planes_test.load(std::memory_order_relaxed), planes = forced < 0 ? g_planes : forced;
+  if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !planes || !planes_supported(*s)) return false;
+  if (planes == 2) return true;
   const double ch = (double)s->C + s->T, root4 = std::sqrt(std::sqrt((double)s->N * s->H * s->W));
   if (s->Rank <= 16) {
     const double few = ch * std::sqrt((double)s->Rank) / root4;

@@ -24,6 +24,7 @@
 
 namespace b200cp {
 
+std::atomic<int> g_planes_test{-1};
 __device__ int g_planes_status = 0;  // 0 ok; otherwise (1 << 16) | (block index & 0xffff): a bounded wait ran out
 
 namespace {
@@ -1055,14 +1056,16 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
 // FFMA, above 32 ranks 0.9 times); for the others FFMA loads single floats: steps of 64x512x512x13x13 R = 18 107 / 120,
 // 32x256x256x11x27 R = 31 59 / 69.  Gradients the same: 16x512x512x47x47 R = 20 213 / 243, 64x432x432x18x37 R = 23 249 / 280, but
 // 64x336x96x40x40 R = 23 358 / 337, 16x448x448x52x52 R = 18 247 / 231.
+std::atomic<int> g_planes_tc_test{-1};   // b200cp_test_set_planes
 struct PlanesOn {
   bool products, gradients;   // on the tensor cores
 };
 PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
-  static const int mode = [] {   // B200CP_PLANES_TC: 0 FFMA, 2 tensor cores, else by the rule
+  static const int env = [] {   // B200CP_PLANES_TC: 0 FFMA, 2 tensor cores, else by the rule
     const char* e = getenv("B200CP_PLANES_TC");
     return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
   }();
+  const int forced = g_planes_tc_test.load(std::memory_order_relaxed), mode = forced < 0 ? env : forced;
   // a sum in a cluster of eight; FFMA has no such limit
   const bool sums = std::max({s.T, s.C, s.Rank}) <= 8u * kTcMaxChunks * kTcK;
   if (mode != 1) return {mode == 2 && sums, mode == 2};
@@ -1255,6 +1258,11 @@ int planes_device_status(int* out) {
 }
 
 }  // namespace b200cp
+
+extern "C" void b200cp_test_set_planes(int planes, int tensor_cores) {
+  b200cp::g_planes_test.store(planes, std::memory_order_relaxed);
+  b200cp::g_planes_tc_test.store(tensor_cores, std::memory_order_relaxed);
+}
 
 extern "C" int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s) {
   const b200cp::PlanesOn on = b200cp::planes_on_tensor_cores(*s);

@@ -17,6 +17,7 @@ struct PlanesJob {
   float *U = nullptr, *dX = nullptr, *dK = nullptr;
 };
 enum { kPlanesFwd = 1, kPlanesBwd = 2, kPlanesGrads = 4, kPlanesNoP = 8, kPlanesNoQ = 16 };   // NoP / NoQ: given or saved
+extern std::atomic<int> g_planes_test;   // b200cp_test_set_planes: which calls take them (abi.cu)
 bool planes_supported(const b200cp_tensor_shape& s);
 size_t planes_workspace(const b200cp_tensor_shape& s, int parts);
 int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st);

@@ -97,6 +97,75 @@ def test_cp3(shape):
         assert_parity(got, ref)
 
 
+# Of the tensor-core kernels: tiles of 128 pixels, of 128 channels and 32 or 64 ranks (gradients) and of up to 256 rows (products),
+# chunks of 64 terms, sums over clusters of 2, 4 and 8 CTAs (some without a chunk), more pixel tiles than resident CTAs.
+TC_SHAPES = SHAPES + [
+    (3, 1, 127, 9, 9, 17), (2, 127, 129, 8, 9, 33), (1, 128, 1, 11, 12, 64), (2, 129, 128, 7, 9, 65), (1, 130, 63, 16, 8, 31),
+    (1, 320, 320, 9, 9, 40), (1, 600, 130, 9, 9, 35), (1, 140, 200, 20, 20, 100), (1, 1030, 70, 5, 5, 200),
+    (16, 65, 33, 49, 51, 33), (10, 33, 130, 63, 61, 17), (64, 5, 6, 28, 22, 70),
+]
+
+
+@pytest.fixture
+def form(request):
+    from paralleltnnlayers_b200._lib import lib
+    lib.b200cp_test_set_planes(2, request.param)
+    yield request.param
+    lib.b200cp_test_set_planes(-1, -1)
+
+
+@pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
+@pytest.mark.parametrize("shape", TC_SHAPES, ids=str)
+def test_both_forms(form, shape):
+    """Every call over planes, in either arithmetic, whatever the rule would take.  Bound: a split product is off by at most 2**-21, its
+    accumulator of 64 terms by 4 * 2**-23 of the partial sums; the rank plane, the stencil and the sum over ranks or pixels follow one
+    another.  In the norm, with random signs, below 4e-7 (measured over drawn shapes: 3e-7, FFMA 6.5e-7)."""
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make(shape, False)
+    want = expect(X, dU, K)
+    x, du, k = offset(X), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+
+    def close(got, refs):
+        for i, (g, r) in enumerate(zip(got, refs)):
+            err = np.linalg.norm(g.detach().double().cpu().numpy() - r) / np.linalg.norm(r)
+            assert err < 1e-6, (i, err)
+
+    U, dX, dK = P.cp4_conv2d_step(x, du, *k)
+    grads = [g.view(r.shape) for g, r in zip(torch.split(dK.flatten(), [w.size for w in want[2:]]), want[2:])]
+    close((U, dX, *grads), want)
+    close((P.cp4_conv2d_forward(x, *k), P.cp4_conv2d_backward_data(du, *k), *P.cp4_conv2d_backward_filter(du, x, *k)), want)
+    X, dU, K = make(shape, True)
+    want = expect(X, dU, K)
+    leaves = [torch.from_numpy(a).cuda().requires_grad_() for a in (X, *K)]
+    y = P.CP3Conv2dFunction.apply(*leaves)
+    close((y, *torch.autograd.grad(y, leaves, torch.from_numpy(dU).cuda())), want)
+    P.device_status()
+
+
+@pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
+@pytest.mark.parametrize("R", [24, 40])
+def test_images_keep_their_own_scale(form, R):
+    """Pixels have their own power of two: an image is as accurate beside any other.  NaN and infinities stay with the pixels that a
+    tap reaches."""
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make((4, 70, 65, 9, 10, R), False)
+    scale = np.array([1e-25, 1.0, 1e25, 1e-8], np.float32)[:, None, None, None]
+    want = expect(X * scale, dU * scale[::-1], K)
+    put = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    x, du, k = put(X * scale), put(dU * scale[::-1]), [put(f) for f in K]
+    U, dX, _ = P.cp4_conv2d_step(x, du, *k)
+    for got, ref in ((U, want[0]), (dX, want[1])):
+        for n in range(4):
+            assert np.linalg.norm(got[n].double().cpu().numpy() - ref[n]) < 1e-6 * np.linalg.norm(ref[n])
+    x[1, 5, 2, 3], x[2, 6, 4, 8] = float("nan"), float("inf")
+    hit = torch.zeros(4, 9, 10, dtype=torch.bool, device="cuda")
+    hit[1, 1:4, 2:5] = hit[2, 3:6, 7:10] = True
+    V = P.cp4_conv2d_forward(x, *k)
+    assert not bool(torch.isfinite(V.movedim(1, -1)[hit]).any())
+    assert torch.equal(V.movedim(1, -1)[~hit], P.cp4_conv2d_forward(put(X * scale), *k).movedim(1, -1)[~hit])
+    P.device_status()
+
+
 def test_more_than_8192_channels():
     """The sum over the channels on the tensor cores ends at 8192 channels (ranks); the products take more, on FFMA, in the same
     launches."""
