@@ -594,13 +594,15 @@ __global__ void __launch_bounds__(kThreads) plane_stencil_kernel(const __grid_co
 }
 
 // ---- partial factor gradients: part[split][row][r] = sum over a pixel range of D[row][q] Z[r][q] ------------------------
-// On the tensor cores: 128 rows of dU or X and NT ranks per CTA, K = pixels, which both operands have contiguous.  A warp
-// takes a row at a time: 64 pixels, two per lane, their largest magnitude by one warp reduction, and 4 bytes of each plane per
-// lane.  A chunk of 64 pixels has an accumulator of its own in half of TMEM (two CTAs per SM); once these are used up
-// they are added to totals in registers, each with the powers of two of its row and its rank in that chunk.
+// On the tensor cores: 128 rows of dU or X and NT ranks per CTA, K = pixels, which both operands have contiguous.  The sum runs
+// over pixels and images, of which one may be any number of binades above the others and add nothing (a masked sample: zeros in the
+// other operand), so no two pixels share an exponent: a value is three bf16 parts, a product six of theirs (gemm_tc.cu).  A warp takes
+// a row at a time: 64 pixels, two per lane, and 4 bytes of each plane per lane.  A chunk of 64 pixels has an accumulator of
+// its own in half of TMEM (two CTAs per SM); once these are used up they are added to totals in registers.
 //
-// What bounds it is the splitting (about 25 instructions per row and chunk) and latency: 64 x 256 14x14 at R = 32 19 us on FFMA,
-// 20 here; 16 x 256 -> 384 27x27 at R = 50 (4-byte loads) 36 and 28.
+// What bounds it is the splitting and latency: 64 x 256 14x14 at R = 32 18 us on FFMA, 22 here; 16 x 256 -> 384 27x27 at R = 50
+// (4-byte loads) 34 and 32.  Fp16 pairs with an exponent per row and 64 pixels took 20 and 28, and lost 3e-4 of the result at 7x7 images
+// beside one of 1e9 without gradient.  Three CTAs per SM with half of the TMEM columns each spill (32 -> 48 us).
 struct PlaneGrad {
   const float* D[2];     // dU, X
   const float* Z[2];     // Z, Zt
@@ -611,14 +613,13 @@ struct PlaneGrad {
   size_t nrows;          // T + C
 };
 constexpr int kGradThreads = 256, kGradRows = 128;
-constexpr int kGradShift = 12;   // between the two powers of two of a sum, for values near the ends of the range
 
 template <int NT>
 struct GradTile {
   static constexpr int chunks = 256 / NT;                            // accumulators
   static constexpr int bplane = NT * 128;
-  static constexpr int stage = 2 * (kTcPlane + bplane);
-  static constexpr size_t smem = 1024 + 2 * (size_t)stage;           // at least the [128][NT + 1] floats of the result
+  static constexpr int stage = 3 * (kTcPlane + bplane);
+  static constexpr size_t smem = 1024 + (size_t)stage;               // at least the [128][NT + 1] floats of the result
 };
 
 template <int NT>
@@ -626,10 +627,8 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
   using T = GradTile<NT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t done[2];
+  __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_slot;
-  __shared__ float fa[T::chunks][kGradRows];
-  __shared__ __align__(16) float fb[T::chunks][NT];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = warp >> 2;
   const int rt = blockIdx.x % g.rtiles, mi = blockIdx.x / g.rtiles, half = mi >= g.mtiles[0] ? 1 : 0;
   const int m0 = (mi - (half ? g.mtiles[0] : 0)) * kGradRows, r0 = rt * NT, rows = half ? g.rows[1] : g.rows[0];
@@ -638,8 +637,7 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
   const float* Z = (half ? g.Z[1] : g.Z[0]) + (size_t)r0 * g.HW;
   const int arows = min(kGradRows, rows - m0), brows = min(NT, g.R - r0);
   if (tid == 0) {
-    tc::mbar_init(&done[0], 1);
-    tc::mbar_init(&done[1], 1);
+    tc::mbar_init(&done, 1);
     tc::fence_barrier_init();
   }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, 256);
@@ -648,7 +646,7 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
   tc::tc_fence_after_sync();
   const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
-  const uint32_t idesc = tc::make_idesc_f16(NT);
+  const uint32_t idesc = tc::make_idesc_bf16(NT);
   const int steps = qe > qb ? (qe - qb + kTcK - 1) / kTcK : 0;
   float tot[NT / 2];
 #pragma unroll
@@ -686,9 +684,8 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
     load_rows(warp);
   }
   for (int s = 0; s < steps; ++s) {
-    const int st = s & 1, c = s % T::chunks;
-    uint8_t* As = sm + st * T::stage;
-    if (s >= 2) fine = tc::mbar_wait(&done[st], (s / 2 - 1) & 1) && fine;
+    const int c = s % T::chunks;
+    if (s) fine = tc::mbar_wait(&done, (s - 1) & 1) && fine;   // (the other CTA of the SM works meanwhile)
 #pragma unroll 1
     for (int i = warp; i < kGroups; i += kWarps) {
       const bool isb = i >= kGradRows / 8;
@@ -702,62 +699,53 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
         pixels(s + 1);
         load_rows(warp);
       }
-      uint8_t* d = As + (isb ? 2 * kTcPlane : 0) + first * 128;
-      const uint32_t lo = isb ? T::bplane : kTcPlane;
-      int mine = 0;
+      uint8_t* d = sm + (isb ? 3 * kTcPlane : 0) + first * 128;
+      const uint32_t plane = isb ? T::bplane : kTcPlane;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int e = tc::row_exponent(__reduce_max_sync(0xffffffffu, max(tc::abs_bits(u[k]), tc::abs_bits(v[k]))), tc::kLeastConv);
-        if (lane == k) mine = e;
-        const float sc = tc::exp2_int(-e), p = u[k] * sc, q = v[k] * sc;
-        const __half2 h = __floats2half2_rn(p, q);
-        const float2 f = __half22float2(h);
+        const tc::Bf3 w = tc::split3(u[k], v[k]);
         uint8_t* o = d + k * 128 + (((lane >> 2) ^ k) << 4) + (lane & 3) * 4;
-        *reinterpret_cast<__half2*>(o) = h;
-        *reinterpret_cast<__half2*>(o + lo) = __floats2half2_rn(p - f.x, q - f.y);
-      }
-      if (lane < 8) {
-        if (isb) fb[c][first + lane] = tc::exp2_int(mine + kGradShift);
-        else fa[c][first + lane] = tc::exp2_int(mine - kGradShift);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint32_t*>(o + q * plane) = w.p[q];
       }
     }
     tc::fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
       tc::tc_fence_after_sync();
-      const uint32_t as = tc::smem_u32(As), bs = as + 2 * kTcPlane, d = tmem + c * NT;
-      const uint64_t ah = d0 + (as >> 4), al = d0 + ((as + kTcPlane) >> 4), bh = d0 + (bs >> 4), bl = d0 + ((bs + T::bplane) >> 4);
+      const uint32_t as = tc::smem_u32(sm), d = tmem + c * NT;
+      const uint64_t a0 = d0 + (as >> 4), b0 = d0 + ((as + 3 * kTcPlane) >> 4);
+      constexpr uint64_t A1 = kTcPlane >> 4, B1 = T::bplane >> 4;
 #pragma unroll
-      for (int i = 0; i < kTcK / 16; ++i) {
-        tc::mma_f16_ss(d, al + i * 2, bh + i * 2, idesc, i > 0);
-        tc::mma_f16_ss(d, ah + i * 2, bl + i * 2, idesc, true);
+      for (int i = 0; i < kTcK / 16; ++i) {   // the products of 2^-16 first
+        tc::mma_f16_ss(d, a0 + 2 * A1 + i * 2, b0 + i * 2, idesc, i > 0);
+        tc::mma_f16_ss(d, a0 + i * 2, b0 + 2 * B1 + i * 2, idesc, true);
+        tc::mma_f16_ss(d, a0 + A1 + i * 2, b0 + B1 + i * 2, idesc, true);
       }
 #pragma unroll
-      for (int i = 0; i < kTcK / 16; ++i) tc::mma_f16_ss(d, ah + i * 2, bh + i * 2, idesc, true);
-      tc::mma_commit(&done[st]);
+      for (int i = 0; i < kTcK / 16; ++i) {
+        tc::mma_f16_ss(d, a0 + A1 + i * 2, b0 + i * 2, idesc, true);
+        tc::mma_f16_ss(d, a0 + i * 2, b0 + B1 + i * 2, idesc, true);
+      }
+#pragma unroll
+      for (int i = 0; i < kTcK / 16; ++i) tc::mma_f16_ss(d, a0 + i * 2, b0 + i * 2, idesc, true);
+      tc::mma_commit(&done);
     }
     if (c + 1 < T::chunks && s + 1 < steps) continue;
     // the accumulators, in the order of the pixels
-    fine = tc::mbar_wait(&done[st], (s / 2) & 1) && fine;
+    fine = tc::mbar_wait(&done, s & 1) && fine;
     tc::tc_fence_after_sync();
     for (int k = 0; k <= c; ++k) {
-      const float f = fa[k][(warp & 3) * 32 + lane];
 #pragma unroll
       for (int j0 = 0; j0 < NT / 2; j0 += 16) {
         float v[16];
         tc::tmem_ld16(lanes + k * NT + grp * (NT / 2) + j0, v);
 #pragma unroll
-        for (int j = 0; j < 16; j += 4) {
-          const float4 w = lds4(&fb[k][grp * (NT / 2) + j0 + j]);
-          tot[j0 + j] = fmaf(v[j], f * w.x, tot[j0 + j]);
-          tot[j0 + j + 1] = fmaf(v[j + 1], f * w.y, tot[j0 + j + 1]);
-          tot[j0 + j + 2] = fmaf(v[j + 2], f * w.z, tot[j0 + j + 2]);
-          tot[j0 + j + 3] = fmaf(v[j + 3], f * w.w, tot[j0 + j + 3]);
-        }
+        for (int j = 0; j < 16; ++j) tot[j0 + j] += v[j];
       }
     }
     tc::tc_fence_before_sync();
-    __syncthreads();   // the accumulators and the powers of two are free
+    __syncthreads();   // the accumulators are free
   }
   if (!fine) atomicCAS(&g_planes_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
   grid_launch_dependents();
@@ -1054,8 +1042,8 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
 // 17 to 32 ranks: products from 2^28 on (0.85, 0.78, 0.78 up to 2^31, over 40 more shapes).  Below, images of H W a multiple of 4
 // gain nothing (step of 64x256x256x14x14 R = 32 73.5 / 73.5, FFMA last; the error of the outputs against float64 is 1.03 times that of
 // FFMA, above 32 ranks 0.9 times); for the others FFMA loads single floats: steps of 64x512x512x13x13 R = 18 107 / 120,
-// 32x256x256x11x27 R = 31 59 / 69.  Gradients the same: 16x512x512x47x47 R = 20 213 / 243, 64x432x432x18x37 R = 23 249 / 280, but
-// 64x336x96x40x40 R = 23 358 / 337, 16x448x448x52x52 R = 18 247 / 231.
+// 32x256x256x11x27 R = 31 59 / 69.  Gradients the same: 16x512x512x47x47 R = 20 225 / 242, 64x432x432x18x37 R = 23 262 / 280, but
+// 64x336x96x40x40 R = 23 372 / 337, 16x448x448x52x52 R = 18 261 / 231.
 std::atomic<int> g_planes_tc_test{-1};   // b200cp_test_set_planes
 struct PlanesOn {
   bool products, gradients;   // on the tensor cores

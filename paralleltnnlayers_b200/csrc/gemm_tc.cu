@@ -31,8 +31,6 @@
 #include <cstdio>
 #include <cstdlib>
 
-#include <cuda_bf16.h>
-
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -490,28 +488,6 @@ __device__ __forceinline__ void split4(float4 v, float sc, Half4& hi, Half4& lo)
   const float2 p = __half22float2(hi.a), q = __half22float2(hi.b);
   lo.a = __floats2half2_rn(v.x - p.x, v.y - p.y);
   lo.b = __floats2half2_rn(v.z - q.x, v.w - q.y);
-}
-// Two values as three bf16 parts each, x = p[0] + p[1] + p[2] exactly (8 + 8 + 8 bits, each part with its own exponent; the last
-// may fall below the smallest float).  A value that would round up to infinity is cut instead.
-struct Bf3 {
-  uint32_t p[3];
-};
-__device__ __forceinline__ Bf3 split3(float a, float b) {
-  Bf3 out;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    float2 f = __bfloat1622float2(h);
-    if (q == 0 && (isinf(f.x) || isinf(f.y))) {
-      if (isinf(f.x)) h.x = __float2bfloat16_rz(a);
-      if (isinf(f.y)) h.y = __float2bfloat16_rz(b);
-      f = __bfloat1622float2(h);
-    }
-    a -= f.x;
-    b -= f.y;
-    out.p[q] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  return out;
 }
 __device__ __forceinline__ unsigned max4(unsigned m, float4 v) {
   return max(max(max(m, abs_bits(v.x)), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));

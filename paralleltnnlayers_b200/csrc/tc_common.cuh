@@ -6,6 +6,7 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -186,8 +187,32 @@ __device__ __forceinline__ void split8(const float* v, float sc, uint4& hi, uint
   hi = make_uint4(h[0], h[1], h[2], h[3]);
   lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
-// Instruction descriptor for kind::f16 with K-major fp16 operands and fp32 accumulation, M = 128 (one CTA).
+// ---- three bf16 parts -------------------------------------------------------------------------------------------------
+// Two values as three bf16 parts each, x = p[0] + p[1] + p[2] exactly (8 + 8 + 8 bits, each part with its own exponent; the last
+// may fall below the smallest float).  A value that would round up to infinity is cut instead.
+struct Bf3 {
+  uint32_t p[3];
+};
+__device__ __forceinline__ Bf3 split3(float a, float b) {
+  Bf3 out;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    float2 f = __bfloat1622float2(h);
+    if (q == 0 && (isinf(f.x) || isinf(f.y))) {
+      if (isinf(f.x)) h.x = __float2bfloat16_rz(a);
+      if (isinf(f.y)) h.y = __float2bfloat16_rz(b);
+      f = __bfloat1622float2(h);
+    }
+    a -= f.x;
+    b -= f.y;
+    out.p[q] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return out;
+}
+// Instruction descriptor for kind::f16 with K-major operands and fp32 accumulation, M = 128 (one CTA): fp16, or bf16.
 __host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+__host__ __device__ constexpr uint32_t make_idesc_bf16(uint32_t n) { return make_idesc_f16(n) | (1u << 7) | (1u << 10); }
 __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
   asm volatile(
       "{\n"

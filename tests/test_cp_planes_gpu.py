@@ -166,6 +166,24 @@ def test_images_keep_their_own_scale(form, R):
     P.device_status()
 
 
+@pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
+@pytest.mark.parametrize("R", [24, 40])
+@pytest.mark.parametrize("where", ["input", "gradient"])
+def test_factor_gradients_beside_a_large_sample(form, R, where):
+    """An image whose gradient (or input) is zero adds nothing to the factor gradients, however large its input (gradient) is."""
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make((6, 70, 65, 5, 9, R), False)
+    big, none = (X, dU) if where == "input" else (dU, X)
+    big[1] *= 1e9
+    big[4, 3] *= 1e15
+    none[[1, 4]] = 0
+    want = expect(X, dU, K)[2:]
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+    dK = P.cp4_conv2d_step(x, du, *k)[2].flatten()
+    for got, ref in zip(torch.split(dK, [w.size for w in want]), want):
+        assert np.linalg.norm(got.view(ref.shape).double().cpu().numpy() - ref) < 1e-6 * np.linalg.norm(ref)
+
+
 def test_more_than_8192_channels():
     """The sum over the channels on the tensor cores ends at 8192 channels (ranks); the products take more, on FFMA, in the same
     launches."""
