@@ -188,26 +188,23 @@ __device__ __forceinline__ void split8(const float* v, float sc, uint4& hi, uint
   lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 // ---- three bf16 parts -------------------------------------------------------------------------------------------------
-// Two values as three bf16 parts each, x = p[0] + p[1] + p[2] exactly (8 + 8 + 8 bits, each part with its own exponent; the last
-// may fall below the smallest float).  A value that would round up to infinity is cut instead.
+// Two values as three bf16 parts each, x = p[0] + p[1] + p[2] exactly (each part with its own exponent; the last may fall below the
+// smallest float).  The first is cut off, so that no finite value becomes infinite; the other two are rounded, so that what a
+// product leaves out (p[1] p[2], 2^-24 of it) has no preferred sign.
 struct Bf3 {
   uint32_t p[3];
 };
 __device__ __forceinline__ Bf3 split3(float a, float b) {
   Bf3 out;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    float2 f = __bfloat1622float2(h);
-    if (q == 0 && (isinf(f.x) || isinf(f.y))) {
-      if (isinf(f.x)) h.x = __float2bfloat16_rz(a);
-      if (isinf(f.y)) h.y = __float2bfloat16_rz(b);
-      f = __bfloat1622float2(h);
-    }
-    a -= f.x;
-    b -= f.y;
-    out.p[q] = *reinterpret_cast<const uint32_t*>(&h);
-  }
+  const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
+  out.p[0] = __byte_perm(x, y, 0x7632);
+  a -= __uint_as_float(x & 0xffff0000u);
+  b -= __uint_as_float(y & 0xffff0000u);
+  const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+  const float2 f = __bfloat1622float2(m);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(a - f.x, b - f.y);
+  out.p[1] = *reinterpret_cast<const uint32_t*>(&m);
+  out.p[2] = *reinterpret_cast<const uint32_t*>(&l);
   return out;
 }
 // Instruction descriptor for kind::f16 with K-major operands and fp32 accumulation, M = 128 (one CTA): fp16, or bf16.
