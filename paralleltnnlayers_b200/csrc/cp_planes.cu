@@ -9,7 +9,8 @@
 // lanes (64 images of 512 x 7x7 at R = 64: 52 us per convolution, 77 us for the factor gradients, for 0.1 GMAC per
 // product; here 31 us and 37 us).  Here a phase is a launch of its own, over the pixels of all images as one flat range, so that a tile is
 // always full and the sum can be split over a cluster; the planes (R of C channels) pass through L2.  The launches are
-// programmatic dependents of one another.  Everything is exact fp32 (FFMA).
+// programmatic dependents of one another.  The products and the factor gradients exist on FFMA and on the tensor cores, where a
+// value is three bf16 parts (24 bits) and a product six of theirs; the stencils are FFMA.
 // Formulas: Cuda_kernels/cp4Conv2dForward.cu:42-134, cp4Conv2dBackwardData.cu:29-109, cp4Conv2dBackwardFilter.cu:64-257.
 #include <algorithm>
 #include <cstdlib>
@@ -226,21 +227,24 @@ __global__ void __launch_bounds__(kThreads) plane_gemm_kernel(const __grid_const
 }
 
 // ---- out[n][m][p] = sum_k F(m, k) in[n][k][p] on the tensor cores ---------------------------------------------------------
-// The products of a CP convolution with whole rank planes: P = K1^T X (F is [K][M]) and U = K0 Z (AK: F is [M][K]).  Scaled fp16
-// hi / lo operands as in gemm_tc.cu: three products, accumulators of 64 terms.
+// The products of a CP convolution with whole rank planes: P = K1^T X (F is [K][M]) and U = K0 Z (AK: F is [M][K]).  Every value is
+// three bf16 parts and a product six of theirs, as in the gradients of gemm_tc.cu: channels and ranks may differ in scale by any
+// factor (that of a rank is free to move between the factor matrices).  Accumulators of 64 terms.
 //
-// 128 pixels are the rows of the tensor-core tile, one per thread and per TMEM lane: a thread loads 64 values of its pixel (the
-// lanes of a warp read 32 neighbours of a plane, at any width or alignment), finds their exponent, and writes the swizzled
-// operand rows itself, so no pass over memory and no exchange between threads is needed.  Two groups of 128 threads take the
-// chunks of 64 in turn: one loads and splits while the other's products run.  Every chunk has its own accumulator in TMEM
-// (chunks x rows <= 512 columns); at the end they are added up, each with its pixel's power of two.  F is split once per CTA,
+// 128 pixels are the rows of the tensor-core tile, one per TMEM lane and G threads: each loads 64 / G values of a chunk (the
+// lanes of a warp read 32 neighbours of a plane, at any width or alignment) and writes them as swizzled operand rows itself, so no
+// pass over memory is needed.  G = 2 where two CTAs fit an SM; else G = 4, and the loads run two chunks ahead.  Every chunk has
+// its own accumulator in TMEM (chunks x rows <= 512 columns); at the end they are added up.  F is split once per CTA,
 // which then walks the pixel tiles; where the pixels alone leave SMs idle the sum is split over a cluster instead.
 //
-// What bounds it is latency: about 3 us until F is split, 1 to 2 us per half chunk loaded, 1 us for the products and 1 to 3 us to
-// store.  Both products of 64 x 256 14x14 at R = 32: P and Q 21.7 us on FFMA, 16.8 here; the outputs 21 and 17.
-constexpr int kTcThreads = 256, kTcPx = 128, kTcK = 64;
-constexpr int kTcPlane = kTcPx * 128;   // bytes of one operand plane (hi or lo) of a chunk
-constexpr int kTcMaxChunks = 16;
+// What bounds it is latency: a chunk's loads 1 to 2 us, its products 0.5, a commit 0.3, the split of F 1 to 3.  Both products of
+// 64 x 256 14x14 at R = 32: P and Q 21.9 us on FFMA, 20.2 here, the outputs 18.2 and 17.0; of 16 x 256 -> 384 27x27 at R = 50: 53.9 and
+// 36.8, 44.4 and 25.0.  Fp16 pairs with an exponent per pixel and chunk took 19.6, 16.4, 36.0 and 23.8, and lost the result where a
+// rank is scaled up in one factor and down in another (R = 24, by 2^-40 to 2^40).  Error against float64 over 60 drawn shapes 0.7
+// times that of FFMA.
+constexpr int kTcPx = 128, kTcK = 64;
+constexpr int kTcPlane = kTcPx * 128;   // bytes of one operand plane of a chunk
+constexpr int kTcMaxChunks = 14;        // that fit in shared memory with rows of 32
 
 struct PlaneTcProduct {
   const float* F;
@@ -255,25 +259,35 @@ struct PlaneTc {
   int first;                // the input is not the work of the kernel before
 };
 
-// eight fp32 values (four at d, four at d2, one plane on) become their hi and lo halves
-__device__ __forceinline__ void split_in_place(uint8_t* d, uint8_t* d2, float sc) {
-  const float4 x = *reinterpret_cast<const float4*>(d), y = *reinterpret_cast<const float4*>(d2);
-  const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-  uint4 hi, lo;
-  tc::split8(v, sc, hi, lo);
-  *reinterpret_cast<uint4*>(d) = hi;
-  *reinterpret_cast<uint4*>(d2) = lo;
+// eight values to 16 bytes of each plane
+__device__ __forceinline__ void put8(uint8_t* d, uint32_t plane, const float* v) {
+  tc::Bf3 w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = tc::split3(v[2 * i], v[2 * i + 1]);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(d + q * plane) = make_uint4(w[0].p[q], w[1].p[q], w[2].p[q], w[3].p[q]);
+}
+// the six products of a chunk of 16 kk terms, the smallest first
+__device__ __forceinline__ void mma_chunk(uint32_t d, uint64_t a, uint64_t A1, uint64_t b, uint64_t B1, uint32_t idesc, int kk) {
+  for (int i = 0; i < kk; ++i) {
+    tc::mma_f16_ss(d, a + 2 * A1 + i * 2, b + i * 2, idesc, i > 0);
+    tc::mma_f16_ss(d, a + i * 2, b + 2 * B1 + i * 2, idesc, true);
+    tc::mma_f16_ss(d, a + A1 + i * 2, b + B1 + i * 2, idesc, true);
+  }
+  for (int i = 0; i < kk; ++i) {
+    tc::mma_f16_ss(d, a + A1 + i * 2, b + i * 2, idesc, true);
+    tc::mma_f16_ss(d, a + i * 2, b + B1 + i * 2, idesc, true);
+  }
+  for (int i = 0; i < kk; ++i) tc::mma_f16_ss(d, a + i * 2, b + i * 2, idesc, true);
 }
 
-template <bool AK>
-__global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_constant__ PlaneTc g) {
+template <bool AK, int G>
+__global__ void __launch_bounds__(G * 128, 4 / G) plane_tc_kernel(const __grid_constant__ PlaneTc g) {
+  constexpr int kThreads = G * 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t done[2];
+  __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_slot;
-  __shared__ unsigned rowmax[256];
-  __shared__ __align__(16) float2 rowscale[256];
-  __shared__ float ea[kTcMaxChunks][kTcPx];
   const int tid = threadIdx.x, warp = tid >> 5, grp = tid >> 7, t = tid & 127;
   const PlaneTcProduct& a = g.p[blockIdx.z / g.splits];
   const int mt = blockIdx.y;
@@ -283,48 +297,51 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
   }
   const int nt = g.nt, m0 = mt * nt, kb = (blockIdx.z % g.splits) * a.kper, ke = min(a.K, kb + a.kper);
   const int nch = ke > kb ? (ke - kb + kTcK - 1) / kTcK : 0;
-  uint8_t* Bs = sm + (g.chunks > 1 ? 4 : 2) * kTcPlane;   // [chunk][hi, lo][nt] rows of 128 bytes
+  uint8_t* Bs = sm + 3 * kTcPlane;   // [chunk][plane][nt] rows of 128 bytes
   if (tid == 0) {
-    tc::mbar_init(&done[0], 1);
-    tc::mbar_init(&done[1], 1);
+    tc::mbar_init(&done, 1);
     tc::fence_barrier_init();
   }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, g.cols);
-  rowmax[tid] = 0;
-  __syncthreads();
-  // a sum of one chunk is shared by the groups, half of it (an accumulator of 32 terms) each
-  const bool halved = nch == 1;
-  const int nacc = halved ? (ke - kb > 32 ? 2 : 1) : nch, span = halved ? 32 : kTcK, slot0 = halved ? grp * 4 : 0;
-  // Half a chunk of this thread's pixel at a time, its loads in flight while the half before is worked on.  (cp.async into the
-  // thread's own row is four lanes to a bank, 4 us a chunk; 64 values at once spill, and code that runs once costs its fetch.)
-  constexpr int kHalf = kTcK / 2;
-  const int halves = (span == kTcK ? 2 : 1) * ((nacc - grp + 1) / 2);   // of this group
-  bool qin;
-  int n, p;             // this thread's pixel
-  float v[kHalf];
+  // Values of this thread's pixel, their loads in flight while chunks before them are worked on.  (cp.async into the thread's own
+  // row is four lanes to a bank, 4 us a chunk; 64 values at once spill, and code that runs once costs its fetch.)
+  constexpr int V = kTcK / G, AHEAD = G / 2;
+  struct Pixel {
+    int n, p;
+    bool in;
+  } at, begun;            // this thread's pixel of the chunk whose loads come next, and of the last tile whose loads have begun
+  int next_tile = blockIdx.x, next_c = 0;
   auto pixel = [&](int tile) {
     const int q = tile * kTcPx + t;
-    qin = q < g.Q;
-    n = qin ? q / g.HW : 0;
-    p = qin ? q - n * g.HW : 0;
+    Pixel x;
+    x.in = tile < g.pxtiles && q < g.Q;
+    x.n = x.in ? q / g.HW : 0;
+    x.p = x.in ? q - x.n * g.HW : 0;
+    return x;
   };
-  auto load_half = [&](int u) {
-    const int k0 = span == kTcK ? ((u >> 1) * 2 + grp) * kTcK + (u & 1) * kHalf : grp * kHalf, kn = ke - kb - k0;
-    const float* src = a.in + ((size_t)n * a.K + kb + k0) * g.HW + p;
+  auto load = [&](float (&v)[V]) {
+    const int k0 = next_c * kTcK + grp * V, kn = ke - kb - k0;
+    const float* src = a.in + ((size_t)at.n * a.K + kb + k0) * g.HW + at.p;
 #pragma unroll
-    for (int k = 0; k < kHalf; ++k) v[k] = qin && k < kn ? src[(size_t)k * g.HW] : 0.f;
+    for (int k = 0; k < V; ++k) v[k] = at.in && k < kn ? src[(size_t)k * g.HW] : 0.f;
+    if (next_c == 0) begun = at;
+    if (++next_c >= nch) {
+      next_c = 0;
+      at = pixel(next_tile += gridDim.x);
+    }
   };
-  pixel(blockIdx.x);
-  if (g.first && halves) load_half(0);
-  // ---- F by items of eight k (lanes along the contiguous index): largest magnitude per row, then the planes.  In between the
-  // values wait as fp32 in the 16 bytes of hi and the 16 of lo that they become.
-  const int k8s = nch * (kTcK / 8), along = max(AK ? k8s : nt, 1), dfast = kTcThreads % along, dslow = kTcThreads / along;
+  float v[AHEAD][V];
+  at = begun = pixel(next_tile);
+  if (g.first)
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) load(v[i]);
+  // ---- F by items of eight k (lanes along the contiguous index)
+  const int k8s = nch * (kTcK / 8), along = max(AK ? k8s : nt, 1), dfast = kThreads % along, dslow = kThreads / along;
   const int items = nt * k8s;
-  auto place = [&](int r, int k8) { return Bs + (k8 >> 3) * 2 * nt * 128 + r * 128 + (((k8 & 7) ^ (r & 7)) << 4); };
   {
     constexpr int kBatch = 4;   // items of a thread whose loads are in flight together (one after the other 0.65 us each)
     int fast = tid % along, slow = tid / along;
-    for (int i = tid; i < items; i += kBatch * kTcThreads) {
+    for (int i = tid; i < items; i += kBatch * kThreads) {
       float f[kBatch][8];
       int r[kBatch], k8[kBatch];
 #pragma unroll
@@ -332,7 +349,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
         r[b] = AK ? slow : fast;
         k8[b] = AK ? fast : slow;
         const int m = m0 + r[b], k = kb + k8[b] * 8;
-        const bool in = i + b * kTcThreads < items && m < a.M;
+        const bool in = i + b * kThreads < items && m < a.M;
         const size_t inc = AK ? 1 : a.M;
         const float* src = AK ? a.F + (size_t)m * a.K + k : a.F + (size_t)k * a.M + m;
 #pragma unroll
@@ -343,128 +360,72 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
       }
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
-        if (i + b * kTcThreads >= items) break;
-        unsigned mx = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) mx = max(mx, tc::abs_bits(f[b][j]));
-        uint8_t* d = place(r[b], k8[b]);
-        *reinterpret_cast<float4*>(d) = make_float4(f[b][0], f[b][1], f[b][2], f[b][3]);
-        *reinterpret_cast<float4*>(d + nt * 128) = make_float4(f[b][4], f[b][5], f[b][6], f[b][7]);
-        atomicMax(&rowmax[r[b]], mx);
+        if (i + b * kThreads >= items) break;
+        put8(Bs + (k8[b] >> 3) * 3 * nt * 128 + r[b] * 128 + (((k8[b] & 7) ^ (r[b] & 7)) << 4), nt * 128, f[b]);
       }
     }
-  }
-  __syncthreads();
-  for (int i = tid, fast = tid % along, slow = tid / along; i < items; i += kTcThreads) {
-    const int r = AK ? slow : fast;
-    uint8_t* d = place(r, AK ? fast : slow);
-    split_in_place(d, d + nt * 128, tc::exp2_int(-tc::row_exponent(rowmax[r], tc::kLeast)));
-    fast += dfast;
-    slow += dslow;
-    if (fast >= along) { fast -= along; ++slow; }
-  }
-  if (tid < nt) {   // 2^(24 + e) of a row in two factors
-    const int e = tc::kRowShift + tc::row_exponent(rowmax[tid], tc::kLeast);
-    rowscale[tid] = make_float2(tc::exp2_int(e >> 1), tc::exp2_int(e - (e >> 1)));
   }
   tc::fence_proxy_async();
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  uint8_t *As = sm + (nch > 1 ? grp * 2 * kTcPlane : 0), *row = As + t * 128;
-  const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
-  const uint32_t idesc = tc::make_idesc_f16(nt);
+  const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B), a0 = d0 + (tc::smem_u32(sm) >> 4);
+  const uint32_t idesc = tc::make_idesc_bf16(nt);
   float* sums = reinterpret_cast<float*>(sm);     // [nt][128], for the cluster
-  const int half = grp * (nt / 2);                // the groups read out half of the rows each
   bool fine = true;
-  int commits = 0;                                // of this group
+  int commits = 0;
   grid_dependency_wait();
-  if (!g.first && halves) load_half(0);
+  if (!g.first)
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) load(v[i]);
+  auto chunk = [&](int c, float (&v)[V]) {
+    if (commits) fine = tc::mbar_wait(&done, (commits - 1) & 1) && fine;   // the operand rows are free
+#pragma unroll
+    for (int j = 0; j < V / 8; ++j) put8(sm + t * 128 + (((grp * (V / 8) + j) ^ (t & 7)) << 4), kTcPlane, v + 8 * j);
+    tc::fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      tc::tc_fence_after_sync();
+      mma_chunk(tmem + c * nt, a0, kTcPlane >> 4, d0 + (tc::smem_u32(Bs + c * 3 * nt * 128) >> 4), (uint32_t)nt * 128 >> 4, idesc,
+                (min(kTcK, ke - kb - c * kTcK) + 15) / 16);
+      tc::mma_commit(&done);
+    }
+    load(v);   // (not before the fence, which may wait for them)
+    ++commits;
+  };
   for (int tile = blockIdx.x; tile < g.pxtiles; tile += gridDim.x) {
-    unsigned mx = 0;
-    for (int u = 0; u < halves; ++u) {
-      // c: the chunk's accumulator; the group's buffer is free when the products of its last chunk are done
-      const int c = span == kTcK ? (u >> 1) * 2 + grp : grp;
-      const bool second = span == kTcK && (u & 1);
-      if (!second) {
-        if (c >= 2) fine = tc::mbar_wait(&done[grp], (commits - 1) & 1) && fine;
-        mx = 0;
-      }
-      const int slot = slot0 + (second ? 4 : 0);
-      // the values wait as fp32 in the hi and lo bytes that they become
-#pragma unroll
-      for (int j = 0; j < kHalf / 8; ++j) {
-        uint8_t* d = row + (((slot + j) ^ (t & 7)) << 4);
-        *reinterpret_cast<float4*>(d) = make_float4(v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3]);
-        *reinterpret_cast<float4*>(d + kTcPlane) = make_float4(v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) mx = max(mx, tc::abs_bits(v[8 * j + k]));
-      }
-      if (u + 1 < halves) load_half(u + 1);
-      if (span == kTcK && !second) continue;
-      const int e = tc::row_exponent(mx, tc::kLeastConv);
-      const float sc = tc::exp2_int(-e);
-      ea[c][t] = tc::exp2_int(e - tc::kRowShift);
-#pragma unroll 2
-      for (int j = 0; j < span / 8; ++j) {
-        uint8_t* d = row + (((slot0 + j) ^ (t & 7)) << 4);
-        split_in_place(d, d + kTcPlane, sc);
-      }
-      tc::fence_proxy_async();
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-      if (t == 0) {
-        tc::tc_fence_after_sync();
-        const uint32_t as = tc::smem_u32(As) + slot0 * 16, d = tmem + c * nt;
-        const uint32_t bs = tc::smem_u32(Bs) + (halved ? slot0 * 16 : c * 2 * nt * 128);
-        const uint64_t ah = d0 + (as >> 4), al = d0 + ((as + kTcPlane) >> 4), bh = d0 + (bs >> 4), bl = d0 + ((bs + nt * 128) >> 4);
-        const int kk = (min(span, ke - kb - c * span) + 15) / 16;
-        for (int i = 0; i < kk; ++i) {
-          tc::mma_f16_ss(d, al + i * 2, bh + i * 2, idesc, i > 0);
-          tc::mma_f16_ss(d, ah + i * 2, bl + i * 2, idesc, true);
-        }
-        for (int i = 0; i < kk; ++i) tc::mma_f16_ss(d, ah + i * 2, bh + i * 2, idesc, true);
-        tc::mma_commit(&done[grp]);
-      }
-      ++commits;
+    const Pixel px = AHEAD == 1 || nch > 1 ? begun : pixel(tile);   // (two ahead, tiles of one chunk: the next tile's)
+    for (int c = 0; c < nch; ++c) {
+      if (AHEAD == 1 || !(commits & 1)) chunk(c, v[0]);
+      else chunk(c, v[AHEAD - 1]);
     }
-    float* out = a.out + ((size_t)n * a.M + m0) * g.HW + p;
-    const int rows = g.splits > 1 ? nt : qin ? a.M - m0 : 0;   // to be written
-    if (tile + gridDim.x < g.pxtiles) {   // the next tile's first loads, while the products run
-      pixel(tile + gridDim.x);
-      if (halves) load_half(0);
-    }
-    if (halves) fine = tc::mbar_wait(&done[grp], (commits - 1) & 1) && fine;
+    const int rows = g.splits > 1 ? nt : px.in ? a.M - m0 : 0;   // to be written
+    if (commits) fine = tc::mbar_wait(&done, (commits - 1) & 1) && fine;
     tc::tc_fence_before_sync();
     __syncthreads();
     tc::tc_fence_after_sync();
     if (tile + gridDim.x >= g.pxtiles) grid_launch_dependents();
     // ---- the accumulators of the chunks, 16 rows at a time
-    float* dst = g.splits > 1 ? sums + half * kTcPx + t : out + (size_t)half * g.HW;
     const size_t inc = g.splits > 1 ? kTcPx : g.HW;
-    for (int c0 = half; c0 < half + nt / 2; c0 += 16) {
+    const int first = (grp * nt / G + 15) / 16 * 16, last = ((grp + 1) * nt / G + 15) / 16 * 16;   // rows that the group reads out
+    float* dst = (g.splits > 1 ? sums + t : a.out + ((size_t)px.n * a.M + m0) * g.HW + px.p) + first * inc;
+    for (int c0 = first; c0 < last; c0 += 16) {
       float s[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) s[j] = 0.f;
-      for (int c = 0; c < nacc; ++c) {
+      for (int c = 0; c < nch; ++c) {
         float x[16];
         tc::tmem_ld16(lanes + c * nt + c0, x);
-        const float f = ea[c][t];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) s[j] = fmaf(x[j], f, s[j]);
+        for (int j = 0; j < 16; ++j) s[j] += x[j];
       }
 #pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        const float4 f = *reinterpret_cast<const float4*>(rowscale + c0 + j);
-        const float y0 = s[j] * f.x * f.y, y1 = s[j + 1] * f.z * f.w;
-        if (c0 + j < rows) *dst = y0;
-        dst += inc;
-        if (c0 + j + 1 < rows) *dst = y1;
-        dst += inc;
-      }
+      for (int j = 0; j < 16; ++j, dst += inc)
+        if (c0 + j < rows) *dst = s[j];
     }
     tc::tc_fence_before_sync();
-    __syncthreads();   // the accumulators and ea are free
+    __syncthreads();   // the accumulators are free
     tc::tc_fence_after_sync();
   }
   if (!fine) atomicCAS(&g_planes_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
@@ -477,7 +438,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
   cl.sync();
   const int quads = nt * (kTcPx / 4), share = (quads + g.splits - 1) / g.splits, e0 = (int)cl.block_rank() * share;
   const int e1 = min(quads, e0 + share);
-  for (int i0 = e0 + tid; i0 < e1; i0 += 4 * kTcThreads) {
+  for (int i0 = e0 + tid; i0 < e1; i0 += 4 * kThreads) {
     float4 x[4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) x[b] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -486,13 +447,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) plane_tc_kernel(const __grid_co
       float4 y[4];
 #pragma unroll
       for (int b = 0; b < 4; ++b)
-        y[b] = i0 + b * kTcThreads < e1 ? lds4(from + (size_t)(i0 + b * kTcThreads) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        y[b] = i0 + b * kThreads < e1 ? lds4(from + (size_t)(i0 + b * kThreads) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int b = 0; b < 4; ++b) { x[b].x += y[b].x; x[b].y += y[b].y; x[b].z += y[b].z; x[b].w += y[b].w; }
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const int i = i0 + b * kTcThreads, m = m0 + i / (kTcPx / 4);
+      const int i = i0 + b * kThreads, m = m0 + i / (kTcPx / 4);
       if (i >= e1 || m >= a.M) break;
       const float w[4] = {x[b].x, x[b].y, x[b].z, x[b].w};
 #pragma unroll
@@ -600,9 +561,9 @@ __global__ void __launch_bounds__(kThreads) plane_stencil_kernel(const __grid_co
 // a row at a time: 64 pixels, two per lane, and 4 bytes of each plane per lane.  A chunk of 64 pixels has an accumulator of
 // its own in half of TMEM (two CTAs per SM); once these are used up they are added to totals in registers.
 //
-// What bounds it is the splitting and latency: 64 x 256 14x14 at R = 32 18 us on FFMA, 22 here; 16 x 256 -> 384 27x27 at R = 50
-// (4-byte loads) 34 and 32.  Fp16 pairs with an exponent per row and 64 pixels took 20 and 28, and lost 3e-4 of the result at 7x7 images
-// beside one of 1e9 without gradient.  Three CTAs per SM with half of the TMEM columns each spill (32 -> 48 us).
+// What bounds it is the splitting and latency: 64 x 256 14x14 at R = 32 17.7 us on FFMA, 18.5 here; 16 x 256 -> 384 27x27 at R = 50
+// (4-byte loads) 34.4 and 26.9.  Fp16 pairs with an exponent per row and 64 pixels took 20.8 and 28.5, and lost 3e-4 of the result at 7x7 images
+// beside one of 1e9 without gradient.  Three CTAs per SM with half of the TMEM columns each spill (27x27: half as long again).
 struct PlaneGrad {
   const float* D[2];     // dU, X
   const float* Z[2];     // Z, Zt
@@ -982,22 +943,36 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
     M = std::max(M, g.p[i].M);
     K = std::max(K, g.p[i].K);
   }
-  const int pxt = ceil_div(g.Q, kTcPx), kchunks = ceil_div(K, kTcK);
-  // outputs: half of TMEM, for two CTAs per SM; ranks: all of them in one tile, which reads the channels once
-  const int most = ak ? 256 : 512;
-  g.nt = (int)align_up(std::min(M, 256), 32);
-  auto fit = [&] {
-    g.chunks = ceil_div(kchunks, g.splits);
-    while (std::max(g.chunks, 2) * g.nt > most && g.nt > 32) g.nt = (int)align_up(g.nt / 2, 32);
+  const int pxt = ceil_div(g.Q, kTcPx), kchunks = ceil_div(K, kTcK), widest = (int)align_up(std::min(M, 256), 32);
+  const auto shared = [&](int chunks, int nt) { return 1024 + 3 * (size_t)kTcPlane + (size_t)chunks * 3 * nt * 128; };
+  // outputs of up to 64 ranks: half of TMEM and of shared memory, for two CTAs per SM; ranks: all of them in one tile, which reads
+  // the channels once
+  const bool two = ak && kchunks == 1;
+  const size_t columns = two ? 256 : 512, bytes = two ? 110 * 1024 : di.smem_optin - 256;
+  const auto fits = [&] { return (size_t)g.chunks * g.nt <= columns && shared(g.chunks, g.nt) <= bytes; };
+  const auto narrow = [&](int least) {
+    while (!fits() && g.nt > least) g.nt = (int)align_up(g.nt / 2, 32);
   };
-  g.splits = 1;
-  fit();
+  const auto split = [&](int splits) {
+    g.splits = splits;
+    g.chunks = ceil_div(kchunks, splits);
+    g.nt = widest;
+  };
+  split(1);
+  if (ak) narrow(32);
   long tiles = 0;
   for (int i = 0; i < nprod; ++i) tiles += (long)ceil_div(g.p[i].M, g.nt) * pxt;
-  // a cluster where that leaves no SM idle that has two chunks to do (one per group)
-  while (g.splits < 8 && ceil_div(kchunks, g.splits) > (tiles * g.splits * 2 <= di.sm_count ? 2 : kTcMaxChunks)) g.splits *= 2;
-  g.nt = (int)align_up(std::min(M, 256), 32);
-  fit();
+  // a cluster where that leaves no SM idle that has two chunks to do, and for all ranks in one tile (64 at least where the CTAs of
+  // the pixels would fill the GPU by themselves)
+  int splits = 1;
+  while (splits < 8 && ceil_div(kchunks, splits) > (tiles * splits * 2 <= di.sm_count ? 2 : kTcMaxChunks)) splits *= 2;
+  split(splits);
+  while (!ak) {
+    if (tiles >= di.sm_count) narrow(64);
+    if (fits() || g.splits == 8 || g.chunks == 1) break;
+    split(g.splits * 2);
+  }
+  narrow(32);
   // few pixels: narrower tiles, whose part of F is split and whose sums are stored sooner
   const auto ctas = [&] {
     long n = 0;
@@ -1005,29 +980,30 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
     return n;
   };
   while (g.nt > 32 && ctas() * 2 <= di.sm_count) g.nt = (int)align_up(g.nt / 2, 32);
-  if (g.chunks > kTcMaxChunks) return fail(B200CP_ERR_UNSUPPORTED, "cp planes: %d channels", K);
+  if (g.chunks > kTcMaxChunks || shared(g.chunks, g.nt) > (size_t)di.smem_optin - 256) return fail(B200CP_ERR_UNSUPPORTED, "cp planes: %d channels", K);
   g.maxmt = 0;
   for (int i = 0; i < nprod; ++i) {
     g.p[i].mtiles = ceil_div(g.p[i].M, g.nt);
     g.p[i].kper = g.chunks * kTcK;
     g.maxmt = std::max(g.maxmt, g.p[i].mtiles);
   }
-  for (g.cols = 32; g.cols < std::max(g.chunks, 2) * g.nt;) g.cols *= 2;
+  for (g.cols = 32; g.cols < g.chunks * g.nt;) g.cols *= 2;
   g.pxtiles = pxt;
-  const size_t smem = 1024 + std::max<size_t>((g.chunks > 1 ? 4 : 2) * kTcPlane + (size_t)g.chunks * 2 * g.nt * 128,
-                                              g.splits > 1 ? sizeof(float) * g.nt * kTcPx : 0);
+  const size_t smem = std::max<size_t>(shared(g.chunks, g.nt), g.splits > 1 ? 1024 + sizeof(float) * g.nt * kTcPx : 0);
   // a CTA per tile, or as many as are resident at once and walk the tiles
-  const int per_sm = g.cols > 256 || smem > 100 * 1024 ? 1 : 2;
+  const int per_sm = g.cols > 256 || smem > 111 * 1024 ? 1 : 2;
   const int walkers = g.splits > 1 ? pxt : std::min(pxt, std::max(1, per_sm * di.sm_count / (g.maxmt * nprod)));
   const dim3 grid((unsigned)ceil_div(pxt, ceil_div(pxt, walkers)), g.maxmt, nprod * g.splits);
-#define PLANE_TC(AK)                                                                                                     \
+#define PLANE_TC(AK, G)                                                                                                 \
   do {                                                                                                                  \
     static std::atomic<int> set[64];                                                                                    \
-    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(plane_tc_kernel<AK>), set, (int)smem));            \
-    B200CP_CUDA_OK(launch_cluster(plane_tc_kernel<AK>, grid, dim3(kTcThreads), smem, st, g.splits, programmatic, g));   \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(plane_tc_kernel<AK, G>), set, (int)smem));         \
+    B200CP_CUDA_OK(launch_cluster(plane_tc_kernel<AK, G>, grid, dim3(G * 128), smem, st, g.splits, programmatic, g));   \
   } while (0)
-  if (ak) PLANE_TC(true);
-  else PLANE_TC(false);
+  if (ak && per_sm == 2) PLANE_TC(true, 2);
+  else if (ak) PLANE_TC(true, 4);
+  else if (per_sm == 2) PLANE_TC(false, 2);
+  else PLANE_TC(false, 4);
 #undef PLANE_TC
   B200CP_LAUNCH_OK("plane_tc_kernel");
   return B200CP_OK;
@@ -1040,8 +1016,7 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
 //   convolution 1.23 1.09 1.03    0.97 0.99 0.82     1.06 0.79 0.80     0.92 0.93 0.78  (smaller shapes 0.85 to 0.97)
 //   gradients   1.47 1.48 1.44    1.12 1.05 1.08     1.05 0.93 0.93     1.02 0.94 0.87  (with the two products before them)
 // 17 to 32 ranks: products from 2^28 on (0.85, 0.78, 0.78 up to 2^31, over 40 more shapes).  Below, images of H W a multiple of 4
-// gain nothing (step of 64x256x256x14x14 R = 32 73.5 / 73.5, FFMA last; the error of the outputs against float64 is 1.03 times that of
-// FFMA, above 32 ranks 0.9 times); for the others FFMA loads single floats: steps of 64x512x512x13x13 R = 18 107 / 120,
+// gain nothing (step of 64x256x256x14x14 R = 32 73.5 / 73.5, FFMA last); for the others FFMA loads single floats: steps of 64x512x512x13x13 R = 18 107 / 120,
 // 32x256x256x11x27 R = 31 59 / 69.  Gradients the same: 16x512x512x47x47 R = 20 225 / 242, 64x432x432x18x37 R = 23 262 / 280, but
 // 64x336x96x40x40 R = 23 372 / 337, 16x448x448x52x52 R = 18 261 / 231.
 std::atomic<int> g_planes_tc_test{-1};   // b200cp_test_set_planes

@@ -172,21 +172,6 @@ constexpr int kLeast = -126, kLeastConv = -100;   // 2^-e and (convolutions) 2^(
 
 __device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 constexpr int kRowShift = 24;   // of totals that take a power of two per step: see SplitGemm::ea
-// eight scaled values to 16 bytes of hi and of lo
-__device__ __forceinline__ void split8(const float* v, float sc, uint4& hi, uint4& lo) {
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float a = v[2 * i] * sc, b = v[2 * i + 1] * sc;
-    const __half2 t = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(t);
-    const __half2 r = __floats2half2_rn(a - f.x, b - f.y);
-    h[i] = *reinterpret_cast<const uint32_t*>(&t);
-    l[i] = *reinterpret_cast<const uint32_t*>(&r);
-  }
-  hi = make_uint4(h[0], h[1], h[2], h[3]);
-  lo = make_uint4(l[0], l[1], l[2], l[3]);
-}
 // ---- three bf16 parts -------------------------------------------------------------------------------------------------
 // Two values as three bf16 parts each, x = p[0] + p[1] + p[2] exactly (each part with its own exponent; the last may fall below the
 // smallest float).  The first is cut off, so that no finite value becomes infinite; the other two are rounded, so that what a

@@ -73,4 +73,4 @@ def test_rule_of_the_plane_products(lib_built):
     assert on(64, 256, 256, 51, 51, 32) == 3
     assert on(64, 256, 256, 14, 14, 33) == 3
     assert on(64, 256, 256, 14, 14, 16) == 0
-    assert on(1, 8192, 24, 20, 20, 65) == 3 and on(1, 8193, 24, 20, 20, 65) == 2   # a cluster's sum has 8192 terms
+    assert on(1, 7168, 24, 20, 20, 65) == 3 and on(1, 7169, 24, 20, 20, 65) == 2   # a cluster's sum has 7168 terms

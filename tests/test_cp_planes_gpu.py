@@ -117,9 +117,10 @@ def form(request):
 @pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
 @pytest.mark.parametrize("shape", TC_SHAPES, ids=str)
 def test_both_forms(form, shape):
-    """Every call over planes, in either arithmetic, whatever the rule would take.  Bound: a split product is off by at most 2**-21, its
-    accumulator of 64 terms by 4 * 2**-23 of the partial sums; the rank plane, the stencil and the sum over ranks or pixels follow one
-    another.  In the norm, with random signs, below 4e-7 (measured over drawn shapes: 3e-7, FFMA 6.5e-7)."""
+    """Every call over planes, in either arithmetic, whatever the rule would take.  Bound: six products of three bf16 parts leave out
+    2**-23 of a term at most, an accumulator of 64 terms is cut off by at most 4 * 2**-23 of its partial sums; the rank plane, the
+    stencil and the sum over ranks or pixels follow one another.  In the norm, with random signs, below 4e-7 (measured over drawn
+    shapes: 2.4e-7, FFMA 6.5e-7)."""
     import paralleltnnlayers_b200 as P
     X, dU, K = make(shape, False)
     want = expect(X, dU, K)
@@ -145,7 +146,7 @@ def test_both_forms(form, shape):
 @pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
 @pytest.mark.parametrize("R", [24, 40])
 def test_images_keep_their_own_scale(form, R):
-    """Pixels have their own power of two: an image is as accurate beside any other.  NaN and infinities stay with the pixels that a
+    """An image is as accurate beside any other.  NaN and infinities stay with the pixels that a
     tap reaches."""
     import paralleltnnlayers_b200 as P
     X, dU, K = make((4, 70, 65, 9, 10, R), False)
@@ -168,6 +169,25 @@ def test_images_keep_their_own_scale(form, R):
 
 @pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
 @pytest.mark.parametrize("R", [24, 40])
+@pytest.mark.parametrize("where", ["ranks", "channels"])
+def test_ranks_and_channels_of_any_scale(form, R, where):
+    """The scale of a rank is free to move between the factor matrices, and a channel of any size may have no weight."""
+    import paralleltnnlayers_b200 as P
+    X, dU, K = make((3, 70, 65, 5, 9, R), False)
+    want = expect(X, dU, K)[:2]
+    if where == "ranks":
+        powers = 2.0 ** np.linspace(-40, 40, R).round()
+        K[0], K[1] = (K[0] * powers).astype(np.float32), (K[1] / powers).astype(np.float32)
+    else:
+        X[:, 3], K[1][3], dU[:, 4], K[0][4] = 1e12, 0, 1e12, 0
+        want = expect(X, dU, K)[:2]
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+    for got, ref in zip(P.cp4_conv2d_step(x, du, *k), want):
+        assert np.linalg.norm(got.double().cpu().numpy() - ref) < 1e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
+@pytest.mark.parametrize("R", [24, 40])
 @pytest.mark.parametrize("where", ["input", "gradient"])
 def test_factor_gradients_beside_a_large_sample(form, R, where):
     """An image whose gradient (or input) is zero adds nothing to the factor gradients, however large its input (gradient) is."""
@@ -184,13 +204,13 @@ def test_factor_gradients_beside_a_large_sample(form, R, where):
         assert np.linalg.norm(got.view(ref.shape).double().cpu().numpy() - ref) < 1e-6 * np.linalg.norm(ref)
 
 
-def test_more_than_8192_channels():
-    """The sum over the channels on the tensor cores ends at 8192 channels (ranks); the products take more, on FFMA, in the same
+def test_more_than_7168_channels():
+    """The sum over the channels on the tensor cores ends at 7168 channels (ranks); the products take more, on FFMA, in the same
     launches."""
     import paralleltnnlayers_b200 as P
     from paralleltnnlayers_b200._lib import lib
     launches = []
-    for C in (8192, 8200):
+    for C in (7168, 8200):
         X, dU, K = make((1, C, 24, 7, 7, 65), False)
         x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
         before = lib.b200cp_launch_count()
