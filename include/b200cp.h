@@ -44,15 +44,19 @@ typedef enum b200cp_status {
 
 /* flags: which arithmetic path runs the two channel contractions. */
 enum {
-  B200CP_PATH_AUTO = 0,   /* the fastest fp32-grade path for the shape (mma.sync today)  */
+  B200CP_PATH_AUTO = 0,   /* the fastest fp32-grade path for the shape (mma.sync; with a workspace also FFMA or tcgen05 products
+                           * over whole rank planes, tcgen05 with three bf16 parts per value: 24 bits at any magnitude) */
   B200CP_PATH_SIMT = 1,   /* exact fp32 FFMA                                        */
   B200CP_PATH_TC3X = 2,   /* tcgen05 kind::tf32, 3-term split (fp32-grade accuracy) */
   B200CP_PATH_TC1X = 3,   /* tcgen05 kind::tf32, single pass (about 1e-3 relative)  */
   B200CP_PATH_MMA = 4,    /* warp-level mma.sync tf32, 3-term split (fp32-grade)    */
   B200CP_PATH_MASK = 7,
   /* Reshaped-CP and dense layers, forward and data gradient: the product with the multiplied-out weight may also run on the
-   * tensor cores (scaled fp16 hi / lo operands: 22 bits, sums as accurate as fp32 ones).  Set in the workspace query and in
-   * the call.  Without it these products are FFMA only. */
+   * tensor cores.  Its operands are fp16 hi / lo pairs with one power of two per row: a sample's features (a pixel's channels)
+   * and the weights of an output.  A value keeps 22 bits down to 2^-18 of the largest of its row; smaller ones have an
+   * absolute error of 2^-39 of that (2^-34 in weights of large layers), which matters where the largest adds little to the
+   * result, as a feature of 1e9 whose weights are 1e-9.  Infinities in a row may come out as NaN.  Sums are as accurate as fp32 ones.
+   * Set in the workspace query and in the call.  Without it these products are FFMA only. */
   B200CP_TENSOR_PRODUCTS = 8
 };
 
@@ -283,8 +287,8 @@ size_t b200cp_dense_recompose_workspace_bytes(int order, const int* idims, const
 int b200cp_dense_recompose(int order, const int* idims, const int* odims, int R, const float* const* F, float* M,
                            void* workspace, size_t workspace_bytes, void* stream);
 
-/* Y[b,o] = sum_i X[b,i] M[i,o] (test/benchmark_dense_cp.py:45-48) with fp32-grade results: tcgen05 with three tf32
- * terms where B, I, O fill its tiles, CUDA cores otherwise. */
+/* Y[b,o] = sum_i X[b,i] M[i,o] (test/benchmark_dense_cp.py:45-48) with fp32-grade results: tcgen05 with three bf16
+ * parts per value and six products where B, I, O fill its tiles, CUDA cores otherwise. */
 size_t b200cp_dense_matmul_workspace_bytes(int B, int I, int O);
 int b200cp_dense_matmul(int B, int I, int O, const float* X, const float* M, float* Y, void* workspace,
                         size_t workspace_bytes, void* stream);

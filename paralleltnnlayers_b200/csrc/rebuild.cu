@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float* __restrict_
 }  // namespace
 
 // Y [B][O] = X [B][I] M [I][O]: X is transposed into the scratch, then the product is the flat gradient GEMM
-// (A^T B with K as rows: tcgen05 with three tf32 terms where the shape fills its tiles, CUDA cores otherwise).
+// (A^T B with K as rows: tcgen05 with three bf16 parts per value where the shape fills its tiles, CUDA cores otherwise).
 size_t dense_matmul_scratch_floats(int B, int I, int O) {
   return align_up((size_t)I * B, 64) + dense_grad_scratch_floats(I, B, O, 1, 1, 1, 1);
 }

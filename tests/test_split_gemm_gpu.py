@@ -93,6 +93,20 @@ def test_rcp(case):
     P.device_status()
 
 
+# More tiles than pairs of SMs (74), the last round of them cut in K, and K, M and N that are no multiples of anything.
+MANY_DENSE = [(2100, (7, 9, 5), (13, 11, 15)), (100, (13, 11, 15), (13, 11, 15)), (19001, (7, 9), (7, 10)), (19001, (9, 9), (3, 5))]
+
+
+@pytest.mark.parametrize("case", MANY_DENSE, ids=str)
+def test_dense_more_tiles_than_pairs(case):
+    test_dense(case, 1)
+
+
+@pytest.mark.parametrize("case", [(6, 55, 58, (5, 7), (10, 7)), (2, 9, 7, (13, 15, 3), (13, 7, 11))], ids=str)
+def test_rcp_more_tiles_than_pairs(case):
+    test_rcp(case)
+
+
 def test_rows_keep_their_own_scale():
     """Every row of the batch has its own power of two, so that a row is as accurate beside any other: magnitudes from 1e-30 to
     the largest float.  Infinities and NaN stay in their row."""
@@ -124,6 +138,61 @@ def test_rows_keep_their_own_scale():
     hit[1:4, 2:5] = True
     assert bool(torch.isnan(w[1][:, hit]).all()) and torch.equal(w[1][:, ~hit], v[1][:, ~hit])
     assert torch.equal(w[[0, 2, 3]], v[[0, 2, 3]])
+
+
+def _bound(x, W, least=2.0 ** -39):
+    """Largest error of x W^T (rows: results): 2**-20 of every term, and what values far below the largest of their row may be off."""
+    ax, aW = x.double().abs(), W.double().abs()
+    far = lambda a: least * a.amax(-1, keepdim=True)
+    return 2.0 ** -20 * ax @ aW.T + far(ax) * aW.sum(-1) + ax.sum(-1, keepdim=True) * far(aW).T
+
+
+@pytest.mark.parametrize("power", [10, 17, 30, 40])
+@pytest.mark.parametrize("odims", [(16, 8), (13, 14, 15)])   # the second: the weight written as planes, 2**5 less range
+def test_dense_values_far_below_the_largest(power, odims):
+    """A feature far above the others that has no weight (an output gradient of an output without one), and small weights along the
+    sum: within the stated bound, entry by entry, and unharmed up to 2**17."""
+    import paralleltnnlayers_b200 as P
+    normal = _normal(power)
+    idims = (15, 13, 16)[:len(odims)]
+    least = 2.0 ** -39 if len(odims) == 2 else 2.0 ** -34
+    F = [normal(i, o, 9) * 0.35 for i, o in zip(idims, odims)]
+    I, O = math.prod(idims), math.prod(odims)
+    F[0][1] = 0          # inputs without weight
+    F[0][2] *= 2.0 ** -power
+    F[0][:, 3] = 0       # outputs without weight
+    W = _kron(F).sum(-1)
+    x, dy = normal(40, I), normal(40, O)
+    x[:, I // idims[0] + 2] = 2.0 ** power
+    dy[:, 3 * (O // odims[0]) + 1] = -2.0 ** power
+    y, ref = P.dense_cp(x, *F).double(), x.double() @ W
+    assert bool(((y - ref).abs() <= _bound(x, W.T, least)).all())
+    dx, rdx = P.dense_cp_backward(x, dy, *F)[0].double(), dy.double() @ W.T
+    assert bool(((dx - rdx).abs() <= _bound(dy, W, least)).all())
+    if power <= 17 and len(odims) == 2:
+        assert _rel(y, ref) < REL and _rel(dx, rdx) < REL
+    P.device_status()
+
+
+@pytest.mark.parametrize("power", [10, 17, 30, 40])
+def test_rcp_values_far_below_the_largest(power):
+    import paralleltnnlayers_b200 as P
+    normal = _normal(power)
+    A, S = [normal(8, 8, 9) * 0.3, normal(9, 10, 9) * 0.3], normal(3, 3, 9) * 0.3
+    A[0][1] = 0
+    A[0][2] *= 2.0 ** -power
+    x = normal(2, 72, 6, 7)
+    x[:, 9 + 2] = 2.0 ** power
+    K = torch.einsum("ctr,yxr->tcyx", _kron(A), S.double()).cpu()
+    conv = lambda u, k: torch.nn.functional.conv2d(u, k, padding=1)
+    ref, y = conv(x.double().cpu(), K), P.conv2d_rcp_fused_nchw(x, *A, S).double().cpu()
+    ax = x.double().abs().cpu()
+    far = ax.amax(1, keepdim=True).expand_as(ax)
+    wide = K.abs().amax((1, 2, 3), keepdim=True).expand_as(K)
+    bound = 2.0 ** -20 * conv(ax, K.abs()) + 2.0 ** -39 * (conv(far, K.abs()) + conv(ax, wide))
+    assert bool(((y - ref).abs() <= bound).all())
+    if power <= 17:
+        assert _rel(y, ref) < REL
 
 
 def test_whole_numbers_are_exact():
