@@ -104,7 +104,8 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // channels per pixel speak for them.  From 17 ranks on the fixed cost counts for less with more pixels; up to 16, where a
 // tile kernel holds every rank of its pixels in one tile, more pixels speak for the tile kernels, which then fill the GPU.
 // The lines are the best ones over 520 random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together,
-// ranks 4 to 128), each measured both ways; against the better form of each shape the choice costs 2 % for a convolution or a
+// ranks 4 to 128), each measured both ways, with fp16 pairs in the tensor-core products (three bf16 parts: a step 0.93 to 1.04 times
+// as long); against the better form of each shape the choice costs 2 % for a convolution or a
 // step, 1 % for a layer or the gradients (geometric mean).  Tile or row kernels / products, us:
 //   ranks       4-16    17-32   33-64   65-128   (sums over the shapes: 210, 113, 88, 109)
 //   convolution 3619/3925  2282/2254  4060/2426  12273/3956
@@ -126,7 +127,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (s->Rank <= 16) {
     const double few = ch * std::sqrt((double)s->Rank) / root4;
     switch (use) {
-      case Planes::kConv: return s->Rank > 8 && few >= 130 && s->W % 4;   // (the row stream takes the others)
+      case Planes::kConv: return s->Rank > 8 && few >= 130 && s->W % 4;   // (the row stream or the row bands take the others)
       case Planes::kStep: return few >= 110;
       case Planes::kSaved: return few >= 100;
       case Planes::kFilter: return few >= 42;
@@ -142,7 +143,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
     case Planes::kConv: return past({256, 129, 0}, {2800, 1000, 0});
     case Planes::kStep: return past({200, 0, 0}, {1300, 0, 0});
     case Planes::kSaved:
-      if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // narrow: the stencil's 16-byte rows decide
+      if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // (measured: narrow layers with odd rows lose)
       return past({160, 0, 0}, {2200, 0, 0});
     case Planes::kFilter:
     case Planes::kFilter3: return past({129, 48, 0}, {2200, 490, 0});

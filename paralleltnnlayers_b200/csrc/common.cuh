@@ -296,8 +296,6 @@ int dense_recompose_launch(int order, const int* a, const int* b, int R, const f
                            cudaStream_t st);
 size_t dense_matmul_scratch_floats(int B, int I, int O);
 int dense_matmul_launch(int B, int I, int O, const float* X, const float* M, float* Y, float* scratch, cudaStream_t st);
-// G[e] = sum over splits of P[split][e], in split order
-void sum_splits_launch(const float* P, float* G, size_t n, int splits, cudaStream_t st);
 size_t contract_scratch_floats(int order, const int* cdims, const int* tdims, int R, int taps, bool has_s);
 int contract_factors_launch(int order, const int* cdims, const int* tdims, int R, int taps, const float* const* A,
                             const float* S, const float* G, float* const* dA, float* dS, float* scratch,

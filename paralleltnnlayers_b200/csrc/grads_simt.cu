@@ -225,14 +225,6 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
   G[i] = s;
 }
 
-}  // namespace
-
-void sum_splits_launch(const float* P, float* G, size_t n, int splits, cudaStream_t st) {
-  sum_splits_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P, G, n, splits);
-}
-
-namespace {
-
 constexpr size_t kPlaneAlign = 256;   // of the tensor path's scratch, which follows G
 
 int pick_splits(long tiles, int kunits, int sm_count) {
