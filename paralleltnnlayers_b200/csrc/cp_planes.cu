@@ -840,43 +840,67 @@ __global__ void __launch_bounds__(kThreads) plane_grad_kernel(const __grid_const
 }
 
 // ---- the sums of the partials, in a fixed order ----------------------------------------------------------------------------
-// 32 entries x 8 groups of partials per CTA; the last CTAs turn the correlation sums into the spatial factors' gradients.
+// EPT x 32 entries x 8 groups of partials per CTA; the last CTAs turn the correlation sums into the spatial factors' gradients.
+// What bounds it is the latency of its reads (9.7 MB from L2 for 512 + 512 channels at R = 64), so a thread has four partials of
+// each of its entries in flight, and a CTA of the correlations two partials of all nine taps: tap after tap with a barrier each it ran for
+// 20.7k cycles where the others had left after 6.2k (64 x 256 14x14 at R = 32).  Steps: that one 66.1 -> 63.0 us, 21 x 64 7x7 at R = 81
+// 27.9 -> 24.1.
 struct PlaneReduce {
   const float* part;     // [splits][entries]
   const float* sums;     // [chunks][9][R]
   const float *KH, *KW;  // null: the free core, whose gradient is the sums themselves
   float* dK;
-  int entries, splits, chunks, R, eblocks;
+  int entries, splits, chunks, R, rblocks;
 };
+template <int EPT>
 __global__ void __launch_bounds__(256) plane_reduce_kernel(const PlaneReduce g) {
-  __shared__ float red[8][32];
-  __shared__ float tap[9][32];
+  __shared__ float red[8][9][32];
   const int x = threadIdx.x, y = threadIdx.y;
   grid_dependency_wait();
-  auto sum = [&](const float* src, size_t stride, int n, bool in) {
-    float v = 0.f;
-    if (in)
-#pragma unroll 4
-      for (int s = y; s < n; s += 8) v += src[(size_t)s * stride];
-    __syncthreads();
-    red[y][x] = v;
-    __syncthreads();
-    if (y == 0)
+  if ((int)blockIdx.x >= g.rblocks) {   // (the correlations take longest and come first)
+    const int e0 = ((int)blockIdx.x - g.rblocks) * 32 * EPT + x;
+    float v[EPT];
 #pragma unroll
-      for (int k = 1; k < 8; ++k) v += red[k][x];
-    return v;
-  };
-  if ((int)blockIdx.x < g.eblocks) {
-    const int e = blockIdx.x * 32 + x;
-    const float v = sum(g.part + e, g.entries, g.splits, e < g.entries);
-    if (y == 0 && e < g.entries) g.dK[e] = v;
+    for (int i = 0; i < EPT; ++i) v[i] = 0.f;
+#pragma unroll 4
+    for (int s = y; s < g.splits; s += 8) {
+      const float* src = g.part + (size_t)s * g.entries + e0;
+#pragma unroll
+      for (int i = 0; i < EPT; ++i)
+        if (e0 + i * 32 < g.entries) v[i] += src[i * 32];
+    }
+#pragma unroll
+    for (int i = 0; i < EPT; ++i) red[y][i][x] = v[i];
+    __syncthreads();
+    if (y < EPT && e0 + y * 32 < g.entries) {
+      float t = red[0][y][x];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) t += red[k][y][x];
+      g.dK[e0 + y * 32] = t;
+    }
     return;
   }
-  const int r = ((int)blockIdx.x - g.eblocks) * 32 + x;
+  const int r = (int)blockIdx.x * 32 + x;
   const bool in = r < g.R;
-  for (int i = 0; i < 9; ++i) {
-    const float v = sum(g.sums + (size_t)i * g.R + r, (size_t)9 * g.R, g.chunks, in);
-    if (y == 0) tap[i][x] = v;
+  float v[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) v[i] = 0.f;
+  if (in)
+#pragma unroll 2
+    for (int s = y; s < g.chunks; s += 8) {
+      const float* src = g.sums + (size_t)s * 9 * g.R + r;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) v[i] += src[(size_t)i * g.R];
+    }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) red[y][i][x] = v[i];
+  __syncthreads();
+  float (&tap)[9][32] = red[0];
+  for (int i = y; i < 9; i += 8) {
+    float t = red[0][i][x];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) t += red[k][i][x];
+    tap[i][x] = t;
   }
   __syncthreads();
   if (!in) return;
@@ -1205,8 +1229,12 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   PlaneReduce r{};
   r.part = b.part; r.sums = b.sums; r.KH = j.KC ? nullptr : j.KH; r.KW = j.KW; r.dK = j.dK;
   r.entries = (T + C) * R; r.splits = gp.splits; r.chunks = gp.chunks; r.R = R;
-  r.eblocks = ceil_div(r.entries, 32);
-  B200CP_CUDA_OK(launch_kernel(plane_reduce_kernel, dim3(r.eblocks + ceil_div(R, 32)), dim3(32, 8), 0, st, true, r));
+  r.rblocks = ceil_div(R, 32);
+  // four entries per thread where that leaves every SM two CTAs
+  if (r.entries >= 128 * 2 * di.sm_count)
+    B200CP_CUDA_OK(launch_kernel(plane_reduce_kernel<4>, dim3(r.rblocks + ceil_div(r.entries, 128)), dim3(32, 8), 0, st, true, r));
+  else
+    B200CP_CUDA_OK(launch_kernel(plane_reduce_kernel<1>, dim3(r.rblocks + ceil_div(r.entries, 32)), dim3(32, 8), 0, st, true, r));
   B200CP_LAUNCH_OK("plane_reduce_kernel");
   return B200CP_OK;
 }

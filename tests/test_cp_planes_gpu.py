@@ -19,6 +19,7 @@ SHAPES = [
     (2, 255, 257, 8, 8, 33), (64, 256, 256, 7, 7, 17), (3, 300, 212, 6, 6, 32), (1, 512, 64, 9, 9, 16),
     (4, 500, 12, 5, 13, 3), (2, 12, 500, 11, 6, 5), (33, 64, 64, 23, 23, 40), (1, 4, 4, 64, 64, 128),
     (12, 64, 70, 28, 28, 40),   # only the backward over planes, from the plane another kernel wrote
+    (2, 291, 301, 5, 5, 64), (1, 300, 303, 6, 5, 63),   # four gradient entries per thread in the last sum: full blocks, and a ragged end
 ]
 
 
