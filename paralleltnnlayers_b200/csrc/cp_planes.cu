@@ -1066,6 +1066,21 @@ PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
   return {sums && (s.Rank > 64 || macs >= 1.3e8), macs >= 1.3e8};
 }
 
+// Units of a CTA of the stencil with correlations: whole turns of its threads, as many as make one to four waves of the five CTAs
+// that an SM has registers for the shortest, where a CTA costs one turn more.  (Eight CTAs per SM and ranges that end
+// within a turn: 32 images of 28x28 at R = 56 took three turns in each of two waves for 2.2 turns of work.  Layer of 16 x 256 -> 384
+// 27x27 at R = 50 95.1 -> 92.5 us; the stencils alone gain nothing.)
+int stencil_range(int units, int R, int sm_count) {
+  const int turns = ceil_div(units, kThreads), resident = 5 * sm_count;
+  long best = 0;
+  int m = 1;
+  for (int waves = 1; waves <= 4; ++waves) {
+    const int k = ceil_div(turns, std::max(1, std::min(waves * resident / R, 65535)));
+    const long cost = (long)ceil_div(R * ceil_div(turns, k), resident) * (k + 1);
+    if (best == 0 || cost < best) { best = cost; m = k; }
+  }
+  return m * kThreads;
+}
 struct GradPlan {
   bool tc;
   int bm, bn, mt0, mt1, rtiles, splits, per;   // gradient products
@@ -1087,8 +1102,7 @@ GradPlan grad_plan(const b200cp_tensor_shape& s, int sm_count) {
   p.per = (int)align_up((size_t)ceil_div(Q, want), p.tc ? kTcK : kDK);
   p.splits = ceil_div(Q, p.per);
   p.units = (int)s.N * ceil_div((int)s.H, 4) * (int)s.W;
-  const int cw = std::max(1, std::min({ceil_div(8 * sm_count, R), ceil_div(p.units, kThreads), 65535}));
-  p.cper = ceil_div(p.units, cw);
+  p.cper = stencil_range(p.units, R, sm_count);
   p.chunks = ceil_div(p.units, p.cper);
   return p;
 }
@@ -1192,7 +1206,8 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
     int k = 0;
     if (fwd) { t.src[k] = P; t.dst[k] = b.Z; t.flip[k++] = 0; }
     if (bwd) { t.src[k] = Q; t.dst[k] = b.Zt; t.flip[k++] = 1; }
-    B200CP_CUDA_OK(launch_kernel(plane_stencil_kernel<false>, dim3(R, gp.chunks, k), dim3(kThreads), 0, st, chained, t));
+    t.per = ceil_div(t.units, std::max(1, std::min({ceil_div(8 * di.sm_count, R), ceil_div(t.units, kThreads), 65535})));
+    B200CP_CUDA_OK(launch_kernel(plane_stencil_kernel<false>, dim3(R, ceil_div(t.units, t.per), k), dim3(kThreads), 0, st, chained, t));
   }
   B200CP_LAUNCH_OK("plane_stencil_kernel");
   np = 0;
