@@ -237,7 +237,10 @@ __global__ void __launch_bounds__(kThreads) plane_gemm_kernel(const __grid_const
 // its own accumulator in TMEM (chunks x rows <= 512 columns); at the end they are added up.  F is split once per CTA,
 // which then walks the pixel tiles; where the pixels alone leave SMs idle the sum is split over a cluster instead.
 //
-// What bounds it is latency: a chunk's loads 1 to 2 us, its products 0.5, a commit 0.3, the split of F 1 to 3.  Both products of
+// What bounds it is latency: before the first chunk 2.6 us (loads, split of F), per chunk 1.5 (0.5 of loads and splitting, 1.0 of products
+// up to their commit), 1 for the read-out.  One elected lane issues the products, once the warp's next loads are on their way: the whole
+// layer of 64 x 512 7x7 at R = 64 64.3 -> 61.9 us, 32 x 128 28x28 at R = 56 88.4 -> 84.5.  (A warp of its own for the issue: chunks of
+// 1.2 us, but 96 registers instead of 125, and all else took as much longer.)  Both products of
 // 64 x 256 14x14 at R = 32: P and Q 21.9 us on FFMA, 20.2 here, the outputs 18.2 and 17.0; of 16 x 256 -> 384 27x27 at R = 50: 53.9 and
 // 36.8, 44.4 and 25.0.  Fp16 pairs with an exponent per pixel and chunk took 19.6, 16.4, 36.0 and 23.8, and lost the result where a
 // rank is scaled up in one factor and down in another (R = 24, by 2^-40 to 2^40).  Error against float64 over 60 drawn shapes 0.7
@@ -268,17 +271,21 @@ __device__ __forceinline__ void put8(uint8_t* d, uint32_t plane, const float* v)
   for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(d + q * plane) = make_uint4(w[0].p[q], w[1].p[q], w[2].p[q], w[3].p[q]);
 }
 // the six products of a chunk of 16 kk terms, the smallest first
-__device__ __forceinline__ void mma_chunk(uint32_t d, uint64_t a, uint64_t A1, uint64_t b, uint64_t B1, uint32_t idesc, int kk) {
-  for (int i = 0; i < kk; ++i) {
+template <int KK>
+__device__ __forceinline__ void mma_chunk(uint32_t d, uint64_t a, uint64_t A1, uint64_t b, uint64_t B1, uint32_t idesc) {
+#pragma unroll
+  for (int i = 0; i < KK; ++i) {
     tc::mma_f16_ss(d, a + 2 * A1 + i * 2, b + i * 2, idesc, i > 0);
     tc::mma_f16_ss(d, a + i * 2, b + 2 * B1 + i * 2, idesc, true);
     tc::mma_f16_ss(d, a + A1 + i * 2, b + B1 + i * 2, idesc, true);
   }
-  for (int i = 0; i < kk; ++i) {
+#pragma unroll
+  for (int i = 0; i < KK; ++i) {
     tc::mma_f16_ss(d, a + A1 + i * 2, b + i * 2, idesc, true);
     tc::mma_f16_ss(d, a + i * 2, b + B1 + i * 2, idesc, true);
   }
-  for (int i = 0; i < kk; ++i) tc::mma_f16_ss(d, a + i * 2, b + i * 2, idesc, true);
+#pragma unroll
+  for (int i = 0; i < KK; ++i) tc::mma_f16_ss(d, a + i * 2, b + i * 2, idesc, true);
 }
 
 template <bool AK, int G>
@@ -288,7 +295,7 @@ __global__ void __launch_bounds__(G * 128, 4 / G) plane_tc_kernel(const __grid_c
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, grp = tid >> 7, t = tid & 127;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), grp = tid >> 7, t = tid & 127;
   const PlaneTcProduct& a = g.p[blockIdx.z / g.splits];
   const int mt = blockIdx.y;
   if (mt >= a.mtiles) {     // (the other product of the launch has more row tiles; a whole cluster leaves)
@@ -385,13 +392,17 @@ __global__ void __launch_bounds__(G * 128, 4 / G) plane_tc_kernel(const __grid_c
     for (int j = 0; j < V / 8; ++j) put8(sm + t * 128 + (((grp * (V / 8) + j) ^ (t & 7)) << 4), kTcPlane, v + 8 * j);
     tc::fence_proxy_async();
     __syncthreads();
-    if (tid == 0) {
+    load(v);   // (not before the fence, which may wait for them; but before the products, whose issue takes longer than a load)
+    if (warp == 0 && tc::elect_one()) {
       tc::tc_fence_after_sync();
-      mma_chunk(tmem + c * nt, a0, kTcPlane >> 4, d0 + (tc::smem_u32(Bs + c * 3 * nt * 128) >> 4), (uint32_t)nt * 128 >> 4, idesc,
-                (min(kTcK, ke - kb - c * kTcK) + 15) / 16);
+      const uint32_t d = tmem + c * nt, B1 = (uint32_t)nt * 128 >> 4;
+      const uint64_t b0 = d0 + (tc::smem_u32(Bs + c * 3 * nt * 128) >> 4);
+      const int left = ke - kb - c * kTcK;
+      if (left > 32) mma_chunk<4>(d, a0, kTcPlane >> 4, b0, B1, idesc);
+      else if (left > 16) mma_chunk<2>(d, a0, kTcPlane >> 4, b0, B1, idesc);
+      else mma_chunk<1>(d, a0, kTcPlane >> 4, b0, B1, idesc);
       tc::mma_commit(&done);
     }
-    load(v);   // (not before the fence, which may wait for them)
     ++commits;
   };
   for (int tile = blockIdx.x; tile < g.pxtiles; tile += gridDim.x) {
@@ -590,7 +601,7 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = warp >> 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), grp = warp >> 2;
   const int rt = blockIdx.x % g.rtiles, mi = blockIdx.x / g.rtiles, half = mi >= g.mtiles[0] ? 1 : 0;
   const int m0 = (mi - (half ? g.mtiles[0] : 0)) * kGradRows, r0 = rt * NT, rows = half ? g.rows[1] : g.rows[0];
   const int qb = blockIdx.y * g.per, qe = min(g.Q, qb + g.per);
@@ -672,24 +683,10 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
     }
     tc::fence_proxy_async();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && tc::elect_one()) {
       tc::tc_fence_after_sync();
-      const uint32_t as = tc::smem_u32(sm), d = tmem + c * NT;
-      const uint64_t a0 = d0 + (as >> 4), b0 = d0 + ((as + 3 * kTcPlane) >> 4);
-      constexpr uint64_t A1 = kTcPlane >> 4, B1 = T::bplane >> 4;
-#pragma unroll
-      for (int i = 0; i < kTcK / 16; ++i) {   // the products of 2^-16 first
-        tc::mma_f16_ss(d, a0 + 2 * A1 + i * 2, b0 + i * 2, idesc, i > 0);
-        tc::mma_f16_ss(d, a0 + i * 2, b0 + 2 * B1 + i * 2, idesc, true);
-        tc::mma_f16_ss(d, a0 + A1 + i * 2, b0 + B1 + i * 2, idesc, true);
-      }
-#pragma unroll
-      for (int i = 0; i < kTcK / 16; ++i) {
-        tc::mma_f16_ss(d, a0 + A1 + i * 2, b0 + i * 2, idesc, true);
-        tc::mma_f16_ss(d, a0 + i * 2, b0 + B1 + i * 2, idesc, true);
-      }
-#pragma unroll
-      for (int i = 0; i < kTcK / 16; ++i) tc::mma_f16_ss(d, a0 + i * 2, b0 + i * 2, idesc, true);
+      const uint32_t as = tc::smem_u32(sm);
+      mma_chunk<kTcK / 16>(tmem + c * NT, d0 + (as >> 4), kTcPlane >> 4, d0 + ((as + 3 * kTcPlane) >> 4), T::bplane >> 4, idesc);
       tc::mma_commit(&done);
     }
     if (c + 1 < T::chunks && s + 1 < steps) continue;
