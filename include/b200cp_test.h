@@ -51,7 +51,9 @@ long long b200cp_test_stream_launches(void);
  * (by the rule unless set).  A workspace query and its call want the same setting.  Process-wide. */
 void b200cp_test_set_planes(int planes, int tensor_cores);
 
-/* Which plane products run on the tensor cores for a shape (3x3, pad 1): bit 0 the channel products, bit 1 the factor gradients. */
+/* Which plane products run on the tensor cores by the size of a shape alone (3x3, pad 1): bit 0 the channel products of one
+ * convolution, bit 1 the factor gradients.  Two convolutions in one launch, and gradients of images of a multiple of 4 pixels, have
+ * lines of their own beside these. */
 int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s);
 
 /* Diagnostics: the row-band kernel writes 64 cycle stamps (long long) per CTA for its first 512 CTAs into this

@@ -1052,39 +1052,54 @@ int tc_launch(PlaneTc g, int nprod, bool ak, bool programmatic, const DeviceInfo
   return B200CP_OK;
 }
 
-// Which kernels form the products and the gradients: lines in multiply-adds (pixels x ranks x channels) per rank class, over 520
-// random shapes measured both ways.  Tensor cores / FFMA, geometric mean over the shapes between 2^26 and 2^27, 2^27 and 2^28,
-// 2^28 and 2^29 multiply-adds:
-//              ranks 4-16         17-32              33-64              65-128
-//   convolution 1.23 1.09 1.03    0.97 0.99 0.82     1.06 0.79 0.80     0.92 0.93 0.78  (smaller shapes 0.85 to 0.97)
-//   gradients   1.47 1.48 1.44    1.12 1.05 1.08     1.05 0.93 0.93     1.02 0.94 0.87  (with the two products before them)
-// 17 to 32 ranks: products from 2^28 on (0.85, 0.78, 0.78 up to 2^31, over 40 more shapes).  Below, images of H W a multiple of 4
-// gain nothing (step of 64x256x256x14x14 R = 32 73.5 / 73.5, FFMA last); for the others FFMA loads single floats: steps of 64x512x512x13x13 R = 18 107 / 120,
-// 32x256x256x11x27 R = 31 59 / 69.  Gradients the same: 16x512x512x47x47 R = 20 225 / 242, 64x432x432x18x37 R = 23 262 / 280, but
-// 64x336x96x40x40 R = 23 372 / 337, 16x448x448x52x52 R = 18 261 / 231.
+// Which kernels form the products and the gradients: lines in multiply-adds (pixels x ranks x channels) per rank class, over 1300
+// random shapes (1 to 64 images of 7x7 to 64x64, 16 to 512 channels) measured both ways.  Where H W is no multiple of 4, FFMA loads
+// single floats.  Tensor cores / FFMA, geometric means of convolutions between these powers of two of multiply-adds:
+//               20-22 22-23 23-25 25-26 26-27 27-28 28-29 29-32
+//   17-32, x 4   1.17  1.09  1.14  1.06  1.08  0.92  0.89  0.84       others  1.07  1.04  1.02  0.98  0.84  0.80  0.75  0.76
+//   33-64, x 4   1.14  1.00  1.04  0.96  0.93  0.93  0.77  0.73       others  0.97  0.93  0.91  0.90  0.85  0.78  0.67  0.64
+//   65-128       0.88  0.84  0.86  0.75  0.78  0.82  0.79  0.68       9-16, x 4  1.05 to 1.41, others  0.80 (from 2^29) to 1.25
+// Gradients, steps with them on the tensor cores / on FFMA: 33-64 ranks 0.87 to 1.01, 65-128 0.83 to 1.02, 9-16 1.00 to 1.06.  17-32
+// ranks: those with 16-byte loads 0.91 to 0.96 at any size (grads_by_quads), with 4-byte loads 0.91 from 2^29 on.
 std::atomic<int> g_planes_tc_test{-1};   // b200cp_test_set_planes
 struct PlanesOn {
   bool products, gradients;   // on the tensor cores
 };
-PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
-  static const int env = [] {   // B200CP_PLANES_TC: 0 FFMA, 2 tensor cores, else by the rule
+int planes_tc_mode() {   // B200CP_PLANES_TC: 0 FFMA, 2 tensor cores, else by the rules
+  static const int env = [] {
     const char* e = getenv("B200CP_PLANES_TC");
     return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
   }();
-  const int forced = g_planes_tc_test.load(std::memory_order_relaxed), mode = forced < 0 ? env : forced;
+  const int forced = g_planes_tc_test.load(std::memory_order_relaxed);
+  return forced < 0 ? env : forced;
+}
+// by the shape alone: one convolution, and gradients whatever their rows
+PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
+  const int mode = planes_tc_mode();
   // a sum in a cluster of eight; FFMA has no such limit
   const bool sums = std::max({s.T, s.C, s.Rank}) <= 8u * kTcMaxChunks * kTcK;
   if (mode != 1) return {mode == 2 && sums, mode == 2};
   const double macs = (double)s.N * s.H * s.W * s.Rank * ((double)s.C + s.T);
   if (s.Rank <= 16) return {false, false};
-  if (s.Rank <= 32) {
-    const bool single = (size_t)s.H * s.W % 4 != 0;
-    return {sums && macs >= (single ? 1e8 : 268435456.0), macs >= 1e9 && single};
-  }
-  if (s.Rank > 64 && s.C + s.T <= 32) return {false, false};   // half of a K stage is padding: a step 1.01 to 1.28 times as long
-  return {sums && (s.Rank > 64 || macs >= 1.3e8), macs >= 1.3e8};
+  const bool single = (size_t)s.H * s.W % 4 != 0;
+  if (s.Rank <= 32) return {sums && macs >= (single ? 1e8 : 268435456.0), macs >= 1e9 && single};
+  // few channels: half of a K stage is padding (C + T up to 32: a step 1.01 to 1.28 times as long; 33 to 64 at 33 to 64 ranks 1.00 to
+  // 1.06 with 16-byte loads, 0.94 to 0.98 without, above that 0.73 to 1.01)
+  if (s.Rank > 64 && s.C + s.T <= 32) return {false, false};
+  return {sums && s.C + s.T > (s.Rank > 64 || single ? 32u : 64u), true};
 }
-
+// Gradients with 16-byte loads (plane_grad_tc_kernel<.., true>; the few buffers that are not aligned have 4-byte loads there)
+bool grads_by_quads(const b200cp_tensor_shape& s) {
+  return planes_tc_mode() == 1 && s.Rank > 16 && (size_t)s.H * s.W % 4 == 0 && (s.Rank <= 64 || s.C + s.T > 32);
+}
+// Two products of about as many channels in one launch (a step) fill the GPU earlier than one does: 17 to 32 ranks, H W a multiple
+// of 4, at least 96 channels, steps between 2^26 and 2^28 multiply-adds 0.84 to 0.98 times as long (64 x 256 14x14 at R = 32
+// 55.6 -> 49.8 us).  Where one has more than 1.5 times the channels of the other, up to 1.25 times.
+bool even_products_on_tensor_cores(const b200cp_tensor_shape& s) {
+  const double most = std::max(s.C, s.T), least = std::min(s.C, s.T);
+  return planes_tc_mode() == 1 && s.Rank > 16 && s.Rank <= 32 && (size_t)s.H * s.W % 4 == 0 && least >= 96 && most <= 1.5 * least &&
+         most <= 8.0 * kTcMaxChunks * kTcK && (double)s.N * s.H * s.W * s.Rank * (most + least) >= 67108864.0;
+}
 // Units of a CTA of the stencil with correlations: whole turns of its threads, as many as make one to four waves of the five CTAs
 // that an SM has registers for the shortest, where a CTA costs one turn more.  (Eight CTAs per SM and ranges that end
 // within a turn: 32 images of 28x28 at R = 56 took three turns in each of two waves for 2.2 turns of work.  Layer of 16 x 256 -> 384
@@ -1108,7 +1123,7 @@ struct GradPlan {
 GradPlan grad_plan(const b200cp_tensor_shape& s, int sm_count) {
   GradPlan p{};
   const int R = (int)s.Rank, Q = (int)(s.N * s.H * s.W);
-  p.tc = planes_on_tensor_cores(s).gradients;
+  p.tc = planes_on_tensor_cores(s).gradients || grads_by_quads(s);
   p.bn = !p.tc && R <= 16 ? 16 : R <= 32 ? 32 : 64;
   p.bm = p.tc || p.bn < 64 ? 128 : 64;
   p.mt0 = ceil_div((int)s.T, p.bm);
@@ -1190,9 +1205,9 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   g.HW = HW;
   g.Q = NQ;
   int np = 0;
-  const bool tc = planes_on_tensor_cores(s).products;
+  const bool one = planes_on_tensor_cores(s).products, two = one || even_products_on_tensor_cores(s);
   auto products = [&](bool ak, bool programmatic) {
-    if (tc) {
+    if (np == 2 ? two : one) {
       g.first = !programmatic;
       return tc_launch(g, np, ak, programmatic, di, st);
     }
