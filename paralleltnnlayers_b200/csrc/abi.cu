@@ -103,16 +103,15 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // dependent launches (about 20 us for a convolution), and after that cost little per rank and channel.  More ranks and
 // channels per pixel speak for them.  From 17 ranks on the fixed cost counts for less with more pixels; up to 16, where a
 // tile kernel holds every rank of its pixels in one tile, more pixels speak for the tile kernels, which then fill the GPU.
-// The lines are the best ones over 520 random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together,
-// ranks 4 to 128), each measured both ways, with fp16 pairs in the tensor-core products (three bf16 parts: a step 0.93 to 1.04 times
-// as long); against the better form of each shape the choice costs 2 % for a convolution or a
-// step, 1 % for a layer or the gradients (geometric mean).  Tile or row kernels / products, us:
-//   ranks       4-16    17-32   33-64   65-128   (sums over the shapes: 210, 113, 88, 109)
-//   convolution 3619/3925  2282/2254  4060/2426  12273/3956
-//   step        10289/10705  7209/6075  14375/7043  33665/12089
-//   gradients   9198/7498  6696/4748  13028/5473  24193/9483
-//   layer       12490/12711  8184/7419  15888/7943  37391/13645
-//   layer (3)   17362/12654  11210/7385  21503/7925  48043/13615
+// The lines are the best ones over random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together, ranks 4 to
+// 128), each measured both ways as calls one after the other: 520 for the backward from a saved plane and the layers, 1500 for the
+// others.  Up to 16 ranks a width that is a multiple of 4 has a row kernel (of these the row stream only loses by the channels), others
+// do not.  Time against the better form of each shape, geometric means, with the lines before (no convolution of W % 4 == 0 up to 16
+// ranks, steps of 17 to 32 ranks by channels, ...) / with these:
+//                 R 4-8, x 4   others       9-16, x 4    others       17-32, x 4   others       33-64, x 4   others
+//   convolution   1.17 / 1.02  1.03 / 1.03  1.18 / 1.02  1.03 / 1.03  1.02 / 1.01  1.02 / 1.01  1.02 / 1.01  1.02 / 1.01
+//   step          1.04 / 1.02  1.06 / 1.05  1.02 / 1.02  1.07 / 1.02  1.11 / 1.00  1.05 / 1.01  1.00         1.00
+//   gradients     1.07 / 1.04  1.04 / 1.02  1.02 / 1.02  1.01 / 1.01  1.05 / 1.01  1.03 / 1.01  1.01         1.01
 const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
   return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
@@ -126,11 +125,13 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   const double ch = (double)s->C + s->T, root4 = std::sqrt(std::sqrt((double)s->N * s->H * s->W));
   if (s->Rank <= 16) {
     const double few = ch * std::sqrt((double)s->Rank) / root4;
+    const bool low = s->Rank <= 8, rows = s->W % 4 == 0 && band_max_rank() == 16;   // (a caller who sets it wants the row bands)
+    const bool streams = s->W % 16 == 8 && s->W <= 56 && s->C % 8 == 0 && s->T % 8 == 0;   // widths of the row stream
     switch (use) {
-      case Planes::kConv: return s->Rank > 8 && few >= 130 && s->W % 4;   // (the row stream or the row bands take the others)
-      case Planes::kStep: return few >= 110;
+      case Planes::kConv: return rows ? (streams ? ch >= 280 : few >= (low ? 64 : 96)) : !low && few >= 130 && s->W % 4;
+      case Planes::kStep: return few >= (low ? 60 : s->W % 4 == 0 ? 110 : 20);
       case Planes::kSaved: return few >= 100;
-      case Planes::kFilter: return few >= 42;
+      case Planes::kFilter: return few >= (low ? 20 : 46);
       case Planes::kFilter3: return few >= 47;
       default: return ch >= 64 && few >= 27;
     }
@@ -140,12 +141,12 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
     return ch >= least[ranks] || ch * root4 >= weighted[ranks];
   };
   switch (use) {
-    case Planes::kConv: return past({256, 129, 0}, {2800, 1000, 0});
-    case Planes::kStep: return past({200, 0, 0}, {1300, 0, 0});
+    case Planes::kConv: return past({224, 100, 0}, {2800, 900, 0});
+    case Planes::kStep: return true;
     case Planes::kSaved:
       if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // (measured: narrow layers with odd rows lose)
       return past({160, 0, 0}, {2200, 0, 0});
-    case Planes::kFilter:
+    case Planes::kFilter: return past({80, 48, 0}, {800, 490, 0});
     case Planes::kFilter3: return past({129, 48, 0}, {2200, 490, 0});
     default: return past({129, 40, 0}, {2200, 400, 0});
   }

@@ -111,6 +111,7 @@ int cp4_mma_launch(const Cp4Args& a, cudaStream_t st);
 // convolutions of the same image size in one launch.  *done = false: not a shape this kernel takes.
 int cp4_band_launch(const Cp4Args* convs, int nconv, cudaStream_t st, bool* done);
 int band_device_status(int* out);
+int band_max_rank();   // 16 unless it was set
 // Row stream (one persistent CTA per SM; 3x3, pad 1, W a multiple of 8 that is 8 or 24 modulo 32, at most 16 ranks,
 // input channels a multiple of 8, at most 256): the same contract as cp4_band_launch.
 int cp4_stream_launch(const Cp4Args* convs, int nconv, cudaStream_t st, bool* done);

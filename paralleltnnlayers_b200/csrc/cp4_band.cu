@@ -978,6 +978,7 @@ int band_tensor_map(const float* ptr, int N, int C, int H, int W, int rows, int 
   return band_map(ptr, N, C, H, W, rows, cb, out);
 }
 
+int band_max_rank() { return g_band_max_rank.load(std::memory_order_relaxed); }
 void band_set_max_rank(int r) { g_band_max_rank.store(std::max(1, std::min(32, r))); }
 void band_force_rows(int rows) { g_band_th.store(rows > 0 ? rows : 0); }
 void band_force_tensor(int on) { g_band_tensor.store(on ? 1 : 0); }
