@@ -8,8 +8,9 @@
 namespace b200cp {
 
 // ---- sum of a cluster's partial tiles ----------------------------------------------------------------------------------
-// Every CTA of the cluster has left its partial tile in shared memory; CTA q adds slice q of all of them in CTA order
-// (the result does not depend on scheduling) and hands each sum to `put`.
+// Every CTA of the cluster (at most 8) has left its partial tile in shared memory; CTA q adds slice q of all of them in CTA order
+// (the result does not depend on scheduling) and hands each sum to `put`.  All CTAs are read at once: a read of another CTA's memory
+// takes half a microsecond.
 template <typename Put>
 __device__ __forceinline__ void cluster_sum(float* tile, int n, int splits, int tid, int nthreads, Put put) {
   namespace cg = cooperative_groups;
@@ -22,9 +23,17 @@ __device__ __forceinline__ void cluster_sum(float* tile, int n, int splits, int 
   cl.sync();
   const int q = (int)cl.block_rank(), per = (n + splits - 1) / splits;
   const int e = min(n, (q + 1) * per);
+  const float* from[8];
+#pragma unroll
+  for (int p = 0; p < 8; ++p) from[p] = cl.map_shared_rank(tile, p < splits ? p : 0);
   for (int i = q * per + tid; i < e; i += nthreads) {
-    float v = 0.f;
-    for (int p = 0; p < splits; ++p) v += cl.map_shared_rank(tile, p)[i];
+    float y[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) y[p] = p < splits ? from[p][i] : 0.f;
+    float v = y[0];
+#pragma unroll
+    for (int p = 1; p < 8; ++p)
+      if (p < splits) v += y[p];
     put(i, v);
   }
   cl.sync();   // nobody reads this CTA's tile any more
