@@ -54,7 +54,13 @@ __device__ __forceinline__ void add_totals(float (&acc)[4][4], const float* tota
 // it; the half products of a chunk of 32 ranks are formed in shared memory on the way (each factor entry is read by
 // 64 lanes of a CTA at most, from L1).  b runs over the fast sizes of B's modes first, so that a row of the tile is
 // stored in runs of their product.
+// What bounds it is the shared-memory pipe, which delivers 128 bytes a clock: 4 columns x 2 rows per thread and rank took 70 cycles per rank
+// and CTA (4096 x 64 at R = 137: 13.9k cycles in all).  So a thread has 8 columns and two or four rows, and groups of threads share out the
+// ranks of a chunk; their sums meet at the end.  4096 -> 64 dense at R = 137 and batch 64 15.6 -> 13.6 us, 360 -> 360 at R = 249 71 -> 64.
+// (8 x 8 for tiles of 64 rows spills: 720 -> 720 at R = 89 18.5 -> 21.2 us; 4 x 8 18.4.)
 constexpr int kKT = 256, kTB = 64, kRC = 32;
+constexpr int kron_rows(int ta) { return ta < 32 ? 2 : 4; }                        // of a thread, which has 8 columns
+constexpr int kron_groups(int ta) { return kKT * kron_rows(ta) * 8 / (ta * kTB); }   // of threads, which share out the ranks of a chunk
 
 struct KronMode {
   const float* F;
@@ -83,14 +89,20 @@ __device__ __forceinline__ void half_decode(const KronMode* m, int n, int s, int
   *out = o;
 }
 
+template <int TA>
+constexpr size_t kron_smem() {
+  constexpr int tiles = kRC * (TA + 4 + kTB + 4), sums = kron_groups(TA) * TA * kTB;
+  return sizeof(float) * (tiles > sums ? tiles : sums);
+}
+
 template <int TA, bool TAP>
-__global__ void __launch_bounds__(kKT) kron_weight_kernel(const __grid_constant__ KronGeom g, float* __restrict__ W) {
-  constexpr int NA = TA / 16;                  // rows per thread
-  __shared__ __align__(16) float tiles[kRC * (TA + 4 + kTB + 4)];
+__global__ void __launch_bounds__(kKT, 2) kron_weight_kernel(const __grid_constant__ KronGeom g, float* __restrict__ W) {
+  constexpr int TI = kron_rows(TA), KG = kron_groups(TA), kGT = kKT / KG;
+  extern __shared__ __align__(16) float tiles[];   // kron_smem<TA>()
   float (*As)[TA + 4] = reinterpret_cast<float (*)[TA + 4]>(tiles);
   float (*Bs)[kTB + 4] = reinterpret_cast<float (*)[kTB + 4]>(tiles + kRC * (TA + 4));
   __shared__ int ea[TA][3], eb[kTB][2], oa[TA], ob[kTB];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, grp = tid / kGT, gx = tid & 7, gy = tid % kGT >> 3;
   const int a0 = blockIdx.y * TA, b0 = blockIdx.x * kTB, PA = g.SA * g.FA, PB = g.SB * g.FB;
   const int rb0 = blockIdx.z * g.rper, re = min(g.R, rb0 + g.rper);
   if (tid < TA) {
@@ -106,11 +118,11 @@ __global__ void __launch_bounds__(kKT) kron_weight_kernel(const __grid_constant_
     eb[i][0] = e[0]; eb[i][1] = e[1];
     ob[i] = o;
   }
-  float acc[NA][4];
+  float acc[TI][8];
 #pragma unroll
-  for (int i = 0; i < NA; ++i)
+  for (int i = 0; i < TI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
   // A warp fills 8 ranks x 4 rows per turn: full sectors from global memory, all banks of the transposed tile.  The
   // entries of the next chunk are fetched, all loads of a thread together, while the current one is multiplied; a mode
   // that a half does not have reads nothing and counts as 1.
@@ -156,36 +168,49 @@ __global__ void __launch_bounds__(kKT) kron_weight_kernel(const __grid_constant_
     __syncthreads();
     if (r0 + kRC < re) fetch(r0 + kRC);
     const int rn = min(kRC, re - r0);
-#pragma unroll 4
-    for (int r = 0; r < rn; ++r) {
-      const float4 b = *reinterpret_cast<const float4*>(&Bs[r][tx * 4]);
-      float a[NA];
-      if (NA == 4) {
-        const float4 t = *reinterpret_cast<const float4*>(&As[r][ty * 4]);
-        a[0] = t.x; a[1] = t.y; a[2 % NA] = t.z; a[3 % NA] = t.w;
-      } else {
-        a[0] = As[r][ty * NA];
-        if (NA > 1) a[1 % NA] = As[r][ty * NA + 1];
-      }
+#pragma unroll 2
+    for (int r = grp; r < rn; r += KG) {
+      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[r][gx * 4]), b1 = *reinterpret_cast<const float4*>(&Bs[r][32 + gx * 4]);
+      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      float a[TI];
 #pragma unroll
-      for (int i = 0; i < NA; ++i) {
-        acc[i][0] = fmaf(a[i], b.x, acc[i][0]);
-        acc[i][1] = fmaf(a[i], b.y, acc[i][1]);
-        acc[i][2] = fmaf(a[i], b.z, acc[i][2]);
-        acc[i][3] = fmaf(a[i], b.w, acc[i][3]);
-      }
+      for (int i = 0; i < TI; ++i) a[i] = As[r][gy * TI + i];
+#pragma unroll
+      for (int i = 0; i < TI; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
   }
   // Not earlier: CTAs of the product that start while this grid still fills up are stacked on few SMs (138 CTAs of
   // small_conv_kernel took 170 us instead of 60).
   grid_launch_dependents();
-  if (gridDim.z > 1) {   // a small weight: the CTAs of a cluster took a share of the ranks each
-    __syncthreads();
-    float* t = tiles;    // [TA][64] fits: TA * 64 <= 32 * (TA + 72)
+  // the groups' sums, [group][TA][64]
+  __syncthreads();
 #pragma unroll
-    for (int i = 0; i < NA; ++i)
-      *reinterpret_cast<float4*>(t + (ty * NA + i) * kTB + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    cluster_sum(t, TA * kTB, gridDim.z, tid, kKT, [&](int i, float v) {
+  for (int i = 0; i < TI; ++i) {
+    float* t = tiles + (grp * TA + gy * TI + i) * kTB + gx * 4;
+    *reinterpret_cast<float4*>(t) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    *reinterpret_cast<float4*>(t + 32) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  const auto total = [&](int row) {
+    const float* t = tiles + row * kTB + tx * 4;
+    float4 v = *reinterpret_cast<const float4*>(t);
+#pragma unroll
+    for (int q = 1; q < KG; ++q) {
+      const float4 w = *reinterpret_cast<const float4*>(t + q * TA * kTB);
+      v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+    }
+    return v;
+  };
+  if (gridDim.z > 1) {   // a small weight: the CTAs of a cluster took a share of the ranks each
+#pragma unroll
+    for (int i = 0; i < TA / 16; ++i) {   // (each thread adds up what only it reads)
+      const float4 v = total(i * 16 + ty);
+      *reinterpret_cast<float4*>(tiles + (i * 16 + ty) * kTB + tx * 4) = v;
+    }
+    cluster_sum(tiles, TA * kTB, gridDim.z, tid, kKT, [&](int i, float v) {
       const int a = i / kTB, b = i % kTB;
       if (a0 + a < PA && b0 + b < PB) W[oa[a] + ob[b]] = v;
     });
@@ -194,16 +219,19 @@ __global__ void __launch_bounds__(kKT) kron_weight_kernel(const __grid_constant_
   const int b = b0 + tx * 4;
   const bool run4 = b + 3 < PB && ob[tx * 4 + 3] - ob[tx * 4] == 3 && !(ob[tx * 4] & 3);
 #pragma unroll
-  for (int i = 0; i < NA; ++i) {
-    if (a0 + ty * NA + i >= PA) continue;
-    float* d = W + oa[ty * NA + i];
-    const int o0 = oa[ty * NA + i];
+  for (int i = 0; i < TA / 16; ++i) {
+    const int row = i * 16 + ty;
+    if (a0 + row >= PA) continue;
+    const float4 v = total(row);
+    const int o0 = oa[row];
+    float* d = W + o0;
     if (run4 && !(o0 & 3)) {
-      *reinterpret_cast<float4*>(d + ob[tx * 4]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4*>(d + ob[tx * 4]) = v;
     } else {
+      const float w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (b + j < PB) d[ob[tx * 4 + j]] = acc[i][j];
+        if (b + j < PB) d[ob[tx * 4 + j]] = w[j];
     }
   }
 }
@@ -789,15 +817,22 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   const int ta = p.ta, splits = p.splits;
   g.rper = p.rper;
   const dim3 grid(p.nb, ceil_div(p.PA, ta), splits);
+#define KRON_T(TAV, TAPV)                                                                                               \
+  do {                                                                                                                  \
+    static std::atomic<int> set[64];                                                                                    \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_weight_kernel<TAV, TAPV>), set, (int)kron_smem<TAV>())); \
+    B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, TAPV>, grid, dim3(kKT), kron_smem<TAV>(), st, splits, false, g, W)); \
+  } while (0)
 #define KRON(TAV)                                                                                                       \
-  do {                                                                                                                 \
-    if (S) B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, true>, grid, dim3(kKT), 0, st, splits, false, g, W));  \
-    else B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, false>, grid, dim3(kKT), 0, st, splits, false, g, W));   \
+  do {                                                                                                                  \
+    if (S) KRON_T(TAV, true);                                                                                           \
+    else KRON_T(TAV, false);                                                                                            \
   } while (0)
   if (ta == 64) KRON(64);
   else if (ta == 32) KRON(32);
   else KRON(16);
 #undef KRON
+#undef KRON_T
   B200CP_LAUNCH_OK("kron_weight_kernel");
   return B200CP_OK;
 }
