@@ -74,6 +74,7 @@ struct KronGeom {
   int SA, FA, SB, FB;      // products of the sizes
   int R, rper;             // ranks; ranks per CTA of a cluster
   int flip;                // A[0] is the tap mode, stored back to front
+  int early;               // all CTAs are resident at once: the product's may be placed now
 };
 
 // entry offset (in ranks) and output offset of half-index (s, f)
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kKT, 2) kron_weight_kernel(const __grid_consta
   float (*As)[TA + 4] = reinterpret_cast<float (*)[TA + 4]>(tiles);
   float (*Bs)[kTB + 4] = reinterpret_cast<float (*)[kTB + 4]>(tiles + kRC * (TA + 4));
   __shared__ int ea[TA][3], eb[kTB][2], oa[TA], ob[kTB];
+  if (g.early) grid_launch_dependents();
   const int tid = threadIdx.x, grp = tid / kGT, gx = tid & 7, gy = tid % kGT >> 3;
   const int a0 = blockIdx.y * TA, b0 = blockIdx.x * kTB, PA = g.SA * g.FA, PB = g.SB * g.FB;
   const int rb0 = blockIdx.z * g.rper, re = min(g.R, rb0 + g.rper);
@@ -181,9 +183,9 @@ __global__ void __launch_bounds__(kKT, 2) kron_weight_kernel(const __grid_consta
         for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
   }
-  // Not earlier: CTAs of the product that start while this grid still fills up are stacked on few SMs (138 CTAs of
-  // small_conv_kernel took 170 us instead of 60).
-  grid_launch_dependents();
+  // Of more CTAs than SMs not earlier: CTAs of the product that start while this grid still fills up are stacked on few SMs (138 CTAs
+  // of small_conv_kernel took 170 us instead of 60).
+  if (!g.early) grid_launch_dependents();
   // the groups' sums, [group][TA][64]
   __syncthreads();
 #pragma unroll
@@ -380,8 +382,8 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
 constexpr int kGStages = 3;
 template <int BM, int BN>
 struct GemmTile {
-  static constexpr int NT = BM == 64 ? 512 : 256;     // 16 warps hide the FFMA and shared-memory latency that 8 do not
-  static constexpr int KG = NT * 16 / (BM * BN);      // 64x64 -> 2, 32x64 -> 2, 16x64 -> 4, 16x32 -> 8
+  static constexpr int NT = BM == 64 || BM == 16 ? 512 : 256;     // 16 warps hide the FFMA and shared-memory latency that 8 do not
+  static constexpr int KG = NT * 16 / (BM * BN);      // 64x64 -> 2, 32x64 -> 2, 16x64 -> 8, 16x32 -> 16, 8x32 -> 16
   static constexpr int BK = KG > 2 ? 64 : 32;         // K rows of a stage
   static constexpr int PA = BK + 4;
   static constexpr int stage = BM * PA + BK * (BN + 4);
@@ -632,8 +634,9 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
 
 // Dynamic shared memory that lets no more CTAs share an SM than the grid needs: CTAs of a programmatic dependent start
 // while the kernel before drains and would otherwise be stacked on the SMs that are free first.
-size_t spread_smem(size_t need, long ctas, const DeviceInfo& di) {
-  const long per = (ctas + di.sm_count - 1) / di.sm_count;
+size_t spread_smem(size_t need, long ctas, int cluster, const DeviceInfo& di) {
+  // (a GPC of fewer than 16 SMs has room for one cluster of 8 only)
+  const long per = std::max<long>((ctas + di.sm_count - 1) / di.sm_count, cluster == 8 && ctas > 64 ? 2 : 1);
   return per > 4 ? need : std::max(need, (size_t)di.smem_optin / per - (per > 1 ? 1024 : 0));
 }
 
@@ -668,8 +671,19 @@ GemmPlan gemm_plan(int M, int N, int K, const DeviceInfo& di) {
   const auto enough = [&](int bm) { return M > bm / 2 && (long)ceil_div(M, bm) * ceil_div(N, 64) * 8 >= di.sm_count; };
   p.bm = enough(64) ? 64 : enough(32) ? 32 : 16;
   p.bn = p.bm == 16 && (long)ceil_div(M, 16) * ceil_div(N, 64) * 8 < di.sm_count ? 32 : 64;
-  p.tiles = (long)ceil_div(M, p.bm) * ceil_div(N, p.bn);
-  p.splits = pick_cluster(p.tiles, K, 64, di.sm_count);
+  const auto tiles = [&] {
+    p.tiles = (long)ceil_div(M, p.bm) * ceil_div(N, p.bn);
+    p.splits = pick_cluster(p.tiles, K, 64, di.sm_count);
+  };
+  tiles();
+  if (p.bn == 32 && (M <= 8 || p.tiles * 8 < di.sm_count)) {   // half of the rows, unless that is many clusters of 8
+    p.bm = 8;
+    tiles();
+    if (p.splits == 8 && p.tiles > 8) {
+      p.bm = 16;
+      tiles();
+    }
+  }
   p.kper = (int)align_up((size_t)ceil_div(K, p.splits), 4);
   return p;
 }
@@ -816,6 +830,7 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   const KronPlan p = kron_plan(order, transposed ? odims : idims, transposed ? idims : odims, R, S ? taps : 1, di);
   const int ta = p.ta, splits = p.splits;
   g.rper = p.rper;
+  g.early = p.ctas <= di.sm_count;
   const dim3 grid(p.nb, ceil_div(p.PA, ta), splits);
 #define KRON_T(TAV, TAPV)                                                                                               \
   do {                                                                                                                  \
@@ -881,7 +896,7 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
 #define SMALL_GEMM_L(BMV, BNV, V, L)                                                                                    \
   do {                                                                                                                  \
     static std::atomic<int> set[64];                                                                                    \
-    const size_t smem = spread_smem(GemmTile<BMV, BNV>::smem(kper), tiles * splits, di);                                \
+    const size_t smem = spread_smem(GemmTile<BMV, BNV>::smem(kper), tiles * splits, splits, di);                                \
     B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(small_gemm_kernel<BMV, BNV, V, L>), set, di.smem_optin)); \
     B200CP_CUDA_OK(launch_cluster(small_gemm_kernel<BMV, BNV, V, L>, grid, dim3(GemmTile<BMV, BNV>::NT), smem, st, splits, true, \
                                   X, W, Y, M, N, K, ldw, kper, splits));                                                \
@@ -891,7 +906,8 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
     if (GemmTile<BMV, BNV>::is_long(kper)) SMALL_GEMM_L(BMV, BNV, V, true);                                             \
     else SMALL_GEMM_L(BMV, BNV, V, false);                                                                              \
   } while (0)
-  if (bn == 32) { if (vec) SMALL_GEMM(16, 32, true); else SMALL_GEMM(16, 32, false); }
+  if (bm == 8) { if (vec) SMALL_GEMM(8, 32, true); else SMALL_GEMM(8, 32, false); }
+  else if (bn == 32) { if (vec) SMALL_GEMM(16, 32, true); else SMALL_GEMM(16, 32, false); }
   else if (bm == 16) { if (vec) SMALL_GEMM(16, 64, true); else SMALL_GEMM(16, 64, false); }
   else if (bm == 32) { if (vec) SMALL_GEMM(32, 64, true); else SMALL_GEMM(32, 64, false); }
   else { if (vec) SMALL_GEMM(64, 64, true); else SMALL_GEMM(64, 64, false); }
@@ -915,7 +931,7 @@ int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const f
   do {                                                                                                                \
     static std::atomic<int> set[64];                                                                                  \
     B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(small_conv_kernel<TTV, CGV>), set, di.smem_optin));   \
-    B200CP_CUDA_OK(launch_cluster(small_conv_kernel<TTV, CGV>, grid, dim3(kCT), spread_smem(smem, tiles * g.splits, di), st, \
+    B200CP_CUDA_OK(launch_cluster(small_conv_kernel<TTV, CGV>, grid, dim3(kCT), spread_smem(smem, tiles * g.splits, g.splits, di), st, \
                                   g.splits, true, g, X, Wt, V));                                                      \
   } while (0)
   if (cgroups == 2) {
