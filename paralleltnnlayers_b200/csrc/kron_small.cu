@@ -90,10 +90,12 @@ __device__ __forceinline__ void half_decode(const KronMode* m, int n, int s, int
   *out = o;
 }
 
+constexpr int kron_tiles(int ta) {   // floats of a chunk of ranks, then of the groups' sums
+  return kRC * (ta + 4 + kTB + 4) > kron_groups(ta) * ta * kTB ? kRC * (ta + 4 + kTB + 4) : kron_groups(ta) * ta * kTB;
+}
 template <int TA>
 constexpr size_t kron_smem() {
-  constexpr int tiles = kRC * (TA + 4 + kTB + 4), sums = kron_groups(TA) * TA * kTB;
-  return sizeof(float) * (tiles > sums ? tiles : sums);
+  return sizeof(float) * (kron_tiles(TA) + ClusterSum::floats(TA * kTB));
 }
 
 template <int TA, bool TAP>
@@ -104,6 +106,7 @@ __global__ void __launch_bounds__(kKT, 2) kron_weight_kernel(const __grid_consta
   float (*Bs)[kTB + 4] = reinterpret_cast<float (*)[kTB + 4]>(tiles + kRC * (TA + 4));
   __shared__ int ea[TA][3], eb[kTB][2], oa[TA], ob[kTB];
   if (g.early) grid_launch_dependents();
+  const ClusterSum shared(tiles + kron_tiles(TA), TA * kTB, gridDim.z);
   const int tid = threadIdx.x, grp = tid / kGT, gx = tid & 7, gy = tid % kGT >> 3;
   const int a0 = blockIdx.y * TA, b0 = blockIdx.x * kTB, PA = g.SA * g.FA, PB = g.SB * g.FB;
   const int rb0 = blockIdx.z * g.rper, re = min(g.R, rb0 + g.rper);
@@ -207,12 +210,17 @@ __global__ void __launch_bounds__(kKT, 2) kron_weight_kernel(const __grid_consta
     return v;
   };
   if (gridDim.z > 1) {   // a small weight: the CTAs of a cluster took a share of the ranks each
+    shared.ready();
 #pragma unroll
-    for (int i = 0; i < TA / 16; ++i) {   // (each thread adds up what only it reads)
+    for (int i = 0; i < TA / 16; ++i) {
       const float4 v = total(i * 16 + ty);
-      *reinterpret_cast<float4*>(tiles + (i * 16 + ty) * kTB + tx * 4) = v;
+      const int o = (i * 16 + ty) * kTB + tx * 4;
+      shared.put(o, v.x);
+      shared.put(o + 1, v.y);
+      shared.put(o + 2, v.z);
+      shared.put(o + 3, v.w);
     }
-    cluster_sum(tiles, TA * kTB, gridDim.z, tid, kKT, [&](int i, float v) {
+    shared.sum(TA * kTB, tid, kKT, [&](int i, float v) {
       const int a = i / kTB, b = i % kTB;
       if (a0 + a < PA && b0 + b < PB) W[oa[a] + ob[b]] = v;
     });
@@ -390,7 +398,7 @@ struct GemmTile {
   static constexpr int flush = kChain / (BK / KG);    // stages of an accumulator
   static constexpr int buf = kGStages * stage > KG * BM * BN ? kGStages * stage : KG * BM * BN;
   static bool is_long(int kper) { return (kper + BK - 1) / BK > flush; }
-  static size_t smem(int kper) { return sizeof(float) * ((size_t)buf + (is_long(kper) ? 16 * NT : 0)); }
+  static size_t smem(int kper) { return sizeof(float) * ((size_t)buf + (is_long(kper) ? 16 * NT : 0) + ClusterSum::floats(BM * BN)); }
 };
 
 // LONG: more than kChain terms per accumulator (without the totals 16.5 instead of 17.0 us for 4096 -> 64 at batch 64)
@@ -436,6 +444,7 @@ __global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const 
       mma::cp_async16_s(d + (unsigned)(k * (kBN + 4) + n) * 4u, in ? W + (size_t)(k0 + k) * ldw + n0 + n : W, in ? 16 : 0);
     }
   };
+  const ClusterSum shared(smem + T::buf + (LONG ? 16 * T::NT : 0), BM * BN, splits);
   const int steps = ke > kb ? (ke - kb + T::BK - 1) / T::BK : 0;
   for (int s = 0; s < kGStages - 1; ++s)
     if (s < steps) load_a(s, kb + s * T::BK);
@@ -486,16 +495,19 @@ __global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const 
     *reinterpret_cast<float4*>(red + (kg * BM + ty * 4 + i) * kBN + tx * 4) =
         make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   __syncthreads();
+  const auto out = [&](int i, float v) {
+    const int m = m0 + i / kBN, n = n0 + i % kBN;
+    if (m < M && n < N) Y[(size_t)m * N + n] = v;
+  };
+  shared.ready();
   for (int i = tid; i < BM * kBN; i += kGT) {
     float v = red[i];
 #pragma unroll
     for (int q = 1; q < T::KG; ++q) v += red[q * BM * kBN + i];
-    red[i] = v;
+    if (splits > 1) shared.put(i, v);
+    else out(i, v);
   }
-  cluster_sum(red, BM * kBN, splits, tid, kGT, [&](int i, float v) {
-    const int m = m0 + i / kBN, n = n0 + i % kBN;
-    if (m < M && n < N) Y[(size_t)m * N + n] = v;
-  });
+  if (splits > 1) shared.sum(BM * kBN, tid, kGT, out);
 }
 
 // ---- 3 x 3 convolution with W[c][tap][t] -----------------------------------------------------------------------------------
@@ -569,6 +581,7 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
   const bool active = pq < g.PXQ;
   const int pr = active ? pq / (g.TC / 4) : 0, pc = active ? (pq - pr * (g.TC / 4)) * 4 : 0;
   const int steps = ce > cb ? (ce - cb + kCC - 1) / kCC : 0;
+  const ClusterSum shared(smem + g.buf + (steps > kFlush ? 16 * kCT : 0), TT * g.TR * g.TC, g.splits);
   if (steps > 0) load_x(0, cb);
   grid_dependency_wait();
   if (steps > 0) load_w(0, cb);
@@ -620,16 +633,19 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
       *reinterpret_cast<float4*>(smem + (grp * TT + tq * 4 + i) * npx + pr * g.TC + pc) =
           make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   __syncthreads();
+  const auto out = [&](int i, float v) {
+    const int t = t0 + i / npx, px = i % npx, h = h0 + px / g.TC, w = w0 + px % g.TC;
+    if (t < g.T && h < g.H && w < g.W) Vn[(size_t)t * HW + h * g.W + w] = v;
+  };
+  shared.ready();
   for (int i = tid; i < TT * npx; i += kCT) {
     float v = smem[i];
 #pragma unroll
     for (int q = 1; q < CG; ++q) v += smem[q * TT * npx + i];
-    smem[i] = v;
+    if (g.splits > 1) shared.put(i, v);
+    else out(i, v);
   }
-  cluster_sum(smem, TT * npx, g.splits, tid, kCT, [&](int i, float v) {
-    const int t = t0 + i / npx, px = i % npx, h = h0 + px / g.TC, w = w0 + px % g.TC;
-    if (t < g.T && h < g.H && w < g.W) Vn[(size_t)t * HW + h * g.W + w] = v;
-  });
+  if (g.splits > 1) shared.sum(TT * npx, tid, kCT, out);
 }
 
 // Dynamic shared memory that lets no more CTAs share an SM than the grid needs: CTAs of a programmatic dependent start
@@ -924,7 +940,8 @@ int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const f
   const SmallConvGeom& g = p.g;
   const int tt = p.tt, cgroups = p.cgroups;
   const long tiles = p.tiles;
-  const size_t smem = sizeof(float) * ((size_t)g.buf + (ceil_div(g.cper, kCC) > conv_flush(cgroups) ? 16 * kCT : 0));
+  const size_t smem = sizeof(float) * ((size_t)g.buf + (ceil_div(g.cper, kCC) > conv_flush(cgroups) ? 16 * kCT : 0) +
+                                        ClusterSum::floats(tt * g.TR * g.TC));
   dim3 grid((unsigned)(N * g.tiles), ceil_div(T, tt), g.splits);
   if ((long)N * g.tiles > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");
 #define SMALL_CONV(TTV, CGV)                                                                                              \
