@@ -12,6 +12,7 @@
 // All exact fp32 (FFMA).  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
 // and past their set-up when the weight is done.  Formulas: Kernels/rcp_fused_nchw.cu:4-77, Kernels/dense_cp.cu:4-46.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "cluster_util.cuh"
@@ -523,15 +524,27 @@ struct SmallConvGeom {
   int TR, TC, tilesW, tiles, PXQ;   // tile rows / columns (a multiple of 4), pixel quads in use
   int P, CS;                        // halo row pitch, halo floats per channel
   int buf;                          // floats of the stages (and the sum over the groups); the totals follow
+  int weight;                       // where the weight is that the CTA forms itself, behind all that
 };
 
-template <int TT, int CG>
+// INSIDE: a small weight is formed by each CTA for its channels, in shared memory, instead of by a launch before it: 16 -> 16 channels at
+// R = 11, eight 32x32 images, 6.8 -> 6.7 us on the device, and 2 us less for the host, which is what such a call then takes (10.2 -> 8.3 us).
+struct ConvWeight {
+  KronMode m[4];
+  unsigned sdiv[4], fdiv[4];   // 2^32 / ns, nf rounded up (0: 1)
+  const float* S;
+  int order, R, flip;
+};
+constexpr int kSP = 12;   // taps of a rank in shared memory: three 16-byte reads
+
+template <int TT, int CG, bool INSIDE>
 __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, const float* __restrict__ X,
-                                                         const float* __restrict__ Wt, float* __restrict__ V) {
+                                                         const float* __restrict__ Wt, float* __restrict__ V,
+                                                         const __grid_constant__ ConvWeight f) {
   constexpr int TG = TT / 4;
   constexpr int WS = kCC * 9 * TT;
   extern __shared__ __align__(16) float smem[];
-  const int xs = kCC * g.CS, stage = xs + WS;
+  const int xs = kCC * g.CS, stage = xs + (INSIDE ? 0 : WS);
   const int tid = threadIdx.x, lane = tid & 31;
   const int grp = tid / (kCT / CG), warp = (tid >> 5) % (kCT / CG / 32);   // CG groups of warps share a stage's channels
   // lanes: 8 pixel quads x 4 channel quads; warps: the remaining channel quads first
@@ -583,20 +596,77 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
   const int steps = ce > cb ? (ce - cb + kCC - 1) / kCC : 0;
   const ClusterSum shared(smem + g.buf + (steps > kFlush ? 16 * kCT : 0), TT * g.TR * g.TC, g.splits);
   if (steps > 0) load_x(0, cb);
-  grid_dependency_wait();
-  if (steps > 0) load_w(0, cb);
-  mma::cp_async_commit();
+  float* weight = smem + g.weight;   // [channel][tap][TT], then the taps of the ranks
+  if constexpr (INSIDE) {
+    mma::cp_async_commit();
+    float* taps = weight + g.cper * 9 * TT;
+    const float tap = tid < f.R * kSP && tid % kSP < 9 ? __ldg(f.S + (size_t)(f.flip ? 8 - tid % kSP : tid % kSP) * f.R + tid / kSP) : 0.f;
+    // this thread's entry (channel, output): where its factors' values of rank 0 are; four ranks of them, on their way early
+    const float* F[4];
+    float p[4];
+    const int ci = cb + tid / TT, ti = t0 + tid % TT;
+    const bool entry = tid < g.cper * TT && ci < ce && ti < g.T;
+    if (entry) {
+      unsigned s = ci, q = ti;
+#pragma unroll
+      for (int k = 3; k >= 0; --k) {
+        if (k >= f.order) continue;
+        const unsigned sn = f.sdiv[k] ? __umulhi(s, f.sdiv[k]) : s, qn = f.fdiv[k] ? __umulhi(q, f.fdiv[k]) : q;
+        F[k] = f.m[k].F + (size_t)((s - sn * f.m[k].ns) * f.m[k].fs + (q - qn * f.m[k].nf) * f.m[k].ff) * f.R;
+        s = sn;
+        q = qn;
+      }
+    }
+    const auto fetch = [&](int r0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool in = r0 + j < f.R;
+        p[j] = in ? __ldg(F[0] + r0 + j) : 0.f;
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+          if (k < f.order && in) p[j] *= __ldg(F[k] + r0 + j);
+      }
+    };
+    if (entry) fetch(0);
+    if (tid < f.R * kSP) taps[tid] = tap;
+    __syncthreads();
+    if (tid < g.cper * TT) {   // at most one entry per thread
+      float w[9];
+#pragma unroll
+      for (int j = 0; j < 9; ++j) w[j] = 0.f;
+      if (entry)
+        for (int r0 = 0; r0 < f.R; r0 += 4) {
+          const float v[4] = {p[0], p[1], p[2], p[3]};
+          if (r0 + 4 < f.R) fetch(r0 + 4);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (r0 + u >= f.R) break;
+            const float* tr = taps + (r0 + u) * kSP;
+            const float4 a = *reinterpret_cast<const float4*>(tr), b = *reinterpret_cast<const float4*>(tr + 4);
+            const float x[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, tr[8]};
+#pragma unroll
+            for (int j = 0; j < 9; ++j) w[j] = fmaf(v[u], x[j], w[j]);
+          }
+        }
+#pragma unroll
+      for (int j = 0; j < 9; ++j) weight[(tid / TT * 9 + j) * TT + tid % TT] = w[j];
+    }
+  } else {
+    grid_dependency_wait();
+    if (steps > 0) load_w(0, cb);
+    mma::cp_async_commit();
+  }
   for (int s = 0; s < steps; ++s) {
     if (s + 1 < steps) {
       load_x((s + 1) & 1, cb + (s + 1) * kCC);
-      load_w((s + 1) & 1, cb + (s + 1) * kCC);
+      if (!INSIDE) load_w((s + 1) & 1, cb + (s + 1) * kCC);
     }
     mma::cp_async_commit();
     mma::cp_async_wait<1>();
     __syncthreads();
     if (active) {
       const float* xb = smem + (s & 1) * stage + pr * g.P + pc + 4;
-      const float* wb = smem + (s & 1) * stage + xs + tq * 4;
+      const float* wb = (INSIDE ? weight + s * WS : smem + (s & 1) * stage + xs) + tq * 4;
 #pragma unroll 2
       for (int cc = 0; cc < kCC / CG; ++cc) {
         const int c = grp * (kCC / CG) + cc;
@@ -704,12 +774,18 @@ GemmPlan gemm_plan(int M, int N, int K, const DeviceInfo& di) {
   return p;
 }
 
+// The CTAs form the weight where that is one entry per thread, of at most so many ranks.  Calls one after the other, weight by a launch /
+// inside (the launch also costs the host 2 us): 16 -> 10 channels at R = 14 9.2 / 8.3 us, 12 at R = 15 11.9 / 10.3; two entries: 60 channels at
+// R = 5 14.4 / 16.4, 192 -> 24 at R = 14 10.3 / 12.3; 28 ranks: 16 -> 12 9.3 / 10.3.
+constexpr int kInside = 16;
+
 struct ConvPlan {
   int tt, cgroups;
   long tiles;
+  size_t floats, inside;   // of shared memory, without the weight and with it formed inside
   SmallConvGeom g;
 };
-ConvPlan conv_plan(int N, int C, int T, int H, int W, const DeviceInfo& di) {
+ConvPlan conv_plan(int N, int C, int T, int H, int W, int R, const DeviceInfo& di) {
   ConvPlan p{};
   SmallConvGeom& g = p.g;
   const int tt = p.tt = T <= 16 ? 16 : T <= 32 ? 32 : 64;
@@ -738,7 +814,20 @@ ConvPlan conv_plan(int N, int C, int T, int H, int W, const DeviceInfo& di) {
   p.tiles = (long)N * g.tiles * ceil_div(T, tt);
   g.splits = pick_cluster(p.tiles, C, 2 * kCC, di.sm_count);
   g.cper = (int)align_up((size_t)ceil_div(C, g.splits), kCC);
-  g.buf = std::max(2 * (kCC * g.CS + kCC * 9 * tt), p.cgroups * tt * g.TR * g.TC);
+  const int stages = 2 * kCC * g.CS, sums = p.cgroups * tt * g.TR * g.TC;
+  const size_t behind = (ceil_div(g.cper, kCC) > conv_flush(p.cgroups) ? 16 * kCT : 0) + ClusterSum::floats(tt * g.TR * g.TC);
+  g.buf = std::max(stages + 2 * kCC * 9 * tt, sums);
+  p.floats = g.buf + behind;
+  // the weight of the CTA's channels and the ranks' taps
+  if (g.cper * tt <= kCT && R <= kInside) {
+    const int buf = std::max(stages, sums);
+    const size_t weight = align_up(buf + behind, 4), all = weight + (size_t)g.cper * 9 * tt + (size_t)R * kSP;
+    if (all * sizeof(float) <= (size_t)di.smem_optin) {
+      g.buf = buf;
+      g.weight = (int)weight;
+      p.inside = all;
+    }
+  }
   return p;
 }
 
@@ -783,16 +872,26 @@ double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* 
     C *= transposed ? tdims[k] : cdims[k];
     T *= transposed ? cdims[k] : tdims[k];
   }
-  const ConvPlan p = conv_plan(N, C, T, H, W, di);
+  const ConvPlan p = conv_plan(N, C, T, H, W, R, di);
   const SmallConvGeom& g = p.g;
   const int px = kCT / p.cgroups / (p.tt / 4) * 4;
   const double w = waves(p.tiles * g.splits, di) * g.cper;
-  return 5.1 + kron_weight_us(order, cdims, tdims, R, 9, transposed) +
+  return 5.1 + (p.inside ? 0.2 * R : kron_weight_us(order, cdims, tdims, R, 9, transposed)) +
          (p.tt == 64 ? 6.71e-6 : 5.19e-6) * w * 9 * p.tt * px + 8.04e-4 * w * (g.TR + 2) * (g.TC + 2);
 }
 
 // Row pitch of the weight: 16-byte rows.
 int kron_weight_ld(int fast) { return (fast + 3) / 4 * 4; }
+
+static KronMode kron_mode(const float* F, int idim, int odim, bool transposed) {
+  KronMode m{};
+  m.F = F;
+  m.ns = transposed ? odim : idim;
+  m.nf = transposed ? idim : odim;
+  m.fs = transposed ? 1 : odim;
+  m.ff = transposed ? odim : 1;
+  return m;
+}
 
 // the modes and halves of a weight with rows of `ld` entries per tap
 static int kron_geom(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S, int taps,
@@ -800,11 +899,7 @@ static int kron_geom(int order, const int* idims, const int* odims, int R, const
   KronMode m[4];
   long slow = 1, fast = 1;
   for (int k = 0; k < order; ++k) {
-    m[k].F = F[k];
-    m[k].ns = transposed ? odims[k] : idims[k];
-    m[k].nf = transposed ? idims[k] : odims[k];
-    m[k].fs = transposed ? 1 : odims[k];
-    m[k].ff = transposed ? odims[k] : 1;
+    m[k] = kron_mode(F[k], idims[k], odims[k], transposed);
     slow *= m[k].ns;
     fast *= m[k].nf;
   }
@@ -933,23 +1028,46 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
   return B200CP_OK;
 }
 
-int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const float* Wt, float* V, cudaStream_t st) {
+// whether the CTAs of the product form the weight themselves (then it needs no workspace)
+bool conv_weight_inside(int N, int C, int T, int H, int W, int R) {
+  DeviceInfo di;
+  return !device_info(&di) && conv_plan(N, C, T, H, W, R, di).inside;
+}
+
+// V = W * X, the weight in Wt, or (Wt null) formed inside
+int small_conv_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, const float* const* A, const float* S,
+                      bool transposed, const float* X, const float* Wt, float* V, cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
-  const ConvPlan p = conv_plan(N, C, T, H, W, di);
+  int C = 1, T = 1;
+  ConvWeight f{};
+  f.order = order; f.R = R; f.S = S; f.flip = transposed;
+  for (int k = 0; k < order; ++k) {
+    f.m[k] = kron_mode(A[k], cdims[k], tdims[k], transposed);
+    f.sdiv[k] = f.m[k].ns > 1 ? (unsigned)((0x100000000ull + f.m[k].ns - 1) / f.m[k].ns) : 0;
+    f.fdiv[k] = f.m[k].nf > 1 ? (unsigned)((0x100000000ull + f.m[k].nf - 1) / f.m[k].nf) : 0;
+    C *= f.m[k].ns;
+    T *= f.m[k].nf;
+  }
+  const ConvPlan p = conv_plan(N, C, T, H, W, Wt ? INT_MAX : R, di);
   const SmallConvGeom& g = p.g;
   const int tt = p.tt, cgroups = p.cgroups;
   const long tiles = p.tiles;
-  const size_t smem = sizeof(float) * ((size_t)g.buf + (ceil_div(g.cper, kCC) > conv_flush(cgroups) ? 16 * kCT : 0) +
-                                        ClusterSum::floats(tt * g.TR * g.TC));
+  const size_t smem = sizeof(float) * (Wt ? p.floats : p.inside);
   dim3 grid((unsigned)(N * g.tiles), ceil_div(T, tt), g.splits);
   if ((long)N * g.tiles > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");
-#define SMALL_CONV(TTV, CGV)                                                                                              \
+#define SMALL_CONV_I(TTV, CGV, IN)                                                                                        \
   do {                                                                                                                \
     static std::atomic<int> set[64];                                                                                  \
-    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(small_conv_kernel<TTV, CGV>), set, di.smem_optin));   \
-    B200CP_CUDA_OK(launch_cluster(small_conv_kernel<TTV, CGV>, grid, dim3(kCT), spread_smem(smem, tiles * g.splits, g.splits, di), st, \
-                                  g.splits, true, g, X, Wt, V));                                                      \
+    const auto kernel = small_conv_kernel<TTV, CGV, IN>;                                                              \
+    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), set, di.smem_optin));                   \
+    B200CP_CUDA_OK(launch_cluster(kernel, grid, dim3(kCT), IN ? smem : spread_smem(smem, tiles * g.splits, g.splits, di), st, \
+                                  g.splits, !IN, g, X, Wt, V, f));                                                    \
+  } while (0)
+#define SMALL_CONV(TTV, CGV)                                                                                              \
+  do {                                                                                                                \
+    if (Wt) SMALL_CONV_I(TTV, CGV, false);                                                                            \
+    else SMALL_CONV_I(TTV, CGV, true);                                                                                \
   } while (0)
   if (cgroups == 2) {
     if (tt == 16) SMALL_CONV(16, 2);
@@ -961,6 +1079,7 @@ int small_conv_launch(int N, int C, int T, int H, int W, const float* X, const f
     else SMALL_CONV(64, 4);
   }
 #undef SMALL_CONV
+#undef SMALL_CONV_I
   B200CP_LAUNCH_OK("small_conv_kernel");
   return B200CP_OK;
 }

@@ -45,7 +45,7 @@ bool tensor_may(int flags, int R, double macs) {
   return gemm_tc_mode() == 2 || (R >= kLeastRanks && macs >= kLeastMacs);
 }
 
-enum class Form { factored, ffma, tensor };
+enum class Form { factored, ffma, tensor, inside };   // inside: ffma, the weight formed by the product's CTAs
 
 // `floats`: of the weight; a form's time is negative where it does not take the sizes
 Form pick(size_t floats, double entries, double ffma_us, double tensor_us, double factored_us) {
@@ -100,7 +100,8 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
   if (p.form == Form::tensor) {
     p.bytes = planes;
   } else if (p.form == Form::ffma) {
-    p.bytes = align_up(p.weight * sizeof(float), 256);
+    p.bytes = align_up(p.weight * sizeof(float), 256);   // (named for either, and used where the weight is not formed inside)
+    if (conv_weight_inside(N, p.K, p.N, H, W, R)) p.form = Form::inside;
   }
   return p;
 }
@@ -142,13 +143,14 @@ int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const i
   if (int rc = check_kron_modes(order, cdims, tdims, R, "rcp")) return rc;
   const bool sizes = N >= 1 && H >= 1 && W >= 1;
   const DensePlan p = sizes ? rcp_plan(N, H, W, order, cdims, tdims, R, FH, FW, transposed, flags) : DensePlan{};
+  if (p.form == Form::inside) return small_conv_launch(N, H, W, order, cdims, tdims, R, A, S, transposed, X, nullptr, V, st);
   if (!fits(p, ws, ws_bytes))
     return rcp_chain_launch(N, H, W, order, cdims, tdims, R, FH, FW, X, A, S, V, transposed, st);
   float* Wt = static_cast<float*>(ws);
   if (p.form == Form::tensor)
     return conv_tc_launch(N, p.K, p.N, H, W, X, KronWeight{order, cdims, tdims, R, A, S, !transposed, transposed}, V, Wt, st);
   if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, FH * FW, transposed, transposed, Wt, st)) return rc;
-  return small_conv_launch(N, p.K, p.N, H, W, X, Wt, V, st);
+  return small_conv_launch(N, H, W, order, cdims, tdims, R, A, S, transposed, X, Wt, V, st);
 }
 
 }  // namespace b200cp

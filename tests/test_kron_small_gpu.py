@@ -59,6 +59,19 @@ def test_rcp_forward_and_data_gradient(case):
     check(P.rcp_conv2d_backward(x, dv, *a, s, need_dw=False)[0], rX, "rcp dX", atol=1e-5 * max(1.0, float(np.abs(rX).max())))
 
 
+# The weight formed by the product's CTAs or by a launch before it: up to 16 ranks, 512 entries (channels of a CTA x its tile of outputs); one to
+# four modes, channels that do not fill a CTA's share, a last tile of outputs that is not full.
+INSIDE = [
+    (2, (4, 4), (4, 4), 9, 8, 16), (2, (4, 4), (4, 4), 9, 8, 17), (1, (2, 2, 2, 2), (2, 2, 2, 3), 5, 6, 16), (1, (13,), (16,), 6, 7, 3),
+    (1, (4, 8), (4, 4), 33, 5, 9), (1, (3, 11), (4, 4), 33, 5, 9), (1, (2, 4), (9, 9), 8, 8, 5), (40, (3, 2, 3), (3, 2, 2), 12, 12, 1),
+]
+
+
+@pytest.mark.parametrize("case", INSIDE, ids=str)
+def test_rcp_weight_formed_inside(case):
+    test_rcp_forward_and_data_gradient(case)
+
+
 def test_rounding_of_long_sums():
     """4096 inputs and 256 channels x 9 taps, not split over CTAs.  A chain of n fp32 additions of random signs is off by about
     2**-24 * sqrt(n / 6) of its result: 1.9e-7 for the 64 to 72 terms of an accumulator, 1.4e-7 for the at most 32 totals,
