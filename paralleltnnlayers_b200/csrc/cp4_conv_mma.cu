@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 #include <cooperative_groups.h>
@@ -324,11 +325,12 @@ __global__ void __launch_bounds__(kNT, (RP <= 16 && MBW1 <= 2) ? 3 : 2) cp4_conv
   // ---------------- phase 2 ----------------
   {
     const int r = tid % RP;           // fixed per thread (kNT is a multiple of RP)
-    if (FS == 3) {
-      float w[9];
+    // F x F taps in registers, strips of eight pixels of a row
+    auto strips = [&](auto taps) {
+      constexpr int F = decltype(taps)::value, SW = 8;
+      float w[F * F];
 #pragma unroll
-      for (int t = 0; t < 9; ++t) w[t] = Ws[t * RP + r];
-      constexpr int SW = 8;
+      for (int t = 0; t < F * F; ++t) w[t] = Ws[t * RP + r];
       const int spr = (g.TW + SW - 1) / SW;
       const int items = g.TH * spr;
       for (int it = tid / RP; it < items; it += kNT / RP) {
@@ -339,17 +341,15 @@ __global__ void __launch_bounds__(kNT, (RP <= 16 && MBW1 <= 2) ? 3 : 2) cp4_conv
         // reads past the tile's last column stay inside the padded row and feed only outputs that are not stored
         const float* p = Pr + (size_t)r * PP + oy * g.TWh + x0;
 #pragma unroll
-        for (int dy = 0; dy < 3; ++dy) {
-          float v[SW + 2];
+        for (int dy = 0; dy < F; ++dy) {
+          float v[SW + F - 1];
 #pragma unroll
-          for (int j = 0; j < SW + 2; ++j) v[j] = p[j];
+          for (int j = 0; j < SW + F - 1; ++j) v[j] = p[j];
           p += g.TWh;
 #pragma unroll
-          for (int j = 0; j < SW; ++j) {
-            z[j] = fmaf(w[dy * 3 + 0], v[j], z[j]);
-            z[j] = fmaf(w[dy * 3 + 1], v[j + 1], z[j]);
-            z[j] = fmaf(w[dy * 3 + 2], v[j + 2], z[j]);
-          }
+          for (int j = 0; j < SW; ++j)
+#pragma unroll
+            for (int dx = 0; dx < F; ++dx) z[j] = fmaf(w[dy * F + dx], v[j + dx], z[j]);
         }
         float* zd = Zs + r * ZP + oy * g.TW + x0;
         if (x0 + SW <= g.TW) {
@@ -361,6 +361,11 @@ __global__ void __launch_bounds__(kNT, (RP <= 16 && MBW1 <= 2) ? 3 : 2) cp4_conv
             if (x0 + j < g.TW) zd[j] = z[j];
         }
       }
+    };
+    if (FS == 3) {
+      strips(std::integral_constant<int, 3>{});
+    } else if (g.Y == 5 && g.X == 5) {   // (tap by tap out of shared memory 8 x 48 -> 256 55x55 at R = 16 took 23.0 us, now 18.4)
+      strips(std::integral_constant<int, 5>{});
     } else {
       for (int op = tid / RP; op < g.OPX; op += kNT / RP) {
         const int oy = op / g.TW, ox = op - oy * g.TW;

@@ -119,3 +119,14 @@ def test_step_shares_the_rank_planes(case):
         off += r.size
     U2, gX2, dK2 = P.cp4_conv2d_step(dX_, ddU, dK0, dK1, dKH, dKW, pad)
     assert torch.equal(dK, dK2) and torch.equal(U, U2)     # bitwise reproducible
+
+
+# 5x5 filters have their taps in registers and strips of eight pixels: tiles of fewer than eight columns, a column more than a multiple of
+# eight, one row or column of pixels, every rank class, pads 0 to 2
+FIVE = [(60, 2, 9, 17, 6, 5, 5, 3, 2, 0.2), (61, 1, 8, 8, 1, 9, 5, 16, 2, 0.2), (62, 3, 20, 24, 17, 33, 5, 17, 2, 0.1), (63, 1, 33, 40, 23, 1, 5, 40, 2, 0.1),
+        (64, 2, 16, 8, 12, 24, 5, 8, 1, 0.2), (65, 1, 24, 16, 13, 10, 5, 65, 0, 0.1)]
+
+
+@pytest.mark.parametrize("case", FIVE, ids=lambda c: "s%d" % c[0])
+def test_five_by_five(case):
+    test_forward_and_backward_data_mma(case)
