@@ -1086,6 +1086,9 @@ PlanesOn planes_on_tensor_cores(const b200cp_tensor_shape& s) {
   // few channels: half of a K stage is padding (C + T up to 32: a step 1.01 to 1.28 times as long; 33 to 64 at 33 to 64 ranks 1.00 to
   // 1.06 with 16-byte loads, 0.94 to 0.98 without, above that 0.73 to 1.01)
   if (s.Rank > 64 && s.C + s.T <= 32) return {false, false};
+  // up to 1000 pixels and 33 to 64 ranks the two are even on average, and a deep sum over few tiles loses (3 x 432 -> 64 17x17 at R = 44
+  // 16.4 us on FFMA, 18.5)
+  if (s.Rank <= 64 && macs < 1.3e8 && (size_t)s.N * s.H * s.W < 1000) return {false, true};
   return {sums && s.C + s.T > (s.Rank > 64 || single ? 32u : 64u), true};
 }
 // Gradients with 16-byte loads (plane_grad_tc_kernel<.., true>; the few buffers that are not aligned have 4-byte loads there)
