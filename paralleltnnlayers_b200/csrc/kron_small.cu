@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
   if constexpr (INSIDE) {
     mma::cp_async_commit();
     float* taps = weight + g.cper * 9 * TT;
-    const float tap = tid < f.R * kSP && tid % kSP < 9 ? __ldg(f.S + (size_t)(f.flip ? 8 - tid % kSP : tid % kSP) * f.R + tid / kSP) : 0.f;
+    const float tap = tid < f.R * kSP && tid % kSP < 9 ? f.S[(size_t)(f.flip ? 8 - tid % kSP : tid % kSP) * f.R + tid / kSP] : 0.f;
     // this thread's entry (channel, output): where its factors' values of rank 0 are; four ranks of them, on their way early
     const float* F[4];
     float p[4];
@@ -621,10 +621,10 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const bool in = r0 + j < f.R;
-        p[j] = in ? __ldg(F[0] + r0 + j) : 0.f;
+        p[j] = in ? F[0][r0 + j] : 0.f;
 #pragma unroll
         for (int k = 1; k < 4; ++k)
-          if (k < f.order && in) p[j] *= __ldg(F[k] + r0 + j);
+          if (k < f.order && in) p[j] *= F[k][r0 + j];
       }
     };
     if (entry) fetch(0);
