@@ -6,8 +6,8 @@
 //
 // The tile kernels do the three phases of a convolution one after the other in each CTA, on tiles of one image: with
 // many ranks or channels, small images, or widths the row kernels do not take, a CTA is one long serial chain with idle
-// lanes (64 images of 512 x 7x7 at R = 64: 52 us per convolution, 77 us for the factor gradients, for 0.1 GMAC per
-// product; here 31 us and 37 us).  Here a phase is a launch of its own, over the pixels of all images as one flat range, so that a tile is
+// lanes (64 images of 512 x 7x7 at R = 64: 51 us per convolution, 208 us for the factor gradients, for 0.1 GMAC per
+// product; here 23 us and 39 us).  Here a phase is a launch of its own, over the pixels of all images as one flat range, so that a tile is
 // always full and the sum can be split over a cluster; the planes (R of C channels) pass through L2.  The launches are
 // programmatic dependents of one another.  The products and the factor gradients exist on FFMA and on the tensor cores, where a
 // value is three bf16 parts (24 bits) and a product six of theirs; the stencils are FFMA.
@@ -241,10 +241,9 @@ __global__ void __launch_bounds__(kThreads) plane_gemm_kernel(const __grid_const
 // up to their commit), 1 for the read-out.  One elected lane issues the products, once the warp's next loads are on their way: the whole
 // layer of 64 x 512 7x7 at R = 64 64.3 -> 61.9 us, 32 x 128 28x28 at R = 56 88.4 -> 84.5.  (A warp of its own for the issue: chunks of
 // 1.2 us, but 96 registers instead of 125, and all else took as much longer.)  Both products of
-// 64 x 256 14x14 at R = 32: P and Q 21.9 us on FFMA, 20.2 here, the outputs 18.2 and 17.0; of 16 x 256 -> 384 27x27 at R = 50: 53.9 and
-// 36.8, 44.4 and 25.0.  Fp16 pairs with an exponent per pixel and chunk took 19.6, 16.4, 36.0 and 23.8, and lost the result where a
-// rank is scaled up in one factor and down in another (R = 24, by 2^-40 to 2^40).  Error against float64 over 60 drawn shapes 0.7
-// times that of FFMA.
+// 64 x 256 14x14 at R = 32: P and Q 19.7 us on FFMA, 16.8 here, the outputs 17.5 and 15.0; of 16 x 256 -> 384 27x27 at R = 50: 39.8 and
+// 34.0, 40.2 and 16.4.  Fp16 pairs with an exponent per pixel and chunk took 2 to 5 % less, and lost the result where a rank is scaled
+// up in one factor and down in another (R = 24, by 2^-40 to 2^40).  Error against float64 over 60 drawn shapes 0.7 times that of FFMA.
 constexpr int kTcPx = 128, kTcK = 64;
 constexpr int kTcPlane = kTcPx * 128;   // bytes of one operand plane of a chunk
 constexpr int kTcMaxChunks = 14;        // that fit in shared memory with rows of 32
@@ -568,8 +567,8 @@ __global__ void __launch_bounds__(kThreads) plane_stencil_kernel(const __grid_co
 // a row at a time: 64 pixels, two per lane, and 4 bytes of each plane per lane.  A chunk of 64 pixels has an accumulator of
 // its own in half of TMEM (two CTAs per SM); once these are used up they are added to totals in registers.
 //
-// What bounds it is the splitting and latency: 64 x 256 14x14 at R = 32 17.7 us on FFMA, 18.5 here; 16 x 256 -> 384 27x27 at R = 50
-// (4-byte loads) 34.4 and 26.9.  Fp16 pairs with an exponent per row and 64 pixels took 20.8 and 28.5, and lost 3e-4 of the result at 7x7 images
+// What bounds it is the splitting and latency: 64 x 256 14x14 at R = 32 17.2 us on FFMA, 14.1 here; 16 x 256 -> 384 27x27 at R = 50
+// (4-byte loads) 33.1 and 26.4.  Fp16 pairs with an exponent per row and 64 pixels were no faster and lost 3e-4 of the result at 7x7 images
 // beside one of 1e9 without gradient.  Three CTAs per SM with half of the TMEM columns each spill (27x27: half as long again).
 struct PlaneGrad {
   const float* D[2];     // dU, X
