@@ -48,11 +48,11 @@ struct ClusterSum {
   __device__ ClusterSum(float* in_, int n, int splits_) : in(in_), splits(splits_), per((n + splits_ - 1) / splits_), rank(0) {
     if (splits == 1) return;
     rank = cooperative_groups::this_cluster().block_rank();
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
   }
   // before the first put: the other CTAs have started
   __device__ void ready() const {
-    if (splits > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (splits > 1) asm volatile("barrier.cluster.wait;" ::: "memory");
   }
   __device__ void put(int i, float v) const {
     const int q = i / per;
@@ -61,8 +61,8 @@ struct ClusterSum {
   // the sums of this CTA's slice of n values
   template <typename Out>
   __device__ void sum(int n, int tid, int nthreads, Out out) const {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     const int first = (int)rank * per, count = min(n - first, per);
     for (int i = tid; i < count; i += nthreads) {
       float y[8];
