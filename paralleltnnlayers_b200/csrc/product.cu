@@ -100,7 +100,7 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
   if (p.form == Form::tensor) {
     p.bytes = planes;
   } else if (p.form == Form::ffma) {
-    p.bytes = align_up(p.weight * sizeof(float), 256);   // (named for either, and used where the weight is not formed inside)
+    p.bytes = align_up(p.weight * sizeof(float), 256);   // (a call without it runs the factored kernels; unused where the weight is formed inside)
     if (conv_weight_inside(N, p.K, p.N, H, W, R)) p.form = Form::inside;
   }
   return p;
@@ -143,9 +143,9 @@ int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const i
   if (int rc = check_kron_modes(order, cdims, tdims, R, "rcp")) return rc;
   const bool sizes = N >= 1 && H >= 1 && W >= 1;
   const DensePlan p = sizes ? rcp_plan(N, H, W, order, cdims, tdims, R, FH, FW, transposed, flags) : DensePlan{};
-  if (p.form == Form::inside) return small_conv_launch(N, H, W, order, cdims, tdims, R, A, S, transposed, X, nullptr, V, st);
   if (!fits(p, ws, ws_bytes))
     return rcp_chain_launch(N, H, W, order, cdims, tdims, R, FH, FW, X, A, S, V, transposed, st);
+  if (p.form == Form::inside) return small_conv_launch(N, H, W, order, cdims, tdims, R, A, S, transposed, X, nullptr, V, st);
   float* Wt = static_cast<float*>(ws);
   if (p.form == Form::tensor)
     return conv_tc_launch(N, p.K, p.N, H, W, X, KronWeight{order, cdims, tdims, R, A, S, !transposed, transposed}, V, Wt, st);
