@@ -142,7 +142,10 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   };
   switch (use) {
     case Planes::kConv: return past({224, 100, 0}, {2800, 900, 0});
-    case Planes::kStep: return true;
+    case Planes::kStep:   // (few channels, 5000 to 80000 pixels and planes that 16-byte loads do not divide: planes / tile kernels 1.10 over 30
+                          // shapes that the line was not fitted on, 98.8 / 72.0 us at 42 x 33 -> 6 x 27x58, R = 29; from 80000 pixels on 0.90
+                          // over 12, 303 / 395 us at 119 x 20 -> 25 x 46x57, R = 17)
+      return ranks || (size_t)s->H * s->W % 4 == 0 || ch > 80 || root4 <= 8.4 || root4 >= 16.8;
     case Planes::kSaved:
       if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // (measured: narrow layers with odd rows lose)
       return past({160, 0, 0}, {2200, 0, 0});
