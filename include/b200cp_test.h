@@ -56,6 +56,11 @@ void b200cp_test_set_planes(int planes, int tensor_cores);
  * lines of their own beside these. */
 int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s);
 
+/* How the 3x3 reshaped-CP convolution (`transposed`: its data gradient) runs: out[0] 0 factored, 1 the weight multiplied out and an FFMA product,
+ * 2 a tensor product, 3 an FFMA product whose CTAs form the weight; for 1 and 3 out[1] CTAs that split the channels, out[2] and out[3]
+ * stages of the first and the last of them, out[4] stages after which an accumulator is added up. */
+int b200cp_test_rcp_product(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int transposed, int flags, int* out);
+
 /* Diagnostics: the row-band kernel writes 64 cycle stamps (long long) per CTA for its first 512 CTAs into this
  * device buffer (512 * 64 * 8 bytes); NULL switches it off.  Process-wide. */
 void b200cp_test_set_band_trace(void* device_buffer);

@@ -40,7 +40,9 @@ __device__ __forceinline__ void cluster_sum(float* tile, int n, int splits, int 
 // the reshaped-CP forward 11.4 -> 10.9.  For the large tiles of plane_gemm_kernel, which a thread would store value by value, reads are
 // faster (64 x 512 7x7 layer at R = 64, all on FFMA, 72 us by reads, 94 by stores).
 struct ClusterSum {
-  float* in;     // this CTA's slice of all CTAs' tiles, [CTA][per], ClusterSum::floats() of memory that nothing else uses
+  // this CTA's slice of all CTAs' tiles, [CTA][per], ClusterSum::floats() of memory that nothing else uses, at the same offset in every
+  // CTA: a store to another CTA goes to this one's own address there
+  float* in;
   int splits, per;
   unsigned rank;
   static __host__ __device__ constexpr int floats(int n) { return n + 8; }   // (at most 8 CTAs)

@@ -245,6 +245,7 @@ double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* 
 double dense_kron_us(int B, int order, const int* idims, const int* odims, int R, bool transposed);
 int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float* Y, cudaStream_t st);
 bool conv_weight_inside(int N, int C, int T, int H, int W, int R);
+int conv_shares(int N, int C, int T, int H, int W, int R, int* out);   // (diagnostic)
 int small_conv_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, const float* const* A, const float* S,
                       bool transposed, const float* X, const float* Wt, float* V, cudaStream_t st);
 // Y = X M (dense) and V = K * X (reshaped-CP conv), or their data gradients (`transposed`), by the form that is

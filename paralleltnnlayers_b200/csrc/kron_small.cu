@@ -524,6 +524,7 @@ struct SmallConvGeom {
   int TR, TC, tilesW, tiles, PXQ;   // tile rows / columns (a multiple of 4), pixel quads in use
   int P, CS;                        // halo row pitch, halo floats per channel
   int buf;                          // floats of the stages (and the sum over the groups); the totals follow
+  int shared;                       // where the cluster's sum is, behind the totals: the same for all CTAs, whatever share of C they have
   int weight;                       // where the weight is that the CTA forms itself, behind all that
 };
 
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
   const bool active = pq < g.PXQ;
   const int pr = active ? pq / (g.TC / 4) : 0, pc = active ? (pq - pr * (g.TC / 4)) * 4 : 0;
   const int steps = ce > cb ? (ce - cb + kCC - 1) / kCC : 0;
-  const ClusterSum shared(smem + g.buf + (steps > kFlush ? 16 * kCT : 0), TT * g.TR * g.TC, g.splits);
+  const ClusterSum shared(smem + g.shared, TT * g.TR * g.TC, g.splits);
   if (steps > 0) load_x(0, cb);
   float* weight = smem + g.weight;   // [channel][tap][TT], then the taps of the ranks
   if constexpr (INSIDE) {
@@ -815,8 +816,10 @@ ConvPlan conv_plan(int N, int C, int T, int H, int W, int R, const DeviceInfo& d
   g.splits = pick_cluster(p.tiles, C, 2 * kCC, di.sm_count);
   g.cper = (int)align_up((size_t)ceil_div(C, g.splits), kCC);
   const int stages = 2 * kCC * g.CS, sums = p.cgroups * tt * g.TR * g.TC;
-  const size_t behind = (ceil_div(g.cper, kCC) > conv_flush(p.cgroups) ? 16 * kCT : 0) + ClusterSum::floats(tt * g.TR * g.TC);
+  const int totals = ceil_div(g.cper, kCC) > conv_flush(p.cgroups) ? 16 * kCT : 0;   // (the last CTA of a cluster may need none)
+  const size_t behind = totals + ClusterSum::floats(tt * g.TR * g.TC);
   g.buf = std::max(stages + 2 * kCC * 9 * tt, sums);
+  g.shared = g.buf + totals;
   p.floats = g.buf + behind;
   // the weight of the CTA's channels and the ranks' taps
   if (g.cper * tt <= kCT && R <= kInside) {
@@ -824,6 +827,7 @@ ConvPlan conv_plan(int N, int C, int T, int H, int W, int R, const DeviceInfo& d
     const size_t weight = align_up(buf + behind, 4), all = weight + (size_t)g.cper * 9 * tt + (size_t)R * kSP;
     if (all * sizeof(float) <= (size_t)di.smem_optin) {
       g.buf = buf;
+      g.shared = buf + totals;
       g.weight = (int)weight;
       p.inside = all;
     }
@@ -1032,6 +1036,18 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
 bool conv_weight_inside(int N, int C, int T, int H, int W, int R) {
   DeviceInfo di;
   return !device_info(&di) && conv_plan(N, C, T, H, W, R, di).inside;
+}
+
+// how a cluster shares out the channels: its CTAs, stages of the first and of the last, stages after which an accumulator is added up
+int conv_shares(int N, int C, int T, int H, int W, int R, int* out) {
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const ConvPlan p = conv_plan(N, C, T, H, W, R, di);
+  out[0] = p.g.splits;
+  out[1] = ceil_div(std::min(C, p.g.cper), kCC);
+  out[2] = ceil_div(std::max(0, C - (p.g.splits - 1) * p.g.cper), kCC);
+  out[3] = conv_flush(p.cgroups);
+  return B200CP_OK;
 }
 
 // V = W * X, the weight in Wt, or (Wt null) formed inside

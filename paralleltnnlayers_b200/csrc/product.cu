@@ -1,7 +1,9 @@
 // Which form of the reshaped-CP conv and the CP dense layer runs: the factored register-tiled kernels, or the weight
 // multiplied out and one product with it.
 #include <algorithm>
+#include <climits>
 
+#include "b200cp_test.h"
 #include "common.cuh"
 
 namespace b200cp {
@@ -154,3 +156,12 @@ int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const i
 }
 
 }  // namespace b200cp
+
+extern "C" int b200cp_test_rcp_product(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int transposed, int flags,
+                                       int* out) {
+  using namespace b200cp;
+  if (int rc = check_kron_modes(order, cdims, tdims, R, "rcp")) return rc;
+  const DensePlan p = rcp_plan(N, H, W, order, cdims, tdims, R, 3, 3, transposed != 0, flags);
+  out[0] = (int)p.form;
+  return conv_shares(N, p.K, p.N, H, W, p.form == Form::inside ? R : INT_MAX, out + 1);
+}

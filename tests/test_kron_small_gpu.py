@@ -72,6 +72,38 @@ def test_rcp_weight_formed_inside(case):
     test_rcp_forward_and_data_gradient(case)
 
 
+# The channels split over a cluster whose last CTA has fewer stages than the others: on the other side of the line from which on accumulators
+# are added to totals (-1), or on the same side (below it 0, above it 1).
+UNEVEN = [
+    (4, (6, 6, 2), (6, 6, 2), 9, 9, 16, False, -1), (4, (6, 6, 2), (6, 6, 2), 9, 9, 16, True, -1), (3, (10, 12), (3, 3), 27, 28, 8, False, -1),
+    (3, (3, 3), (10, 12), 27, 28, 8, True, -1), (2, (3, 3, 8), (3, 3, 8), 23, 23, 4, False, -1), (4, (10, 5, 3), (3, 4, 3), 11, 11, 24, False, -1),
+    (2, (6, 4, 3), (2, 3, 10), 25, 25, 52, False, -1), (14, (6, 12), (6, 12), 7, 7, 20, True, -1), (2, (10, 12), (4, 6), 28, 28, 40, False, -1),
+    (2, (7, 8), (6, 12), 20, 20, 20, False, 0), (2, (13, 8), (6, 12), 20, 20, 20, False, 1),
+]
+
+
+@pytest.mark.parametrize("case", UNEVEN, ids=str)
+def test_rcp_uneven_shares_of_a_cluster(case):
+    import ctypes
+    import paralleltnnlayers_b200 as P
+    from paralleltnnlayers_b200._lib import int_array, lib
+    N, cd, td, H, W, R, transposed, side = case
+    out = (ctypes.c_int * 5)()
+    assert lib.b200cp_test_rcp_product(N, H, W, len(cd), int_array(cd), int_array(td), R, transposed, 8, out) == 0
+    form, ctas, first, last, line = out
+    assert form == 1 and ctas > 1 and first > last
+    assert (first > line, last > line) == {-1: (True, False), 0: (False, False), 1: (True, True)}[side]
+    X, A, S, dV = O.make_rcp_inputs(13, N, cd, td, H, W, 3, 3, R)
+    x, s, dv = dev(X, S, dV)
+    a = dev(*A)
+    if transposed:
+        ref, got = O.rcp_backward(X, dV, A, S)[0], lambda: P.rcp_conv2d_backward(x, dv, *a, s, need_dw=False)[0]
+    else:
+        ref, got = O.rcp_forward(X, A, S), lambda: P.conv2d_rcp_fused_nchw(x, *a, s)
+    for _ in range(3):   # (what is left in shared memory differs from call to call)
+        check(got(), ref, "rcp", atol=1e-5 * max(1.0, float(np.abs(ref).max())))
+
+
 def test_rounding_of_long_sums():
     """4096 inputs and 256 channels x 9 taps, not split over CTAs.  A chain of n fp32 additions of random signs is off by about
     2**-24 * sqrt(n / 6) of its result: 1.9e-7 for the 64 to 72 terms of an accumulator, 1.4e-7 for the at most 32 totals,
