@@ -121,6 +121,7 @@ def _load():
         "b200cp_test_stream_launches": (C.c_longlong, []),
         "b200cp_test_set_planes": (None, [i, i]),
         "b200cp_test_planes_on_tensor_cores": (i, [sp]),
+        "b200cp_test_planes_choice": (i, [sp]),
         "b200cp_test_rcp_product": (i, [i, i, i, i, ip, ip, i, i, i, ip]),
         "b200cp_test_set_p2p_wait_cycles": (None, [C.c_longlong]),
         "b200cp_test_p2p_connect_local": (i, [vp, pp]),

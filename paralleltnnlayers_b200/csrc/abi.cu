@@ -1301,6 +1301,13 @@ const char* b200cp_status_string(int status) {
   }
 }
 
+int b200cp_test_planes_choice(const b200cp_tensor_shape* s) {
+  int out = planes_forms(*s);
+  const Planes uses[] = {Planes::kConv, Planes::kStep, Planes::kSaved, Planes::kFilter, Planes::kSaved3, Planes::kFilter3};
+  for (int i = 0; i < 6; ++i) out |= takes_planes(s, 0, uses[i]) ? 8 << i : 0;
+  return out;
+}
+
 unsigned long long b200cp_launch_count(void) { return g_launches.load(); }
 int b200cp_version(void) { return 100; }
 

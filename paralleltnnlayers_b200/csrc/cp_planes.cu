@@ -1102,6 +1102,10 @@ bool even_products_on_tensor_cores(const b200cp_tensor_shape& s) {
   return planes_tc_mode() == 1 && s.Rank > 16 && s.Rank <= 32 && (size_t)s.H * s.W % 4 == 0 && least >= 96 && most <= 1.5 * least &&
          most <= 8.0 * kTcMaxChunks * kTcK && (double)s.N * s.H * s.W * s.Rank * (most + least) >= 67108864.0;
 }
+bool two_products_on_tensor_cores(const b200cp_tensor_shape& s) {
+  return planes_on_tensor_cores(s).products || even_products_on_tensor_cores(s);
+}
+bool grads_on_tensor_cores(const b200cp_tensor_shape& s) { return planes_on_tensor_cores(s).gradients || grads_by_quads(s); }
 // Units of a CTA of the stencil with correlations: whole turns of its threads, as many as make one to four waves of the five CTAs
 // that an SM has registers for the shortest, where a CTA costs one turn more.  (Eight CTAs per SM and ranges that end
 // within a turn: 32 images of 28x28 at R = 56 took three turns in each of two waves for 2.2 turns of work.  Layer of 16 x 256 -> 384
@@ -1125,7 +1129,7 @@ struct GradPlan {
 GradPlan grad_plan(const b200cp_tensor_shape& s, int sm_count) {
   GradPlan p{};
   const int R = (int)s.Rank, Q = (int)(s.N * s.H * s.W);
-  p.tc = planes_on_tensor_cores(s).gradients || grads_by_quads(s);
+  p.tc = grads_on_tensor_cores(s);
   p.bn = !p.tc && R <= 16 ? 16 : R <= 32 ? 32 : 64;
   p.bm = p.tc || p.bn < 64 ? 128 : 64;
   p.mt0 = ceil_div((int)s.T, p.bm);
@@ -1207,9 +1211,8 @@ int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st
   g.HW = HW;
   g.Q = NQ;
   int np = 0;
-  const bool one = planes_on_tensor_cores(s).products, two = one || even_products_on_tensor_cores(s);
   auto products = [&](bool ak, bool programmatic) {
-    if (np == 2 ? two : one) {
+    if (np == 2 ? two_products_on_tensor_cores(s) : planes_on_tensor_cores(s).products) {
       g.first = !programmatic;
       return tc_launch(g, np, ak, programmatic, di, st);
     }
@@ -1300,6 +1303,10 @@ int planes_device_status(int* out) {
   if (v) B200CP_CUDA_OK(cudaMemcpyToSymbol(g_planes_status, &zero, sizeof(int)));
   *out = v;
   return B200CP_OK;
+}
+
+int planes_forms(const b200cp_tensor_shape& s) {
+  return (planes_on_tensor_cores(s).products ? 1 : 0) | (two_products_on_tensor_cores(s) ? 2 : 0) | (grads_on_tensor_cores(s) ? 4 : 0);
 }
 
 }  // namespace b200cp

@@ -22,5 +22,6 @@ bool planes_supported(const b200cp_tensor_shape& s);
 size_t planes_workspace(const b200cp_tensor_shape& s, int parts);
 int planes_launch(const PlanesJob& j, void* ws, size_t ws_bytes, cudaStream_t st);
 int planes_device_status(int* out);
+int planes_forms(const b200cp_tensor_shape& s);   // on the tensor cores: bit 0 one product, 1 two in a launch, 2 the factor gradients
 
 }  // namespace b200cp

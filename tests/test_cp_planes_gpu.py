@@ -10,6 +10,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
+import test_planes_rule as planes_rule
 from gpu_util import check
 from oracle import cp_oracle as O
 
@@ -82,15 +83,16 @@ def test_cp4(shape, aligned):
         assert_parity(got, ref)
 
 
-# Both sides of the lines between the kernels: two even products in one launch (96 channels, 1.5 times as many, 2**26 multiply-adds), gradients
-# with 16-byte loads from 17 ranks on, rows of a multiple of 4 with many channels (8, 9 and 16 ranks; of a width of the row stream),
-# and steps of few channels with planes that 16-byte loads do not divide (5000 pixels, 80 channels).
+# Shapes near the lines between the kernels, whichever of them the rules choose (test_planes_rule.py says which).
 LINES = [
     (45, 96, 144, 14, 14, 32), (44, 96, 144, 14, 14, 32), (45, 96, 145, 14, 14, 32), (45, 95, 142, 14, 14, 32), (46, 96, 96, 20, 16, 17),
     (1, 8, 8, 4, 4, 17), (1, 8, 8, 4, 4, 16), (2, 64, 64, 8, 12, 8), (1, 100, 60, 12, 12, 9), (1, 144, 136, 6, 24, 12), (1, 136, 136, 6, 24, 12),
     (1, 40, 25, 9, 9, 33), (1, 40, 24, 8, 8, 33), (1, 17, 16, 9, 9, 40),
     (11, 40, 40, 21, 22, 18), (10, 40, 40, 21, 22, 18), (11, 40, 41, 21, 22, 18), (11, 40, 40, 21, 24, 18),
 ]
+
+
+LINES += sorted({s for _, *both in planes_rule.LINES for s in both if s[0] * s[3] * s[4] * (s[1] + s[2]) < 2e6 and s not in LINES})
 
 
 @pytest.mark.parametrize("aligned", [True, False])

@@ -1,0 +1,46 @@
+"""Which calls run over whole rank planes, and which of their products on the tensor cores: a shape on either side of each line of the rules."""
+import ctypes
+
+import pytest
+
+FORMS = ["one", "two", "grads", "conv", "step", "saved", "filter", "saved3", "filter3"]   # bits of b200cp_test_planes_choice
+
+# what a line decides, a shape (N, C, T, H, W, R) past it and one before
+LINES = [
+    # up to 16 ranks: channels per pixel, and where the width is one of the row stream's (8 modulo 16) channels
+    ("conv", (2, 45, 45, 10, 12, 8), (2, 45, 44, 10, 12, 8)), ("conv", (2, 45, 45, 8, 12, 16), (2, 45, 44, 8, 12, 16)),
+    ("conv", (1, 144, 136, 6, 24, 12), (1, 136, 136, 6, 24, 12)), ("conv", (1, 49, 49, 9, 9, 16), (1, 49, 48, 9, 9, 16)),
+    ("step", (2, 38, 38, 9, 9, 8), (2, 38, 37, 9, 9, 8)), ("step", (1, 39, 39, 8, 8, 16), (1, 39, 38, 8, 8, 16)),
+    ("step", (2, 9, 9, 9, 9, 16), (2, 9, 8, 9, 9, 16)), ("saved", (1, 36, 35, 8, 8, 16), (1, 35, 35, 8, 8, 16)),
+    ("filter", (1, 11, 11, 9, 9, 8), (1, 11, 10, 9, 9, 8)), ("filter", (1, 18, 17, 9, 9, 16), (1, 17, 17, 9, 9, 16)),
+    # more ranks: channels, alone or with the pixels
+    ("conv", (1, 112, 112, 9, 9, 24), (1, 112, 111, 9, 9, 24)), ("conv", (32, 112, 111, 28, 28, 17), (32, 111, 111, 28, 28, 17)),
+    ("conv", (1, 50, 50, 5, 5, 40), (1, 50, 49, 5, 5, 40)), ("conv", (10, 48, 47, 27, 30, 40), (10, 47, 47, 27, 30, 40)),
+    ("step", (10, 40, 40, 21, 22, 18), (11, 40, 40, 21, 22, 18)), ("step", (11, 40, 41, 21, 22, 18), (11, 40, 40, 21, 22, 18)),
+    ("step", (11, 40, 40, 21, 24, 18), (11, 40, 40, 21, 22, 18)), ("step", (66, 8, 8, 35, 35, 17), (64, 8, 8, 35, 35, 17)),
+    ("filter", (1, 40, 40, 9, 9, 20), (1, 40, 39, 9, 9, 20)), ("filter", (18, 40, 39, 24, 25, 20), (18, 39, 39, 24, 25, 20)),
+    ("filter", (1, 24, 24, 9, 9, 40), (1, 24, 23, 9, 9, 40)),
+    # products on the tensor cores: channels, pixels, the longest sum, multiply-adds
+    ("one", (16, 40, 25, 8, 8, 33), (16, 40, 24, 8, 8, 33)), ("one", (13, 17, 16, 9, 9, 40), (13, 16, 16, 9, 9, 40)),
+    ("one", (1, 17, 16, 8, 8, 65), (1, 16, 16, 8, 8, 65)), ("one", (13, 25, 25, 9, 9, 40), (12, 25, 25, 9, 9, 40)),
+    ("one", (1, 7168, 24, 20, 20, 65), (1, 7169, 24, 20, 20, 65)), ("one", (64, 384, 384, 14, 14, 32), (64, 320, 320, 14, 14, 32)),
+    ("one", (64, 512, 512, 13, 13, 18), (32, 32, 32, 39, 39, 24)),
+    # two of about as many channels
+    ("two", (45, 96, 144, 14, 14, 32), (44, 96, 144, 14, 14, 32)), ("two", (45, 96, 144, 14, 14, 32), (45, 96, 145, 14, 14, 32)),
+    ("two", (45, 96, 144, 14, 14, 32), (45, 95, 142, 14, 14, 32)), ("two", (1, 7168, 7168, 20, 20, 32), (1, 7169, 7169, 20, 20, 32)),
+    # gradients: ranks, 16-byte loads, channels
+    ("grads", (1, 8, 8, 4, 4, 17), (1, 8, 8, 4, 4, 16)), ("grads", (64, 256, 256, 51, 51, 32), (64, 256, 256, 15, 15, 32)),
+    ("grads", (1, 17, 16, 8, 8, 65), (1, 16, 16, 8, 8, 65)),
+]
+
+
+def chosen(shape):
+    from paralleltnnlayers_b200._lib import TensorShape, lib
+    N, C, T, H, W, R = shape
+    bits = lib.b200cp_test_planes_choice(ctypes.byref(TensorShape(N=N, H=H, W=W, pad=1, T=T, C=C, Y=3, X=3, Rank=R)))
+    return {name for i, name in enumerate(FORMS) if bits >> i & 1}
+
+
+@pytest.mark.parametrize("what, past, before", LINES, ids=str)
+def test_both_sides_of_a_line(lib_built, what, past, before):
+    assert what in chosen(past) and what not in chosen(before)
