@@ -45,8 +45,9 @@ typedef enum b200cp_status {
 /* flags: which arithmetic path runs the two channel contractions. */
 enum {
   B200CP_PATH_AUTO = 0,   /* the fastest fp32-grade path for the shape (mma.sync; with a workspace also FFMA or tcgen05 products
-                           * over whole rank planes, tcgen05 with three bf16 parts per value: 24 bits at any magnitude) */
-  B200CP_PATH_SIMT = 1,   /* exact fp32 FFMA                                        */
+                           * over whole rank planes, tcgen05 with three bf16 parts per value: 24 bits at any magnitude).  An
+                           * infinity comes out as in fp32 over rank planes, as NaN from the mma.sync kernels */
+  B200CP_PATH_SIMT = 1,   /* exact fp32 FFMA (infinities too)                       */
   B200CP_PATH_TC3X = 2,   /* tcgen05 kind::tf32, 3-term split (fp32-grade accuracy) */
   B200CP_PATH_TC1X = 3,   /* tcgen05 kind::tf32, single pass (about 1e-3 relative)  */
   B200CP_PATH_MMA = 4,    /* warp-level mma.sync tf32, 3-term split (fp32-grade)    */

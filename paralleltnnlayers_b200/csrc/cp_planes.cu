@@ -287,6 +287,41 @@ __device__ __forceinline__ void mma_chunk(uint32_t d, uint64_t a, uint64_t A1, u
   for (int i = 0; i < KK; ++i) tc::mma_f16_ss(d, a + i * 2, b + i * 2, idesc, true);
 }
 
+// An infinite value has no three parts: the second is inf - inf, and every sum that meets it comes out NaN.  Such sums are formed anew in
+// fp32, which gives the infinity, or the NaN, that each is.  (Sums of finite values are NaN only where fp32 overflows too.)
+__device__ __forceinline__ float sum_fp32(const float* a, size_t ia, const float* b, size_t ib, int n) {
+  float v = 0.f;
+  for (int k = 0; k < n && v == v; ++k) v = fmaf(a[k * ia], b[k * ib], v);
+  return v;
+}
+template <int N>
+__device__ __forceinline__ bool any_nan(const float (&x)[N]) {   // (or infinities of both signs)
+  float t[N / 2];
+#pragma unroll
+  for (int j = 0; j < N / 2; ++j) t[j] = x[j] + x[N / 2 + j];
+#pragma unroll
+  for (int n = N / 4; n; n /= 2)
+#pragma unroll
+    for (int j = 0; j < n; ++j) t[j] += t[n + j];
+  return t[0] != t[0];
+}
+// rows that a group of the G x 128 threads reads out, 16 at a time
+template <int G>
+__device__ __forceinline__ int group_row(int grp, int nt) { return (grp * nt / G + 15) / 16 * 16; }
+// what this thread read out of a tile
+template <bool AK, int G>
+__device__ __noinline__ void plane_sums_fp32(const PlaneTc& g, int tile, float* sums) {
+  const PlaneTcProduct& a = g.p[blockIdx.z / g.splits];
+  const int t = threadIdx.x & 127, grp = threadIdx.x >> 7, q = tile * kTcPx + t, m0 = blockIdx.y * g.nt;
+  const int kb = (blockIdx.z % g.splits) * a.kper, n = min(a.K, kb + a.kper) - kb, image = q / g.HW, p = q - image * g.HW;
+  if (q >= g.Q) return;
+  for (int r = group_row<G>(grp, g.nt); r < min(group_row<G>(grp + 1, g.nt), a.M - m0); ++r) {
+    float* d = g.splits > 1 ? sums + r * kTcPx + t : a.out + ((size_t)image * a.M + m0 + r) * g.HW + p;
+    const float* F = AK ? a.F + (size_t)(m0 + r) * a.K + kb : a.F + (size_t)kb * a.M + m0 + r;
+    if (*d != *d) *d = sum_fp32(F, AK ? 1 : a.M, a.in + ((size_t)image * a.K + kb) * g.HW + p, g.HW, n);
+  }
+}
+
 template <bool AK, int G>
 __global__ void __launch_bounds__(G * 128, 4 / G) plane_tc_kernel(const __grid_constant__ PlaneTc g) {
   constexpr int kThreads = G * 128;
@@ -418,8 +453,9 @@ __global__ void __launch_bounds__(G * 128, 4 / G) plane_tc_kernel(const __grid_c
     if (tile + gridDim.x >= g.pxtiles) grid_launch_dependents();
     // ---- the accumulators of the chunks, 16 rows at a time
     const size_t inc = g.splits > 1 ? kTcPx : g.HW;
-    const int first = (grp * nt / G + 15) / 16 * 16, last = ((grp + 1) * nt / G + 15) / 16 * 16;   // rows that the group reads out
+    const int first = group_row<G>(grp, nt), last = group_row<G>(grp + 1, nt);
     float* dst = (g.splits > 1 ? sums + t : a.out + ((size_t)px.n * a.M + m0) * g.HW + px.p) + first * inc;
+    bool nan = false;
     for (int c0 = first; c0 < last; c0 += 16) {
       float s[16];
 #pragma unroll
@@ -433,7 +469,9 @@ __global__ void __launch_bounds__(G * 128, 4 / G) plane_tc_kernel(const __grid_c
 #pragma unroll
       for (int j = 0; j < 16; ++j, dst += inc)
         if (c0 + j < rows) *dst = s[j];
+      nan |= any_nan(s);
     }
+    if (nan) plane_sums_fp32<AK, G>(g, tile, sums);
     tc::tc_fence_before_sync();
     __syncthreads();   // the accumulators are free
     tc::tc_fence_after_sync();
@@ -589,6 +627,17 @@ struct GradTile {
   static constexpr size_t smem = 1024 + (size_t)stage;               // at least the [128][NT + 1] floats of the result
 };
 
+// an entry that met an infinite value, over pixels qb .. qe - 1 of rows that the images have `dn` and `zn` of (see sum_fp32)
+__device__ __noinline__ float grad_sum_fp32(const float* D, int dn, const float* Z, int zn, int HW, int qb, int qe) {
+  float v = 0.f;
+  for (int q = qb; q < qe && v == v;) {
+    const int n = q / HW, p = q - n * HW, len = min(HW - p, qe - q);
+    v += sum_fp32(D + (size_t)n * dn * HW + p, 1, Z + (size_t)n * zn * HW + p, 1, len);
+    q += len;
+  }
+  return v;
+}
+
 // VEC: H * W is a multiple of 4 and the rows are 16-byte aligned; a lane has four neighbours of every other row instead of two of each.
 // (Half of the 4300 cycles of a chunk went into addresses and 4-byte loads: gradients in a step of 64 x 256 14x14 at R = 32 16.4 -> 13.2 us,
 // layer of 32 x 128 28x28 at R = 56 84.1 -> 79.8.)
@@ -733,7 +782,7 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
 #pragma unroll
   for (int j = 0; j < NT / 2; ++j) tile[((warp & 3) * 32 + lane) * (NT + 1) + grp * (NT / 2) + j] = tot[j];
   tc::tc_fence_before_sync();
-  __syncthreads();
+  const bool nan = __syncthreads_or(any_nan(tot));
   if (warp == 0) {
     tc::tc_fence_after_sync();
     tc::tmem_dealloc(tmem, 256);
@@ -743,6 +792,12 @@ __global__ void __launch_bounds__(kGradThreads, 2) plane_grad_tc_kernel(const __
     const int m = i / NT, r = i % NT;
     if (r < brows) out[(size_t)m * g.R + r] = tile[m * (NT + 1) + r];
   }
+  if (nan)
+    for (int i = tid; i < arows * NT; i += kGradThreads) {
+      const int m = i / NT, r = i % NT;
+      if (r < brows && tile[m * (NT + 1) + r] != tile[m * (NT + 1) + r])
+        out[(size_t)m * g.R + r] = grad_sum_fp32(D + (size_t)m * g.HW, rows, Z + (size_t)r * g.HW, g.R, g.HW, qb, qe);
+    }
 }
 
 // ---- the same on FFMA ------------------------------------------------------------------------------------------------------

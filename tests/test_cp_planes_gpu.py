@@ -224,6 +224,36 @@ def test_factor_gradients_beside_a_large_sample(form, R, where):
         assert np.linalg.norm(got.view(ref.shape).double().cpu().numpy() - ref) < 1e-6 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("form", [0, 2], indirect=True, ids=["ffma", "tensor"])
+@pytest.mark.parametrize("shape", [(3, 70, 65, 5, 9, 24), (2, 20, 130, 8, 8, 40), (1, 600, 130, 9, 9, 35), (16, 65, 33, 49, 51, 33)], ids=str)
+@pytest.mark.parametrize("where, value", [("input", "inf"), ("gradient", "-inf"), ("factor", "inf")])
+def test_infinities(form, shape, where, value):
+    """An infinite value gives what fp32 arithmetic gives: infinities of its sign, with factors of one sign, and nothing elsewhere."""
+    import paralleltnnlayers_b200 as P
+    X, dU, K = [[np.abs(a) for a in v] if isinstance(v, list) else np.abs(v) for v in make(shape, False)]
+    N, C, T, H, W, R = shape
+    at = {"input": X[N - 1, C - 2], "gradient": dU[N - 1, T - 1], "factor": K[1]}[where]
+    at[H // 2, W - 3 if where != "factor" else R - 2] = float(value)
+    x, du, k = torch.from_numpy(X).cuda(), torch.from_numpy(dU).cuda(), [torch.from_numpy(f).cuda() for f in K]
+    # (over rank planes too: with the factors multiplied out, the padding's zeros would meet infinite weights)
+    ref = [torch.tensor(a, dtype=torch.float64, requires_grad=True) for a in (X, *K)]
+    taps = torch.einsum("yr,xr->ryx", *ref[3:])[:, None]
+    Z = torch.nn.functional.conv2d(torch.einsum("cr,nchw->nrhw", ref[2], ref[0]), taps, padding=1, groups=R)
+    y = torch.einsum("tr,nrhw->nthw", ref[1], Z)
+    want = [g.detach().numpy() for g in (y, *torch.autograd.grad(y, ref, torch.tensor(dU, dtype=torch.float64)))]
+    U, dX, dK = P.cp4_conv2d_step(x, du, *k)
+    dK = [g.view(r.shape) for g, r in zip(torch.split(dK.flatten(), [w.size for w in want[2:]]), want[2:])]
+    many = 0
+    for got, ref in zip((U, dX, *dK), want):
+        got, fin = got.cpu().double().numpy(), np.isfinite(ref)
+        assert not np.isnan(ref).any()
+        assert np.array_equal(got[~fin], ref[~fin])
+        assert np.abs(got[fin] - ref[fin]).max(initial=0) <= 1e-5 * np.abs(ref[fin]).max(initial=0)
+        many += (~fin).sum()
+    assert many
+    P.device_status()
+
+
 def test_more_than_7168_channels():
     """The sum over the channels on the tensor cores ends at 7168 channels (ranks); the products take more, on FFMA, in the same
     launches."""
