@@ -58,7 +58,8 @@ int b200cp_test_planes_on_tensor_cores(const b200cp_tensor_shape* s);
 
 /* What the rules choose for a shape (3x3, pad 1) on the default path.  Over rank planes, on the tensor cores: bit 0 one product, bit 1 two
  * products in one launch, bit 2 the factor gradients.  Run over rank planes, where the workspace is there: bit 3 one convolution, bit 4
- * the step, bit 5 the CP4 backward from the forward's plane, bit 6 the CP4 factor gradients, bits 7 and 8 the last two of CP3. */
+ * the step, bit 5 the CP4 backward from the forward's plane, bit 6 the CP4 factor gradients, bits 7 and 8 the last two of CP3,
+ * bit 9 a convolution that saves its plane, bit 10 the CP4 factor gradients from both planes. */
 int b200cp_test_planes_choice(const b200cp_tensor_shape* s);
 
 /* How the 3x3 reshaped-CP convolution (`transposed`: its data gradient) runs: out[0] 0 factored, 1 the weight multiplied out and an FFMA product,

@@ -116,8 +116,14 @@ const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
   return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
 }();
-// one convolution; the step; the backward from the forward's plane; the factor gradients; the last two of CP3
-enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3 };
+// one convolution; the step; the backward from the forward's plane; the factor gradients; the last two of CP3; a layer's forward, which keeps
+// its plane; the factor gradients of a layer's backward, from both planes.
+// A layer's forward and backward take the host about 90 us, whatever runs on the GPU, and a launch more 2 to 3: where the GPU takes less,
+// a convolution in three launches instead of one only loses.  So below 10^7 inputs and outputs the last two have lines of their own.  Of 191 layers
+// drawn between the two lines those below took 1.06 times as long with the lines of kConv, calls one after the other (58 x 208 -> 296
+// 12x12 at R = 12 93.9 -> 101.3 us, on the device alone 50.5 -> 29.2), those above 0.91 times (59 x 460 32x32 at R = 4 307 -> 254).  Of 109
+// at the lines of kFilter as many gained as lost.
+enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3, kConvSaved, kFilterSaved };
 bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   const int forced = g_planes_test.load(std::memory_order_relaxed), planes = forced < 0 ? g_planes : forced;
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !planes || !planes_supported(*s)) return false;
@@ -128,10 +134,14 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
     const bool low = s->Rank <= 8, rows = s->W % 4 == 0 && band_max_rank() == 16;   // (a caller who sets it wants the row bands)
     const bool streams = s->W % 16 == 8 && s->W <= 56 && s->C % 8 == 0 && s->T % 8 == 0;   // widths of the row stream
     switch (use) {
+      case Planes::kConvSaved:
+        if (rows && ch * s->N * s->H * s->W < 1e7) return false;
+        [[fallthrough]];
       case Planes::kConv: return rows ? (streams ? ch >= 280 : few >= (low ? 64 : 96)) : !low && few >= 130 && s->W % 4;
       case Planes::kStep: return few >= (low ? 60 : s->W % 4 == 0 ? 110 : 20);
       case Planes::kSaved: return few >= 100;
       case Planes::kFilter: return few >= (low ? 20 : 46);
+      case Planes::kFilterSaved: return few >= 42;
       case Planes::kFilter3: return few >= 47;
       default: return ch >= 64 && few >= 27;
     }
@@ -142,6 +152,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   };
   switch (use) {
     case Planes::kConv: return past({224, 100, 0}, {2800, 900, 0});
+    case Planes::kConvSaved: return past({256, 129, 0}, {2800, 1000, 0});
     case Planes::kStep:   // (few channels, 5000 to 80000 pixels and planes that 16-byte loads do not divide: planes / tile kernels 1.10 over 30
                           // shapes that the line was not fitted on, 98.8 / 72.0 us at 42 x 33 -> 6 x 27x58, R = 29; from 80000 pixels on 0.90
                           // over 12, 303 / 395 us at 119 x 20 -> 25 x 46x57, R = 17)
@@ -150,6 +161,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
       if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // (measured: narrow layers with odd rows lose)
       return past({160, 0, 0}, {2200, 0, 0});
     case Planes::kFilter: return past({80, 48, 0}, {800, 490, 0});
+    case Planes::kFilterSaved:
     case Planes::kFilter3: return past({129, 48, 0}, {2200, 490, 0});
     default: return past({129, 40, 0}, {2200, 400, 0});
   }
@@ -248,7 +260,7 @@ int b200cp_cp4_bwd_data(const b200cp_tensor_shape* s, const float* dU, const flo
 
 // ---- the convolutions with a workspace, and the whole backward from the forward's rank plane ----------------------
 static size_t conv_ws_bytes(const b200cp_tensor_shape* s, int part, int saves_plane, int flags) {
-  if (!takes_planes(s, flags, Planes::kConv)) return 0;
+  if (!takes_planes(s, flags, saves_plane ? Planes::kConvSaved : Planes::kConv)) return 0;
   return planes_workspace(*s, part | (saves_plane ? kPlanesNoP | kPlanesNoQ : 0));
 }
 static bool has_ws(const void* ws, size_t have, size_t need) {
@@ -858,7 +870,7 @@ int b200cp_cp4_fwd_bwd_data(const b200cp_tensor_shape* s, const float* X, const 
 size_t b200cp_cp4_bwd_filter_saved_workspace_bytes(const b200cp_tensor_shape* s, int flags) {
   if (check_shape(s, "b200cp_cp4_bwd_filter_saved_workspace_bytes")) return 0;
   const size_t need = std::max(cp4_bwd_filter_saved_workspace(*s), cp4_grad_band_workspace(*s));
-  return takes_planes(s, flags, Planes::kFilter) ? std::max(need, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ)) : need;
+  return takes_planes(s, flags, Planes::kFilterSaved) ? std::max(need, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ)) : need;
 }
 
 int b200cp_cp4_bwd_filter_saved(const b200cp_tensor_shape* s, const float* X, const float* dU, const float* P,
@@ -869,7 +881,7 @@ int b200cp_cp4_bwd_filter_saved(const b200cp_tensor_shape* s, const float* X, co
   if (!step_shares_planes(s, flags))
     return fail(B200CP_ERR_UNSUPPORTED, "b200cp_cp4_bwd_filter_saved: 3x3 filters with pad 1 on the default (mma) path only");
   if (!workspace) return fail(B200CP_ERR_WORKSPACE, "b200cp_cp4_bwd_filter_saved: workspace is null");
-  if (takes_planes(s, flags, Planes::kFilter) &&
+  if (takes_planes(s, flags, Planes::kFilterSaved) &&
       has_ws(workspace, workspace_bytes, planes_workspace(*s, kPlanesGrads | kPlanesNoP | kPlanesNoQ))) {
     PlanesJob j;
     j.s = s; j.X = X; j.dU = dU; j.P = P; j.Q = Q; j.KH = KH; j.KW = KW; j.dK = dK_packed;
@@ -1303,8 +1315,9 @@ const char* b200cp_status_string(int status) {
 
 int b200cp_test_planes_choice(const b200cp_tensor_shape* s) {
   int out = planes_forms(*s);
-  const Planes uses[] = {Planes::kConv, Planes::kStep, Planes::kSaved, Planes::kFilter, Planes::kSaved3, Planes::kFilter3};
-  for (int i = 0; i < 6; ++i) out |= takes_planes(s, 0, uses[i]) ? 8 << i : 0;
+  const Planes uses[] = {Planes::kConv,   Planes::kStep,    Planes::kSaved,     Planes::kFilter,
+                         Planes::kSaved3, Planes::kFilter3, Planes::kConvSaved, Planes::kFilterSaved};
+  for (int i = 0; i < 8; ++i) out |= takes_planes(s, 0, uses[i]) ? 8 << i : 0;
   return out;
 }
 

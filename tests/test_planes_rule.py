@@ -3,7 +3,7 @@ import ctypes
 
 import pytest
 
-FORMS = ["one", "two", "grads", "conv", "step", "saved", "filter", "saved3", "filter3"]   # bits of b200cp_test_planes_choice
+FORMS = ["one", "two", "grads", "conv", "step", "saved", "filter", "saved3", "filter3", "conv, plane kept", "filter from planes"]   # bits of b200cp_test_planes_choice
 
 # what a line decides, a shape (N, C, T, H, W, R) past it and one before
 LINES = [
@@ -20,6 +20,11 @@ LINES = [
     ("step", (11, 40, 40, 21, 24, 18), (11, 40, 40, 21, 22, 18)), ("step", (66, 8, 8, 35, 35, 17), (64, 8, 8, 35, 35, 17)),
     ("filter", (1, 40, 40, 9, 9, 20), (1, 40, 39, 9, 9, 20)), ("filter", (18, 40, 39, 24, 25, 20), (18, 39, 39, 24, 25, 20)),
     ("filter", (1, 24, 24, 9, 9, 40), (1, 24, 23, 9, 9, 40)),
+    # a layer: its convolution by the values in and out where the line above is of launches, older lines elsewhere
+    ("conv, plane kept", (16, 170, 170, 39, 48, 16), (16, 170, 170, 38, 48, 16)), ("conv, plane kept", (32, 224, 224, 28, 28, 8), (2, 45, 45, 10, 12, 8)),
+    ("conv, plane kept", (1, 49, 49, 9, 9, 16), (1, 49, 48, 9, 9, 16)), ("conv, plane kept", (1, 128, 128, 9, 9, 24), (1, 128, 127, 9, 9, 24)),
+    ("conv, plane kept", (1, 65, 64, 5, 5, 40), (1, 64, 64, 5, 5, 40)), ("filter from planes", (1, 16, 16, 9, 9, 16), (1, 16, 15, 9, 9, 16)),
+    ("filter from planes", (1, 65, 64, 9, 9, 20), (1, 64, 64, 9, 9, 20)),
     # products on the tensor cores: channels, pixels, the longest sum, multiply-adds
     ("one", (16, 40, 25, 8, 8, 33), (16, 40, 24, 8, 8, 33)), ("one", (13, 17, 16, 9, 9, 40), (13, 16, 16, 9, 9, 40)),
     ("one", (1, 17, 16, 8, 8, 65), (1, 16, 16, 8, 8, 65)), ("one", (13, 25, 25, 9, 9, 40), (12, 25, 25, 9, 9, 40)),
