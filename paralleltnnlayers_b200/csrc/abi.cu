@@ -137,7 +137,9 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
       case Planes::kConvSaved:
         if (rows && ch * s->N * s->H * s->W < 1e7) return false;
         [[fallthrough]];
-      case Planes::kConv: return rows ? (streams ? ch >= 280 : few >= (low ? 64 : 96)) : !low && few >= 130 && s->W % 4;
+      case Planes::kConv:   // (row-stream widths of 9 to 16 ranks below the line of the others: planes 1.03 over 8)
+        if (!rows) return !low && few >= 130 && s->W % 4;
+        return (!streams || ch >= 280) && few >= (low ? streams ? 0 : 64 : 96);
       case Planes::kStep: return few >= (low ? 60 : s->W % 4 == 0 ? 110 : 20);
       case Planes::kSaved: return few >= 100;
       case Planes::kFilter: return few >= (low ? 20 : 46);
@@ -151,7 +153,12 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
     return ch >= least[ranks] || ch * root4 >= weighted[ranks];
   };
   switch (use) {
-    case Planes::kConv: return past({224, 100, 0}, {2800, 900, 0});
+    case Planes::kConv:   // below the lines of kConvSaved, planes / tile kernels over drawn shapes:
+      // 17 to 32 ranks, 224 to 255 channels: 2000 to 12000 pixels 0.89 (50), fewer 1.07 (27), more 1.00 (23)
+      if (ranks == 0 && ch >= 224 && root4 >= 6.7 && root4 < 10.5) return true;
+      // 33 to 64 ranks, 100 to 128 channels: 0.70 where inputs and outputs are 32 and more (54), 1.10 where one of them is less (36)
+      if (ranks == 1 && ch >= 100 && s->C >= 32 && s->T >= 32) return true;
+      [[fallthrough]];
     case Planes::kConvSaved: return past({256, 129, 0}, {2800, 1000, 0});
     case Planes::kStep:   // (few channels, 5000 to 80000 pixels and planes that 16-byte loads do not divide: planes / tile kernels 1.10 over 30
                           // shapes that the line was not fitted on, 98.8 / 72.0 us at 42 x 33 -> 6 x 27x58, R = 29; from 80000 pixels on 0.90

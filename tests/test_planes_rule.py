@@ -10,12 +10,17 @@ LINES = [
     # up to 16 ranks: channels per pixel, and where the width is one of the row stream's (8 modulo 16) channels
     ("conv", (2, 45, 45, 10, 12, 8), (2, 45, 44, 10, 12, 8)), ("conv", (2, 45, 45, 8, 12, 16), (2, 45, 44, 8, 12, 16)),
     ("conv", (1, 144, 136, 6, 24, 12), (1, 136, 136, 6, 24, 12)), ("conv", (1, 49, 49, 9, 9, 16), (1, 49, 48, 9, 9, 16)),
+    ("conv", (54, 160, 160, 24, 24, 16), (56, 160, 160, 24, 24, 16)),
     ("step", (2, 38, 38, 9, 9, 8), (2, 38, 37, 9, 9, 8)), ("step", (1, 39, 39, 8, 8, 16), (1, 39, 38, 8, 8, 16)),
     ("step", (2, 9, 9, 9, 9, 16), (2, 9, 8, 9, 9, 16)), ("saved", (1, 36, 35, 8, 8, 16), (1, 35, 35, 8, 8, 16)),
     ("filter", (1, 11, 11, 9, 9, 8), (1, 11, 10, 9, 9, 8)), ("filter", (1, 18, 17, 9, 9, 16), (1, 17, 17, 9, 9, 16)),
     # more ranks: channels, alone or with the pixels
-    ("conv", (1, 112, 112, 9, 9, 24), (1, 112, 111, 9, 9, 24)), ("conv", (32, 112, 111, 28, 28, 17), (32, 111, 111, 28, 28, 17)),
-    ("conv", (1, 50, 50, 5, 5, 40), (1, 50, 49, 5, 5, 40)), ("conv", (10, 48, 47, 27, 30, 40), (10, 47, 47, 27, 30, 40)),
+    ("conv", (1, 112, 112, 46, 46, 24), (1, 112, 111, 46, 46, 24)), ("conv", (1, 112, 112, 46, 46, 24), (1, 112, 112, 44, 44, 24)),
+    ("conv", (1, 112, 112, 110, 110, 24), (1, 112, 112, 111, 111, 24)), ("conv", (1, 128, 128, 9, 9, 24), (1, 128, 127, 9, 9, 24)),
+    ("conv", (32, 112, 111, 28, 28, 17), (32, 111, 111, 28, 28, 17)),
+    ("conv", (1, 50, 50, 5, 5, 40), (1, 50, 49, 5, 5, 40)), ("conv", (1, 32, 70, 5, 5, 40), (1, 31, 71, 5, 5, 40)),
+    ("conv", (1, 70, 32, 5, 5, 40), (1, 71, 31, 5, 5, 40)), ("conv", (1, 9, 120, 5, 5, 40), (1, 9, 119, 5, 5, 40)),
+    ("conv", (10, 48, 48, 35, 36, 40), (10, 47, 47, 35, 36, 40)),
     ("step", (10, 40, 40, 21, 22, 18), (11, 40, 40, 21, 22, 18)), ("step", (11, 40, 41, 21, 22, 18), (11, 40, 40, 21, 22, 18)),
     ("step", (11, 40, 40, 21, 24, 18), (11, 40, 40, 21, 22, 18)), ("step", (66, 8, 8, 35, 35, 17), (64, 8, 8, 35, 35, 17)),
     ("filter", (1, 40, 40, 9, 9, 20), (1, 40, 39, 9, 9, 20)), ("filter", (18, 40, 39, 24, 25, 20), (18, 39, 39, 24, 25, 20)),
