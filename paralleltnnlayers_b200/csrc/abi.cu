@@ -129,6 +129,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !planes || !planes_supported(*s)) return false;
   if (planes == 2) return true;
   const double ch = (double)s->C + s->T, root4 = std::sqrt(std::sqrt((double)s->N * s->H * s->W));
+  const bool quads = (size_t)s->H * s->W % 4 == 0;   // (the FFMA products and the gradients load 16 bytes of a plane)
   if (s->Rank <= 16) {
     const double few = ch * std::sqrt((double)s->Rank) / root4;
     const bool low = s->Rank <= 8, rows = s->W % 4 == 0 && band_max_rank() == 16;   // (a caller who sets it wants the row bands)
@@ -140,7 +141,11 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
       case Planes::kConv:   // (row-stream widths of 9 to 16 ranks below the line of the others: planes 1.03 over 8)
         if (!rows) return !low && few >= 130 && s->W % 4;
         return (!streams || ch >= 280) && few >= (low ? streams ? 0 : 64 : 96);
-      case Planes::kStep: return few >= (low ? 60 : s->W % 4 == 0 ? 110 : 20);
+      case Planes::kStep:   // Planes / row or tile kernels over drawn shapes below 110: a width of a multiple of 4, up to 8 ranks: 0.79 from 10000 pixels
+        // on (33), 1.02 before, where the launches take the host longer (35).  Others whose planes are a multiple of 4: 0.86 (229); 4-byte loads:
+        // 0.90 up to 20000 pixels (365), from there on 1.04 (160)
+        if (s->W % 4 == 0) return few >= (low && root4 >= 10 ? 60 : 110);
+        return few >= (quads || root4 < 11.9 ? low ? 60 : 20 : 110);
       case Planes::kSaved: return few >= 100;
       case Planes::kFilter: return few >= (low ? 20 : 46);
       case Planes::kFilterSaved: return few >= 42;
@@ -160,10 +165,8 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
       if (ranks == 1 && ch >= 100 && s->C >= 32 && s->T >= 32) return true;
       [[fallthrough]];
     case Planes::kConvSaved: return past({256, 129, 0}, {2800, 1000, 0});
-    case Planes::kStep:   // (few channels, 5000 to 80000 pixels and planes that 16-byte loads do not divide: planes / tile kernels 1.10 over 30
-                          // shapes that the line was not fitted on, 98.8 / 72.0 us at 42 x 33 -> 6 x 27x58, R = 29; from 80000 pixels on 0.90
-                          // over 12, 303 / 395 us at 119 x 20 -> 25 x 46x57, R = 17)
-      return ranks || (size_t)s->H * s->W % 4 == 0 || ch > 80 || root4 <= 8.4 || root4 >= 16.8;
+    case Planes::kStep:   // (17 to 32 ranks, 4-byte loads, below the last two lines: 0.89 up to 5000 pixels (159), from there on 1.02 (48); 16-byte loads 0.80)
+      return quads || root4 < 8.4 || past({200, 0, 0}, {1300, 0, 0});
     case Planes::kSaved:
       if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // (measured: narrow layers with odd rows lose)
       return past({160, 0, 0}, {2200, 0, 0});
