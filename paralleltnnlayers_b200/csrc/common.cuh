@@ -241,10 +241,10 @@ struct KronWeight {   // of a product with the multiplied-out weight: rows are t
 double rcp_factored_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, int FH, int FW,
                        bool transposed, double enough);
 double dense_factored_us(int B, int order, const int* idims, const int* odims, int R, bool transposed, double enough);
-double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, bool transposed);
+// *inside: whether the product's CTAs form the weight themselves
+double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, bool transposed, bool* inside);
 double dense_kron_us(int B, int order, const int* idims, const int* odims, int R, bool transposed);
 int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float* Y, cudaStream_t st);
-bool conv_weight_inside(int N, int C, int T, int H, int W, int R);
 int conv_shares(int N, int C, int T, int H, int W, int R, int* out);   // (diagnostic)
 int small_conv_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, const float* const* A, const float* S,
                       bool transposed, const float* X, const float* Wt, float* V, cudaStream_t st);

@@ -868,7 +868,7 @@ double dense_kron_us(int B, int order, const int* idims, const int* odims, int R
          (p.bm == 64 ? 7.93e-6 : p.bm == 32 ? 9.39e-6 : 7.69e-6) * work + 1.54e-6 * ((double)B * K + (double)B * N);
 }
 
-double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, bool transposed) {
+double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, bool transposed, bool* inside) {
   DeviceInfo di;
   if (device_info(&di)) return -1;
   int C = 1, T = 1;
@@ -878,6 +878,7 @@ double rcp_kron_us(int N, int H, int W, int order, const int* cdims, const int* 
   }
   const ConvPlan p = conv_plan(N, C, T, H, W, R, di);
   const SmallConvGeom& g = p.g;
+  *inside = p.inside > 0;
   const int px = kCT / p.cgroups / (p.tt / 4) * 4;
   const double w = waves(p.tiles * g.splits, di) * g.cper;
   return 5.1 + (p.inside ? 0.2 * R : kron_weight_us(order, cdims, tdims, R, 9, transposed)) +
@@ -1030,12 +1031,6 @@ int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float
 #undef SMALL_GEMM
   B200CP_LAUNCH_OK("small_gemm_kernel");
   return B200CP_OK;
-}
-
-// whether the CTAs of the product form the weight themselves (then it needs no workspace)
-bool conv_weight_inside(int N, int C, int T, int H, int W, int R) {
-  DeviceInfo di;
-  return !device_info(&di) && conv_plan(N, C, T, H, W, R, di).inside;
 }
 
 // how a cluster shares out the channels: its CTAs, stages of the first and of the last, stages after which an accumulator is added up

@@ -90,7 +90,8 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
   if (FH != 3 || FW != 3) return p;
   p.K = (int)prod(transposed ? tdims : cdims, order);
   p.N = (int)prod(transposed ? cdims : tdims, order);
-  const double ffma = rcp_kron_us(N, H, W, order, cdims, tdims, R, transposed);
+  bool inside = false;
+  const double ffma = rcp_kron_us(N, H, W, order, cdims, tdims, R, transposed, &inside);
   const bool may = tensor_may(flags, R, 9.0 * N * H * W * p.K * p.N) && conv_tc_takes(N, p.K, p.N, H, W);
   const size_t planes = may ? align_up(conv_tc_scratch_floats(N, p.K, p.N, H, W) * sizeof(float), 256) : 0;
   const double tensor = may && planes <= kMostPlanes
@@ -103,7 +104,7 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
     p.bytes = planes;
   } else if (p.form == Form::ffma) {
     p.bytes = align_up(p.weight * sizeof(float), 256);   // (a call without it runs the factored kernels; unused where the weight is formed inside)
-    if (conv_weight_inside(N, p.K, p.N, H, W, R)) p.form = Form::inside;
+    if (inside) p.form = Form::inside;
   }
   return p;
 }
