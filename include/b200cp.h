@@ -240,7 +240,7 @@ int b200cp_rcp_fwd(int N, int H, int W, int order, const int* cdims, const int* 
                    const float* X, const float* const* A, const float* S, float* V, void* stream, int flags);
 
 /* The same with a workspace (16-byte aligned; b200cp_rcp_fwd_workspace_bytes bytes), in which the layer's weight is multiplied
- * out.  The size is 0 where the factored kernels are estimated to be faster (low ranks, many pixels), at most 256 MB where
+ * out (256 bytes where the weight is small enough to be formed in shared memory).  The size is 0 where the factored kernels are estimated to be faster (low ranks, many pixels), at most 256 MB where
  * they take the layer, and up to 4 GB for layers that only this call takes.  Too small or NULL: as b200cp_rcp_fwd. */
 size_t b200cp_rcp_fwd_workspace_bytes(int N, int H, int W, int order, const int* cdims, const int* tdims, int R,
                                       int FH, int FW, int flags);

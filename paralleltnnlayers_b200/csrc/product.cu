@@ -103,7 +103,8 @@ DensePlan rcp_plan(int N, int H, int W, int order, const int* cdims, const int* 
   if (p.form == Form::tensor) {
     p.bytes = planes;
   } else if (p.form == Form::ffma) {
-    p.bytes = align_up(p.weight * sizeof(float), 256);   // (a call without it runs the factored kernels; unused where the weight is formed inside)
+    // (formed inside nothing is stored; but a call without a workspace runs the factored kernels, so this one asks for some)
+    p.bytes = inside ? 256 : align_up(p.weight * sizeof(float), 256);
     if (inside) p.form = Form::inside;
   }
   return p;

@@ -72,6 +72,28 @@ def test_rcp_weight_formed_inside(case):
     test_rcp_forward_and_data_gradient(case)
 
 
+def test_workspace_of_a_weight_formed_inside():
+    """The launch that forms the weight itself takes none of the weight's size, and a call without any runs the factored kernels."""
+    import ctypes
+    import torch
+    from paralleltnnlayers_b200._lib import int_array, lib, ptr_array
+    N, cd, td, H, W, R = 2, (4, 4), (4, 4), 9, 8, 16
+    X, A, S, _ = O.make_rcp_inputs(14, N, cd, td, H, W, 3, 3, R)
+    x, s, *a = dev(X, S, *A)
+    shape = (N, H, W, 2, int_array(cd), int_array(td), R, 3, 3)
+    assert lib.b200cp_rcp_fwd_workspace_bytes(*shape, 8) == 256
+    ws = torch.empty(256, dtype=torch.uint8, device="cuda")
+    ref = O.rcp_forward(X, A, S)
+    for pointer, size in ((ws.data_ptr(), 256), (None, 0)):
+        v = torch.empty(ref.shape, device="cuda")
+        before = lib.b200cp_launch_count()
+        vp = ctypes.c_void_p
+        assert lib.b200cp_rcp_fwd_ws(*shape, vp(x.data_ptr()), ptr_array([t.data_ptr() for t in a]), vp(s.data_ptr()), vp(v.data_ptr()),
+                                     vp(pointer), size, vp(torch.cuda.current_stream().cuda_stream), 8) == 0
+        assert lib.b200cp_launch_count() - before == 1
+        check(v, ref, "rcp", atol=1e-5 * max(1.0, float(np.abs(ref).max())))
+
+
 # The channels split over a cluster whose last CTA has fewer stages than the others: on the other side of the line from which on accumulators
 # are added to totals (-1), or on the same side (below it 0, above it 1).
 UNEVEN = [
