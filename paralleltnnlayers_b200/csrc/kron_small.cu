@@ -402,7 +402,7 @@ struct GemmTile {
   static size_t smem(int kper) { return sizeof(float) * ((size_t)buf + (is_long(kper) ? 16 * NT : 0) + ClusterSum::floats(BM * BN)); }
 };
 
-// LONG: more than kChain terms per accumulator (without the totals 16.5 instead of 17.0 us for 4096 -> 64 at batch 64)
+// LONG: more than kChain terms per accumulator (4096 -> 64 at batch 64, whose chains are short enough, 12.6 us without the totals and 12.9 with)
 template <int BM, int BN, bool VECA, bool LONG>
 __global__ void __launch_bounds__(GemmTile<BM, BN>::NT) small_gemm_kernel(const float* __restrict__ X, const float* __restrict__ W,
                                                          float* __restrict__ Y, int M, int N, int K, int ldw, int kper,
@@ -839,9 +839,13 @@ double waves(long ctas, const DeviceInfo& di) { return (double)((ctas + di.sm_co
 
 }  // namespace
 
-// Estimated microseconds of the two forms: waves of CTAs times the work of one, and the weight's entries written.  Least-
-// squares fit to the layers that the factored kernels' estimate is fitted to (chain_simt.cu).  Choosing by the two, 5 of
-// 1202 layers run more than 10 % and 2 us behind the other form, and all together 0.3 % behind the best choice.
+// Estimated microseconds of the two forms: waves of CTAs times the work of one, and the weight's entries written.  The coefficients are a
+// least-squares fit to the first form of these kernels (tiles of 16 and more rows, 4 x 4 values per thread of the weight, cluster sums by
+// reads); with the present ones the estimates are 0.84 to 1.18 of the time of eight of ten products (formed inside: 1.05 to 1.45).  They only
+// have to choose: over 1000 drawn products (one to four modes of 1-16, up to 8192 features or 1024 channels, batches to 8192 and images to
+// 64 x 64, ranks 1-300), each measured in every form that takes it, the choice is 0.6 % behind the best one all together, and 16 products
+// run more than 10 % and 2 us behind: 35 samples 3000 -> 1920 at R = 16 84 us on the tensor cores and 55 here, 69 samples 30 -> 30 at R = 1 10.2
+// here and 7.2 factored.
 double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed) {
   DeviceInfo di;
   if (device_info(&di)) return 1e300;
