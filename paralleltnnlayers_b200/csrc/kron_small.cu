@@ -954,8 +954,10 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   const dim3 grid(p.nb, ceil_div(p.PA, ta), splits);
 #define KRON_T(TAV, TAPV)                                                                                               \
   do {                                                                                                                  \
-    static std::atomic<int> set[64];                                                                                    \
-    B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_weight_kernel<TAV, TAPV>), set, (int)kron_smem<TAV>())); \
+    if constexpr (kron_smem<TAV>() > 44 * 1024) {   /* (48 KB with the offsets need no limit raised) */                  \
+      static std::atomic<int> set[64];                                                                                  \
+      B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_weight_kernel<TAV, TAPV>), set, (int)kron_smem<TAV>())); \
+    }                                                                                                                   \
     B200CP_CUDA_OK(launch_cluster(kron_weight_kernel<TAV, TAPV>, grid, dim3(kKT), kron_smem<TAV>(), st, splits, false, g, W)); \
   } while (0)
 #define KRON(TAV)                                                                                                       \
