@@ -721,9 +721,10 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
 
 // Dynamic shared memory that lets no more CTAs share an SM than the grid needs: CTAs of a programmatic dependent start
 // while the kernel before drains and would otherwise be stacked on the SMs that are free first.
+// (A GPC of fewer than 16 SMs has room for one cluster of 8 only: with a CTA per SM 15 clusters are resident at once, 16 are not.  128 -> 16
+// channels 7x7 at R = 18, images = clusters, a CTA per SM / two: 11 8.0 / 9.3 us, 14 8.2 / 9.5, 15 8.4 / 9.4, 16 11.9 / 9.6.)
 size_t spread_smem(size_t need, long ctas, int cluster, const DeviceInfo& di) {
-  // (a GPC of fewer than 16 SMs has room for one cluster of 8 only)
-  const long per = std::max<long>((ctas + di.sm_count - 1) / di.sm_count, cluster == 8 && ctas > 64 ? 2 : 1);
+  const long per = std::max<long>((ctas + di.sm_count - 1) / di.sm_count, cluster == 8 && ctas > 14 * 8 ? 2 : 1);
   return per > 4 ? need : std::max(need, (size_t)di.smem_optin / per - (per > 1 ? 1024 : 0));
 }
 
