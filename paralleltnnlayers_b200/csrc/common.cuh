@@ -219,11 +219,12 @@ int dense_fast_launch(int B, const int* fsi, const int* fso, int R, const float*
 int dense_chain_launch(int B, int order, const int* idims, const int* odims, int R, const float* X,
                        const float* const* F, float* Y, bool transposed, cudaStream_t st);
 // The two layers by their multiplied-out weight (kron_small.cu).  Weight: W[slow][ld] or, with S, W[slow][tap][ld];
-// slow = inputs and fast = outputs, or the other way round with `transposed`; `flip`: taps back to front.
+// slow = inputs and fast = outputs, or the other way round with `transposed`; `flip`: taps back to front; `stacked`: the launch that
+// follows puts two CTAs on an SM.
 int kron_weight_ld(int fast);
 double kron_weight_us(int order, const int* idims, const int* odims, int R, int taps, bool transposed);
 int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
-                       int taps, bool transposed, bool flip, float* W, cudaStream_t st);
+                       int taps, bool transposed, bool flip, float* W, cudaStream_t st, bool stacked = false);
 // the same as operand planes of the tensor-core product: rows of ldo values, hi and `plane` on lo, an exponent per row
 bool kron_planes_takes(int order, const int* idims, const int* odims, int R, int sm_count);   // where that is faster
 int kron_planes_launch(int order, const int* idims, const int* odims, int R, const float* const* F, bool transposed, int ldo,
@@ -247,7 +248,7 @@ double dense_kron_us(int B, int order, const int* idims, const int* odims, int R
 int small_gemm_launch(int M, int N, int K, const float* X, const float* W, float* Y, cudaStream_t st);
 int conv_shares(int N, int C, int T, int H, int W, int R, int* out);   // (diagnostic)
 int small_conv_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, const float* const* A, const float* S,
-                      bool transposed, const float* X, const float* Wt, float* V, cudaStream_t st);
+                      bool transposed, const float* X, float* Wt, float* V, cudaStream_t st);
 // Y = X M (dense) and V = K * X (reshaped-CP conv), or their data gradients (`transposed`), by the form that is
 // fastest for the sizes (product.cu); the workspace may be null (or too small): then the factored kernels run.
 size_t dense_product_workspace(int B, int order, const int* idims, const int* odims, int R, bool transposed, int flags);

@@ -723,8 +723,9 @@ __global__ void __launch_bounds__(kCT) small_conv_kernel(const SmallConvGeom g, 
 // while the kernel before drains and would otherwise be stacked on the SMs that are free first.
 // (A GPC of fewer than 16 SMs has room for one cluster of 8 only: with a CTA per SM 15 clusters are resident at once, 16 are not.  128 -> 16
 // channels 7x7 at R = 18, images = clusters, a CTA per SM / two: 11 8.0 / 9.3 us, 14 8.2 / 9.5, 15 8.4 / 9.4, 16 11.9 / 9.6.)
+bool paired_clusters(long ctas, int cluster) { return cluster == 8 && ctas > 14 * 8; }
 size_t spread_smem(size_t need, long ctas, int cluster, const DeviceInfo& di) {
-  const long per = std::max<long>((ctas + di.sm_count - 1) / di.sm_count, cluster == 8 && ctas > 14 * 8 ? 2 : 1);
+  const long per = std::max<long>((ctas + di.sm_count - 1) / di.sm_count, paired_clusters(ctas, cluster) ? 2 : 1);
   return per > 4 ? need : std::max(need, (size_t)di.smem_optin / per - (per > 1 ? 1024 : 0));
 }
 
@@ -941,7 +942,7 @@ static int kron_geom(int order, const int* idims, const int* odims, int R, const
 // W[s][ld] (dense) or W[s][tap][ld] (S given): slow side = inputs, or outputs with `transposed`; with `flip` the taps run
 // backwards (a data gradient)
 int kron_weight_launch(int order, const int* idims, const int* odims, int R, const float* const* F, const float* S,
-                       int taps, bool transposed, bool flip, float* W, cudaStream_t st) {
+                       int taps, bool transposed, bool flip, float* W, cudaStream_t st, bool stacked) {
   long fast = 1, rows;
   for (int k = 0; k < order; ++k) fast *= transposed ? idims[k] : odims[k];
   KronGeom g;
@@ -951,7 +952,8 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   const KronPlan p = kron_plan(order, transposed ? odims : idims, transposed ? idims : odims, R, S ? taps : 1, di);
   const int ta = p.ta, splits = p.splits;
   g.rper = p.rper;
-  g.early = p.ctas <= di.sm_count;
+  // (two CTAs of the product to an SM, beside this grid's, would all be placed as pairs: 160 -> 192 channels 10x10 at R = 28 16.7 us, later 12.8)
+  g.early = p.ctas <= (stacked ? di.sm_count / 2 : di.sm_count);
   const dim3 grid(p.nb, ceil_div(p.PA, ta), splits);
 #define KRON_T(TAV, TAPV)                                                                                               \
   do {                                                                                                                  \
@@ -1052,9 +1054,9 @@ int conv_shares(int N, int C, int T, int H, int W, int R, int* out) {
   return B200CP_OK;
 }
 
-// V = W * X, the weight in Wt, or (Wt null) formed inside
+// V = W * X, the weight multiplied out to Wt, or (Wt null) formed inside
 int small_conv_launch(int N, int H, int W, int order, const int* cdims, const int* tdims, int R, const float* const* A, const float* S,
-                      bool transposed, const float* X, const float* Wt, float* V, cudaStream_t st) {
+                      bool transposed, const float* X, float* Wt, float* V, cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   int C = 1, T = 1;
@@ -1074,6 +1076,9 @@ int small_conv_launch(int N, int H, int W, int order, const int* cdims, const in
   const size_t smem = sizeof(float) * (Wt ? p.floats : p.inside);
   dim3 grid((unsigned)(N * g.tiles), ceil_div(T, tt), g.splits);
   if ((long)N * g.tiles > 0x7fffffffL) return fail(B200CP_ERR_UNSUPPORTED, "rcp: too many tiles");
+  if (Wt)
+    if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, 9, transposed, transposed, Wt, st, paired_clusters(tiles * g.splits, g.splits)))
+      return rc;
 #define SMALL_CONV_I(TTV, CGV, IN)                                                                                        \
   do {                                                                                                                \
     static std::atomic<int> set[64];                                                                                  \

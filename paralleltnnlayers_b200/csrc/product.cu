@@ -153,7 +153,6 @@ int rcp_product_launch(int N, int H, int W, int order, const int* cdims, const i
   float* Wt = static_cast<float*>(ws);
   if (p.form == Form::tensor)
     return conv_tc_launch(N, p.K, p.N, H, W, X, KronWeight{order, cdims, tdims, R, A, S, !transposed, transposed}, V, Wt, st);
-  if (int rc = kron_weight_launch(order, cdims, tdims, R, A, S, FH * FW, transposed, transposed, Wt, st)) return rc;
   return small_conv_launch(N, H, W, order, cdims, tdims, R, A, S, transposed, X, Wt, V, st);
 }
 
