@@ -106,8 +106,8 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // The lines are the best ones over random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together, ranks 4 to
 // 128), each measured both ways as calls one after the other: 520 for the backward from a saved plane and the layers, 1500 for the
 // others.  Up to 16 ranks a width that is a multiple of 4 has a row kernel (of these the row stream only loses by the channels), others
-// do not.  800 convolutions, 900 steps and 300 layers more, drawn between higher lines of the same form and these: 0.68, 0.86 and 0.98 of the
-// time (geometric mean), 38, 45 and 6 of them more than 3 % longer.  The factor gradients are within 1 to 4 % of the better form of each shape.
+// do not.  800 convolutions, 1300 steps and 300 layers more, drawn between higher lines of the same form and these: 0.67, 0.87 and 0.98 of the
+// time (geometric mean; the better form of each convolution 0.665, step 0.865), 22, 69 and 6 of them more than 3 % longer.  The factor gradients are within 1 to 4 % of the better form of each shape.
 const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
   return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
@@ -125,6 +125,7 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   if (path_of(flags) != B200CP_PATH_AUTO || !g_auto_mma || g_auto_tc || !planes || !planes_supported(*s)) return false;
   if (planes == 2) return true;
   const double ch = (double)s->C + s->T, root4 = std::sqrt(std::sqrt((double)s->N * s->H * s->W));
+  const double values = ch * s->N * s->H * s->W;
   const bool quads = (size_t)s->H * s->W % 4 == 0;   // (the FFMA products and the gradients load 16 bytes of a plane)
   if (s->Rank <= 16) {
     const double few = ch * std::sqrt((double)s->Rank) / root4;
@@ -132,15 +133,15 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
     const bool streams = s->W % 16 == 8 && s->W <= 56 && s->C % 8 == 0 && s->T % 8 == 0;   // widths of the row stream
     switch (use) {
       case Planes::kConvSaved:
-        if (rows && ch * s->N * s->H * s->W < 1e7) return false;
+        if (rows && values < 1e7) return false;
         [[fallthrough]];
       case Planes::kConv:   // (row-stream widths of 9 to 16 ranks below the line of the others: planes 1.03 over 8)
         if (!rows) return !low && few >= 130 && s->W % 4;
         return (!streams || ch >= 280) && few >= (low ? streams ? 0 : 64 : 96);
-      case Planes::kStep:   // Planes / row or tile kernels over drawn shapes below 110: a width of a multiple of 4, up to 8 ranks: 0.79 from 10000 pixels
-        // on (33), 1.02 before, where the launches take the host longer (35).  Others whose planes are a multiple of 4: 0.86 (229); 4-byte loads:
-        // 0.90 up to 20000 pixels (365), from there on 1.04 (160)
-        if (s->W % 4 == 0) return few >= (low && root4 >= 10 ? 60 : 110);
+      case Planes::kStep:   // Planes / row or tile kernels over drawn shapes below 110: a width of a multiple of 4, up to 8 ranks: 0.78 from 4 images
+        // on (44), 1.10 below (24: on the device 0.74, but the row kernels take the host a launch less).  Others whose planes are a multiple of
+        // 4: 0.85 (229); 4-byte loads: 0.90 up to 20000 pixels (311), from there on 1.07 (141)
+        if (s->W % 4 == 0) return few >= (low && s->N >= 4 ? 60 : 110);
         return few >= (quads || root4 < 11.9 ? low ? 60 : 20 : 110);
       case Planes::kSaved: return few >= 100;
       case Planes::kFilter: return few >= (low ? 20 : 46);
@@ -161,8 +162,8 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
       if (ranks == 1 && ch >= 100 && s->C >= 32 && s->T >= 32) return true;
       [[fallthrough]];
     case Planes::kConvSaved: return past({256, 129, 0}, {2800, 1000, 0});
-    case Planes::kStep:   // (17 to 32 ranks, 4-byte loads, below the last two lines: 0.89 up to 5000 pixels (159), from there on 1.02 (48); 16-byte loads 0.80)
-      return quads || root4 < 8.4 || past({200, 0, 0}, {1300, 0, 0});
+    case Planes::kStep:   // (17 to 32 ranks, 4-byte loads, below the last two lines: 0.91 up to 2 10^6 values in and out (190), 1.07 above (17); 16-byte loads 0.79)
+      return quads || values < 2e6 || past({200, 0, 0}, {1300, 0, 0});
     case Planes::kSaved:
       if (ranks == 1) return (ch >= 64 || s->W % 4 == 0) && ch * root4 >= 155;   // (measured: narrow layers with odd rows lose)
       return past({160, 0, 0}, {2200, 0, 0});

@@ -12,7 +12,7 @@ LINES = [
     ("conv", (1, 144, 136, 6, 24, 12), (1, 136, 136, 6, 24, 12)), ("conv", (1, 49, 49, 9, 9, 16), (1, 49, 48, 9, 9, 16)),
     ("conv", (54, 160, 160, 24, 24, 16), (56, 160, 160, 24, 24, 16)),
     ("step", (2, 38, 38, 9, 9, 8), (2, 38, 37, 9, 9, 8)), ("step", (1, 39, 39, 8, 8, 16), (1, 39, 38, 8, 8, 16)),
-    ("step", (13, 110, 110, 28, 28, 8), (12, 110, 110, 28, 28, 8)), ("step", (1, 55, 55, 8, 8, 8), (1, 55, 54, 8, 8, 8)),
+    ("step", (4, 70, 70, 20, 20, 8), (3, 70, 70, 20, 20, 8)), ("step", (4, 70, 70, 20, 20, 8), (4, 68, 66, 20, 20, 8)), ("step", (1, 55, 55, 8, 8, 8), (1, 55, 54, 8, 8, 8)),
     ("step", (400, 125, 126, 7, 7, 8), (410, 125, 126, 7, 7, 8)), ("step", (410, 165, 165, 10, 14, 8), (410, 165, 165, 11, 13, 8)),
     ("step", (400, 30, 30, 7, 7, 16), (410, 30, 30, 7, 7, 16)), ("step", (20, 32, 32, 36, 34, 16), (20, 32, 32, 35, 35, 16)),
     ("step", (2, 9, 9, 9, 9, 16), (2, 9, 8, 9, 9, 16)), ("saved", (1, 36, 35, 8, 8, 16), (1, 35, 35, 8, 8, 16)),
@@ -24,8 +24,8 @@ LINES = [
     ("conv", (1, 50, 50, 5, 5, 40), (1, 50, 49, 5, 5, 40)), ("conv", (1, 32, 70, 5, 5, 40), (1, 31, 71, 5, 5, 40)),
     ("conv", (1, 70, 32, 5, 5, 40), (1, 71, 31, 5, 5, 40)), ("conv", (1, 9, 120, 5, 5, 40), (1, 9, 119, 5, 5, 40)),
     ("conv", (10, 48, 48, 35, 36, 40), (10, 47, 47, 35, 36, 40)),
-    ("step", (10, 40, 40, 21, 22, 18), (11, 40, 40, 21, 22, 18)), ("step", (11, 100, 100, 21, 22, 18), (11, 100, 53, 21, 22, 18)),
-    ("step", (11, 77, 78, 21, 22, 18), (11, 77, 76, 21, 22, 18)), ("step", (11, 40, 40, 21, 24, 18), (11, 40, 40, 21, 22, 18)),
+    ("step", (50, 40, 40, 21, 22, 18), (60, 40, 40, 21, 22, 18)), ("step", (60, 100, 100, 21, 22, 18), (60, 40, 40, 21, 22, 18)),
+    ("step", (60, 51, 51, 21, 22, 18), (60, 51, 49, 21, 22, 18)), ("step", (60, 40, 40, 21, 24, 18), (60, 40, 40, 21, 22, 18)),
     ("filter", (1, 40, 40, 9, 9, 20), (1, 40, 39, 9, 9, 20)), ("filter", (18, 40, 39, 24, 25, 20), (18, 39, 39, 24, 25, 20)),
     ("filter", (1, 24, 24, 9, 9, 40), (1, 24, 23, 9, 9, 40)),
     # a layer: its convolution by the values in and out where the line above is of launches, older lines elsewhere
