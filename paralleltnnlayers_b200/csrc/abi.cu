@@ -107,7 +107,7 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // 128), each measured both ways as calls one after the other: 520 for the backward from a saved plane and the layers, 1500 for the
 // others.  Up to 16 ranks a width that is a multiple of 4 has a row kernel (of these the row stream only loses by the channels), others
 // do not.  800 convolutions, 1300 steps and 300 layers more, drawn between higher lines of the same form and these: 0.67, 0.87 and 0.98 of the
-// time (geometric mean; the better form of each convolution 0.665, step 0.865), 22, 69 and 6 of them more than 3 % longer.  The factor gradients are within 1 to 4 % of the better form of each shape.
+// time (geometric mean; the better form of each convolution 0.665, step 0.865), 18, 69 and 6 of them more than 3 % longer.  The factor gradients are within 1 to 4 % of the better form of each shape.
 const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
   return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
@@ -156,8 +156,9 @@ bool takes_planes(const b200cp_tensor_shape* s, int flags, Planes use) {
   };
   switch (use) {
     case Planes::kConv:   // below the lines of kConvSaved, planes / tile kernels over drawn shapes:
-      // 17 to 32 ranks, 224 to 255 channels: 2000 to 12000 pixels 0.89 (50), fewer 1.07 (27), more 1.00 (23)
-      if (ranks == 0 && ch >= 224 && root4 >= 6.7 && root4 < 10.5) return true;
+      // 17 to 32 ranks, 224 to 255 channels: with fewer than 80 inputs or outputs 0.86 up to 10000 pixels (28), 1.07 above (16); others 0.84 from
+      // 4000 pixels on (27), 1.15 below (29)
+      if (ranks == 0 && ch >= 224 && (std::min(s->C, s->T) < 80 ? root4 < 10 : root4 >= 7.95)) return true;
       // 33 to 64 ranks, 100 to 128 channels: 0.70 where inputs and outputs are 32 and more (54), 1.10 where one of them is less (36)
       if (ranks == 1 && ch >= 100 && s->C >= 32 && s->T >= 32) return true;
       [[fallthrough]];

@@ -18,8 +18,9 @@ LINES = [
     ("step", (2, 9, 9, 9, 9, 16), (2, 9, 8, 9, 9, 16)), ("saved", (1, 36, 35, 8, 8, 16), (1, 35, 35, 8, 8, 16)),
     ("filter", (1, 11, 11, 9, 9, 8), (1, 11, 10, 9, 9, 8)), ("filter", (1, 18, 17, 9, 9, 16), (1, 17, 17, 9, 9, 16)),
     # more ranks: channels, alone or with the pixels
-    ("conv", (1, 112, 112, 46, 46, 24), (1, 112, 111, 46, 46, 24)), ("conv", (1, 112, 112, 46, 46, 24), (1, 112, 112, 44, 44, 24)),
-    ("conv", (1, 112, 112, 110, 110, 24), (1, 112, 112, 111, 111, 24)), ("conv", (1, 128, 128, 9, 9, 24), (1, 128, 127, 9, 9, 24)),
+    ("conv", (1, 112, 112, 64, 64, 24), (1, 112, 111, 64, 64, 24)), ("conv", (1, 112, 112, 64, 64, 24), (1, 112, 112, 63, 63, 24)),
+    ("conv", (1, 144, 80, 64, 64, 24), (1, 144, 80, 63, 63, 24)), ("conv", (1, 145, 79, 63, 63, 24), (1, 144, 79, 63, 63, 24)),
+    ("conv", (1, 145, 79, 99, 99, 24), (1, 145, 79, 100, 100, 24)), ("conv", (1, 128, 128, 9, 9, 24), (1, 128, 127, 9, 9, 24)),
     ("conv", (32, 112, 111, 28, 28, 17), (32, 111, 111, 28, 28, 17)),
     ("conv", (1, 50, 50, 5, 5, 40), (1, 50, 49, 5, 5, 40)), ("conv", (1, 32, 70, 5, 5, 40), (1, 31, 71, 5, 5, 40)),
     ("conv", (1, 70, 32, 5, 5, 40), (1, 71, 31, 5, 5, 40)), ("conv", (1, 9, 120, 5, 5, 40), (1, 9, 119, 5, 5, 40)),
