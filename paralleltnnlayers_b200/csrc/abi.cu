@@ -106,8 +106,8 @@ Cp4Args conv_args(const b200cp_tensor_shape* s, const float* in, const float* K0
 // The lines are the best ones over random shapes (1 to 64 images of 7x7 to 64x64, 16 to 1000 channels in and out together, ranks 4 to
 // 128), each measured both ways as calls one after the other: 520 for the backward from a saved plane and the layers, 1500 for the
 // others.  Up to 16 ranks a width that is a multiple of 4 has a row kernel (of these the row stream only loses by the channels), others
-// do not.  800 convolutions, 1300 steps and 300 layers more, drawn between higher lines of the same form and these: 0.67, 0.87 and 0.98 of the
-// time (geometric mean; the better form of each convolution 0.665, step 0.865), 18, 69 and 6 of them more than 3 % longer.  The factor gradients are within 1 to 4 % of the better form of each shape.
+// do not.  800 convolutions, 1300 steps and 600 layers more, drawn between higher lines of the same form and these: 0.67, 0.87 and 0.98 of the
+// time (geometric mean; the better form of each convolution 0.665, step 0.865), 18, 69 and 7 of them more than 3 % longer.  The factor gradients are within 1 to 4 % of the better form of each shape.
 const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
   const char* e = getenv("B200CP_PLANES");
   return e && e[0] == '0' ? 0 : e && e[0] == '2' ? 2 : 1;
