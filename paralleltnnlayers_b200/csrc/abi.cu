@@ -116,7 +116,7 @@ const int g_planes = [] {   // 0 off, 1 by the rule, 2 wherever they can
 // its plane; the factor gradients of a layer's backward, from both planes.
 // A layer's forward and backward take the host about 90 us, whatever runs on the GPU, and a launch more 2 to 3: where the GPU takes less,
 // a convolution in three launches instead of one only loses.  So below 10^7 inputs and outputs the last two have lines of their own.  Of 191 layers
-// drawn between the two lines those below took 1.06 times as long with the lines of kConv, calls one after the other (58 x 208 -> 296
+// drawn between the two lines those below took 1.06 times as long with the lines of kConv, calls one after the other (15 x 208 -> 296
 // 12x12 at R = 12 93.9 -> 101.3 us, on the device alone 50.5 -> 29.2), those above 0.91 times (59 x 460 32x32 at R = 4 307 -> 254).  Of 109
 // at the lines of kFilter as many gained as lost.
 enum class Planes { kConv, kStep, kSaved, kFilter, kSaved3, kFilter3, kConvSaved, kFilterSaved };
