@@ -250,23 +250,54 @@ __global__ void __launch_bounds__(kKT, 2) kron_weight_kernel(const __grid_consta
 // ---- the weight as the operand planes of the tensor-core product (gemm_tc.cu) ------------------------------------------
 // Row s of the weight gets the exponent of a bound, sum_r prod_k max_f |F_k[s_k, f, r]|, which needs no pass over the weight (it is
 // some 2^5 above the largest entry; of the 18 binades below a row's largest value that keep 22 bits this costs five).
-// One warp per row.
-__global__ void __launch_bounds__(256) kron_exponent_kernel(const __grid_constant__ KronGeom g, int rows, int* __restrict__ ex) {
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+// What bounds this is latency: the largest values of all slices of the modes go to shared memory once, the loads of a thread together,
+// and a row, one warp, multiplies one of each mode.  4096 x 4096 at R = 32: 5.2 us; a warp that read the slices of its row
+// from global memory, eight rows per CTA, 13.5.
+constexpr int kRowsEx = 32;       // rows, and warps, of a CTA
+__host__ __device__ __forceinline__ const KronMode& kron_mode_of(const KronGeom& g, int k) { return k < g.nA ? g.A[k] : g.B[k - g.nA]; }
+
+__device__ __forceinline__ float largest_of_slice(const KronMode& m, int slice, int R, int r) {
+  const float* src = m.F + (size_t)slice * m.fs * R + r;
+  unsigned mx = 0;
+  for (int f0 = 0; f0 < m.nf; f0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __ldg(src + (size_t)(min(f0 + j, m.nf - 1) * m.ff) * R);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mx = max(mx, tc::abs_bits(v[j]));
+  }
+  return __uint_as_float(mx);
+}
+
+__global__ void __launch_bounds__(32 * kRowsEx) kron_exponent_kernel(const __grid_constant__ KronGeom g, int rows, int* __restrict__ ex) {
+  extern __shared__ float largest[];   // [slice of all modes][rank]: at most 4 x 16 slices of kKeep ranks
+  const int lane = threadIdx.x & 31, row = blockIdx.x * kRowsEx + (threadIdx.x >> 5), order = g.nA + g.nB;
+  grid_launch_dependents();
+  int at[4] = {0, 0, 0, 0}, slices = 0;   // the row's slice of each mode
+  for (int k = 0; k < order; ++k) slices += kron_mode_of(g, k).ns;
+  for (int i = threadIdx.x; i < slices * g.R; i += 32 * kRowsEx) {
+    int slice = i / g.R, k = 0;
+    const int r = i - slice * g.R;
+    for (; slice >= kron_mode_of(g, k).ns; ++k) slice -= kron_mode_of(g, k).ns;
+    largest[i] = largest_of_slice(kron_mode_of(g, k), slice, g.R, r);
+  }
+  int s = row;
+#pragma unroll
+  for (int k = 3; k >= 0; --k)
+    if (k < order) {
+      const int ns = kron_mode_of(g, k).ns;
+      slices -= ns;
+      at[k] = slices + s % ns;
+      s /= ns;
+    }
+  __syncthreads();
   if (row >= rows) return;
   float sum = 0.f;
   for (int r = lane; r < g.R; r += 32) {
     float prod = 1.f;
-    int s = row;
-    for (int k = g.nA + g.nB - 1; k >= 0; --k) {
-      const KronMode& m = k < g.nA ? g.A[k] : g.B[k - g.nA];
-      const int sk = s % m.ns;
-      s /= m.ns;
-      unsigned mx = 0;
-#pragma unroll 4
-      for (int f = 0; f < m.nf; ++f) mx = max(mx, tc::abs_bits(__ldg(m.F + (size_t)(sk * m.fs + f * m.ff) * g.R + r)));
-      prod *= __uint_as_float(mx);
-    }
+#pragma unroll
+    for (int k = 3; k >= 0; --k)
+      if (k < order) prod *= largest[at[k] * g.R + r];
     sum += prod;
   }
 #pragma unroll
@@ -277,15 +308,16 @@ __global__ void __launch_bounds__(256) kron_exponent_kernel(const __grid_constan
 // 128 x 128 entries per CTA and tile, 8 x 8 per thread (four 16-byte reads per 64 FFMA).  A CTA keeps its half products A and
 // walks the tiles of B; ranks in chunks of 32, A's formed once.  Each entry is stored as its hi and lo
 // halves, 8 bytes of each where four are neighbours.
-// 4096 x 4096 at R = 32: the weight in fp32 (64 x 64 tiles, one per CTA) 68 us and 18 us more to split it, here 56 and 6 for the exponents.
+// 4096 x 4096 at R = 32: the weight in fp32 (64 x 64 tiles, one per CTA) 68 us and 18 us more to split it, here 50 (53 with a division by the
+// pitch per four entries) and 5 for the exponents.
 constexpr int kPT = 128, kPP = kPT + 4, kKeep = 256;
 __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_constant__ KronGeom g, int pitch, int btiles,
-                                                          const int* __restrict__ ex, __half* __restrict__ hi, size_t plane) {
+                                                          const int* ex, __half* __restrict__ hi, size_t plane) {
   extern __shared__ __align__(16) float smem[];
   const int keep = (g.R + kRC - 1) / kRC * kRC;   // at most kKeep
   float* As = smem;                       // [keep][kPP]
   float* Bs = As + keep * kPP;            // [kRC][kPP]
-  __shared__ int ea[kPT][2], eb[kPT][2], oa[kPT], ob[kPT];
+  __shared__ int ea[kPT][2], eb[kPT][2], oa[kPT], ob[kPT], ra[kPT], rb[kPT];   // ra + rb: the entry's row
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int a0 = blockIdx.y * kPT, PA = g.SA * g.FA, PB = g.SB * g.FB;
   constexpr int NM = 2;   // modes of a half
@@ -294,6 +326,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
     if (a0 + tid < PA) half_decode(g.A, g.nA, (a0 + tid) / g.FA, (a0 + tid) % g.FA, 0, e, &o);
     ea[tid][0] = e[0]; ea[tid][1] = e[1];
     oa[tid] = o;
+    ra[tid] = o / pitch;
   }
   // half products of ranks r0 .. r0 + 31 to dst[rank][row]; a warp forms 8 ranks x 4 rows per turn
   const int rl = tid & 7, row0 = (tid >> 5) * 4 + ((tid >> 3) & 3);
@@ -329,6 +362,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
       if (b0 + tid < PB) half_decode(g.B, g.nB, (b0 + tid) / g.FB, (b0 + tid) % g.FB, 0, e, &o);
       eb[tid][0] = e[0]; eb[tid][1] = e[1];
       ob[tid] = o;
+      rb[tid] = o / pitch;
     }
     float acc[8][8];
 #pragma unroll
@@ -352,6 +386,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
           for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
       }
     }
+    grid_dependency_wait();   // the exponents
 #pragma unroll
     for (int j4 = 0; j4 < 2; ++j4) {
       const int jb = j4 * 64 + tx * 4, left = PB - (b0 + jb);
@@ -363,7 +398,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         const float* v = acc[i] + j4 * 4;
         const int o = oa[ia] + ob[jb];
         if (run4 && !(oa[ia] & 3)) {   // four neighbours of one row
-          const float sc = tc::exp2_int(-__ldg(ex + o / pitch));
+          const float sc = tc::exp2_int(-ex[ra[ia] + rb[jb]]);
           const __half2 h0 = __floats2half2_rn(v[0] * sc, v[1] * sc), h1 = __floats2half2_rn(v[2] * sc, v[3] * sc);
           const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
           const __half2 l0 = __floats2half2_rn(v[0] * sc - f0.x, v[1] * sc - f0.y), l1 = __floats2half2_rn(v[2] * sc - f1.x, v[3] * sc - f1.y);
@@ -374,7 +409,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
           for (int j = 0; j < 4; ++j)
             if (j < left) {
               const int oj = oa[ia] + ob[jb + j];
-              const float w = v[j] * tc::exp2_int(-__ldg(ex + oj / pitch));
+              const float w = v[j] * tc::exp2_int(-ex[ra[ia] + rb[jb + j]]);
               const __half h = __float2half_rn(w);
               hi[oj] = h;
               hi[plane + oj] = __float2half_rn(w - __half2float(h));
@@ -993,17 +1028,22 @@ int kron_planes_launch(int order, const int* idims, const int* odims, int R, con
   if (int rc = kron_geom(order, idims, odims, R, F, nullptr, 1, transposed, false, ldo, &rows, &g)) return rc;
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
-  kron_exponent_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(g, (int)rows, ex);
+  if (R > kKeep) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight: rank %d", R);
+  size_t table = 0;
+  for (int k = 0; k < order; ++k) table += sizeof(float) * kron_mode_of(g, k).ns * R;
+  static std::atomic<int> exset[64];
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_exponent_kernel), exset, (int)table));
+  kron_exponent_kernel<<<(unsigned)((rows + kRowsEx - 1) / kRowsEx), 32 * kRowsEx, table, st>>>(g, (int)rows, ex);
   B200CP_LAUNCH_OK("kron_exponent_kernel");
   const int atiles = ceil_div(g.SA * g.FA, kPT), btiles = ceil_div(g.SB * g.FB, kPT);
-  if (atiles > 65535 || R > kKeep) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight too large");
+  if (atiles > 65535) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight too large");
   const size_t smem = sizeof(float) * (align_up((size_t)R, kRC) + kRC) * kPP;
   static std::atomic<int> set[64];
   B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_planes_kernel), set, (int)smem));
   // as many CTAs as are resident at once share the tiles of B
   const int walkers = std::min(btiles, std::max(1, 2 * di.sm_count / atiles));
   const dim3 grid(ceil_div(btiles, ceil_div(btiles, walkers)), atiles);
-  kron_planes_kernel<<<grid, 256, smem, st>>>(g, ldo, btiles, ex, static_cast<__half*>(hi), plane);
+  B200CP_CUDA_OK(launch_kernel(kron_planes_kernel, grid, dim3(256), smem, st, true, g, ldo, btiles, ex, static_cast<__half*>(hi), plane));
   B200CP_LAUNCH_OK("kron_planes_kernel");
   return B200CP_OK;
 }
