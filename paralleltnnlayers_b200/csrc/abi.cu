@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "contract.cuh"
 #include "cp_planes.cuh"
 #include "b200cp_test.h"
 
@@ -1285,6 +1286,8 @@ int b200cp_device_status(void) {
   if (v) return fail(B200CP_ERR_TIMEOUT, "cp4 gradient band kernel: a bounded wait ran out in block %d", v & 0xffff);
   if (int rc = planes_device_status(&v)) return rc;
   if (v) return fail(B200CP_ERR_TIMEOUT, "cp plane products: a bounded wait ran out in block %d", v & 0xffff);
+  if (int rc = halves_device_status(&v)) return rc;
+  if (v) return fail(B200CP_ERR_TIMEOUT, "factor contraction: a bounded wait ran out in block %d", v & 0xffff);
   return B200CP_OK;
 }
 

@@ -1,4 +1,4 @@
-// Factor gradients of the reshaped-CP conv and the CP dense layer from the dense gradient G.
+// Factor gradients of the reshaped-CP conv and the CP dense layer from the dense gradient G.  (Large ones: contract_halves.cu.)
 //
 // Index modes: the m factor modes with pair index p_j = c_j * t_dim_j + t_j (the factor's own [c][t] layout, vector
 // vec_j[p_j][r] = A_j[c_j][t_j][r]) and, for the conv, the tap mode with vector S[tap][r].  For every mode q
@@ -17,7 +17,7 @@
 // 28x28 at R = 16 took 448 us a call, now 438, one of 609 samples 800 -> 2560 at R = 81 242, now 222.
 #include <algorithm>
 
-#include "common.cuh"
+#include "contract.cuh"
 
 namespace b200cp {
 
@@ -29,12 +29,6 @@ constexpr int kRows0 = 64;    // rows of G per batch in the first peel
 constexpr int kGPad = 4;      // padding of a staged row of G, floats
 constexpr int kMaxNb = 256;   // entries of one mode (c_dim * t_dim)
 constexpr int kGridCap = 592; // CTAs per level (fixed: the order of the partial sums must not depend on the device)
-
-struct PeelMode {
-  int nc, nt;      // p = c * nt + t
-  long gc, gt;     // G offset per c and per t (first peel only)
-  const float* vec;  // [nc * nt][R]
-};
 
 struct PeelGeom {
   int R, nouter, nb, nbp;  // nbp: nb padded to the kernel's entry count
@@ -345,6 +339,7 @@ void peel_plan(PeelPlan& pl, int order, const int* cdims, const int* tdims, int 
 size_t contract_scratch_floats(int order, const int* cdims, const int* tdims, int R, int taps, bool has_s) {
   PeelPlan pl;
   peel_plan(pl, order, cdims, tdims, R, taps, has_s);
+  if (halves_take(pl.L, pl.nmode, has_s)) return halves_scratch_floats(pl.L, pl.nmode, R);
   return pl.s_floats[0] + pl.s_floats[1] + pl.part_floats + 8;
 }
 
@@ -380,6 +375,7 @@ int contract_factors_launch(int order, const int* cdims, const int* tdims, int R
   for (int k = 0; k < L; ++k)
     if (modes[k].nc * modes[k].nt > kMaxNb)
       return fail(B200CP_ERR_UNSUPPORTED, "factor contraction: a mode has %d > %d entries", modes[k].nc * modes[k].nt, kMaxNb);
+  if (halves_take(L, pl.nmode, S != nullptr)) return halves_launch(L, modes, R, G, grads, scratch, st);
   float* sbuf[2] = {scratch, scratch + ((pl.s_floats[0] + 3) & ~size_t(3))};
   float* part = sbuf[1] + ((pl.s_floats[1] + 3) & ~size_t(3));
   const float* src = G;
