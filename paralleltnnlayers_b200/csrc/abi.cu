@@ -1286,6 +1286,8 @@ int b200cp_device_status(void) {
   if (v) return fail(B200CP_ERR_TIMEOUT, "cp4 gradient band kernel: a bounded wait ran out in block %d", v & 0xffff);
   if (int rc = planes_device_status(&v)) return rc;
   if (v) return fail(B200CP_ERR_TIMEOUT, "cp plane products: a bounded wait ran out in block %d", v & 0xffff);
+  if (int rc = kron_device_status(&v)) return rc;
+  if (v) return fail(B200CP_ERR_TIMEOUT, "weight as operand planes: a bounded wait ran out in block %d", v & 0xffff);
   if (int rc = halves_device_status(&v)) return rc;
   if (v) return fail(B200CP_ERR_TIMEOUT, "factor contraction: a bounded wait ran out in block %d", v & 0xffff);
   return B200CP_OK;

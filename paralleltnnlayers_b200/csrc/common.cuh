@@ -273,6 +273,7 @@ bool gemm_tc_supported(int K, int M, int N);
 size_t gemm_tc_scratch_floats(int K, int M, int N);
 int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st);
 int gemm_tc_status(int* out);
+int kron_device_status(int* out);
 // conv form of the same kernel: G[tap][T][C] from NCHW operands (padded, transposed planes in the scratch)
 bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW);
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW);

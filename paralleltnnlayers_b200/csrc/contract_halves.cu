@@ -8,8 +8,8 @@
 // A CTA has 128 entries of a and walks tiles of 64 entries of b.  A tile of G is split into three bf16 parts (tc_common.cuh) once; it is the
 // K-major A operand of the first product and the MN-major B operand of the second, whose A operand are the parts of VA:
 //   D1[128 a][hi | mid | low] += G_hi (V_hi | V_mid | V_low) + G_mid (0 | V_hi | V_mid) + G_low (0 | 0 | V_hi)        K = 64
-//   D2[part, r][64 b]          = V_part (G_low + G_mid + G_hi), the smallest first                                     K = 128
-// so the parts of V share an instruction and G is read from shared memory once per part.  D1 is added to totals in registers after each
+//   D2[part, r][64 b | 64 b]  = V_part (G_hi | G_mid + G_low)                                                            K = 128
+// so the parts of V share an instruction, G_hi and G_mid one of twice the columns in D2.  D1 is added to totals in registers after each
 // tile, D2 goes out as a partial sum per 128 entries of a: no accumulator is longer than 64 (D1) or 128 terms.  An entry that met an infinite value
 // comes out NaN and is formed anew in fp32.
 //

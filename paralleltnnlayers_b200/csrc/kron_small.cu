@@ -9,7 +9,7 @@
 //   kron_weight_kernel : W[s][f] = sum_r prod_k F_k[s_k, f_k, r]   (conv: W[c][tap][t], with S as one more mode)
 //   small_gemm_kernel  : Y[m][n] = sum_k X[m][k] W[k][n]
 //   small_conv_kernel  : V[n,t,h,w] = sum_{c,y,x} W[c][y,x][t] X[n,c,h+y-1,w+x-1]
-// All exact fp32 (FFMA).  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
+// All exact fp32 (FFMA); large weights for the tensor-core product come from kron_planes_kernel.  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
 // and past their set-up when the weight is done.  Formulas: Kernels/rcp_fused_nchw.cu:4-77, Kernels/dense_cp.cu:4-46.
 #include <algorithm>
 #include <climits>
@@ -270,7 +270,7 @@ __device__ __forceinline__ float largest_of_slice(const KronMode& m, int slice, 
 }
 
 __global__ void __launch_bounds__(32 * kRowsEx) kron_exponent_kernel(const __grid_constant__ KronGeom g, int rows, int* __restrict__ ex) {
-  extern __shared__ float largest[];   // [slice of all modes][rank]: at most 4 x 16 slices of kKeep ranks
+  extern __shared__ float largest[];   // [slice of all modes][rank]: at most 4 x 16 slices of 256 ranks
   const int lane = threadIdx.x & 31, row = blockIdx.x * kRowsEx + (threadIdx.x >> 5), order = g.nA + g.nB;
   grid_launch_dependents();
   int at[4] = {0, 0, 0, 0}, slices = 0;   // the row's slice of each mode
@@ -305,118 +305,223 @@ __global__ void __launch_bounds__(32 * kRowsEx) kron_exponent_kernel(const __gri
   if (lane == 0) ex[row] = tc::row_exponent(tc::abs_bits(sum * 1.001f), tc::kLeast);
 }
 
-// 128 x 128 entries per CTA and tile, 8 x 8 per thread (four 16-byte reads per 64 FFMA).  A CTA keeps its half products A and
-// walks the tiles of B; ranks in chunks of 32, A's formed once.  Each entry is stored as its hi and lo
-// halves, 8 bytes of each where four are neighbours.
-// 4096 x 4096 at R = 32: the weight in fp32 (64 x 64 tiles, one per CTA) 68 us and 18 us more to split it, here 50 (53 with a division by the
-// pitch per four entries) and 5 for the exponents.
-constexpr int kPT = 128, kPP = kPT + 4, kKeep = 256;
+// 128 x 128 entries per CTA and tile on the tensor cores: the half products of 64 ranks at a time as three bf16 parts, K-major, six products
+// of parts (tc_common.cuh), the smallest first; an accumulator has at most 128 ranks.  A CTA keeps A's parts, where R is at most 64,
+// and walks the tiles of B.  A thread splits the 64 entries that it has of one row of the tile into hi and lo; through shared memory, a warp
+// for itself, they are stored as runs of 64 bytes of a row.
+//
+// What bounds it are the phases of a tile one after the other, of which the stores take the longest (a CTA forms, multiplies and stores in 2300,
+// 1300 and 5500 of 9600 cycles; two per SM overlap).  4096 x 4096, times in us at R = 4 / 16 / 32 / 64 / 256: 31 / 31 / 33 / 45 / 166, with 128 x 128
+// tiles of FFMA 33 / 42 / 53 / 84 / 345.  One accumulator for all six products: an error of the layer's output of 6.4e-7 at R = 100, now
+// 1.7e-7, FFMA 2.4e-7 (R = 32: 2.0, 1.75 and 1.93e-7).
+__device__ int g_kron_status = 0;   // 0 ok; otherwise (1 << 16) | (block index & 0xffff): a bounded wait ran out
+constexpr int kPT = 128, kKeep = 256, kPart = kPT * 128;   // bytes of a part of a half: 64 ranks
+constexpr size_t kPlanesSmem = 1024 + 6 * kPart;
+
+struct KronTile {   // entries of a half in a tile
+  int e[kPT][2], o[kPT], row[kPT];   // entry of each mode (in ranks), offset and row in the weight (both add up)
+};
+
+template <bool MANY>   // more than 64 ranks
 __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_constant__ KronGeom g, int pitch, int btiles,
-                                                          const int* ex, __half* __restrict__ hi, size_t plane) {
-  extern __shared__ __align__(16) float smem[];
-  const int keep = (g.R + kRC - 1) / kRC * kRC;   // at most kKeep
-  float* As = smem;                       // [keep][kPP]
-  float* Bs = As + keep * kPP;            // [kRC][kPP]
-  __shared__ int ea[kPT][2], eb[kPT][2], oa[kPT], ob[kPT], ra[kPT], rb[kPT];   // ra + rb: the entry's row
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+                                                          const int* ex, __half* __restrict__ hi, size_t plane, bool vec) {
+  extern __shared__ __align__(16) uint8_t raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+  __shared__ KronTile ta, tb[2];
+  __shared__ __align__(8) uint64_t done;
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), quarter = warp & 3, grp = warp >> 2;
   const int a0 = blockIdx.y * kPT, PA = g.SA * g.FA, PB = g.SB * g.FB;
-  constexpr int NM = 2;   // modes of a half
-  if (tid < kPT) {
+  auto table = [&](bool isA, int first, int i, KronTile& t) {
     int e[3] = {0, 0, 0}, o = 0;
-    if (a0 + tid < PA) half_decode(g.A, g.nA, (a0 + tid) / g.FA, (a0 + tid) % g.FA, 0, e, &o);
-    ea[tid][0] = e[0]; ea[tid][1] = e[1];
-    oa[tid] = o;
-    ra[tid] = o / pitch;
+    if (isA && first + i < PA) half_decode(g.A, g.nA, (first + i) / g.FA, (first + i) % g.FA, 0, e, &o);
+    if (!isA && first + i < PB) half_decode(g.B, g.nB, (first + i) / g.FB, (first + i) % g.FB, 0, e, &o);
+    t.e[i][0] = e[0] * g.R; t.e[i][1] = e[1] * g.R;
+    t.o[i] = o;
+    t.row[i] = o / pitch;
+  };
+  if (tid == 0) {
+    tc::mbar_init(&done, 1);
+    tc::fence_barrier_init();
   }
-  // half products of ranks r0 .. r0 + 31 to dst[rank][row]; a warp forms 8 ranks x 4 rows per turn
-  const int rl = tid & 7, row0 = (tid >> 5) * 4 + ((tid >> 3) & 3);
-  auto form = [&](bool isA, int first, int count, int r0, float* dst) {
-    const KronMode* m = isA ? g.A : g.B;
-    const int n = isA ? g.nA : g.nB;
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, 256);
+  if (tid < kPT) table(true, a0, tid, ta);
+  else table(false, blockIdx.x * kPT, tid - kPT, tb[0]);
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+  // the half products of ranks r0 .. r0 + 63 as parts, [row][rank]; two ranks of a row per lane, rows four apart in the halves of a warp
+  // (16 bytes of a row and of the one four on are in different banks)
+  auto form = [&](const KronMode* m, int n, const KronTile& t, int r0, uint8_t* dst) {
+    const float *f0 = m[0].F, *f1 = m[n - 1].F;
+    for (int h = 0; h < 2 && r0 + h * 32 < g.R; ++h) {
+      const int k = h * 32 + (lane & 15) * 2, r = r0 + k, c0 = min(r, g.R - 1), c1 = min(r + 1, g.R - 1);
 #pragma unroll
-    for (int i = 0; i < kPT / 32; ++i) {
-      const int row = i * 32 + row0;
-      const bool in = first + row < count;
-      float v[kRC / 8];
+      for (int i0 = 0; i0 < 8; i0 += 4) {
+        float x[4][4];
 #pragma unroll
-      for (int rb = 0; rb < kRC / 8; ++rb) v[rb] = in && r0 + rb * 8 + rl < g.R ? 1.f : 0.f;
-#pragma unroll
-      for (int k = 0; k < NM; ++k)
-        if (in && k < n) {
-          const float* src = m[k].F + (size_t)(isA ? ea[row][k] : eb[row][k]) * g.R + r0 + rl;
-#pragma unroll
-          for (int rb = 0; rb < kRC / 8; ++rb)
-            if (r0 + rb * 8 + rl < g.R) v[rb] *= __ldg(src + rb * 8);
+        for (int i = 0; i < 4; ++i) {
+          const int row = warp * 16 + i0 * 2 + i + (lane >> 4) * 4;
+          const float *p = f0 + t.e[row][0], *q = f1 + t.e[row][n - 1];
+          x[i][0] = __ldg(p + c0); x[i][1] = __ldg(p + c1); x[i][2] = __ldg(q + c0); x[i][3] = __ldg(q + c1);
         }
 #pragma unroll
-      for (int rb = 0; rb < kRC / 8; ++rb) dst[(rb * 8 + rl) * kPP + row] = v[rb];
+        for (int i = 0; i < 4; ++i) {
+          const int row = warp * 16 + i0 * 2 + i + (lane >> 4) * 4;
+          const float u = n > 1 ? x[i][0] * x[i][2] : x[i][0], v = n > 1 ? x[i][1] * x[i][3] : x[i][1];
+          const tc::Bf3 w = tc::split3(r < g.R ? u : 0.f, r + 1 < g.R ? v : 0.f);
+          uint8_t* d = dst + row * 128 + ((((k >> 3) ^ row) & 7) << 4) + (k & 7) * 2;
+#pragma unroll
+          for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(d + j * kPart) = w.p[j];
+        }
+      }
     }
   };
-  __syncthreads();
-  for (int r0 = 0; r0 < keep; r0 += kRC) form(true, a0, PA, r0, As + r0 * kPP);
-  for (int bt = blockIdx.x; bt < btiles; bt += gridDim.x) {
+  const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
+  constexpr uint32_t idesc = tc::make_idesc_bf16(kPT);
+  // Each instruction cuts its sum off, a third of 2^-24 of it in the mean (measured for 4 to 256 ranks).  That is given back, except where the
+  // sum of the small products is nothing: values of eight bits, such as small whole numbers, have exact sums.
+  const float back = (min(g.R, 64) + 15) / 16 * 0.33f / (1 << 24);
+  const int srow = ta.row[quarter * 32 + lane];
+  bool fine = true;
+  int waits = 0;
+  if (!MANY) form(g.A, g.nA, ta, 0, sm);
+  int turn = 0;
+  for (int bt = blockIdx.x; bt < btiles; bt += gridDim.x, turn ^= 1) {
     const int b0 = bt * kPT;
-    __syncthreads();   // the tile before is done with the tables
-    if (tid < kPT) {
-      int e[2] = {0, 0}, o = 0;
-      if (b0 + tid < PB) half_decode(g.B, g.nB, (b0 + tid) / g.FB, (b0 + tid) % g.FB, 0, e, &o);
-      eb[tid][0] = e[0]; eb[tid][1] = e[1];
-      ob[tid] = o;
-      rb[tid] = o / pitch;
-    }
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    for (int r0 = 0; r0 < g.R; r0 += kRC) {
+    const KronTile& t = tb[turn];
+    float tot[MANY ? 64 : 1];
+    int scale[4];   // exponents of this lane's row in the first column of each 16
+    for (int r0 = 0; r0 < (MANY ? g.R : 1); r0 += 64) {
+      if (MANY) form(g.A, g.nA, ta, r0, sm);
+      form(g.B, g.nB, t, r0, sm + 3 * kPart);
+      tc::fence_proxy_async();
       __syncthreads();
-      form(false, b0, PB, r0, Bs);
-      __syncthreads();
-      const float* Ar = As + r0 * kPP;
-      const int rn = min(kRC, g.R - r0);
-#pragma unroll 2
-      for (int r = 0; r < rn; ++r) {
-        const float4 x0 = *reinterpret_cast<const float4*>(Ar + r * kPP + ty * 4), x1 = *reinterpret_cast<const float4*>(Ar + r * kPP + 64 + ty * 4);
-        const float4 y0 = *reinterpret_cast<const float4*>(Bs + r * kPP + tx * 4), y1 = *reinterpret_cast<const float4*>(Bs + r * kPP + 64 + tx * 4);
-        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+      if (warp == 0 && tc::elect_one()) {
+        tc::tc_fence_after_sync();
+        const uint64_t ad = d0 + (tc::smem_u32(sm) >> 4), bd = ad + (3 * kPart >> 4), p1 = kPart >> 4;
+        const int steps = min(4, (g.R - r0 + 15) / 16);
+        for (int k = 0; k < steps; ++k) {
+          tc::mma_f16_ss(tmem + kPT, ad + 2 * p1 + k * 2, bd + k * 2, idesc, r0 > 0 || k > 0);
+          tc::mma_f16_ss(tmem + kPT, ad + k * 2, bd + 2 * p1 + k * 2, idesc, true);
+          tc::mma_f16_ss(tmem + kPT, ad + p1 + k * 2, bd + p1 + k * 2, idesc, true);
+          tc::mma_f16_ss(tmem + kPT, ad + p1 + k * 2, bd + k * 2, idesc, true);
+          tc::mma_f16_ss(tmem + kPT, ad + k * 2, bd + p1 + k * 2, idesc, true);
+          tc::mma_f16_ss(tmem, ad + k * 2, bd + k * 2, idesc, k > 0);
+        }
+        tc::mma_commit(&done);
+      }
+      __syncwarp();
+      if (r0 == 0 && tid >= kPT) table(false, (bt + gridDim.x) * kPT, tid - kPT, tb[turn ^ 1]);
+      if (!MANY || r0 + 64 >= g.R) {
+        grid_dependency_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int q = 0; q < 4; ++q) scale[q] = ex[srow + t.row[grp * 64 + q * 16]];
+      }
+      fine = tc::mbar_wait(&done, waits++ & 1) && fine;   // (the other CTA of the SM works meanwhile)
+      __syncwarp();
+      tc::tc_fence_after_sync();
+      if constexpr (MANY) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+        for (int j0 = 0; j0 < 64; j0 += 16) {
+          float v[16];
+          tc::tmem_ld16(lanes + grp * 64 + j0, v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) tot[j0 + j] = r0 ? tot[j0 + j] + v[j] : v[j];
+        }
+        tc::tc_fence_before_sync();
       }
     }
-    grid_dependency_wait();   // the exponents
+    uint8_t* stage = sm + 3 * kPart + warp * 4096;   // [hi | lo][32 rows][64 bytes], B is used up
 #pragma unroll
-    for (int j4 = 0; j4 < 2; ++j4) {
-      const int jb = j4 * 64 + tx * 4, left = PB - (b0 + jb);
-      const bool run4 = left >= 4 && ob[jb + 3] - ob[jb] == 3 && !(ob[jb] & 3);
+    for (int j0 = 0; j0 < 64; j0 += 32) {
+      const int c0 = grp * 64 + j0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int ia = (i >> 2) * 64 + ty * 4 + (i & 3);
-        if (a0 + ia >= PA) continue;
-        const float* v = acc[i] + j4 * 4;
-        const int o = oa[ia] + ob[jb];
-        if (run4 && !(oa[ia] & 3)) {   // four neighbours of one row
-          const float sc = tc::exp2_int(-ex[ra[ia] + rb[jb]]);
-          const __half2 h0 = __floats2half2_rn(v[0] * sc, v[1] * sc), h1 = __floats2half2_rn(v[2] * sc, v[3] * sc);
-          const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-          const __half2 l0 = __floats2half2_rn(v[0] * sc - f0.x, v[1] * sc - f0.y), l1 = __floats2half2_rn(v[2] * sc - f1.x, v[3] * sc - f1.y);
-          *reinterpret_cast<uint2*>(hi + o) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
-          *reinterpret_cast<uint2*>(hi + plane + o) = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+      for (int q = 0; q < 2; ++q) {
+        const int cq = c0 + q * 16;
+        float v[16], w[16];
+        if constexpr (MANY) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = tot[j0 + q * 16 + j];
+        } else {
+          tc::tmem_ld16(lanes + cq, v);
+        }
+        tc::tmem_ld16(lanes + kPT + cq, w);
+        if (t.row[cq] == t.row[cq + 15]) {   // one row of the weight (b's rows do not descend; columns past the end have row 0)
+          const float sc = tc::exp2_int(-scale[j0 / 16 + q]);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = (v[j] + fmaf(v[j], w[j] != 0.f ? back : 0.f, w[j])) * sc;
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (j < left) {
-              const int oj = oa[ia] + ob[jb + j];
-              const float w = v[j] * tc::exp2_int(-ex[ra[ia] + rb[jb + j]]);
-              const __half h = __float2half_rn(w);
-              hi[oj] = h;
-              hi[plane + oj] = __float2half_rn(w - __half2float(h));
-            }
+          for (int j = 0; j < 16; ++j) v[j] = (v[j] + fmaf(v[j], w[j] != 0.f ? back : 0.f, w[j])) * tc::exp2_int(-ex[srow + t.row[cq + j]]);
+        }
+        uint32_t h[8], l[8];
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          const __half2 a = __floats2half2_rn(v[j], v[j + 1]);
+          const float2 f = __half22float2(a);
+          const __half2 b = __floats2half2_rn(v[j] - f.x, v[j + 1] - f.y);
+          h[j / 2] = *reinterpret_cast<const uint32_t*>(&a);
+          l[j / 2] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint8_t* d = stage + lane * 64 + (((q * 2 + c) ^ (lane >> 1)) & 3) * 16;
+          *reinterpret_cast<uint4*>(d) = make_uint4(h[c * 4], h[c * 4 + 1], h[c * 4 + 2], h[c * 4 + 3]);
+          *reinterpret_cast<uint4*>(d + 2048) = make_uint4(l[c * 4], l[c * 4 + 1], l[c * 4 + 2], l[c * 4 + 3]);
         }
       }
+      __syncwarp();
+      const int c = c0 + (lane & 3) * 8, left = PB - (b0 + c), ob = t.o[c];
+      const bool run8 = vec && left >= 8 && t.o[c + 7] - ob == 7, run4 = left >= 4 && t.o[c + 3] - ob == 3, next4 = left >= 8 && t.o[c + 7] - t.o[c + 4] == 3;
+      uint4 hs[4], ls[4];
+      int oas[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = i * 8 + (lane >> 2);
+        const uint8_t* src = stage + row * 64 + (((lane & 3) ^ (row >> 1)) & 3) * 16;
+        hs[i] = *reinterpret_cast<const uint4*>(src);
+        ls[i] = *reinterpret_cast<const uint4*>(src + 2048);
+        oas[i] = ta.o[quarter * 32 + row];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int a = quarter * 32 + i * 8 + (lane >> 2), oa = oas[i], o = oa + ob;
+        const uint4 h = hs[i], l = ls[i];
+        if (a0 + a >= PA) continue;
+        if (run8 && !(o & 7)) {
+          *reinterpret_cast<uint4*>(hi + o) = h;
+          *reinterpret_cast<uint4*>(hi + plane + o) = l;
+          continue;
+        }
+        const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, lw[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int oq = oa + t.o[c + q * 4];
+          if ((q ? next4 : run4) && !(oq & 3)) {
+            *reinterpret_cast<uint2*>(hi + oq) = make_uint2(hw[q * 2], hw[q * 2 + 1]);
+            *reinterpret_cast<uint2*>(hi + plane + oq) = make_uint2(lw[q * 2], lw[q * 2 + 1]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (q * 4 + j < left) {
+                const int oj = oa + t.o[c + q * 4 + j];
+                hi[oj] = __ushort_as_half((unsigned short)(hw[q * 2 + j / 2] >> (j & 1) * 16));
+                hi[plane + oj] = __ushort_as_half((unsigned short)(lw[q * 2 + j / 2] >> (j & 1) * 16));
+              }
+          }
+        }
+      }
+      __syncwarp();
     }
+    tc::tc_fence_before_sync();
+    __syncthreads();   // the accumulators and B are free, the table of the next tile written
+  }
+  if (!fine) atomicCAS(&g_kron_status, 0, (1 << 16) | (blockIdx.x & 0xffff));
+  if (warp == 0) {
+    tc::tc_fence_after_sync();
+    tc::tmem_dealloc(tmem, 256);
   }
 }
 
@@ -1012,7 +1117,7 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   return B200CP_OK;
 }
 
-// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 62 us with the exponents, against 86 for the fp32 weight and
+// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 37 us with the exponents, against 86 for the fp32 weight and
 // its split; but 1000 x 1000 at R = 16 21 against 13, 4096 x 64 at R = 64 50 against 20.
 bool kron_planes_takes(int order, const int* idims, const int* odims, int R, int sm_count) {
   double pa = 1, pb = 1;
@@ -1037,14 +1142,24 @@ int kron_planes_launch(int order, const int* idims, const int* odims, int R, con
   B200CP_LAUNCH_OK("kron_exponent_kernel");
   const int atiles = ceil_div(g.SA * g.FA, kPT), btiles = ceil_div(g.SB * g.FB, kPT);
   if (atiles > 65535) return fail(B200CP_ERR_UNSUPPORTED, "multiplied-out weight too large");
-  const size_t smem = sizeof(float) * (align_up((size_t)R, kRC) + kRC) * kPP;
-  static std::atomic<int> set[64];
-  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kron_planes_kernel), set, (int)smem));
+  static std::atomic<int> set[2][64];
+  const auto kernel = R > 64 ? kron_planes_kernel<true> : kron_planes_kernel<false>;
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), set[R > 64], (int)kPlanesSmem));
   // as many CTAs as are resident at once share the tiles of B
   const int walkers = std::min(btiles, std::max(1, 2 * di.sm_count / atiles));
-  const dim3 grid(ceil_div(btiles, ceil_div(btiles, walkers)), atiles);
-  B200CP_CUDA_OK(launch_kernel(kron_planes_kernel, grid, dim3(256), smem, st, true, g, ldo, btiles, ex, static_cast<__half*>(hi), plane));
+  const dim3 grid(walkers, atiles);
+  const bool vec = !(ldo & 7) && !(plane & 7) && !(reinterpret_cast<uintptr_t>(hi) & 15);
+  B200CP_CUDA_OK(launch_kernel(kernel, grid, dim3(256), kPlanesSmem, st, true, g, ldo, btiles, ex, static_cast<__half*>(hi), plane, vec));
   B200CP_LAUNCH_OK("kron_planes_kernel");
+  return B200CP_OK;
+}
+
+// Reads (and clears) the status word; the caller has synchronised the device.
+int kron_device_status(int* out) {
+  int v = 0, zero = 0;
+  B200CP_CUDA_OK(cudaMemcpyFromSymbol(&v, g_kron_status, sizeof(int)));
+  if (v) B200CP_CUDA_OK(cudaMemcpyToSymbol(g_kron_status, &zero, sizeof(int)));
+  *out = v;
   return B200CP_OK;
 }
 

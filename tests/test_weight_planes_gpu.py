@@ -1,5 +1,6 @@
 """The multiplied-out weight written as operand planes: the exponents of its rows from a table of the factors' slices, up to
-64 of 256 ranks, at row counts off the 32 of a block and ranks off the 32 of a warp.  B200CP_GEMM_TC=2 takes the tensor
+64 of 256 ranks, at row counts off the 32 of a block and ranks off the 16 of an
+instruction and the 64 of a stage, one or two modes in a half, rows in runs of any length.  B200CP_GEMM_TC=2 takes the tensor
 product at every size.
 
 Bound: 5e-7 in the norm, as in test_split_gemm_gpu.py; a row's exponent that is too small would overflow its fp16 values, one that is too
