@@ -646,11 +646,15 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
     const int seg = segs == 1 ? 0 : i / quads;
     return load4(s + (size_t)seg * p.ld, (i - seg * quads) * 4, len, p.vec);
   };
+  if (segs == 1 && p.vec && !(len & 3)) {   // no condition between the loads: 4096 x 4096 24.8 -> 22.4 us
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    v[q] = q * tpr + sub < n ? at(q * tpr + sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-    mx = max4(mx, v[q]);
+    for (int q = 0; q < Q; ++q) v[q] = q * tpr + sub < n ? *reinterpret_cast<const float4*>(s + (q * tpr + sub) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = q * tpr + sub < n ? at(q * tpr + sub) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
+#pragma unroll
+  for (int q = 0; q < Q; ++q) mx = max4(mx, v[q]);
   for (int i = Q * tpr + sub; i < n; i += tpr) mx = max4(mx, at(i));
   mx = __reduce_max_sync(0xffffffffu, mx);
   if (wide) {
@@ -782,9 +786,7 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constan
   bool any = false;
 #pragma unroll
   for (int j = 0; j < 4; ++j) sc[j] = c + j < cols ? exp2_int(-p.ex[c + j]) : 1.f;
-#pragma unroll 4
-  for (int r = r0 + threadIdx.y; r < r1; r += 4) {
-    const float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
+  const auto put = [&](int r, const float4& v) {
     const float x = window_value(v.x, sc[0], any), y = window_value(v.y, sc[1], any), z = window_value(v.z, sc[2], any),
                 w = window_value(v.w, sc[3], any);
     uint16_t* d = p.hi + (size_t)r * p.ldo + c;
@@ -793,7 +795,20 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constan
     window_pair(z, w, h.y, l.y);
     *reinterpret_cast<uint2*>(d) = h;
     *reinterpret_cast<uint2*>(d + p.plane) = l;
-  }
+  };
+  // Four rows of a thread in flight, without a condition between the loads: both operands of 4096 x 4096 50 -> 41 us (eight rows 49).
+  constexpr int B = 4;
+  int r = r0 + threadIdx.y;
+  if (p.vec && c + 4 <= cols)
+    for (; r + 4 * (B - 1) < r1; r += 4 * B) {
+      float4 v[B];
+#pragma unroll
+      for (int i = 0; i < B; ++i) v[i] = *reinterpret_cast<const float4*>(p.src + (size_t)(r + 4 * i) * cols + c);
+#pragma unroll
+      for (int i = 0; i < B; ++i) put(r + 4 * i, v[i]);
+    }
+#pragma unroll 4
+  for (; r < r1; r += 4) put(r, load4(p.src + (size_t)r * cols, c, cols, p.vec));
   if (!any) return;
   for (int r = r0 + threadIdx.y; r < r1; r += 4)
     for (int j = 0; j < 4 && c + j < cols; ++j) {
