@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         for (int i = 0; i < 4; ++i) {
           const int row = warp * 16 + i0 * 2 + i + (lane >> 4) * 4;
           const float *p = f0 + t.e[row][0], *q = f1 + t.e[row][n - 1];
-          x[i][0] = __ldg(p + c0); x[i][1] = __ldg(p + c1); x[i][2] = __ldg(q + c0); x[i][3] = __ldg(q + c1);
+          x[i][0] = p[c0]; x[i][1] = p[c1]; x[i][2] = q[c0]; x[i][3] = q[c1];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
