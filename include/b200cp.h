@@ -289,8 +289,7 @@ int b200cp_dense_recompose(int order, const int* idims, const int* odims, int R,
                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* Y[b,o] = sum_i X[b,i] M[i,o] (test/benchmark_dense_cp.py:45-48) with fp32-grade results: tcgen05 with three bf16
- * parts per value and six products, or (large sizes, values within 29 binades in a column) fp16 pairs and three, where B, I, O fill
- * its tiles; CUDA cores otherwise. */
+ * parts per value and six products where B, I, O fill its tiles, CUDA cores otherwise. */
 size_t b200cp_dense_matmul_workspace_bytes(int B, int I, int O);
 int b200cp_dense_matmul(int B, int I, int O, const float* X, const float* M, float* Y, void* workspace,
                         size_t workspace_bytes, void* stream);

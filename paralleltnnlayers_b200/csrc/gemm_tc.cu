@@ -6,14 +6,11 @@
 // have an absolute error of 2^-40 of it.  The product is hi*hi + hi*lo + lo*hi (three tcgen05.mma.kind::f16; a tf32 split has
 // the same 22 bits at half the rate).
 // Gradient products.  The sum runs over samples (pixels) there, and one of them may be any number of binades above the others and
-// still add nothing (a masked sample: its gradient is zero).  No exponent that samples share keeps the others exact, so there are
-// two forms, and the data choose on the device:
-// * three bf16 values per value, 24 bits, each with its own exponent, and six products (without those below 2^-24);
-// * two fp16 values and three products, at half the tensor work, where every value of a column is within a window of 29
-//   binades, in which the pair has 22 bits (see kWindowLow; the low parts are held times 2^11 and their products have an
-//   accumulator of their own, which is what widens the window from 18).  The few values outside it (of normally distributed ones about one
-//   in ten million) are left out of the planes and added to the result in fp32, one by one; with more than kMostOutside of them
-//   in an operand the product is of the first form.  No value is ever less exact than its 22 bits, whatever the others are.
+// still add nothing (a masked sample: its gradient is zero).  No exponent that samples share keeps the others exact, so each
+// value keeps its own: x is the sum of three bf16 values, 24 bits, and the product six of theirs (without those below 2^-24).
+// Twice the tensor work: 4096 x 4096 x 4096 637 us, nine taps of 256 x 256 at 32 x 28 x 28 153, where fp16 pairs with
+// an exponent per column took 326 and 84 and lost all others beside one sample of 1e12.  (Pairs only where all of a column's values lie
+// within 29 binades, 318 and 77, still hold 23 of the 24 bits: a value in four is one unit off, and 2049 x 2049 is not exact.)
 // The tensor core cuts its fp32 sums off instead of rounding them, which over thousands of terms is a bias of 1e-5 (4096
 // terms in one accumulator: 2.9e-5 against float64 in the factor gradients).  So an accumulator holds 64 or 32 terms, the small
 // products first, and is then added to a total in registers, in fp32 with rounding.
@@ -47,27 +44,18 @@ namespace {
 using namespace tc;
 
 constexpr int kBM = 256;              // rows of a pair's tile: 128 per CTA
-constexpr int kKS = 64, kThreeKS = 32; // K of one step: of pairs, and of three parts
+constexpr int kKS = 64, kGradKS = 32; // K of one step, K-major and MN-major
 
-// Operands of a product: K-major pairs (products with the weight), MN-major three parts or pairs (gradients).
-enum Form { kRowPairs, kThree, kColumnPairs };
-
-template <int BN, int FORM>
+template <int BN, bool MN>
 struct Tile {
-  static constexpr bool MN = FORM != kRowPairs;
-  static constexpr int ks = FORM == kThree ? kThreeKS : kKS, planes = FORM == kThree ? 3 : 2;
+  static constexpr int ks = MN ? kGradKS : kKS, planes = MN ? 3 : 2;
   static constexpr int box = planes * ks * 128;                         // MN-major: 64 rows, all planes
   static constexpr int aplane = MN ? ks * 128 : 128 * 128, bplane = MN ? ks * 128 : BN / 2 * 128;   // from one plane to the next
   static constexpr int abytes = planes * 128 * ks * 2;
-  static constexpr int stage = abytes + planes * BN / 2 * ks * 2;       // 64, 48, 40 KB; three parts: 48, 36 KB
-  static constexpr int stages = FORM == kThree ? (BN == 256 ? 4 : 5) : BN == 256 ? 3 : BN == 128 ? 4 : 5;
-  static constexpr int accumulators = BN == 256 ? 2 : 4;
-  static constexpr int tmem_cols = accumulators * BN;                   // 512, 512, 256
-  // Column pairs: the last accumulator holds the products with a low part, over all of K (they are 2^-11 of the others, and so is
-  // what the cut costs them); the others hold 64 terms of the high parts.  With one of those (256 columns) the read-out
-  // has the time of the other two products of a step.
-  static constexpr int depth = accumulators - (FORM == kColumnPairs);
-  static constexpr int cross = depth;
+  static constexpr int stage = abytes + planes * BN / 2 * ks * 2;       // 64, 48, 40 KB; MN-major: 48, 36 KB
+  static constexpr int stages = MN ? (BN == 256 ? 4 : 5) : BN == 256 ? 3 : BN == 128 ? 4 : 5;
+  static constexpr int depth = BN == 256 ? 2 : 4;                       // accumulators
+  static constexpr int tmem_cols = depth * BN;                          // 512, 512, 256
   static constexpr int cols = BN == 64 ? 32 : 64;                       // of a read-out warp
   static constexpr int readers = 4 * BN / cols;                         // read-out warps: 16, 8, 8
   static constexpr int threads = 64 + 32 * readers;                     // warp 0 TMA, warp 1 MMA, the others read-out
@@ -80,15 +68,13 @@ struct SplitGemm {
   // Work units in the order in which the pairs take them: `whole` tiles with all K steps, as many as fill the pairs an
   // integer number of times, then the tiles left over, each cut into `splits` ranges of `steps` K steps.
   int whole, units, splits, steps, total;
-  int steps3, total3;            // the same in steps of three parts
   int group;                     // K of an accumulator, in instructions of 16 (see kShortSum)
   int kc, Kc;                    // K-major: steps and channels per tap (dense: one tap); MN-major: Kc = rows of K
   int FW, padH, padW, Wp;        // a filter tap (y, x) shifts the rows of A by (y - padH) * Wp + (x - padW)
-  // Pairs: a value of A stands for 2^ea of itself, one of B for 2^eb.  Rows of A with one exponent over all of K: added at the end.
+  // K-major: a value of A stands for 2^ea of itself, one of B for 2^eb.  Rows of A with one exponent over all of K: added at the end.
   // In a convolution the row that a step reads moves with the tap, so the totals take 2^(ea - 24) of each step and
   // 2^(eb + 24) at the end: 24 binades for sums of values near the largest float.
   const int *ea, *eb;
-  const struct Window* win;      // gradients: which form (null: three parts)
   float* out;                    // entry (m, n) of result p at out + p * result + off(m) + n * ldn
   size_t result;
   float* partial;                // [unit - whole][BN][256] sums of the cut tiles, without the exponents
@@ -154,9 +140,10 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
       : "memory");
 }
 
-// Instruction descriptor for kind::f16 with fp32 accumulation, M = 256 (a pair); operands of fp16 or (bf) bf16.
-__host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n, uint32_t mn, uint32_t bf) {
-  return (1u << 4) | (bf << 7) | (bf << 10) | (mn << 15) | (mn << 16) | ((n >> 3) << 17) | ((256u >> 4) << 24);
+// Instruction descriptor for kind::f16 with fp32 accumulation, M = 256 (a pair).
+// MN-major operands are bf16.
+__host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n, uint32_t mn) {
+  return (1u << 4) | (mn << 7) | (mn << 10) | (mn << 15) | (mn << 16) | ((n >> 3) << 17) | ((256u >> 4) << 24);
 }
 
 // Bounded wait shared by the roles: gives up after about a second, or as soon as another role of the CTA has given up.
@@ -192,18 +179,17 @@ __device__ __forceinline__ int tap_shift(const SplitGemm& g, int tap);
 struct UnitAt {
   int m0, n0, tap, shift, first, nsteps;   // tap of the result; shift: of the rows of A (MN-major), by that tap
 };
-template <int BN, int FORM>
+template <int BN, bool MN>
 __device__ __forceinline__ UnitAt unit_at(const SplitGemm& g, int unit) {
   UnitAt t;
-  const int steps = FORM == kThree ? g.steps3 : g.steps, total = FORM == kThree ? g.total3 : g.total;
   const int v = unit - g.whole, tile = v < 0 ? unit : g.whole + v / g.splits;
   const int per = g.tiles_m * g.tiles_n, r = tile % per;
   t.tap = tile / per;
   t.n0 = (r / g.tiles_m) * BN;
   t.m0 = (r % g.tiles_m) * kBM;
-  t.shift = FORM != kRowPairs ? tap_shift(g, t.tap) : 0;
-  t.first = v < 0 ? 0 : (v % g.splits) * steps;
-  t.nsteps = v < 0 ? total : min(steps, total - t.first);
+  t.shift = MN ? tap_shift(g, t.tap) : 0;
+  t.first = v < 0 ? 0 : (v % g.splits) * g.steps;
+  t.nsteps = v < 0 ? g.total : min(g.steps, g.total - t.first);
   return t;
 }
 // Where a step of a unit is in K: its tap (of the sum over taps of a convolution) and its place in the tap.
@@ -245,41 +231,11 @@ __device__ __forceinline__ bool row_at(const SplitGemm& g, int m, long* off) {
   return in;
 }
 
-// ---- values outside the window ------------------------------------------------------------------------------------------
-// The exponent of a column comes from a sample of it, whose largest magnitude it puts into [2^11, 2^12): values up to 16 times that
-// are still in the range of fp16.  From 2^-13 on a pair (hi, 2^11 lo) is off by at most 2^-23 of the value.
-constexpr float kWindowLow = 1.f / 8192, kWindowHigh = 65504.f;
-constexpr float kLowScale = 2048.f;
-// What four products of 16 terms lose by cutting off, on average, of their sum: given back at the end (factor gradients of 12 layers
-// against float64: 0.97 of the error of three parts, without it 1.02).  Where no value has a low part nothing is cut
-// off (whole numbers), and nothing is given back.
-constexpr float kCutOff = 1.5f / (1 << 24);
-constexpr int kMostOutside = 64;   // of an operand, that are added one by one
-constexpr int kManySampled = 4;    // in the samples: the data are wide, and the pairs are not tried
-struct Outside {
-  int k, col;
-  float value;
-};
-struct Window {
-  int wide, count[2];
-  Outside list[2][kMostOutside];
-};
-__device__ __forceinline__ bool outside_window(float v) {   // of a scaled value; infinities and NaN are outside
-  return !(fabsf(v) <= kWindowHigh) || (v != 0.f && fabsf(v) < kWindowLow);
-}
-__device__ __forceinline__ bool pairs_overflow(const Window& w) { return w.count[0] > kMostOutside || w.count[1] > kMostOutside; }
-__device__ __forceinline__ bool takes_three(const Window* w) { return !w || w->wide || pairs_overflow(*w); }
-__device__ __forceinline__ int window_exponent(unsigned bits) { return bits == 0 ? 0 : max((int)(bits >> 23) - 138, kLeast); }
-__device__ __forceinline__ void add_outside(Window* w, int operand, int k, int col, float value) {
-  if (*(volatile int*)&w->count[operand] > kMostOutside) return;
-  const int i = atomicAdd(&w->count[operand], 1);
-  if (i < kMostOutside) w->list[operand][i] = Outside{k, col, value};
-}
-
-template <int BN, int FORM, bool CONV>
-__device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap& mapA, const CUtensorMap& mapB) {
-  using T = Tile<BN, FORM>;
-  constexpr bool MN = T::MN;
+template <int BN, bool MN, bool CONV>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Tile<BN, MN>::threads, 1)
+split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ CUtensorMap mapA,
+                  const __grid_constant__ CUtensorMap mapB) {
+  using T = Tile<BN, MN>;
   constexpr int kStages = T::stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -290,7 +246,6 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
   uint64_t* accfree = accfull + 4;       // [depth] the leader's: read out by the warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert(T::accumulators <= 4, "barriers");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -300,7 +255,7 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
-    for (int i = 0; i < T::accumulators; ++i) {
+    for (int i = 0; i < T::depth; ++i) {
       mbar_init(&accfull[i], 1);
       mbar_init(&accfree[i], 2 * T::readers);
     }
@@ -325,7 +280,7 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
       int it = 0;
       bool ok = true;
       for (int unit = pair; unit < g.units && ok; unit += npairs) {
-        const UnitAt t = unit_at<BN, FORM>(g, unit);
+        const UnitAt t = unit_at<BN, MN>(g, unit);
         StepAt k = step_at<CONV>(g, t.first);
         for (int s = 0; s < t.nsteps; ++s, ++it, next_step<CONV>(g, k)) {
           const int slot = it % kStages;
@@ -333,7 +288,7 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
           if (rank == 0) mbar_expect_tx(&full[slot], 2 * T::stage);
           const uint32_t bar = leader_addr(fullb + slot * 8);
           const uint32_t a = smem_u32(sm) + slot * T::stage, b = a + T::abytes;
-          if (MN) {   // boxes of 64 rows x the k, all planes; rows of K outside the tensor read as zero
+          if (MN) {   // boxes of 64 rows x 32 k, all planes; rows of K outside the tensor read as zero
 #pragma unroll
             for (int q = 0; q < 2; ++q)
               tma_load_pair(a + q * T::box, &mapA, bar, t.m0 + rank * 128 + q * 64, k.c * T::ks + t.shift, 0);
@@ -351,16 +306,16 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
   } else if (warp == 1) {
     // ================= MMA issuer: one thread of the pair ====================================================================
     if (rank == 0 && lane == 0) {
-      const uint32_t idesc = make_idesc_f16(BN, MN, FORM == kThree);
+      const uint32_t idesc = make_idesc_f16(BN, MN ? 1 : 0);
       // K-major: rows of 128 bytes, 8 rows per swizzle atom (SBO 1024); 16 k = 32 bytes on.
       // MN-major: 64 rows of the operand (128 bytes) per k, 8 k per atom (SBO 1024), the next 64 rows LBO on; 16 k = 2048 bytes on.
       const uint64_t d0 = make_smem_desc(0, MN ? T::box : 16, 1024, kSwizzle128B);
       constexpr uint32_t kstep = MN ? 2048 : 32;
       const uint32_t base = smem_u32(sm);
-      int it = 0, gi = 0, nu = 0;   // steps, accumulators, units
+      int it = 0, gi = 0;   // steps, accumulators
       bool ok = true;
-      for (int unit = pair; unit < g.units && ok; unit += npairs, ++nu) {
-        const UnitAt t = unit_at<BN, FORM>(g, unit);
+      for (int unit = pair; unit < g.units && ok; unit += npairs) {
+        const UnitAt t = unit_at<BN, MN>(g, unit);
         StepAt k = step_at<CONV>(g, t.first);
         for (int s = 0; s < t.nsteps && ok; ++s, ++it, next_step<CONV>(g, k)) {
           const int slot = it % kStages, kk = k16_of<T::ks>(g, k.c);
@@ -369,56 +324,32 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
           const uint32_t a = base + slot * T::stage, b = a + T::abytes;
           const uint64_t ah = d0 + (a >> 4), bh = d0 + (b >> 4);
           constexpr uint64_t A1 = T::aplane >> 4, B1 = T::bplane >> 4, A2 = 2 * A1, B2 = 2 * B1;   // to the further planes
-          if constexpr (FORM == kColumnPairs) {
-            constexpr uint32_t low = T::cross * BN;
-            const int buf = gi % T::depth;
+          for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
+            const int buf = gi % T::depth, i1 = min(kk, i0 + g.group);
             if (gi >= T::depth && !(ok = wait_or_abort(accfreeb + buf * 8, (gi / T::depth - 1) & 1, abortb))) break;
             tc_fence_after_sync();
-            for (int i = 0; i < kk; ++i) {
+            const uint32_t d = tmem_base + buf * BN;
+            if (MN) {   // products of 2^-16 first
+              for (int i = i0; i < i1; ++i) {
+                const uint64_t o = (uint64_t)((i * kstep) >> 4);
+                mma_f16_pair(d, ah + A2 + o, bh + o, idesc, i > i0);
+                mma_f16_pair(d, ah + o, bh + B2 + o, idesc, true);
+                mma_f16_pair(d, ah + A1 + o, bh + B1 + o, idesc, true);
+              }
+            }
+            for (int i = i0; i < i1; ++i) {
               const uint64_t o = (uint64_t)((i * kstep) >> 4);
-              mma_f16_pair(tmem_base + buf * BN, ah + o, bh + o, idesc, i > 0);
+              mma_f16_pair(d, ah + A1 + o, bh + o, idesc, MN || i > i0);
+              mma_f16_pair(d, ah + o, bh + B1 + o, idesc, true);
+            }
+            for (int i = i0; i < i1; ++i) {
+              const uint64_t o = (uint64_t)((i * kstep) >> 4);
+              mma_f16_pair(d, ah + o, bh + o, idesc, true);
             }
             commit_pair(accfullb + buf * 8);
-            ++gi;
-            if (s == 0 && nu > 0) {
-              if (!(ok = wait_or_abort(accfreeb + T::cross * 8, (nu - 1) & 1, abortb))) break;
-              tc_fence_after_sync();
-            }
-            for (int i = 0; i < kk; ++i) {
-              const uint64_t o = (uint64_t)((i * kstep) >> 4);
-              mma_f16_pair(tmem_base + low, ah + A1 + o, bh + o, idesc, s > 0 || i > 0);
-              mma_f16_pair(tmem_base + low, ah + o, bh + B1 + o, idesc, true);
-            }
-            commit_pair(emptyb + slot * 8);
-            if (s == t.nsteps - 1) commit_pair(accfullb + T::cross * 8);
-          } else {
-            for (int i0 = 0; i0 < kk; i0 += g.group, ++gi) {
-              const int buf = gi % T::depth, i1 = min(kk, i0 + g.group);
-              if (gi >= T::depth && !(ok = wait_or_abort(accfreeb + buf * 8, (gi / T::depth - 1) & 1, abortb))) break;
-              tc_fence_after_sync();
-              const uint32_t d = tmem_base + buf * BN;
-              if (FORM == kThree) {   // products of 2^-16 first
-                for (int i = i0; i < i1; ++i) {
-                  const uint64_t o = (uint64_t)((i * kstep) >> 4);
-                  mma_f16_pair(d, ah + A2 + o, bh + o, idesc, i > i0);
-                  mma_f16_pair(d, ah + o, bh + B2 + o, idesc, true);
-                  mma_f16_pair(d, ah + A1 + o, bh + B1 + o, idesc, true);
-                }
-              }
-              for (int i = i0; i < i1; ++i) {
-                const uint64_t o = (uint64_t)((i * kstep) >> 4);
-                mma_f16_pair(d, ah + A1 + o, bh + o, idesc, FORM == kThree || i > i0);
-                mma_f16_pair(d, ah + o, bh + B1 + o, idesc, true);
-              }
-              for (int i = i0; i < i1; ++i) {
-                const uint64_t o = (uint64_t)((i * kstep) >> 4);
-                mma_f16_pair(d, ah + o, bh + o, idesc, true);
-              }
-              commit_pair(accfullb + buf * 8);
-            }
-            if (!ok) break;
-            commit_pair(emptyb + slot * 8);
           }
+          if (!ok) break;
+          commit_pair(emptyb + slot * 8);
         }
       }
     }
@@ -427,15 +358,15 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
     constexpr int NC = T::cols;
     const int qd = warp & 3, c0 = ((warp - 2) >> 2) * NC;   // the TMEM lane quarter this warp may read, and its columns
     const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + c0;
-    int gi = 0, nu = 0;
+    int gi = 0;
     bool ok = true;
-    for (int unit = pair; unit < g.units && ok; unit += npairs, ++nu) {
+    for (int unit = pair; unit < g.units && ok; unit += npairs) {
       float tot[NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) tot[j] = 0.f;
       int buf = 0;
       {
-        const UnitAt t = unit_at<BN, FORM>(g, unit);
+        const UnitAt t = unit_at<BN, MN>(g, unit);
         StepAt k = step_at<CONV>(g, t.first);
         for (int left = t.nsteps; left > 0 && ok; --left, next_step<CONV>(g, k)) {
           float f = 0.f;
@@ -452,7 +383,7 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
             for (int j0 = 0; j0 < NC; j0 += 16) {
               float v[16];
               tmem_ld16(taddr + buf * BN + j0, v);
-              if (j0 + 16 == NC && (FORM == kColumnPairs || left > 1 || i0 + g.group < kk)) {
+              if (j0 + 16 == NC && (left > 1 || i0 + g.group < kk)) {
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) arrive_cluster(leader_addr(accfreeb + buf * 8));
@@ -464,50 +395,30 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
         }
       }
       if (!ok) break;
-      if (FORM == kColumnPairs) {   // the products with a low part
-        buf = T::cross;
-        if (!(ok = __all_sync(0xffffffffu, wait_or_abort(accfullb + buf * 8, nu & 1, abortb)))) break;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int j0 = 0; j0 < NC; j0 += 16) {
-#pragma unroll
-          for (int h = 0; h < 16; h += 8) {
-            float v[8];
-            tmem_ld8(taddr + buf * BN + j0 + h, v);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float x = fmaf(v[j], 1.f / kLowScale, tot[j0 + h + j]);
-              tot[j0 + h + j] = v[j] != 0.f ? fmaf(x, kCutOff, x) : x;
-            }
-          }
-          tmem_st16(taddr + buf * BN + j0, tot + j0);
-        }
-      }
       // The totals go through the accumulator just read, so that a short loop stores them: unrolled over registers the
       // stores are 30 KB of code that every tile fetches anew: 8 us a tile (4096 x 4096 x 1024: 121 us, now 99).
-      if (FORM != kColumnPairs)
 #pragma unroll
       for (int j0 = 0; j0 < NC; j0 += 16) tmem_st16(taddr + buf * BN + j0, tot + j0);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      const UnitAt t = unit_at<BN, FORM>(g, unit);   // again: cheaper than registers held through the loop
+      const UnitAt t = unit_at<BN, MN>(g, unit);   // again: cheaper than registers held through the loop
       const int row = rank * 128 + qd * 32 + lane, m = t.m0 + row;
       const bool cut = unit >= g.whole && g.splits > 1;
       long off = row;
       bool in = true;
       if (!cut) in = row_at<CONV>(g, m, &off);
       const long ldn = cut ? kBM : g.ldn;
-      const int e = cut || FORM == kThree ? 0 : CONV ? kRowShift : in ? g.ea[m] : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
+      const int e = cut || MN ? 0 : CONV ? kRowShift : in ? g.ea[m] : 0, n0 = t.n0 + c0, N = cut ? t.n0 + BN : g.N;
       float* dst = cut ? g.partial + ((size_t)(unit - g.whole) * BN + c0) * kBM + off
                        : g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn;
       const int* eb = g.eb + n0 + (lane & 15);
-      int next = FORM != kThree && !cut && n0 + (lane & 15) < N ? *eb : 0;
+      int next = !MN && !cut && n0 + (lane & 15) < N ? *eb : 0;
 #pragma unroll 1
       for (int j0 = 0; j0 < NC; j0 += 16) {
         float v[16];
         tmem_ld16(taddr + buf * BN + j0, v);
         const int ebv = next, left = N - n0 - j0;
-        next = FORM != kThree && !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? eb[j0 + 16] : 0;
-        if (FORM != kThree) {
+        next = !MN && !cut && j0 + 16 + (lane & 15) < min(NC, N - n0) ? eb[j0 + 16] : 0;
+        if (!MN) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
         }
@@ -542,36 +453,17 @@ __device__ __forceinline__ void gemm_role(const SplitGemm& g, const CUtensorMap&
   }
 }
 
-// KIND: kRowPairs, kThree, or kColumnPairs: the form of a gradient that its operands allow.
-template <int BN, int KIND, bool CONV>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Tile<BN, KIND>::threads, 1)
-split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ CUtensorMap mapA,
-                  const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapA3,
-                  const __grid_constant__ CUtensorMap mapB3) {
-  if (KIND == kColumnPairs) {
-    grid_dependency_wait();
-    if (takes_three(g.win))
-      gemm_role<BN, kThree, CONV>(g, mapA3, mapB3);
-    else
-      gemm_role<BN, kColumnPairs, CONV>(g, mapA, mapB);
-  } else {
-    gemm_role<BN, KIND, CONV>(g, mapA, mapB);
-  }
-}
-
-
 // The sums of a cut tile, in the order of K, and the exponents.  grid (cut tiles, BN / 8), one row per
 // thread: enough CTAs to keep the L2 busy (34 tiles cut in two: 24 us with 32 columns per CTA, 6 with 8).
 constexpr int kJoinCols = 8;
-template <int BN, int KIND, bool CONV>
+template <int BN, bool MN, bool CONV>
 __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__ SplitGemm g) {
   grid_dependency_wait();
-  const bool plain = KIND != kRowPairs && takes_three(g.win);   // no exponents
-  const UnitAt t = unit_at<BN, KIND>(g, g.whole + blockIdx.x * g.splits);
+  const UnitAt t = unit_at<BN, MN>(g, g.whole + blockIdx.x * g.splits);
   const int m = t.m0 + threadIdx.x;
   long off;
   if (!row_at<CONV>(g, m, &off)) return;
-  const int e = plain ? 0 : CONV ? kRowShift : g.ea[m];
+  const int e = MN ? 0 : CONV ? kRowShift : g.ea[m];
   const int n0 = t.n0 + blockIdx.y * kJoinCols;
   const float* src = g.partial + ((size_t)blockIdx.x * g.splits * BN + blockIdx.y * kJoinCols) * kBM + threadIdx.x;
   float* dst = g.out + (size_t)t.tap * g.result + off;
@@ -583,7 +475,7 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
     for (int j = 0; j < kJoinCols; ++j) v[j] += __ldcs(src + ((size_t)q * BN + j) * kBM);
 #pragma unroll
   for (int j = 0; j < kJoinCols; ++j)
-    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = plain ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
+    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
 }
 
 // ---- operand planes -----------------------------------------------------------------------------------------------------
@@ -681,122 +573,21 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
   for (int i = Q * tpr + sub; i < n; i += tpr) put(i, at(i));
 }
 
-// Exponents of the columns of the two operands [rows][len] of a gradient, from kSamples rows of them, and how many of the samples
-// are outside their window (`bad`, one entry per CTA).  Block (32, 16): 128 columns.
-constexpr int kSamples = 128;
-__global__ void __launch_bounds__(512) sample_columns_kernel(const __grid_constant__ SplitJobs jobs, Window* win, int* bad) {
-  __shared__ unsigned red[16][128];
-  grid_dependency_wait();
-  const int first = (jobs.job[0].len + 127) / 128;
-  const bool second = (int)blockIdx.x >= first;
-  const SplitJob& p = jobs.job[second];
-  const int cols = p.len, c = (blockIdx.x - (second ? first : 0)) * 128 + threadIdx.x * 4;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) win->count[0] = win->count[1] = 0;
-  constexpr int Q = kSamples / 16;
-  float4 v[Q];
-  uint4 m = make_uint4(0, 0, 0, 0);
-  const auto finite = [](float x) { return abs_bits(x) < 0x7f800000u ? abs_bits(x) : 0u; };
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const long r = (long)(q * 16 + threadIdx.y) * p.rows / kSamples;
-    v[q] = c < cols ? load4(p.src + (size_t)r * cols, c, cols, p.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    m.x = max(m.x, finite(v[q].x));
-    m.y = max(m.y, finite(v[q].y));
-    m.z = max(m.z, finite(v[q].z));
-    m.w = max(m.w, finite(v[q].w));
-  }
-  *reinterpret_cast<uint4*>(&red[threadIdx.y][threadIdx.x * 4]) = m;
-  __syncthreads();
-  int e[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    unsigned x = red[0][threadIdx.x * 4 + j];
-#pragma unroll
-    for (int i = 1; i < 16; ++i) x = max(x, red[i][threadIdx.x * 4 + j]);
-    e[j] = window_exponent(x);
-    if (threadIdx.y == 0 && c + j < cols) p.ex[c + j] = e[j];
-  }
-  int out = 0;
-#pragma unroll
-  for (int q = 0; q < Q; ++q)
-    out += outside_window(v[q].x * exp2_int(-e[0])) + outside_window(v[q].y * exp2_int(-e[1])) +
-           outside_window(v[q].z * exp2_int(-e[2])) + outside_window(v[q].w * exp2_int(-e[3]));
-  const int some = __syncthreads_count(out > 0), many = __syncthreads_or(out > kManySampled);
-  if (threadIdx.x == 0 && threadIdx.y == 0) bad[blockIdx.x] = many ? kManySampled : some;
-}
-
-// Which form a split writes: of the first launch (`again` false) by the samples, of the second three parts where the pairs have too many
-// values outside.  Every thread of the CTA calls it.
-struct FormOf {
-  Window* win;    // null: three parts
-  const int* bad;
-  int nbad;
-  bool again;
-};
-enum { kWriteNothing, kWritePairs, kWriteThree };
-__device__ __forceinline__ int form_of(const FormOf& f, int tid, int threads, bool first) {
-  if (!f.win) return kWriteThree;
-  if (f.again) return !f.win->wide && pairs_overflow(*f.win) ? kWriteThree : kWriteNothing;
-  int n = 0;
-  for (int i = tid; i < f.nbad; i += threads) n = max(n, f.bad[i]);
-  const bool wide = __syncthreads_count(n > 0) >= kManySampled || __syncthreads_or(n >= kManySampled);
-  if (first && tid == 0) f.win->wide = wide;
-  return wide ? kWriteThree : kWritePairs;
-}
-// A scaled value, or zero where it is outside (the caller lists it later: a branch between the loads would keep them apart)
-__device__ __forceinline__ float window_value(float v, float sc, bool& any) {
-  const float x = v * sc;
-  const bool out = outside_window(x);
-  any |= out;
-  return out ? 0.f : x;
-}
-// hi and 2^11 lo of two of them
-__device__ __forceinline__ void window_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(a, b);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn((a - f.x) * kLowScale, (b - f.y) * kLowScale);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// [rows][len] as three bf16 planes or as pairs with the exponents of the columns.  Block (64, 4): 256 columns, every fourth row of a range.
-__global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constant__ SplitJobs jobs, const __grid_constant__ FormOf form) {
+// [rows][len] as three bf16 planes.  Block (64, 4): 256 columns, every fourth row of a range.
+__global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constant__ SplitJobs jobs) {
   grid_dependency_wait();
   const bool second = (int)blockIdx.x >= jobs.first;
   const SplitJob& p = jobs.job[second];
   const int cols = p.len, c = (blockIdx.x - (second ? jobs.first : 0)) * 256 + threadIdx.x * 4;
   const int r0 = blockIdx.y * p.per, r1 = min(p.rows, r0 + p.per);
-  const int write = form_of(form, threadIdx.y * 64 + threadIdx.x, 256, blockIdx.x == 0 && blockIdx.y == 0);
-  if (c >= cols || write == kWriteNothing) return;
-  if (write == kWriteThree) {
-#pragma unroll 4
-    for (int r = r0 + threadIdx.y; r < r1; r += 4) {
-      const float4 v = load4(p.src + (size_t)r * cols, c, cols, p.vec);
-      const Bf3 x = split3(v.x, v.y), y = split3(v.z, v.w);
-      uint16_t* d = p.hi + (size_t)r * p.ldo + c;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(d + q * p.plane) = make_uint2(x.p[q], y.p[q]);
-    }
-    return;
-  }
-  float sc[4];
-  bool any = false;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) sc[j] = c + j < cols ? exp2_int(-p.ex[c + j]) : 1.f;
+  if (c >= cols) return;
   const auto put = [&](int r, const float4& v) {
-    const float x = window_value(v.x, sc[0], any), y = window_value(v.y, sc[1], any), z = window_value(v.z, sc[2], any),
-                w = window_value(v.w, sc[3], any);
+    const Bf3 x = split3(v.x, v.y), y = split3(v.z, v.w);
     uint16_t* d = p.hi + (size_t)r * p.ldo + c;
-    uint2 h, l;
-    window_pair(x, y, h.x, l.x);
-    window_pair(z, w, h.y, l.y);
-    *reinterpret_cast<uint2*>(d) = h;
-    *reinterpret_cast<uint2*>(d + p.plane) = l;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(d + q * p.plane) = make_uint2(x.p[q], y.p[q]);
   };
-  // Four rows of a thread in flight, without a condition between the loads: both operands of 4096 x 4096 50 -> 41 us (eight rows 49).
+  // Four rows of a thread in flight, without a condition between the loads: both operands of 4096 x 4096 52 -> 50 us.
   constexpr int B = 4;
   int r = r0 + threadIdx.y;
   if (p.vec && c + 4 <= cols)
@@ -809,12 +600,6 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constan
     }
 #pragma unroll 4
   for (; r < r1; r += 4) put(r, load4(p.src + (size_t)r * cols, c, cols, p.vec));
-  if (!any) return;
-  for (int r = r0 + threadIdx.y; r < r1; r += 4)
-    for (int j = 0; j < 4 && c + j < cols; ++j) {
-      const float v = p.src[(size_t)r * cols + c + j];
-      if (outside_window(v * sc[j])) add_outside(form.win, second, r, c + j, v);
-    }
 }
 
 // NCHW -> [n][pixel][channel] planes with padW zero pixels after each row and padH zero rows after each image: what a filter
@@ -824,56 +609,23 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constan
 struct Images {
   int N, H, W, padH, padW;
 };
-// The same sample for the channels of two tensors [N][len][H][W]: a warp per channel, eight runs of 32 pixels.
-__global__ void __launch_bounds__(256) sample_channels_kernel(const __grid_constant__ SplitJobs jobs, const Images im, Window* win, int* bad) {
-  grid_dependency_wait();
-  const int ch = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const bool second = ch >= jobs.job[0].len;
-  const SplitJob& p = jobs.job[second];
-  const int c = second ? ch - jobs.job[0].len : ch, HW = im.H * im.W;
-  const long all = (long)im.N * HW;
-  if (blockIdx.x == 0 && threadIdx.x == 0) win->count[0] = win->count[1] = 0;
-  float v[8];
-  unsigned m = 0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const long at = min(q * all / 8 + lane, all - 1), n = at / HW;
-    v[q] = c < p.len ? p.src[((size_t)n * p.len + c) * HW + (at - n * HW)] : 0.f;
-  }
-#pragma unroll
-  for (int q = 0; q < 8; ++q) m = max(m, abs_bits(v[q]) < 0x7f800000u ? abs_bits(v[q]) : 0u);
-  const int e = window_exponent(__reduce_max_sync(0xffffffffu, m));
-  if (lane == 0 && c < p.len) p.ex[c] = e;
-  int out = 0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) out += outside_window(v[q] * exp2_int(-e));
-  const int some = __syncthreads_count(out > 0), many = __syncthreads_or(out > kManySampled);
-  if (threadIdx.x == 0) bad[blockIdx.x] = many ? kManySampled : some;
-}
-
 // What bounds it is memory latency, so a thread has the loads of 32 channels of its pixel in flight and four CTAs share an SM; four channels of a
 // pixel are together in shared memory (16-byte accesses, eight bytes of a plane per store).  32 images of 256 channels 28x28: pairs by pixel 14.9
-// -> 11.6 us, both operands of a gradient 32.5 -> 23.5 (with 16 loads in flight and channels apart; three or four CTAs alike, five 12.4 and 25.4).
+// -> 11.6 us (with 16 loads in flight and channels apart; three or four CTAs alike, five 12.4).
 constexpr int kPxTile = 32, kPxPitch = kPxTile + 1;   // of four channels
-// GRAD: the operands of a gradient (bf16 planes, or pairs with an exponent per channel); otherwise pairs with an exponent per pixel.
-template <bool GRAD>
-__global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_constant__ SplitJobs jobs, const Images im,
-                                                           const __grid_constant__ FormOf form) {
+template <bool THREE>
+__global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_constant__ SplitJobs jobs, const Images im) {
   extern __shared__ float px_smem[];
   __shared__ unsigned red[8][kPxTile];
   const bool second = (int)blockIdx.x >= jobs.first;
   const SplitJob& job = jobs.job[second];
   const int CH = job.len, HW = im.H * im.W;
   const int quads = (CH + 3) / 4;
-  float4* tile = reinterpret_cast<float4*>(px_smem);            // [quads][kPxPitch]
-  float* scale = px_smem + 4 * quads * kPxPitch;                // [kPxTile], of gradients [4 * quads]
+  float4* tile = reinterpret_cast<float4*>(px_smem);      // [quads][kPxPitch]
+  float* scale = px_smem + 4 * quads * kPxPitch;          // [kPxTile]
   const int Wp = im.W + im.padW, PP = (im.H + im.padH) * Wp, rows = job.rows;
   const int p0 = (blockIdx.x - (second ? jobs.first : 0)) * kPxTile, tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
   grid_dependency_wait();
-  const int write = GRAD ? form_of(form, tid, 256, blockIdx.x == 0) : kWritePairs;
-  if (write == kWriteNothing) return;
-  if (GRAD && write == kWritePairs)
-    for (int c = tid; c < 4 * quads; c += 256) scale[c] = c < CH ? exp2_int(-job.ex[c]) : 0.f;
   {
     const int p = p0 + tx, n = p / PP, q = p - n * PP, h = q / Wp, w = q - h * Wp;
     const bool in = p < rows && h < im.H && w < im.W;
@@ -899,7 +651,7 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
     red[ty][tx] = m;
   }
   __syncthreads();
-  if (!GRAD) {
+  if (!THREE) {
     if (tid < kPxTile) {
       unsigned m = red[0][tid];
 #pragma unroll
@@ -910,28 +662,18 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
     }
     __syncthreads();
   }
-  // a warp writes the channels of a pixel, two per lane
-  [[maybe_unused]] bool any = false;
+  // a warp writes the channels of a pixel, four per lane
   for (int k = tx; k < quads; k += 32) {
-    const float4 sc = GRAD && write == kWritePairs ? *reinterpret_cast<const float4*>(scale + 4 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < kPxTile / 8; ++j) {
       const int i = ty + j * 8;
       if (p0 + i >= rows) break;
       uint16_t* d = job.hi + (size_t)(p0 + i) * job.ldo + 4 * k;
       const float4 v = tile[k * kPxPitch + i];
-      if (GRAD && write == kWriteThree) {
+      if (THREE) {
         const Bf3 x = split3(v.x, v.y), y = split3(v.z, v.w);
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(d + q * job.plane) = make_uint2(x.p[q], y.p[q]);
-      } else if (GRAD) {
-        uint2 h, l;
-        const float a = window_value(v.x, sc.x, any), b = window_value(v.y, sc.y, any), c = window_value(v.z, sc.z, any),
-                    e = window_value(v.w, sc.w, any);
-        window_pair(a, b, h.x, l.x);
-        window_pair(c, e, h.y, l.y);
-        *reinterpret_cast<uint2*>(d) = h;
-        *reinterpret_cast<uint2*>(d + job.plane) = l;
       } else {
         Half4 h, l;
         split4(v, scale[i], h, l);
@@ -939,81 +681,6 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
         *reinterpret_cast<Half4*>(d + job.plane) = l;
       }
     }
-  }
-  if constexpr (GRAD) {
-    if (!any || write != kWritePairs) return;
-    for (int i = ty; i < kPxTile && p0 + i < rows; i += 8)
-      for (int k = tx; k < quads; k += 32)   // (what this thread has written)
-        for (int c = 4 * k; c < min(CH, 4 * k + 4); ++c) {
-          const float v = reinterpret_cast<const float*>(tile + k * kPxPitch + i)[c & 3];
-          if (outside_window(v * scale[c])) add_outside(form.win, second, p0 + i, c, v);
-        }
-  }
-}
-
-// Adds the products of the values outside the window to the gradient, in fp32 and in the order of (k, column).  grid (ceil(N / 32),
-// taps, ceil(M / 1024)): a CTA has 32 rows x 1024 columns of a result [N][M] to itself.  First the values of operand 0 (a column of the rows each), then those of
-// operand 1 (a row each), whose products with a value of operand 0 that is outside too are there already.
-struct OutsideSource {
-  const float* src[2];
-  int len[2];
-  const int* ex0;      // exponents of operand 0
-  int K, H, W, Wp, PP; // PP == 0: [K][len]; else pixels of images [n][len][H][W] with padding, as the planes have them
-};
-__device__ __forceinline__ bool source_at(const OutsideSource& s, int operand, int k, int col, float* v) {   // false: padding
-  if (k < 0 || k >= s.K) return false;
-  if (s.PP == 0) {
-    *v = s.src[operand][(size_t)k * s.len[operand] + col];
-    return true;
-  }
-  const int n = k / s.PP, p = k - n * s.PP, h = p / s.Wp, w = p - h * s.Wp;
-  if (h >= s.H || w >= s.W) return false;
-  *v = s.src[operand][(((size_t)n * s.len[operand] + col) * s.H + h) * s.W + w];
-  return true;
-}
-__global__ void __launch_bounds__(256) add_outside_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ OutsideSource src) {
-  __shared__ Outside list[2][kMostOutside];
-  grid_dependency_wait();
-  const Window& win = *g.win;
-  const int n[2] = {win.count[0], win.count[1]}, tid = threadIdx.x;
-  if (takes_three(&win) || n[0] + n[1] == 0) return;
-  if (tid < 2 * kMostOutside) {   // sorted: the order in which they were found is not that of the next call
-    const int q = tid / kMostOutside, i = tid % kMostOutside;
-    if (i < n[q]) {
-      const Outside a = win.list[q][i];
-      int at = 0;
-      for (int j = 0; j < n[q]; ++j) {
-        const Outside b = win.list[q][j];
-        at += b.k < a.k || (b.k == a.k && b.col < a.col);
-      }
-      list[q][at] = a;
-    }
-  }
-  __syncthreads();
-  const int tap = blockIdx.y, shift = tap_shift(g, tap), r0 = blockIdx.x * 32, m0 = blockIdx.z * 1024, lane = tid & 31, warp = tid >> 5;
-  float* out = g.out + (size_t)tap * g.result;   // entry (m, n): m columns of operand 0, n of operand 1
-  for (int i = 0; i < n[0]; ++i) {
-    const Outside a = list[0][i];
-    float y;
-    if ((a.col & 7) == warp && a.col / 1024 == (int)blockIdx.z && r0 + lane < g.N && source_at(src, 1, a.k - shift, r0 + lane, &y))
-      out[a.col + (long)(r0 + lane) * g.ldn] += a.value * y;
-  }
-  __syncthreads();
-  for (int i = 0; i < n[1]; ++i) {
-    const Outside a = list[1][i];
-    if (a.col < r0 || a.col >= r0 + 32) continue;
-    float* row = out + (long)a.col * g.ldn;
-    float x[4], sum[4];
-    bool in[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + j * 256 + tid;
-      in[j] = m < g.M && source_at(src, 0, a.k + shift, m, &x[j]) && !outside_window(x[j] * exp2_int(-src.ex0[m]));
-      sum[j] = in[j] ? row[m] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (in[j]) row[m0 + j * 256 + tid] = sum[j] + a.value * x[j];
   }
 }
 
@@ -1078,44 +745,27 @@ int split_rows(const SplitJob& a, const SplitJob& b, cudaStream_t st) {
   B200CP_LAUNCH_OK("split_rows_kernel");
   return B200CP_OK;
 }
-// The operands of a gradient, of the same number of rows: three parts, or (form.win) pairs where the data allow them.
-int split_columns(SplitJob a, SplitJob b, FormOf form, cudaStream_t st) {
-  a.per = b.per = std::max(16, ceil_div(a.rows, 128));
+int split_columns(SplitJob a, SplitJob b, cudaStream_t st) {   // of the same number of rows
+  a.per = b.per = std::max(16, ceil_div(a.rows, 64));
   SplitJobs jobs{{a, b}, ceil_div(a.len, 256)};
-  const dim3 ctas(jobs.first + ceil_div(b.len, 256), ceil_div(a.rows, a.per));
-  if (form.win) {
-    form.nbad = ceil_div(a.len, 128) + ceil_div(b.len, 128);
-    B200CP_CUDA_OK(launch_kernel(sample_columns_kernel, dim3(form.nbad), dim3(32, 16), 0, st, true, jobs, form.win, const_cast<int*>(form.bad)));
-    B200CP_LAUNCH_OK("sample_columns_kernel");
-  }
-  for (int again = 0; again <= (form.win != nullptr); ++again) {
-    form.again = again;
-    B200CP_CUDA_OK(launch_kernel(split_columns_kernel, ctas, dim3(64, 4), 0, st, true, jobs, form));
-    B200CP_LAUNCH_OK("split_columns_kernel");
-  }
+  B200CP_CUDA_OK(launch_kernel(split_columns_kernel, dim3(jobs.first + ceil_div(b.len, 256), ceil_div(a.rows, a.per)), dim3(64, 4), 0,
+                               st, true, jobs));
+  B200CP_LAUNCH_OK("split_columns_kernel");
   return B200CP_OK;
 }
 constexpr int kMostChannels = 1024;   // of split_pixels_kernel's tile: 139 KB
-// the pairs of one tensor, or (GRAD) the operands of a gradient
-template <bool GRAD>
-int split_pixels(const SplitJob& a, const SplitJob& b, const Images& im, FormOf form, cudaStream_t st) {
+// the fp16 planes of one tensor, or (THREE) the bf16 planes of two
+template <bool THREE>
+int split_pixels(const SplitJob& a, const SplitJob& b, const Images& im, cudaStream_t st) {
   const SplitJobs jobs{{a, b}, ceil_div(a.rows, kPxTile)};
   const int most = std::max(a.len, b.len);
   const int channels = (most + 3) / 4 * 4;
-  const size_t smem = sizeof(float) * ((size_t)channels * kPxPitch + (GRAD ? std::max(channels, kPxTile) : kPxTile));
+  const size_t smem = sizeof(float) * ((size_t)channels * kPxPitch + kPxTile);
   static std::atomic<int> set[64];
-  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_pixels_kernel<GRAD>), set, (int)smem));
-  if (form.win) {
-    form.nbad = ceil_div(a.len + b.len, 8);
-    B200CP_CUDA_OK(launch_kernel(sample_channels_kernel, dim3(form.nbad), dim3(256), 0, st, true, jobs, im, form.win, const_cast<int*>(form.bad)));
-    B200CP_LAUNCH_OK("sample_channels_kernel");
-  }
-  for (int again = 0; again <= (form.win != nullptr); ++again) {
-    form.again = again;
-    B200CP_CUDA_OK(launch_kernel(split_pixels_kernel<GRAD>, dim3(jobs.first + ceil_div(b.rows, kPxTile)), dim3(32, 8), smem, st, true,
-                                 jobs, im, form));
-    B200CP_LAUNCH_OK("split_pixels_kernel");
-  }
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_pixels_kernel<THREE>), set, (int)smem));
+  B200CP_CUDA_OK(launch_kernel(split_pixels_kernel<THREE>, dim3(jobs.first + ceil_div(b.rows, kPxTile)), dim3(32, 8), smem, st, true, jobs,
+                               im));
+  B200CP_LAUNCH_OK("split_pixels_kernel");
   return B200CP_OK;
 }
 
@@ -1128,7 +778,7 @@ struct TcTiles {
   int bn, tiles_m, tiles_n, whole, splits, steps, cut;   // cut: tiles that are cut
   double us;
 };
-// Measured us of a step (twelve instructions: 64 k, three parts 32) and of a unit beside its steps.  128 and 64 columns are not in proportion: the rows of A are read
+// Measured us of a step (twelve instructions: 64 k, MN-major 32) and of a unit beside its steps.  128 and 64 columns are not in proportion: the rows of A are read
 // from shared memory once per instruction, whatever its width.
 double step_us(int bn) { return bn == 256 ? 1.35 : bn == 128 ? 0.95 : 0.7; }
 constexpr double kUnitUs = 2.0;
@@ -1158,46 +808,33 @@ TcTiles tc_tiles(long M, long N, int total, int results, bool mn, const DeviceIn
 }
 size_t partial_floats(const TcTiles& t) { return t.splits > 1 ? (size_t)t.cut * t.splits * t.bn * kBM : 0; }
 
-struct Maps {   // of the operands, and of a gradient's in three parts where it takes either form
-  CUtensorMap a, b, a3, b3;
-};
-template <int BN, int KIND, bool CONV>
-int launch_tile(const SplitGemm& g, int cut, const Maps& m, const DeviceInfo& di, cudaStream_t st) {
+template <int BN, bool MN, bool CONV>
+int launch_tile(const SplitGemm& g, int cut, const CUtensorMap& a, const CUtensorMap& b, const DeviceInfo& di, cudaStream_t st) {
   static std::atomic<int> set[64];
-  const size_t smem = std::max(Tile<BN, KIND>::smem, KIND == kColumnPairs ? Tile<BN, kThree>::smem : 0);
-  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_gemm_kernel<BN, KIND, CONV>), set, (int)smem));
+  B200CP_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(split_gemm_kernel<BN, MN, CONV>), set, (int)Tile<BN, MN>::smem));
   const int pairs = std::min(g.units, di.sm_count / 2);
-  B200CP_CUDA_OK(launch_kernel(split_gemm_kernel<BN, KIND, CONV>, dim3(2 * pairs), dim3(Tile<BN, KIND>::threads), smem, st, true, g, m.a,
-                               m.b, m.a3, m.b3));
+  B200CP_CUDA_OK(launch_kernel(split_gemm_kernel<BN, MN, CONV>, dim3(2 * pairs), dim3(Tile<BN, MN>::threads),
+                               Tile<BN, MN>::smem, st, true, g, a, b));
   B200CP_LAUNCH_OK("split_gemm_kernel");
   if (g.splits > 1) {
-    B200CP_CUDA_OK(launch_kernel(join_tiles_kernel<BN, KIND, CONV>, dim3(cut, BN / kJoinCols), dim3(kBM), 0, st, true, g));
+    B200CP_CUDA_OK(launch_kernel(join_tiles_kernel<BN, MN, CONV>, dim3(cut, BN / kJoinCols), dim3(kBM), 0, st, true, g));
     B200CP_LAUNCH_OK("join_tiles_kernel");
   }
   return B200CP_OK;
 }
 // g has the sizes, exponents and strides of the result; `partial` holds partial_floats(t)
-int run_split_gemm(SplitGemm& g, const TcTiles& t, size_t result, Form form, bool conv, const Maps& m, float* out, float* partial,
-                   const DeviceInfo& di, cudaStream_t st) {
-  g.tiles_m = t.tiles_m; g.tiles_n = t.tiles_n; g.whole = t.whole; g.splits = t.splits;
+int run_split_gemm(SplitGemm g, const TcTiles& t, size_t result, bool mn, bool conv, const CUtensorMap& a, const CUtensorMap& b,
+                   float* out, float* partial, const DeviceInfo& di, cudaStream_t st) {
+  g.tiles_m = t.tiles_m; g.tiles_n = t.tiles_n; g.whole = t.whole; g.splits = t.splits; g.steps = t.steps;
   g.units = t.whole + t.cut * t.splits;
-  if (form == kThree) {
-    g.steps3 = t.steps;
-    g.total3 = g.total;
-  } else {   // (two steps of three parts are one of pairs: no range of theirs is empty)
-    g.steps = t.steps;
-    g.steps3 = 2 * t.steps;
-    g.total3 = ceil_div(g.Kc, kThreeKS);
-  }
-  g.group = form == kThree || (form == kRowPairs && g.total <= kShortSum) ? 2 : 4;
+  g.group = mn || g.total <= kShortSum ? 2 : 4;
   g.result = result;
   g.out = out;
   g.partial = partial;
-#define TILE(BN, KIND, CONV) launch_tile<BN, KIND, CONV>(g, t.cut, m, di, st)
-  if (form == kThree) return t.bn == 256 ? TILE(256, kThree, false) : TILE(128, kThree, false);
-  if (form == kColumnPairs) return t.bn == 256 ? TILE(256, kColumnPairs, false) : TILE(128, kColumnPairs, false);
-  if (conv) return t.bn == 256 ? TILE(256, kRowPairs, true) : t.bn == 128 ? TILE(128, kRowPairs, true) : TILE(64, kRowPairs, true);
-  return t.bn == 256 ? TILE(256, kRowPairs, false) : t.bn == 128 ? TILE(128, kRowPairs, false) : TILE(64, kRowPairs, false);
+#define TILE(BN, MN, CONV) launch_tile<BN, MN, CONV>(g, t.cut, a, b, di, st)
+  if (mn) return t.bn == 256 ? TILE(256, true, false) : TILE(128, true, false);
+  if (conv) return t.bn == 256 ? TILE(256, false, true) : t.bn == 128 ? TILE(128, false, true) : TILE(64, false, true);
+  return t.bn == 256 ? TILE(256, false, false) : t.bn == 128 ? TILE(128, false, false) : TILE(64, false, false);
 #undef TILE
 }
 
@@ -1206,74 +843,10 @@ int run_split_gemm(SplitGemm& g, const TcTiles& t, size_t result, Form form, boo
 // ---- gradient products: both operands have the batch (or pixels) as rows -------------------------------------------------
 // G[M][N] = A^T B with A [K][M], B [K][N]: rows of the kernel's result are the N columns of G, which are contiguous.
 namespace {
-// Which form a gradient asks for, and its tiles.  Pairs halve the product and cost three small launches (the sample, the second split
-// that mostly returns at once, the values outside: 10 us together, and 15 are saved at the line).  4096 x 4096 x 4096: 624 -> 318 us,
-// nine taps of 256 x 256 at 32 x 28 x 28: 153 -> 77; layers a little above the line (1467 -> 1536 features, 7 images of 256 channels 18x29): 0.95 and 1.0.
-constexpr double kPairsFromUs = 30.0;   // of the product of three parts
-struct GradPlan {
-  Form form;
-  TcTiles t;
-  int total;
-};
-GradPlan grad_plan(long K, int M, int N, int results, const DeviceInfo& di) {
-  GradPlan p{kThree, {}, (int)((K + kThreeKS - 1) / kThreeKS)};
-  p.t = tc_tiles(N, M, p.total, results, true, di);
-  if (gemm_tc_mode() == 2 || p.t.us >= kPairsFromUs) {
-    p.form = kColumnPairs;
-    p.total = (int)((K + kKS - 1) / kKS);
-    p.t = tc_tiles(N, M, p.total, results, true, di);
-  }
-  return p;
-}
-// of both operands (K rows of M and of N values), the window with its exponents and samples, and the cut tiles
-size_t grad_floats(const GradPlan& p, size_t K, int M, int N) {
-  return triple_floats(K, ld8(M)) + triple_floats(K, ld8(N)) + align_up(sizeof(Window) / 4 + 2 * ((size_t)M + N) + 16, 64) +
-         partial_floats(p.t);
-}
-struct GradOperands {
-  Planes a, b;   // of N and of M values a row
-  FormOf form;
-};
-GradOperands take_operands(float*& at, const GradPlan& p, size_t K, int M, int N) {
-  GradOperands o{};
-  o.a = take_triple(at, K, ld8(N));
-  o.b = take_triple(at, K, ld8(M));
-  int* w = reinterpret_cast<int*>(at);
-  at += align_up(sizeof(Window) / 4 + 2 * ((size_t)M + N) + 16, 64);
-  o.a.ex = w + sizeof(Window) / 4;
-  o.b.ex = o.a.ex + N;
-  if (p.form == kColumnPairs) o.form = FormOf{reinterpret_cast<Window*>(w), o.b.ex + M, 0, false};
-  return o;
-}
+TcTiles grad_tiles(int K, int M, int N, const DeviceInfo& di) { return tc_tiles(N, M, ceil_div(K, kGradKS), 1, true, di); }
 // planes of an operand with K rows of n values
-int encode_rows(CUtensorMap* map, const Planes& p, int n, size_t K, Form form) {
-  const int planes = form == kThree ? 3 : 2;
-  return encode_planes(map, p.hi, planes, {(size_t)n, K, 1}, {(size_t)p.ld, p.plane}, p.plane,
-                       {64, (unsigned)(form == kThree ? kThreeKS : kKS), 1});
-}
-// g has the shape of the result and of its taps
-int run_grad(SplitGemm& g, const GradPlan& p, const GradOperands& o, int K, int M, int N, float* G, float* partial, OutsideSource src,
-             const DeviceInfo& di, cudaStream_t st) {
-  Maps m;
-  if (int rc = encode_rows(&m.a3, o.a, N, K, kThree)) return rc;
-  if (int rc = encode_rows(&m.b3, o.b, M, K, kThree)) return rc;
-  m.a = m.a3;
-  m.b = m.b3;
-  if (p.form == kColumnPairs) {
-    if (int rc = encode_rows(&m.a, o.a, N, K, kColumnPairs)) return rc;
-    if (int rc = encode_rows(&m.b, o.b, M, K, kColumnPairs)) return rc;
-  }
-  g.M = N; g.N = M; g.total = p.total; g.kc = g.total; g.Kc = K;
-  g.ldm = 1; g.ldn = N;
-  g.ea = o.a.ex; g.eb = o.b.ex; g.win = o.form.win;
-  if (int rc = run_split_gemm(g, p.t, (size_t)M * N, p.form, false, m, G, partial, di, st)) return rc;
-  if (p.form == kColumnPairs) {
-    src.len[0] = N; src.len[1] = M; src.ex0 = o.a.ex; src.K = K;
-    const int taps = p.t.tiles_m * p.t.tiles_n ? (p.t.whole + p.t.cut) / (p.t.tiles_m * p.t.tiles_n) : 1;
-    B200CP_CUDA_OK(launch_kernel(add_outside_kernel, dim3(ceil_div(M, 32), taps, ceil_div(N, 1024)), dim3(256), 0, st, true, g, src));
-    B200CP_LAUNCH_OK("add_outside_kernel");
-  }
-  return B200CP_OK;
+int encode_rows(CUtensorMap* map, const Planes& p, int n, size_t K) {
+  return encode_planes(map, p.hi, 3, {(size_t)n, K, 1}, {(size_t)p.ld, p.plane}, p.plane, {64, kGradKS, 1});
 }
 }  // namespace
 
@@ -1285,19 +858,24 @@ bool gemm_tc_supported(int K, int M, int N) {
 size_t gemm_tc_scratch_floats(int K, int M, int N) {
   DeviceInfo di;
   if (device_info(&di)) di.sm_count = 148;
-  return grad_floats(grad_plan(K, M, N, 1, di), K, M, N);
+  return triple_floats(K, ld8(M)) + triple_floats(K, ld8(N)) + partial_floats(grad_tiles(K, M, N, di));
 }
 
 int gemm_tc_launch(int K, int M, int N, const float* A, const float* B, float* G, float* scratch, cudaStream_t st) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
-  const GradPlan p = grad_plan(K, M, N, 1, di);
   float* at = scratch;
-  const GradOperands o = take_operands(at, p, K, M, N);
-  if (int rc = split_columns(job_of(B, K, 1, N, N, o.a), job_of(A, K, 1, M, M, o.b), o.form, st)) return rc;
+  const Planes pn = take_triple(at, K, ld8(N)), pm = take_triple(at, K, ld8(M));
+  if (int rc = split_columns(job_of(B, K, 1, N, N, pn), job_of(A, K, 1, M, M, pm), st)) return rc;
+  CUtensorMap mn, mm;
+  if (int rc = encode_rows(&mn, pn, N, K)) return rc;
+  if (int rc = encode_rows(&mm, pm, M, K)) return rc;
+  const TcTiles t = grad_tiles(K, M, N, di);
   SplitGemm g{};
+  g.M = N; g.N = M; g.total = ceil_div(K, kGradKS); g.kc = g.total; g.Kc = K;
   g.FW = 1;
-  return run_grad(g, p, o, K, M, N, G, at, OutsideSource{{B, A}}, di, st);
+  g.ldm = 1; g.ldn = N;
+  return run_split_gemm(g, t, (size_t)M * N, true, false, mn, mm, G, at, di, st);
 }
 
 // G[tap][t][c] = sum_{n,h,w} dV[n,t,h,w] * Xpad[n,c,h+y,w+x]: K = the pixels of the padded planes; the taps are as many
@@ -1306,7 +884,7 @@ namespace {
 struct GradConv {
   int PP, taps;
   long K;
-  GradPlan plan;
+  TcTiles t;
 };
 bool grad_conv(GradConv& p, int N, int T, int C, int H, int W, int FH, int FW) {
   const int mode = gemm_tc_mode();
@@ -1317,7 +895,7 @@ bool grad_conv(GradConv& p, int N, int T, int C, int H, int W, int FH, int FW) {
   if (p.K > 0x3fffff00L || (mode == 1 && (p.K < 1024 || T < 128 || C < 128))) return false;
   DeviceInfo di;
   if (device_info(&di)) di.sm_count = 148;
-  p.plan = grad_plan(p.K, T, C, p.taps, di);
+  p.t = tc_tiles(C, T, (int)((p.K + kGradKS - 1) / kGradKS), p.taps, true, di);
   return get_encode_tiled() != nullptr;
 }
 }  // namespace
@@ -1330,7 +908,7 @@ bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW) {
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW) {
   GradConv p;
   if (!grad_conv(p, N, T, C, H, W, FH, FW)) return 0;
-  return grad_floats(p.plan, p.K, T, C);
+  return triple_floats(p.K, ld8(C)) + triple_floats(p.K, ld8(T)) + partial_floats(p.t);
 }
 
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
@@ -1341,14 +919,17 @@ int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const
   if (int rc = device_info(&di)) return rc;
   const int padH = (FH - 1) / 2, padW = (FW - 1) / 2;
   float* at = scratch;
-  const GradOperands o = take_operands(at, p.plan, p.K, T, C);
-  const Images im{N, H, W, padH, padW};
-  if (int rc = split_pixels<true>(job_of(X, (int)p.K, 1, C, 0, o.a), job_of(dV, (int)p.K, 1, T, 0, o.b), im, o.form, st)) return rc;
+  const Planes px = take_triple(at, p.K, ld8(C)), pv = take_triple(at, p.K, ld8(T));
+  if (int rc = split_pixels<true>(job_of(X, (int)p.K, 1, C, 0, px), job_of(dV, (int)p.K, 1, T, 0, pv), Images{N, H, W, padH, padW}, st))
+    return rc;
+  CUtensorMap mx, mv;
+  if (int rc = encode_rows(&mx, px, C, p.K)) return rc;
+  if (int rc = encode_rows(&mv, pv, T, p.K)) return rc;
   SplitGemm g{};
+  g.M = C; g.N = T; g.total = ceil_div((int)p.K, kGradKS); g.kc = g.total; g.Kc = (int)p.K;
   g.FW = FW; g.padH = padH; g.padW = padW; g.Wp = W + padW;
-  OutsideSource src{{X, dV}};
-  src.H = H; src.W = W; src.Wp = W + padW; src.PP = p.PP;
-  return run_grad(g, p.plan, o, (int)p.K, T, C, G, at, src, di, st);
+  g.ldm = 1; g.ldn = C;
+  return run_split_gemm(g, p.t, (size_t)T * C, true, false, mx, mv, G, at, di, st);
 }
 
 // ---- products with the multiplied-out weight --------------------------------------------------------------------------------
@@ -1403,12 +984,10 @@ int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, fl
     if (int rc = split_rows(job_of(W, N, 1, K, kron_weight_ld(K), pw), job_of(X, B, 1, K, K, px), st)) return rc;
   }
   const Planes &pa = d.rows_are_batch ? px : pw, &pb = d.rows_are_batch ? pw : px;
-  Maps m;
-  if (int rc = encode_planes(&m.a, pa.hi, 2, {(size_t)K, 1, pa.rows}, {(size_t)pa.ld, (size_t)pa.ld}, pa.plane, {64, 1, 128})) return rc;
-  if (int rc = encode_planes(&m.b, pb.hi, 2, {(size_t)K, 1, pb.rows}, {(size_t)pb.ld, (size_t)pb.ld}, pb.plane,
+  CUtensorMap ma, mb;
+  if (int rc = encode_planes(&ma, pa.hi, 2, {(size_t)K, 1, pa.rows}, {(size_t)pa.ld, (size_t)pa.ld}, pa.plane, {64, 1, 128})) return rc;
+  if (int rc = encode_planes(&mb, pb.hi, 2, {(size_t)K, 1, pb.rows}, {(size_t)pb.ld, (size_t)pb.ld}, pb.plane,
                              {64, 1, (unsigned)d.t.bn / 2})) return rc;
-  m.a3 = m.a;
-  m.b3 = m.b;
   SplitGemm g{};
   g.M = (int)pa.rows; g.N = (int)pb.rows; g.total = ceil_div(K, kKS); g.kc = g.total; g.Kc = K;
   g.FW = 1;
@@ -1416,7 +995,7 @@ int dense_tc_launch(int B, int K, int N, const float* X, const KronWeight& w, fl
   g.ldm = d.rows_are_batch ? N : 1;
   g.ldn = d.rows_are_batch ? 1 : N;
   g.vec = d.rows_are_batch && N % 4 == 0 && !(reinterpret_cast<uintptr_t>(Y) & 15);
-  return run_split_gemm(g, d.t, 0, kRowPairs, false, m, Y, at, di, st);
+  return run_split_gemm(g, d.t, 0, false, false, ma, mb, Y, at, di, st);
 }
 
 // V[n,t,h,w] = sum_{c,y,x} W[t][y,x][c] X[n,c,h+y-1,w+x-1] (3 x 3): rows are the padded pixels, and a
@@ -1460,20 +1039,18 @@ int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const Kron
   pw.ld = (int)ldk;
   const SplitJob none{};
   if (int rc = split_rows(job_of(Wt, T, kTaps, C, ldw, pw), none, st)) return rc;
-  if (int rc = split_pixels<false>(job_of(X, (int)px, 1, C, 0, pa), none, Images{N, H, W, kPad, kPad}, FormOf{}, st)) return rc;
-  Maps m;
-  if (int rc = encode_planes(&m.a, pa.hi, 2, {(size_t)C, 1, px}, {ldk, ldk}, pa.plane, {64, 1, 128})) return rc;
-  if (int rc = encode_planes(&m.b, pw.hi, 2, {(size_t)C, kTaps, (size_t)T}, {ldk, kTaps * ldk}, pw.plane, {64, 1, (unsigned)t.bn / 2}))
+  if (int rc = split_pixels<false>(job_of(X, (int)px, 1, C, 0, pa), none, Images{N, H, W, kPad, kPad}, st)) return rc;
+  CUtensorMap ma, mb;
+  if (int rc = encode_planes(&ma, pa.hi, 2, {(size_t)C, 1, px}, {ldk, ldk}, pa.plane, {64, 1, 128})) return rc;
+  if (int rc = encode_planes(&mb, pw.hi, 2, {(size_t)C, kTaps, (size_t)T}, {ldk, kTaps * ldk}, pw.plane, {64, 1, (unsigned)t.bn / 2}))
     return rc;
-  m.a3 = m.a;
-  m.b3 = m.b;
   SplitGemm g{};
   g.M = (int)px; g.N = T; g.kc = ceil_div(C, kKS); g.total = kTaps * g.kc; g.Kc = C;
   g.FW = 3; g.padH = g.padW = kPad; g.Wp = Wp;
   g.ea = pa.ex; g.eb = pw.ex;
   g.ldn = (long)H * W;
   g.H = H; g.W = W; g.PP = PP;
-  return run_split_gemm(g, t, 0, kRowPairs, true, m, V, at, di, st);
+  return run_split_gemm(g, t, 0, false, true, ma, mb, V, at, di, st);
 }
 
 // Reads (and clears) the status word of the GEMM kernel; the caller has synchronised the device.

@@ -1,9 +1,9 @@
-"""Factor gradients of the dense and reshaped-CP layers where values of the operands are outside the window in which a pair of fp16
-numbers holds 22 bits: none, a few (added one by one), more than 64 in an operand or more than 3 in its samples (three bf16 parts).
-B200CP_GEMM_TC=2 takes the tensor products at every size.
+"""Factor gradients of the dense and reshaped-CP layers where some values of the operands are far above or below the others, finite or not:
+none, one, tens, thousands of them, up to 29 binades and more apart in a column.  Every value has its own exponent, so all of them
+count with their 24 bits.  B200CP_GEMM_TC=2 takes the tensor products at every size.
 
-Bound: as in test_split_gemm_gpu.py, 1e-6 in the norm (pairs: 2**-22 of a term and 2**-22 for the product of the low parts, sums
-that are cut off by 2e-7, the contraction with the other factors in fp32)."""
+Bound: as in test_split_gemm_gpu.py, 1e-6 in the norm (2**-24 of a term left out, sums that are cut off by 2e-7, the contraction
+with the other factors)."""
 import math
 
 import pytest
@@ -58,7 +58,7 @@ def test_dense(case, few, where):
     first = P.dense_cp_backward(x, dy, *F)[1]
     for got, want in zip(first, ref):
         assert _rel(got, want) < 1e-6
-    for got, again in zip(first, P.dense_cp_backward(x, dy, *F)[1]):   # whatever the order in which the values are found
+    for got, again in zip(first, P.dense_cp_backward(x, dy, *F)[1]):
         assert torch.equal(got, again)
     P.device_status()
 
@@ -110,16 +110,15 @@ def test_values_that_are_not_finite(value, count):
         assert _rel(f[keep], want[keep]) < 1e-6
     A, S = [normal(8, 8, 9) * 0.3 for _ in range(2)], normal(3, 3, 9) * 0.3
     u, dv = normal(2, 64, 9, 11), normal(2, 64, 9, 11)
-    u[0, 3 * 8 + 2, 0, 0] = value   # a corner: the taps beside the image do not meet it
+    u[0, 3 * 8 + 2, 0, 0] = value   # a corner (the taps beside the image meet it too, times a zero of the padding)
     _, dA, dS = P.rcp_conv2d_backward(u, dv, *A, S)
     assert not bool(torch.isfinite(dA[0][3]).any()) and bool(torch.isfinite(dA[0][4:]).all())
-    met = torch.isfinite(dS).all(-1)
-    assert not bool(met[:2, :2].any()) and bool(met[2].all()) and bool(met[:, 2].all())
+    assert not bool(torch.isfinite(dS[:2, :2]).any())
     P.device_status()
 
 
 def test_whole_numbers_stay_exact():
-    """Nothing is cut off where no value has a low part: gradients by order-1 factors of rank 1, which are sums of whole numbers."""
+    """Nothing is cut off where all sums are short: gradients by order-1 factors of rank 1, which are sums of whole numbers."""
     import paralleltnnlayers_b200 as P
     gen = torch.Generator(device="cuda").manual_seed(1)
     integers = lambda *s: torch.randint(-9, 10, s, generator=gen, device="cuda").float()

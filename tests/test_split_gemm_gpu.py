@@ -1,4 +1,4 @@
-"""The tensor-core products of the dense and reshaped-CP layers (scaled fp16 hi / lo operands, in the gradients three bf16 parts or pairs, by the data) at the
+"""The tensor-core products of the dense and reshaped-CP layers (scaled fp16 hi / lo operands, in the gradients three bf16 parts) at the
 edges of their tiles: 256 x 256 / 128 / 64 results, K steps of 64 (gradients: 32) in instructions of 16, odd row lengths, operands off the 16-byte grid, rows of very
 different magnitude.  B200CP_GEMM_TC=2 takes them at every size.
 
