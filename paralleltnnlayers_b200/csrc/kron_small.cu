@@ -305,15 +305,16 @@ __global__ void __launch_bounds__(32 * kRowsEx) kron_exponent_kernel(const __gri
   if (lane == 0) ex[row] = tc::row_exponent(tc::abs_bits(sum * 1.001f), tc::kLeast);
 }
 
-// 128 x 128 entries per CTA and tile on the tensor cores: the half products of 64 ranks at a time as three bf16 parts, K-major, six products
-// of parts (tc_common.cuh), the smallest first; an accumulator has at most 128 ranks.  A CTA keeps A's parts, where R is at most 64,
-// and walks the tiles of B.  A thread splits the 64 entries that it has of one row of the tile into hi and lo; through shared memory, a warp
+// 128 x 128 entries per CTA and tile on the tensor cores: the half products of 64 ranks at a time as three bf16 parts, the first of six bits
+// (split3_short in tc_common.cuh), K-major, and eight products of parts, the smallest first; an accumulator of the largest has 64 ranks, that of
+// the others all.  A CTA keeps A's parts, where R is at most 64, and walks the tiles of B.  A thread splits the 64 entries that it has of one row of the tile into hi and lo; through shared memory, a warp
 // for itself, they are stored as runs of 64 bytes of a row.
 //
 // What bounds it are the phases of a tile one after the other, of which the stores take the longest (a CTA forms, multiplies and stores in 2300,
-// 1300 and 5500 of 9600 cycles; two per SM overlap).  4096 x 4096, times in us at R = 4 / 16 / 32 / 64 / 256: 31 / 31 / 33 / 45 / 166, with 128 x 128
-// tiles of FFMA 33 / 42 / 53 / 84 / 345.  One accumulator for all six products: an error of the layer's output of 6.4e-7 at R = 100, now
-// 1.7e-7, FFMA 2.4e-7 (R = 32: 2.0, 1.75 and 1.93e-7).
+// 1300 and 5500 of 9600 cycles; two per SM overlap).  4096 x 4096, times in us at R = 4 / 32 / 64 / 100 / 256: 33 / 36 / 50 / 106 / 187, with 128 x 128
+// tiles of FFMA 33 / 53 / 84 / - / 345.  Error of a layer's output against float64, of 44 layers of 4 to 256 ranks, over that with FFMA: 0.55 (256
+// ranks) to 1.00 (4).  With first parts of eight bits and six products, 2 to 10 % faster, it was up to 1.08; with one accumulator for
+// all products 3.3 (R = 100).
 __device__ int g_kron_status = 0;   // 0 ok; otherwise (1 << 16) | (block index & 0xffff): a bounded wait ran out
 constexpr int kPT = 128, kKeep = 256, kPart = kPT * 128;   // bytes of a part of a half: 64 ranks
 constexpr size_t kPlanesSmem = 1024 + 6 * kPart;
@@ -370,7 +371,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         for (int i = 0; i < 4; ++i) {
           const int row = warp * 16 + i0 * 2 + i + (lane >> 4) * 4;
           const float u = n > 1 ? x[i][0] * x[i][2] : x[i][0], v = n > 1 ? x[i][1] * x[i][3] : x[i][1];
-          const tc::Bf3 w = tc::split3(r < g.R ? u : 0.f, r + 1 < g.R ? v : 0.f);
+          const tc::Bf3 w = tc::split3_short<true>(r < g.R ? u : 0.f, r + 1 < g.R ? v : 0.f);
           uint8_t* d = dst + row * 128 + ((((k >> 3) ^ row) & 7) << 4) + (k & 7) * 2;
 #pragma unroll
           for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(d + j * kPart) = w.p[j];
@@ -380,9 +381,6 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
   };
   const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
   constexpr uint32_t idesc = tc::make_idesc_bf16(kPT);
-  // Each instruction cuts its sum off, a third of 2^-24 of it in the mean (measured for 4 to 256 ranks).  That is given back, except where the
-  // sum of the small products is nothing: values of eight bits, such as small whole numbers, have exact sums.
-  const float back = (min(g.R, 64) + 15) / 16 * 0.33f / (1 << 24);
   const int srow = ta.row[quarter * 32 + lane];
   bool fine = true;
   int waits = 0;
@@ -403,7 +401,9 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         const uint64_t ad = d0 + (tc::smem_u32(sm) >> 4), bd = ad + (3 * kPart >> 4), p1 = kPart >> 4;
         const int steps = min(4, (g.R - r0 + 15) / 16);
         for (int k = 0; k < steps; ++k) {
-          tc::mma_f16_ss(tmem + kPT, ad + 2 * p1 + k * 2, bd + k * 2, idesc, r0 > 0 || k > 0);
+          tc::mma_f16_ss(tmem + kPT, ad + 2 * p1 + k * 2, bd + p1 + k * 2, idesc, r0 > 0 || k > 0);
+          tc::mma_f16_ss(tmem + kPT, ad + p1 + k * 2, bd + 2 * p1 + k * 2, idesc, true);
+          tc::mma_f16_ss(tmem + kPT, ad + 2 * p1 + k * 2, bd + k * 2, idesc, true);
           tc::mma_f16_ss(tmem + kPT, ad + k * 2, bd + 2 * p1 + k * 2, idesc, true);
           tc::mma_f16_ss(tmem + kPT, ad + p1 + k * 2, bd + p1 + k * 2, idesc, true);
           tc::mma_f16_ss(tmem + kPT, ad + p1 + k * 2, bd + k * 2, idesc, true);
@@ -451,10 +451,10 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         if (t.row[cq] == t.row[cq + 15]) {   // one row of the weight (b's rows do not descend; columns past the end have row 0)
           const float sc = tc::exp2_int(-scale[j0 / 16 + q]);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (v[j] + fmaf(v[j], w[j] != 0.f ? back : 0.f, w[j])) * sc;
+          for (int j = 0; j < 16; ++j) v[j] = (v[j] + w[j]) * sc;
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (v[j] + fmaf(v[j], w[j] != 0.f ? back : 0.f, w[j])) * tc::exp2_int(-ex[srow + t.row[cq + j]]);
+          for (int j = 0; j < 16; ++j) v[j] = (v[j] + w[j]) * tc::exp2_int(-ex[srow + t.row[cq + j]]);
         }
         uint32_t h[8], l[8];
 #pragma unroll
@@ -1117,7 +1117,7 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   return B200CP_OK;
 }
 
-// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 37 us with the exponents, against 86 for the fp32 weight and
+// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 41 us with the exponents, against 86 for the fp32 weight and
 // its split; but 1000 x 1000 at R = 16 21 against 13, 4096 x 64 at R = 64 50 against 20.
 bool kron_planes_takes(int order, const int* idims, const int* odims, int R, int sm_count) {
   double pa = 1, pb = 1;

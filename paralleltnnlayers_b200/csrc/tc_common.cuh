@@ -200,6 +200,28 @@ __device__ __forceinline__ Bf3 split3(float a, float b) {
   out.p[2] = *reinterpret_cast<const uint32_t*>(&l);
   return out;
 }
+// The same with a first part of six bits, rounded: the products of two of them have twelve, so that an instruction adds sixteen without
+// cutting any off unless one is 2^-12 of another (with eight bits 2^-8, and the sums of an instruction are 2e-8 too small in the mean).
+// The three parts still hold all 24 bits; the second is up to 2^-6 of the value, so that its products with the third count too.  (A value
+// that would round to infinity, within 1 % of the largest, is cut off instead and may lose its last bit; without FINITE it becomes one.)
+template <bool FINITE>
+__device__ __forceinline__ Bf3 split3_short(float a, float b) {
+  Bf3 out;
+  const auto first = [](float v) {
+    const uint32_t u = __float_as_uint(v), up = u + 0x20000u;
+    return (FINITE && (up & 0x7f800000u) == 0x7f800000u ? u : up) & 0xfffc0000u;
+  };
+  const uint32_t x = first(a), y = first(b);
+  out.p[0] = __byte_perm(x, y, 0x7632);
+  a -= __uint_as_float(x);
+  b -= __uint_as_float(y);
+  const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+  const float2 f = __bfloat1622float2(m);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(a - f.x, b - f.y);
+  out.p[1] = *reinterpret_cast<const uint32_t*>(&m);
+  out.p[2] = *reinterpret_cast<const uint32_t*>(&l);
+  return out;
+}
 // Instruction descriptor for kind::f16 with K-major operands and fp32 accumulation, M = 128 (one CTA): fp16, or bf16.
 __host__ __device__ constexpr uint32_t make_idesc_f16(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
 __host__ __device__ constexpr uint32_t make_idesc_bf16(uint32_t n) { return make_idesc_f16(n) | (1u << 7) | (1u << 10); }

@@ -70,3 +70,19 @@ def test_convolution_gradient_of_whole_numbers(most, count):
     assert want.abs().max() < 2 ** 24
     dA = P.rcp_conv2d_backward(x, dy, torch.ones(C, T, 1, device="cuda"), S)[1][0]
     assert torch.equal(dA[:, :, 0].double(), want)
+
+
+@pytest.mark.parametrize("R", [9, 64, 100])
+def test_weight_of_whole_numbers(R):
+    """One rank of whole numbers whose product has 22 bits, the other ranks zero: samples with a single 1 read the weight's rows."""
+    import paralleltnnlayers_b200 as P
+    gen = _generator(R)
+    idims, odims, most = (15, 13, 16), (13, 14, 15), (2047, 45, 45)
+    F = [torch.zeros(i, o, R, device="cuda") for i, o in zip(idims, odims)]
+    for f, m in zip(F, most):
+        f[:, :, R // 2] = torch.randint(-m, m + 1, f.shape[:2], generator=gen, device="cuda").float()
+    W = torch.einsum("ai,bj,ck->abcijk", *[f[:, :, R // 2].double() for f in F]).reshape(15 * 13 * 16, 13 * 14 * 15)
+    at = torch.randint(len(W), (40,), generator=gen, device="cuda")
+    x = torch.zeros(40, len(W), device="cuda")
+    x[torch.arange(40, device="cuda"), at] = 1
+    assert torch.equal(P.dense_cp(x, *F).double(), W[at])
