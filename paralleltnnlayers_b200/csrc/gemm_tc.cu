@@ -81,6 +81,7 @@ struct SplitGemm {
   long ldm, ldn;                 // off(m) = m * ldm, or, for the pixels of a convolution:
   int vec;                       // ldn == 1 and 16-byte rows
   int H, W, PP;                  // rows are n * PP + h * Wp + w; off = (n * N * H + h) * W + w, ring pixels have none
+  const float *x, *dv;           // gradient of a filter with a ring: the images [n][M][H][W] and [n][N][H][W] (see pixel_sums)
 };
 
 // ---- PTX of a CTA pair --------------------------------------------------------------------------------------------------
@@ -229,6 +230,41 @@ __device__ __forceinline__ bool row_at(const SplitGemm& g, int m, long* off) {
     *off = ((long)n * g.N * g.H + h) * g.W + w;
   }
   return in;
+}
+
+// A pixel of the ring is zero, and a pixel that is not finite makes NaN of it, in taps that reach beside the image.  So the entries of a gradient
+// that are NaN are formed anew over the pixels that a tap does reach, in fp32: by a warp, whose lanes have a row and `count` columns of the result
+// at `dst`.  An image whose pixel in the middle gives NaN ends it at once (a sample that is NaN throughout).
+__device__ __noinline__ void pixel_sums(const SplitGemm& g, int tap, int m, int n0, int count, float* dst) {
+  const int lane = threadIdx.x & 31, m0 = __shfl_sync(0xffffffffu, m, 0), HW = g.H * g.W;
+  const int y = tap / g.FW - g.padH, x = tap % g.FW - g.padW, h0 = max(0, -y), w0 = max(0, -x);
+  const int hh = g.H - abs(y), ww = g.W - abs(x), images = g.Kc / g.PP, pixels = hh > 0 && ww > 0 ? hh * ww : 0;
+  for (int j = 0; j < count; ++j, dst += g.ldn) {
+    const bool in = m < g.M && n0 + j < g.N;
+    const float have = in ? *dst : 0.f;
+    for (unsigned todo = __ballot_sync(0xffffffffu, have != have); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const auto term = [&](int image, int pixel, float sum) {
+        const int h = h0 + pixel / ww, w = w0 + pixel % ww;
+        return fmaf(g.dv[((size_t)image * g.N + n0 + j) * HW + h * g.W + w], g.x[((size_t)image * g.M + m0 + l) * HW + (h + y) * g.W + w + x], sum);
+      };
+      float v = 0.f;
+      if (pixels)
+        for (int i = lane; i < images; i += 32) v = term(i, (hh >> 1) * ww + (ww >> 1), v);
+      if (__all_sync(0xffffffffu, v == v)) {
+        v = 0.f;
+        for (long i = 0, end = (long)images * pixels; i < end && __all_sync(0xffffffffu, v == v); i += 256)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const long k = i + q * 32 + lane;
+            if (k < end) v = term((int)(k / pixels), (int)(k % pixels), v);
+          }
+      }
+#pragma unroll
+      for (int q = 16; q; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+      if (lane == l) *dst = v;
+    }
+  }
 }
 
 template <int BN, bool MN, bool CONV>
@@ -412,6 +448,7 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
                        : g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn;
       const int* eb = g.eb + n0 + (lane & 15);
       int next = !MN && !cut && n0 + (lane & 15) < N ? *eb : 0;
+      bool nan = false;
 #pragma unroll 1
       for (int j0 = 0; j0 < NC; j0 += 16) {
         float v[16];
@@ -421,6 +458,9 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
         if (!MN) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) nan = nan || v[j] != v[j];
         }
         if (!CONV && g.vec && !cut) {   // 16-byte stores along a row
 #pragma unroll
@@ -436,6 +476,8 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) arrive_cluster(leader_addr(accfreeb + buf * 8));
+      if (MN && g.x && !cut && __any_sync(0xffffffffu, nan))
+        pixel_sums(g, t.tap, m, n0, NC, g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn);
     }
   }
   tc_fence_before_sync();
@@ -456,13 +498,15 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
 // The sums of a cut tile, in the order of K, and the exponents.  grid (cut tiles, BN / 8), one row per
 // thread: enough CTAs to keep the L2 busy (34 tiles cut in two: 24 us with 32 columns per CTA, 6 with 8).
 constexpr int kJoinCols = 8;
+// (Eight CTAs per SM: without the bound pixel_sums takes 80 registers of its callers.)
 template <int BN, bool MN, bool CONV>
-__global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__ SplitGemm g) {
+__global__ void __launch_bounds__(kBM, 8) join_tiles_kernel(const __grid_constant__ SplitGemm g) {
   grid_dependency_wait();
   const UnitAt t = unit_at<BN, MN>(g, g.whole + blockIdx.x * g.splits);
   const int m = t.m0 + threadIdx.x;
   long off;
-  if (!row_at<CONV>(g, m, &off)) return;
+  const bool in = row_at<CONV>(g, m, &off);
+  if (!MN && !in) return;
   const int e = MN ? 0 : CONV ? kRowShift : g.ea[m];
   const int n0 = t.n0 + blockIdx.y * kJoinCols;
   const float* src = g.partial + ((size_t)blockIdx.x * g.splits * BN + blockIdx.y * kJoinCols) * kBM + threadIdx.x;
@@ -473,9 +517,13 @@ __global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__
   for (int q = 1; q < g.splits; ++q)
 #pragma unroll
     for (int j = 0; j < kJoinCols; ++j) v[j] += __ldcs(src + ((size_t)q * BN + j) * kBM);
+  bool nan = false;
 #pragma unroll
-  for (int j = 0; j < kJoinCols; ++j)
-    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
+  for (int j = 0; j < kJoinCols; ++j) {
+    if (in && n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
+    nan = nan || v[j] != v[j];
+  }
+  if (MN && g.x && __any_sync(0xffffffffu, nan)) pixel_sums(g, t.tap, m, n0, kJoinCols, dst + (long)n0 * g.ldn);
 }
 
 // ---- operand planes -----------------------------------------------------------------------------------------------------
@@ -928,6 +976,8 @@ int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const
   SplitGemm g{};
   g.M = C; g.N = T; g.total = ceil_div((int)p.K, kGradKS); g.kc = g.total; g.Kc = (int)p.K;
   g.FW = FW; g.padH = padH; g.padW = padW; g.Wp = W + padW;
+  g.H = H; g.W = W; g.PP = p.PP;
+  if (padH || padW) { g.x = X; g.dv = dV; }
   g.ldm = 1; g.ldn = C;
   return run_split_gemm(g, p.t, (size_t)T * C, true, false, mx, mv, G, at, di, st);
 }

@@ -58,7 +58,7 @@ def test_dense(case, few, where):
     first = P.dense_cp_backward(x, dy, *F)[1]
     for got, want in zip(first, ref):
         assert _rel(got, want) < 1e-6
-    for got, again in zip(first, P.dense_cp_backward(x, dy, *F)[1]):
+    for got, again in zip(first, P.dense_cp_backward(x, dy, *F)[1]):   # whatever the order in which the values are found
         assert torch.equal(got, again)
     P.device_status()
 
@@ -110,10 +110,11 @@ def test_values_that_are_not_finite(value, count):
         assert _rel(f[keep], want[keep]) < 1e-6
     A, S = [normal(8, 8, 9) * 0.3 for _ in range(2)], normal(3, 3, 9) * 0.3
     u, dv = normal(2, 64, 9, 11), normal(2, 64, 9, 11)
-    u[0, 3 * 8 + 2, 0, 0] = value   # a corner (the taps beside the image meet it too, times a zero of the padding)
+    u[0, 3 * 8 + 2, 0, 0] = value   # a corner: the taps beside the image do not meet it
     _, dA, dS = P.rcp_conv2d_backward(u, dv, *A, S)
     assert not bool(torch.isfinite(dA[0][3]).any()) and bool(torch.isfinite(dA[0][4:]).all())
-    assert not bool(torch.isfinite(dS[:2, :2]).any())
+    met = torch.isfinite(dS).all(-1)
+    assert not bool(met[:2, :2].any()) and bool(met[2].all()) and bool(met[:, 2].all())
     P.device_status()
 
 
