@@ -81,7 +81,9 @@ struct SplitGemm {
   long ldm, ldn;                 // off(m) = m * ldm, or, for the pixels of a convolution:
   int vec;                       // ldn == 1 and 16-byte rows
   int H, W, PP;                  // rows are n * PP + h * Wp + w; off = (n * N * H + h) * W + w, ring pixels have none
-  const float *x, *dv;           // gradient of a filter with a ring: the images [n][M][H][W] and [n][N][H][W] (see pixel_sums)
+  // Gradient of a filter with a ring: the images [n][M][H][W] and [n][N][H][W], and a word per 32 pixels of each (see edge_pixels)
+  const float *x, *dv;
+  const int* dropped;
 };
 
 // ---- PTX of a CTA pair --------------------------------------------------------------------------------------------------
@@ -232,39 +234,52 @@ __device__ __forceinline__ bool row_at(const SplitGemm& g, int m, long* off) {
   return in;
 }
 
-// A pixel of the ring is zero, and a pixel that is not finite makes NaN of it, in taps that reach beside the image.  So the entries of a gradient
-// that are NaN are formed anew over the pixels that a tap does reach, in fp32: by a warp, whose lanes have a row and `count` columns of the result
-// at `dst`.  An image whose pixel in the middle gives NaN ends it at once (a sample that is NaN throughout).
-__device__ __noinline__ void pixel_sums(const SplitGemm& g, int tap, int m, int n0, int count, float* dst) {
-  const int lane = threadIdx.x & 31, m0 = __shfl_sync(0xffffffffu, m, 0), HW = g.H * g.W;
-  const int y = tap / g.FW - g.padH, x = tap % g.FW - g.padW, h0 = max(0, -y), w0 = max(0, -x);
-  const int hh = g.H - abs(y), ww = g.W - abs(x), images = g.Kc / g.PP, pixels = hh > 0 && ww > 0 ? hh * ww : 0;
-  for (int j = 0; j < count; ++j, dst += g.ldn) {
-    const bool in = m < g.M && n0 + j < g.N;
-    const float have = in ? *dst : 0.f;
-    for (unsigned todo = __ballot_sync(0xffffffffu, have != have); todo; todo &= todo - 1) {
-      const int l = __ffs(todo) - 1;
-      const auto term = [&](int image, int pixel, float sum) {
-        const int h = h0 + pixel / ww, w = w0 + pixel % ww;
-        return fmaf(g.dv[((size_t)image * g.N + n0 + j) * HW + h * g.W + w], g.x[((size_t)image * g.M + m0 + l) * HW + (h + y) * g.W + w + x], sum);
-      };
-      float v = 0.f;
-      if (pixels)
-        for (int i = lane; i < images; i += 32) v = term(i, (hh >> 1) * ww + (ww >> 1), v);
-      if (__all_sync(0xffffffffu, v == v)) {
-        v = 0.f;
-        for (long i = 0, end = (long)images * pixels; i < end && __all_sync(0xffffffffu, v == v); i += 256)
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const long k = i + q * 32 + lane;
-            if (k < end) v = term((int)(k / pixels), (int)(k % pixels), v);
+// A pixel of the ring is zero, and one at the edge of an image that is not finite would make NaN of it, in the taps that reach beside the image
+// there.  So split_pixels_kernel takes such pixels for zero and says which 32 (a step) hold one, and here those of a unit's steps make NaN of the sums
+// that do meet them (as the products of their parts would): a read-out warp for its own rows and columns.  Finite images pay for a look at a
+// word per step; in 32 of 256 channels 28x28 a corner of one, of all channels, costs 13 us, and a row of every image 67.
+template <int BN>
+__device__ __noinline__ void edge_pixels(const SplitGemm& g, int unit) {
+  constexpr int count = Tile<BN, true>::cols;
+  const UnitAt u = unit_at<BN, true>(g, unit);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = ((warp - 2) >> 2) * count, HW = g.H * g.W, padH = g.padH, padW = g.padW;
+  const int in_tile = (int)cluster_rank() * 128 + (warp & 3) * 32 + lane, m = u.m0 + in_tile, n0 = u.n0 + c0;
+  const bool cut = unit >= g.whole && g.splits > 1;
+  const long ldn = cut ? kBM : g.ldn;
+  float* dst = cut ? g.partial + ((size_t)(unit - g.whole) * BN + c0) * kBM + in_tile : g.out + u.tap * g.result + m + n0 * ldn;   // (ldm is 1)
+  const int y = u.tap / g.FW - padH, x = u.tap % g.FW - padW, steps = (g.Kc + kGradKS - 1) / kGradKS, end = u.first + u.nsteps;
+  bool row = false;
+#pragma unroll 8
+  for (int c = 0; c < count; ++c) row |= m < g.M && n0 + c < g.N && dst[c * ldn] == dst[c * ldn];
+  if (!__any_sync(0xffffffffu, row)) return;   // NaN already: whole images of it
+  row = false;
+  uint64_t cols = 0;
+#pragma unroll 1
+  for (int grad = 0; grad < 2; ++grad) {
+    const int dy = grad ? y : -y, dx = grad ? x : -x;   // a pixel of x at (h, w) is met by one of dv at (h - y, w - x)
+    for (int k0 = u.first; k0 < end; k0 += 32)
+      for (unsigned todo = __ballot_sync(0xffffffffu, k0 + lane < end && g.dropped[grad * steps + min(k0 + lane, end - 1)]); todo; todo &= todo - 1) {
+        const int first = (k0 + __ffs(todo) - 1) * kGradKS;
+#pragma unroll 4
+        for (int i = 0; i < kGradKS; ++i) {
+          const int n = (first + i) / g.PP, q = first + i - n * g.PP, h = q / g.Wp, w = q - h * g.Wp;
+          if (first + i >= g.Kc || h >= g.H || w >= g.W || h + dy < 0 || h + dy >= g.H || w + dx < 0 || w + dx >= g.W) continue;
+          if (h >= padH && h < g.H - padH && w >= padW && w < g.W - padW) continue;
+          const size_t at = (size_t)h * g.W + w;
+          if (!grad) {
+            row = row || (m < g.M && abs_bits(g.x[((size_t)n * g.M + m) * HW + at]) >= 0x7f800000u);
+          } else {
+            for (int c = 0; c < count; c += 32) {
+              const bool in = c + lane < count && n0 + c + lane < g.N;
+              cols |= (uint64_t)__ballot_sync(0xffffffffu, in && abs_bits(g.dv[((size_t)n * g.N + (in ? n0 + c + lane : 0)) * HW + at]) >= 0x7f800000u) << c;
+            }
           }
+        }
       }
-#pragma unroll
-      for (int q = 16; q; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
-      if (lane == l) *dst = v;
-    }
   }
+  if (m >= g.M) return;
+  for (int c = 0; c < count && n0 + c < g.N; ++c)
+    if (row || (cols >> c & 1)) dst[c * ldn] = __int_as_float(0x7fffffff);
 }
 
 template <int BN, bool MN, bool CONV>
@@ -282,6 +297,7 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
   uint64_t* accfree = accfull + 4;       // [depth] the leader's: read out by the warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* edges = abort_flag + 1;   // pixels at the edges were taken for zero
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -296,6 +312,7 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       mbar_init(&accfree[i], 2 * T::readers);
     }
     *abort_flag = 0;
+    *edges = 0;
     fence_barrier_init();
     tma_prefetch_desc(&mapA);
     tma_prefetch_desc(&mapB);
@@ -394,6 +411,12 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
     constexpr int NC = T::cols;
     const int qd = warp & 3, c0 = ((warp - 2) >> 2) * NC;   // the TMEM lane quarter this warp may read, and its columns
     const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + c0;
+    if (MN && g.dropped) {   // while the first stages are on their way
+      int any = 0;
+      for (int i = tid - 64, end = 2 * ((g.Kc + kGradKS - 1) / kGradKS); i < end; i += 32 * T::readers) any |= g.dropped[i];
+      if (any) *edges = 1;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * T::readers) : "memory");
+    }
     int gi = 0;
     bool ok = true;
     for (int unit = pair; unit < g.units && ok; unit += npairs) {
@@ -448,7 +471,6 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
                        : g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn;
       const int* eb = g.eb + n0 + (lane & 15);
       int next = !MN && !cut && n0 + (lane & 15) < N ? *eb : 0;
-      bool nan = false;
 #pragma unroll 1
       for (int j0 = 0; j0 < NC; j0 += 16) {
         float v[16];
@@ -458,9 +480,6 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
         if (!MN) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = scale_by(v[j], e + __shfl_sync(0xffffffffu, ebv, j));
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) nan = nan || v[j] != v[j];
         }
         if (!CONV && g.vec && !cut) {   // 16-byte stores along a row
 #pragma unroll
@@ -476,8 +495,7 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) arrive_cluster(leader_addr(accfreeb + buf * 8));
-      if (MN && g.x && !cut && __any_sync(0xffffffffu, nan))
-        pixel_sums(g, t.tap, m, n0, NC, g.out + (size_t)t.tap * g.result + off + (long)n0 * ldn);
+      if (MN && *edges) edge_pixels<BN>(g, unit);
     }
   }
   tc_fence_before_sync();
@@ -498,15 +516,13 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
 // The sums of a cut tile, in the order of K, and the exponents.  grid (cut tiles, BN / 8), one row per
 // thread: enough CTAs to keep the L2 busy (34 tiles cut in two: 24 us with 32 columns per CTA, 6 with 8).
 constexpr int kJoinCols = 8;
-// (Eight CTAs per SM: without the bound pixel_sums takes 80 registers of its callers.)
 template <int BN, bool MN, bool CONV>
-__global__ void __launch_bounds__(kBM, 8) join_tiles_kernel(const __grid_constant__ SplitGemm g) {
+__global__ void __launch_bounds__(kBM) join_tiles_kernel(const __grid_constant__ SplitGemm g) {
   grid_dependency_wait();
   const UnitAt t = unit_at<BN, MN>(g, g.whole + blockIdx.x * g.splits);
   const int m = t.m0 + threadIdx.x;
   long off;
-  const bool in = row_at<CONV>(g, m, &off);
-  if (!MN && !in) return;
+  if (!row_at<CONV>(g, m, &off)) return;
   const int e = MN ? 0 : CONV ? kRowShift : g.ea[m];
   const int n0 = t.n0 + blockIdx.y * kJoinCols;
   const float* src = g.partial + ((size_t)blockIdx.x * g.splits * BN + blockIdx.y * kJoinCols) * kBM + threadIdx.x;
@@ -517,13 +533,9 @@ __global__ void __launch_bounds__(kBM, 8) join_tiles_kernel(const __grid_constan
   for (int q = 1; q < g.splits; ++q)
 #pragma unroll
     for (int j = 0; j < kJoinCols; ++j) v[j] += __ldcs(src + ((size_t)q * BN + j) * kBM);
-  bool nan = false;
 #pragma unroll
-  for (int j = 0; j < kJoinCols; ++j) {
-    if (in && n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
-    nan = nan || v[j] != v[j];
-  }
-  if (MN && g.x && __any_sync(0xffffffffu, nan)) pixel_sums(g, t.tap, m, n0, kJoinCols, dst + (long)n0 * g.ldn);
+  for (int j = 0; j < kJoinCols; ++j)
+    if (n0 + j < g.N) dst[(long)(n0 + j) * g.ldn] = MN ? v[j] : scale_by(v[j], e + g.eb[n0 + j]);
 }
 
 // ---- operand planes -----------------------------------------------------------------------------------------------------
@@ -656,11 +668,13 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const __grid_constan
 // (THREE) bf16 planes.  In a job: len = channels, rows = N (H + padH) (W + padW).
 struct Images {
   int N, H, W, padH, padW;
+  int* dropped;   // THREE: a word per 32 pixels of both operands (null: the filter has no ring)
 };
 // What bounds it is memory latency, so a thread has the loads of 32 channels of its pixel in flight and four CTAs share an SM; four channels of a
 // pixel are together in shared memory (16-byte accesses, eight bytes of a plane per store).  32 images of 256 channels 28x28: pairs by pixel 14.9
 // -> 11.6 us (with 16 loads in flight and channels apart; three or four CTAs alike, five 12.4).
-constexpr int kPxTile = 32, kPxPitch = kPxTile + 1;   // of four channels
+constexpr int kPxTile = kGradKS, kPxPitch = kPxTile + 1;   // pitch: of four channels; a tile is a step of the gradient (see edge_pixels)
+static_assert(kPxTile == 32, "");   // a pixel per lane
 template <bool THREE>
 __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_constant__ SplitJobs jobs, const Images im) {
   extern __shared__ float px_smem[];
@@ -696,9 +710,21 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
           m = max(m, max(max(abs_bits(v[j][0]), abs_bits(v[j][1])), max(abs_bits(v[j][2]), abs_bits(v[j][3]))));
         }
     }
-    red[ty][tx] = m;
+    if (THREE) {
+      const bool edge = h < im.padH || h >= im.H - im.padH || w < im.padW || w >= im.W - im.padW, drop = im.dropped && edge && m >= 0x7f800000u;
+      if (drop)   // (see edge_pixels)
+        for (int k = ty; k < quads; k += 8) {
+          float4& v = tile[k * kPxPitch + tx];
+          const auto finite = [](float f) { return abs_bits(f) < 0x7f800000u ? f : 0.f; };
+          v = make_float4(finite(v.x), finite(v.y), finite(v.z), finite(v.w));
+        }
+      const int any = __syncthreads_or(drop);
+      if (im.dropped && tid == 0) im.dropped[blockIdx.x] = any;
+    } else {
+      red[ty][tx] = m;
+      __syncthreads();
+    }
   }
-  __syncthreads();
   if (!THREE) {
     if (tid < kPxTile) {
       unsigned m = red[0][tid];
@@ -764,6 +790,7 @@ struct Planes {
   int ld;
 };
 size_t pair_floats(size_t rows, size_t ld, size_t exps) { return align_up(rows * ld, 64) + align_up(exps, 64); }
+size_t dropped_words(size_t pixels) { return align_up(2 * ((pixels + kPxTile - 1) / kPxTile), 64); }
 size_t triple_floats(size_t rows, size_t ld) { return align_up(rows * ld / 2 * 3, 64); }   // (ld is even)
 Planes take_pair(float*& at, size_t rows, size_t ld, size_t exps) {
   Planes p{reinterpret_cast<uint16_t*>(at), nullptr, rows, rows * ld, (int)ld};
@@ -956,7 +983,7 @@ bool conv_gemm_tc_supported(int N, int T, int C, int H, int W, int FH, int FW) {
 size_t conv_gemm_tc_scratch_floats(int N, int T, int C, int H, int W, int FH, int FW) {
   GradConv p;
   if (!grad_conv(p, N, T, C, H, W, FH, FW)) return 0;
-  return triple_floats(p.K, ld8(C)) + triple_floats(p.K, ld8(T)) + partial_floats(p.t);
+  return triple_floats(p.K, ld8(C)) + triple_floats(p.K, ld8(T)) + dropped_words(p.K) + partial_floats(p.t);
 }
 
 int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const float* dV, const float* X, float* G,
@@ -968,7 +995,9 @@ int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const
   const int padH = (FH - 1) / 2, padW = (FW - 1) / 2;
   float* at = scratch;
   const Planes px = take_triple(at, p.K, ld8(C)), pv = take_triple(at, p.K, ld8(T));
-  if (int rc = split_pixels<true>(job_of(X, (int)p.K, 1, C, 0, px), job_of(dV, (int)p.K, 1, T, 0, pv), Images{N, H, W, padH, padW}, st))
+  int* dropped = padH || padW ? reinterpret_cast<int*>(at) : nullptr;
+  at += dropped_words(p.K);
+  if (int rc = split_pixels<true>(job_of(X, (int)p.K, 1, C, 0, px), job_of(dV, (int)p.K, 1, T, 0, pv), Images{N, H, W, padH, padW, dropped}, st))
     return rc;
   CUtensorMap mx, mv;
   if (int rc = encode_rows(&mx, px, C, p.K)) return rc;
@@ -977,7 +1006,7 @@ int conv_gemm_tc_launch(int N, int T, int C, int H, int W, int FH, int FW, const
   g.M = C; g.N = T; g.total = ceil_div((int)p.K, kGradKS); g.kc = g.total; g.Kc = (int)p.K;
   g.FW = FW; g.padH = padH; g.padW = padW; g.Wp = W + padW;
   g.H = H; g.W = W; g.PP = p.PP;
-  if (padH || padW) { g.x = X; g.dv = dV; }
+  g.x = X; g.dv = dV; g.dropped = dropped;
   g.ldm = 1; g.ldn = C;
   return run_split_gemm(g, p.t, (size_t)T * C, true, false, mx, mv, G, at, di, st);
 }
@@ -1089,7 +1118,7 @@ int conv_tc_launch(int N, int C, int T, int H, int W, const float* X, const Kron
   pw.ld = (int)ldk;
   const SplitJob none{};
   if (int rc = split_rows(job_of(Wt, T, kTaps, C, ldw, pw), none, st)) return rc;
-  if (int rc = split_pixels<false>(job_of(X, (int)px, 1, C, 0, pa), none, Images{N, H, W, kPad, kPad}, st)) return rc;
+  if (int rc = split_pixels<false>(job_of(X, (int)px, 1, C, 0, pa), none, Images{N, H, W, kPad, kPad, nullptr}, st)) return rc;
   CUtensorMap ma, mb;
   if (int rc = encode_planes(&ma, pa.hi, 2, {(size_t)C, 1, px}, {ldk, ldk}, pa.plane, {64, 1, 128})) return rc;
   if (int rc = encode_planes(&mb, pw.hi, 2, {(size_t)C, kTaps, (size_t)T}, {ldk, kTaps * ldk}, pw.plane, {64, 1, (unsigned)t.bn / 2}))
