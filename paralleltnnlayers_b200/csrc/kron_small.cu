@@ -12,6 +12,7 @@
 // All exact fp32 (FFMA); large weights for the tensor-core product come from kron_planes_kernel.  The product kernels are programmatic dependents of the weight kernel: their CTAs are resident
 // and past their set-up when the weight is done.  Formulas: Kernels/rcp_fused_nchw.cu:4-77, Kernels/dense_cp.cu:4-46.
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 
@@ -311,17 +312,43 @@ __global__ void __launch_bounds__(32 * kRowsEx) kron_exponent_kernel(const __gri
 // for itself, they are stored as runs of 64 bytes of a row.
 //
 // What bounds it are the phases of a tile one after the other, of which the stores take the longest (a CTA forms, multiplies and stores in 2300,
-// 1300 and 5500 of 9600 cycles; two per SM overlap).  4096 x 4096, times in us at R = 4 / 32 / 64 / 100 / 256: 33 / 36 / 50 / 106 / 187, with 128 x 128
+// 1300 and 5500 of 9600 cycles; two per SM overlap).  4096 x 4096, times in us at R = 4 / 32 / 64 / 100 / 256: 33 / 37 / 51 / 107 / 193, with 128 x 128
 // tiles of FFMA 33 / 53 / 84 / - / 345.  Error of a layer's output against float64, of 44 layers of 4 to 256 ranks, over that with FFMA: 0.55 (256
 // ranks) to 1.00 (4).  With first parts of eight bits and six products, 2 to 10 % faster, it was up to 1.08; with one accumulator for
 // all products 3.3 (R = 100).
+// A part is a bf16 number, whose subnormals begin at 2^-126 like those of fp32, and the third is 2^-16 of the value: so the half products are lifted by
+// 2^17 and keep their 24 bits down to the smallest normal number.  Where one of a tile is above 2^43, what overflows for that (half products above
+// 2^111, weights above 2^94) is formed anew in fp32 (form_entries).  Without the look at the largest and the lift: 0.5 us less at R = 32.
 __device__ int g_kron_status = 0;   // 0 ok; otherwise (1 << 16) | (block index & 0xffff): a bounded wait ran out
 constexpr int kPT = 128, kKeep = 256, kPart = kPT * 128;   // bytes of a part of a half: 64 ranks
+constexpr float kDrop = 1.f / (tc::kLift * tc::kLift), kLarge = 5.76460752303423488e17f;   // 2^59: no sum of 256 products of less overflows
 constexpr size_t kPlanesSmem = 1024 + 6 * kPart;
 
 struct KronTile {   // entries of a half in a tile
   int e[kPT][2], o[kPT], row[kPT];   // entry of each mode (in ranks), offset and row in the weight (both add up)
 };
+
+// the entries of row a of a tile in the runs of 16 columns from c0 on that `which` has bits of; none where a half product of the row is infinite or NaN
+__device__ __noinline__ void form_entries(const KronGeom& g, const KronTile& ta, const KronTile& tb, int a, int c0, int count, unsigned which, int pitch,
+                                          const int* ex, __half* hi, size_t plane) {
+  const float *a0 = g.A[0].F + ta.e[a][0], *a1 = g.A[g.nA - 1].F + ta.e[a][g.nA - 1];
+  const auto of_row = [&](int r) { return g.nA > 1 ? a0[r] * a1[r] : a0[r]; };
+  float none = 0.f;
+#pragma unroll 8
+  for (int r = 0; r < g.R; ++r) none = fmaf(of_row(r), 0.f, none);
+  if (none != 0.f) return;
+  for (int c = 0; c < count; ++c) {
+    if (!(which >> (c >> 4) & 1)) continue;
+    const float *b0 = g.B[0].F + tb.e[c0 + c][0], *b1 = g.B[g.nB - 1].F + tb.e[c0 + c][g.nB - 1];
+    float v = 0.f;
+    for (int r = 0; r < g.R && v == v; ++r) v = fmaf(of_row(r), g.nB > 1 ? b0[r] * b1[r] : b0[r], v);
+    const int o = ta.o[a] + tb.o[c0 + c];
+    v *= tc::exp2_int(-ex[o / pitch]);
+    const __half h = __float2half_rn(v);
+    hi[o] = h;
+    hi[plane + o] = __float2half_rn(v - __half2float(h));
+  }
+}
 
 template <bool MANY>   // more than 64 ranks
 __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_constant__ KronGeom g, int pitch, int btiles,
@@ -354,7 +381,8 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
   const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)(quarter * 32) << 16);
   // the half products of ranks r0 .. r0 + 63 as parts, [row][rank]; two ranks of a row per lane, rows four apart in the halves of a warp
   // (16 bytes of a row and of the one four on are in different banks)
-  auto form = [&](const KronMode* m, int n, const KronTile& t, int r0, uint8_t* dst) {
+  auto form = [&](const KronMode* m, int n, const KronTile& t, int r0, uint8_t* dst) {   // returns the largest, NaN apart
+    float most = 0.f;
     const float *f0 = m[0].F, *f1 = m[n - 1].F;
     for (int h = 0; h < 2 && r0 + h * 32 < g.R; ++h) {
       const int k = h * 32 + (lane & 15) * 2, r = r0 + k, c0 = min(r, g.R - 1), c1 = min(r + 1, g.R - 1);
@@ -370,7 +398,8 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int row = warp * 16 + i0 * 2 + i + (lane >> 4) * 4;
-          const float u = n > 1 ? x[i][0] * x[i][2] : x[i][0], v = n > 1 ? x[i][1] * x[i][3] : x[i][1];
+          const float p = x[i][0] * tc::kLift, q = x[i][1] * tc::kLift, u = n > 1 ? p * x[i][2] : p, v = n > 1 ? q * x[i][3] : q;
+          most = tc::most_of(most, u, v);
           const tc::Bf3 w = tc::split3_short<true>(r < g.R ? u : 0.f, r + 1 < g.R ? v : 0.f);
           uint8_t* d = dst + row * 128 + ((((k >> 3) ^ row) & 7) << 4) + (k & 7) * 2;
 #pragma unroll
@@ -378,24 +407,27 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         }
       }
     }
+    return most;
   };
   const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
   constexpr uint32_t idesc = tc::make_idesc_bf16(kPT);
   const int srow = ta.row[quarter * 32 + lane];
   bool fine = true;
   int waits = 0;
-  if (!MANY) form(g.A, g.nA, ta, 0, sm);
+  float most_a = 0.f;
+  if (!MANY) most_a = form(g.A, g.nA, ta, 0, sm);
   int turn = 0;
   for (int bt = blockIdx.x; bt < btiles; bt += gridDim.x, turn ^= 1) {
     const int b0 = bt * kPT;
     const KronTile& t = tb[turn];
     float tot[MANY ? 64 : 1];
+    bool large = false;
     int scale[4];   // exponents of this lane's row in the first column of each 16
     for (int r0 = 0; r0 < (MANY ? g.R : 1); r0 += 64) {
-      if (MANY) form(g.A, g.nA, ta, r0, sm);
-      form(g.B, g.nB, t, r0, sm + 3 * kPart);
+      if (MANY) most_a = form(g.A, g.nA, ta, r0, sm);
+      const float most = fmaxf(most_a, form(g.B, g.nB, t, r0, sm + 3 * kPart));
       tc::fence_proxy_async();
-      __syncthreads();
+      large = __syncthreads_or(most >= kLarge) || (r0 && large);
       if (warp == 0 && tc::elect_one()) {
         tc::tc_fence_after_sync();
         const uint64_t ad = d0 + (tc::smem_u32(sm) >> 4), bd = ad + (3 * kPart >> 4), p1 = kPart >> 4;
@@ -434,6 +466,7 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
       }
     }
     uint8_t* stage = sm + 3 * kPart + warp * 4096;   // [hi | lo][32 rows][64 bytes], B is used up
+    unsigned bad = 0;   // runs of 16 columns with an entry that is not finite
 #pragma unroll
     for (int j0 = 0; j0 < 64; j0 += 32) {
       const int c0 = grp * 64 + j0;
@@ -448,13 +481,21 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
           tc::tmem_ld16(lanes + cq, v);
         }
         tc::tmem_ld16(lanes + kPT + cq, w);
-        if (t.row[cq] == t.row[cq + 15]) {   // one row of the weight (b's rows do not descend; columns past the end have row 0)
-          const float sc = tc::exp2_int(-scale[j0 / 16 + q]);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (v[j] + w[j]) * sc;
+        for (int j = 0; j < 16; ++j) v[j] += w[j];
+        if (large) {
+          float most = 0.f;
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) most = tc::most_nan(most, v[j], v[j + 1]);
+          if (!(most <= FLT_MAX)) bad |= 1u << (j0 / 16 + q);
+        }
+        if (t.row[cq] == t.row[cq + 15]) {   // one row of the weight (b's rows do not descend; columns past the end have row 0)
+          const float sc = kDrop * tc::exp2_int(-scale[j0 / 16 + q]);   // (2^-148 at least)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] *= sc;
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (v[j] + w[j]) * tc::exp2_int(-ex[srow + t.row[cq + j]]);
+          for (int j = 0; j < 16; ++j) v[j] *= kDrop * tc::exp2_int(-ex[srow + t.row[cq + j]]);
         }
         uint32_t h[8], l[8];
 #pragma unroll
@@ -513,8 +554,10 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
           }
         }
       }
-      __syncwarp();
+      __syncwarp();   // (an entry formed anew replaces what another lane has stored)
     }
+    if (bad && a0 + quarter * 32 + lane < PA)
+      form_entries(g, ta, t, quarter * 32 + lane, grp * 64, min(64, PB - b0 - grp * 64), bad, pitch, ex, hi, plane);
     tc::tc_fence_before_sync();
     __syncthreads();   // the accumulators and B are free, the table of the next tile written
   }

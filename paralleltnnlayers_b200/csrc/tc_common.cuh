@@ -178,6 +178,17 @@ __device__ __forceinline__ int row_exponent(unsigned bits, int least) {
 }
 constexpr int kLeast = -126, kLeastConv = -100;   // 2^-e and (convolutions) 2^(e - 24) stay normal numbers
 
+// the largest and the least of three magnitudes, one instruction; a NaN is neither, but the largest with most_nan
+#define B200CP_MAGNITUDES(name, op)                                                                                            \
+  __device__ __forceinline__ float name(float a, float b, float c) {                                                           \
+    float d;                                                                                                                   \
+    asm("{\n.reg .f32 x, y;\nabs.f32 x, %2;\nabs.f32 y, %3;\n" op ".f32 %0, %1, x, y;\n}" : "=f"(d) : "f"(a), "f"(b), "f"(c)); \
+    return d;                                                                                                                  \
+  }
+B200CP_MAGNITUDES(most_of, "max")
+B200CP_MAGNITUDES(most_nan, "max.NaN")
+B200CP_MAGNITUDES(least_of, "min")
+#undef B200CP_MAGNITUDES
 __device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 constexpr int kRowShift = 24;   // of totals that take a power of two per step: see SplitGemm::ea
 // ---- three bf16 parts -------------------------------------------------------------------------------------------------
@@ -187,6 +198,7 @@ constexpr int kRowShift = 24;   // of totals that take a power of two per step: 
 struct Bf3 {
   uint32_t p[3];
 };
+constexpr float kLift = 131072.f;   // 2^17: values times it have normal parts wherever they are normal themselves
 __device__ __forceinline__ Bf3 split3(float a, float b) {
   Bf3 out;
   const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
