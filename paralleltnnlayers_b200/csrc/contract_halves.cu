@@ -10,14 +10,17 @@
 //   D1[128 a][hi | mid | low] += G_hi (V_hi | V_mid | V_low) + G_mid (0 | V_hi | V_mid) + G_low (0 | 0 | V_hi)        K = 64
 //   D2[part, r][64 b | 64 b]  = V_part (G_hi | G_mid + G_low)                                                            K = 128
 // so the parts of V share an instruction, G_hi and G_mid one of twice the columns in D2.  D1 is added to totals in registers after each
-// tile, D2 goes out as a partial sum per 128 entries of a: no accumulator is longer than 64 (D1) or 128 terms.  An entry that met an infinite value
-// comes out NaN and is formed anew in fp32.
+// tile, D2 goes out as a partial sum per 128 entries of a: no accumulator is longer than 64 (D1) or 128 terms.
+// G and the vectors are lifted by 2^17 (as in kron_small.cu: the third part of a value is 2^-16 of it).  A tile in which one of them is above 2^43 or
+// infinite, or a product of two vectors below the smallest normal number, is multiplied in fp32 instead, one vector after the other (exact_tile).  (A NaN
+// makes the same sums NaN either way.)
 //
 // What bounds it: the phases of a tile follow one another, load - split - products - sums, and two CTAs per SM overlap only in part (issue 40 %,
 // shared memory 46 %, tensor pipe 19 %, DRAM 20 %; a tile takes 5000 cycles of an SM, of which G's 32 KB need 1400 and the
 // products, bound by what they read from shared memory, 1700).  G of 4096 x 4096 at R = 32: 54 us and 12 for the sums, mode by mode 104 + 23 + 9;
 // the layer's step with a batch of 4096 1460 -> 1405 us.  8x5x16x4 -> 5x10x12x4 at R = 201: 947 -> 161 us.
 #include <algorithm>
+#include <cfloat>
 
 #include "contract.cuh"
 #include "tc_common.cuh"
@@ -30,6 +33,7 @@ __device__ int g_halves_status = 0;   // 0 ok; otherwise (1 << 16) | (block inde
 
 constexpr int kHT = 256, kHA = 128, kHB = 64, kHR = 32;   // threads; entries of a and b and ranks of a tile
 constexpr int kPlaneG = kHA * 128, kVBlock = 3 * kHR * 128;   // bytes of a part of G, of the parts of V for 64 entries
+constexpr float kDrop = 1.f / (tc::kLift * tc::kLift), kLeastProduct = FLT_MIN * tc::kLift, kMost = 1.152921504606846976e18f;   // 2^60: no sum of 128 products overflows
 constexpr size_t kHalvesSmem = 1024 + 3 * kPlaneG + 3 * kVBlock;
 // The second product reads 128 rows of the 96 that VA's blocks have: the others are the block behind, VB's after the last, and
 // their results stay unread.
@@ -69,33 +73,75 @@ __device__ __forceinline__ int half_entry(const Half& h, int i, int (&e)[2]) {
     }
   return off;
 }
-__device__ __forceinline__ float half_value(const Half& h, const int* e, int R, int r) {
-  const float v = h.m[0].vec[(size_t)e[0] * R + r];
-  return h.n > 1 ? v * h.m[1].vec[(size_t)e[1] * R + r] : v;
-}
-
 struct HalfTable {   // of a tile
   int off[kHA], e[kHA][2];
 };
 
-// sums that met an infinite value (contract_peel.cu's order of a sum does not matter to them)
-__device__ __noinline__ float sum_over_b(const HalvesGeom& g, int offa, int b0, int b1, int r) {
-  float v = 0.f;
-  for (int b = b0; b < b1 && v == v; ++b) {
-    int e[2];
-    const int off = half_entry(g.b, b, e);
-    v = fmaf(g.G[offa + off], half_value(g.b, e, g.R, r), v);
+// A tile in fp32, the inner mode first as in contract_peel.cu: SB's sums to `out`, SA's to shared memory [r][a].  `sm` has the room of G's parts (G by
+// [a][b], then the values of b's outer mode by [b][r]), `inner` that of the parts of VB.  G of 4096 x 4096 at R = 32, all tiles this way: 430 us instead of 54.
+constexpr int kExactPitch = kHB + 4;
+static_assert((kHA * kExactPitch + kHB * kHR) * 4 <= 3 * kPlaneG && kHB * kHR * 4 <= kVBlock, "");
+__device__ __noinline__ void exact_tile(const HalvesGeom& g, float* sm, float* inner, const HalfTable& ta, const int* offb, const int (*eb)[2], int r0,
+                                        float* out) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = r0 + lane, rv = min(r, g.R - 1);
+  float *G = sm, *v0 = sm + kHA * kExactPitch, *v1 = inner;
+  const float *b0 = g.b.m[0].vec + rv, *b1 = g.b.m[g.b.n - 1].vec + rv, *a0 = g.a.m[0].vec + rv, *a1 = g.a.m[g.a.n - 1].vec + rv;
+#pragma unroll 8
+  for (int i = tid; i < kHA * kHB; i += kHT) {
+    const int a = i / kHB, b = i % kHB, oa = ta.off[a], ob = offb[b];
+    G[a * kExactPitch + b] = oa >= 0 && ob >= 0 ? g.G[oa + ob] : 0.f;
   }
-  return v;
-}
-__device__ __noinline__ float sum_over_a(const HalvesGeom& g, int offb, int a0, int a1, int r) {
-  float v = 0.f;
-  for (int a = a0; a < a1 && v == v; ++a) {
-    int e[2];
-    const int off = half_entry(g.a, a, e);
-    v = fmaf(g.G[off + offb], half_value(g.a, e, g.R, r), v);
+#pragma unroll
+  for (int b = warp; b < kHB; b += 8) {   // (past the end G is 0, and so are they: 0 times infinity)
+    v0[b * kHR + lane] = offb[b] >= 0 ? b0[(size_t)eb[b][0] * g.R] : 0.f;
+    v1[b * kHR + lane] = g.b.n > 1 && offb[b] >= 0 ? b1[(size_t)eb[b][1] * g.R] : 1.f;
   }
-  return v;
+  __syncthreads();
+  float v[8];   // of entries 8 * warp on of b
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = 0.f;
+  for (int a8 = 0; a8 < kHA; a8 += 8) {
+    float x[8], y[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int a = a8 + q;
+      x[q] = ta.off[a] >= 0 ? a0[(size_t)ta.e[a][0] * g.R] : 0.f;
+      y[q] = ta.off[a] >= 0 && g.a.n > 1 ? a1[(size_t)ta.e[a][1] * g.R] : 1.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4 *p = reinterpret_cast<const float4*>(G + (a8 + q) * kExactPitch + 8 * warp), c = p[0], d = p[1];
+      const float w[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = fmaf(w[i] * y[q], x[q], v[i]);
+    }
+  }
+  if (r < g.R)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (offb[8 * warp + i] >= 0) out[(size_t)(8 * warp + i) * g.R + lane] = v[i];
+  const int a = (warp & 3) * 32 + lane, j0 = (warp >> 2) * 16;
+  float w[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) w[j] = 0.f;
+  for (int b4 = 0; b4 < kHB; b4 += 4) {
+    const float4 c = *reinterpret_cast<const float4*>(G + a * kExactPitch + b4);
+    const float x[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) {
+        const float4 y = *reinterpret_cast<const float4*>(v1 + (b4 + b) * kHR + j0 + j), z = *reinterpret_cast<const float4*>(v0 + (b4 + b) * kHR + j0 + j);
+        w[j] = fmaf(x[b] * y.x, z.x, w[j]);
+        w[j + 1] = fmaf(x[b] * y.y, z.y, w[j + 1]);
+        w[j + 2] = fmaf(x[b] * y.z, z.z, w[j + 2]);
+        w[j + 3] = fmaf(x[b] * y.w, z.w, w[j + 3]);
+      }
+  }
+  __syncthreads();   // G and the values are read
+#pragma unroll
+  for (int j = 0; j < 16; ++j) sm[(j0 + j) * kHA + a] = w[j];
+  __syncthreads();
 }
 
 // VEC: rows of four entries of b are neighbours in G and 16-byte aligned
@@ -155,11 +201,29 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
         f[i][j] = v1[e[k][1] * g.R];
       }
   };
-  auto multiply_values = [&](const Half& h, const int* off) {
+  auto multiply_values = [&](const Half& h, const int* off) {   // true: a value is out of the range of the parts
+    float p[4][2], most = 0.f, least = FLT_MAX;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        p[i][j] = y[i][j] * tc::kLift;
+        if (h.n > 1) p[i][j] *= f[i][j];
+      }
+      most = tc::most_of(most, p[i][0], p[i][1]);
+      least = tc::least_of(least, p[i][0], p[i][1]);
+    }
+    bool out = most >= kMost;
+    if (h.n > 1 && least < kLeastProduct)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) out = out || (fabsf(p[i][j]) < kLeastProduct && y[i][j] != 0.f && f[i][j] != 0.f);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) y[i][j] = r < g.R && off[entry(i) + j] >= 0 ? (h.n > 1 ? y[i][j] * f[i][j] : y[i][j]) : 0.f;
+      for (int j = 0; j < 2; ++j) y[i][j] = r < g.R && off[entry(i) + j] >= 0 ? p[i][j] : 0.f;
+    return out;
   };
   auto split_values = [&](uint8_t* block) {
 #pragma unroll
@@ -172,10 +236,10 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
     }
   };
   load_values(g.a, ta.e);
-  multiply_values(g.a, ta.off);
+  bool outa = multiply_values(g.a, ta.off);
   split_values(va);
   load_values(g.a, ta.e + 64);
-  multiply_values(g.a, ta.off + 64);
+  outa = multiply_values(g.a, ta.off + 64) || outa;
   split_values(va + kVBlock);
 
   const uint64_t d0 = tc::make_smem_desc(0, 16, 1024, tc::kSwizzle128B);
@@ -208,10 +272,20 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
     }
   };
   load_values(g.b, tbe[0]);
-  multiply_values(g.b, tboff[0]);
+  bool outb = multiply_values(g.b, tboff[0]);
   grid_dependency_wait();   // G
   load_tile(0);
-  for (int s = 0; s < steps; ++s) {
+  for (int s = 0, issued = 0; s < steps; ++s) {
+    float most = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        x[i][j] *= tc::kLift;
+        x[i][j + 1] *= tc::kLift;
+        most = tc::most_of(most, x[i][j], x[i][j + 1]);
+      }
+    const bool out = outa || outb || most >= kMost;
     split_values(vb);
     load_values(g.b, tbe[(s + 1) % 3]);
 #pragma unroll
@@ -221,7 +295,8 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
       if constexpr (VEC) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const tc::Bf3 w0 = tc::split3(v[4 * k], v[4 * k + 1]), w1 = tc::split3(v[4 * k + 2], v[4 * k + 3]);
+          const tc::Bf3 w0 = tc::split3(v[4 * k], v[4 * k + 1]),
+                        w1 = tc::split3(v[4 * k + 2], v[4 * k + 3]);
           const int row = 2 * k + (lane >> 4);
           uint8_t* o = d + row * 128 + ((((lane & 15) >> 1) ^ row) << 4) + (lane & 1) * 8;
 #pragma unroll
@@ -238,8 +313,8 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
       }
     }
     tc::fence_proxy_async();
-    __syncthreads();
-    if (warp == 0 && tc::elect_one()) {
+    const bool exact = __syncthreads_or(out);
+    if (!exact && warp == 0 && tc::elect_one()) {
       tc::tc_fence_after_sync();
       const uint64_t gd2 = tc::make_smem_desc(0, kPlaneG, 1024, tc::kSwizzle128B) + (tc::smem_u32(sm) >> 4);   // (64 rows on: the next part)
       const uint64_t gd = d0 + (tc::smem_u32(sm) >> 4), ad = d0 + (tc::smem_u32(va) >> 4), bd = d0 + (tc::smem_u32(vb) >> 4);
@@ -259,13 +334,21 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
     }
     __syncwarp();
     if (s + 1 < steps) load_tile(s + 1);
-    multiply_values(g.b, tboff[(s + 1) % 3]);
+    outb = multiply_values(g.b, tboff[(s + 1) % 3]);
     if (tid >= kHT - kHB) table_b(s + 2, tid - (kHT - kHB));
-    fine = tc::mbar_wait(&done, s & 1) && fine;   // (the other CTA of the SM works meanwhile)
+    float* dst = g.sb + ((size_t)blockIdx.x * g.b.size + (size_t)(t0 + s) * kHB) * g.R + r0;
+    float* sums = reinterpret_cast<float*>(sm);
+    if (exact) {
+      exact_tile(g, sums, reinterpret_cast<float*>(vb), ta, tboff[s % 3], tbe[s % 3], r0, dst);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) tot[j] += sums[(grp * 16 + j) * kHA + quarter * 32 + lane];
+      __syncthreads();   // the sums are read
+      continue;
+    }
+    fine = tc::mbar_wait(&done, issued++ & 1) && fine;   // (the other CTA of the SM works meanwhile)
     __syncwarp();
     tc::tc_fence_after_sync();
-    float* sums = reinterpret_cast<float*>(sm);   // [part][b][r]: the parts of G are used up
-    {
+    {   // sums by [part][b][r]: the parts of G are used up
       float v[16], w[16];
       tc::tmem_ld16(lanes + 2 * kHR + grp * 16, v);
       tc::tmem_ld16(lanes + kHR + grp * 16, w);
@@ -273,7 +356,7 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
       for (int j = 0; j < 16; ++j) v[j] += w[j];
       tc::tmem_ld16(lanes + grp * 16, w);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) tot[j] += w[j] + v[j];
+      for (int j = 0; j < 16; ++j) tot[j] = fmaf(w[j] + v[j], kDrop, tot[j]);
       if (quarter < 3) {
 #pragma unroll
         for (int j0 = 0; j0 < 32; j0 += 16) {
@@ -287,22 +370,12 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
     tc::tc_fence_before_sync();
     __syncthreads();   // and the accumulators are free
     const int* off = tboff[s % 3];
-    float* out = g.sb + ((size_t)blockIdx.x * g.b.size + (size_t)(t0 + s) * kHB) * g.R + r;
-    float v[kHB / 8];
-    bool nan = false;
-#pragma unroll
-    for (int i = 0; i < kHB / 8; ++i) {
-      const float* p = sums + (warp + i * 8) * kHR + lane;
-      v[i] = p[0] + (p[kHB * kHR] + p[2 * kHB * kHR]);
-      nan = nan || v[i] != v[i];
-    }
     if (r < g.R) {
 #pragma unroll
-      for (int i = 0; i < kHB / 8; ++i)
-        if (off[warp + i * 8] >= 0) out[(size_t)(warp + i * 8) * g.R] = v[i];
-      if (nan)
-        for (int b = warp; b < kHB; b += 8)
-          if (off[b] >= 0 && out[(size_t)b * g.R] != out[(size_t)b * g.R]) out[(size_t)b * g.R] = sum_over_a(g, off[b], a0, a0 + arows, r);
+      for (int i = 0; i < kHB / 8; ++i) {
+        const float* p = sums + (warp + i * 8) * kHR + lane;
+        if (off[warp + i * 8] >= 0) dst[(size_t)(warp + i * 8) * g.R + lane] = (p[0] + (p[kHB * kHR] + p[2 * kHB * kHR])) * kDrop;
+      }
     }
     __syncthreads();   // the sums are read
   }
@@ -312,15 +385,9 @@ __global__ void __launch_bounds__(kHT, 2) halves_kernel(const __grid_constant__ 
   if (a < arows) {
     float* out = g.sa + ((size_t)blockIdx.y * g.a.size + a0 + a) * g.R + r0 + grp * 16;
     const int have = g.R - r0 - grp * 16;
-    bool nan = false;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < 16; ++j)
       if (j < have) out[j] = tot[j];
-      nan = nan || tot[j] != tot[j];
-    }
-    if (nan)
-      for (int j = 0; j < min(16, have); ++j)
-        if (out[j] != out[j]) out[j] = sum_over_b(g, ta.off[a], t0 * kHB, min(g.b.size, (t0 + steps) * kHB), r0 + grp * 16 + j);
   }
   tc::tc_fence_before_sync();
   __syncthreads();
