@@ -86,3 +86,19 @@ def test_rcp(idims, odims, R):
     want = _gradients(_by_pairs(G, idims, odims), [S.double().reshape(9, R)] + _vectors(F))
     _check([dS, *dF], want, [S.shape, *[f.shape for f in F]])
     P.device_status()
+
+
+@pytest.mark.parametrize("idims, odims, R", [((15, 9, 7), (16, 5, 13), 31), ((16, 16, 16), (4, 8, 4), 32), ((8, 4, 4, 4), (4, 8, 4, 4), 20)], ids=str)
+def test_sums_of_one_sign(idims, odims, R):
+    """What the tensor core cuts off has one sign.  A dense gradient of whole numbers (one sample, exact) and positive factors: a unit of fp32, 2**-23 in the
+    norm, half of it for what is rounded (the product of two vectors, sums of tiles and of parts), half for what is cut off."""
+    import paralleltnnlayers_b200 as P
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    whole = lambda n: torch.randint(1, 2048, (1, n), generator=gen, device="cuda").float()
+    x, dy = whole(math.prod(idims)), whole(math.prod(odims))
+    F = [torch.rand(i, o, R, generator=gen, device="cuda") + 0.01 for i, o in zip(idims, odims)]
+    got = P.dense_cp_backward(x, dy, *F)[1]
+    want = _gradients(_by_pairs(dy.double().T @ x.double(), idims, odims), _vectors(F))
+    for g, w in zip(got, want):
+        w = w.reshape(g.shape)
+        assert float((g.double() - w).norm() / w.norm()) < 2 ** -23
