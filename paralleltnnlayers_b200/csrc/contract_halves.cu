@@ -525,10 +525,11 @@ HalvesPlan halves_plan(int L, const int* sizes, int R) {
 // modes from 1e6 0.17 to 0.69, taps and three modes from 1e5 0.36 to 0.88, taps and two modes 0.62 to 1.08, three modes from 5e5 0.53 to 1.15 (0.83 in
 // the mean), of fewer 0.63 to 1.48 (1.0 in the mean).
 bool halves_take(int L, const int* sizes, bool has_s) {
-  if (L < 3 || L > 4) return false;
+  const int mode = gemm_tc_mode();   // 0: no tensor products, 2: at every size
+  if (L < 3 || L > 4 || !mode) return false;
   double entries = 1;
   for (int k = 0; k < L; ++k) entries *= sizes[k];
-  return entries >= (L == 3 && !has_s ? 5e5 : 1e5) && entries < 2147483647.0;
+  return (mode == 2 || entries >= (L == 3 && !has_s ? 5e5 : 1e5)) && entries < 2147483647.0;
 }
 
 size_t halves_scratch_floats(int L, const int* sizes, int R) {

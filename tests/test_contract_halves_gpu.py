@@ -102,3 +102,32 @@ def test_sums_of_one_sign(idims, odims, R):
     for g, w in zip(got, want):
         w = w.reshape(g.shape)
         assert float((g.double() - w).norm() / w.norm()) < 2 ** -23
+
+
+def _kernels(call):
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return " ".join(e.key for e in p.key_averages())
+
+
+def test_mode(monkeypatch):
+    """B200CP_GEMM_TC=0 keeps the contraction off the tensor cores at any size, 2 takes it there at any."""
+    import paralleltnnlayers_b200 as P
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    normal = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    large = [normal(i, o, 5) for i, o in zip((15, 13, 16), (13, 14, 15))]
+    x, dy = normal(3, 15 * 13 * 16), normal(3, 13 * 14 * 15)
+    small = [normal(i, o, 7) for i, o in zip(*RCP[-1][:2])]
+    S, u, dv = normal(3, 3, 7), normal(2, 64, 6, 5), normal(2, 96, 6, 5)
+    calls = [lambda: P.dense_cp_backward(x, dy, *large)[1], lambda: P.rcp_conv2d_backward(u, dv, *small, S)[1]]
+    for call in calls:
+        out = {}
+        for mode, here, other in (("2", "halves_kernel", "peel_"), ("0", "peel_", "halves_")):
+            monkeypatch.setenv("B200CP_GEMM_TC", mode)
+            out[mode] = call()
+            names = _kernels(call)
+            assert here in names and other not in names
+        for a, b in zip(out["0"], out["2"]):
+            assert float((a - b).norm() / b.norm()) < 1e-6
