@@ -11,7 +11,7 @@ struct PeelMode {
   const float* vec;  // [nc * nt][R]
 };
 
-bool halves_take(int L, const int* sizes, bool has_s);
+bool halves_take(int L, const int* sizes, int R, bool has_s);
 size_t halves_scratch_floats(int L, const int* sizes, int R);
 int halves_launch(int L, const PeelMode* modes, int R, const float* G, float* const* grads, float* scratch, cudaStream_t st);
 int halves_device_status(int* out);

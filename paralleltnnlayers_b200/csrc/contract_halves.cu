@@ -520,16 +520,23 @@ HalvesPlan halves_plan(int L, const int* sizes, int R) {
 
 }  // namespace
 
-// Three modes from half a million entries of G, four, and the taps with two or three, from 1e5; with fewer the set-up weighs more than the
-// pass, and two modes have at most 65536.  180 drawn layers of 4e4 to 1.7e7 entries and 4 to 256 ranks, kernel times against the peeled ones: four
-// modes from 1e6 0.17 to 0.69, taps and three modes from 1e5 0.36 to 0.88, taps and two modes 0.62 to 1.08, three modes from 5e5 0.53 to 1.15 (0.83 in
-// the mean), of fewer 0.63 to 1.48 (1.0 in the mean).
-bool halves_take(int L, const int* sizes, bool has_s) {
+// Where this is faster than the peel.  2100 drawn layers of 4e4 to 1e7 entries and 4 to 256 ranks, kernel times over the peeled ones where the rule takes it,
+// and where it does not:
+//   three modes           2e6 entries, or 7e5 where the first is alone a; three tiles of b      0.45 to 1.03 (mean 0.73)   0.63 to 1.53 (0.95)
+//   taps and two modes    1e5 entries, three tiles of b and 96 ranks at most                    0.57 to 0.96 (0.72)        0.59 to 1.55 (0.89)
+//   four, taps and three  1e5 entries and three tiles of a, or 4e5 entries                      0.09 to 1.03 (0.63)        0.40 to 1.39 (0.85)
+// A side of fewer tiles leaves most of an SM's time to the set-up; near these lines the times are 18 to 30 us.  (Two modes have at most 65536 entries.)
+bool halves_take(int L, const int* sizes, int R, bool has_s) {
   const int mode = gemm_tc_mode();   // 0: no tensor products, 2: at every size
   if (L < 3 || L > 4 || !mode) return false;
   double entries = 1;
   for (int k = 0; k < L; ++k) entries *= sizes[k];
-  return (mode == 2 || entries >= (L == 3 && !has_s ? 5e5 : 1e5)) && entries < 2147483647.0;
+  if (entries >= 2147483647.0) return false;
+  if (mode == 2) return true;
+  const HalvesPlan p = halves_plan(L, sizes, R);
+  if (L == 4) return entries >= 4e5 || (entries >= 1e5 && p.atiles >= 3);
+  if (has_s) return entries >= 1e5 && p.btiles >= 3 && R <= 96;
+  return entries >= (p.na == 1 ? 7e5 : 2e6) && p.btiles >= 3;
 }
 
 size_t halves_scratch_floats(int L, const int* sizes, int R) {

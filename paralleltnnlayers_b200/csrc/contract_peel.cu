@@ -339,7 +339,7 @@ void peel_plan(PeelPlan& pl, int order, const int* cdims, const int* tdims, int 
 size_t contract_scratch_floats(int order, const int* cdims, const int* tdims, int R, int taps, bool has_s) {
   PeelPlan pl;
   peel_plan(pl, order, cdims, tdims, R, taps, has_s);
-  if (halves_take(pl.L, pl.nmode, has_s)) return halves_scratch_floats(pl.L, pl.nmode, R);
+  if (halves_take(pl.L, pl.nmode, R, has_s)) return halves_scratch_floats(pl.L, pl.nmode, R);
   return pl.s_floats[0] + pl.s_floats[1] + pl.part_floats + 8;
 }
 
@@ -375,7 +375,7 @@ int contract_factors_launch(int order, const int* cdims, const int* tdims, int R
   for (int k = 0; k < L; ++k)
     if (modes[k].nc * modes[k].nt > kMaxNb)
       return fail(B200CP_ERR_UNSUPPORTED, "factor contraction: a mode has %d > %d entries", modes[k].nc * modes[k].nt, kMaxNb);
-  if (halves_take(L, pl.nmode, S != nullptr)) return halves_launch(L, modes, R, G, grads, scratch, st);
+  if (halves_take(L, pl.nmode, R, S != nullptr)) return halves_launch(L, modes, R, G, grads, scratch, st);
   float* sbuf[2] = {scratch, scratch + ((pl.s_floats[0] + 3) & ~size_t(3))};
   float* part = sbuf[1] + ((pl.s_floats[1] + 3) & ~size_t(3));
   const float* src = G;
