@@ -526,6 +526,25 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
         ls[i] = *reinterpret_cast<const uint4*>(src + 2048);
         oas[i] = ta.o[quarter * 32 + row];
       }
+      // Rows of odd length begin anywhere: where the lanes' runs are not on a grid of four, a lane has a column and the warp a row at a time (a lane's
+      // eight values one by one are a sector each: 14x11x11 -> 12x15x12 at R = 21 54 us, this way 25, FFMA 39).
+      bool grid4 = run4 && next4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) grid4 = grid4 && !((oas[i] + ob) & 3) && !((oas[i] + t.o[c + 4]) & 3);
+      if (!__all_sync(0xffffffffu, left <= 0 || grid4)) {
+        const int col = c0 + lane, oc = t.o[col];
+#pragma unroll 4
+        for (int row = 0; row < 32; ++row) {
+          const uint8_t* src = stage + row * 64 + (((lane >> 3) ^ (row >> 1)) & 3) * 16 + (lane & 7) * 2;
+          const int o = ta.o[quarter * 32 + row] + oc;
+          if (a0 + quarter * 32 + row < PA && b0 + col < PB) {
+            hi[o] = *reinterpret_cast<const __half*>(src);
+            hi[plane + o] = *reinterpret_cast<const __half*>(src + 2048);
+          }
+        }
+        __syncwarp();
+        continue;
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int a = quarter * 32 + i * 8 + (lane >> 2), oa = oas[i], o = oa + ob;
@@ -536,23 +555,12 @@ __global__ void __launch_bounds__(256, 2) kron_planes_kernel(const __grid_consta
           *reinterpret_cast<uint4*>(hi + plane + o) = l;
           continue;
         }
-        const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, lw[4] = {l.x, l.y, l.z, l.w};
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int oq = oa + t.o[c + q * 4];
-          if ((q ? next4 : run4) && !(oq & 3)) {
-            *reinterpret_cast<uint2*>(hi + oq) = make_uint2(hw[q * 2], hw[q * 2 + 1]);
-            *reinterpret_cast<uint2*>(hi + plane + oq) = make_uint2(lw[q * 2], lw[q * 2 + 1]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (q * 4 + j < left) {
-                const int oj = oa + t.o[c + q * 4 + j];
-                hi[oj] = __ushort_as_half((unsigned short)(hw[q * 2 + j / 2] >> (j & 1) * 16));
-                hi[plane + oj] = __ushort_as_half((unsigned short)(lw[q * 2 + j / 2] >> (j & 1) * 16));
-              }
-          }
-        }
+        if (left <= 0) continue;
+        const int o4 = oa + t.o[c + 4];
+        *reinterpret_cast<uint2*>(hi + o) = make_uint2(h.x, h.y);
+        *reinterpret_cast<uint2*>(hi + plane + o) = make_uint2(l.x, l.y);
+        *reinterpret_cast<uint2*>(hi + o4) = make_uint2(h.z, h.w);
+        *reinterpret_cast<uint2*>(hi + plane + o4) = make_uint2(l.z, l.w);
       }
       __syncwarp();   // (an entry formed anew replaces what another lane has stored)
     }

@@ -40,3 +40,9 @@ def test_weight_planes(idims, odims, R, turned, monkeypatch):
     # an output against its row of the weight (the output itself may be a small difference): no row is worse than four times the mean
     assert float((off.norm(dim=0) / W.norm(dim=0)).max()) < 19 ** 0.5 * 2e-6
     P.device_status()
+
+
+@pytest.mark.parametrize("turned", [False, True])
+def test_rows_off_the_grid(turned, monkeypatch):
+    """Runs of 84 neighbours (eight bytes of a plane at a time) and of 63 (a row at a time), the last tile of a half not full."""
+    test_weight_planes((9, 7, 7, 12), (8, 7, 9, 7), 21, turned, monkeypatch)
