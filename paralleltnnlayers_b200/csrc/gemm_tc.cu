@@ -29,6 +29,7 @@
 // Roles (TMA warp, MMA warp, read-out warps) meet only through mbarriers; every wait is bounded, and a wait that
 // runs out sets a status word and lets the CTA leave through its normal exit (TMEM released).
 #include <algorithm>
+#include <cfloat>
 #include <cstdio>
 #include <cstdlib>
 
@@ -495,7 +496,8 @@ split_gemm_kernel(const __grid_constant__ SplitGemm g, const __grid_constant__ C
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) arrive_cluster(leader_addr(accfreeb + buf * 8));
-      if (MN && *edges) edge_pixels<BN>(g, unit);
+      if constexpr (MN)
+        if (*edges) edge_pixels<BN>(g, unit);
     }
   }
   tc_fence_before_sync();
@@ -693,6 +695,7 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
     const bool in = p < rows && h < im.H && w < im.W;
     const float* s = job.src + (((size_t)n * CH) * im.H + h) * im.W + w;
     unsigned m = 0;
+    float most = 0.f;      // (three-way maxima of floats: a third of the instructions)
     constexpr int B = 8;   // quads of a thread whose loads are in flight together
     for (int k0 = ty; k0 < quads; k0 += 8 * B) {
       float v[B][4];
@@ -707,11 +710,12 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
       for (int j = 0; j < B; ++j)
         if (k0 + j * 8 < quads) {
           tile[(k0 + j * 8) * kPxPitch + tx] = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
-          m = max(m, max(max(abs_bits(v[j][0]), abs_bits(v[j][1])), max(abs_bits(v[j][2]), abs_bits(v[j][3]))));
+          if (THREE) most = most_nan(most_nan(most, v[j][0], v[j][1]), v[j][2], v[j][3]);
+          else m = max(m, max(max(abs_bits(v[j][0]), abs_bits(v[j][1])), max(abs_bits(v[j][2]), abs_bits(v[j][3]))));
         }
     }
     if (THREE) {
-      const bool edge = h < im.padH || h >= im.H - im.padH || w < im.padW || w >= im.W - im.padW, drop = im.dropped && edge && m >= 0x7f800000u;
+      const bool edge = h < im.padH || h >= im.H - im.padH || w < im.padW || w >= im.W - im.padW, drop = im.dropped && edge && !(most <= FLT_MAX);
       if (drop)   // (see edge_pixels)
         for (int k = ty; k < quads; k += 8) {
           float4& v = tile[k * kPxPitch + tx];
@@ -736,25 +740,33 @@ __global__ void __launch_bounds__(256, 4) split_pixels_kernel(const __grid_const
     }
     __syncthreads();
   }
-  // a warp writes the channels of a pixel, four per lane
-  for (int k = tx; k < quads; k += 32) {
+  const auto put = [&](int i, int k) {
+    uint16_t* d = job.hi + (size_t)(p0 + i) * job.ldo + 4 * k;
+    const float4 v = tile[k * kPxPitch + i];
+    if (THREE) {
+      const Bf3 x = split3(v.x, v.y), y = split3(v.z, v.w);
 #pragma unroll
-    for (int j = 0; j < kPxTile / 8; ++j) {
-      const int i = ty + j * 8;
-      if (p0 + i >= rows) break;
-      uint16_t* d = job.hi + (size_t)(p0 + i) * job.ldo + 4 * k;
-      const float4 v = tile[k * kPxPitch + i];
-      if (THREE) {
-        const Bf3 x = split3(v.x, v.y), y = split3(v.z, v.w);
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(d + q * job.plane) = make_uint2(x.p[q], y.p[q]);
+    } else {
+      Half4 h, l;
+      split4(v, scale[i], h, l);
+      *reinterpret_cast<Half4*>(d) = h;
+      *reinterpret_cast<Half4*>(d + job.plane) = l;
+    }
+  };
+  if (quads > 16) {   // a warp writes the channels of a pixel, four per lane
+    for (int k = tx; k < quads; k += 32) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(d + q * job.plane) = make_uint2(x.p[q], y.p[q]);
-      } else {
-        Half4 h, l;
-        split4(v, scale[i], h, l);
-        *reinterpret_cast<Half4*>(d) = h;
-        *reinterpret_cast<Half4*>(d + job.plane) = l;
+      for (int j = 0; j < kPxTile / 8; ++j) {
+        const int i = ty + j * 8;
+        if (p0 + i >= rows) break;
+        put(i, k);
       }
     }
+  } else {            // of several: pairs of 19 images of 32 channels 29x29 4.75 -> 4.27 us (4.19 where a lane had two channels)
+    const int log = quads > 8 ? 4 : quads > 4 ? 3 : 2, k = tx & ((1 << log) - 1);
+    for (int i = (ty * 32 + tx) >> log; i < kPxTile; i += 256 >> log)
+      if (k < quads && p0 + i < rows) put(i, k);
   }
 }
 
