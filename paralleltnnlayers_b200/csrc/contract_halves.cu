@@ -18,10 +18,10 @@
 // infinite, or a product of two vectors below the smallest normal number, is multiplied in fp32 instead, one vector after the other (exact_tile).  (A NaN
 // makes the same sums NaN either way.)
 //
-// What bounds it: the phases of a tile follow one another, load - split - products - sums, and two CTAs per SM overlap only in part (issue 40 %,
-// shared memory 46 %, tensor pipe 19 %, DRAM 20 %; a tile takes 5000 cycles of an SM, of which G's 32 KB need 1400 and the
-// products, bound by what they read from shared memory, 1700).  G of 4096 x 4096 at R = 32: 54 us and 12 for the sums, mode by mode 104 + 23 + 9;
-// the layer's step with a batch of 4096 1460 -> 1405 us.  8x5x16x4 -> 5x10x12x4 at R = 201: 947 -> 161 us.
+// What bounds it: the phases of a tile follow one another, load - split - products - sums, and two CTAs per SM overlap only in part (issue 45 %,
+// shared memory 47 %, tensor pipe 22 %, DRAM 16 %; a tile takes 5000 cycles of an SM, of which G's 32 KB need 1400 and the
+// products, bound by what they read from shared memory, 1700).  G of 4096 x 4096 at R = 32: 52 us and 12 for the sums, mode by mode 104 + 26 + 9;
+// the layer's step with a batch of 4096 1812 -> 1699 us with the weight's planes of kron_small.cu.  5x13x11 -> 13x7x7 at R = 246 362 -> 130 us.
 #include <algorithm>
 #include <cfloat>
 

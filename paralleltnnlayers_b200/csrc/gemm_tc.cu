@@ -1045,7 +1045,7 @@ bool dense_tc_takes() { return gemm_tc_mode() && get_encode_tiled() != nullptr; 
 double dense_tc_us(int B, int K, int N, const KronWeight& w) {
   DeviceInfo di;
   if (device_info(&di)) return 1e300;
-  const double entries = (double)N * K;   // as planes, 2^24 entries: 38 us at R = 4, 41 at 32, 55 at 64, 192 at 256
+  const double entries = (double)N * K;   // as planes, 2^24 entries: 38 us at R = 4, 42 at 32, 58 at 64, 213 at 256
   const double weight = kron_planes_takes(w.order, w.idims, w.odims, w.R, di.sm_count)
                             ? 8.0 + entries * (1.35e-6 + (w.R <= 64 ? 2.2e-8 : 4.0e-8) * w.R)
                             : kron_weight_us(w.order, w.idims, w.odims, w.R, 1, w.transposed) + split_us(entries);

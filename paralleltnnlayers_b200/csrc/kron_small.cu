@@ -1168,7 +1168,7 @@ int kron_weight_launch(int order, const int* idims, const int* odims, int R, con
   return B200CP_OK;
 }
 
-// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 41 us with the exponents, against 86 for the fp32 weight and
+// Large weights, whose 128 x 128 tiles fill the GPU: 4096 x 4096 at R = 32 42 us with the exponents, against 86 for the fp32 weight and
 // its split; but 1000 x 1000 at R = 16 21 against 13, 4096 x 64 at R = 64 50 against 20.
 bool kron_planes_takes(int order, const int* idims, const int* odims, int R, int sm_count) {
   double pa = 1, pb = 1;
